@@ -293,6 +293,13 @@ int64_t mlpsp_group_records_scratch_bytes(int64_t num_records, int32_t n);
 int mlpsp_group_records(const int32_t* primitive_ids, int64_t num_records, int32_t n, int64_t* offsets,
                         int64_t* order, void* scratch, int64_t scratch_bytes, void* stream);
 
+/* group_records with the records' rows: additionally writes x6_out[R,6] = x6[order], grad4_out[R,4] = grad4[order] and
+ * masks_out[R,2] = relu_masks[order] (each pair NULL when not wanted), in the launch that writes the permutation.
+ * x6 and masks 8-byte, grad4 16-byte aligned; scratch as mlpsp_group_records. */
+int mlpsp_group_rows(const int32_t* primitive_ids, int64_t num_records, int32_t n, const float* x6, const float* grad4,
+                     const int32_t* relu_masks, int64_t* offsets, int64_t* order, float* x6_out, float* grad4_out,
+                     int32_t* masks_out, void* scratch, int64_t scratch_bytes, void* stream);
+
 /* prepare_groups (primitive_gemm.py:186-203): split every primitive's records into segments of at
  * most segment_size.  group_offsets[n+1] int64 is always written; of primitives/starts ([G] int64, may be
  * NULL) the first min(G, max_groups) entries are written, so a caller may ask for G first (max_groups = 0)
@@ -329,6 +336,19 @@ int mlpsp_records_reverse(const int32_t* ids, const int64_t* offsets, const floa
                           int64_t pixels, int64_t total_records, int32_t n, float* d4, float* grad_pos,
                           float* grad_log_scales, float* grad_quats, void* stream);
 
+/* The same with the caller's scratch (mlpsp_records_reverse takes it from the stream's memory pool) and with the
+ * argument checks on the device: *findings_host (HOST, or NULL) receives an OR of the bits below (0: none), for which
+ * the call waits for the checks -- not for the gradients; with a bit set the outputs are undefined.  grad_quats must be
+ * 16-byte aligned as well. */
+#define MLPSP_REVERSE_BAD_OFFSETS 1  /* offsets do not start at zero, end at total_records or ascend */
+#define MLPSP_REVERSE_BAD_IDS 2      /* an id outside [0, n) */
+int64_t mlpsp_records_reverse_scratch_bytes(int64_t total_records, int32_t n);
+int mlpsp_records_reverse_checked(const int32_t* ids, const int64_t* offsets, const float* x6, const float* raw,
+                                  const float* log_scales, const float* quats, const float* grad_rgb, const float* grad_t,
+                                  int64_t pixels, int64_t total_records, int32_t n, float* d4, float* grad_pos,
+                                  float* grad_log_scales, float* grad_quats, void* scratch, int64_t scratch_bytes,
+                                  int32_t* findings_host, void* stream);
+
 /* Floats per primitive of the packed gradient row: W1[32,72] b1[32] W2[32,32] b2[32] W3[4,32] b3[4] = 3,524. */
 int64_t mlpsp_grouped_gradient_floats(void);
 
@@ -344,11 +364,22 @@ int64_t mlpsp_grouped_gradient_floats(void);
  * binary16, 1 otherwise).  *nonfinite: bit 0 = a sum is not finite -- the caller retries a mixed-precision call
  * with MLPSP_PRECISION_F32 and loss_scale 1 as primitive_gemm.py:64-98 does (the host mirror does);
  * bit 1 = a device-side wait gave up, results invalid. */
+/* The segments follow from the offsets and segment_size, so the call plans them itself (seg_prim, seg_start, seg_offsets
+ * and partial are checked and otherwise unused; its scratch comes from the stream's memory pool). */
 int mlpsp_grouped_weight_gradients(const mlpsp_scene* scene, const int64_t* offsets, const float* x6, const float* d4,
                                    const int32_t* relu_masks, const int64_t* seg_prim, const int64_t* seg_start,
                                    const int64_t* seg_offsets, int64_t num_segments, int32_t segment_size,
                                    int32_t precision, float loss_scale, float* partial, float* result,
                                    int32_t* nonfinite, void* stream);
+
+/* The same gradients written to the six gradient tensors (dW1[n,32,72] db1[n,32] dW2[n,32,32] db2[n,32] dW3[n,4,32]
+ * db3[n,4]), with the caller's scratch and without a prepared layout.  num_records = offsets[n].  *nonfinite_host (HOST)
+ * receives the flag word described above; the call waits for it. */
+int64_t mlpsp_weight_gradients_scratch_bytes(int64_t num_records, int32_t n, int32_t segment_size);
+int mlpsp_weight_gradients(const mlpsp_scene* scene, const int64_t* offsets, const float* x6, const float* d4,
+                           const int32_t* relu_masks, int64_t num_records, int32_t segment_size, int32_t precision,
+                           float loss_scale, float* dW1, float* db1, float* dW2, float* db2, float* dW3, float* db3,
+                           void* scratch, int64_t scratch_bytes, int32_t* nonfinite_host, void* stream);
 
 /* ---- the step after the feature map: feature decoder and text query ---- */
 

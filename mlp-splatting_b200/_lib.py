@@ -19,6 +19,7 @@ BIT_PAIR_OVERFLOW, BIT_RECORD_OVERFLOW, BIT_NUMERIC, BIT_TIMEOUT = 8, 16, 64, 12
 BIT_TILE_ORIGINS, BIT_CONE_TOO_WIDE, BIT_FEAT_INEXACT = 256, 512, 1024
 BIT_PIXEL_HITS = 32
 ORDER_PER_PIXEL = 2
+REVERSE_BAD_OFFSETS, REVERSE_BAD_IDS = 1, 2
 PRECISION_F32, PRECISION_F16, PRECISION_BF16 = 0, 1, 2
 MAX_WAVES = 32
 GEOM_FLOATS = 16
@@ -72,9 +73,15 @@ _SIGS = {
     "mlpsp_pack_weights_bf16": (C.c_int, [C.POINTER(Scene), _fp, _fp, _fp]),
     "mlpsp_pack_features_f16": (C.c_int, [C.POINTER(Scene), _fp, _fp, _fp]),
     "mlpsp_records_reverse": (C.c_int, [_fp, _fp, _fp, _fp, _fp, _fp, _fp, _fp, C.c_int64, C.c_int64, C.c_int32, _fp, _fp, _fp, _fp, _fp]),
+    "mlpsp_records_reverse_scratch_bytes": (C.c_int64, [C.c_int64, C.c_int32]),
+    "mlpsp_records_reverse_checked": (C.c_int, [_fp, _fp, _fp, _fp, _fp, _fp, _fp, _fp, C.c_int64, C.c_int64, C.c_int32, _fp, _fp,
+                                                _fp, _fp, _fp, C.c_int64, _fp, _fp]),
     "mlpsp_grouped_gradient_floats": (C.c_int64, []),
     "mlpsp_grouped_weight_gradients": (C.c_int, [C.POINTER(Scene), _fp, _fp, _fp, _fp, _fp, _fp, _fp, C.c_int64, C.c_int32,
                                                  C.c_int32, C.c_float, _fp, _fp, _fp, _fp]),
+    "mlpsp_weight_gradients_scratch_bytes": (C.c_int64, [C.c_int64, C.c_int32, C.c_int32]),
+    "mlpsp_weight_gradients": (C.c_int, [C.POINTER(Scene), _fp, _fp, _fp, _fp, C.c_int64, C.c_int32, C.c_int32, C.c_float,
+                                         _fp, _fp, _fp, _fp, _fp, _fp, _fp, C.c_int64, _fp, _fp]),
     "mlpsp_decoder_packed_bytes": (C.c_int64, [C.POINTER(Decoder), C.c_int32]),
     "mlpsp_pack_decoder": (C.c_int, [C.POINTER(Decoder), C.c_int32, _fp, _fp, _fp]),
     "mlpsp_decode_features": (C.c_int, [C.POINTER(Decoder), C.c_int32, _fp, _fp, C.c_int32, C.c_int32, _fp, _fp, _fp, _fp]),
@@ -99,6 +106,7 @@ _SIGS = {
     "mlpsp_mlp_grouped": (C.c_int, [C.POINTER(Scene), C.c_int32, _fp, _fp, C.c_int64, _fp, _fp, C.c_int64, _fp, _fp]),
     "mlpsp_group_records_scratch_bytes": (C.c_int64, [C.c_int64, C.c_int32]),
     "mlpsp_group_records": (C.c_int, [_fp, C.c_int64, C.c_int32, _fp, _fp, _fp, C.c_int64, _fp]),
+    "mlpsp_group_rows": (C.c_int, [_fp, C.c_int64, C.c_int32, _fp, _fp, _fp, _fp, _fp, _fp, _fp, _fp, _fp, C.c_int64, _fp]),
     "mlpsp_prepare_groups": (C.c_int, [_fp, C.c_int32, C.c_int64, _fp, _fp, _fp, C.c_int64, C.POINTER(C.c_int64), _fp]),
     "mlpsp_prepare_groups_static": (C.c_int, [_fp, C.c_int32, C.c_int64, _fp, _fp, _fp, C.c_int64, C.POINTER(C.c_int64), _fp]),
 }

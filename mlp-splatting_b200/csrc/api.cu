@@ -8,6 +8,23 @@ namespace mlpsp {
 
 static thread_local char g_err[512] = "";
 
+int sm_count() {
+  static int known[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  if (!known[dev]) {
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    known[dev] = sms;
+  }
+  return known[dev];
+}
+
+HostWords& host_words() {
+  static thread_local HostWords w;
+  return w;
+}
+
 void set_error(const char* fmt, ...) {
   va_list ap;
   va_start(ap, fmt);

@@ -10,11 +10,11 @@
 // per primitive, with its records' encoded inputs E, saved ReLU masks and output adjoints D3,
 //   D2 = (D3 W3) * mask2,  D1 = (D2 W2) * mask1,
 //   dW3 = D3^T H2, db3 = sum D3, dW2 = D2^T H1, db2 = sum D2, dW1 = D1^T E, db1 = sum D1.
-// One CTA handles one prepared segment of one primitive in blocks of 128 records (thread = record for the
-// forward recomputation and the adjoints, then thread = output element for the D^T X products over the block
-// in shared memory) and writes a partial 3,524-vector; a second kernel adds a primitive's partials in segment
-// order, so the result does not depend on scheduling, and raises the non-finite flag.
+// A segment (at most segment_size records of one primitive) is summed by one CTA.  A primitive with one segment, the
+// usual case, gets its gradients straight from that CTA; the partial 3,524-vectors of the others are added in segment
+// order by a second kernel, so the result does not depend on scheduling.
 #include "frame.cuh"
+#include "vjp.cuh"
 
 namespace mlpsp {
 
@@ -70,30 +70,64 @@ __device__ __forceinline__ void quat_adjoint(float w, float x, float y, float z,
 // The reference walks a pixel's records backwards in one thread and issues ten (warp-aggregated) global atomics per
 // record from inside that walk (primitive_records.cuh:3-49).  Here the walk is reduced to what is sequential -- the
 // recurrence of the colour that lies behind a record -- and everything else runs record-parallel afterwards:
-//   k_reverse_pixels    thread = pixel: the recurrence, the three colour adjoints of every record, and
-//                       g_sigma * decay parked in the fourth adjoint;
-//   k_reverse_geometry  thread = record: the opacity adjoint is finished, the position / log-scale / quaternion
-//                       contributions are computed and summed per primitive in a shared-memory table first (records
-//                       that follow one another belong to neighbouring pixels, which mostly see the same
-//                       primitives), so that global memory sees one set of atomics per primitive and chunk of
-//                       records instead of one per record.
-__global__ void k_reverse_pixels(const int64_t* __restrict__ offsets, const float* __restrict__ raw,
+//   k_reverse_check     the argument checks of the caller (offsets, ids) as one status word;
+//   k_reverse_pixels    thread = pixel: the recurrence, the four adjoints of every record and
+//                       k = g_sigma * sigma_raw * decay, the weight of the record's geometry terms;
+//   k_reverse_geometry  thread = record.  decay = exp(-1/2 q^T M q) with q = R^T d, M = diag(exp(-2 ls)): the position,
+//                       log-scale and quaternion gradients of a primitive are linear in the nine sums of k q and
+//                       k q q^T over its records, so only those are accumulated -- in a shared-memory table first
+//                       (records that follow one another belong to neighbouring pixels, which mostly see the same
+//                       primitives), so that global memory sees one set of vector reductions per primitive and chunk;
+//   k_reverse_finish    thread = primitive: the gradients from the nine sums.
+constexpr int kRevAcc = 12;          // floats per primitive: k q (3), k q q^T (6), padding to three 16-byte reductions
+
+__global__ void __launch_bounds__(256) k_reverse_check(const int32_t* __restrict__ ids, int64_t total, int n,
+                                                       const int64_t* __restrict__ offsets, int64_t pixels,
+                                                       int32_t* __restrict__ bad, volatile int32_t* bad_host) {
+  chain_wait();
+  chain_release();
+  int b = 0;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x, t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (int64_t i = t; i < total; i += stride) b |= (uint32_t)__ldg(ids + i) >= (uint32_t)n ? MLPSP_REVERSE_BAD_IDS : 0;
+  for (int64_t i = t; i < pixels; i += stride) b |= __ldg(offsets + i + 1) < __ldg(offsets + i) ? MLPSP_REVERSE_BAD_OFFSETS : 0;
+  if (t == 0 && (offsets[0] != 0 || offsets[pixels] != total)) b |= MLPSP_REVERSE_BAD_OFFSETS;
+  if (b) { atomicOr(bad, b); if (bad_host) atomicOr_system(const_cast<int32_t*>(bad_host), b); }
+}
+
+// Four records at a time: their loads do not depend on the recurrence, so they are in flight together.
+__global__ void __launch_bounds__(128) k_reverse_pixels(const int64_t* __restrict__ offsets, const float* __restrict__ raw,
                                  const float* __restrict__ grgb, const float* __restrict__ gt, int64_t pixels,
-                                 float* __restrict__ d4) {
+                                 float* __restrict__ d4, float* __restrict__ kw, const int32_t* __restrict__ bad) {
+  chain_wait();
+  chain_release();
   const int64_t pix = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (pix >= pixels) return;
+  if (pix >= pixels || *bad) return;
   const float gr = grgb[pix * 3], gg = grgb[pix * 3 + 1], gb = grgb[pix * 3 + 2];
   float behind = gt[pix];   // adjoint of the transmittance that reaches whatever lies behind the current record
-  for (int64_t r = offsets[pix + 1] - 1; r >= offsets[pix]; --r) {
-    const float4 a = *reinterpret_cast<const float4*>(raw + r * 8);        // R, G, B, sigma_raw
-    const float4 c = *reinterpret_cast<const float4*>(raw + r * 8 + 4);    // trans before, alpha, decay, sigma logit
-    const float colour = gr * a.x + gg * a.y + gb * a.z;
-    const float g_alpha = c.x * (colour - behind);
-    behind = behind * (1.f - c.y) + colour * c.y;
-    const float g_sigma = g_alpha * __expf(-a.w * c.z);   // d alpha / d (sigma_raw * decay) = 1 - alpha
-    const float w = c.x * c.y;
-    *reinterpret_cast<float4*>(d4 + r * 4) = make_float4(gr * w * a.x * (1.f - a.x), gg * w * a.y * (1.f - a.y),
-                                                         gb * w * a.z * (1.f - a.z), g_sigma * c.z);
+  const int64_t first = offsets[pix];
+  const float4* raw4 = reinterpret_cast<const float4*>(raw);
+  for (int64_t r = offsets[pix + 1] - 1; r >= first; r -= 4) {
+    float4 a4[4], c4[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int64_t q = r - u >= first ? r - u : first;
+      a4[u] = __ldg(raw4 + 2 * q);         // R, G, B, sigma_raw
+      c4[u] = __ldg(raw4 + 2 * q + 1);     // trans before, alpha, decay, sigma logit
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (r - u < first) break;
+      const float4 a = a4[u], c = c4[u];
+      const float colour = gr * a.x + gg * a.y + gb * a.z;
+      const float g_alpha = c.x * (colour - behind);
+      behind = behind * (1.f - c.y) + colour * c.y;
+      const float g_sigma = g_alpha * __expf(-a.w * c.z);   // d alpha / d (sigma_raw * decay) = 1 - alpha
+      const float w = c.x * c.y, parked = g_sigma * c.z;
+      *reinterpret_cast<float4*>(d4 + (r - u) * 4) =
+          make_float4(gr * w * a.x * (1.f - a.x), gg * w * a.y * (1.f - a.y), gb * w * a.z * (1.f - a.z),
+                      parked * sigmoid_fast(c.w));          // softplus' = sigmoid
+      kw[r - u] = parked * a.w;                             // g_decay * decay
+    }
   }
 }
 
@@ -102,41 +136,34 @@ constexpr int kRevChunk = 4096;      // records per CTA
 constexpr int kRevTable = 1024;      // shared-memory accumulator rows (a power of two)
 constexpr int kRevProbe = 16;        // probes before a record goes to global memory directly
 
+__device__ __forceinline__ void red_add4(float* dst, float a, float b, float c, float d) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+
 __global__ void __launch_bounds__(kRevThreads) k_reverse_geometry(
-    const int32_t* __restrict__ ids, const float* __restrict__ x6, const float* __restrict__ raw,
-    const float* __restrict__ logs, const float* __restrict__ quats, int64_t total, float* __restrict__ d4,
-    float* __restrict__ gp, float* __restrict__ gs, float* __restrict__ gq) {
+    const int32_t* __restrict__ ids, const float* __restrict__ x6, const float* __restrict__ kw,
+    const float* __restrict__ quats, int64_t total, float* __restrict__ acc, const int32_t* __restrict__ bad) {
+  chain_wait();
+  chain_release();
   __shared__ int s_key[kRevTable];
-  __shared__ float s_acc[kRevTable][10];
+  __shared__ float s_acc[9][kRevTable];
+  if (*bad) return;
   for (int i = threadIdx.x; i < kRevTable; i += kRevThreads) {
     s_key[i] = -1;
 #pragma unroll
-    for (int j = 0; j < 10; ++j) s_acc[i][j] = 0.f;
+    for (int j = 0; j < 9; ++j) s_acc[j][i] = 0.f;
   }
   __syncthreads();
   const int64_t r0 = (int64_t)blockIdx.x * kRevChunk;
   const int64_t r1 = r0 + kRevChunk < total ? r0 + kRevChunk : total;
   for (int64_t r = r0 + threadIdx.x; r < r1; r += kRevThreads) {
     const int p = ids[r];
-    const float4 a = *reinterpret_cast<const float4*>(raw + r * 8);        // .w = sigma_raw
-    const float4 c = *reinterpret_cast<const float4*>(raw + r * 8 + 4);    // .z = decay, .w = sigma logit
-    const float parked = d4[r * 4 + 3];                                    // g_sigma * decay
-    d4[r * 4 + 3] = parked * sigmoid_fast(c.w);                            // softplus' = sigmoid
-    // decay = exp(-1/2 q^T M q), q = R^T d, d = c - foot point (x6[3..5]), M = diag(exp(-2 ls))
-    const float k = parked * a.w;                                          // g_decay * decay = g_sigma * sigma_raw * decay
-    const V3 d = {x6[r * 6 + 3], x6[r * 6 + 4], x6[r * 6 + 5]};
-    const float4 qt = *reinterpret_cast<const float4*>(quats + (size_t)p * 4);
+    const float k = kw[r];
+    const V3 d = {x6[r * 6 + 3], x6[r * 6 + 4], x6[r * 6 + 5]};            // centre - foot point
+    const float4 qt = __ldg(reinterpret_cast<const float4*>(quats) + p);
     const V3 q = rot_conj_fast(qt.x, qt.y, qt.z, qt.w, d);
-    const float mx = __expf(-2.f * logs[p * 3]), my = __expf(-2.f * logs[p * 3 + 1]), mz = __expf(-2.f * logs[p * 3 + 2]);
-    const V3 gl = {-k * mx * q.x, -k * my * q.y, -k * mz * q.z};           // adjoint of q
-    const V3 gd = rot_quat(qt.x, qt.y, qt.z, qt.w, gl);                    // adjoint of d, hence of the centre
-    // q = R^T d  =>  adjoint of R is d gl^T
-    const float Gm[9] = {d.x * gl.x, d.x * gl.y, d.x * gl.z, d.y * gl.x, d.y * gl.y, d.y * gl.z,
-                         d.z * gl.x, d.z * gl.y, d.z * gl.z};
-    float gquat[4];
-    quat_adjoint(qt.x, qt.y, qt.z, qt.w, Gm, gquat);
-    const float v[10] = {gd.x, gd.y, gd.z, k * mx * q.x * q.x, k * my * q.y * q.y, k * mz * q.z * q.z,
-                         gquat[0], gquat[1], gquat[2], gquat[3]};
+    const float kx = k * q.x, ky = k * q.y, kz = k * q.z;
+    const float v[9] = {kx, ky, kz, kx * q.x, ky * q.y, kz * q.z, kx * q.y, kx * q.z, ky * q.z};
     // the primitive's row of the table: linear probing from a multiplicative hash
     int slot = (int)(((uint32_t)p * 2654435761u) >> 22) & (kRevTable - 1);
     bool placed = false;
@@ -147,172 +174,486 @@ __global__ void __launch_bounds__(kRevThreads) k_reverse_geometry(
     }
     if (placed) {
 #pragma unroll
-      for (int j = 0; j < 10; ++j) atomicAdd(&s_acc[slot][j], v[j]);
+      for (int j = 0; j < 9; ++j) atomicAdd(&s_acc[j][slot], v[j]);
     } else {
-      atomicAdd(gp + p * 3, v[0]); atomicAdd(gp + p * 3 + 1, v[1]); atomicAdd(gp + p * 3 + 2, v[2]);
-      atomicAdd(gs + p * 3, v[3]); atomicAdd(gs + p * 3 + 1, v[4]); atomicAdd(gs + p * 3 + 2, v[5]);
-      atomicAdd(gq + p * 4, v[6]); atomicAdd(gq + p * 4 + 1, v[7]); atomicAdd(gq + p * 4 + 2, v[8]); atomicAdd(gq + p * 4 + 3, v[9]);
+      float* dst = acc + (size_t)p * kRevAcc;
+      red_add4(dst, v[0], v[1], v[2], v[3]);
+      red_add4(dst + 4, v[4], v[5], v[6], v[7]);
+      red_add4(dst + 8, v[8], 0.f, 0.f, 0.f);
     }
   }
   __syncthreads();
   for (int i = threadIdx.x; i < kRevTable; i += kRevThreads) {
     const int p = s_key[i];
     if (p < 0) continue;
-    atomicAdd(gp + p * 3, s_acc[i][0]); atomicAdd(gp + p * 3 + 1, s_acc[i][1]); atomicAdd(gp + p * 3 + 2, s_acc[i][2]);
-    atomicAdd(gs + p * 3, s_acc[i][3]); atomicAdd(gs + p * 3 + 1, s_acc[i][4]); atomicAdd(gs + p * 3 + 2, s_acc[i][5]);
-    atomicAdd(gq + p * 4, s_acc[i][6]); atomicAdd(gq + p * 4 + 1, s_acc[i][7]);
-    atomicAdd(gq + p * 4 + 2, s_acc[i][8]); atomicAdd(gq + p * 4 + 3, s_acc[i][9]);
+    float* dst = acc + (size_t)p * kRevAcc;
+    red_add4(dst, s_acc[0][i], s_acc[1][i], s_acc[2][i], s_acc[3][i]);
+    red_add4(dst + 4, s_acc[4][i], s_acc[5][i], s_acc[6][i], s_acc[7][i]);
+    red_add4(dst + 8, s_acc[8][i], 0.f, 0.f, 0.f);
   }
+}
+
+__global__ void __launch_bounds__(128) k_reverse_finish(const float* __restrict__ acc, const float* __restrict__ logs,
+                                                        const float* __restrict__ quats, int n, float* __restrict__ gp,
+                                                        float* __restrict__ gs, float* __restrict__ gq) {
+  chain_wait();
+  chain_release();
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= n) return;
+  const float4 a = *reinterpret_cast<const float4*>(acc + (size_t)p * kRevAcc);
+  const float4 b = *reinterpret_cast<const float4*>(acc + (size_t)p * kRevAcc + 4);
+  const float syz = acc[(size_t)p * kRevAcc + 8];
+  const float S[9] = {a.w, b.z, b.w, b.z, b.x, syz, b.w, syz, b.y};        // sum of k q q^T
+  const float4 qt = __ldg(reinterpret_cast<const float4*>(quats) + p);
+  const float m[3] = {__expf(-2.f * logs[(size_t)p * 3]), __expf(-2.f * logs[(size_t)p * 3 + 1]), __expf(-2.f * logs[(size_t)p * 3 + 2])};
+  // adjoint of q is -k M q; of d (hence of the centre) R times that; of R, with q = R^T d, d (-k M q)^T
+  const V3 gd = rot_quat(qt.x, qt.y, qt.z, qt.w, V3{-m[0] * a.x, -m[1] * a.y, -m[2] * a.z});
+  gp[(size_t)p * 3] = gd.x; gp[(size_t)p * 3 + 1] = gd.y; gp[(size_t)p * 3 + 2] = gd.z;
+  gs[(size_t)p * 3] = m[0] * S[0]; gs[(size_t)p * 3 + 1] = m[1] * S[4]; gs[(size_t)p * 3 + 2] = m[2] * S[8];
+  float Gm[9];
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {      // column j of sum d gl^T = R (-m_j S_.j)
+    const V3 c = rot_quat(qt.x, qt.y, qt.z, qt.w, V3{-m[j] * S[j], -m[j] * S[3 + j], -m[j] * S[6 + j]});
+    Gm[j] = c.x; Gm[3 + j] = c.y; Gm[6 + j] = c.z;
+  }
+  float gquat[4];
+  quat_adjoint(qt.x, qt.y, qt.z, qt.w, Gm, gquat);
+  *reinterpret_cast<float4*>(gq + (size_t)p * 4) = make_float4(gquat[0], gquat[1], gquat[2], gquat[3]);
 }
 
 // --------------------------------------------------------- grouped weight gradients ----
-constexpr int kGH = 32, kGIN = 72, kGSeg = 128;
-constexpr int kOW1 = 0, kOb1 = kOW1 + kGH * kGIN, kOW2 = kOb1 + kGH, kOb2 = kOW2 + kGH * kGH, kOW3 = kOb2 + kGH,
-              kOb3 = kOW3 + 4 * kGH, kGradLen = kOb3 + 4;   // 3,524 = the reference's packed gradient row
-static_assert(kGradLen == 3524, "gradient row layout");
-
-// shared memory: weights of the primitive, then per record E[72], H1[32], H2[32], D1[32], D2[32], D3[4]
-constexpr int kRowF = kGIN + 4 * kGH + 4;                       // 204 floats per record
-constexpr int kGradSmem = (kGH * kGIN + kGH * kGH + 4 * kGH + 2 * kGH) * 4 + kGSeg * kRowF * 4;
-
-constexpr int kOutPerThread = (kGradLen + kGSeg - 1) / kGSeg;   // 28
-
-__global__ void __launch_bounds__(kGSeg) k_grouped_vjp(
-    const float* __restrict__ x6, const float* __restrict__ d4, const int32_t* __restrict__ masks,
-    const int64_t* __restrict__ offsets, const int64_t* __restrict__ seg_prim, const int64_t* __restrict__ seg_start,
-    int segment_size, const float* __restrict__ freq, const float* __restrict__ att, const float* __restrict__ W1,
-    const float* __restrict__ b1, const float* __restrict__ W2, const float* __restrict__ b2,
-    const float* __restrict__ W3, float scale, float* __restrict__ partial) {
-  extern __shared__ float sm[];
-  float* sW1 = sm;
-  float* sW2 = sW1 + kGH * kGIN;
-  float* sW3 = sW2 + kGH * kGH;
-  float* sb1 = sW3 + 4 * kGH;
-  float* sb2 = sb1 + kGH;
-  float* rows = sb2 + kGH;
-  const int seg = blockIdx.x, tid = threadIdx.x;
-  const int p = (int)seg_prim[seg];
-  const int64_t begin = seg_start[seg];
-  const int total = (int)min((int64_t)segment_size, offsets[p + 1] - begin);
-  for (int i = tid; i < kGH * kGIN; i += kGSeg) sW1[i] = W1[(size_t)p * kGH * kGIN + i];
-  for (int i = tid; i < kGH * kGH; i += kGSeg) sW2[i] = W2[(size_t)p * kGH * kGH + i];
-  for (int i = tid; i < 4 * kGH; i += kGSeg) sW3[i] = W3[(size_t)p * 4 * kGH + i];
-  if (tid < kGH) { sb1[tid] = b1[(size_t)p * kGH + tid]; sb2[tid] = b2[(size_t)p * kGH + tid]; }
-  float acc[kOutPerThread];
-#pragma unroll
-  for (int k = 0; k < kOutPerThread; ++k) acc[k] = 0.f;
-  float* me = rows + (size_t)tid * kRowF;
-  float* E = me, *H1 = me + kGIN, *H2 = H1 + kGH, *D1 = H2 + kGH, *D2 = D1 + kGH, *D3 = D2 + kGH;
-  for (int sub = 0; sub < total; sub += kGSeg) {
-    const int cnt = min(kGSeg, total - sub);
-    __syncthreads();   // weights loaded / the previous block's rows consumed
-    if (tid < cnt) {
-      const int64_t r = begin + sub + tid;
-      // encoding as scannet/cumodel.py:183-195: index c*F + f holds sin, + 36 holds cos
-      for (int c = 0; c < 6; ++c) {
-        const float v = x6[r * 6 + c];
-        for (int f = 0; f < 6; ++f) {
-          const float ph = v * freq[f] * att[f];
-          E[c * 6 + f] = sinf(ph);
-          E[36 + c * 6 + f] = cosf(ph);
-        }
-      }
-      uint32_t m1 = 0, m2 = 0;
-      if (masks) { m1 = (uint32_t)masks[r * 2]; m2 = (uint32_t)masks[r * 2 + 1]; }
-      for (int h = 0; h < kGH; ++h) {
-        float a = sb1[h];
-        for (int j = 0; j < kGIN; ++j) a = fmaf(sW1[h * kGIN + j], E[j], a);
-        if (!masks && a > 0.f) m1 |= 1u << h;
-        H1[h] = a > 0.f ? a : 0.f;
-      }
-      for (int q = 0; q < kGH; ++q) {
-        float a = sb2[q];
-        for (int h = 0; h < kGH; ++h) a = fmaf(sW2[q * kGH + h], H1[h], a);
-        if (!masks && a > 0.f) m2 |= 1u << q;
-        H2[q] = a > 0.f ? a : 0.f;
-      }
-      for (int c = 0; c < 4; ++c) D3[c] = d4[r * 4 + c] * scale;
-      for (int h = 0; h < kGH; ++h) {
-        float a = 0.f;
-        for (int c = 0; c < 4; ++c) a = fmaf(D3[c], sW3[c * kGH + h], a);
-        D2[h] = ((m2 >> h) & 1u) ? a : 0.f;
-      }
-      for (int h = 0; h < kGH; ++h) {
-        float a = 0.f;
-        for (int q = 0; q < kGH; ++q) a = fmaf(D2[q], sW2[q * kGH + h], a);
-        D1[h] = ((m1 >> h) & 1u) ? a : 0.f;
-      }
-    }
-    __syncthreads();
-    // thread = output element: sums over the block's records in record order
-#pragma unroll
-    for (int k = 0; k < kOutPerThread; ++k) {
-      const int o = tid + k * kGSeg;
-      if (o >= kGradLen) break;
-      int a_off, b_off;   // offsets of the two factors inside a record's row; b_off < 0: plain sum of the first
-      if (o < kOb1) { a_off = kGIN + 2 * kGH + (o / kGIN); b_off = o % kGIN; }                                   // D1[h] * E[j]
-      else if (o < kOW2) { a_off = kGIN + 2 * kGH + (o - kOb1); b_off = -1; }                                    // sum D1[h]
-      else if (o < kOb2) { const int e = o - kOW2; a_off = kGIN + 3 * kGH + e / kGH; b_off = kGIN + e % kGH; }   // D2[q] * H1[h]
-      else if (o < kOW3) { a_off = kGIN + 3 * kGH + (o - kOb2); b_off = -1; }                                    // sum D2[q]
-      else if (o < kOb3) { const int e = o - kOW3; a_off = kGIN + 4 * kGH + e / kGH; b_off = kGIN + kGH + e % kGH; }  // D3[c] * H2[h]
-      else { a_off = kGIN + 4 * kGH + (o - kOb3); b_off = -1; }                                                  // sum D3[c]
-      float a = acc[k];
-      if (b_off >= 0) for (int r = 0; r < cnt; ++r) a = fmaf(rows[(size_t)r * kRowF + a_off], rows[(size_t)r * kRowF + b_off], a);
-      else for (int r = 0; r < cnt; ++r) a += rows[(size_t)r * kRowF + a_off];
-      acc[k] = a;
-    }
+// Segments of the launch, planned on the device (no count travels to the host): the order of the items does not matter,
+// a primitive of several segments owns consecutive partial rows and an entry of the multi list, a primitive without
+// records an entry with no rows (its gradients are zero).
+__global__ void __launch_bounds__(256) k_vjp_plan(const int64_t* __restrict__ offsets, int n, int segment_size,
+                                                  VjpItem* __restrict__ items, VjpItem* __restrict__ multi,
+                                                  int32_t* __restrict__ counters) {
+  chain_wait();
+  chain_release();
+  __shared__ int warp_sums[32];
+  __shared__ int base[3];
+  const int p = blockIdx.x * 256 + threadIdx.x;
+  int64_t start = 0, count = 0;
+  if (p < n) { start = offsets[p]; count = offsets[p + 1] - start; }
+  const int segs = count > 0 ? (int)((count + segment_size - 1) / segment_size) : 0;
+  const int rows = segs > 1 ? segs : 0, listed = p < n && segs != 1;
+  int ts, tr, tm;
+  const int es = block_exclusive_scan(segs, warp_sums, ts);
+  const int er = block_exclusive_scan(rows, warp_sums, tr);
+  const int em = block_exclusive_scan(listed, warp_sums, tm);
+  if (threadIdx.x == 0) {
+    base[0] = ts ? atomicAdd(counters + kVpItems, ts) : 0;
+    base[1] = tr ? atomicAdd(counters + kVpRows, tr) : 0;
+    base[2] = tm ? atomicAdd(counters + kVpMulti, tm) : 0;
   }
-  float* out = partial + (size_t)seg * kGradLen;
-  const float inv = 1.f / scale;
-#pragma unroll
-  for (int k = 0; k < kOutPerThread; ++k) {
-    const int o = tid + k * kGSeg;
-    if (o < kGradLen) out[o] = acc[k] * inv;
+  __syncthreads();
+  for (int g = 0; g < segs; ++g) {
+    VjpItem it = {};
+    it.start = start + (int64_t)g * segment_size;
+    it.rows = (int)min((int64_t)segment_size, count - (int64_t)g * segment_size);
+    it.prim = p;
+    it.dest = segs > 1 ? base[1] + er + g : -1;
+    items[base[0] + es + g] = it;
+  }
+  if (listed) {
+    VjpItem it = {};
+    it.start = base[1] + er;
+    it.rows = rows;
+    it.prim = p;
+    multi[base[2] + em] = it;
   }
 }
 
-// result[p] = sum of the partial rows of p's segments, in segment order; nonfinite |= any non-finite sum
-__global__ void k_reduce_partials(const float* __restrict__ partial, const int64_t* __restrict__ seg_offsets, int n,
-                                  float* __restrict__ result, int32_t* __restrict__ nonfinite) {
-  const int p = blockIdx.x;
-  const int o = blockIdx.y * blockDim.x + threadIdx.x;
-  if (p >= n || o >= kGradLen) return;
-  float acc = 0.f;
-  for (int64_t g = seg_offsets[p]; g < seg_offsets[p + 1]; ++g) acc += partial[(size_t)g * kGradLen + o];
-  result[(size_t)p * kGradLen + o] = acc;
-  if (!(fabsf(acc) <= 3.4028235e38f)) atomicOr(nonfinite, 1);
+// IEEE FP32 on the CUDA cores, sums in record order.  A CTA of 128 threads takes 64 records at a time; everything per
+// record lies transposed in shared memory ([quantity][record], rows of 68 floats: 16-byte reads of eight different rows
+// meet eight different bank groups), so that the record-major products (layers, adjoints) give a thread a tile of four
+// records x four units and the contractions over the records (the gradients) 2 x 9 + 2 x 4 + 1 sums in registers, both
+// fed by 16-byte reads: 16 multiply-adds per two reads and 104 per nineteen.  Bound: FP32 issue (about 8,000 multiply-adds
+// per record).  A thread-per-record version with one 4-byte read per multiply-add took 616 us where this one takes
+// 150 us (117,000 records of 2,000 primitives).
+constexpr int kGfRec = 64, kGfThreads = 128, kGfRow = kGfRec + 4, kGfCtas = 3;
+constexpr int kGfE = 0, kGfH1 = kGfE + kGIN * kGfRow, kGfH2 = kGfH1 + kGH * kGfRow, kGfD1 = kGfH2 + kGH * kGfRow,
+              kGfD2 = kGfD1 + kGH * kGfRow, kGfD3 = kGfD2 + kGH * kGfRow, kGfMask = kGfD3 + 4 * kGfRow,
+              kGfW1T = kGfMask + 2 * kGfRec, kGfW2T = kGfW1T + kGIN * kGH, kGfW2 = kGfW2T + kGH * kGH, kGfW2Row = kGH + 4,
+              kGfW3 = kGfW2 + kGH * kGfW2Row, kGfB = kGfW3 + 4 * kGH, kGfFloats = kGfB + 2 * kGH;
+constexpr int kGradSmem = kGfFloats * 4;
+static_assert(kGfCtas * (kGradSmem + 1024) <= 228 * 1024, "resident CTAs");
+
+__device__ __forceinline__ void fma4(float4& a, float s, const float4 v) {
+  a.x = fmaf(s, v.x, a.x); a.y = fmaf(s, v.y, a.y); a.z = fmaf(s, v.z, a.z); a.w = fmaf(s, v.w, a.w);
+}
+// acc + the products of four consecutive records, in record order
+__device__ __forceinline__ float dot4(float acc, const float4 a, const float4 b) {
+  return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, acc))));
+}
+
+__global__ void __launch_bounds__(kGfThreads, kGfCtas) k_grouped_vjp(
+    const float* __restrict__ x6, const float* __restrict__ d4, const int32_t* __restrict__ masks,
+    const VjpItem* __restrict__ items, int32_t* __restrict__ counters, const float* __restrict__ freq,
+    const float* __restrict__ att, const float* __restrict__ W1, const float* __restrict__ b1, const float* __restrict__ W2,
+    const float* __restrict__ b2, const float* __restrict__ W3, float scale, VjpOut out, float* __restrict__ partial) {
+  chain_wait();
+  chain_release();
+  extern __shared__ __align__(16) float sm[];
+  const int G = counters[kVpItems];
+  const int tid = threadIdx.x;
+  const int hg = tid & 7, rg = tid >> 3;         // units 4 hg .. + 3 of records 4 rg .. + 3; gradient rows 2 rg, 2 rg + 1
+  const float inv = 1.f / scale;
+  bool bad = false;
+  uint32_t* sMask = reinterpret_cast<uint32_t*>(sm + kGfMask);
+  float fr[6], at[6];
+#pragma unroll
+  for (int f = 0; f < 6; ++f) { fr[f] = __ldg(freq + f); at[f] = __ldg(att + f); }
+  for (int idx = blockIdx.x; idx < G; idx += gridDim.x) {
+    const VjpItem it = load_item(items + idx);
+    const size_t p = (size_t)it.prim;
+    __syncthreads();                             // the previous item's last block has been consumed
+#pragma unroll
+    for (int u = 0; u < 18; ++u) {               // W1 transposed: lane = row, so the stores are conflict-free
+      const int k = u * 4 + (tid >> 5), h = tid & 31;
+      sm[kGfW1T + k * kGH + h] = __ldg(W1 + p * (kGH * kGIN) + h * kGIN + k);
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int e = u * kGfThreads + tid, q = e >> 5, h = e & 31;
+      sm[kGfW2 + q * kGfW2Row + h] = __ldg(W2 + p * (kGH * kGH) + e);
+      const int k = u * 4 + (tid >> 5), r = tid & 31;
+      sm[kGfW2T + k * kGH + r] = __ldg(W2 + p * (kGH * kGH) + r * kGH + k);
+    }
+    sm[kGfW3 + tid] = __ldg(W3 + p * (4 * kGH) + tid);
+    if (tid < 2 * kGH) sm[kGfB + tid] = tid < kGH ? __ldg(b1 + p * kGH + tid) : __ldg(b2 + p * kGH + tid - kGH);
+    float g1[2][9], g2[2][4], g3 = 0.f, gb = 0.f;
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+#pragma unroll
+      for (int i = 0; i < 9; ++i) g1[a][i] = 0.f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) g2[a][i] = 0.f;
+    }
+    for (int sub = 0; sub < it.rows; sub += kGfRec) {
+      const int cnt = min(kGfRec, it.rows - sub);
+      if (sub > 0) __syncthreads();              // the previous block's rows have been consumed
+      {
+        // encoding as scannet/cumodel.py:183-195: index c*F + f holds sin, + 36 holds cos; a thread takes three coordinates
+        const int rec = tid & (kGfRec - 1), part = tid >> 6;
+        const bool valid = rec < cnt;
+        const int64_t r = it.start + sub + rec;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const int cc = part * 3 + c;
+          const float v = valid ? __ldg(x6 + r * 6 + cc) : 0.f;
+#pragma unroll
+          for (int f = 0; f < 6; ++f) {
+            float sn, cs;
+            sincosf(v * fr[f] * at[f], &sn, &cs);
+            sm[kGfE + (cc * 6 + f) * kGfRow + rec] = valid ? sn : 0.f;
+            sm[kGfE + (36 + cc * 6 + f) * kGfRow + rec] = valid ? cs : 0.f;
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+          sm[kGfD3 + (part * 2 + c) * kGfRow + rec] = valid ? __ldg(d4 + r * 4 + part * 2 + c) * scale : 0.f;
+        if (masks) sMask[part * kGfRec + rec] = valid ? (uint32_t)__ldg(masks + r * 2 + part) : 0u;
+      }
+      __syncthreads();
+      const int r4 = rg * 4, h4 = hg * 4;
+      uint32_t m1[4], m2[4];
+      if (masks) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { m1[j] = sMask[r4 + j] >> h4; m2[j] = sMask[kGfRec + r4 + j] >> h4; }
+      }
+      // a tile acc[u] = (four records) of unit h4 + u; gate: the records' mask bits of that unit
+      float4 acc[4];
+      auto product = [&](int x_off, int K, int w_off, int w_row) {
+#pragma unroll 8
+        for (int k = 0; k < K; ++k) {
+          const float4 x = *reinterpret_cast<const float4*>(sm + x_off + k * kGfRow + r4);
+          const float4 w = *reinterpret_cast<const float4*>(sm + w_off + k * w_row + h4);
+          fma4(acc[0], w.x, x); fma4(acc[1], w.y, x); fma4(acc[2], w.z, x); fma4(acc[3], w.w, x);
+        }
+      };
+      auto hidden = [&](int dst, uint32_t (&m)[4]) {
+        if (!masks) { m[0] = m[1] = m[2] = m[3] = 0u; }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          float4 a = acc[u];
+          if (!masks) {
+            m[0] |= (a.x > 0.f ? 1u : 0u) << u; m[1] |= (a.y > 0.f ? 1u : 0u) << u;
+            m[2] |= (a.z > 0.f ? 1u : 0u) << u; m[3] |= (a.w > 0.f ? 1u : 0u) << u;
+          }
+          a.x = a.x > 0.f ? a.x : 0.f; a.y = a.y > 0.f ? a.y : 0.f; a.z = a.z > 0.f ? a.z : 0.f; a.w = a.w > 0.f ? a.w : 0.f;
+          *reinterpret_cast<float4*>(sm + dst + (h4 + u) * kGfRow + r4) = a;
+        }
+      };
+      auto adjoint = [&](int dst, const uint32_t (&m)[4]) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          float4 a = acc[u];
+          a.x = ((m[0] >> u) & 1u) ? a.x : 0.f; a.y = ((m[1] >> u) & 1u) ? a.y : 0.f;
+          a.z = ((m[2] >> u) & 1u) ? a.z : 0.f; a.w = ((m[3] >> u) & 1u) ? a.w : 0.f;
+          *reinterpret_cast<float4*>(sm + dst + (h4 + u) * kGfRow + r4) = a;
+        }
+      };
+      auto start = [&](const float* bias) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) { const float b = bias ? bias[h4 + u] : 0.f; acc[u] = make_float4(b, b, b, b); }
+      };
+      start(sm + kGfB);
+      product(kGfE, kGIN, kGfW1T, kGH);
+      hidden(kGfH1, m1);
+      __syncthreads();
+      start(sm + kGfB + kGH);
+      product(kGfH1, kGH, kGfW2T, kGH);
+      hidden(kGfH2, m2);
+      start(nullptr);
+      product(kGfD3, 4, kGfW3, kGH);
+      adjoint(kGfD2, m2);
+      __syncthreads();
+      start(nullptr);
+      product(kGfD2, kGH, kGfW2, kGfW2Row);
+      adjoint(kGfD1, m1);
+      __syncthreads();
+      // ---- sums over the block's records, four at a time (rows past the last record hold zero adjoints) ----
+      const int gr = rg * 2;
+      for (int r = 0; r < cnt; r += 4) {
+        auto at4 = [&](int off, int row) { return *reinterpret_cast<const float4*>(sm + off + row * kGfRow + r); };
+        {
+          const float4 a0 = at4(kGfD1, gr), a1 = at4(kGfD1, gr + 1);
+#pragma unroll
+          for (int i = 0; i < 9; ++i) {
+            const float4 e = at4(kGfE, hg + 8 * i);
+            g1[0][i] = dot4(g1[0][i], a0, e);
+            g1[1][i] = dot4(g1[1][i], a1, e);
+          }
+        }
+        {
+          const float4 a0 = at4(kGfD2, gr), a1 = at4(kGfD2, gr + 1);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float4 e = at4(kGfH1, hg + 8 * i);
+            g2[0][i] = dot4(g2[0][i], a0, e);
+            g2[1][i] = dot4(g2[1][i], a1, e);
+          }
+        }
+        g3 = dot4(g3, at4(kGfD3, tid >> 5), at4(kGfH2, tid & 31));
+        if (tid < 68) {
+          const float4 v = tid < 32 ? at4(kGfD1, tid) : (tid < 64 ? at4(kGfD2, tid - 32) : at4(kGfD3, tid - 64));
+          gb = ((gb + v.x) + v.y) + v.z + v.w;
+        }
+      }
+    }
+    const VjpOut o = vjp_row(out, partial, it);
+    auto put = [&](float* dst, float v) {
+      const float g = v * inv;
+      bad |= !(fabsf(g) <= 3.4028235e38f);
+      *dst = g;
+    };
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+#pragma unroll
+      for (int i = 0; i < 9; ++i) put(o.W1 + (rg * 2 + a) * kGIN + hg + 8 * i, g1[a][i]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) put(o.W2 + (rg * 2 + a) * kGH + hg + 8 * i, g2[a][i]);
+    }
+    put(o.W3 + tid, g3);
+    if (tid < 32) put(o.b1 + tid, gb);
+    else if (tid < 64) put(o.b2 + tid - 32, gb);
+    else if (tid < 68) put(o.b3 + tid - 64, gb);
+  }
+  if (bad) atomicOr(counters + kVpFlag, 1);
+}
+
+// The gradients of the primitives on the multi list: their partial rows in segment order (no rows: zero).
+__global__ void __launch_bounds__(256) k_vjp_reduce(const VjpItem* __restrict__ multi, const float* __restrict__ partial,
+                                                    VjpOut out, int32_t* __restrict__ counters) {
+  chain_wait();
+  chain_release();
+  const int M = counters[kVpMulti];
+  bool bad = false;
+  for (int e = blockIdx.x; e < M; e += gridDim.x) {
+    VjpItem it = load_item(multi + e);
+    it.dest = -1;
+    const VjpOut o = vjp_row(out, nullptr, it);
+    for (int i = threadIdx.x; i < kGradLen; i += 256) {
+      float acc = 0.f;
+      for (int g = 0; g < it.rows; ++g) acc += partial[(size_t)(it.start + g) * kGradLen + i];
+      float* dst = i < kOb1 ? o.W1 + i : i < kOW2 ? o.b1 + i - kOb1 : i < kOb2 ? o.W2 + i - kOW2 : i < kOW3 ? o.b2 + i - kOb2
+                   : i < kOb3 ? o.W3 + i - kOW3 : o.b3 + i - kOb3;
+      *dst = acc;
+      bad |= !(fabsf(acc) <= 3.4028235e38f);
+    }
+  }
+  if (bad) atomicOr(counters + kVpFlag, 1);
+}
+
+int launch_grouped_vjp_tc(bool bf16, const float* x6, const float* d4, const int32_t* masks, const VjpItem* items,
+                          int64_t max_items, int32_t* counters, const mlpsp_scene* sc, float scale, const VjpOut& out,
+                          float* partial, cudaStream_t st);
+
+// scratch of a launch: counters | items | multi list | partial rows
+struct VjpScratch { int64_t items, multi, partial, bytes, max_items, max_rows; };
+static VjpScratch vjp_scratch(int64_t R, int n, int segment_size) {
+  VjpScratch s;
+  s.max_items = R / segment_size + std::min<int64_t>(n, R);
+  s.max_rows = std::min<int64_t>(2 * (R / segment_size), s.max_items);     // a primitive of c > 1 segments owns more than c / 2 of them in full
+  int64_t off = 256;
+  auto take = [&](int64_t bytes) { const int64_t o = off; off += align_up(bytes, 256); return o; };
+  s.items = take((int64_t)sizeof(VjpItem) * s.max_items);
+  s.multi = take((int64_t)sizeof(VjpItem) * n);
+  s.partial = take(4ll * kGradLen * s.max_rows);
+  s.bytes = off + 256;
+  return s;
+}
+
+static int weight_gradients(const mlpsp_scene* sc, const int64_t* offsets, const float* x6, const float* d4, const int32_t* masks,
+                            int64_t R, int segment_size, int precision, float loss_scale, const VjpOut& out, void* scratch,
+                            int64_t scratch_bytes, int32_t* flag_host, int32_t* flag_dev, cudaStream_t st) {
+  const VjpScratch L = vjp_scratch(R, sc->n, segment_size);
+  MLPSP_REQUIRE(scratch && scratch_bytes >= L.bytes, MLPSP_E_SCRATCH, "mlpsp_weight_gradients: scratch needs %lld bytes", (long long)L.bytes);
+  char* base = reinterpret_cast<char*>(align_up((int64_t)reinterpret_cast<uintptr_t>(scratch), 256));
+  int32_t* counters = reinterpret_cast<int32_t*>(base);
+  VjpItem* items = reinterpret_cast<VjpItem*>(base + L.items);
+  VjpItem* multi = reinterpret_cast<VjpItem*>(base + L.multi);
+  float* partial = reinterpret_cast<float*>(base + L.partial);
+  LaunchScope scope(kKMisc, R > 0 ? 3 : 2, st);
+  MLPSP_CUDA_OK(cudaMemsetAsync(counters, 0, 4 * kVpCounters, st));
+  launch_chained(k_vjp_plan, dim3((sc->n + 255) / 256), dim3(256), 0, st, offsets, sc->n, segment_size, items, multi, counters);
+  if (R > 0 && precision != MLPSP_PRECISION_F32) {
+    const int rc = launch_grouped_vjp_tc(precision == MLPSP_PRECISION_BF16, x6, d4, masks, items, L.max_items, counters, sc, loss_scale,
+                                         out, partial, st);
+    if (rc) return rc;
+  } else if (R > 0) {
+    static DeviceOnce attr_once;
+    if (attr_once.first())
+      MLPSP_CUDA_OK(cudaFuncSetAttribute(k_grouped_vjp, cudaFuncAttributeMaxDynamicSharedMemorySize, kGradSmem));
+    launch_chained(k_grouped_vjp, dim3((unsigned)std::min<int64_t>(L.max_items, (int64_t)sm_count() * kGfCtas)), dim3(kGfThreads), kGradSmem, st,
+                   x6, d4, masks, items, counters, sc->freq, sc->att, sc->W1, sc->b1, sc->W2, sc->b2, sc->W3, loss_scale, out, partial);
+  }
+  launch_chained(k_vjp_reduce, dim3((unsigned)std::min(sc->n, sm_count() * 8)), dim3(256), 0, st, multi, partial, out, counters);
+  if (flag_dev) MLPSP_CUDA_OK(cudaMemcpyAsync(flag_dev, counters + kVpFlag, 4, cudaMemcpyDeviceToDevice, st));
+  if (flag_host) {
+    HostWords& hw = host_words();
+    cudaEvent_t ev = nullptr;
+    const int rc = hw.open(&ev);
+    if (rc) return rc;
+    MLPSP_CUDA_OK(cudaMemcpyAsync(hw.word, counters + kVpFlag, 4, cudaMemcpyDeviceToHost, st));
+    MLPSP_CUDA_OK(cudaEventRecord(ev, st));
+    MLPSP_CUDA_OK(cudaEventSynchronize(ev));
+    *flag_host = *static_cast<volatile int32_t*>(hw.word);
+  }
+  return cuda_check(cudaGetLastError(), "weight_gradients");
 }
 
 }  // namespace mlpsp
 
 using namespace mlpsp;
 
+// scratch: findings of the argument checks | the nine sums of every primitive | one weight per record
+extern "C" int64_t mlpsp_records_reverse_scratch_bytes(int64_t total_records, int32_t n) {
+  if (total_records < 0 || n < 0) return -1;
+  return 256 + align_up(4ll * kRevAcc * n, 256) + align_up(4 * total_records, 256) + 256;
+}
+
+extern "C" int mlpsp_records_reverse_checked(const int32_t* ids, const int64_t* offsets, const float* x6, const float* raw,
+                                             const float* log_scales, const float* quats, const float* grad_rgb,
+                                             const float* grad_t, int64_t pixels, int64_t total_records, int32_t n, float* d4,
+                                             float* grad_pos, float* grad_log_scales, float* grad_quats, void* scratch,
+                                             int64_t scratch_bytes, int32_t* findings_host, void* stream) {
+  MLPSP_REQUIRE(pixels >= 0 && n >= 0 && total_records >= 0, MLPSP_E_ARG, "mlpsp_records_reverse: negative size");
+  MLPSP_REQUIRE(offsets && (n == 0 || (log_scales && quats && grad_pos && grad_log_scales && grad_quats)) &&
+                    (pixels == 0 || (grad_rgb && grad_t)) && (total_records == 0 || (ids && x6 && raw && d4 && quats)),
+                MLPSP_E_ARG, "mlpsp_records_reverse: null pointer");
+  MLPSP_REQUIRE(((reinterpret_cast<uintptr_t>(raw) | reinterpret_cast<uintptr_t>(d4) | reinterpret_cast<uintptr_t>(quats) |
+                  reinterpret_cast<uintptr_t>(grad_quats)) & 15) == 0,
+                MLPSP_E_ARG, "mlpsp_records_reverse: raw, d4, quats and grad_quats must be 16-byte aligned");
+  MLPSP_REQUIRE(scratch && scratch_bytes >= mlpsp_records_reverse_scratch_bytes(total_records, n), MLPSP_E_SCRATCH,
+                "mlpsp_records_reverse: scratch too small");
+  cudaStream_t st = (cudaStream_t)stream;
+  char* base = reinterpret_cast<char*>(align_up((int64_t)reinterpret_cast<uintptr_t>(scratch), 256));
+  int32_t* bad = reinterpret_cast<int32_t*>(base);          // cleared together with the sums behind it
+  float* acc = reinterpret_cast<float*>(base + 256);
+  float* kw = reinterpret_cast<float*>(base + 256 + align_up(4ll * kRevAcc * n, 256));
+  HostWords& hw = host_words();
+  cudaEvent_t ev = nullptr;
+  if (findings_host) {
+    const int rc = hw.open(&ev);
+    if (rc) return rc;
+    hw.word[0] = 0;
+  }
+  LaunchScope scope(kKMisc, 4, st);
+  MLPSP_CUDA_OK(cudaMemsetAsync(base, 0, 256 + 4ll * kRevAcc * n, st));
+  const int64_t most = std::max(total_records, pixels);
+  launch_chained(k_reverse_check, dim3((unsigned)std::min<int64_t>(148 * 8, most / 1024 + 1)), dim3(256), 0, st, ids, total_records, n, offsets,
+                 pixels, bad, findings_host ? hw.word : nullptr);
+  if (findings_host) MLPSP_CUDA_OK(cudaEventRecord(ev, st));
+  if (pixels > 0 && total_records > 0) {
+    launch_chained(k_reverse_pixels, dim3((unsigned)((pixels + 127) / 128)), dim3(128), 0, st, offsets, raw, grad_rgb, grad_t, pixels, d4, kw, bad);
+    launch_chained(k_reverse_geometry, dim3((unsigned)((total_records + kRevChunk - 1) / kRevChunk)), dim3(kRevThreads), 0, st, ids, x6, kw, quats,
+                   total_records, acc, bad);
+  }
+  if (n > 0) launch_chained(k_reverse_finish, dim3((n + 127) / 128), dim3(128), 0, st, acc, log_scales, quats, n, grad_pos, grad_log_scales, grad_quats);
+  MLPSP_CUDA_OK(cudaGetLastError());
+  if (findings_host) {
+    MLPSP_CUDA_OK(cudaEventSynchronize(ev));
+    *findings_host = *static_cast<volatile int32_t*>(hw.word);
+  }
+  return MLPSP_OK;
+}
+
 extern "C" int mlpsp_records_reverse(const int32_t* ids, const int64_t* offsets, const float* x6, const float* raw,
                                      const float* log_scales, const float* quats, const float* grad_rgb,
                                      const float* grad_t, int64_t pixels, int64_t total_records, int32_t n, float* d4,
                                      float* grad_pos, float* grad_log_scales, float* grad_quats, void* stream) {
-  MLPSP_REQUIRE(pixels >= 0 && n >= 0, MLPSP_E_ARG, "mlpsp_records_reverse: negative size");
+  // the variant with the caller's scratch, which this signature has no room for: taken from the stream's pool
   MLPSP_REQUIRE(offsets && grad_pos && grad_log_scales && grad_quats, MLPSP_E_ARG, "mlpsp_records_reverse: null pointer");
+  const int64_t bytes = mlpsp_records_reverse_scratch_bytes(total_records, n);
+  MLPSP_REQUIRE(bytes >= 0, MLPSP_E_ARG, "mlpsp_records_reverse: negative size");
   cudaStream_t st = (cudaStream_t)stream;
-  MLPSP_CUDA_OK(cudaMemsetAsync(grad_pos, 0, sizeof(float) * 3 * (size_t)n, st));
-  MLPSP_CUDA_OK(cudaMemsetAsync(grad_log_scales, 0, sizeof(float) * 3 * (size_t)n, st));
-  MLPSP_CUDA_OK(cudaMemsetAsync(grad_quats, 0, sizeof(float) * 4 * (size_t)n, st));
-  if (pixels == 0) return MLPSP_OK;
-  MLPSP_REQUIRE(ids && x6 && raw && log_scales && quats && grad_rgb && grad_t && d4, MLPSP_E_ARG,
-                "mlpsp_records_reverse: null pointer");
-  MLPSP_REQUIRE(total_records >= 0, MLPSP_E_ARG, "mlpsp_records_reverse: negative record count");
-  MLPSP_REQUIRE((reinterpret_cast<uintptr_t>(raw) & 15) == 0 && (reinterpret_cast<uintptr_t>(d4) & 15) == 0 &&
-                    (reinterpret_cast<uintptr_t>(quats) & 15) == 0, MLPSP_E_ARG,
-                "mlpsp_records_reverse: raw, d4 and quats must be 16-byte aligned");
-  LaunchScope scope(kKMisc, 2, st);
-  k_reverse_pixels<<<(unsigned)((pixels + 127) / 128), 128, 0, st>>>(offsets, raw, grad_rgb, grad_t, pixels, d4);
-  if (total_records > 0)
-    k_reverse_geometry<<<(unsigned)((total_records + kRevChunk - 1) / kRevChunk), kRevThreads, 0, st>>>(
-        ids, x6, raw, log_scales, quats, total_records, d4, grad_pos, grad_log_scales, grad_quats);
-  return cuda_check(cudaGetLastError(), "records_reverse");
+  char* work = nullptr;
+  MLPSP_CUDA_OK(cudaMallocAsync(&work, bytes, st));
+  const int rc = mlpsp_records_reverse_checked(ids, offsets, x6, raw, log_scales, quats, grad_rgb, grad_t, pixels, total_records, n,
+                                               d4, grad_pos, grad_log_scales, grad_quats, work, bytes, nullptr, stream);
+  cudaFreeAsync(work, st);
+  return rc;
 }
 
 extern "C" int64_t mlpsp_grouped_gradient_floats(void) { return kGradLen; }
+
+static int check_gradient_args(const mlpsp_scene* sc, const float* d4, int64_t segment_size, int precision, float loss_scale,
+                               const char* who) {
+  MLPSP_REQUIRE(sc->hidden == kGH && sc->num_freq == 6, MLPSP_E_LIMIT,
+                "grouped backward requires the 72→32→32→4 architecture");
+  MLPSP_REQUIRE(sc->W1 && sc->b1 && sc->W2 && sc->b2 && sc->W3 && sc->freq && sc->att, MLPSP_E_ARG,
+                "%s: FP32 weights missing", who);
+  MLPSP_REQUIRE(loss_scale > 0.f && segment_size > 0, MLPSP_E_ARG, "%s: bad loss scale, segment size or segment count", who);
+  MLPSP_REQUIRE(precision == MLPSP_PRECISION_F32 || precision == MLPSP_PRECISION_F16 || precision == MLPSP_PRECISION_BF16,
+                MLPSP_E_ARG, "%s: unsupported operand precision %d", who, precision);
+  MLPSP_REQUIRE(precision == MLPSP_PRECISION_F32 || (reinterpret_cast<uintptr_t>(d4) & 15) == 0, MLPSP_E_ARG,
+                "%s: d4 must be 16-byte aligned", who);
+  return MLPSP_OK;
+}
+
+extern "C" int64_t mlpsp_weight_gradients_scratch_bytes(int64_t num_records, int32_t n, int32_t segment_size) {
+  if (num_records < 0 || n < 0 || segment_size <= 0) return -1;
+  return vjp_scratch(num_records, n, segment_size).bytes;
+}
+
+extern "C" int mlpsp_weight_gradients(const mlpsp_scene* sc, const int64_t* offsets, const float* x6, const float* d4,
+                                      const int32_t* relu_masks, int64_t num_records, int32_t segment_size, int32_t precision,
+                                      float loss_scale, float* dW1, float* db1, float* dW2, float* db2, float* dW3, float* db3,
+                                      void* scratch, int64_t scratch_bytes, int32_t* nonfinite_host, void* stream) {
+  MLPSP_REQUIRE(sc && offsets && nonfinite_host && num_records >= 0, MLPSP_E_ARG, "mlpsp_weight_gradients: null pointer");
+  int rc = check_gradient_args(sc, d4, segment_size, precision, loss_scale, "mlpsp_weight_gradients");
+  if (rc) return rc;
+  *nonfinite_host = 0;
+  if (sc->n == 0) return MLPSP_OK;
+  MLPSP_REQUIRE(dW1 && db1 && dW2 && db2 && dW3 && db3 && (num_records == 0 || (x6 && d4)), MLPSP_E_ARG,
+                "mlpsp_weight_gradients: null pointer");
+  MLPSP_REQUIRE(num_records / segment_size + sc->n < (1ll << 31), MLPSP_E_LIMIT, "mlpsp_weight_gradients: too many segments");
+  const VjpOut out = {dW1, db1, dW2, db2, dW3, db3, kGH * kGIN, kGH, kGH * kGH, kGH, 4 * kGH, 4};
+  return weight_gradients(sc, offsets, x6, d4, relu_masks, num_records, segment_size, precision, loss_scale, out, scratch,
+                          scratch_bytes, nonfinite_host, nullptr, (cudaStream_t)stream);
+}
 
 extern "C" int mlpsp_grouped_weight_gradients(const mlpsp_scene* sc, const int64_t* offsets, const float* x6,
                                               const float* d4, const int32_t* relu_masks, const int64_t* seg_prim,
@@ -320,43 +661,26 @@ extern "C" int mlpsp_grouped_weight_gradients(const mlpsp_scene* sc, const int64
                                               int32_t segment_size, int32_t precision, float loss_scale, float* partial,
                                               float* result, int32_t* nonfinite, void* stream) {
   MLPSP_REQUIRE(sc && offsets && result && nonfinite, MLPSP_E_ARG, "mlpsp_grouped_weight_gradients: null pointer");
-  MLPSP_REQUIRE(sc->hidden == kGH && sc->num_freq == 6, MLPSP_E_LIMIT,
-                "grouped backward requires the 72->32->32->4 architecture");
-  MLPSP_REQUIRE(sc->W1 && sc->b1 && sc->W2 && sc->b2 && sc->W3 && sc->freq && sc->att, MLPSP_E_ARG,
-                "mlpsp_grouped_weight_gradients: FP32 weights missing");
-  MLPSP_REQUIRE(loss_scale > 0.f && num_segments >= 0 && num_segments < (1ll << 31) && segment_size > 0, MLPSP_E_ARG,
+  MLPSP_REQUIRE(num_segments >= 0 && num_segments < (1ll << 31), MLPSP_E_ARG,
                 "mlpsp_grouped_weight_gradients: bad loss scale, segment size or segment count");
-  MLPSP_REQUIRE(precision == MLPSP_PRECISION_F32 || precision == MLPSP_PRECISION_F16 || precision == MLPSP_PRECISION_BF16,
-                MLPSP_E_ARG, "mlpsp_grouped_weight_gradients: unsupported operand precision %d", precision);
   // every pointer a launch below reads is checked before the first CUDA call
   MLPSP_REQUIRE(sc->n == 0 || num_segments == 0 || (x6 && d4 && seg_prim && seg_start && seg_offsets && partial),
                 MLPSP_E_ARG, "mlpsp_grouped_weight_gradients: null pointer");
+  int rc = check_gradient_args(sc, d4, segment_size, precision, loss_scale, "mlpsp_grouped_weight_gradients");
+  if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   MLPSP_CUDA_OK(cudaMemsetAsync(nonfinite, 0, 4, st));
   if (sc->n == 0) return MLPSP_OK;
-  if (num_segments == 0) {
-    // no records at all: every primitive's gradient row is zero
-    return cuda_check(cudaMemsetAsync(result, 0, sizeof(float) * (size_t)sc->n * kGradLen, st), "grouped_weight_gradients");
-  }
-  LaunchScope scope(kKMisc, 2, st);
-  if (precision != MLPSP_PRECISION_F32) {
-    // binary16 / bfloat16 operands on the tensor cores, FP32 accumulation over the segment
-    MLPSP_REQUIRE((reinterpret_cast<uintptr_t>(d4) & 15) == 0, MLPSP_E_ARG,
-                  "mlpsp_grouped_weight_gradients: d4 must be 16-byte aligned");
-    const int rc = launch_grouped_vjp_tc(precision == MLPSP_PRECISION_BF16, x6, d4, relu_masks, offsets, seg_prim, seg_start,
-                                         num_segments, segment_size, sc, loss_scale, partial, nonfinite, st);
-    if (rc) return rc;
-    const dim3 grid_r(sc->n, (kGradLen + 255) / 256);
-    k_reduce_partials<<<grid_r, 256, 0, st>>>(partial, seg_offsets, sc->n, result, nonfinite);
-    return cuda_check(cudaGetLastError(), "grouped_weight_gradients");
-  }
-  static DeviceOnce attr_once;
-  if (attr_once.first())
-    MLPSP_CUDA_OK(cudaFuncSetAttribute(k_grouped_vjp, cudaFuncAttributeMaxDynamicSharedMemorySize, kGradSmem));
-  k_grouped_vjp<<<(unsigned)num_segments, kGSeg, kGradSmem, st>>>(x6, d4, relu_masks, offsets, seg_prim, seg_start, segment_size,
-                                                                  sc->freq, sc->att, sc->W1, sc->b1, sc->W2, sc->b2, sc->W3,
-                                                                  loss_scale, partial);
-  const dim3 grid(sc->n, (kGradLen + 255) / 256);
-  k_reduce_partials<<<grid, 256, 0, st>>>(partial, seg_offsets, sc->n, result, nonfinite);
-  return cuda_check(cudaGetLastError(), "grouped_weight_gradients");
+  // The segments follow from the offsets and the segment size, so the launch plans them itself; its scratch, which this
+  // signature has no room for, comes from the stream's pool.  num_segments * segment_size bounds the record count.
+  const int64_t records = num_segments * segment_size;
+  const int64_t bytes = vjp_scratch(records, sc->n, segment_size).bytes;
+  char* work = nullptr;
+  MLPSP_CUDA_OK(cudaMallocAsync(&work, bytes, st));
+  float* r = result;
+  const VjpOut out = {r + kOW1, r + kOb1, r + kOW2, r + kOb2, r + kOW3, r + kOb3, kGradLen, kGradLen, kGradLen, kGradLen, kGradLen, kGradLen};
+  rc = weight_gradients(sc, offsets, x6, d4, relu_masks, records, segment_size, precision, loss_scale, out, work, bytes, nullptr,
+                        nonfinite, st);
+  cudaFreeAsync(work, st);
+  return rc;
 }

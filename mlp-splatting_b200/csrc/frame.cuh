@@ -168,6 +168,9 @@ int cuda_check(cudaError_t e, const char* what);
     if (!(cond)) { ::mlpsp::set_error(__VA_ARGS__); return (code); }\
   } while (0)
 
+// SMs of the current device (asked once per device)
+int sm_count();
+
 // Per-device "first use" marker for settings that CUDA keeps per device (the opt-in dynamic shared-memory
 // size of a kernel, for one): a process that drives several GPUs must apply them once on each.  The caller
 // keeps one DeviceOnce per setting; first() answers true the first time it is asked with a given device current.
@@ -181,6 +184,29 @@ struct DeviceOnce {
     return true;
   }
 };
+
+// A few words of page-locked host memory that kernels write directly, and an event to wait for the kernel that does so:
+// a finding reaches the host without a copy, and without waiting for whatever was launched behind it.  One per host
+// thread (and, for the event, device), so calls of different threads do not meet; released with the thread.
+struct HostWords {
+  static constexpr int kWords = 16;
+  int32_t* word = nullptr;
+  cudaEvent_t event[64] = {nullptr};
+  int open(cudaEvent_t* ev) {
+    int dev = 0;
+    MLPSP_CUDA_OK(cudaGetDevice(&dev));
+    MLPSP_REQUIRE(dev >= 0 && dev < 64, MLPSP_E_LIMIT, "device ordinal %d beyond 63", dev);
+    if (!word) MLPSP_CUDA_OK(cudaHostAlloc((void**)&word, 4 * kWords, cudaHostAllocPortable | cudaHostAllocMapped));
+    if (!event[dev]) MLPSP_CUDA_OK(cudaEventCreateWithFlags(&event[dev], cudaEventDisableTiming));
+    *ev = event[dev];
+    return MLPSP_OK;
+  }
+  ~HostWords() {
+    if (word) cudaFreeHost(word);
+    for (cudaEvent_t e : event) if (e) cudaEventDestroy(e);
+  }
+};
+HostWords& host_words();
 
 // stage launchers (defined in the .cu files)
 // order_lists = false leaves every tile list in scatter order for a following launch_sort(unordered_input = true).
@@ -209,10 +235,6 @@ int launch_mlp_f32(const mlpsp_scene* sc, const RecIn* rec_in, const int32_t* pr
                    cudaStream_t st, int grid_cap = 0);
 // bf16: bfloat16 operands (sc->wbf16) instead of binary16 (sc->w16)
 // work_small: the wave's small-group list (launch_prim_scan with split_small), or null when every item is on `work`
-// per-primitive weight gradients with binary16 / bfloat16 operands on tcgen05 (vjp_tc.cu); flag bit 1 = a wait gave up
-int launch_grouped_vjp_tc(bool bf16, const float* x6, const float* d4, const int32_t* masks, const int64_t* offsets,
-                          const int64_t* seg_prim, const int64_t* seg_start, int64_t num_segments, int segment_size,
-                          const mlpsp_scene* sc, float scale, float* partial, int32_t* flag, cudaStream_t st);
 int launch_mlp_f16(const mlpsp_scene* sc, const RecIn* rec_in, const int32_t* prim_off, const int4* work,
                    const int32_t* counters, float4* rec_out, float4* rec_ext, int out_mode, int32_t* status,
                    cudaStream_t st, bool bf16 = false, int grid_cap = 0, const int4* work_small = nullptr);

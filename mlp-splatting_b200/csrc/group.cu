@@ -2,87 +2,169 @@
 // record ids by primitive + bincount + cumsum) and scannet/primitive_gemm.py:186-203
 // (prepare_groups: fixed-size segments of every primitive's record range).
 //
-// group_records is a device-wide stable LSD radix sort (4-bit digits) of (primitive id, record
-// index) pairs.  A block owns 2048 consecutive items; inside it, chunks of 32 items are ranked with
-// match.any, per-(digit, chunk) counts are scanned digit-major, and a global scan of per-block digit
-// totals (digit-major, block-minor) gives every block its scatter bases, so equal ids keep their
-// record order.
+// group_records is a device-wide stable LSD radix sort of (primitive id, record index) pairs with digits of up to
+// eight bits (two passes up to 65,535 primitives, three beyond).  A block owns 4,096 consecutive items, a warp 512 of
+// them in order.  Per pass: the blocks' digit counts, one scan per digit over the blocks, and the scatter, which ranks
+// the items of a warp with match.any against per-warp digit counters, orders the block's items by digit in shared
+// memory and writes them out in runs, so equal ids keep their record order.  The last kernel writes the permutation,
+// the CSR offsets (by binary search in the sorted keys: no counting pass) and the caller's record rows in the new order.
 #include "frame.cuh"
 
 namespace mlpsp {
 
 int launch_scan_i32(const int32_t* in, int64_t n, int32_t* blk, int32_t* out, cudaStream_t st);
 
-constexpr int kGsItems = 2048, kGsThreads = 256, kGsChunks = kGsItems / 32;
+constexpr int kGsThreads = 256, kGsRounds = 16, kGsItems = kGsThreads * kGsRounds, kGsWarps = kGsThreads / 32;
+constexpr int kGsBins = 256;
 
-__global__ void __launch_bounds__(kGsThreads) k_gs_hist(const uint32_t* __restrict__ keys, int64_t n, int shift,
-                                                        int nblocks, int32_t* __restrict__ ghist) {
-  __shared__ int h[16];
-  if (threadIdx.x < 16) h[threadIdx.x] = 0;
+// an id outside [0, nprim) sorts behind every primitive, as key nprim
+__device__ __forceinline__ uint32_t gs_key(int32_t id, int nprim) { return (uint32_t)id < (uint32_t)nprim ? (uint32_t)id : (uint32_t)nprim; }
+
+// digit counts of every block, digit-major: ghist[digit * nblocks + block]
+template <bool FIRST>
+__global__ void __launch_bounds__(kGsThreads) k_gs_hist(const uint32_t* __restrict__ keys, int64_t n, int nprim, int shift,
+                                                        int dbits, int nblocks, int32_t* __restrict__ ghist) {
+  chain_wait();
+  chain_release();
+  __shared__ int h[kGsBins];
+  h[threadIdx.x] = 0;
   __syncthreads();
   const int64_t base = (int64_t)blockIdx.x * kGsItems;
-  for (int j = threadIdx.x; j < kGsItems; j += kGsThreads)
-    if (base + j < n) atomicAdd(&h[(keys[base + j] >> shift) & 15u], 1);
+  const uint32_t dmask = (1u << dbits) - 1u;
+#pragma unroll
+  for (int r = 0; r < kGsRounds; ++r) {
+    const int64_t i = base + r * kGsThreads + threadIdx.x;
+    if (i < n) {
+      const uint32_t k = FIRST ? gs_key((int32_t)keys[i], nprim) : keys[i];
+      atomicAdd(&h[(k >> shift) & dmask], 1);
+    }
+  }
   __syncthreads();
-  if (threadIdx.x < 16) ghist[threadIdx.x * nblocks + blockIdx.x] = h[threadIdx.x];
+  if (threadIdx.x < (1u << dbits)) ghist[(size_t)threadIdx.x * nblocks + blockIdx.x] = h[threadIdx.x];
 }
 
+// block = one digit: exclusive prefix of its counts over the blocks, in place, and its total
+__global__ void __launch_bounds__(kGsThreads) k_gs_scan(int nblocks, int32_t* __restrict__ ghist, int32_t* __restrict__ dtot) {
+  chain_wait();
+  chain_release();
+  __shared__ int warp_sums[32];
+  int32_t* row = ghist + (size_t)blockIdx.x * nblocks;
+  int run = 0;
+  for (int b0 = 0; b0 < nblocks; b0 += kGsThreads) {
+    const int b = b0 + threadIdx.x;
+    const int v = b < nblocks ? row[b] : 0;
+    int total;
+    const int ex = block_exclusive_scan(v, warp_sums, total);
+    if (b < nblocks) row[b] = run + ex;
+    run += total;
+  }
+  if (threadIdx.x == 0) dtot[blockIdx.x] = run;
+}
+
+template <bool FIRST>
 __global__ void __launch_bounds__(kGsThreads) k_gs_scatter(
-    const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals, int64_t n, int shift, int nblocks,
-    const int32_t* __restrict__ gbase, uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out) {
-  __shared__ int cnt[16 * kGsChunks];
+    const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals, int64_t n, int nprim, int shift, int dbits, int nblocks,
+    const int32_t* __restrict__ ghist, const int32_t* __restrict__ dtot, uint32_t* __restrict__ keys_out,
+    uint32_t* __restrict__ vals_out) {
+  chain_wait();
+  chain_release();
+  __shared__ int s_cnt[kGsWarps][kGsBins];   // running digit counts per warp, then each warp's first position of a digit
+  __shared__ int s_dst[kGsBins];             // global position of the block's first item of a digit, minus its position here
+  __shared__ uint2 s_item[kGsItems];
   __shared__ int warp_sums[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t base = (int64_t)blockIdx.x * kGsItems;
-  for (int i = tid; i < 16 * kGsChunks; i += kGsThreads) cnt[i] = 0;
-  __syncthreads();
-  for (int c = warp; c < kGsChunks; c += kGsThreads / 32) {
-    const int64_t i = base + c * 32 + lane;
-    const bool valid = i < n;
-    const uint32_t d = valid ? ((keys[i] >> shift) & 15u) : 0xffffffffu;
+  const uint32_t dmask = (1u << dbits) - 1u, lt = (1u << lane) - 1u;
+  for (int i = lane; i < kGsBins; i += 32) s_cnt[warp][i] = 0;
+  __syncwarp();
+  uint32_t key[kGsRounds];
+  int rank[kGsRounds];
+#pragma unroll
+  for (int r = 0; r < kGsRounds; ++r) {
+    const int64_t i = base + warp * (kGsRounds * 32) + r * 32 + lane;
+    key[r] = i < n ? (FIRST ? gs_key((int32_t)keys[i], nprim) : keys[i]) : 0xffffffffu;
+  }
+#pragma unroll
+  for (int r = 0; r < kGsRounds; ++r) {
+    const bool valid = base + warp * (kGsRounds * 32) + r * 32 + lane < n;
+    const uint32_t d = valid ? ((key[r] >> shift) & dmask) : 0x1000u;
     const uint32_t peers = __match_any_sync(0xffffffffu, d);
-    if (valid && lane == __ffs(peers) - 1) cnt[d * kGsChunks + c] = __popc(peers);
+    const int before = valid ? s_cnt[warp][d] : 0;
+    rank[r] = before + __popc(peers & lt);
+    __syncwarp();
+    if (valid && (peers & lt) == 0u) s_cnt[warp][d] = before + __popc(peers);
+    __syncwarp();
   }
   __syncthreads();
-  constexpr int per = 16 * kGsChunks / kGsThreads;  // 4
-  int local = 0;
+  // thread = digit: the warps' first positions inside the digit, the digit's first position in the block and in the output
+  int mine = 0;
 #pragma unroll
-  for (int j = 0; j < per; ++j) local += cnt[tid * per + j];
+  for (int w = 0; w < kGsWarps; ++w) { const int c = s_cnt[w][tid]; s_cnt[w][tid] = mine; mine += c; }
   int total;
-  int ex = block_exclusive_scan(local, warp_sums, total);
+  const int local = block_exclusive_scan(mine, warp_sums, total);
+  const bool live = tid < (1 << dbits);
+  int unused;
+  const int global = block_exclusive_scan(live ? dtot[tid] : 0, warp_sums, unused);
+  s_dst[tid] = live ? global + ghist[(size_t)tid * nblocks + blockIdx.x] - local : 0;
 #pragma unroll
-  for (int j = 0; j < per; ++j) { const int v = cnt[tid * per + j]; cnt[tid * per + j] = ex; ex += v; }
+  for (int w = 0; w < kGsWarps; ++w) s_cnt[w][tid] += local;
   __syncthreads();
-  for (int c = warp; c < kGsChunks; c += kGsThreads / 32) {
-    const int64_t i = base + c * 32 + lane;
-    const bool valid = i < n;
-    const uint32_t k = valid ? keys[i] : 0u;
-    const uint32_t d = valid ? ((k >> shift) & 15u) : 0xffffffffu;
-    const uint32_t peers = __match_any_sync(0xffffffffu, d);
-    if (valid) {
-      const int64_t dst = (int64_t)gbase[d * nblocks + blockIdx.x] + (cnt[d * kGsChunks + c] - cnt[d * kGsChunks]) +
-                          __popc(peers & ((1u << lane) - 1u));
-      keys_out[dst] = k;
-      vals_out[dst] = vals[i];
+#pragma unroll
+  for (int r = 0; r < kGsRounds; ++r) {
+    const int64_t i = base + warp * (kGsRounds * 32) + r * 32 + lane;
+    if (i < n) {
+      const uint32_t d = (key[r] >> shift) & dmask;
+      s_item[s_cnt[warp][d] + rank[r]] = make_uint2(key[r], FIRST ? (uint32_t)i : vals[i]);
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < kGsRounds; ++r) {
+    const int j = r * kGsThreads + tid;
+    if (j < total) {
+      const uint2 it = s_item[j];
+      const int dst = s_dst[(it.x >> shift) & dmask] + j;
+      keys_out[dst] = it.x;
+      vals_out[dst] = it.y;
     }
   }
 }
 
-__global__ void k_gs_init(const int32_t* __restrict__ ids, int64_t n, int nprim, uint32_t* __restrict__ keys,
-                          uint32_t* __restrict__ vals, int32_t* __restrict__ counts) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int32_t p = ids[i];
-  keys[i] = (uint32_t)p;
-  vals[i] = (uint32_t)i;
-  if (p >= 0 && p < nprim) atomicAdd(counts + p, 1);
-}
-
-__global__ void k_gs_finish(const uint32_t* __restrict__ vals, int64_t n, int64_t* __restrict__ order,
-                            const int32_t* __restrict__ off32, int nprim, int64_t* __restrict__ offsets) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) order[i] = (int64_t)vals[i];
-  if (i <= nprim) offsets[i] = (int64_t)off32[i];
+// Permutation, CSR offsets and, where given, the records' rows in primitive-major order.  Bound by the random row
+// reads; every output is written in full lines (three consecutive threads move the three 8-byte words of an x6 row).
+// 4.3 M records of 48 bytes: see the figures at mlpsp_group_rows.
+__global__ void __launch_bounds__(256) k_gs_finish(
+    const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals, int64_t n, int nprim, int64_t* __restrict__ order,
+    int64_t* __restrict__ offsets, const float2* __restrict__ x6, const float4* __restrict__ d4, const int2* __restrict__ masks,
+    float2* __restrict__ x6_out, float4* __restrict__ d4_out, int2* __restrict__ masks_out) {
+  chain_wait();
+  chain_release();
+  __shared__ uint32_t s_val[256];
+  const int64_t base = (int64_t)blockIdx.x * 256;
+  const int64_t i = base + threadIdx.x;
+  const int rows = (int)max((int64_t)0, min((int64_t)256, n - base));
+  if (i < n) {
+    const uint32_t v = vals[i];
+    s_val[threadIdx.x] = v;
+    order[i] = (int64_t)v;
+    if (d4) d4_out[i] = __ldg(d4 + v);
+    if (masks) masks_out[i] = __ldg(masks + v);
+  }
+  if (i <= nprim) {      // first position whose key is not below i
+    int64_t lo = 0, hi = n;
+    while (lo < hi) {
+      const int64_t mid = (lo + hi) >> 1;
+      if (__ldg(keys + mid) < (uint32_t)i) lo = mid + 1; else hi = mid;
+    }
+    offsets[i] = lo;
+  }
+  if (!x6) return;
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < 3; ++u) {
+    const int w = u * 256 + threadIdx.x;
+    if (w < rows * 3) x6_out[base * 3 + w] = __ldg(x6 + (size_t)s_val[w / 3] * 3 + w % 3);
+  }
 }
 
 // total64 (zeroed by the caller) receives the exact number of groups: the per-primitive counts and their
@@ -113,22 +195,65 @@ __global__ void k_groups_fill(const int64_t* __restrict__ offsets, int n, int64_
     if (g < max_groups) { primitives[g] = i; starts[g] = offsets[i] + (int64_t)(g - g0) * seg; }
 }
 
-// scratch: counts[n+1] | off32[n+2] | scan blocks | ghist[16*nblocks] | gbase[16*nblocks+1] | 4 x uint32[R]
-struct GsLayout { int64_t o[9]; int64_t bytes; };
-static GsLayout gs_layout(int64_t R, int n) {
+// digits of the primitive ids (and of the key that stands for an invalid one): equal passes of at most eight bits
+struct GsPlan { int passes, dbits, nblocks; };
+static GsPlan gs_plan(int64_t R, int n) {
+  int bits = 1;
+  while (bits < 31 && (1ll << bits) <= (int64_t)n) ++bits;      // keys 0 .. n
+  GsPlan g;
+  g.passes = (bits + 7) / 8;
+  g.dbits = (bits + g.passes - 1) / g.passes;
+  g.nblocks = (int)((R + kGsItems - 1) / kGsItems);
+  return g;
+}
+
+// scratch: digit totals | block counts | 2 x keys | 2 x indices
+struct GsLayout { int64_t dtot, hist, key[2], val[2], bytes; };
+static GsLayout gs_layout(int64_t R) {
   GsLayout L;
   int64_t off = 0;
   auto take = [&](int64_t bytes) { int64_t o = off; off += align_up(bytes, 256); return o; };
-  const int64_t nblocks = std::max<int64_t>((R + kGsItems - 1) / kGsItems, 1);
-  L.o[0] = take(4 * ((int64_t)n + 1));
-  L.o[1] = take(4 * ((int64_t)n + 2));
-  const int64_t scan_n = std::max<int64_t>((int64_t)n + 1, 16 * nblocks);
-  L.o[2] = take(4 * (scan_n / kScanItems + 4));
-  L.o[3] = take(4 * 16 * nblocks);
-  L.o[4] = take(4 * (16 * nblocks + 1));
-  for (int i = 5; i < 9; ++i) L.o[i] = take(4 * R);
+  L.dtot = take(4 * kGsBins);
+  L.hist = take(4 * kGsBins * std::max<int64_t>((R + kGsItems - 1) / kGsItems, 1));
+  for (int i = 0; i < 2; ++i) { L.key[i] = take(4 * R); L.val[i] = take(4 * R); }
   L.bytes = off;
   return L;
+}
+
+static int group_rows(const int32_t* ids, int64_t R, int n, int64_t* offsets, int64_t* order, const float* x6, const float* d4,
+                      const int32_t* masks, float* x6_out, float* d4_out, int32_t* masks_out, void* scratch,
+                      int64_t scratch_bytes, cudaStream_t st, const char* who) {
+  MLPSP_REQUIRE(R >= 0 && n >= 0 && offsets, MLPSP_E_ARG, "%s: bad arguments", who);
+  MLPSP_REQUIRE(R < (1ll << 31), MLPSP_E_LIMIT, "%s: more than 2^31-1 records", who);
+  MLPSP_REQUIRE(R == 0 || (ids && order), MLPSP_E_ARG, "%s: null pointer", who);
+  MLPSP_REQUIRE((!x6 || x6_out) && (!d4 || d4_out) && (!masks || masks_out), MLPSP_E_ARG, "%s: null pointer", who);
+  const GsLayout L = gs_layout(R);
+  MLPSP_REQUIRE(scratch && scratch_bytes >= L.bytes, MLPSP_E_SCRATCH, "%s: scratch needs %lld bytes", who, (long long)L.bytes);
+  if (R == 0) return cuda_check(cudaMemsetAsync(offsets, 0, 8 * ((size_t)n + 1), st), who);
+  const GsPlan g = gs_plan(R, n);
+  LaunchScope scope(kKMisc, 3 * g.passes + 1, st);
+  char* b = (char*)scratch;
+  int32_t* dtot = (int32_t*)(b + L.dtot);
+  int32_t* hist = (int32_t*)(b + L.hist);
+  const uint32_t* k_in = reinterpret_cast<const uint32_t*>(ids);
+  const uint32_t* v_in = nullptr;
+  for (int pass = 0; pass < g.passes; ++pass) {
+    const int shift = pass * g.dbits;
+    uint32_t* k_out = (uint32_t*)(b + L.key[pass & 1]);
+    uint32_t* v_out = (uint32_t*)(b + L.val[pass & 1]);
+    if (pass == 0) launch_chained(k_gs_hist<true>, dim3(g.nblocks), dim3(kGsThreads), 0, st, k_in, R, n, shift, g.dbits, g.nblocks, hist);
+    else launch_chained(k_gs_hist<false>, dim3(g.nblocks), dim3(kGsThreads), 0, st, k_in, R, n, shift, g.dbits, g.nblocks, hist);
+    launch_chained(k_gs_scan, dim3(1 << g.dbits), dim3(kGsThreads), 0, st, g.nblocks, hist, dtot);
+    if (pass == 0) launch_chained(k_gs_scatter<true>, dim3(g.nblocks), dim3(kGsThreads), 0, st, k_in, v_in, R, n, shift, g.dbits, g.nblocks, hist, dtot, k_out, v_out);
+    else launch_chained(k_gs_scatter<false>, dim3(g.nblocks), dim3(kGsThreads), 0, st, k_in, v_in, R, n, shift, g.dbits, g.nblocks, hist, dtot, k_out, v_out);
+    k_in = k_out;
+    v_in = v_out;
+  }
+  const int64_t span = std::max<int64_t>(R, (int64_t)n + 1);
+  launch_chained(k_gs_finish, dim3((unsigned)((span + 255) / 256)), dim3(256), 0, st, k_in, v_in, R, n, order, offsets,
+                 reinterpret_cast<const float2*>(x6), reinterpret_cast<const float4*>(d4), reinterpret_cast<const int2*>(masks),
+                 reinterpret_cast<float2*>(x6_out), reinterpret_cast<float4*>(d4_out), reinterpret_cast<int2*>(masks_out));
+  return cuda_check(cudaGetLastError(), who);
 }
 
 }  // namespace mlpsp
@@ -137,45 +262,25 @@ using namespace mlpsp;
 
 extern "C" int64_t mlpsp_group_records_scratch_bytes(int64_t num_records, int32_t n) {
   if (num_records < 0 || n < 0) return -1;
-  return gs_layout(num_records, n).bytes;
+  return gs_layout(num_records).bytes;
 }
 
 extern "C" int mlpsp_group_records(const int32_t* primitive_ids, int64_t num_records, int32_t n, int64_t* offsets,
                                    int64_t* order, void* scratch, int64_t scratch_bytes, void* stream) {
-  cudaStream_t st = (cudaStream_t)stream;
-  MLPSP_REQUIRE(num_records >= 0 && n >= 0 && offsets, MLPSP_E_ARG, "mlpsp_group_records: bad arguments");
-  MLPSP_REQUIRE(num_records < (1ll << 31), MLPSP_E_LIMIT, "mlpsp_group_records: more than 2^31-1 records");
-  MLPSP_REQUIRE(num_records == 0 || (primitive_ids && order), MLPSP_E_ARG, "mlpsp_group_records: null pointer");
-  const int64_t R = num_records;
-  const int nblocks = (int)((R + kGsItems - 1) / kGsItems);
-  GsLayout L = gs_layout(R, n);
-  MLPSP_REQUIRE(scratch && scratch_bytes >= L.bytes, MLPSP_E_SCRATCH, "mlpsp_group_records: scratch needs %lld bytes",
-                (long long)L.bytes);
-  const int64_t o_cnt = L.o[0], o_off = L.o[1], o_blk = L.o[2], o_gh = L.o[3], o_gb = L.o[4];
-  const int64_t o_k0 = L.o[5], o_k1 = L.o[6], o_v0 = L.o[7], o_v1 = L.o[8];
-  char* b = (char*)scratch;
-  int32_t* counts = (int32_t*)(b + o_cnt); int32_t* off32 = (int32_t*)(b + o_off); int32_t* blk = (int32_t*)(b + o_blk);
-  int32_t* ghist = (int32_t*)(b + o_gh); int32_t* gbase = (int32_t*)(b + o_gb);
-  uint32_t* k[2] = {(uint32_t*)(b + o_k0), (uint32_t*)(b + o_k1)};
-  uint32_t* v[2] = {(uint32_t*)(b + o_v0), (uint32_t*)(b + o_v1)};
-  MLPSP_CUDA_OK(cudaMemsetAsync(counts, 0, 4 * ((size_t)n + 1), st));
-  if (R > 0) k_gs_init<<<(unsigned)((R + 255) / 256), 256, 0, st>>>(primitive_ids, R, n, k[0], v[0], counts);
-  int rc = launch_scan_i32(counts, (int64_t)n, blk, off32, st);
-  if (rc) return rc;
-  if (n == 0) MLPSP_CUDA_OK(cudaMemsetAsync(off32, 0, 4, st));
-  int cur = 0;
-  int bits = 1;
-  while (bits < 32 && (1ll << bits) < (int64_t)std::max(n, 1)) ++bits;
-  for (int shift = 0; shift < bits && R > 0; shift += 4) {
-    k_gs_hist<<<nblocks, kGsThreads, 0, st>>>(k[cur], R, shift, nblocks, ghist);
-    rc = launch_scan_i32(ghist, 16ll * nblocks, blk, gbase, st);
-    if (rc) return rc;
-    k_gs_scatter<<<nblocks, kGsThreads, 0, st>>>(k[cur], v[cur], R, shift, nblocks, gbase, k[cur ^ 1], v[cur ^ 1]);
-    cur ^= 1;
-  }
-  const int64_t span = std::max<int64_t>(R, (int64_t)n + 1);
-  k_gs_finish<<<(unsigned)((span + 255) / 256), 256, 0, st>>>(v[cur], R, order, off32, n, offsets);
-  return cuda_check(cudaGetLastError(), "group_records");
+  return group_rows(primitive_ids, num_records, n, offsets, order, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, scratch,
+                    scratch_bytes, (cudaStream_t)stream, "mlpsp_group_records");
+}
+
+extern "C" int mlpsp_group_rows(const int32_t* primitive_ids, int64_t num_records, int32_t n, const float* x6,
+                                const float* grad4, const int32_t* relu_masks, int64_t* offsets, int64_t* order,
+                                float* x6_out, float* grad4_out, int32_t* masks_out, void* scratch, int64_t scratch_bytes,
+                                void* stream) {
+  MLPSP_REQUIRE(((reinterpret_cast<uintptr_t>(x6) | reinterpret_cast<uintptr_t>(x6_out) | reinterpret_cast<uintptr_t>(relu_masks) |
+                  reinterpret_cast<uintptr_t>(masks_out)) & 7) == 0 &&
+                    ((reinterpret_cast<uintptr_t>(grad4) | reinterpret_cast<uintptr_t>(grad4_out)) & 15) == 0,
+                MLPSP_E_ARG, "mlpsp_group_rows: x6 and masks must be 8-byte aligned, grad4 16-byte aligned");
+  return group_rows(primitive_ids, num_records, n, offsets, order, x6, grad4, relu_masks, x6_out, grad4_out, masks_out, scratch,
+                    scratch_bytes, (cudaStream_t)stream, "mlpsp_group_rows");
 }
 
 extern "C" int mlpsp_prepare_groups(const int64_t* offsets, int32_t n, int64_t segment_size, int64_t* group_offsets,

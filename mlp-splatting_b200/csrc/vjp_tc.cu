@@ -2,81 +2,146 @@
 // the mixed-precision modes of grouped_weight_gradients (scannet/primitive_gemm.py:101-166: binary16 or bfloat16
 // operands, FP32 accumulation over the whole segment, adjoints scaled before the cast and unscaled in FP32).
 //
-// One CTA owns one prepared segment of one primitive and walks it in blocks of 128 records (thread = record).
-// All operand tiles of a block live in shared memory as chunks of [128 records][8 elements] (16 bytes per record,
-// 2,048 bytes per chunk).  That one layout serves two kinds of product:
+// The launch is persistent: a CTA walks the planned segments (VjpItem, backward.cu) round-robin in blocks of 128
+// records (thread = record).  All operand tiles of a block live in shared memory as chunks of [128 records][8 elements]
+// (16 bytes per record, 2,048 bytes per chunk).  That one layout serves two kinds of product:
 //   * record-major products (rows of D = records), the tile is the K-major A operand as in the evaluator:
-//       H1 = relu(E W1^T + b1), H2 = relu(H1 W2^T + b2), D2 = (D3 W3) * mask2, D1 = (D2 W2) * mask1;
+//       H1 = relu(E W1^T + b1), H2 = relu(H1 W2^T + b2), D1 = (D2 W2) * mask1
+//     (W2 is stored once: K-major for layer 2, the same bytes MN-major for D1);
 //   * the weight gradients contract over the records, so the same bytes are read as MN-major operands
 //     (eight records x eight elements = one 128-byte core matrix with the element dimension contiguous):
-//       dW1^T [72 x 32] += E^T D1,   dW2^T [32 x 32] += H1^T D2,   dW3^T [32 x 4] += H2^T D3
+//       dW1^T [72 x 32] += E^T D1,   [H1 | H2]^T [D2 | D3]: dW2^T [32 x 32] and dW3^T [32 x 4] are two blocks of it
 //     with M = 128 rows of the tensor core over the element dimension (rows past the operand's width read the
-//     chunks that follow and land in accumulator lanes nobody looks at), N = 32 or 16, K = 16 records per MMA.
-//     A chunk of ones directly behind E, H1 and H2 makes the bias gradients the next accumulator lane:
-//     db1 = sum D1 is lane 72 of dW1^T, db2 / db3 lane 32 of dW2^T / dW3^T -- FP32 sums of the rounded adjoints,
-//     as primitive_gemm.py:157-160 takes them.
-// The three gradient accumulators stay in tensor memory for the whole segment and are written, divided by the
-// scale, as the segment's partial row; k_reduce_partials (backward.cu) adds the rows of a primitive in order.
+//     chunks that follow and land in accumulator lanes nobody looks at), K = 16 records per MMA, as many K steps as the
+//     block has records.  A chunk of ones directly behind E, H1 and H2 makes the bias gradients the next accumulator
+//     lane -- FP32 sums of the rounded adjoints, as primitive_gemm.py:157-160 takes them.
+// D2 = (D3 W3) * mask2 has K = 4 and is done by the threads from the rounded operands.
+// The gradient accumulators stay in tensor memory for the whole segment and are written, divided by the scale, to the
+// primitive's gradient tensors, or -- for a primitive of several segments -- to the segment's partial row.
 //
-// A block costs five MMA round trips (layer 1, layer 2, D2, D1, gradients), each: operand tile complete ->
-// fence -> CTA barrier -> one thread issues and commits -> everyone waits on the mbarrier (bounded: a wait that
-// gives up sets bit 1 of the flag word and the CTA leaves after freeing its tensor memory).  The gradient MMAs
-// of a block run while the threads compute the next block's encoding in registers.
+// What bounds it: the chain of MMA round trips of a block (operand tile complete -> fence -> CTA barrier -> one thread
+// issues and commits -> everyone waits on the mbarrier, bounded), about a microsecond each; bytes (weights in, gradients
+// out, 48 B per record) would take a quarter of the time.  So the chain is kept short -- with saved masks the adjoint
+// chain does not depend on the forward one, and the halves of D1 ride with layer 1 and layer 2: three round trips per
+// block instead of five -- the last one (the gradients) overlaps the next block's encoding, and the next block's
+// records and weights are loaded into registers while the current block's MMAs run.
 #include "frame.cuh"
 #include "tc.cuh"
+#include "vjp.cuh"
 
 namespace mlpsp {
 
-constexpr int kVjpRows = 128, kVjpChunk = kVjpRows * 16;
+constexpr int kVjpRows = kVjpBlock, kVjpChunk = kVjpRows * 16;
 // chunk indices of the operand tiles
 constexpr int kVcE = 0, kVcOneE = 9, kVcH1 = 10, kVcOneH1 = 14, kVcH2 = 15, kVcOneH2 = 19, kVcD1 = 20, kVcD2 = 24,
               kVcD3 = 28, kVcEnd = 30;
-// weight operands (K-major B: [K / 8 chunks][32 rows][8 elements], 512 bytes per chunk)
+// weight operands ([K / 8 chunks][32 rows][8 elements], 512 bytes per chunk)
 constexpr int kVoW1 = kVcEnd * kVjpChunk;          // W1[h][j], 10 chunks (the last one zero: it meets the ones behind E)
 constexpr int kVoW2 = kVoW1 + 10 * 512;            // W2[q][h], 4 chunks
-constexpr int kVoW2T = kVoW2 + 4 * 512;            // rows h, K = q: W2[q][h]
-constexpr int kVoW3T = kVoW2T + 4 * 512;           // rows h, K = output c (4 of 16): W3[c][h]
-constexpr int kVoBias = kVoW3T + 2 * 512;          // b1[32], b2[32] as FP32
+constexpr int kVoW3 = kVoW2 + 4 * 512;             // W3[c][h], rounded to the operand format, as FP32: [32][4]
+constexpr int kVoBias = kVoW3 + 512;               // b1[32], b2[32] as FP32
 constexpr int kVoBar = kVoBias + 256;
 constexpr int kVjpSmem = kVoBar + 16;
-constexpr int kVjpTmemCols = 128;                  // [0,32) transient, [32,64) dW1^T, [64,96) dW2^T, [96,112) dW3^T
-static_assert((kVcH2 + 16) * kVjpChunk <= kVoW2, "an M = 128 window from any tile start stays inside the allocation");
+// tensor memory: [0,32) layers, [32,64) dW1^T, [64,112) dW2^T | dW3^T, [112,128) one half of D1
+constexpr int kVjpTmemCols = 128, kVtG1 = 32, kVtG2 = 64, kVtD1 = 112;
+constexpr int kVjpCtas = 3;
+static_assert((kVcH1 + 16) * kVjpChunk <= kVoW1, "an M = 128 window from any tile start stays inside the tiles");
+static_assert(kVjpCtas * (kVjpSmem + 1024) <= 227 * 1024, "resident CTAs");
 
-constexpr int kVW1 = 32 * 72, kVW2 = 32 * 32, kVW3 = 4 * 32;
-constexpr int kVOb1 = kVW1, kVOW2 = kVOb1 + 32, kVOb2 = kVOW2 + kVW2, kVOW3 = kVOb2 + 32, kVOb3 = kVOW3 + kVW3;
-static_assert(kVOb3 + 4 == 3524, "gradient row layout");
-
-// instruction descriptor with both operands MN-major (bits 15 and 16)
-__host__ __device__ constexpr uint32_t vjp_idesc_mn(int M, int N, bool bf16) { return instr_desc(M, N, bf16) | (1u << 15) | (1u << 16); }
+// bits 15 / 16 of the instruction descriptor: A / B is MN-major
+constexpr uint32_t kMnA = 1u << 15, kMnB = 1u << 16;
 
 template <bool BF16>
 __device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
   return make_uint4(pack_h2<BF16>(v[0], v[1]), pack_h2<BF16>(v[2], v[3]), pack_h2<BF16>(v[4], v[5]), pack_h2<BF16>(v[6], v[7]));
 }
-
+// the two values of a packed word, as FP32
 template <bool BF16>
-__global__ void __launch_bounds__(kVjpRows, 3) k_grouped_vjp_tc(
+__device__ __forceinline__ float2 unpack_h2(uint32_t w) {
+  if (BF16) return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w));
+  return __half22float2(*reinterpret_cast<const __half2*>(&w));
+}
+
+// ReLU + rounding of 32 accumulator columns (+ FP32 bias) into a hidden tile; returns the sign mask
+template <bool BF16>
+__device__ __forceinline__ uint32_t vjp_hidden(const uint32_t (&acc)[32], const float* __restrict__ bias, char* dst) {
+  uint32_t sign = 0u;
+#pragma unroll
+  for (int kc = 0; kc < 4; ++kc) {
+    uint32_t w[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int j = kc * 8 + q * 2;
+      const float v0 = __uint_as_float(acc[j]) + bias[j], v1 = __uint_as_float(acc[j + 1]) + bias[j + 1];
+      sign |= (v0 > 0.f ? 1u : 0u) << j;
+      sign |= (v1 > 0.f ? 1u : 0u) << (j + 1);
+      w[q] = pack_h2_relu<BF16>(v0, v1);
+    }
+    *reinterpret_cast<uint4*>(dst + kc * kVjpChunk) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+  return sign;
+}
+
+// N accumulator columns (N / 8 chunks of an adjoint tile), masked and rounded; m holds the mask bits of these columns
+template <bool BF16, int N>
+__device__ __forceinline__ void vjp_adjoint(const uint32_t (&acc)[N], uint32_t m, char* dst) {
+#pragma unroll
+  for (int kc = 0; kc < N / 8; ++kc) {
+    uint32_t w[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int j = kc * 8 + q * 2;
+      const float v0 = ((m >> j) & 1u) ? __uint_as_float(acc[j]) : 0.f;
+      const float v1 = ((m >> (j + 1)) & 1u) ? __uint_as_float(acc[j + 1]) : 0.f;
+      w[q] = pack_h2<BF16>(v0, v1);
+    }
+    *reinterpret_cast<uint4*>(dst + kc * kVjpChunk) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+
+// D2 = (D3 W3) * mask2 of one record, from the rounded operands
+template <bool BF16>
+__device__ __forceinline__ void vjp_d2(uint32_t d01, uint32_t d23, uint32_t m2, const float4* __restrict__ w3, char* dst) {
+  const float2 a = unpack_h2<BF16>(d01), b = unpack_h2<BF16>(d23);
+#pragma unroll
+  for (int kc = 0; kc < 4; ++kc) {
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float4 w = w3[kc * 8 + i];
+      const float s = fmaf(a.x, w.x, fmaf(a.y, w.y, fmaf(b.x, w.z, b.y * w.w)));
+      v[i] = ((m2 >> (kc * 8 + i)) & 1u) ? s : 0.f;
+    }
+    *reinterpret_cast<uint4*>(dst + kc * kVjpChunk) = pack8<BF16>(v);
+  }
+}
+
+// MASKS: the records carry saved ReLU masks.  Without them the signs come from the recomputed layers, the adjoint chain
+// has to follow the forward one, and a block takes four round trips.  vec: rows may be loaded in 16- and 8-byte pieces.
+template <bool BF16, bool MASKS>
+__global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
     const float* __restrict__ x6, const float* __restrict__ d4, const int32_t* __restrict__ masks,
-    const int64_t* __restrict__ offsets, const int64_t* __restrict__ seg_prim, const int64_t* __restrict__ seg_start,
-    int segment_size, const float* __restrict__ freq, const float* __restrict__ att, const float* __restrict__ W1,
-    const float* __restrict__ b1, const float* __restrict__ W2, const float* __restrict__ b2,
-    const float* __restrict__ W3, float scale, float* __restrict__ partial, int32_t* __restrict__ flag) {
+    const VjpItem* __restrict__ items, int32_t* __restrict__ counters, const float* __restrict__ freq,
+    const float* __restrict__ att, const float* __restrict__ W1, const float* __restrict__ b1, const float* __restrict__ W2,
+    const float* __restrict__ b2, const float* __restrict__ W3, int vec, float scale, VjpOut out, float* __restrict__ partial) {
+  chain_wait();
+  chain_release();
   extern __shared__ __align__(128) char smem[];
-  const int seg = blockIdx.x, tid = threadIdx.x, warp = tid >> 5;
-  const int p = (int)seg_prim[seg];
-  const int64_t begin = seg_start[seg];
-  const int total = (int)min((int64_t)segment_size, offsets[p + 1] - begin);
+  const int G = counters[kVpItems];
+  int idx = blockIdx.x;
+  if (idx >= G) return;
+  const int tid = threadIdx.x, warp = tid >> 5;
   uint64_t* s_bar = reinterpret_cast<uint64_t*>(smem + kVoBar);
   uint32_t* s_misc = reinterpret_cast<uint32_t*>(s_bar + 1);
-  float* s_b1 = reinterpret_cast<float*>(smem + kVoBias);
-  float* s_b2 = s_b1 + 32;
+  float* s_bias = reinterpret_cast<float*>(smem + kVoBias);
+  float* s_w3 = reinterpret_cast<float*>(smem + kVoW3);
   const uint32_t sb = smem_u32(smem), bar = smem_u32(s_bar);
   if (tid == 0) {
     mbar_init(bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) tmem_alloc(smem_u32(&s_misc[0]), kVjpTmemCols);
-  // tiles: zeros, except the three chunks of ones
+  // tiles: zeros, except the three chunks of ones; W1's last chunk stays zero
   {
     const uint32_t one2 = BF16 ? 0x3f803f80u : 0x3c003c00u;
     for (int i = tid; i < kVcEnd * kVjpRows; i += kVjpRows) {
@@ -84,60 +149,31 @@ __global__ void __launch_bounds__(kVjpRows, 3) k_grouped_vjp_tc(
       const uint32_t v = (chunk == kVcOneE || chunk == kVcOneH1 || chunk == kVcOneH2) ? one2 : 0u;
       *reinterpret_cast<uint4*>(smem + (size_t)i * 16) = make_uint4(v, v, v, v);
     }
-  }
-  // the primitive's weights in the operand format (RN), as primitive_gemm.py:118-120 casts them
-  {
-    const float* w1 = W1 + (size_t)p * kVW1;
-    const float* w2 = W2 + (size_t)p * kVW2;
-    const float* w3 = W3 + (size_t)p * kVW3;
-    float v[8];
-    for (int g = tid; g < 320; g += kVjpRows) {
-      const int n = g & 31, kc = g >> 5;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = kc < 9 ? __ldg(w1 + n * 72 + kc * 8 + i) : 0.f;
-      *reinterpret_cast<uint4*>(smem + kVoW1 + kc * 512 + n * 16) = pack8<BF16>(v);
-    }
-    {
-      const int n = tid & 31, kc = tid >> 5;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = __ldg(w2 + n * 32 + kc * 8 + i);
-      *reinterpret_cast<uint4*>(smem + kVoW2 + kc * 512 + n * 16) = pack8<BF16>(v);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = __ldg(w2 + (kc * 8 + i) * 32 + n);
-      *reinterpret_cast<uint4*>(smem + kVoW2T + kc * 512 + n * 16) = pack8<BF16>(v);
-    }
-    if (tid < 64) {
-      const int n = tid & 31, kc = tid >> 5;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = (kc == 0 && i < 4) ? __ldg(w3 + i * 32 + n) : 0.f;
-      *reinterpret_cast<uint4*>(smem + kVoW3T + kc * 512 + n * 16) = pack8<BF16>(v);
-    }
-    if (tid < 32) { s_b1[tid] = __ldg(b1 + (size_t)p * 32 + tid); s_b2[tid] = __ldg(b2 + (size_t)p * 32 + tid); }
+    if (tid < 32) *reinterpret_cast<uint4*>(smem + kVoW1 + 9 * 512 + tid * 16) = make_uint4(0u, 0u, 0u, 0u);
   }
   float mult[6];
 #pragma unroll
   for (int f = 0; f < 6; ++f) mult[f] = __ldg(freq + f) * __ldg(att + f);
-  fence_async_smem();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = s_misc[0];
   const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
 
-  const uint32_t idesc_h = instr_desc(kVjpRows, 32, BF16);
-  const uint32_t idesc_g32 = vjp_idesc_mn(kVjpRows, 32, BF16), idesc_g16 = vjp_idesc_mn(kVjpRows, 16, BF16);
+  constexpr uint32_t idesc_h = instr_desc(kVjpRows, 32, BF16), idesc_d1 = instr_desc(kVjpRows, 32, BF16) | kMnB,
+                     idesc_d1h = instr_desc(kVjpRows, 16, BF16) | kMnB,
+                     idesc_g1 = instr_desc(kVjpRows, 32, BF16) | kMnA | kMnB, idesc_g2 = instr_desc(kVjpRows, 48, BF16) | kMnA | kMnB;
   auto tile = [&](int chunk) { return sb + (uint32_t)chunk * kVjpChunk; };
   // record-major A operand (K-major): K chunks a chunk apart, groups of eight records 128 bytes apart
   auto a_rows = [&](int chunk) { return smem_desc(tile(chunk), kVjpChunk, 128); };
-  // K-major B operand of the weights
-  auto b_w = [&](int off) { return smem_desc(sb + off, 512, 128); };
   // MN-major operand: groups of eight elements a chunk apart, groups of eight records 128 bytes apart
   auto mn = [&](int chunk) { return smem_desc(tile(chunk), 128, kVjpChunk); };
   auto adv = [](uint64_t desc, int bytes) { return desc + (uint64_t)(bytes >> 4); };
+  const uint64_t w1_desc = smem_desc(sb + kVoW1, 512, 128), w2_desc = smem_desc(sb + kVoW2, 512, 128);
+  const uint64_t w2t_desc = smem_desc(sb + kVoW2, 128, 512);      // N = h (a chunk per eight), K = q (128 bytes per eight)
 
   char* my = smem + tid * 16;
   uint32_t ph = 0u;
-  bool ok = true;
   // tile writes visible to the tensor core, tensor-memory reads retired, then one thread issues and commits
   auto issue_phase = [&](auto issue) {
     fence_async_smem();
@@ -155,213 +191,271 @@ __global__ void __launch_bounds__(kVjpRows, 3) k_grouped_vjp_tc(
     tc_fence_after();
     return __syncthreads_and(done) != 0;
   };
-  auto round_trip = [&](auto issue) -> bool {
-    issue_phase(issue);
-    return wait_phase();
-  };
-  bool grads_pending = false;     // the previous block's gradient MMAs still read its tiles
 
-  for (int sub = 0; sub < total && ok; sub += kVjpRows) {
-    const int cnt = min(kVjpRows, total - sub);
-    const bool valid = tid < cnt;
-    const int64_t r = begin + sub + tid;
-    uint32_t m1 = 0u, m2 = 0u;
+  // ---- a step's inputs in registers: one record per thread, and with a new primitive its weights ----
+  float rx[6];
+  float4 rg;
+  uint32_t rm1 = 0u, rm2 = 0u;
+  auto load_rec = [&](const VjpItem& it, int sub) {
+#pragma unroll
+    for (int c = 0; c < 6; ++c) rx[c] = 0.f;
+    rg = make_float4(0.f, 0.f, 0.f, 0.f);
+    rm1 = rm2 = 0u;
+    if (sub + tid < it.rows) {
+      const int64_t r = it.start + sub + tid;
+      if (vec) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const float2 v = __ldg(reinterpret_cast<const float2*>(x6) + r * 3 + c);
+          rx[2 * c] = v.x; rx[2 * c + 1] = v.y;
+        }
+      } else {
+#pragma unroll
+        for (int c = 0; c < 6; ++c) rx[c] = __ldg(x6 + r * 6 + c);
+      }
+      rg = __ldg(reinterpret_cast<const float4*>(d4) + r);
+      if (MASKS) { rm1 = (uint32_t)__ldg(masks + r * 2); rm2 = (uint32_t)__ldg(masks + r * 2 + 1); }
+    }
+  };
+  // W1 as 288 groups of eight consecutive k of one row, W2 as 128, W3 and the biases one value per thread
+  float wv[4][8], wr3 = 0.f, wrb = 0.f;
+  auto load8 = [&](const float* p, float (&v)[8]) {
+    if (vec) {
+      const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+      v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = __ldg(p + i);
+    }
+  };
+  auto load_weights = [&](int prim) {
+    const float* w1 = W1 + (size_t)prim * (kGH * kGIN);
+#pragma unroll
+    for (int u = 0; u < 3; ++u) {
+      const int g = u * kVjpRows + tid;
+      if (u < 2 || g < 288) load8(w1 + (g & 31) * kGIN + (g >> 5) * 8, wv[u]);
+    }
+    load8(W2 + (size_t)prim * (kGH * kGH) + (tid & 31) * kGH + (tid >> 5) * 8, wv[3]);
+    wr3 = __ldg(W3 + (size_t)prim * (4 * kGH) + tid);
+    if (tid < 64) wrb = __ldg((tid < 32 ? b1 : b2) + (size_t)prim * kGH + (tid & 31));
+  };
+  auto store_weights = [&]() {
+#pragma unroll
+    for (int u = 0; u < 3; ++u) {
+      const int g = u * kVjpRows + tid;
+      if (u < 2 || g < 288) *reinterpret_cast<uint4*>(smem + kVoW1 + (g >> 5) * 512 + (g & 31) * 16) = pack8<BF16>(wv[u]);
+    }
+    *reinterpret_cast<uint4*>(smem + kVoW2 + (tid >> 5) * 512 + (tid & 31) * 16) = pack8<BF16>(wv[3]);
+    s_w3[(tid & 31) * 4 + (tid >> 5)] = unpack_h2<BF16>(pack_h2<BF16>(wr3, 0.f)).x;
+    if (tid < 64) s_bias[tid] = wrb;
+  };
+  // the gradients of a finished segment: accumulator lane = input of the layer (its ones lane: the bias), column = output
+  const float inv = 1.f / scale;
+  bool bad = false;
+  auto emit = [&](const VjpItem& it) {
+    const VjpOut o = vjp_row(out, partial, it);
+    uint32_t acc[32];
+    auto put = [&](float* p, uint32_t v) {
+      const float g = __uint_as_float(v) * inv;
+      bad |= !(fabsf(g) <= 3.4028235e38f);
+      *p = g;
+    };
+    if (warp < 3) {
+      tmem_ld32(trow + kVtG1, acc);
+      if (tid < 72) {
+#pragma unroll
+        for (int h = 0; h < 32; ++h) put(o.W1 + h * 72 + tid, acc[h]);
+      } else if (tid == 72) {
+#pragma unroll
+        for (int h = 0; h < 32; ++h) put(o.b1 + h, acc[h]);
+      }
+    }
+    if (warp < 2) {
+      tmem_ld32(trow + kVtG2, acc);
+      if (tid < 32) {
+#pragma unroll
+        for (int q = 0; q < 32; ++q) put(o.W2 + q * 32 + tid, acc[q]);
+      } else if (tid == 32) {
+#pragma unroll
+        for (int q = 0; q < 32; ++q) put(o.b2 + q, acc[q]);
+      }
+    }
+    if (warp == 1 || warp == 2) {      // the H2 rows of the window follow H1's four chunks and its ones
+      uint32_t o3[4];
+      tmem_ld4(trow + kVtG2 + 32, o3);
+      if (tid >= 40 && tid < 72) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) put(o.W3 + c * 32 + tid - 40, o3[c]);
+      } else if (tid == 72) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) put(o.b3 + c, o3[c]);
+      }
+    }
+  };
+
+  VjpItem it = load_item(items + idx), it_n = it, it_p = it;
+  const int stride = (int)gridDim.x;
+  bool has_n = idx + stride < G;
+  if (has_n) it_n = load_item(items + idx + stride);
+  load_weights(it.prim);
+  load_rec(it, 0);
+  int sub = 0;
+  bool ok = true, pending = false, finished = false;      // gradient MMAs in flight; they complete segment it_p
+
+  for (;;) {
     // ---- encoding (index c * 6 + f holds sin, 36 + c * 6 + f holds cos: scannet/cumodel.py:183-195) and D3,
     //      into registers while the previous block's gradient MMAs finish ----
+    const bool valid = sub + tid < it.rows;
     uint32_t ew[36];                                            // 32-bit word = two consecutive encoding entries
 #pragma unroll
     for (int c = 0; c < 6; ++c) {
-      float sn[6], cs[6];
-      const float v = valid ? __ldg(x6 + r * 6 + c) : 0.f;
-#pragma unroll
-      for (int f = 0; f < 6; ++f) {
-        if (valid) __sincosf(v * mult[f], &sn[f], &cs[f]);
-        else { sn[f] = 0.f; cs[f] = 0.f; }
-      }
 #pragma unroll
       for (int g = 0; g < 3; ++g) {
-        ew[3 * c + g] = pack_h2<BF16>(sn[2 * g], sn[2 * g + 1]);
-        ew[18 + 3 * c + g] = pack_h2<BF16>(cs[2 * g], cs[2 * g + 1]);
+        float s0, c0, s1, c1;
+        __sincosf(rx[c] * mult[2 * g], &s0, &c0);
+        __sincosf(rx[c] * mult[2 * g + 1], &s1, &c1);
+        ew[3 * c + g] = valid ? pack_h2<BF16>(s0, s1) : 0u;
+        ew[18 + 3 * c + g] = valid ? pack_h2<BF16>(c0, c1) : 0u;
       }
     }
-    float4 g4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (valid) {
-      g4 = __ldg(reinterpret_cast<const float4*>(d4) + r);
-      if (masks) { m1 = (uint32_t)__ldg(masks + r * 2); m2 = (uint32_t)__ldg(masks + r * 2 + 1); }
-    }
-    if (grads_pending) {
+    const uint32_t d01 = pack_h2<BF16>(rg.x * scale, rg.y * scale), d23 = pack_h2<BF16>(rg.z * scale, rg.w * scale);
+    uint32_t m1 = rm1, m2 = rm2;
+    if (pending) {
       ok = wait_phase();
-      grads_pending = false;
       if (!ok) break;
+      if (finished) emit(it_p);
     }
+    if (sub == 0) store_weights();
 #pragma unroll
     for (int kc = 0; kc < 9; ++kc)
       *reinterpret_cast<uint4*>(my + (kVcE + kc) * kVjpChunk) = make_uint4(ew[4 * kc], ew[4 * kc + 1], ew[4 * kc + 2], ew[4 * kc + 3]);
-    *reinterpret_cast<uint4*>(my + kVcD3 * kVjpChunk) =
-        make_uint4(pack_h2<BF16>(g4.x * scale, g4.y * scale), pack_h2<BF16>(g4.z * scale, g4.w * scale), 0u, 0u);
-    // ---- layer 1: K = 80 (the ones behind E meet the zero chunk of W1) ----
-    ok = round_trip([&]() {
-      const uint64_t a = a_rows(kVcE), b = b_w(kVoW1);
-#pragma unroll
-      for (int ks = 0; ks < 5; ++ks) mma_f16(tmem, adv(a, ks * 2 * kVjpChunk), adv(b, ks * 2 * 512), idesc_h, ks > 0);
-    });
-    if (!ok) break;
-    {
-      uint32_t acc[32];
-      tmem_ld32(trow, acc);
-      uint32_t sign = 0u;
-#pragma unroll
-      for (int kc = 0; kc < 4; ++kc) {
-        uint32_t w[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int j = kc * 8 + q * 2;
-          const float v0 = __uint_as_float(acc[j]) + s_b1[j], v1 = __uint_as_float(acc[j + 1]) + s_b1[j + 1];
-          sign |= (v0 > 0.f ? 1u : 0u) << j;
-          sign |= (v1 > 0.f ? 1u : 0u) << (j + 1);
-          w[q] = pack_h2_relu<BF16>(v0, v1);
-        }
-        *reinterpret_cast<uint4*>(my + (kVcH1 + kc) * kVjpChunk) = make_uint4(w[0], w[1], w[2], w[3]);
-      }
-      if (!masks) m1 = sign;
+    *reinterpret_cast<uint4*>(my + kVcD3 * kVjpChunk) = make_uint4(d01, d23, 0u, 0u);
+    if (MASKS) {
+      if (sub == 0) __syncthreads();                            // W3 of the new primitive
+      vjp_d2<BF16>(d01, d23, m2, reinterpret_cast<const float4*>(s_w3), my + kVcD2 * kVjpChunk);
     }
-    // ---- layer 2 ----
-    ok = round_trip([&]() {
-      const uint64_t a = a_rows(kVcH1), b = b_w(kVoW2);
-#pragma unroll
-      for (int ks = 0; ks < 2; ++ks) mma_f16(tmem, adv(a, ks * 2 * kVjpChunk), adv(b, ks * 2 * 512), idesc_h, ks > 0);
-    });
-    if (!ok) break;
-    {
-      uint32_t acc[32];
-      tmem_ld32(trow, acc);
-      uint32_t sign = 0u;
-#pragma unroll
-      for (int kc = 0; kc < 4; ++kc) {
-        uint32_t w[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int j = kc * 8 + q * 2;
-          const float v0 = __uint_as_float(acc[j]) + s_b2[j], v1 = __uint_as_float(acc[j + 1]) + s_b2[j + 1];
-          sign |= (v0 > 0.f ? 1u : 0u) << j;
-          sign |= (v1 > 0.f ? 1u : 0u) << (j + 1);
-          w[q] = pack_h2_relu<BF16>(v0, v1);
-        }
-        *reinterpret_cast<uint4*>(my + (kVcH2 + kc) * kVjpChunk) = make_uint4(w[0], w[1], w[2], w[3]);
-      }
-      if (!masks) m2 = sign;
-    }
-    // ---- D2 = (D3 W3) * mask2: K = 16 ----
-    ok = round_trip([&]() { mma_f16(tmem, a_rows(kVcD3), b_w(kVoW3T), idesc_h, 0u); });
-    if (!ok) break;
-    {
-      uint32_t acc[32];
-      tmem_ld32(trow, acc);
-#pragma unroll
-      for (int kc = 0; kc < 4; ++kc) {
-        uint32_t w[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int j = kc * 8 + q * 2;
-          const float v0 = ((m2 >> j) & 1u) ? __uint_as_float(acc[j]) : 0.f;
-          const float v1 = ((m2 >> (j + 1)) & 1u) ? __uint_as_float(acc[j + 1]) : 0.f;
-          w[q] = pack_h2<BF16>(v0, v1);
-        }
-        *reinterpret_cast<uint4*>(my + (kVcD2 + kc) * kVjpChunk) = make_uint4(w[0], w[1], w[2], w[3]);
-      }
-    }
-    // ---- D1 = (D2 W2) * mask1: K = 32 ----
-    ok = round_trip([&]() {
-      const uint64_t a = a_rows(kVcD2), b = b_w(kVoW2T);
-#pragma unroll
-      for (int ks = 0; ks < 2; ++ks) mma_f16(tmem, adv(a, ks * 2 * kVjpChunk), adv(b, ks * 2 * 512), idesc_h, ks > 0);
-    });
-    if (!ok) break;
-    {
-      uint32_t acc[32];
-      tmem_ld32(trow, acc);
-#pragma unroll
-      for (int kc = 0; kc < 4; ++kc) {
-        uint32_t w[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int j = kc * 8 + q * 2;
-          const float v0 = ((m1 >> j) & 1u) ? __uint_as_float(acc[j]) : 0.f;
-          const float v1 = ((m1 >> (j + 1)) & 1u) ? __uint_as_float(acc[j + 1]) : 0.f;
-          w[q] = pack_h2<BF16>(v0, v1);
-        }
-        *reinterpret_cast<uint4*>(my + (kVcD1 + kc) * kVjpChunk) = make_uint4(w[0], w[1], w[2], w[3]);
-      }
-    }
-    // ---- gradients: contraction over the block's 128 records, 16 per MMA ----
-    const uint32_t keep = sub > 0 ? 1u : 0u;
+    // ---- layer 1: K = 80 (the ones behind E meet the zero chunk of W1); with masks the first half of D1 ----
     issue_phase([&]() {
-      const uint64_t e = mn(kVcE), h1 = mn(kVcH1), h2 = mn(kVcH2), d1 = mn(kVcD1), d2 = mn(kVcD2), d3 = mn(kVcD3);
+      const uint64_t a = a_rows(kVcE);
 #pragma unroll
-      for (int ks = 0; ks < kVjpRows / 16; ++ks) {
-        const uint32_t acc = (keep || ks > 0) ? 1u : 0u;
-        mma_f16(tmem + 32, adv(e, ks * 256), adv(d1, ks * 256), idesc_g32, acc);
-        mma_f16(tmem + 64, adv(h1, ks * 256), adv(d2, ks * 256), idesc_g32, acc);
-        mma_f16(tmem + 96, adv(h2, ks * 256), adv(d3, ks * 256), idesc_g16, acc);
+      for (int ks = 0; ks < 5; ++ks) mma_f16(tmem, adv(a, ks * 2 * kVjpChunk), adv(w1_desc, ks * 2 * 512), idesc_h, ks > 0);
+      if (MASKS) {
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) mma_f16(tmem + kVtD1, adv(a_rows(kVcD2), ks * 2 * kVjpChunk), adv(w2t_desc, ks * 256), idesc_d1h, ks > 0);
       }
     });
-    grads_pending = true;
-  }
-  if (ok && grads_pending) ok = wait_phase();
-
-  if (ok) {
-    float* out = partial + (size_t)seg * 3524;
-    const float inv = 1.f / scale;
-    uint32_t acc[32];
-    tmem_ld32(trow + 32, acc);                       // lane j of dW1^T: dW1[h][j] for the 32 h; lane 72: db1
-    if (tid < 72) {
-#pragma unroll
-      for (int h = 0; h < 32; ++h) out[h * 72 + tid] = __uint_as_float(acc[h]) * inv;
-    } else if (tid == 72) {
-#pragma unroll
-      for (int h = 0; h < 32; ++h) out[kVOb1 + h] = __uint_as_float(acc[h]) * inv;
+    // ---- the next step's loads, in flight from here on ----
+    const int cnt = min(kVjpRows, it.rows - sub);
+    const bool last = sub + kVjpRows >= it.rows;
+    const VjpItem it_c = it;
+    const int sub_c = sub;
+    bool more = true;
+    if (!last) {
+      sub += kVjpRows;
+      load_rec(it, sub);
+    } else if (has_n) {
+      it = it_n;
+      sub = 0;
+      idx += stride;
+      load_rec(it, 0);
+      load_weights(it.prim);
+      has_n = idx + stride < G;
+      if (has_n) it_n = load_item(items + idx + stride);
+    } else {
+      more = false;
     }
-    if (warp < 2) {                                  // lanes 0..31: dW2[q][h = lane], dW3[c][h = lane]; lane 32: db2, db3
-      tmem_ld32(trow + 64, acc);
-      uint32_t o3[4];
-      tmem_ld4(trow + 96, o3);
-      if (tid < 32) {
+    ok = wait_phase();
+    if (!ok) break;
+    {
+      uint32_t acc[32];
+      tmem_ld32(trow, acc);
+      const uint32_t sign = vjp_hidden<BF16>(acc, s_bias, my + kVcH1 * kVjpChunk);
+      if (!MASKS) m1 = sign;
+    }
+    if (MASKS) {
+      uint32_t acc[16];
+      tmem_ld16(trow + kVtD1, acc);
+      vjp_adjoint<BF16, 16>(acc, m1, my + kVcD1 * kVjpChunk);
+    }
+    // ---- layer 2; with masks the second half of D1 ----
+    issue_phase([&]() {
+      const uint64_t a = a_rows(kVcH1);
 #pragma unroll
-        for (int q = 0; q < 32; ++q) out[kVOW2 + q * 32 + tid] = __uint_as_float(acc[q]) * inv;
+      for (int ks = 0; ks < 2; ++ks) mma_f16(tmem, adv(a, ks * 2 * kVjpChunk), adv(w2_desc, ks * 2 * 512), idesc_h, ks > 0);
+      if (MASKS) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) out[kVOW3 + c * 32 + tid] = __uint_as_float(o3[c]) * inv;
-      } else if (tid == 32) {
-#pragma unroll
-        for (int q = 0; q < 32; ++q) out[kVOb2 + q] = __uint_as_float(acc[q]) * inv;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) out[kVOb3 + c] = __uint_as_float(o3[c]) * inv;
+        for (int ks = 0; ks < 2; ++ks)
+          mma_f16(tmem + kVtD1, adv(a_rows(kVcD2), ks * 2 * kVjpChunk), adv(w2t_desc, 2 * 512 + ks * 256), idesc_d1h, ks > 0);
       }
+    });
+    ok = wait_phase();
+    if (!ok) break;
+    {
+      uint32_t acc[32];
+      tmem_ld32(trow, acc);
+      const uint32_t sign = vjp_hidden<BF16>(acc, s_bias + 32, my + kVcH2 * kVjpChunk);
+      if (!MASKS) m2 = sign;
     }
-  } else if (tid == 0) {
-    atomicOr(flag, 2);
+    if (MASKS) {
+      uint32_t acc[16];
+      tmem_ld16(trow + kVtD1, acc);
+      vjp_adjoint<BF16, 16>(acc, m1 >> 16, my + (kVcD1 + 2) * kVjpChunk);
+    } else {
+      vjp_d2<BF16>(d01, d23, m2, reinterpret_cast<const float4*>(s_w3), my + kVcD2 * kVjpChunk);
+      issue_phase([&]() {
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) mma_f16(tmem, adv(a_rows(kVcD2), ks * 2 * kVjpChunk), adv(w2t_desc, ks * 256), idesc_d1, ks > 0);
+      });
+      ok = wait_phase();
+      if (!ok) break;
+      uint32_t acc[32];
+      tmem_ld32(trow, acc);
+      vjp_adjoint<BF16, 32>(acc, m1, my + kVcD1 * kVjpChunk);
+    }
+    // ---- gradients: contraction over the block's records, 16 per MMA ----
+    issue_phase([&]() {
+      const uint64_t e = mn(kVcE), h = mn(kVcH1), d1 = mn(kVcD1), d23t = mn(kVcD2);
+      const int steps = (cnt + 15) >> 4;
+      for (int ks = 0; ks < steps; ++ks) {
+        const uint32_t acc = (sub_c > 0 || ks > 0) ? 1u : 0u;
+        mma_f16(tmem + kVtG1, adv(e, ks * 256), adv(d1, ks * 256), idesc_g1, acc);
+        mma_f16(tmem + kVtG2, adv(h, ks * 256), adv(d23t, ks * 256), idesc_g2, acc);
+      }
+    });
+    pending = true;
+    finished = last;
+    it_p = it_c;
+    if (!more) break;
   }
+  if (ok) {
+    ok = wait_phase();
+    if (ok) emit(it_p);
+  }
+  if (bad) atomicOr(counters + kVpFlag, 1);
+  if (!ok && tid == 0) atomicOr(counters + kVpFlag, 2);
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_free(tmem, kVjpTmemCols);
 }
 
-int launch_grouped_vjp_tc(bool bf16, const float* x6, const float* d4, const int32_t* masks, const int64_t* offsets,
-                          const int64_t* seg_prim, const int64_t* seg_start, int64_t num_segments, int segment_size,
-                          const mlpsp_scene* sc, float scale, float* partial, int32_t* flag, cudaStream_t st) {
+int launch_grouped_vjp_tc(bool bf16, const float* x6, const float* d4, const int32_t* masks, const VjpItem* items,
+                          int64_t max_items, int32_t* counters, const mlpsp_scene* sc, float scale, const VjpOut& out,
+                          float* partial, cudaStream_t st) {
   static DeviceOnce attr_once;
   if (attr_once.first()) {
-    MLPSP_CUDA_OK(cudaFuncSetAttribute(k_grouped_vjp_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kVjpSmem));
-    MLPSP_CUDA_OK(cudaFuncSetAttribute(k_grouped_vjp_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kVjpSmem));
+    MLPSP_CUDA_OK(cudaFuncSetAttribute(k_grouped_vjp_tc<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kVjpSmem));
+    MLPSP_CUDA_OK(cudaFuncSetAttribute(k_grouped_vjp_tc<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kVjpSmem));
+    MLPSP_CUDA_OK(cudaFuncSetAttribute(k_grouped_vjp_tc<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kVjpSmem));
+    MLPSP_CUDA_OK(cudaFuncSetAttribute(k_grouped_vjp_tc<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kVjpSmem));
   }
-  if (bf16)
-    k_grouped_vjp_tc<true><<<(unsigned)num_segments, kVjpRows, kVjpSmem, st>>>(x6, d4, masks, offsets, seg_prim, seg_start, segment_size,
-                                                                             sc->freq, sc->att, sc->W1, sc->b1, sc->W2, sc->b2,
-                                                                             sc->W3, scale, partial, flag);
-  else
-    k_grouped_vjp_tc<false><<<(unsigned)num_segments, kVjpRows, kVjpSmem, st>>>(x6, d4, masks, offsets, seg_prim, seg_start, segment_size,
-                                                                              sc->freq, sc->att, sc->W1, sc->b1, sc->W2, sc->b2,
-                                                                              sc->W3, scale, partial, flag);
-  return cuda_check(cudaGetLastError(), "grouped_vjp_tc");
+  auto* kernel = bf16 ? (masks ? k_grouped_vjp_tc<true, true> : k_grouped_vjp_tc<true, false>)
+                      : (masks ? k_grouped_vjp_tc<false, true> : k_grouped_vjp_tc<false, false>);
+  const int vec = ((reinterpret_cast<uintptr_t>(sc->W1) | reinterpret_cast<uintptr_t>(sc->W2)) & 15) == 0 &&
+                  (reinterpret_cast<uintptr_t>(x6) & 7) == 0;
+  const int grid = (int)std::min<int64_t>(max_items, (int64_t)sm_count() * kVjpCtas);
+  return cuda_check(launch_chained(kernel, dim3(grid), dim3(kVjpRows), kVjpSmem, st, x6, d4, masks, items, counters, sc->freq, sc->att,
+                                   sc->W1, sc->b1, sc->W2, sc->b2, sc->W3, vec, scale, out, partial),
+                    "grouped_vjp_tc");
 }
 
 }  // namespace mlpsp

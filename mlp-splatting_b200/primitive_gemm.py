@@ -46,7 +46,7 @@ class GroupLayout:
         return self
 
 
-def prepare_groups(csr, segment_size=512):
+def _check_group_inputs(csr, segment_size):
     if not isinstance(segment_size, int) or isinstance(segment_size, bool) or segment_size <= 0:
         raise ValueError("segment_size must be a positive integer")
     if csr.offsets.ndim != 1 or csr.offsets.dtype != torch.int64 or not csr.offsets.is_contiguous():
@@ -55,6 +55,10 @@ def prepare_groups(csr, segment_size=512):
         raise ValueError("CSR offsets must include the initial zero")
     if not csr.offsets.is_cuda:
         raise RuntimeError("prepare_groups runs on a CUDA device; there is no CPU path")
+
+
+def prepare_groups(csr, segment_size=512):
+    _check_group_inputs(csr, segment_size)
     lib = L.load()
     dev = csr.offsets.device
     n = int(csr.offsets.numel()) - 1
@@ -197,14 +201,19 @@ def grouped_weight_gradients(csr, freq, attenuation, weights, *, dtype=torch.flo
             csr.relu_masks.dtype != torch.int32 or not csr.relu_masks.is_contiguous()
             or csr.relu_masks.device != w1.device or csr.relu_masks.shape != (len(csr.x6), 2)):
         raise ValueError("saved ReLU masks must be contiguous CUDA int32 with shape (records,2)")
-    groups = resolve_groups(csr, segment_size, groups)
+    # the segments follow from the offsets and the segment size: the launch plans them on the device, so a layout the
+    # caller shares between consumers is checked against this CSR and nothing is prepared when there is none
+    if groups is None:
+        _check_group_inputs(csr, segment_size)
+    else:
+        resolve_groups(csr, segment_size, groups)
     scale = float(4096 if dtype == torch.float16 else 1) if loss_scale is None else float(loss_scale)
     if not math.isfinite(scale) or scale <= 0:
         raise ValueError("loss_scale must be finite and strictly positive")
     lib = L.load()
     dev = w1.device
-    glen = int(lib.mlpsp_grouped_gradient_floats())
-    G = int(groups.primitives.numel())
+    R = len(csr.x6)
+    nbytes = int(lib.mlpsp_weight_gradients_scratch_bytes(R, n, int(segment_size)))
     sc = L.Scene()
     sc.n, sc.hidden, sc.num_freq = n, 32, 6
     sc.W1, sc.b1, sc.W2, sc.b2, sc.W3, sc.b3 = (L.ptr(t) for t in weights)
@@ -213,21 +222,17 @@ def grouped_weight_gradients(csr, freq, attenuation, weights, *, dtype=torch.flo
 
     def launch(operand_dtype, operand_scale):
         """One unguarded launch, shared by the normal path and the FP32 retry (primitive_gemm.py:215-232)."""
-        partial = torch.empty((max(G, 1), glen), device=dev, dtype=torch.float32)
-        result = torch.empty((n, glen), device=dev, dtype=torch.float32)
-        nonfinite = torch.zeros((), device=dev, dtype=torch.int32)
+        grads = [torch.empty_like(w) for w in weights]
+        scratch = torch.empty(nbytes, device=dev, dtype=torch.uint8)
+        word = C.c_int32(0)
         with torch.cuda.device(dev):
             st = C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
-            L.check(lib.mlpsp_grouped_weight_gradients(
-                C.byref(sc), L.ptr(csr.offsets), L.ptr(csr.x6), L.ptr(csr.grad4), L.ptr(csr.relu_masks),
-                L.ptr(groups.primitives), L.ptr(groups.starts), L.ptr(groups.offsets), G, int(segment_size),
-                precisions[operand_dtype], float(operand_scale), L.ptr(partial), L.ptr(result), L.ptr(nonfinite), st),
-                "mlpsp_grouped_weight_gradients")
-        word = int(nonfinite.item())
-        if word & 2:
+            L.check(lib.mlpsp_weight_gradients(
+                C.byref(sc), L.ptr(csr.offsets), L.ptr(csr.x6), L.ptr(csr.grad4), L.ptr(csr.relu_masks), R, int(segment_size),
+                precisions[operand_dtype], float(operand_scale), *(L.ptr(g) for g in grads), L.ptr(scratch), nbytes,
+                C.byref(word), st), "mlpsp_weight_gradients")
+        if word.value & 2:
             raise RuntimeError("grouped_weight_gradients: a device-side wait gave up; results discarded")
-        return result, bool(word & 1)
+        return grads, bool(word.value & 1)
 
-    result = _checked_grouped_vjp(launch, dtype, scale)
-    sizes = [2304, 32, 1024, 32, 128, 4]
-    return [v.reshape(w.shape).contiguous() for v, w in zip(result.split(sizes, dim=1), weights)]
+    return _checked_grouped_vjp(launch, dtype, scale)
