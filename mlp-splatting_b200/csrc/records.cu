@@ -26,6 +26,8 @@ constexpr int kWinMax = 2048;
 
 // squared bounding radius in units of the largest scale, with the 2 % margin surely_misses() relies on
 static inline float miss_bound2(float thr) { return (float)(-2.0 * log((double)thr) * 1.02); }
+// threshold of the quadratic form, -2 ln thr; 0 (no form) where decay could underflow before it reaches thr
+static inline float form_threshold(float thr) { const double k = -2.0 * log((double)thr); return k > 0.0 && k < 170.0 ? (float)k : 0.f; }
 
 // -------------------------------------------------------------------------- frame init ----
 // One launch prepares a frame: pixel state and the output image, the list of live tiles and the wave counters,
@@ -59,107 +61,298 @@ __global__ void k_init_frame(int64_t P, float4* __restrict__ px_state, float2* _
 }
 
 // --------------------------------------------------------------------------- hit pass ----
-// 8 warps per tile: warp w owns pixel half (w & 1) and candidates (w >> 1) + 4j of the window.
-// REF: the hit decision in the reference kernels' arithmetic (frame.hit_arith = 1).
+// The exact decision (hit_test) costs about 130 FP32 operations per pixel and candidate.  Almost every decision is far
+// from the threshold, and for a candidate and the rays of one tile, which leave one origin, it is the sign of a quadratic
+// form: with the rays as a + alpha u + beta v up to scale (an orthonormal frame of the tile) and x, e the primitive-frame
+// offset and direction divided by its scales, decay > thr <=> |x cross e|^2 < K |e|^2 with K = -2 ln thr -- six
+// coefficients per (tile, candidate), computed by one lane, and five multiply-adds per pixel.  The pixel's value decides
+// when it is further from zero than the candidate's tolerance; the few pixels in between are decided by hit_test itself,
+// so every decision is hit_test's.
+//
+// Tolerance, relative to |e|^2 (u = 2^-24, S = |c - o| + |o|, im = largest inverse scale): building x and e from rounded
+// matrices costs |x cross e| at most 45 u S im |e| (frame and ray rounding included), hence the form 90 u sqrt(K) S im =
+// 5.4e-6 sqrt(K) S im near the threshold; hit_test's own foot point p = o + t d is off by u S per axis, 6 u sqrt(K) S im;
+// its relative errors (r^2, the exponential, the rounded threshold) stay below 20 u K, and those of |e| below
+// 12 u K im / |e|; evaluating the polynomial adds 10 u times the sum M of its terms' magnitudes.  The constants below are
+// above the sum of these.  t > 0 is decided for the whole tile from x . e with a margin of 1e-3 |x||e| (rounding is below
+// 10 u im (|c - o||e| + |x|)); a candidate that is neither surely in front nor surely behind, or not finite, is left to
+// hit_test altogether.
+struct RayFrame {
+  V3 o, a, u, v;           // common origin and frame
+  float A, B;              // largest |alpha|, |beta| of the tile
+  bool fast;               // the tile has such a frame
+};
+
+__device__ __forceinline__ void hit_form(const Geom& g, const RayFrame& f, float K, float4& q0, float4& q1) {
+  const float kAll = __int_as_float(0x7f800000);
+  const PrimWhiten pw = make_whiten(g);
+  const float vx = g.cx - f.o.x, vy = g.cy - f.o.y, vz = g.cz - f.o.z;
+  const V3 x = whiten(pw, vx, vy, vz);
+  const V3 e0 = whiten(pw, f.a.x, f.a.y, f.a.z), e1 = whiten(pw, f.u.x, f.u.y, f.u.z), e2 = whiten(pw, f.v.x, f.v.y, f.v.z);
+  const V3 w0 = {x.y * e0.z - x.z * e0.y, x.z * e0.x - x.x * e0.z, x.x * e0.y - x.y * e0.x};
+  const V3 w1 = {x.y * e1.z - x.z * e1.y, x.z * e1.x - x.x * e1.z, x.x * e1.y - x.y * e1.x};
+  const V3 w2 = {x.y * e2.z - x.z * e2.y, x.z * e2.x - x.x * e2.z, x.x * e2.y - x.y * e2.x};
+  auto dot = [](const V3& p, const V3& q) { return p.x * q.x + p.y * q.y + p.z * q.z; };
+  const float e00 = dot(e0, e0), e11 = dot(e1, e1), e22 = dot(e2, e2);
+  const float c0 = dot(w0, w0) - K * e00;
+  const float b1 = 2.f * (dot(w0, w1) - K * dot(e0, e1)), b2 = 2.f * (dot(w0, w2) - K * dot(e0, e2));
+  const float a11 = dot(w1, w1) - K * e11, a22 = dot(w2, w2) - K * e22, a12 = 2.f * (dot(w1, w2) - K * dot(e1, e2));
+  const float M = dot(w0, w0) + K * e00 + f.A * (fabsf(b1) + f.A * fabsf(a11) + f.B * fabsf(a12)) + f.B * (fabsf(b2) + f.B * fabsf(a22));
+  const float emax = sqrtf(e00) + f.A * sqrtf(e11) + f.B * sqrtf(e22);
+  const float dist = fabsf(vx) + fabsf(vy) + fabsf(vz), S = dist + fabsf(f.o.x) + fabsf(f.o.y) + fabsf(f.o.z);
+  float tol = ((8e-6f * sqrtf(K) * S * pw.ismax + 1e-4f * K) * emax + 1e-6f * K * pw.ismax) * emax + 1e-6f * M;
+  const float xn = sqrtf(dot(x, x)), mid = dot(x, e0), var = f.A * fabsf(dot(x, e1)) + f.B * fabsf(dot(x, e2));
+  const float margin = 1e-3f * xn * emax + 3e-6f * pw.ismax * (dist * emax + xn);
+  if (!(e00 > 1e-14f) || !(mid - var > margin)) tol = kAll;
+  q0 = make_float4(c0, b1, b2, tol);
+  q1 = make_float4(a11, a12, a22, 0.f);
+  if (mid + var < -margin && e00 > 1e-14f) { q0 = make_float4(1.f, 0.f, 0.f, 0.f); q1 = make_float4(0.f, 0.f, 0.f, 0.f); }   // behind every ray's origin
+  if (!f.fast) q0.w = kAll;
+}
+
+// A warp's view of a tile: lane l owns the pixels l and 32 + l.
+struct HitPixels {
+  RayFrame f;
+  float al[2], be[2];
+  int pix[2];
+  uint32_t act[2];         // live pixels of the two halves
+};
+
+__device__ __forceinline__ HitPixels hit_pixels(const float* __restrict__ rays_o, const float* __restrict__ rays_d,
+                                                const float4* __restrict__ px_state, int tile, int ntx, int W, int H, bool allow) {
+  HitPixels h;
+  const int lane = threadIdx.x & 31;
+  V3 o[2], d[2];
+  bool valid[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const TilePix tp = tile_pixel(tile, k * 32 + lane, ntx, W, H);
+    valid[k] = tp.valid;
+    h.pix[k] = tp.pix;
+    o[k] = d[k] = V3{0.f, 0.f, 0.f};
+    bool live = false;
+    if (tp.valid) {
+      o[k] = load3(rays_o, tp.pix);
+      d[k] = load3(rays_d, tp.pix);
+      live = px_state[tp.pix].w >= MLPSP_TERM;
+    }
+    h.act[k] = __ballot_sync(0xffffffffu, live);
+  }
+  // the frame around one of the central rays (pixel (3, 3), or the tile's first at the image's border)
+  const uint32_t v0 = __ballot_sync(0xffffffffu, valid[0]);
+  const int src = (v0 >> 27) & 1u ? 27 : 0;
+  h.f.o = V3{__shfl_sync(0xffffffffu, o[0].x, src), __shfl_sync(0xffffffffu, o[0].y, src), __shfl_sync(0xffffffffu, o[0].z, src)};
+  h.f.a = V3{__shfl_sync(0xffffffffu, d[0].x, src), __shfl_sync(0xffffffffu, d[0].y, src), __shfl_sync(0xffffffffu, d[0].z, src)};
+  V3 a = h.f.a;
+  const float ra = rsqrtf(a.x * a.x + a.y * a.y + a.z * a.z);
+  a.x *= ra; a.y *= ra; a.z *= ra;
+  V3 u = fabsf(a.x) < 0.6f ? V3{0.f, a.z, -a.y} : V3{-a.z, 0.f, a.x};
+  const float ru = rsqrtf(u.x * u.x + u.y * u.y + u.z * u.z);
+  u.x *= ru; u.y *= ru; u.z *= ru;
+  h.f.a = a; h.f.u = u;
+  h.f.v = V3{a.y * u.z - a.z * u.y, a.z * u.x - a.x * u.z, a.x * u.y - a.y * u.x};
+  bool same = allow;
+  float A = 0.f, B = 0.f;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const float da = d[k].x * a.x + d[k].y * a.y + d[k].z * a.z;
+    const float r = __fdividef(1.f, da);
+    h.al[k] = (d[k].x * u.x + d[k].y * u.y + d[k].z * u.z) * r;
+    h.be[k] = (d[k].x * h.f.v.x + d[k].y * h.f.v.y + d[k].z * h.f.v.z) * r;
+    if (!valid[k]) { h.al[k] = h.be[k] = 0.f; continue; }
+    const float dd = d[k].x * d[k].x + d[k].y * d[k].y + d[k].z * d[k].z;
+    same = same && o[k].x == h.f.o.x && o[k].y == h.f.o.y && o[k].z == h.f.o.z && da > 0.7f && dd < 1.01f;
+    A = fmaxf(A, fabsf(h.al[k])); B = fmaxf(B, fabsf(h.be[k]));
+  }
+  h.f.fast = __all_sync(0xffffffffu, same);
+  h.f.A = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(A)));
+  h.f.B = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(B)));
+  return h;
+}
+
 template <bool REF>
-__global__ void __launch_bounds__(256, 6) k_hits(
-    const float* __restrict__ rays_o, const float* __restrict__ rays_d, const float4* __restrict__ geom, int n,
-    const int32_t* __restrict__ tile_offsets, const int32_t* __restrict__ tile_len, const int32_t* __restrict__ sorted_prims, int W, int H, int ntx,
-    float thr, float bound2, const int32_t* __restrict__ active, const int32_t* __restrict__ active_count, int lo,
-    int hi, const float4* __restrict__ px_state, uint32_t* __restrict__ masks32, uint32_t* __restrict__ pair_base,
-    int32_t* __restrict__ prim_cnt, int32_t* __restrict__ counters, int64_t max_records,
-    int32_t* __restrict__ status, int32_t* __restrict__ reset_count) {
+__device__ __noinline__ bool hit_exact(const float* __restrict__ rays_o, const float* __restrict__ rays_d, const float4* __restrict__ geom,
+                                       int p, int pix, float thr, float bound2) {
+  const V3 o = load3(rays_o, pix), d = load3(rays_d, pix);
+  const Geom g = load_geom(geom, p);
+  if (surely_misses(g, o, d, bound2)) return false;
+  Hit h;
+  return REF ? hit_test_ref(load_geom_ref(geom, p), o, d, thr, h) : hit_test(g, o, d, thr, h);
+}
+
+// Hit masks (m0, m1: the tile's two pixel halves) of the candidate ids p_lane of a chunk of cnt <= 32 candidates, lane l
+// holding the l-th; s_q: the warp's 64 float4 of shared memory.
+template <bool REF>
+__device__ __forceinline__ void hit_chunk(const HitPixels& h, const float* __restrict__ rays_o, const float* __restrict__ rays_d,
+                                          const float4* __restrict__ geom, int n, int p_lane, int cnt, float K, float thr,
+                                          float bound2, float4* s_q, uint32_t& m0, uint32_t& m1) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+  if (lane < cnt) {
+    float4 q0 = make_float4(1.f, 0.f, 0.f, 0.f), q1 = make_float4(0.f, 0.f, 0.f, 0.f);     // misses
+    if (p_lane >= 0 && p_lane < n) hit_form(load_geom(geom, p_lane), h.f, K, q0, q1);
+    s_q[2 * lane] = q0;
+    s_q[2 * lane + 1] = q1;
+  }
+  __syncwarp();
+  m0 = m1 = 0u;
+  const bool live0 = (h.act[0] >> lane) & 1u, live1 = (h.act[1] >> lane) & 1u;
+#pragma unroll 2
+  for (int t = 0; t < cnt; ++t) {
+    const float4 q0 = s_q[2 * t], q1 = s_q[2 * t + 1];
+    const float f0 = fmaf(fmaf(q1.x, h.al[0], fmaf(q1.y, h.be[0], q0.y)), h.al[0], fmaf(fmaf(q1.z, h.be[0], q0.z), h.be[0], q0.x));
+    const float f1 = fmaf(fmaf(q1.x, h.al[1], fmaf(q1.y, h.be[1], q0.y)), h.al[1], fmaf(fmaf(q1.z, h.be[1], q0.z), h.be[1], q0.x));
+    bool hit0 = f0 < -q0.w, hit1 = f1 < -q0.w;
+    const bool amb0 = live0 && !(fabsf(f0) > q0.w), amb1 = live1 && !(fabsf(f1) > q0.w);
+    if (__any_sync(0xffffffffu, amb0 || amb1)) {
+      const int p = __shfl_sync(0xffffffffu, p_lane, t);
+      if (amb0) hit0 = hit_exact<REF>(rays_o, rays_d, geom, p, h.pix[0], thr, bound2);
+      if (amb1) hit1 = hit_exact<REF>(rays_o, rays_d, geom, p, h.pix[1], thr, bound2);
+    }
+    const uint32_t b0 = __ballot_sync(0xffffffffu, hit0) & h.act[0], b1 = __ballot_sync(0xffffffffu, hit1) & h.act[1];
+    if (lane == t) { m0 = b0; m1 = b1; }
+  }
+}
+
+struct HitArgs {
+  const float* rays_o; const float* rays_d; const float4* geom; int n;
+  const int32_t* tile_offsets; const int32_t* tile_len; const int32_t* sorted_prims; int W, H, ntx;
+  float thr, bound2, K;            // K <= 0: no quadratic form (thresholds the exponential underflows at)
+  const int32_t* active; const int32_t* active_count; int lo, hi;
+  const float4* px_state; uint2* masks; uint32_t* pair_base; int32_t* prim_cnt; int32_t* counters; int64_t max_records;
+  int32_t* status; int32_t* reset_count;
+};
+
+__device__ __forceinline__ int warp_inclusive_scan(int v) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += u;
+  }
+  return v;
+}
+
+// Windows of up to 32 CH candidates: one warp per tile, nothing shared between warps.
+constexpr int kHitWarps = 4;
+template <bool REF, int CH>
+__global__ void __launch_bounds__(32 * kHitWarps) k_hits_warp(const HitArgs a) {
   chain_wait();
   chain_release();
-  __shared__ uint32_t s_m[2][kWinMax];
-  __shared__ int32_t s_pref[kWinMax];
-  __shared__ int warp_sums[32];
-  __shared__ int s_tile_base;
-  if (status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
+  __shared__ float4 s_q[kHitWarps][64];
+  if (a.status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
   // a view of a batch clears the count of the list its compositing pass of this wave will append to (the
   // per-primitive scan does that for a frame rendered alone)
-  if (reset_count && blockIdx.x == 0 && threadIdx.x == 0) *reset_count = 0;
-  const int n_active = *active_count;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int half = warp & 1;
-  for (int slot_i = blockIdx.x; slot_i < n_active; slot_i += gridDim.x) {
-  const int tile = active[slot_i];
-  const int s = tile_offsets[tile];
-  const int len = tile_len[tile];
-  const int wlo = min(lo, len), whi = min(hi, len);
-  const int nwin = whi - wlo;
-  if (nwin <= 0) continue;
-  const TilePix tp = tile_pixel(tile, half * 32 + lane, ntx, W, H);
-  V3 o = {0.f, 0.f, 0.f}, d = {0.f, 0.f, 0.f};
-  bool act = false;
-  if (tp.valid) {
-    o = load3(rays_o, tp.pix); d = load3(rays_d, tp.pix);
-    act = px_state[tp.pix].w >= MLPSP_TERM;
-  }
-  // The 32 rays of this warp normally leave one origin; then R^T (c - o) is a per-candidate constant, computed by
-  // one lane per candidate for a batch of 32 candidates and handed round by shuffles (same operations on the
-  // same inputs: same bits as computing it in every lane).
-  const uint32_t vmask = __ballot_sync(0xffffffffu, tp.valid);
-  V3 o0 = o;
-  bool uni = false;
-  if (vmask) {
-    const int src = __ffs(vmask) - 1;
-    o0.x = __shfl_sync(0xffffffffu, o.x, src); o0.y = __shfl_sync(0xffffffffu, o.y, src); o0.z = __shfl_sync(0xffffffffu, o.z, src);
-    uni = __all_sync(0xffffffffu, !tp.valid || (o.x == o0.x && o.y == o0.y && o.z == o0.z));
-  }
-  for (int b0 = wlo + (warp >> 1); b0 < whi; b0 += 128) {
-    const int il = b0 + 4 * lane;
-    int pl = -1;
-    V3 vll = {0.f, 0.f, 0.f};
-    if (il < whi) {
-      pl = sorted_prims[s + il];
-      if (!REF && uni && pl >= 0 && pl < n) vll = local_offset(load_geom(geom, pl), o0);
-    }
-    const int cnt = min(32, (whi - b0 + 3) >> 2);
-    for (int t = 0; t < cnt; ++t) {
-      const int i = b0 + 4 * t;
-      const int p = __shfl_sync(0xffffffffu, pl, t);
-      const V3 vl = {__shfl_sync(0xffffffffu, vll.x, t), __shfl_sync(0xffffffffu, vll.y, t), __shfl_sync(0xffffffffu, vll.z, t)};
-      bool hit = false;
-      if (act && p >= 0 && p < n) {
-        const Geom g = load_geom(geom, p);
-        if (!surely_misses(g, o, d, bound2)) {
-          Hit h;
-          if (REF) hit = hit_test_ref(load_geom_ref(geom, p), o, d, thr, h);
-          else hit = uni ? hit_test_t<true>(g, o, d, vl, thr, h) : hit_test_t<false>(g, o, d, vl, thr, h);
-        }
+  if (a.reset_count && blockIdx.x == 0 && threadIdx.x == 0) *a.reset_count = 0;
+  const int n_active = *a.active_count;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
+  for (int slot_i = blockIdx.x * wpb + warp; slot_i < n_active; slot_i += gridDim.x * wpb) {
+    const int tile = a.active[slot_i];
+    const int s = a.tile_offsets[tile], len = a.tile_len[tile];
+    const int wlo = min(a.lo, len), nwin = min(a.hi, len) - wlo;
+    if (nwin <= 0) continue;
+    const HitPixels h = hit_pixels(a.rays_o, a.rays_d, a.px_state, tile, a.ntx, a.W, a.H, a.K > 0.f);
+    int p[CH], c[CH], total = 0;
+#pragma unroll
+    for (int ch = 0; ch < CH; ++ch) {
+      const int j = ch * 32 + lane;
+      p[ch] = j < nwin ? a.sorted_prims[s + wlo + j] : -1;
+      c[ch] = 0;
+      if (ch * 32 < nwin) {
+        uint32_t m0, m1;
+        hit_chunk<REF>(h, a.rays_o, a.rays_d, a.geom, a.n, p[ch], min(32, nwin - ch * 32), a.K, a.thr, a.bound2, s_q[warp], m0, m1);
+        if (j < nwin) a.masks[(size_t)(s + wlo) + j] = make_uint2(m0, m1);
+        c[ch] = __popc(m0) + __popc(m1);
+        total += c[ch];
+        if (c[ch] > 0) atomicAdd(a.prim_cnt + p[ch], c[ch]);
       }
-      const uint32_t m = __ballot_sync(0xffffffffu, hit);
-      if (lane == 0) s_m[half][i - wlo] = m;
+    }
+    total = __reduce_add_sync(0xffffffffu, total);
+    int base = 0;
+    if (lane == 0 && total > 0) {
+      base = atomicAdd(a.counters + kCtrRecords, total);
+      if ((int64_t)base + total > a.max_records) atomicOr(a.status + MLPSP_ST_BITS, MLPSP_ST_RECORD_OVERFLOW);
+    }
+    base = __shfl_sync(0xffffffffu, base, 0);
+#pragma unroll
+    for (int ch = 0; ch < CH; ++ch) {
+      if (ch * 32 < nwin) {
+        const int inc = warp_inclusive_scan(c[ch]);
+        if (ch * 32 + lane < nwin) a.pair_base[(size_t)(s + wlo) + ch * 32 + lane] = (uint32_t)(base + inc - c[ch]);
+        base += __shfl_sync(0xffffffffu, inc, 31);
+      }
     }
   }
-  __syncthreads();
-  int running = 0;
-  for (int j0 = 0; j0 < nwin; j0 += 256) {
-    const int j = j0 + tid;
-    const int c = (j < nwin) ? __popc(s_m[0][j]) + __popc(s_m[1][j]) : 0;
-    int total;
-    const int ex = block_exclusive_scan(c, warp_sums, total);
-    if (j < nwin) s_pref[j] = running + ex;
-    running += total;
+}
+
+// Wider windows: eight warps per tile, each takes every eighth chunk of 32 candidates.
+template <bool REF>
+__global__ void __launch_bounds__(256) k_hits(const HitArgs a) {
+  chain_wait();
+  chain_release();
+  __shared__ float4 s_q[8][64];
+  __shared__ uint2 s_m[kWinMax];
+  __shared__ int warp_sums[32];
+  __shared__ int s_tile_base, s_total;
+  if (a.status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
+  if (a.reset_count && blockIdx.x == 0 && threadIdx.x == 0) *a.reset_count = 0;
+  const int n_active = *a.active_count;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int slot_i = blockIdx.x; slot_i < n_active; slot_i += gridDim.x) {
+    const int tile = a.active[slot_i];
+    const int s = a.tile_offsets[tile], len = a.tile_len[tile];
+    const int wlo = min(a.lo, len), nwin = min(a.hi, len) - wlo;
+    if (nwin <= 0) continue;
+    __syncthreads();   // the previous tile's masks have been read
+    if (tid == 0) s_total = 0;
+    const HitPixels h = hit_pixels(a.rays_o, a.rays_d, a.px_state, tile, a.ntx, a.W, a.H, a.K > 0.f);
+    __syncthreads();
+    int mine = 0;
+    for (int j0 = warp * 32; j0 < nwin; j0 += 256) {
+      const int j = j0 + lane;
+      const int p = j < nwin ? a.sorted_prims[s + wlo + j] : -1;
+      uint32_t m0, m1;
+      hit_chunk<REF>(h, a.rays_o, a.rays_d, a.geom, a.n, p, min(32, nwin - j0), a.K, a.thr, a.bound2, s_q[warp], m0, m1);
+      const int c = __popc(m0) + __popc(m1);
+      if (j < nwin) s_m[j] = a.masks[(size_t)(s + wlo) + j] = make_uint2(m0, m1);
+      if (c > 0) atomicAdd(a.prim_cnt + p, c);
+      mine += c;
+    }
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if (lane == 0 && mine) atomicAdd(&s_total, mine);
+    __syncthreads();
+    if (tid == 0) {
+      const int total = s_total;
+      const int base = total > 0 ? atomicAdd(a.counters + kCtrRecords, total) : 0;
+      s_tile_base = base;
+      if ((int64_t)base + total > a.max_records) atomicOr(a.status + MLPSP_ST_BITS, MLPSP_ST_RECORD_OVERFLOW);
+    }
+    __syncthreads();
+    int running = s_tile_base;
+    for (int j0 = 0; j0 < nwin; j0 += 256) {
+      const int j = j0 + tid;
+      const int c = (j < nwin) ? __popc(s_m[j].x) + __popc(s_m[j].y) : 0;
+      int total;
+      const int ex = block_exclusive_scan(c, warp_sums, total);
+      if (j < nwin) a.pair_base[(size_t)(s + wlo) + j] = (uint32_t)(running + ex);
+      running += total;
+    }
   }
-  if (tid == 0) {
-    const int base = running > 0 ? atomicAdd(counters + kCtrRecords, running) : 0;
-    s_tile_base = base;
-    if ((int64_t)base + running > max_records) atomicOr(status + MLPSP_ST_BITS, MLPSP_ST_RECORD_OVERFLOW);
+}
+
+static int launch_hits(const HitArgs& a, bool ref_arith, int tiles, int sms, bool idle_tail, cudaStream_t st) {
+  const int win = a.hi - a.lo;
+  if (win > 128) {
+    const dim3 grid(idle_tail ? sms : std::min(tiles, sms * 8));
+    return cuda_check(ref_arith ? launch_chained(k_hits<true>, grid, dim3(256), 0, st, a) : launch_chained(k_hits<false>, grid, dim3(256), 0, st, a), "hits");
   }
-  __syncthreads();
-  const int base = s_tile_base;
-  for (int j = tid; j < nwin; j += 256) {
-    const uint32_t m0 = s_m[0][j], m1 = s_m[1][j];
-    masks32[2 * (size_t)(s + wlo + j)] = m0;
-    masks32[2 * (size_t)(s + wlo + j) + 1] = m1;
-    pair_base[s + wlo + j] = (uint32_t)(base + s_pref[j]);
-    const int c = __popc(m0) + __popc(m1);
-    if (c > 0) atomicAdd(prim_cnt + sorted_prims[s + wlo + j], c);
-  }
-  __syncthreads();   // shared arrays are reused by the next tile of this CTA
-  }
+  // small images spread their tiles over the SMs one warp at a time
+  const int wpb = tiles >= sms * 2 * kHitWarps ? kHitWarps : 1;
+  const dim3 grid(std::min((tiles + wpb - 1) / wpb, idle_tail ? sms : sms * 16)), block(32 * wpb);
+  auto* kernel = win <= 32 ? (ref_arith ? k_hits_warp<true, 1> : k_hits_warp<false, 1>)
+               : win <= 64 ? (ref_arith ? k_hits_warp<true, 2> : k_hits_warp<false, 2>)
+                           : (ref_arith ? k_hits_warp<true, 4> : k_hits_warp<false, 4>);
+  return cuda_check(launch_chained(kernel, grid, block, 0, st, a), "hits");
 }
 
 // Geometric hit masks of all pairs (no transmittance state): the superset the waves draw from.
@@ -962,18 +1155,17 @@ int launch_render_sorted(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scr
     const int cap_mlp = idle_tail ? sms : 0;
     const int32_t* act = s.active[cur];
     const int32_t* act_n = s.counters + kCtrActive0 + cur;
-    { LaunchScope scope(kKHits, 1, st);
-    if (ref_arith)
-      launch_chained(k_hits<true>, dim3(grid_hits), dim3(256), 0, st, fr->rays_o, fr->rays_d, (const float4*)sc->geom, n, fr->tile_offsets, s.tile_len, fr->sorted_prims,
-                              W, H, ntx, fr->threshold, miss_bound2(fr->threshold), act, act_n, lo, hi, s.px_state,
-                              s.masks32, s.pair_base,
-                              s.prim_cnt + (size_t)(w & 1) * prim_cnt_stride(n), s.counters, fr->max_records, fr->status, nullptr);
-    else
-      launch_chained(k_hits<false>, dim3(grid_hits), dim3(256), 0, st, fr->rays_o, fr->rays_d, (const float4*)sc->geom, n, fr->tile_offsets, s.tile_len, fr->sorted_prims,
-                              W, H, ntx, fr->threshold, miss_bound2(fr->threshold), act, act_n, lo, hi, s.px_state,
-                              s.masks32, s.pair_base,
-                              s.prim_cnt + (size_t)(w & 1) * prim_cnt_stride(n), s.counters, fr->max_records, fr->status, nullptr); }
-    int rc = launch_prim_scan(s, n, nxt, fr->status, st, split_small, w);
+    int rc;
+    {
+      LaunchScope scope(kKHits, 1, st);
+      const HitArgs ha = {fr->rays_o, fr->rays_d, (const float4*)sc->geom, n, fr->tile_offsets, s.tile_len, fr->sorted_prims, W, H, ntx,
+                          fr->threshold, miss_bound2(fr->threshold), form_threshold(fr->threshold), act, act_n, lo, hi, s.px_state,
+                          reinterpret_cast<uint2*>(s.masks32), s.pair_base, s.prim_cnt + (size_t)(w & 1) * prim_cnt_stride(n), s.counters,
+                          fr->max_records, fr->status, nullptr};
+      rc = launch_hits(ha, ref_arith, T, sms, idle_tail, st);
+      if (rc) return rc;
+    }
+    rc = launch_prim_scan(s, n, nxt, fr->status, st, split_small, w);
     if (rc) return rc;
     { LaunchScope scope(kKFill, 1, st);
     launch_chained(k_fill, dim3(grid_hits), dim3(256), 0, st, fr->rays_o, fr->rays_d, (const float4*)sc->geom, fr->tile_offsets, s.tile_len, fr->sorted_prims,
@@ -1096,24 +1288,21 @@ int launch_render_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scr
     const int grid_comp = idle_tail ? sms : std::min(T, sms * 32);
     const int cap_mlp = idle_tail ? sms : 0;
     int32_t* cnt = lead.prim_cnt + (size_t)(w & 1) * prim_cnt_stride(n);
+    int rc = MLPSP_OK;
     {
       LaunchScope scope(kKHits, V, st);
       for (int v = 0; v < V; ++v) {
         const mlpsp_frame* fr = frs + v;
         const Scratch& s = ss[v];
-        if (ref_arith)
-          launch_chained(k_hits<true>, dim3(grid_hits), dim3(256), 0, st, fr->rays_o, fr->rays_d, (const float4*)sc->geom, n, fr->tile_offsets, s.tile_len,
-                                                  fr->sorted_prims, W, H, ntx, f0->threshold, miss_bound2(f0->threshold), s.active[cur],
-                                                  s.counters + kCtrActive0 + cur, lo, hi, s.px_state, s.masks32, s.pair_base, cnt,
-                                                  lead.counters, f0->max_records, f0->status, s.counters + kCtrActive0 + nxt);
-        else
-          launch_chained(k_hits<false>, dim3(grid_hits), dim3(256), 0, st, fr->rays_o, fr->rays_d, (const float4*)sc->geom, n, fr->tile_offsets, s.tile_len,
-                                                   fr->sorted_prims, W, H, ntx, f0->threshold, miss_bound2(f0->threshold), s.active[cur],
-                                                   s.counters + kCtrActive0 + cur, lo, hi, s.px_state, s.masks32, s.pair_base, cnt,
-                                                   lead.counters, f0->max_records, f0->status, s.counters + kCtrActive0 + nxt);
+        const HitArgs ha = {fr->rays_o, fr->rays_d, (const float4*)sc->geom, n, fr->tile_offsets, s.tile_len, fr->sorted_prims, W, H, ntx,
+                            f0->threshold, miss_bound2(f0->threshold), form_threshold(f0->threshold), s.active[cur],
+                            s.counters + kCtrActive0 + cur, lo, hi, s.px_state, reinterpret_cast<uint2*>(s.masks32), s.pair_base, cnt,
+                            lead.counters, f0->max_records, f0->status, s.counters + kCtrActive0 + nxt};
+        rc = launch_hits(ha, ref_arith, T, sms, idle_tail, st);
+        if (rc) return rc;
       }
     }
-    int rc = launch_prim_scan(lead, n, nxt, f0->status, st, split_small, w);
+    rc = launch_prim_scan(lead, n, nxt, f0->status, st, split_small, w);
     if (rc) return rc;
     {
       LaunchScope scope(kKFill, V, st);
