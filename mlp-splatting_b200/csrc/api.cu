@@ -329,11 +329,6 @@ extern "C" int mlpsp_export_records(const mlpsp_scene* sc, const mlpsp_frame* fr
 // ------------------------------------------------------------ grouped evaluator on records ----
 namespace mlpsp {
 
-__global__ void k_grouped_counts(const int64_t* __restrict__ offsets, int n, int32_t* __restrict__ cnt) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) cnt[i] = (int32_t)(offsets[i + 1] - offsets[i]);
-}
-
 __global__ void k_grouped_records(const float* __restrict__ x6, int64_t R, RecIn* __restrict__ rec) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= R) return;
@@ -350,10 +345,6 @@ static Scratch grouped_layout(void* base, int64_t R, int n) {
   char* p = (char*)base;
   int64_t off = 0;
   auto take = [&](int64_t bytes) { char* r = p ? p + off : nullptr; off += align_up(bytes, 256); return r; };
-  s.prim_cnt = (int32_t*)take(4 * 2 * ((int64_t)n + 4));
-  s.prim_cursor = (int32_t*)take(4 * ((int64_t)n + 1));
-  s.prim_off = (int32_t*)take(4 * ((int64_t)n + 2));
-  s.scan_blk = (int32_t*)take(4 * 3 * ((int64_t)n / kPrimScanItems + 4));
   s.max_work = (int64_t)n + R / kRowsPerItem + 2;
   s.work = (int4*)take(16 * s.max_work);
   s.max_work_small = 2 * (int64_t)n + 2;
@@ -385,16 +376,15 @@ extern "C" int mlpsp_mlp_grouped(const mlpsp_scene* sc, int32_t precision, const
   if (n == 0 || num_records == 0) return MLPSP_OK;
   Scratch s = grouped_layout(scratch, num_records, n);
   MLPSP_CUDA_OK(cudaMemsetAsync(s.counters, 0, 4 * kNumCounters, st));
-  { LaunchScope scope(kKMisc, 2, st);
-  k_grouped_counts<<<(n + 255) / 256, 256, 0, st>>>(offsets, n, s.prim_cnt);
+  { LaunchScope scope(kKMisc, 1, st);
   k_grouped_records<<<(unsigned)((num_records + 255) / 256), 256, 0, st>>>(x6, num_records, s.rec_in); }
   const bool tc = precision == MLPSP_PRECISION_F16 || precision == MLPSP_PRECISION_BF16;
   const bool split_small = tc && num_records < 64 * (int64_t)n;     // fewer than 64 records per primitive on average
-  int rc = launch_prim_scan(s, n, 0, status, st, split_small);
+  int rc = launch_prim_scan(s, n, offsets, status, st, split_small, 0);
   if (rc) return rc;
   if (tc)
-    return launch_mlp_f16(sc, s.rec_in, s.prim_off, s.work, s.counters, (float4*)out4, nullptr, kOutSigmaRaw, status, st,
+    return launch_mlp_f16(sc, s.rec_in, s.work, s.counters, (float4*)out4, nullptr, kOutSigmaRaw, status, st,
                           precision == MLPSP_PRECISION_BF16, 0, split_small ? s.work_small : nullptr);
   MLPSP_REQUIRE(precision == MLPSP_PRECISION_F32, MLPSP_E_ARG, "mlpsp_mlp_grouped: unknown precision %d", precision);
-  return launch_mlp_f32(sc, s.rec_in, s.prim_off, s.work, s.counters, (float4*)out4, nullptr, kOutSigmaRaw, status, st);
+  return launch_mlp_f32(sc, s.rec_in, s.work, s.counters, (float4*)out4, nullptr, kOutSigmaRaw, status, st);
 }

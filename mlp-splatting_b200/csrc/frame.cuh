@@ -14,13 +14,14 @@ constexpr int kRowsPerSmallItem = 32;
 // counters[] slots (device int32)
 enum Counter {
   kCtrRecords = 0,   // records appended by the hit pass of the current wave
-  kCtrWork = 1,      // evaluator work items of the current wave
   kCtrWorkNext = 2,  // dynamic work cursor of the evaluator
   kCtrActive0 = 3,   // active tile count, list 0
   kCtrActive1 = 4,   // active tile count, list 1
   kCtrPairs = 5,     // total candidate pairs (binning)
   kCtrScratch = 6,   // three words (record export, long-tile list of the sort)
-  kCtrWorkSmall = 10, // small-group work items of the current wave
+  kCtrWaveRecords = 10, // records of the current wave
+  kCtrWork = 12,     // evaluator work items of the current wave, and, as the upper half of the same 64-bit word,
+  kCtrWorkSmall = 13, // small-group work items
   kNumCounters = 16
 };
 
@@ -42,8 +43,7 @@ struct Scratch {
   uint32_t* masks32;     // [2*max_pairs] evaluated-hit mask halves per pair
   uint32_t* pair_base;   // [max_pairs] first compositing slot of the pair
   int32_t* prim_cnt;     // [2][n] records per primitive in the current wave (even waves use the first half, odd the second)
-  int32_t* prim_cursor;  // [n]
-  int32_t* prim_off;     // [n+1]
+  int32_t* prim_pos;     // [n] where the primitive's next record of the current wave goes
   int4* work;            // [max_work] (primitive, first record, rows, 0)
   int4* work_small;      // [max_work_small] the same for items of at most kRowsPerSmallItem rows
   RecIn* rec_in;         // [max_records] primitive-major, reused by every wave
@@ -84,16 +84,13 @@ inline Scratch carve_scratch(void* base, int n, int W, int H, int ts, int64_t ma
   s.tile_diff = (int32_t*)take(4 * (int64_t)((W + ts - 1) / ts + 1) * ((H + ts - 1) / ts + 1));
   s.tile_fill = (int32_t*)take(4 * T);
   s.rect = (uint2*)take(8 * (int64_t)n);
-  const int64_t nblk = std::max<int64_t>((std::max<int64_t>(T, P + 1) + kScanItems - 1) / kScanItems,
-                                         ((int64_t)n + kPrimScanItems - 1) / kPrimScanItems) + 2;
-  s.scan_blk = (int32_t*)take(4 * 3 * nblk);
+  s.scan_blk = (int32_t*)take(4 * ((std::max<int64_t>(T, P + 1) + kScanItems - 1) / kScanItems + 2));
   s.px_state = (float4*)take(16 * P);
   s.px_depth = (float2*)take(8 * P);
   s.masks32 = (uint32_t*)take(8 * max_pairs);
   s.pair_base = (uint32_t*)take(4 * max_pairs);
   s.prim_cnt = (int32_t*)take(4 * 2 * ((int64_t)n + 4));
-  s.prim_cursor = (int32_t*)take(4 * (int64_t)n);
-  s.prim_off = (int32_t*)take(4 * ((int64_t)n + 1));
+  s.prim_pos = (int32_t*)take(4 * (int64_t)n);
   s.max_work = (int64_t)n + max_records / kRowsPerItem + 2;
   s.work = (int4*)take(16 * s.max_work);
   s.max_work_small = 2 * (int64_t)n + 2;
@@ -230,12 +227,12 @@ int launch_render_sorted(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scr
                          bool lists_refined = false);
 // rec_ext (optional): per record (sigma_raw, sigma_logit, layer-1 ReLU bitmask, layer-2 ReLU bitmask)
 // grid_cap > 0 limits the number of CTAs (a wave that is expected to be idle)
-int launch_mlp_f32(const mlpsp_scene* sc, const RecIn* rec_in, const int32_t* prim_off, const int4* work,
+int launch_mlp_f32(const mlpsp_scene* sc, const RecIn* rec_in, const int4* work,
                    const int32_t* counters, float4* rec_out, float4* rec_ext, int out_mode, int32_t* status,
                    cudaStream_t st, int grid_cap = 0);
 // bf16: bfloat16 operands (sc->wbf16) instead of binary16 (sc->w16)
 // work_small: the wave's small-group list (launch_prim_scan with split_small), or null when every item is on `work`
-int launch_mlp_f16(const mlpsp_scene* sc, const RecIn* rec_in, const int32_t* prim_off, const int4* work,
+int launch_mlp_f16(const mlpsp_scene* sc, const RecIn* rec_in, const int4* work,
                    const int32_t* counters, float4* rec_out, float4* rec_ext, int out_mode, int32_t* status,
                    cudaStream_t st, bool bf16 = false, int grid_cap = 0, const int4* work_small = nullptr);
 int launch_scan_i32(const int32_t* in, int64_t n, int32_t* blk, int32_t* out, cudaStream_t st);
@@ -252,12 +249,12 @@ constexpr int kOutSigmaRaw = 1;  // (R,G,B, softplus(o3)) scattered to rec.slot
 bool feature_tc_supported(const mlpsp_scene* sc);
 int launch_feature_tc(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, const uint32_t* used32, cudaStream_t st);
 
-// multi-block exclusive scan of per-primitive record counts plus evaluator work-item emission
+// positions of the primitives' records and the evaluator's work items from the per-primitive counts (or from fixed)
 // split_small: remainders of at most 64 records go to the small-group list (s.work_small)
 // distance in elements between the count arrays of even and odd waves (keeps the second one 16-byte aligned)
 __host__ __device__ inline size_t prim_cnt_stride(int n) { return ((size_t)n + 3) & ~(size_t)3; }
 int launch_render_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scratch* ss, int V, cudaStream_t st, bool lists_refined);
 int scan_launches(int64_t n);   // kernels launch_scan_i32 launches for n items
-int launch_prim_scan(const Scratch& s, int n, int next_list, int32_t* status, cudaStream_t st, bool split_small = false, int wave = 0);
+int launch_prim_scan(const Scratch& s, int n, const int64_t* fixed, int32_t* status, cudaStream_t st, bool split_small, int wave);
 
 }  // namespace mlpsp

@@ -13,7 +13,7 @@ __global__ void __launch_bounds__(kRowsPerItem) k_mlp_f32(
     const float* __restrict__ W1, const float* __restrict__ b1, const float* __restrict__ W2,
     const float* __restrict__ b2, const float* __restrict__ W3, const float* __restrict__ b3,
     const float* __restrict__ freq, const float* __restrict__ att, int F, int H,
-    const RecIn* __restrict__ rec_in, const int32_t* __restrict__ prim_off, const int4* __restrict__ work,
+    const RecIn* __restrict__ rec_in, const int4* __restrict__ work,
     int32_t* __restrict__ counters, float4* __restrict__ rec_out, float4* __restrict__ rec_ext, int out_mode,
     const int32_t* __restrict__ status) {
   extern __shared__ float sW[];
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(kRowsPerItem) k_mlp_f32_std(
   }
 }
 
-int launch_mlp_f32(const mlpsp_scene* sc, const RecIn* rec_in, const int32_t* prim_off, const int4* work,
+int launch_mlp_f32(const mlpsp_scene* sc, const RecIn* rec_in, const int4* work,
                    const int32_t* counters, float4* rec_out, float4* rec_ext, int out_mode, int32_t* status,
                    cudaStream_t st, int grid_cap) {
   const int H = sc->hidden, F = sc->num_freq;
@@ -219,10 +219,10 @@ int launch_mlp_f32(const mlpsp_scene* sc, const RecIn* rec_in, const int32_t* pr
         status);
   } else if (H <= 32) {
     k_mlp_f32<32><<<grid, kRowsPerItem, smem, st>>>(sc->W1, sc->b1, sc->W2, sc->b2, sc->W3, sc->b3, sc->freq, sc->att,
-                                                   F, H, rec_in, prim_off, work, ctr, rec_out, rec_ext, out_mode, status);
+                                                   F, H, rec_in, work, ctr, rec_out, rec_ext, out_mode, status);
   } else {
     k_mlp_f32<64><<<grid, kRowsPerItem, smem, st>>>(sc->W1, sc->b1, sc->W2, sc->b2, sc->W3, sc->b3, sc->freq, sc->att,
-                                                   F, H, rec_in, prim_off, work, ctr, rec_out, rec_ext, out_mode, status);
+                                                   F, H, rec_in, work, ctr, rec_out, rec_ext, out_mode, status);
   }
   return cuda_check(cudaGetLastError(), "mlp_f32");
 }

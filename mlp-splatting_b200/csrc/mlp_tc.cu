@@ -821,7 +821,7 @@ static int launch_tc(const mlpsp_scene* sc, const char* image, const RecIn* rec_
   return cuda_check(cudaGetLastError(), "mlp_f16");
 }
 
-int launch_mlp_f16(const mlpsp_scene* sc, const RecIn* rec_in, const int32_t* prim_off, const int4* work,
+int launch_mlp_f16(const mlpsp_scene* sc, const RecIn* rec_in, const int4* work,
                    const int32_t* counters, float4* rec_out, float4* rec_ext, int out_mode, int32_t* status,
                    cudaStream_t st, bool bf16, int grid_cap, const int4* work_small) {
   MLPSP_REQUIRE((sc->hidden == 32 || sc->hidden == 64) && sc->num_freq == 6, MLPSP_E_LIMIT,
@@ -830,7 +830,6 @@ int launch_mlp_f16(const mlpsp_scene* sc, const RecIn* rec_in, const int32_t* pr
   MLPSP_REQUIRE(image && sc->freq && sc->att, MLPSP_E_ARG, "%s evaluator needs the packed weight image",
                 bf16 ? "bf16" : "fp16");
   MLPSP_REQUIRE((reinterpret_cast<uintptr_t>(image) & 15) == 0, MLPSP_E_ARG, "the packed weight image must be 16-byte aligned");
-  (void)prim_off;
   if (sc->hidden == 64)
     return launch_tc<64>(sc, image, rec_in, work, work_small, counters, rec_out, rec_ext, out_mode, status, st, bf16, grid_cap);
   return launch_tc<32>(sc, image, rec_in, work, work_small, counters, rec_out, rec_ext, out_mode, status, st, bf16, grid_cap);

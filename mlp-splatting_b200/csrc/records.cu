@@ -37,8 +37,7 @@ __global__ void k_init_frame(int64_t P, float4* __restrict__ px_state, float2* _
                              float* __restrict__ rgb, float* __restrict__ alpha, float* __restrict__ depth_t,
                              float bgr, float bgg, float bgb, int T, int32_t* __restrict__ active0,
                              int32_t* __restrict__ counters, const int32_t* __restrict__ tile_offsets,
-                             int32_t* __restrict__ tile_len, int lists_refined, int n, int32_t* __restrict__ prim_cnt,
-                             int32_t* __restrict__ prim_cursor) {
+                             int32_t* __restrict__ tile_len, int lists_refined, int n, int32_t* __restrict__ prim_cnt) {
   chain_wait();
   chain_release();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -53,9 +52,9 @@ __global__ void k_init_frame(int64_t P, float4* __restrict__ px_state, float2* _
     active0[i] = (int)i;
     if (!lists_refined) tile_len[i] = tile_offsets[i + 1] - tile_offsets[i];
   }
-  if (i < n) { prim_cnt[i] = 0; prim_cnt[prim_cnt_stride(n) + i] = 0; prim_cursor[i] = 0; }   // the counts of even and odd waves
+  if (i < n) { prim_cnt[i] = 0; prim_cnt[prim_cnt_stride(n) + i] = 0; }   // the counts of even and odd waves
   if (i == 0) {
-    counters[kCtrRecords] = 0; counters[kCtrWork] = 0; counters[kCtrWorkNext] = 0; counters[kCtrWorkSmall] = 0;
+    counters[kCtrRecords] = 0;
     counters[kCtrActive0] = T; counters[kCtrActive1] = 0;
   }
 }
@@ -220,8 +219,14 @@ struct HitArgs {
   float thr, bound2, K;            // K <= 0: no quadratic form (thresholds the exponential underflows at)
   const int32_t* active; const int32_t* active_count; int lo, hi;
   const float4* px_state; uint2* masks; uint32_t* pair_base; int32_t* prim_cnt; int32_t* counters; int64_t max_records;
-  int32_t* status; int32_t* reset_count;
+  int32_t* status; int32_t* next_count;
 };
+
+// the wave's counters start at zero, and the list its compositing pass will append to starts empty
+__device__ __forceinline__ void reset_wave(const HitArgs& a) {
+  *a.next_count = 0;
+  a.counters[kCtrWork] = 0; a.counters[kCtrWorkSmall] = 0; a.counters[kCtrWorkNext] = 0; a.counters[kCtrWaveRecords] = 0;
+}
 
 __device__ __forceinline__ int warp_inclusive_scan(int v) {
   const int lane = threadIdx.x & 31;
@@ -241,9 +246,7 @@ __global__ void __launch_bounds__(32 * kHitWarps) k_hits_warp(const HitArgs a) {
   chain_release();
   __shared__ float4 s_q[kHitWarps][64];
   if (a.status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
-  // a view of a batch clears the count of the list its compositing pass of this wave will append to (the
-  // per-primitive scan does that for a frame rendered alone)
-  if (a.reset_count && blockIdx.x == 0 && threadIdx.x == 0) *a.reset_count = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) reset_wave(a);
   const int n_active = *a.active_count;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   for (int slot_i = blockIdx.x * wpb + warp; slot_i < n_active; slot_i += gridDim.x * wpb) {
@@ -295,7 +298,7 @@ __global__ void __launch_bounds__(256) k_hits(const HitArgs a) {
   __shared__ int warp_sums[32];
   __shared__ int s_tile_base, s_total;
   if (a.status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
-  if (a.reset_count && blockIdx.x == 0 && threadIdx.x == 0) *a.reset_count = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) reset_wave(a);
   const int n_active = *a.active_count;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int slot_i = blockIdx.x; slot_i < n_active; slot_i += gridDim.x) {
@@ -399,127 +402,93 @@ __device__ __forceinline__ int small_items_of(int cnt, int split) {
   return (rem > 0 && rem <= kRowsPerSmallItem) ? 1 : 0;
 }
 
-__global__ void k_prim_partial(const int32_t* __restrict__ prim_cnt, int n, int split, int32_t* __restrict__ blk,
-                               const int32_t* __restrict__ status) {
+// One launch per wave: every block scans its own 1,024 counts, reserves its share of the wave's record range and work
+// lists with one atomic each (their order among the blocks does not matter: a primitive's records only have to be
+// contiguous), writes the primitives' first positions and work items, and clears the counts the NEXT wave will add to
+// (waves alternate between two count arrays, so nothing this launch reads is written by it).  An exclusive scan over
+// the blocks, which this replaces, took two dependent launches (18 -> 8 us per wave at 100,000 primitives).
+// fixed (optional): the primitives' first positions are given (records already lie in primitive order).
+__global__ void __launch_bounds__(kPrimScanItems / 4) k_prim_alloc(
+    const int32_t* __restrict__ prim_cnt, int32_t* __restrict__ prim_cnt_next, const int64_t* __restrict__ fixed, int n, int split,
+    int32_t* __restrict__ prim_pos, int4* __restrict__ work, int64_t max_work, int4* __restrict__ work_small,
+    int64_t max_work_small, int32_t* __restrict__ counters, int32_t* __restrict__ status) {
   chain_wait();
   chain_release();
   __shared__ int warp_sums[32];
-  if (status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
-  const int64_t base = (int64_t)blockIdx.x * kPrimScanItems + (int64_t)threadIdx.x * 4;
-  int a = 0, b = 0, m = 0;
-#pragma unroll
-  for (int j = 0; j < 4; ++j)
-    if (base + j < n) { const int c = prim_cnt[base + j]; a += c; b += items_of(c, split); m += small_items_of(c, split); }
-  int ta, tb, tm;
-  block_exclusive_scan(a, warp_sums, ta);
-  block_exclusive_scan(b, warp_sums, tb);
-  block_exclusive_scan(m, warp_sums, tm);
-  if (threadIdx.x == 0) { blk[3 * blockIdx.x] = ta; blk[3 * blockIdx.x + 1] = tb; blk[3 * blockIdx.x + 2] = tm; }
-}
-
-// Second pass: every block sums the partial totals of the blocks before it (a few hundred at most), scans
-// its own 1,024 counts, writes the CSR offsets and the evaluator's work items and clears the counts the NEXT wave
-// will add to (waves alternate between two count arrays, so nothing this launch reads is written by it); the last
-// block also publishes the wave's totals.  blk == nullptr: there was no first pass -- the block sums the counts
-// of the blocks before it itself (worth it up to a few blocks: one launch instead of two).
-__global__ void k_prim_final(const int32_t* __restrict__ prim_cnt, int32_t* __restrict__ prim_cnt_next,
-                             int32_t* __restrict__ prim_cursor, int n, int split,
-                             const int32_t* __restrict__ blk, int32_t* __restrict__ prim_off,
-                             int4* __restrict__ work, int64_t max_work, int4* __restrict__ work_small, int64_t max_work_small,
-                             int32_t* __restrict__ counters, int next_list, int32_t* __restrict__ status) {
-  chain_wait();
-  chain_release();
-  __shared__ int warp_sums[32];
+  __shared__ int s_base[3];
   if (status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) {
     // after a record overflow, leave the size the wave asked for so the caller can grow its scratch
     if (blockIdx.x == 0 && threadIdx.x == 0 && (status[MLPSP_ST_BITS] & MLPSP_ST_RECORD_OVERFLOW))
       atomicMax(status + MLPSP_ST_WAVE_RECORDS, counters[kCtrRecords]);
     return;
   }
-  int pa = 0, pb = 0, pm = 0;
-  if (blk) {
-    for (int i = threadIdx.x; i < (int)blockIdx.x; i += blockDim.x) { pa += blk[3 * i]; pb += blk[3 * i + 1]; pm += blk[3 * i + 2]; }
-  } else {
-    const int4* c4 = reinterpret_cast<const int4*>(prim_cnt);     // both count arrays start 16-byte aligned
-    const int before4 = (int)blockIdx.x * (kPrimScanItems / 4);
-#pragma unroll 2
-    for (int i = threadIdx.x; i < before4; i += blockDim.x) {
-      const int4 c = c4[i];
-      pa += c.x + c.y + c.z + c.w;
-      pb += items_of(c.x, split) + items_of(c.y, split) + items_of(c.z, split) + items_of(c.w, split);
-      pm += small_items_of(c.x, split) + small_items_of(c.y, split) + small_items_of(c.z, split) + small_items_of(c.w, split);
-    }
-  }
-  int base_a, base_b, base_m;
-  block_exclusive_scan(pa, warp_sums, base_a);
-  block_exclusive_scan(pb, warp_sums, base_b);
-  block_exclusive_scan(pm, warp_sums, base_m);
   const int64_t base = (int64_t)blockIdx.x * kPrimScanItems + (int64_t)threadIdx.x * 4;
-  int c[4], a = 0, b = 0, m = 0;
+  int c[4] = {0, 0, 0, 0}, a = 0, b = 0, m = 0;
+  if (fixed) {
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    c[j] = (base + j < n) ? prim_cnt[base + j] : 0;
-    a += c[j]; b += items_of(c[j], split); m += small_items_of(c[j], split);
+    for (int j = 0; j < 4; ++j) if (base + j < n) c[j] = (int)(fixed[base + j + 1] - fixed[base + j]);
+  } else if (base < n) {     // both count arrays start 16-byte aligned and are padded to a multiple of four
+    const int4 v = *reinterpret_cast<const int4*>(prim_cnt + base);
+    c[0] = v.x; c[1] = base + 1 < n ? v.y : 0; c[2] = base + 2 < n ? v.z : 0; c[3] = base + 3 < n ? v.w : 0;
+    *reinterpret_cast<int4*>(prim_cnt_next + base) = make_int4(0, 0, 0, 0);
   }
-  int ta, tb, tm;
-  int ea = block_exclusive_scan(a, warp_sums, ta) + base_a;
-  int eb = block_exclusive_scan(b, warp_sums, tb) + base_b;
-  int em = block_exclusive_scan(m, warp_sums, tm) + base_m;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) { a += c[j]; b += items_of(c[j], split); m += small_items_of(c[j], split); }
+  int ta, tb, tm = 0;
+  int ea = block_exclusive_scan(a, warp_sums, ta);
+  if (ta == 0) {           // no records here: positions that nobody will use
+    return;
+  }
+  int eb = block_exclusive_scan(b, warp_sums, tb);
+  int em = split ? block_exclusive_scan(m, warp_sums, tm) : 0;
+  if (threadIdx.x == 0) {
+    const int r0 = atomicAdd(counters + kCtrWaveRecords, ta);
+    // both work lists in one 64-bit word, so that the last block to come sees the totals of both
+    const unsigned long long w0 = atomicAdd(reinterpret_cast<unsigned long long*>(counters + kCtrWork),
+                                            (unsigned long long)(uint32_t)tb | ((unsigned long long)(uint32_t)tm << 32));
+    s_base[0] = r0;
+    s_base[1] = (int)(uint32_t)w0;
+    s_base[2] = (int)(w0 >> 32);
+    if ((int64_t)s_base[1] + tb > max_work || (int64_t)s_base[2] + tm > max_work_small)
+      atomicOr(status + MLPSP_ST_BITS, MLPSP_ST_RECORD_OVERFLOW);
+    atomicAdd((unsigned long long*)(status + MLPSP_ST_RECORDS_LO), (unsigned long long)ta);
+    atomicMax(status + MLPSP_ST_WAVE_RECORDS, r0 + ta);
+    atomicMax(status + MLPSP_ST_WORK_ITEMS, s_base[1] + tb + s_base[2] + tm);
+    if (tb + tm) atomicAdd(status + MLPSP_ST_WORK_TOTAL, tb + tm);
+    if (tm) atomicAdd(status + MLPSP_ST_WORK_SMALL, tm);
+    if (r0 == 0) atomicAdd(status + MLPSP_ST_WAVES, 1);
+  }
+  __syncthreads();
+  ea += s_base[0]; eb += s_base[1]; em += s_base[2];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    if (base + j < n) {
-      prim_off[base + j] = ea;
-      const int it = items_of(c[j], split), sm = small_items_of(c[j], split);
+    if (c[j] > 0) {
+      const int first = fixed ? (int)fixed[base + j] : ea;
+      if (prim_pos) prim_pos[base + j] = first;
+      const int it = items_of(c[j], split);
       for (int q = 0; q < it; ++q)
         if ((int64_t)eb + q < max_work)
-          work[eb + q] = make_int4((int)(base + j), ea + q * kRowsPerItem, min(kRowsPerItem, c[j] - q * kRowsPerItem), 0);
-      const int first_small = c[j] - c[j] % kRowsPerItem;     // the remainder starts behind the full blocks
-      for (int q = 0; q < sm; ++q)
-        if ((int64_t)em + q < max_work_small)
-          work_small[em + q] = make_int4((int)(base + j), ea + first_small + q * kRowsPerSmallItem,
-                                         min(kRowsPerSmallItem, c[j] - first_small - q * kRowsPerSmallItem), 0);
-      ea += c[j]; eb += it; em += sm;
-      prim_cnt_next[base + j] = 0;
-      prim_cursor[base + j] = 0;
-    }
-  }
-  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
-    const int R = base_a + ta;
-    int G = base_b + tb, Gs = base_m + tm;
-    if ((int64_t)G > max_work) { G = (int)max_work; atomicOr(status + MLPSP_ST_BITS, MLPSP_ST_RECORD_OVERFLOW); }
-    if ((int64_t)Gs > max_work_small) { Gs = (int)max_work_small; atomicOr(status + MLPSP_ST_BITS, MLPSP_ST_RECORD_OVERFLOW); }
-    prim_off[n] = R;
-    counters[kCtrWork] = G;
-    counters[kCtrWorkSmall] = Gs;
-    counters[kCtrWorkNext] = 0;
-    counters[kCtrActive0 + next_list] = 0;   // kCtrRecords keeps counting: compositing slots are unique per frame
-    if (R > 0) {
-      atomicAdd((unsigned long long*)(status + MLPSP_ST_RECORDS_LO), (unsigned long long)R);
-      atomicMax(status + MLPSP_ST_WAVE_RECORDS, R);
-      atomicMax(status + MLPSP_ST_WORK_ITEMS, G + Gs);
-      atomicAdd(status + MLPSP_ST_WORK_TOTAL, G + Gs);
-      atomicAdd(status + MLPSP_ST_WORK_SMALL, Gs);
-      atomicAdd(status + MLPSP_ST_WAVES, 1);
+          work[eb + q] = make_int4((int)(base + j), first + q * kRowsPerItem, min(kRowsPerItem, c[j] - q * kRowsPerItem), 0);
+      if (small_items_of(c[j], split)) {                      // the remainder starts behind the full blocks
+        const int rem = c[j] % kRowsPerItem;
+        if ((int64_t)em < max_work_small) work_small[em] = make_int4((int)(base + j), first + c[j] - rem, rem, 0);
+        ++em;
+      }
+      ea += c[j]; eb += it;
     }
   }
 }
 
-// Up to 8,192 primitives the scan is one launch.  Beyond that the block that sums the most counts becomes the
-// launch's critical path (100,000 primitives: 23 us in one launch against 18 us in two).
-constexpr int kPrimScanSoloBlocks = 8;
-
-int launch_prim_scan(const Scratch& s, int n, int next_list, int32_t* status, cudaStream_t st, bool split_small, int wave) {
+int launch_prim_scan(const Scratch& s, int n, const int64_t* fixed, int32_t* status, cudaStream_t st, bool split_small, int wave) {
   const int nblk = (n + kPrimScanItems - 1) / kPrimScanItems;
   if (nblk == 0) return MLPSP_OK;
-  const bool solo = nblk <= kPrimScanSoloBlocks;
-  LaunchScope scope(kKScan, solo ? 1 : 2, st);
+  LaunchScope scope(kKScan, 1, st);
   const int split = split_small && s.work_small ? 1 : 0;
-  const int32_t* cnt = s.prim_cnt + (size_t)(wave & 1) * prim_cnt_stride(n);
+  int32_t* cnt = s.prim_cnt + (size_t)(wave & 1) * prim_cnt_stride(n);
   int32_t* cnt_next = s.prim_cnt + (size_t)((wave & 1) ^ 1) * prim_cnt_stride(n);
-  if (!solo) launch_chained(k_prim_partial, dim3(nblk), dim3(kPrimScanItems / 4), 0, st, cnt, n, split, s.scan_blk, status);
-  launch_chained(k_prim_final, dim3(nblk), dim3(kPrimScanItems / 4), 0, st, cnt, cnt_next, s.prim_cursor, n, split, solo ? nullptr : s.scan_blk, s.prim_off, s.work,
-                                     s.max_work, s.work_small, s.max_work_small, s.counters, next_list, status);
-  return cuda_check(cudaGetLastError(), "prim_scan");
+  return cuda_check(launch_chained(k_prim_alloc, dim3(nblk), dim3(kPrimScanItems / 4), 0, st, cnt, cnt_next, fixed, n, split, s.prim_pos, s.work,
+                                   s.max_work, s.work_small, s.max_work_small, s.counters, status),
+                    "prim_scan");
 }
 
 // -------------------------------------------------------------------------- fill pass ----
@@ -545,7 +514,7 @@ __global__ void __launch_bounds__(256) k_fill(
     const int32_t* __restrict__ tile_offsets, const int32_t* __restrict__ tile_len, const int32_t* __restrict__ sorted_prims, int W, int H, int ntx,
     float thr, const int32_t* __restrict__ active, const int32_t* __restrict__ active_count, int lo, int hi,
     const uint32_t* __restrict__ masks32, const uint32_t* __restrict__ pair_base,
-    const int32_t* __restrict__ prim_off, int32_t* __restrict__ prim_cursor, RecIn* __restrict__ rec_in,
+    int32_t* __restrict__ prim_pos, RecIn* __restrict__ rec_in,
     float* __restrict__ rec_t, float4* __restrict__ rec_gate, float beta, float tau, int exact_hits, int ref_arith,
     const int32_t* __restrict__ status) {
   chain_wait();
@@ -580,7 +549,7 @@ __global__ void __launch_bounds__(256) k_fill(
     int q0 = 0;
     if (c > 0) {
       const int p = sorted_prims[s + wlo + j];
-      q0 = prim_off[p] + atomicAdd(prim_cursor + p, c);
+      q0 = atomicAdd(prim_pos + p, c);
     }
     s_q0[j] = q0;
     if (j == nwin - 1) s_pref[nwin] = s_pref[j] + c;
@@ -621,6 +590,19 @@ __global__ void __launch_bounds__(256) k_fill(
   }
 }
 
+// Transpose of the 32 x 32 bit matrix whose row l is lane l's word.
+__device__ __forceinline__ uint32_t transpose32(uint32_t w) {
+  const int lane = threadIdx.x & 31;
+  uint32_t m = 0x0000ffffu;
+#pragma unroll
+  for (int s = 16; s; s >>= 1) {
+    const uint32_t other = __shfl_xor_sync(0xffffffffu, w, s);
+    w = (lane & s) ? (w & ~m) | ((other & ~m) >> s) : (w & m) | ((other & m) << s);
+    m ^= m << (s >> 1);
+  }
+  return w;
+}
+
 // --------------------------------------------------------------------------- composite ----
 // 64 threads per tile; each warp owns 32 pixels and stops as soon as none of them is live.
 struct PrimStats {
@@ -659,6 +641,59 @@ __global__ void __launch_bounds__(64) k_composite(
   int used = 0;
   float gtr = 0.f, gtg = 0.f, gtb = 0.f;
   if (STATS && tp.valid) { gtr = ps.gt_rgb[(size_t)tp.pix * 3]; gtg = ps.gt_rgb[(size_t)tp.pix * 3 + 1]; gtb = ps.gt_rgb[(size_t)tp.pix * 3 + 2]; }
+  if (!STATS) {
+  for (int i0 = wlo; i0 < whi && __any_sync(0xffffffffu, act); i0 += 32) {
+    const int idx = i0 + lane;
+    uint32_t mine = 0u, first = 0u;       // pair i0 + lane: this half's hit mask and the slot of its first record
+    if (idx < whi) {
+      const uint2 mm = *reinterpret_cast<const uint2*>(masks32 + 2 * (size_t)(s + idx));
+      mine = half ? mm.y : mm.x;
+      first = pair_base[s + idx] + (half ? __popc(mm.x) : 0);
+    }
+    // A pixel meets about one candidate in eight, so every lane walks its own hits (bit j of todo: pair i0 + j) instead of
+    // the warp walking the pairs: four of a lane's records are requested at a time, whether its pixel will still be live or
+    // not, then blended in list order.
+    uint32_t todo = transpose32(mine), taken = 0u;
+    if (!act) todo = 0u;
+    while (__any_sync(0xffffffffu, todo != 0u)) {
+      float4 rr[4];
+      uint32_t slot4[4], bit4[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int j = todo ? __ffs(todo) - 1 : lane;
+        bit4[u] = todo & (0u - todo);
+        todo &= todo - 1u;
+        const uint32_t mj = __shfl_sync(0xffffffffu, mine, j), fj = __shfl_sync(0xffffffffu, first, j);
+        slot4[u] = fj + __popc(mj & lt);
+        rr[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (bit4[u]) rr[u] = rec_out[slot4[u]];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const bool take = act && bit4[u];
+        if (take) {
+          const float4 r = rr[u];
+          const float w = st.w * r.w;
+          st.x = fmaf(w, r.x, st.x); st.y = fmaf(w, r.y, st.y); st.z = fmaf(w, r.z, st.z);
+          if (depth_t) { dp.x = fmaf(w, rec_t[slot4[u]], dp.x); dp.y += w; }
+          if (rec_w) rec_w[slot4[u]] = w;
+          if (rec_tr) rec_tr[slot4[u]] = st.w;
+          st.w *= (1.f - r.w);
+          act = st.w >= MLPSP_TERM;
+          taken |= bit4[u];
+        }
+      }
+      if (!act) todo = 0u;
+    }
+    used += __popc(taken);
+    if (mask_used32) {
+      const uint32_t um = transpose32(taken);
+      if (um) mask_used32[2 * (size_t)(s + idx) + half] = um;
+    }
+  }
+    used = __reduce_add_sync(0xffffffffu, used);
+  } else {
+  // statistics: the warp walks the pairs together, so that a pair's contributions are summed before they go to memory
   for (int i0 = wlo; i0 < whi && __any_sync(0xffffffffu, act); i0 += 32) {
     const int idx = i0 + lane;
     uint2 mm = make_uint2(0u, 0u);
@@ -734,6 +769,7 @@ __global__ void __launch_bounds__(64) k_composite(
         (void)m04;
       }
     }
+  }
   }
   if (tp.valid) {
     px_state[tp.pix] = st;
@@ -1118,7 +1154,7 @@ int launch_render_sorted(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scr
     const int64_t span = std::max<int64_t>(std::max<int64_t>(P, T), n);
     launch_chained(k_init_frame, dim3((unsigned)((span + 255) / 256)), dim3(256), 0, st, P, s.px_state, s.px_depth, fr->rgb, fr->alpha, fr->depth_t, bg[0], bg[1],
                                                                 bg[2], T, s.active[0], s.counters, fr->tile_offsets, s.tile_len,
-                                                                lists_refined ? 1 : 0, n, s.prim_cnt, s.prim_cursor);
+                                                                lists_refined ? 1 : 0, n, s.prim_cnt);
   }
   if (used32) MLPSP_CUDA_OK(cudaMemsetAsync(used32, 0, 8 * (size_t)fr->max_pairs, st));
   if (n == 0) {
@@ -1161,23 +1197,23 @@ int launch_render_sorted(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scr
       const HitArgs ha = {fr->rays_o, fr->rays_d, (const float4*)sc->geom, n, fr->tile_offsets, s.tile_len, fr->sorted_prims, W, H, ntx,
                           fr->threshold, miss_bound2(fr->threshold), form_threshold(fr->threshold), act, act_n, lo, hi, s.px_state,
                           reinterpret_cast<uint2*>(s.masks32), s.pair_base, s.prim_cnt + (size_t)(w & 1) * prim_cnt_stride(n), s.counters,
-                          fr->max_records, fr->status, nullptr};
+                          fr->max_records, fr->status, s.counters + kCtrActive0 + nxt};
       rc = launch_hits(ha, ref_arith, T, sms, idle_tail, st);
       if (rc) return rc;
     }
-    rc = launch_prim_scan(s, n, nxt, fr->status, st, split_small, w);
+    rc = launch_prim_scan(s, n, nullptr, fr->status, st, split_small, w);
     if (rc) return rc;
     { LaunchScope scope(kKFill, 1, st);
     launch_chained(k_fill, dim3(grid_hits), dim3(256), 0, st, fr->rays_o, fr->rays_d, (const float4*)sc->geom, fr->tile_offsets, s.tile_len, fr->sorted_prims,
-                              W, H, ntx, fr->threshold, act, act_n, lo, hi, s.masks32, s.pair_base, s.prim_off,
-                              s.prim_cursor, s.rec_in, (want_t || per_pixel) ? s.rec_t : nullptr,
+                              W, H, ntx, fr->threshold, act, act_n, lo, hi, s.masks32, s.pair_base, s.prim_pos,
+                              s.rec_in, (want_t || per_pixel) ? s.rec_t : nullptr,
                               (want_feat && sc->feat_slots > 1) ? s.rec_gate : nullptr, sc->gate_beta,
                               sc->gate_tau, per_pixel ? 1 : 0, ref_arith ? 1 : 0, fr->status); }
     if (tc_path)
-      rc = launch_mlp_f16(sc, s.rec_in, s.prim_off, s.work, s.counters, s.rec_out, keep ? s.rec_ext : nullptr, kOutAlpha,
+      rc = launch_mlp_f16(sc, s.rec_in, s.work, s.counters, s.rec_out, keep ? s.rec_ext : nullptr, kOutAlpha,
                           fr->status, st, fr->precision == MLPSP_PRECISION_BF16, cap_mlp, split_small ? s.work_small : nullptr);
     else
-      rc = launch_mlp_f32(sc, s.rec_in, s.prim_off, s.work, s.counters, s.rec_out, keep ? s.rec_ext : nullptr, kOutAlpha,
+      rc = launch_mlp_f32(sc, s.rec_in, s.work, s.counters, s.rec_out, keep ? s.rec_ext : nullptr, kOutAlpha,
                           fr->status, st, cap_mlp);
     if (rc) return rc;
     if (per_pixel) {
@@ -1261,7 +1297,7 @@ int launch_render_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scr
       const int64_t span = std::max<int64_t>(std::max<int64_t>(P, T), nv);
       launch_chained(k_init_frame, dim3((unsigned)((span + 255) / 256)), dim3(256), 0, st, P, ss[v].px_state, ss[v].px_depth, fr->rgb, fr->alpha, nullptr, bg[0], bg[1],
                                                                   bg[2], T, ss[v].active[0], ss[v].counters, fr->tile_offsets,
-                                                                  ss[v].tile_len, lists_refined ? 1 : 0, nv, lead.prim_cnt, lead.prim_cursor);
+                                                                  ss[v].tile_len, lists_refined ? 1 : 0, nv, lead.prim_cnt);
     }
   }
   if (n == 0) return cuda_check(cudaGetLastError(), "render_batch");
@@ -1302,7 +1338,7 @@ int launch_render_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scr
         if (rc) return rc;
       }
     }
-    rc = launch_prim_scan(lead, n, nxt, f0->status, st, split_small, w);
+    rc = launch_prim_scan(lead, n, nullptr, f0->status, st, split_small, w);
     if (rc) return rc;
     {
       LaunchScope scope(kKFill, V, st);
@@ -1311,15 +1347,15 @@ int launch_render_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scr
         const Scratch& s = ss[v];
         launch_chained(k_fill, dim3(grid_hits), dim3(256), 0, st, fr->rays_o, fr->rays_d, (const float4*)sc->geom, fr->tile_offsets, s.tile_len, fr->sorted_prims,
                                           W, H, ntx, f0->threshold, s.active[cur], s.counters + kCtrActive0 + cur, lo, hi, s.masks32,
-                                          s.pair_base, lead.prim_off, lead.prim_cursor, lead.rec_in, nullptr, nullptr, sc->gate_beta,
+                                          s.pair_base, lead.prim_pos, lead.rec_in, nullptr, nullptr, sc->gate_beta,
                                           sc->gate_tau, 0, ref_arith ? 1 : 0, f0->status);
       }
     }
     if (tc_path)
-      rc = launch_mlp_f16(sc, lead.rec_in, lead.prim_off, lead.work, lead.counters, lead.rec_out, nullptr, kOutAlpha, f0->status, st,
+      rc = launch_mlp_f16(sc, lead.rec_in, lead.work, lead.counters, lead.rec_out, nullptr, kOutAlpha, f0->status, st,
                           f0->precision == MLPSP_PRECISION_BF16, cap_mlp, split_small ? lead.work_small : nullptr);
     else
-      rc = launch_mlp_f32(sc, lead.rec_in, lead.prim_off, lead.work, lead.counters, lead.rec_out, nullptr, kOutAlpha, f0->status, st, cap_mlp);
+      rc = launch_mlp_f32(sc, lead.rec_in, lead.work, lead.counters, lead.rec_out, nullptr, kOutAlpha, f0->status, st, cap_mlp);
     if (rc) return rc;
     {
       LaunchScope scope(kKComposite, V, st);
