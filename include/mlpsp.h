@@ -253,6 +253,13 @@ int mlpsp_render_sorted(const mlpsp_scene* scene, const mlpsp_frame* frame, void
  * what sorted_prims holds afterwards. */
 int mlpsp_render_frame(const mlpsp_scene* scene, const mlpsp_frame* frame, void* stream);
 
+/* The same with less around it: the status block is reset by the call; rays_raw (DEVICE [W*H,3], or NULL) are directions
+ * of any length, whose unit vectors are written to frame->rays_d first; view_dev and proj_dev (DEVICE [16], or NULL)
+ * replace the frame's host matrices, so that a camera that lives on the device is not copied back; status_host
+ * (page-locked HOST [MLPSP_STATUS_WORDS], or NULL) receives the status block, for which the call synchronises. */
+int mlpsp_render_frame_rays(const mlpsp_scene* scene, const mlpsp_frame* frame, const float* rays_raw, const float* view_dev,
+                            const float* proj_dev, int32_t* status_host, void* stream);
+
 /* Several views of one scene in one call (no reference counterpart: the reference renders view by view,
  * scannet/cumodel.py:951).  frames[0..num_frames) are complete frames as for mlpsp_render_frame -- own rays,
  * matrices, tile-list buffers, outputs and scratch block each -- of one shape, threshold, precision, tile

@@ -254,23 +254,47 @@ extern "C" int mlpsp_render_sorted(const mlpsp_scene* sc, const mlpsp_frame* fr,
   return render_sorted_checked(sc, fr, s, (cudaStream_t)stream);
 }
 
-extern "C" int mlpsp_render_frame(const mlpsp_scene* sc, const mlpsp_frame* fr, void* stream) {
-  int rc = check_frame_common(sc, fr, "mlpsp_render_frame");
+static int render_frame(const mlpsp_scene* sc, const mlpsp_frame* fr, const float* rays_raw, const float* view_dev,
+                        const float* proj_dev, bool reset_status, cudaStream_t st, const char* who) {
+  int rc = check_frame_common(sc, fr, who);
   if (rc) return rc;
-  MLPSP_REQUIRE(fr->view && fr->proj, MLPSP_E_ARG, "mlpsp_render_frame: view/proj matrices missing");
-  MLPSP_REQUIRE(fr->rays_o && fr->rays_d, MLPSP_E_ARG, "mlpsp_render_frame: rays missing");
+  MLPSP_REQUIRE((fr->view && fr->proj) || (view_dev && proj_dev), MLPSP_E_ARG, "%s: view/proj matrices missing", who);
+  MLPSP_REQUIRE(fr->rays_o && fr->rays_d, MLPSP_E_ARG, "%s: rays missing", who);
+  MLPSP_REQUIRE(fr->rgb && fr->alpha, MLPSP_E_ARG, "render: rays or outputs missing");
   Scratch s;
-  rc = get_scratch(sc, fr, s, "mlpsp_render_frame");
+  rc = get_scratch(sc, fr, s, who);
   if (rc) return rc;
-  cudaStream_t st = (cudaStream_t)stream;
   // consumed-record masks are indexed by position in the full sorted list, so the pre-test stays off for them
   const bool pretest = fr->tile_pretest == 0 && fr->mask_used == nullptr && fr->tile == 8;
-  rc = launch_bin(sc, fr, s, st, /*order_lists=*/false, pretest);
+  if (pretest) {
+    rc = launch_frame_begin(sc, fr, s, rays_raw, reset_status, s.prim_cnt, st);
+    if (rc) return rc;
+  } else {
+    if (reset_status) MLPSP_CUDA_OK(cudaMemsetAsync(fr->status, 0, 4 * MLPSP_STATUS_WORDS, st));
+    if (rays_raw) {
+      rc = mlpsp_normalize_rows(rays_raw, const_cast<float*>(fr->rays_d), (int64_t)fr->width * fr->height, 3, st);
+      if (rc) return rc;
+    }
+  }
+  rc = launch_bin(sc, fr, s, st, /*order_lists=*/false, pretest, view_dev, proj_dev);
   if (rc) return rc;
   rc = launch_sort(sc, fr, nullptr, st, /*unordered_input=*/true, s.active[1], s.counters + kCtrScratch + 2,
                    pretest ? s.tile_len : nullptr);
   if (rc) return rc;
   return render_sorted_checked(sc, fr, s, st, pretest);
+}
+
+extern "C" int mlpsp_render_frame(const mlpsp_scene* sc, const mlpsp_frame* fr, void* stream) {
+  return render_frame(sc, fr, nullptr, nullptr, nullptr, false, (cudaStream_t)stream, "mlpsp_render_frame");
+}
+
+extern "C" int mlpsp_render_frame_rays(const mlpsp_scene* sc, const mlpsp_frame* fr, const float* rays_raw, const float* view_dev,
+                                       const float* proj_dev, int32_t* status_host, void* stream) {
+  cudaStream_t st = (cudaStream_t)stream;
+  const int rc = render_frame(sc, fr, rays_raw, view_dev, proj_dev, true, st, "mlpsp_render_frame_rays");
+  if (rc || !status_host) return rc;
+  MLPSP_CUDA_OK(cudaMemcpyAsync(status_host, fr->status, 4 * MLPSP_STATUS_WORDS, cudaMemcpyDeviceToHost, st));
+  return cuda_check(cudaStreamSynchronize(st), "render_frame");
 }
 
 extern "C" int mlpsp_render_frames(const mlpsp_scene* sc, const mlpsp_frame* frames, int32_t num_frames, void* stream) {
@@ -303,7 +327,10 @@ extern "C" int mlpsp_render_frames(const mlpsp_scene* sc, const mlpsp_frame* fra
   for (int v = 0; v < num_frames; ++v) {
     const mlpsp_frame* fr = frames + v;
     const Scratch& s = ss[(size_t)v];
-    int rc = launch_bin(sc, fr, s, st, /*order_lists=*/false, pretest);
+    int rc = MLPSP_OK;
+    if (pretest) rc = launch_frame_begin(sc, fr, s, nullptr, false, v == 0 ? s.prim_cnt : nullptr, st);
+    if (rc) return rc;
+    rc = launch_bin(sc, fr, s, st, /*order_lists=*/false, pretest);
     if (rc) return rc;
     rc = launch_sort(sc, fr, nullptr, st, /*unordered_input=*/true, s.active[1], s.counters + kCtrScratch + 2,
                      pretest ? s.tile_len : nullptr);

@@ -163,11 +163,39 @@ __device__ __forceinline__ void for_each_tile_flat(bool has, int x0, int x1, int
   __syncwarp();
 }
 
-__global__ void __launch_bounds__(256) k_bin_count(const float4* __restrict__ geom, int n, BinCam cam,
+struct BinMats { const float* view; const float* proj; };
+
+// pixels per unit of x / z (cumodel.py:1016-1020), the same operations on the host and on the device
+__host__ __device__ __forceinline__ float bin_focal(float p00, float p11, int W, int H) {
+#ifdef __CUDA_ARCH__
+  return fmul(fadd(fdiv(fmul(p00, (float)W), 2.0f), fdiv(fmul(p11, (float)H), 2.0f)), 0.5f);
+#else
+  const float fx = (p00 * (float)W) / 2.0f, fy = (p11 * (float)H) / 2.0f;
+  return (fx + fy) * 0.5f;
+#endif
+}
+
+// the block's camera in shared memory (all threads of the block call this)
+__device__ __forceinline__ void device_camera(BinCam& cam, const BinCam& host_cam, const BinMats& mats) {
+  if (threadIdx.x == 0) {
+    cam = host_cam;
+    if (mats.view) cam.focal = bin_focal(__ldg(mats.proj), __ldg(mats.proj + 5), host_cam.W, host_cam.H);
+  }
+  __syncthreads();
+  if (mats.view) {
+    if (threadIdx.x < 16) cam.view[threadIdx.x] = __ldg(mats.view + threadIdx.x);
+    else if (threadIdx.x < 32) cam.proj[threadIdx.x - 16] = __ldg(mats.proj + threadIdx.x - 16);
+    __syncthreads();
+  }
+}
+
+__global__ void __launch_bounds__(256) k_bin_count(const float4* __restrict__ geom, int n, const BinCam host_cam, const BinMats mats,
                                                    uint2* __restrict__ rect, int32_t* __restrict__ tile_cnt) {
   chain_wait();
   chain_release();
   __shared__ WarpRects s_wr[8];
+  __shared__ BinCam cam;
+  device_camera(cam, host_cam, mats);
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   int r[4] = {1, 0, 1, 0};
   const bool has = (p < n) && prim_rect(geom, p, cam, r);
@@ -180,10 +208,13 @@ __global__ void __launch_bounds__(256) k_bin_count(const float4* __restrict__ ge
 // The count pass without a walk over the tiles: a rectangle adds its four corners to a 2-D difference array
 // (+1, -1, -1, +1), and the 2-D prefix sum of that array is the number of rectangles over each tile.  Four atomics
 // per primitive instead of one per (tile, primitive) pair (100,000 against 2.9 million on the bench frame).
-__global__ void __launch_bounds__(256) k_bin_corners(const float4* __restrict__ geom, int n, BinCam cam,
-                                                     uint2* __restrict__ rect, int32_t* __restrict__ diff) {
+// mats (optional): the view and projection matrices in device memory, in place of the camera's own.
+__global__ void __launch_bounds__(256) k_bin_corners(const float4* __restrict__ geom, int n, const BinCam host_cam,
+                                                     const BinMats mats, uint2* __restrict__ rect, int32_t* __restrict__ diff) {
   chain_wait();
   chain_release();
+  __shared__ BinCam cam;
+  device_camera(cam, host_cam, mats);
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
   int r[4] = {1, 0, 1, 0};
@@ -209,30 +240,60 @@ __global__ void __launch_bounds__(1024) k_bin_offsets(const int32_t* __restrict_
   __shared__ int warp_sums[32];
   chain_wait();
   chain_release();
-  const int sx = ntx + 1, T = ntx * nty, tid = threadIdx.x;
+  const int sx = ntx + 1, T = ntx * nty, tid = threadIdx.x, lane = tid & 31;
+#pragma unroll 4
   for (int i = tid; i < sx * (nty + 1); i += 1024) s_cnt[i] = diff[i];
   __syncthreads();
-  for (int y = tid; y < nty; y += 1024) {
+  for (int y = tid >> 5; y < nty; y += 32) {          // a warp per row
     int acc = 0;
-    for (int x = 0; x < ntx; ++x) { acc += s_cnt[y * sx + x]; s_cnt[y * sx + x] = acc; }
+    for (int x0 = 0; x0 < ntx; x0 += 32) {
+      const int x = x0 + lane;
+      int v = x < ntx ? s_cnt[y * sx + x] : 0;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += u;
+      }
+      v += acc;
+      acc = __shfl_sync(0xffffffffu, v, 31);
+      if (x < ntx) s_cnt[y * sx + x] = v;
+    }
   }
   __syncthreads();
-  for (int x = tid; x < ntx; x += 1024) {
+  for (int x = tid; x < ntx; x += 1024) {             // a thread per column
     int acc = 0;
-    for (int y = 0; y < nty; ++y) { acc += s_cnt[y * sx + x]; s_cnt[y * sx + x] = acc; }
+    int y = 0;
+    for (; y + 8 <= nty; y += 8) {
+      int v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = s_cnt[(y + u) * sx + x];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) { acc += v[u]; s_cnt[(y + u) * sx + x] = acc; }
+    }
+    for (; y < nty; ++y) { acc += s_cnt[y * sx + x]; s_cnt[y * sx + x] = acc; }
   }
   __syncthreads();
   const int per = (T + 1023) / 1024;
   const int b = min(T, tid * per), e = min(T, b + per);
   int sum = 0, mx = 0;
+  int at = (b / ntx) * sx + b % ntx, col = b % ntx;   // a row of tiles is followed by one word of padding
   for (int t = b; t < e; ++t) {
-    const int c = s_cnt[(t / ntx) * sx + t % ntx];
+    const int c = s_cnt[at];
     sum += c;
     mx = max(mx, c);
+    ++at;
+    if (++col == ntx) { col = 0; ++at; }
   }
   int total;
   int ex = block_exclusive_scan(sum, warp_sums, total);
-  for (int t = b; t < e; ++t) { tile_offsets[t] = ex; ex += s_cnt[(t / ntx) * sx + t % ntx]; }
+  at = (b / ntx) * sx + b % ntx;
+  col = b % ntx;
+  for (int t = b; t < e; ++t) {
+    tile_offsets[t] = ex;
+    ex += s_cnt[at];
+    ++at;
+    if (++col == ntx) { col = 0; ++at; }
+  }
   mx = __reduce_max_sync(0xffffffffu, mx);
   if ((tid & 31) == 0 && mx > 0) {
     atomicMax(status + MLPSP_ST_MAX_TILE_LEN, mx);
@@ -446,15 +507,18 @@ int launch_scan_i32(const int32_t* in, int64_t n, int32_t* blk, int32_t* out, cu
 
 constexpr int kSortCap = 2048;  // per-tile sort capacity (>= tile capacity 1536)
 
+bool bin_uses_corners(const mlpsp_frame* fr) {
+  return 4 * (size_t)((fr->width + fr->tile - 1) / fr->tile + 1) * ((fr->height + fr->tile - 1) / fr->tile + 1) <= 200 * 1024;
+}
+
 int launch_bin(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, cudaStream_t st, bool order_lists,
-               bool pretest) {
+               bool pretest, const float* view_dev, const float* proj_dev) {
   const int T = num_tiles(fr->width, fr->height, fr->tile);
   BinCam cam;
-  for (int i = 0; i < 16; ++i) { cam.view[i] = fr->view[i]; cam.proj[i] = fr->proj[i]; }
+  const BinMats mats = {view_dev, proj_dev};
+  for (int i = 0; i < 16; ++i) { cam.view[i] = view_dev ? 0.f : fr->view[i]; cam.proj[i] = view_dev ? 0.f : fr->proj[i]; }
   cam.radius_mult = (float)sqrt(-2.0 * log((double)fr->threshold));
-  const float fx = (cam.proj[0] * (float)fr->width) / 2.0f;
-  const float fy = (cam.proj[5] * (float)fr->height) / 2.0f;
-  cam.focal = (fx + fy) * 0.5f;
+  cam.focal = bin_focal(cam.proj[0], cam.proj[5], fr->width, fr->height);
   cam.W = fr->width; cam.H = fr->height; cam.ts = fr->tile;
   cam.ntx = (fr->width + fr->tile - 1) / fr->tile;
   cam.nty = (fr->height + fr->tile - 1) / fr->tile;
@@ -476,21 +540,22 @@ int launch_bin(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, c
   // count pass: rectangle corners + one CTA's 2-D prefix when the corner array fits its shared memory (frames up
   // to about 3,500 x 3,500 pixels), else one atomic per (tile, primitive) pair and the multi-block scan
   const size_t diff_bytes = 4 * (size_t)(cam.ntx + 1) * (cam.nty + 1);
-  const bool corners = diff_bytes <= 200 * 1024;
-  if (corners) MLPSP_CUDA_OK(cudaMemsetAsync(s.tile_diff, 0, diff_bytes, st));
-  else MLPSP_CUDA_OK(cudaMemsetAsync(s.tile_cnt, 0, 4 * (size_t)(T + 1), st));
-  MLPSP_CUDA_OK(cudaMemsetAsync(fill, 0, 4 * (size_t)T, st));
-  LaunchScope scope(kKBin, (n > 0 ? (order_lists ? 3 : 2) : 0) + (corners ? 1 : 1 + scan_launches(T)) + (pretest ? 1 : 0), st);
-  if (pretest) launch_tile_frames(fr, s.tile_frame, st);
+  const bool corners = bin_uses_corners(fr);
+  if (!pretest) {      // k_frame_begin has cleared these for the fused path
+    if (corners) MLPSP_CUDA_OK(cudaMemsetAsync(s.tile_diff, 0, diff_bytes, st));
+    else MLPSP_CUDA_OK(cudaMemsetAsync(s.tile_cnt, 0, 4 * (size_t)(T + 1), st));
+    MLPSP_CUDA_OK(cudaMemsetAsync(fill, 0, 4 * (size_t)T, st));
+  }
+  LaunchScope scope(kKBin, (n > 0 ? (order_lists ? 3 : 2) : 0) + (corners ? 1 : 1 + scan_launches(T)), st);
   if (corners) {
     static DeviceOnce attr_once;
     if (attr_once.first())
       MLPSP_CUDA_OK(cudaFuncSetAttribute(k_bin_offsets, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    if (n > 0) launch_chained(k_bin_corners, dim3((n + 255) / 256), dim3(256), 0, st, (const float4*)sc->geom, n, cam, s.rect, s.tile_diff);
+    if (n > 0) launch_chained(k_bin_corners, dim3((n + 255) / 256), dim3(256), 0, st, (const float4*)sc->geom, n, cam, mats, s.rect, s.tile_diff);
     launch_chained(k_bin_offsets, dim3(1), dim3(1024), diff_bytes, st, s.tile_diff, cam.ntx, cam.nty, fr->tile_offsets, fr->tile_capacity,
                    fr->max_pairs, fr->status, s.counters);
   } else {
-    if (n > 0) launch_chained(k_bin_count, dim3((n + 255) / 256), dim3(256), 0, st, (const float4*)sc->geom, n, cam, s.rect, s.tile_cnt);
+    if (n > 0) launch_chained(k_bin_count, dim3((n + 255) / 256), dim3(256), 0, st, (const float4*)sc->geom, n, cam, mats, s.rect, s.tile_cnt);
     int rc = launch_scan_i32(s.tile_cnt, T, s.scan_blk, fr->tile_offsets, st);
     if (rc) return rc;
     launch_chained(k_bin_finish, dim3(std::min(64, (T + 255) / 256)), dim3(256), 0, st, s.tile_cnt, T, fr->tile_offsets, fr->tile_capacity,

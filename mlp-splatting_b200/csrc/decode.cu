@@ -726,9 +726,7 @@ extern "C" int mlpsp_decode_features(const mlpsp_decoder* dec, int32_t mode, con
   if (decode_once.first()) {
     MLPSP_CUDA_OK(cudaFuncSetAttribute(k_decode_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kDecSmem));
   }
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   const int tiles_x = (width + kDecTileW - 1) / kDecTileW, tiles_y = (height + kDecTileH - 1) / kDecTileH;
   const int num_tiles = tiles_x * tiles_y;
   cudaStream_t st = (cudaStream_t)stream;
@@ -745,9 +743,7 @@ extern "C" int mlpsp_classify_features(const float* feat, int64_t pixels, int32_
   MLPSP_REQUIRE(num_classes <= kMaxClasses && pixels <= (int64_t)kQM * 0x7fffffff, MLPSP_E_LIMIT,
                 "mlpsp_classify_features: at most %d classes", kMaxClasses);
   if (pixels == 0) return MLPSP_OK;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   cudaStream_t st = (cudaStream_t)stream;
   LaunchScope scope(kKMisc, 1, st);
   long long* lab = reinterpret_cast<long long*>(labels);

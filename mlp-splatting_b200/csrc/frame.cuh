@@ -209,10 +209,15 @@ HostWords& host_words();
 // order_lists = false leaves every tile list in scatter order for a following launch_sort(unordered_input = true).
 // pretest: write only the (tile, primitive) pairs that some ray of the tile can hit; s.tile_len receives the
 // number kept per tile (they sit at the front of the tile's span), tile_offsets stay those of the full lists.
+// Pre-tested binning works on what launch_frame_begin has prepared.  view_dev / proj_dev: the matrices in device memory,
+// in place of the frame's host matrices.
 int launch_bin(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, cudaStream_t st, bool order_lists = true,
-               bool pretest = false);
-// ray frame of every 8x8 tile (TileFrame), from the frame's rays
-void launch_tile_frames(const mlpsp_frame* fr, TileFrame* frames, cudaStream_t st);
+               bool pretest = false, const float* view_dev = nullptr, const float* proj_dev = nullptr);
+// the count pass adds rectangle corners (the corner array fits one CTA's shared memory: frames to about 3,500 x 3,500)
+bool bin_uses_corners(const mlpsp_frame* fr);
+// everything the fused path reads, in one launch (see k_frame_begin); prim_cnt null: the counts are another frame's
+int launch_frame_begin(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, const float* rays_raw, bool reset_status,
+                       int32_t* prim_cnt, cudaStream_t st);
 int launch_bin_mosaic(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, const int32_t* tile_view,
                       const float* views_host, int num_views, cudaStream_t st);
 int launch_bin_raycone(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, cudaStream_t st);
@@ -222,7 +227,7 @@ int launch_bin_raycone(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scrat
 int launch_sort(const mlpsp_scene* sc, const mlpsp_frame* fr, float* keys_out, cudaStream_t st, bool unordered_input,
                 int32_t* long_list, int32_t* long_count, const int32_t* list_len = nullptr);
 int launch_hit_masks(const mlpsp_scene* sc, const mlpsp_frame* fr, uint64_t* mask_geo, cudaStream_t st);
-// lists_refined: s.tile_len already holds the traversal length of every tile (written by launch_sort)
+// lists_refined: launch_frame_begin has prepared the frame and s.tile_len holds the traversal length of every tile
 int launch_render_sorted(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, cudaStream_t st,
                          bool lists_refined = false);
 // rec_ext (optional): per record (sigma_raw, sigma_logit, layer-1 ReLU bitmask, layer-2 ReLU bitmask)

@@ -207,9 +207,7 @@ int launch_mlp_f32(const mlpsp_scene* sc, const RecIn* rec_in, const int4* work,
                 "FP32 evaluator needs the FP32 weight arrays");
   const int IN = 12 * F;
   const size_t smem = sizeof(float) * (size_t)(H * IN + H + H * H + H + 4 * H + 4 + 2 * F);
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   const int grid = grid_cap > 0 ? std::min(grid_cap, sms * 8) : sms * 8;
   int32_t* ctr = const_cast<int32_t*>(counters);
   LaunchScope scope(kKMlp, 1, st);

@@ -791,9 +791,7 @@ static int launch_tc(const mlpsp_scene* sc, const char* image, const RecIn* rec_
                      const int32_t* counters, float4* rec_out, float4* rec_ext, int out_mode, int32_t* status, cudaStream_t st,
                      bool bf16, int grid_cap) {
   using N = Net<H>;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   int grid = sms * N::kCtas;
   if (grid_cap > 0) grid = std::min(grid, grid_cap);
   LaunchScope scope(kKMlp, (work_small && !rec_ext) ? 2 : 1, st);

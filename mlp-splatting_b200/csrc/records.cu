@@ -30,14 +30,14 @@ static inline float miss_bound2(float thr) { return (float)(-2.0 * log((double)t
 static inline float form_threshold(float thr) { const double k = -2.0 * log((double)thr); return k > 0.0 && k < 170.0 ? (float)k : 0.f; }
 
 // -------------------------------------------------------------------------- frame init ----
-// One launch prepares a frame: pixel state and the output image, the list of live tiles and the wave counters,
+// One launch prepares a frame whose lists come from the caller (k_frame_begin prepares the fused path): pixel state and the output image, the list of live tiles and the wave counters,
 // and the per-primitive counts and cursors of the first wave.
-// tile_len (when not already written by the sort's tile pre-test) = the length of the caller's list.
+// tile_len = the length of the caller's list.
 __global__ void k_init_frame(int64_t P, float4* __restrict__ px_state, float2* __restrict__ px_depth,
                              float* __restrict__ rgb, float* __restrict__ alpha, float* __restrict__ depth_t,
                              float bgr, float bgg, float bgb, int T, int32_t* __restrict__ active0,
                              int32_t* __restrict__ counters, const int32_t* __restrict__ tile_offsets,
-                             int32_t* __restrict__ tile_len, int lists_refined, int n, int32_t* __restrict__ prim_cnt) {
+                             int32_t* __restrict__ tile_len, int n, int32_t* __restrict__ prim_cnt) {
   chain_wait();
   chain_release();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -50,13 +50,159 @@ __global__ void k_init_frame(int64_t P, float4* __restrict__ px_state, float2* _
   }
   if (i < T) {
     active0[i] = (int)i;
-    if (!lists_refined) tile_len[i] = tile_offsets[i + 1] - tile_offsets[i];
+    tile_len[i] = tile_offsets[i + 1] - tile_offsets[i];
   }
   if (i < n) { prim_cnt[i] = 0; prim_cnt[prim_cnt_stride(n) + i] = 0; }   // the counts of even and odd waves
   if (i == 0) {
     counters[kCtrRecords] = 0;
     counters[kCtrActive0] = T; counters[kCtrActive1] = 0;
   }
+}
+
+// consumed-record masks of the pairs the tiles will traverse
+__global__ void __launch_bounds__(256) k_clear_used(const int32_t* __restrict__ tile_offsets, const int32_t* __restrict__ tile_len,
+                                                    int T, uint2* __restrict__ used, const int32_t* __restrict__ status) {
+  chain_wait();
+  chain_release();
+  if (status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
+  const int tile = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (tile >= T) return;
+  const int s = tile_offsets[tile], len = tile_len[tile];
+  for (int i = threadIdx.x & 31; i < len; i += 32) used[s + i] = make_uint2(0u, 0u);
+}
+
+// ------------------------------------------------------------------------- frame begin ----
+// The fused frame path starts with one launch that prepares everything the chain behind it reads: unit ray directions
+// (from the caller's raw ones, when given), the ray frame of every tile for the binning pre-test, pixel state and output
+// image, the per-primitive counts, the binning's corner array and fill counters, the tile lists' cursors and the wave
+// counters, the status block.  (One warp per tile, two pixels per lane; the flat arrays by all threads.)  It replaces a
+// normalising launch, two preparing launches and four memsets.
+struct BeginArgs {
+  const float* rays_o; const float* rays_raw; float* rays_d;   // rays_raw null: rays_d already holds unit directions
+  int W, H, ntx, T;
+  TileFrame* frames; int32_t* fill; int32_t* zero; int64_t zero_words;     // corner array (or tile counts) of the binning
+  float4* px_state; float2* px_depth; float* rgb; float* alpha; float* depth_t; float bgr, bgg, bgb;
+  int32_t* active0; int32_t* counters; int64_t cnt_words; int32_t* prim_cnt;
+  int32_t* status;                                             // null: the caller has reset it
+};
+
+__global__ void __launch_bounds__(256) k_frame_begin(const BeginArgs a) {
+  chain_wait();
+  chain_release();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t gid = (int64_t)blockIdx.x * 256 + threadIdx.x, gn = (int64_t)gridDim.x * 256;
+  for (int64_t i = gid; i * 4 < a.cnt_words; i += gn) *reinterpret_cast<int4*>(a.prim_cnt + i * 4) = make_int4(0, 0, 0, 0);
+  for (int64_t i = gid; i < a.zero_words; i += gn) a.zero[i] = 0;
+  if (blockIdx.x == 0 && threadIdx.x < kNumCounters)
+    a.counters[threadIdx.x] = threadIdx.x == kCtrActive0 ? a.T : 0;
+  if (a.status && blockIdx.x == 0 && threadIdx.x < MLPSP_STATUS_WORDS) a.status[threadIdx.x] = 0;
+  for (int tile = blockIdx.x * 8 + warp; tile < a.T; tile += gridDim.x * 8) {
+    const int tx = tile % a.ntx, ty = tile / a.ntx;
+    V3 dd[2], o0;
+    bool same = true;
+    float sx = 0.f, sy = 0.f, sz = 0.f;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int k = h * 32 + lane;
+      const int x = tx * 8 + (k & 7), y = ty * 8 + (k >> 3);
+      const bool valid = x < a.W && y < a.H;
+      // pixels past the image edge repeat the edge pixel: they add no new ray
+      const int64_t pix = (int64_t)min(y, a.H - 1) * a.W + min(x, a.W - 1);
+      const V3 o = load3(a.rays_o, pix);
+      if (h == 0) { o0.x = __shfl_sync(0xffffffffu, o.x, 0); o0.y = __shfl_sync(0xffffffffu, o.y, 0); o0.z = __shfl_sync(0xffffffffu, o.z, 0); }
+      V3 d;
+      if (a.rays_raw) {
+        d = load3(a.rays_raw, pix);
+        const float nrm = fmaxf(__fsqrt_rn(ffma(d.z, d.z, ffma(d.y, d.y, fmul(d.x, d.x)))), 1e-12f);
+        d = V3{fdiv(d.x, nrm), fdiv(d.y, nrm), fdiv(d.z, nrm)};
+        if (valid) { a.rays_d[pix * 3] = d.x; a.rays_d[pix * 3 + 1] = d.y; a.rays_d[pix * 3 + 2] = d.z; }
+      } else {
+        d = V3{a.rays_d[pix * 3], a.rays_d[pix * 3 + 1], a.rays_d[pix * 3 + 2]};
+      }
+      dd[h] = d;
+      same = same && o.x == o0.x && o.y == o0.y && o.z == o0.z;
+      sx += d.x; sy += d.y; sz += d.z;
+      if (valid) {
+        a.px_state[pix] = make_float4(0.f, 0.f, 0.f, 1.f);
+        a.rgb[pix * 3] = a.bgr; a.rgb[pix * 3 + 1] = a.bgg; a.rgb[pix * 3 + 2] = a.bgb;
+        a.alpha[pix] = 0.f;
+        if (a.depth_t) { a.depth_t[pix] = 0.f; a.px_depth[pix] = make_float2(0.f, 0.f); }
+      }
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      sx += __shfl_xor_sync(0xffffffffu, sx, off);
+      sy += __shfl_xor_sync(0xffffffffu, sy, off);
+      sz += __shfl_xor_sync(0xffffffffu, sz, off);
+    }
+    const float inv = rsqrtf(sx * sx + sy * sy + sz * sz);
+    const float ax = sx * inv, ay = sy * inv, az = sz * inv;
+    // u: the image's x direction made orthogonal to a (direction of pixel 7 minus pixel 0 of the first row);
+    // a fixed axis when the tile is one pixel wide
+    float ux = __shfl_sync(0xffffffffu, dd[0].x, 7) - __shfl_sync(0xffffffffu, dd[0].x, 0);
+    float uy = __shfl_sync(0xffffffffu, dd[0].y, 7) - __shfl_sync(0xffffffffu, dd[0].y, 0);
+    float uz = __shfl_sync(0xffffffffu, dd[0].z, 7) - __shfl_sync(0xffffffffu, dd[0].z, 0);
+    if (!(ux * ux + uy * uy + uz * uz > 1e-12f)) {
+      ux = fabsf(ax) < 0.57f ? 1.f : 0.f; uy = fabsf(ax) < 0.57f ? 0.f : 1.f; uz = 0.f;
+    }
+    const float ua = ux * ax + uy * ay + uz * az;
+    ux -= ua * ax; uy -= ua * ay; uz -= ua * az;
+    const float uinv = rsqrtf(ux * ux + uy * uy + uz * uz);
+    ux *= uinv; uy *= uinv; uz *= uinv;
+    const float vx = ay * uz - az * uy, vy = az * ux - ax * uz, vz = ax * uy - ay * ux;
+    float a0 = 3e38f, a1 = -3e38f, b0 = 3e38f, b1 = -3e38f, cmin = 3e38f;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float da = dd[h].x * ax + dd[h].y * ay + dd[h].z * az;
+      const float al = (dd[h].x * ux + dd[h].y * uy + dd[h].z * uz) / da;
+      const float be = (dd[h].x * vx + dd[h].y * vy + dd[h].z * vz) / da;
+      const float len2 = dd[h].x * dd[h].x + dd[h].y * dd[h].y + dd[h].z * dd[h].z;
+      cmin = fminf(cmin, da * rsqrtf(len2));
+      same = same && (al == al) && (be == be) && fabsf(al) < 1e6f && fabsf(be) < 1e6f;
+      a0 = fminf(a0, al); a1 = fmaxf(a1, al); b0 = fminf(b0, be); b1 = fmaxf(b1, be);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      a0 = fminf(a0, __shfl_xor_sync(0xffffffffu, a0, off)); a1 = fmaxf(a1, __shfl_xor_sync(0xffffffffu, a1, off));
+      b0 = fminf(b0, __shfl_xor_sync(0xffffffffu, b0, off)); b1 = fmaxf(b1, __shfl_xor_sync(0xffffffffu, b1, off));
+      cmin = fminf(cmin, __shfl_xor_sync(0xffffffffu, cmin, off));
+    }
+    same = __all_sync(0xffffffffu, same);
+    const bool ok = same && cmin > 0.5f && (ax == ax) && (ux == ux) && fabsf(o0.x) < 1e30f && fabsf(o0.y) < 1e30f &&
+                    fabsf(o0.z) < 1e30f;
+    if (lane == 0) {
+      TileFrame f;
+      // inflate the rectangle: rounding of the coordinates themselves
+      const float pa = 1e-5f + 1e-3f * (a1 - a0), pb = 1e-5f + 1e-3f * (b1 - b0);
+      f.ox = o0.x; f.oy = o0.y; f.oz = o0.z; f.ax = ax; f.ay = ay; f.az = az;
+      f.ux = ux; f.uy = uy; f.uz = uz; f.vx = vx; f.vy = vy; f.vz = vz;
+      f.a0 = ok ? a0 - pa : 1.f; f.a1 = ok ? a1 + pa : -1.f;
+      f.b0 = b0 - pb; f.b1 = b1 + pb;
+      a.frames[tile] = f;
+      a.fill[tile] = 0;
+      a.active0[tile] = tile;
+    }
+  }
+}
+
+int launch_frame_begin(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, const float* rays_raw, bool reset_status,
+                       int32_t* prim_cnt, cudaStream_t st) {
+  BeginArgs a;
+  a.rays_o = fr->rays_o; a.rays_raw = rays_raw; a.rays_d = const_cast<float*>(fr->rays_d);
+  a.W = fr->width; a.H = fr->height; a.ntx = (fr->width + 7) / 8; a.T = num_tiles(fr->width, fr->height, 8);
+  a.frames = s.tile_frame; a.fill = s.tile_len;
+  const bool corners = bin_uses_corners(fr);
+  a.zero = corners ? s.tile_diff : s.tile_cnt;
+  a.zero_words = corners ? (int64_t)(a.ntx + 1) * ((fr->height + 7) / 8 + 1) : a.T + 1;
+  a.px_state = s.px_state; a.px_depth = s.px_depth; a.rgb = fr->rgb; a.alpha = fr->alpha; a.depth_t = fr->depth_t;
+  a.bgr = a.bgg = a.bgb = 0.f;
+  if (fr->bg_color) { a.bgr = fr->bg_color[0]; a.bgg = fr->bg_color[1]; a.bgb = fr->bg_color[2]; }
+  a.active0 = s.active[0]; a.counters = s.counters;
+  a.prim_cnt = prim_cnt; a.cnt_words = prim_cnt ? 2 * (int64_t)prim_cnt_stride(sc->n) : 0;
+  a.status = reset_status ? fr->status : nullptr;
+  LaunchScope scope(kKMisc, 1, st);
+  const int grid = std::max((a.T + 7) / 8, (int)std::min<int64_t>(sm_count() * 8, (a.cnt_words / 4 + 255) / 256));
+  return cuda_check(launch_chained(k_frame_begin, dim3(grid), dim3(256), 0, st, a), "frame_begin");
 }
 
 // --------------------------------------------------------------------------- hit pass ----
@@ -1149,14 +1295,19 @@ int launch_render_sorted(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scr
   // record export reads the consumed masks from the scratch copy, so a caller-owned mask buffer is
   // filled by a device copy afterwards
   uint32_t* used32 = (keep || want_feat) ? s.used32 : (uint32_t*)fr->mask_used;
-  {
+  if (!lists_refined) {
     LaunchScope scope(kKMisc, 1, st);
     const int64_t span = std::max<int64_t>(std::max<int64_t>(P, T), n);
     launch_chained(k_init_frame, dim3((unsigned)((span + 255) / 256)), dim3(256), 0, st, P, s.px_state, s.px_depth, fr->rgb, fr->alpha, fr->depth_t, bg[0], bg[1],
                                                                 bg[2], T, s.active[0], s.counters, fr->tile_offsets, s.tile_len,
-                                                                lists_refined ? 1 : 0, n, s.prim_cnt);
+                                                                n, s.prim_cnt);
   }
-  if (used32) MLPSP_CUDA_OK(cudaMemsetAsync(used32, 0, 8 * (size_t)fr->max_pairs, st));
+  if (used32 && fr->mask_used) {
+    MLPSP_CUDA_OK(cudaMemsetAsync(used32, 0, 8 * (size_t)fr->max_pairs, st));     // the caller sees all of it
+  } else if (used32) {
+    LaunchScope scope(kKMisc, 1, st);
+    launch_chained(k_clear_used, dim3((T + 7) / 8), dim3(256), 0, st, fr->tile_offsets, s.tile_len, T, reinterpret_cast<uint2*>(used32), fr->status);
+  }
   if (n == 0) {
     if (want_feat) MLPSP_CUDA_OK(cudaMemsetAsync(fr->feat, 0, 4 * (size_t)P * sc->feat_dim, st));
     return cuda_check(cudaGetLastError(), "render_sorted");
@@ -1169,9 +1320,7 @@ int launch_render_sorted(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scr
   // extra launch per wave costs more than the few remainders gain (measured: 250,000 primitives on 816,000 pixels
   // lose 4 % of evaluator time with the second list, 500,000 gain 2 %, 2,000,000 with 64 hidden units gain 21 %).  (Record export keeps one list.)
   const bool split_small = tc_path && !keep && (int64_t)n * 3 > P;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   // CTAs walk the active-tile list with a grid stride, so a wave with few (or no) live tiles costs a
   // launch of a few thousand CTAs, not one per tile of the image
   const int wave_grid = std::min(T, sms * 16);
@@ -1287,7 +1436,7 @@ int launch_render_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scr
   const int64_t P = (int64_t)W * H;
   const int n = sc->n;
   const PrimStats no_stats = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-  {
+  if (!lists_refined) {
     LaunchScope scope(kKMisc, V, st);
     for (int v = 0; v < V; ++v) {
       const mlpsp_frame* fr = frs + v;
@@ -1297,7 +1446,7 @@ int launch_render_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scr
       const int64_t span = std::max<int64_t>(std::max<int64_t>(P, T), nv);
       launch_chained(k_init_frame, dim3((unsigned)((span + 255) / 256)), dim3(256), 0, st, P, ss[v].px_state, ss[v].px_depth, fr->rgb, fr->alpha, nullptr, bg[0], bg[1],
                                                                   bg[2], T, ss[v].active[0], ss[v].counters, fr->tile_offsets,
-                                                                  ss[v].tile_len, lists_refined ? 1 : 0, nv, lead.prim_cnt);
+                                                                  ss[v].tile_len, nv, lead.prim_cnt);
     }
   }
   if (n == 0) return cuda_check(cudaGetLastError(), "render_batch");
@@ -1307,9 +1456,7 @@ int launch_render_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scr
   // (measured with and without: fourview_500k in one batch of 4 views 2.51 -> 2.31 ms, stress_2m in batches of 16
   // views 72.2 -> 65.8 ms of evaluator time)
   const bool split_small = tc_path && (int64_t)n * 20 > P * V;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   const int wave_grid = std::min(T, sms * 16);
   const int nw = f0->num_waves > 0 ? f0->num_waves : (int)(sizeof(kDefaultWaves) / sizeof(int));
   int lo = 0;

@@ -302,87 +302,6 @@ __global__ void __launch_bounds__(THREADS) k_sort_long(
   }
 }
 
-// ---- per-tile ray frames for the tile pre-test: one warp per tile, two pixels per lane ----
-__global__ void __launch_bounds__(256) k_tile_frames(const float* __restrict__ rays_o, const float* __restrict__ rays_d,
-                                                     int W, int H, int ntx, int T, TileFrame* __restrict__ frames) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tile = blockIdx.x * 8 + warp;
-  if (tile >= T) return;
-  const int tx = tile % ntx, ty = tile / ntx;
-  V3 dd[2];
-  bool same = true;
-  const int64_t p0 = (int64_t)min(ty * 8, H - 1) * W + min(tx * 8, W - 1);
-  const V3 o0 = load3(rays_o, p0);
-  float sx = 0.f, sy = 0.f, sz = 0.f;
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int k = h * 32 + lane;
-    // pixels past the image edge repeat the edge pixel: they add no new ray
-    const int64_t pix = (int64_t)min(ty * 8 + (k >> 3), H - 1) * W + min(tx * 8 + (k & 7), W - 1);
-    const V3 o = load3(rays_o, pix);
-    dd[h] = load3(rays_d, pix);
-    same = same && o.x == o0.x && o.y == o0.y && o.z == o0.z;
-    sx += dd[h].x; sy += dd[h].y; sz += dd[h].z;
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    sx += __shfl_xor_sync(0xffffffffu, sx, off);
-    sy += __shfl_xor_sync(0xffffffffu, sy, off);
-    sz += __shfl_xor_sync(0xffffffffu, sz, off);
-  }
-  const float inv = rsqrtf(sx * sx + sy * sy + sz * sz);
-  const float ax = sx * inv, ay = sy * inv, az = sz * inv;
-  // u: the image's x direction made orthogonal to a (direction of pixel 7 minus pixel 0 of the first row);
-  // a fixed axis when the tile is one pixel wide
-  const int64_t p7 = (int64_t)min(ty * 8, H - 1) * W + min(tx * 8 + 7, W - 1);
-  const V3 d0 = load3(rays_d, p0), d7 = load3(rays_d, p7);
-  float ux = d7.x - d0.x, uy = d7.y - d0.y, uz = d7.z - d0.z;
-  if (!(ux * ux + uy * uy + uz * uz > 1e-12f)) {
-    ux = fabsf(ax) < 0.57f ? 1.f : 0.f; uy = fabsf(ax) < 0.57f ? 0.f : 1.f; uz = 0.f;
-  }
-  const float ua = ux * ax + uy * ay + uz * az;
-  ux -= ua * ax; uy -= ua * ay; uz -= ua * az;
-  const float uinv = rsqrtf(ux * ux + uy * uy + uz * uz);
-  ux *= uinv; uy *= uinv; uz *= uinv;
-  const float vx = ay * uz - az * uy, vy = az * ux - ax * uz, vz = ax * uy - ay * ux;
-  float a0 = 3e38f, a1 = -3e38f, b0 = 3e38f, b1 = -3e38f, cmin = 3e38f;
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const float da = dd[h].x * ax + dd[h].y * ay + dd[h].z * az;
-    const float al = (dd[h].x * ux + dd[h].y * uy + dd[h].z * uz) / da;
-    const float be = (dd[h].x * vx + dd[h].y * vy + dd[h].z * vz) / da;
-    const float len2 = dd[h].x * dd[h].x + dd[h].y * dd[h].y + dd[h].z * dd[h].z;
-    cmin = fminf(cmin, da * rsqrtf(len2));
-    same = same && (al == al) && (be == be) && fabsf(al) < 1e6f && fabsf(be) < 1e6f;
-    a0 = fminf(a0, al); a1 = fmaxf(a1, al); b0 = fminf(b0, be); b1 = fmaxf(b1, be);
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    a0 = fminf(a0, __shfl_xor_sync(0xffffffffu, a0, off)); a1 = fmaxf(a1, __shfl_xor_sync(0xffffffffu, a1, off));
-    b0 = fminf(b0, __shfl_xor_sync(0xffffffffu, b0, off)); b1 = fmaxf(b1, __shfl_xor_sync(0xffffffffu, b1, off));
-    cmin = fminf(cmin, __shfl_xor_sync(0xffffffffu, cmin, off));
-  }
-  same = __all_sync(0xffffffffu, same);
-  const bool ok = same && cmin > 0.5f && (ax == ax) && (ux == ux) && fabsf(o0.x) < 1e30f && fabsf(o0.y) < 1e30f &&
-                  fabsf(o0.z) < 1e30f;
-  if (lane == 0) {
-    TileFrame f;
-    // inflate the rectangle: rounding of the coordinates themselves
-    const float pa = 1e-5f + 1e-3f * (a1 - a0), pb = 1e-5f + 1e-3f * (b1 - b0);
-    f.ox = o0.x; f.oy = o0.y; f.oz = o0.z; f.ax = ax; f.ay = ay; f.az = az;
-    f.ux = ux; f.uy = uy; f.uz = uz; f.vx = vx; f.vy = vy; f.vz = vz;
-    f.a0 = ok ? a0 - pa : 1.f; f.a1 = ok ? a1 + pa : -1.f;
-    f.b0 = b0 - pb; f.b1 = b1 + pb;
-    frames[tile] = f;
-  }
-}
-
-void launch_tile_frames(const mlpsp_frame* fr, TileFrame* frames, cudaStream_t st) {
-  const int T = num_tiles(fr->width, fr->height, 8);
-  const int ntx = (fr->width + 7) / 8;
-  k_tile_frames<<<(T + 7) / 8, 256, 0, st>>>(fr->rays_o, fr->rays_d, fr->width, fr->height, ntx, T, frames);
-}
-
 int launch_sort(const mlpsp_scene* sc, const mlpsp_frame* fr, float* keys_out, cudaStream_t st, bool unordered_input,
                 int32_t* long_list, int32_t* long_count, const int32_t* list_len) {
   const int T = num_tiles(fr->width, fr->height, fr->tile);
@@ -390,10 +309,9 @@ int launch_sort(const mlpsp_scene* sc, const mlpsp_frame* fr, float* keys_out, c
   MLPSP_REQUIRE(fr->tile_capacity > 0 && fr->tile_capacity <= kSortCap, MLPSP_E_LIMIT,
                 "tile_capacity must be in [1, %d]", kSortCap);
   MLPSP_REQUIRE(long_list && long_count, MLPSP_E_ARG, "sort: scratch for the long-tile list missing");
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  MLPSP_CUDA_OK(cudaMemsetAsync(long_count, 0, 8, st));   // tile cursors: [0] of k_sort_long, [1] of k_sort_tiles
+  const int sms = sm_count();
+  // tile cursors: [0] of k_sort_long, [1] of k_sort_tiles (a frame that k_frame_begin prepared starts with both at zero)
+  if (!list_len) MLPSP_CUDA_OK(cudaMemsetAsync(long_count, 0, 8, st));
   LaunchScope scope(kKSort, 2, st);
   const int grid = std::min((T + kTilesPerCta - 1) / kTilesPerCta, sms * 6);
   const int grid_long = std::min(T, sms * 6);

@@ -174,7 +174,8 @@ class NeuralPrimitiveSceneTileCUDA(nn.Module):
             raise RuntimeError("NeuralPrimitiveSceneTileCUDA must be moved to a CUDA device before rendering.")
         if device.index is None:
             device = torch.device("cuda", torch.cuda.current_device())
-        torch.cuda.set_device(device.index)
+        if device.index != torch.cuda.current_device():
+            torch.cuda.set_device(device.index)
         return device
 
     def _resolve_tile_order_mode(self) -> str:
@@ -188,18 +189,17 @@ class NeuralPrimitiveSceneTileCUDA(nn.Module):
         return mode
 
     # --------------------------------------------------------------------------- internals ----
-    def _params(self):
-        ps = [self.positions, self.log_scales, self.quats, self.W1, self.b1, self.W2, self.b2, self.W3, self.b3]
-        if self.feat_attr is not None:
-            ps.append(self.feat_attr)
-        return ps
-
     def packed_scene(self) -> PackedScene:
         """Packed parameters on the module's device, rebuilt when a parameter changed in place."""
         device = self._activate_cuda_device()
         w = self.encoder.runtime_frequency_weights
-        key = (str(device), self.precision) + tuple((p.data_ptr(), p._version) for p in self._params()) + \
-              (w.data_ptr(), w._version)
+        ps = self._parameters
+        key = (device.index, self.precision, w.data_ptr(), w._version,
+               *((p.data_ptr(), p._version) for p in (ps["positions"], ps["log_scales"], ps["quats"], ps["W1"], ps["b1"], ps["W2"],
+                                                      ps["b2"], ps["W3"], ps["b3"])))
+        fa = self.feat_attr
+        if fa is not None:
+            key += (fa.data_ptr(), fa._version)
         if self._packed is None or self._packed_key != key:
             with torch.no_grad():
                 freq = self.encoder.freq_bands.to(device=device, dtype=torch.float32)
@@ -216,13 +216,15 @@ class NeuralPrimitiveSceneTileCUDA(nn.Module):
     def _renderer(self, device) -> FrameRenderer:
         W, H = self.image_size
         capacity = _tile_ext_build_config(self.tile_size)["tile_candidate_capacity"]
-        key = (str(device), W, H, capacity)
+        key = (device.index, W, H, capacity)
         if key not in self._renderers:
             self._renderers[key] = FrameRenderer(W, H, device=device, tile_capacity=capacity)
         return self._renderers[key]
 
     def _render(self, ray_o, ray_d, score_threshold, bg_color, view_matrix, proj_matrix, culled_prim_indices,
-                tile_offsets, want_depth, path_name, want_feat=False, sort_key=0, stats=None):
+                tile_offsets, want_depth, path_name, want_feat=False, sort_key=0, stats=None, want_alpha=True):
+        """(rgb, alpha, depth or None, feature map or None) of one frame, in tensors of the caller's own (alpha only when
+        want_alpha)."""
         if self.image_size is None:
             raise ValueError("image_size must be set on NeuralPrimitiveSceneTileCUDA before calling forward.")
         W, H = self.image_size
@@ -265,19 +267,23 @@ class NeuralPrimitiveSceneTileCUDA(nn.Module):
             bg = torch.as_tensor(bg_color, dtype=torch.float32).detach().cpu().reshape(-1)
             bg = bg.repeat(3) if bg.numel() == 1 else bg
             bg = bg.numpy()
-        view = None if lists is not None else view_matrix.detach().float().cpu().numpy()
-        proj = None if lists is not None else proj_matrix.detach().float().cpu().numpy()
+        view = proj = None
+        if lists is None:
+            view, proj = view_matrix.detach().float(), proj_matrix.detach().float()
+            if ts == 16 or not (view.is_cuda and proj.is_cuda):
+                view, proj = view.cpu().numpy(), proj.cpu().numpy()
+            else:
+                view, proj = view.contiguous(), proj.contiguous()       # read by the frame's own kernels
         prec = L.PRECISION_F32
         if self.precision == "fp16" and scene.has_f16:
             prec = L.PRECISION_F16
         elif self.precision == "bf16" and scene.has_bf16:
             prec = L.PRECISION_BF16
         render = r.render_tile16 if ts == 16 else r.render      # 16x16: culling and order per 16x16 tile, as the reference
-        rgb, alpha = render(scene, ray_o.detach().float().contiguous(), ray_d.detach().float().contiguous(),
-                            float(score_threshold), view=view, proj=proj, precision=prec, bg=bg,
-                            want_depth=want_depth, tile_lists=lists, path_name=path_name, want_feat=want_feat,
-                            sort_key=sort_key, prim_stats=stats)
-        return r, rgb, alpha
+        return render(scene, ray_o.detach().float().contiguous(), ray_d.detach().float().contiguous(),
+                      float(score_threshold), view=view, proj=proj, precision=prec, bg=bg,
+                      want_depth=want_depth, tile_lists=lists, path_name=path_name, want_feat=want_feat,
+                      sort_key=sort_key, prim_stats=stats, fresh="rgb alpha" if want_alpha else "rgb")
 
     @torch.no_grad()
     def build_tilecenter_culling_from_tile_views(self, tile_view_ids, view_matrices, proj_matrix,
@@ -320,13 +326,12 @@ class NeuralPrimitiveSceneTileCUDA(nn.Module):
         if return_feature and self.feat_attr is None:
             raise RuntimeError("return_feature=True requested but feat_attr is not initialized.")
         if return_feature:
-            r, rgb, _alpha = self._render(ray_o, ray_d, score_threshold, bg_color, view_matrix, proj_matrix,
-                                          culled_prim_indices, tile_offsets, False,
-                                          "render_tiles_forward_tilecenter_with_feat", want_feat=True)
-            return rgb.clone(), r.feat.clone()
-        _r, rgb, _alpha = self._render(ray_o, ray_d, score_threshold, bg_color, view_matrix, proj_matrix,
-                                       culled_prim_indices, tile_offsets, False, "render_tiles_forward_tilecenter")
-        return rgb.clone()
+            rgb, _alpha, _depth, feat = self._render(ray_o, ray_d, score_threshold, bg_color, view_matrix, proj_matrix,
+                                                     culled_prim_indices, tile_offsets, False,
+                                                     "render_tiles_forward_tilecenter_with_feat", want_feat=True, want_alpha=False)
+            return rgb, feat
+        return self._render(ray_o, ray_d, score_threshold, bg_color, view_matrix, proj_matrix, culled_prim_indices, tile_offsets,
+                            False, "render_tiles_forward_tilecenter", want_alpha=False)[0]
 
     @torch.no_grad()
     def render_rgb_alpha_no_grad(self, ray_o, ray_d, score_threshold=1e-3, bg_color=None, view_matrix=None,
@@ -356,10 +361,8 @@ class NeuralPrimitiveSceneTileCUDA(nn.Module):
             stats = (gt, self.stat_sum_w, self.stat_max_w, self.stat_hits, self.stat_sum_werr, self.stat_contrib_count)
         # the reference's statistics kernel orders a tile by the Euclidean depth of the centres along the
         # tile-centre ray (np_tile_kernels.cu:2248-2256), its plain forward by t*: both are kept
-        _r, rgb, alpha = self._render(ray_o, ray_d, score_threshold, bg_color, view_matrix, proj_matrix,
-                                      culled_prim_indices, tile_offsets, False, "render_tiles_forward_tilecenter",
-                                      stats=stats, sort_key=1 if stats is not None else 0)
-        return rgb.clone(), alpha.clone()
+        return self._render(ray_o, ray_d, score_threshold, bg_color, view_matrix, proj_matrix, culled_prim_indices, tile_offsets,
+                            False, "render_tiles_forward_tilecenter", stats=stats, sort_key=1 if stats is not None else 0)[:2]
 
     @torch.no_grad()
     def reset_w_stats(self):
@@ -378,10 +381,10 @@ class NeuralPrimitiveSceneTileCUDA(nn.Module):
         """(rgb, expected depth t [B,1], alpha) as cumodel.py:1385-1525.  The reference's expected-depth
         kernel orders a tile by Euclidean depth along the tile-centre ray (np_tile_kernels.cu:5538-5543),
         not by t*, so this call does too."""
-        r, rgb, alpha = self._render(ray_o, ray_d, score_threshold, bg_color, view_matrix, proj_matrix,
-                                     culled_prim_indices, tile_offsets, True, "render_tiles_forward_tilecenter_with_t",
-                                     sort_key=1)
-        return rgb.clone(), r.depth_t.clone(), alpha.clone()
+        rgb, alpha, depth, _feat = self._render(ray_o, ray_d, score_threshold, bg_color, view_matrix, proj_matrix,
+                                                culled_prim_indices, tile_offsets, True, "render_tiles_forward_tilecenter_with_t",
+                                                sort_key=1)
+        return rgb, depth, alpha
 
     @torch.no_grad()
     def render_feature_map(self, ray_o, ray_d, score_threshold=1e-3, view_matrix=None, proj_matrix=None,

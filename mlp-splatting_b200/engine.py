@@ -22,6 +22,24 @@ def _stream_ptr(device):
     return C.c_void_p(torch.cuda.current_stream(device).cuda_stream)
 
 
+class _on:
+    """torch.cuda.device(d) that costs nothing when d is the current device already."""
+    __slots__ = ("d", "ctx")
+
+    def __init__(self, d):
+        self.d = d
+
+    def __enter__(self):
+        self.ctx = None
+        if torch.cuda.current_device() != (self.d.index if self.d.index is not None else torch.cuda.current_device()):
+            self.ctx = torch.cuda.device(self.d)
+            self.ctx.__enter__()
+
+    def __exit__(self, *exc):
+        if self.ctx is not None:
+            self.ctx.__exit__(*exc)
+
+
 def _dev_f32(x, device):
     t = torch.as_tensor(x)
     return t.to(device=device, dtype=torch.float32).contiguous()
@@ -275,9 +293,23 @@ class FrameRenderer:
         self._view = np.zeros(16, np.float32)
         self._proj = np.zeros(16, np.float32)
         self._bg = np.zeros(3, np.float32)
-        self.last_stats: FrameStats | None = None
+        self._view_ptr, self._proj_ptr = self._view.ctypes.data, self._proj.ctypes.data
+        self._stats = None          # FrameStats of the last checked frame, or its status words until somebody asks
         self._last_frame = None
+        self._frames = {}           # prepared frame structures by what they depend on (see _frame)
+        self._buffers = 0           # counts reallocations of the buffers those structures point at
+        self._status_np = self.status_host.numpy()
         self.f32_fallbacks = 0   # frames re-rendered in FP32 after an fp16 overflow
+
+    @property
+    def last_stats(self) -> "FrameStats | None":
+        if isinstance(self._stats, np.ndarray):
+            self._stats = self._parse_stats(self._stats)
+        return self._stats
+
+    @last_stats.setter
+    def last_stats(self, value):
+        self._stats = value
 
     # -- buffers ------------------------------------------------------------------------------
     def _ensure_scratch(self, n):
@@ -289,32 +321,67 @@ class FrameRenderer:
             self.scratch = None
             self.scratch = torch.empty(nbytes + 256, device=self.device, dtype=torch.uint8)
             self._scratch_key = key
+            self._buffers += 1
         return self.scratch
 
     def _frame(self, scene: PackedScene, rays_o, rays_d_unit, thr, precision, view, proj, bg, want_depth,
                want_mask_used, waves, want_feat=False, keep_records=False, sort_key=0, tile_rows=None,
-               tile_pretest=True, prim_stats=None, tail_hint=False, hit_arith=0) -> L.Frame:
-        f = L.Frame()
-        f.rays_o, f.rays_d = L.ptr(rays_o), L.ptr(rays_d_unit)
-        f.width, f.height, f.tile, f.threshold = self.W, self.H, self.tile, float(thr)
-        f.tile_capacity, f.precision = self.capacity, int(precision)
+               tile_pretest=True, prim_stats=None, tail_hint=False, hit_arith=0, outs=None) -> L.Frame:
+        """The frame structure of a call.  Filling its sixty fields costs more than the launches of a small frame, so a
+        structure is kept per configuration and only what changes from frame to frame is set: rays, matrices, outputs."""
+        key = None
+        if bg is None and prim_stats is None and not want_mask_used:
+            self._ensure_scratch(scene.n)
+            key = (self._buffers, self.capacity, scene.n, scene.feat_dim if want_feat else 0, thr, precision, want_depth, want_feat,
+                   tuple(waves) if waves else None, keep_records, sort_key, tile_rows, tile_pretest, tail_hint, hit_arith)
+            f = self._frames.get(key)
+            if f is not None:
+                return self._frame_io(f, scene, rays_o, rays_d_unit, view, proj, want_depth, want_feat, outs)
+        f = self._new_frame(scene, thr, precision, bg, want_mask_used, waves, want_feat, keep_records, sort_key, tile_rows,
+                            tile_pretest, prim_stats, tail_hint, hit_arith)
+        if key is not None:
+            if len(self._frames) >= 16:
+                self._frames.clear()
+            # (keyed again: preparing it may have allocated)
+            self._frames[(self._buffers,) + key[1:]] = f
+        return self._frame_io(f, scene, rays_o, rays_d_unit, view, proj, want_depth, want_feat, outs)
+
+    def _frame_io(self, f, scene, rays_o, rays_d_unit, view, proj, want_depth, want_feat, outs):
+        f.rays_o, f.rays_d, f.status = L.ptr(rays_o), L.ptr(rays_d_unit), self.status.data_ptr()
         if view is not None:
             self._view[:] = np.asarray(view, dtype=np.float32).reshape(16)
             self._proj[:] = np.asarray(proj, dtype=np.float32).reshape(16)
-            f.view, f.proj = self._view.ctypes.data, self._proj.ctypes.data
-        f.tile_offsets, f.tile_prims, f.sorted_prims = L.ptr(self.tile_offsets), L.ptr(self.tile_prims), L.ptr(self.sorted_prims)
-        f.max_pairs = self.max_pairs
+            f.view, f.proj = self._view_ptr, self._proj_ptr
+        else:
+            f.view = f.proj = None
+        if outs is not None:
+            rgb, alpha, depth, feat = outs
+            f.rgb, f.alpha, f.depth_t, f.feat = rgb.data_ptr(), alpha.data_ptr(), L.ptr(depth), L.ptr(feat)
+            return f
         f.rgb, f.alpha = L.ptr(self.rgb), L.ptr(self.alpha)
         if want_depth:
             if self.depth_t is None:
                 self.depth_t = torch.empty((self.P, 1), device=self.device, dtype=torch.float32)
             f.depth_t = L.ptr(self.depth_t)
+        else:
+            f.depth_t = None
         if want_feat:
-            if scene.feat_attr is None:
-                raise RuntimeError("feature rendering requested but the scene has no feat_attr")
             if self.feat is None or self.feat.shape[1] != scene.feat_dim:
                 self.feat = torch.empty((self.P, scene.feat_dim), device=self.device, dtype=torch.float32)
             f.feat = L.ptr(self.feat)
+        else:
+            f.feat = None
+        return f
+
+    def _new_frame(self, scene, thr, precision, bg, want_mask_used, waves, want_feat, keep_records, sort_key, tile_rows,
+                   tile_pretest, prim_stats, tail_hint, hit_arith) -> L.Frame:
+        f = L.Frame()
+        f.width, f.height, f.tile, f.threshold = self.W, self.H, self.tile, float(thr)
+        f.tile_capacity, f.precision = self.capacity, int(precision)
+        f.tile_offsets, f.tile_prims, f.sorted_prims = L.ptr(self.tile_offsets), L.ptr(self.tile_prims), L.ptr(self.sorted_prims)
+        f.max_pairs = self.max_pairs
+        if want_feat and scene.feat_attr is None:
+            raise RuntimeError("feature rendering requested but the scene has no feat_attr")
         if want_mask_used:
             if self.mask_used is None:
                 self.mask_used = torch.zeros(max(self.max_pairs, 1), device=self.device, dtype=torch.int64)
@@ -338,24 +405,25 @@ class FrameRenderer:
             f.stat_hits, f.stat_sum_werr, f.stat_contrib = L.ptr(hits), L.ptr(sum_werr), L.ptr(contrib)
         if tile_rows is not None:
             f.tile_row_begin, f.tile_row_end = int(tile_rows[0]), int(tile_rows[1])
-        f.status = L.ptr(self.status)
         if waves:
             f.num_waves = len(waves)
             for i, w in enumerate(waves):
                 f.wave_len[i] = int(w)
         return f
 
-    def _read_status(self):
-        self.status_host.copy_(self.status, non_blocking=True)
-        torch.cuda.current_stream(self.device).synchronize()
-        s = self.status_host.numpy()
+    @staticmethod
+    def _parse_stats(s):
         u = s.view(np.uint32)
         rec = int(u[L.ST_RECORDS_LO]) | (int(u[L.ST_RECORDS_LO + 1]) << 32)
         used = int(u[L.ST_USED_LO]) | (int(u[L.ST_USED_LO + 1]) << 32)
-        stats = FrameStats(int(s[L.ST_PAIRS]), int(s[L.ST_MAX_TILE_LEN]), rec, used, int(s[L.ST_WAVES]),
-                           int(s[L.ST_WAVE_RECORDS]), int(s[L.ST_WORK_ITEMS]), int(s[L.ST_WORK_TOTAL]), int(s[L.ST_PAIRS_KEPT]),
-                           int(s[L.ST_WORK_SMALL]))
-        return int(s[L.ST_BITS]), stats
+        return FrameStats(int(s[L.ST_PAIRS]), int(s[L.ST_MAX_TILE_LEN]), rec, used, int(s[L.ST_WAVES]),
+                          int(s[L.ST_WAVE_RECORDS]), int(s[L.ST_WORK_ITEMS]), int(s[L.ST_WORK_TOTAL]), int(s[L.ST_PAIRS_KEPT]),
+                          int(s[L.ST_WORK_SMALL]))
+
+    def _read_status(self):
+        self.status_host.copy_(self.status, non_blocking=True)
+        torch.cuda.current_stream(self.device).synchronize()
+        return int(self._status_np[L.ST_BITS]), self._parse_stats(self._status_np.copy())
 
     def _grow(self, bits, stats):
         """Resize after an overflow finding; returns True when the frame should be retried."""
@@ -365,6 +433,7 @@ class FrameRenderer:
             self.tile_prims = torch.empty(self.max_pairs, device=d, dtype=torch.int32)
             self.sorted_prims = torch.empty(self.max_pairs, device=d, dtype=torch.int32)
             self.mask_used = None
+            self._buffers += 1
             return True
         if bits & L.BIT_RECORD_OVERFLOW:
             self.max_records = int(max(stats.wave_records, self.max_records) * 2) + 4096
@@ -389,7 +458,7 @@ class FrameRenderer:
                bg=None, want_depth=False, want_mask_used=False, waves=None, tile_lists=None,
                rays_normalized=False, check=True, path_name="render_tiles_forward_tilecenter", want_feat=False,
                keep_records=False, sort_key=0, tile_rows=None, tile_pretest=True, prim_stats=None, hit_arith=0,
-               presorted=False):
+               presorted=False, fresh=None):
         """One frame.  tile_lists=(culled_prim_indices, tile_offsets) replaces binning (external culling);
         presorted=True says those lists are already in compositing order (no per-tile sort).
 
@@ -398,23 +467,49 @@ class FrameRenderer:
         tensors that receive the per-primitive contribution statistics of this frame (accumulated, not reset).
         hit_arith=1 computes the tile-centre key, the hit decision and the hit values in the reference kernels' own
         arithmetic (hardware exponential, compiler-contracted expressions) instead of the IEEE-only one: order, masks,
-        record lists and CSR offsets are then those of the reference's kernels on the same GPU."""
+        record lists and CSR offsets are then those of the reference's kernels on the same GPU.
+        view / proj may be float32 tensors on this renderer's device: they are then read there, without a copy to the host.
+        fresh="rgb" or "rgb alpha" renders these, and the depth and feature map if wanted, into new tensors, which the caller
+        owns, and returns (rgb, alpha, depth or None, feature map or None); otherwise the renderer's own (rgb, alpha) are
+        returned, valid until the next frame."""
         lib, d = self.lib, self.device
         if precision is None:
             precision = L.PRECISION_F16 if scene.has_f16 else L.PRECISION_F32
         auto = waves is None
         if auto:
             waves = getattr(self, "_auto_waves", None)
-        with torch.cuda.device(d):
+        view_dev = proj_dev = None
+        if tile_lists is None and torch.is_tensor(view) and view.is_cuda:
+            view_dev, proj_dev = view, torch.as_tensor(proj)
+            if (proj_dev.device == view.device == self.rgb.device and view.dtype == proj_dev.dtype == torch.float32
+                    and view.is_contiguous() and proj_dev.is_contiguous() and view.numel() == proj_dev.numel() == 16):
+                view = proj = None
+            else:
+                view, proj = view.detach().float().cpu().numpy(), proj_dev.detach().float().cpu().numpy()
+                view_dev = proj_dev = None
+        with _on(d):
             st = _stream_ptr(d)
+            outs = None
+            if fresh:
+                if want_feat and scene.feat_attr is None:
+                    raise RuntimeError("feature rendering requested but the scene has no feat_attr")
+                outs = (torch.empty((self.P, 3), device=d, dtype=torch.float32),
+                        torch.empty((self.P, 1), device=d, dtype=torch.float32) if "alpha" in fresh else self.alpha,
+                        torch.empty((self.P, 1), device=d, dtype=torch.float32) if want_depth else None,
+                        torch.empty((self.P, scene.feat_dim), device=d, dtype=torch.float32) if want_feat else None)
+            raw = None
             if rays_normalized:
                 rd = rays_d
             else:
-                L.check(lib.mlpsp_normalize_rows(L.ptr(rays_d), L.ptr(self.rays_d_unit), self.P, 3, st), "mlpsp_normalize_rows")
                 rd = self.rays_d_unit
+                if tile_lists is None:
+                    raw = rays_d.data_ptr()          # the frame's first launch writes the unit directions
+                else:
+                    L.check(lib.mlpsp_normalize_rows(L.ptr(rays_d), L.ptr(rd), self.P, 3, st), "mlpsp_normalize_rows")
+            result = outs if fresh else (self.rgb, self.alpha)
             for _attempt in range(8):
-                L.check(lib.mlpsp_status_reset(L.ptr(self.status), st), "mlpsp_status_reset")
                 if tile_lists is not None:
+                    L.check(lib.mlpsp_status_reset(L.ptr(self.status), st), "mlpsp_status_reset")
                     prims, offs = tile_lists
                     m = int(prims.numel())
                     if m > self.max_pairs:
@@ -422,6 +517,7 @@ class FrameRenderer:
                         self.tile_prims = torch.empty(max(m, 1), device=d, dtype=torch.int32)
                         self.sorted_prims = torch.empty(max(m, 1), device=d, dtype=torch.int32)
                         self.mask_used = None
+                        self._buffers += 1
                     self.tile_prims[:m].copy_(prims)
                     if presorted:
                         self.sorted_prims[:m].copy_(prims)
@@ -432,20 +528,28 @@ class FrameRenderer:
                 f = self._frame(scene, rays_o, rd, threshold, precision, view, proj, bg, want_depth, want_mask_used, waves,
                                 want_feat=want_feat, keep_records=keep_records, sort_key=sort_key, tile_rows=tile_rows,
                                 tile_pretest=tile_pretest, prim_stats=prim_stats, tail_hint=auto and waves is not None,
-                                hit_arith=hit_arith)
+                                hit_arith=hit_arith, outs=outs)
                 self._last_frame = (f, scene)
                 if tile_lists is None:
-                    L.check(lib.mlpsp_render_frame(C.byref(scene.c), C.byref(f), st), "mlpsp_render_frame")
+                    L.check(lib.mlpsp_render_frame_rays(C.byref(scene.c), C.byref(f), raw, L.ptr(view_dev), L.ptr(proj_dev),
+                                                        self.status_host.data_ptr() if check else None, st), "mlpsp_render_frame")
                 else:
                     if not presorted:
                         L.check(lib.mlpsp_sort_tiles(C.byref(scene.c), C.byref(f), None, st), "mlpsp_sort_tiles")
                     L.check(lib.mlpsp_render_sorted(C.byref(scene.c), C.byref(f), st), "mlpsp_render_sorted")
+                    if check:
+                        self.status_host.copy_(self.status, non_blocking=True)
+                        torch.cuda.current_stream(d).synchronize()
                 if not check:
-                    return self.rgb, self.alpha
-                bits, stats = self._read_status()
-                self.last_stats = stats
-                if auto and bits == 0 and sort_key != L.ORDER_PER_PIXEL:
-                    self._adapt_waves(stats.waves)
+                    return result
+                words = self._status_np
+                bits = int(words[L.ST_BITS])
+                self._stats = words.copy()
+                if bits == 0:
+                    if auto and sort_key != L.ORDER_PER_PIXEL:
+                        self._adapt_waves(int(words[L.ST_WAVES]))
+                    return result
+                stats = self.last_stats
                 if bits & (L.BIT_BAD_OFFSETS | L.BIT_TILE_CAPACITY | L.BIT_BAD_IDS | L.BIT_TIMEOUT):
                     raise_for_status(bits, stats.max_tile_len, self.capacity, path_name)
                 if self._grow(bits, stats):
@@ -462,7 +566,7 @@ class FrameRenderer:
                     self.f32_fallbacks += 1
                     precision = L.PRECISION_F32
                     continue
-                return self.rgb, self.alpha
+                return result
             raise RenderError(f"{path_name}: scratch kept overflowing after 8 attempts")
 
     def tile16_lists(self, scene: PackedScene, rays_o, rays_d_unit, threshold, view, proj, sort_key=0,
@@ -495,6 +599,7 @@ class FrameRenderer:
                 c.max_pairs = m
                 c.tile_prims = torch.empty(max(m, 1), device=d, dtype=torch.int32)
                 c.sorted_prims = torch.empty(max(m, 1), device=d, dtype=torch.int32)
+                c._buffers += 1
             c.tile_prims[:m].copy_(prims16)
             c.tile_offsets.copy_(offs16)
             with torch.cuda.device(d):
@@ -713,6 +818,7 @@ class ViewBatchRenderer:
                         r.max_pairs = min(grown, r.T * r.capacity)
                         r.tile_prims = torch.empty(r.max_pairs, device=d, dtype=torch.int32)
                         r.sorted_prims = torch.empty(r.max_pairs, device=d, dtype=torch.int32)
+                        r._buffers += 1
                     continue
                 if bits & L.BIT_RECORD_OVERFLOW:
                     lead.max_records = int(max(stats.wave_records, lead.max_records) * 2) + 4096
