@@ -131,7 +131,6 @@ __device__ __forceinline__ void for_each_tile(bool has, int x0, int x1, int y0, 
 // rectangle j with pref[j] <= i < pref[j + 1].  Iterations are independent, so the atomics of several
 // of them are in flight at once, whatever the sizes of the individual rectangles.
 struct WarpRects { int pref[33]; int x0[32], y0[32], w[32], p[32]; };
-struct WarpWhiten { PrimWhiten w[8]; };   // whitening maps of a warp's primitives (pre-tested scatter)
 
 template <typename F>
 __device__ __forceinline__ void for_each_tile_flat(bool has, int x0, int x1, int y0, int y1, int ntx, int p,
@@ -307,23 +306,23 @@ __global__ void __launch_bounds__(1024) k_bin_offsets(const int32_t* __restrict_
   }
 }
 
-// PRETEST: a (tile, primitive) pair that no ray of the tile can hit (tile_surely_misses) is not
+// PRETEST: a (tile, primitive) pair that no ray of the tile can hit (ellipse_misses) is not
 // written; tile_fill then ends as the number of candidates kept per tile, packed at the front of the
 // tile's span of tile_prims (the span itself keeps the size the count pass gave it).
-// PPW primitives per warp: the pre-tested variant does a few hundred instructions and three dependent memory
-// round trips per pair, so it spreads the pairs over four times as many warps.
+// PPW primitives per warp: the pre-tested variant takes the pairs of eight primitives, whose ellipses one lane each
+// computes into shared memory; a pair is then one 16-byte load and about thirty operations (against a test of the
+// whitened quadratic form per pair: 102 -> 52 us on the 100k frame, 2.9 million pairs).
 template <bool PRETEST, int PPW>
 __global__ void __launch_bounds__(256) k_bin_scatter(int n, int ntx, const uint2* __restrict__ rect,
                                                      const int32_t* __restrict__ tile_offsets,
                                                      int32_t* __restrict__ tile_fill, int32_t* __restrict__ tile_prims,
                                                      const float4* __restrict__ geom,
-                                                     const TileFrame* __restrict__ frames, float K0,
-                                                     const int32_t* __restrict__ status) {
+                                                     const FramePlane* __restrict__ plane, const float4* __restrict__ tile_rect,
+                                                     float K0, const int32_t* __restrict__ status) {
   chain_wait();
   chain_release();
   __shared__ WarpRects s_wr[8];
-  __shared__ WarpWhiten s_ww[PRETEST ? 8 : 1];
-  static_assert(!PRETEST || PPW <= 8, "WarpWhiten holds eight maps per warp");
+  __shared__ float4 s_el[PRETEST ? 8 : 1][PPW][2];
   if (status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gwarp = blockIdx.x * 8 + warp;
@@ -335,16 +334,17 @@ __global__ void __launch_bounds__(256) k_bin_scatter(int n, int ntx, const uint2
     x0 = r.x & 0xffff; x1 = r.x >> 16; y0 = r.y & 0xffff; y1 = r.y >> 16;
   }
   const bool has = mine && x0 <= x1 && y0 <= y1;
-  if (PRETEST && has) s_ww[warp].w[lane] = make_whiten(load_geom(geom, p));
+  if (PRETEST && has) {
+    const PlaneEllipse e = plane_ellipse(load_geom(geom, p), *plane, K0);
+    s_el[warp][lane][0] = make_float4(e.zx, e.zy, e.a11, e.a12);
+    s_el[warp][lane][1] = make_float4(e.a22, e.r1, e.r2, e.rho);
+  }
   // (for_each_tile_flat synchronises the warp before the first item is read)
   for_each_tile_flat(has, x0, x1, y0, y1, ntx, PRETEST ? lane : p, s_wr[warp], [&](int t, int q) {
     int id = q;
     if (PRETEST) {
-      // q is the lane that brought the primitive: its map sits in shared memory
-      const float4* fp = reinterpret_cast<const float4*>(frames + t);
-      const float4 f0 = __ldg(fp), f1 = __ldg(fp + 1), f2 = __ldg(fp + 2), f3 = __ldg(fp + 3);
-      const TileFrame f = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w, f2.x, f2.y, f2.z, f2.w, f3.x, f3.y, f3.z, f3.w};
-      if (tile_surely_misses(s_ww[warp].w[q], f, K0)) return;
+      // q is the lane that brought the primitive: its ellipse sits in shared memory
+      if (ellipse_misses(s_el[warp][q][0], s_el[warp][q][1], __ldg(tile_rect + t))) return;
       id = gwarp * PPW + q;
     }
     const int slot = atomicAdd(tile_fill + t, 1);
@@ -564,11 +564,11 @@ int launch_bin(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, c
   if (n > 0) {
     if (pretest)
       launch_chained(k_bin_scatter<true, 8>, dim3((n + 63) / 64), dim3(256), 0, st, n, cam.ntx, s.rect, fr->tile_offsets, fill, fr->tile_prims,
-                                                           (const float4*)sc->geom, s.tile_frame,
+                                                           (const float4*)sc->geom, s.plane, s.tile_rect,
                                                            (float)(-2.0 * log((double)fr->threshold)), fr->status);
     else
       launch_chained(k_bin_scatter<false, 32>, dim3((n + 255) / 256), dim3(256), 0, st, n, cam.ntx, s.rect, fr->tile_offsets, fill, fr->tile_prims,
-                                                            nullptr, nullptr, 0.f, fr->status);
+                                                            nullptr, nullptr, nullptr, 0.f, fr->status);
     if (order_lists) k_sort_ids<256, kSortCap><<<T, 256, 0, st>>>(fr->tile_offsets, fr->tile_prims, fr->status);
   }
   return cuda_check(cudaGetLastError(), "bin");

@@ -245,29 +245,14 @@ __device__ __forceinline__ bool hit_test_ref(const GeomRef& g, V3 o, V3 d, float
   return decay > thr;
 }
 
-// ---- per-tile ray frame and the (tile, primitive) pre-test of the fused frame path ----
-// All rays of a tile leave one origin o; with an orthonormal frame (a, u, v), a along the tile's mean
-// direction, every ray direction is a + alpha u + beta v up to scale (alpha = d.u / d.a, beta = d.v / d.a),
-// and the tile's 64 rays lie inside the rectangle [a0, a1] x [b0, b1] of those coordinates (slightly
-// inflated).  a0 > a1 marks a tile without such a frame (several origins, a ray more than 60 degrees off the
-// mean, non-finite input): no candidate of it is ever rejected.
-struct __align__(16) TileFrame {
-  float ox, oy, oz, a0;
-  float ax, ay, az, a1;
-  float ux, uy, uz, b0;
-  float vx, vy, vz, b1;
+// ---- the (tile, primitive) pre-test of the fused frame path ----
+// The frame's tangent plane: origin o and an orthonormal frame (a, u, v) around the central ray.  A ray direction d from
+// that origin is a + alpha u + beta v up to scale (alpha = d.u / d.a, beta = d.v / d.a), and the rays of a tile lie in the
+// rectangle [a0, a1] x [b0, b1] of those coordinates (slightly inflated).  A tile whose rays do not all leave o, or lie
+// 75 degrees and more off the central ray, has no rectangle (NaN): no candidate of it is ever rejected.
+struct __align__(16) FramePlane {
+  float ox, oy, oz, pad0, ax, ay, az, pad1, ux, uy, uz, pad2, vx, vy, vz, pad3;
 };
-
-__device__ __forceinline__ float quad_min_1d(float A, float B, float C, float lo, float hi) {
-  // min over [lo, hi] of A t^2 + 2 B t + C
-  const float qlo = fmaf(fmaf(A, lo, 2.f * B), lo, C), qhi = fmaf(fmaf(A, hi, 2.f * B), hi, C);
-  float m = fminf(qlo, qhi);
-  if (A > 0.f) {
-    const float t = fminf(fmaxf(__fdividef(-B, A), lo), hi);
-    m = fminf(m, fmaf(fmaf(A, t, 2.f * B), t, C));
-  }
-  return m;
-}
 
 // Whitening map of one primitive: x -> diag(1 / exp(ls)) R^T x as a 3x3 matrix (row-major), its centre, the
 // largest inverse scale.  Built once per primitive, used for every tile of its rectangle.
@@ -295,55 +280,65 @@ __device__ __forceinline__ V3 whiten(const PrimWhiten& w, float x, float y, floa
   return r;
 }
 
-// True only when no ray of the tile's rectangle can reach decay > thr against this primitive, i.e. when
-// every such line stays outside the ellipsoid r^2 <= K0 = -2 ln thr.  In the primitive's whitened frame
-// (rotate by R^T, divide axis k by exp(ls_k)) the ellipsoid is the sphere of radius sqrt(K0) around the
-// origin and a line from x with direction e meets it iff |x cross e|^2 <= K0 |e|^2.  Both sides are
-// quadratic in (alpha, beta), so q = |x cross e|^2 - K |e|^2 is minimised exactly over the rectangle
-// (stationary point, four edges).  K carries a 0.2 % margin and tol bounds the rounding of this test and of
-// hit_test (which works in world space, where a position error of a few ulps of |c - o| is magnified by the
-// largest inverse scale); both are orders of magnitude above the error of the approximate divisions and
-// square roots used here.  So a rejected pair is one hit_test rejects for every pixel of the tile, and the
-// rendered result does not depend on the pre-test.  Any NaN makes the test answer false.
-__device__ __forceinline__ bool tile_surely_misses(const PrimWhiten& pw, const TileFrame& f, float K0) {
-  if (!(f.a0 <= f.a1)) return false;
-  const float vx = pw.cx - f.ox, vy = pw.cy - f.oy, vz = pw.cz - f.oz;
+// What a primitive's threshold ellipsoid r^2 <= K cuts out of the tangent plane: the lines from o that meet it form the
+// ellipse (z - z0)^T A (z - z0) <= rho around z0.  In the primitive's whitened frame (rotate by R^T, divide axis k by
+// exp(ls_k)) the ellipsoid is a sphere of radius sqrt(K) around the origin, and the line from x with direction e meets it
+// iff |x cross e|^2 <= K |e|^2.  The coordinates are taken relative to the direction of the centre, for which the cross
+// product vanishes, so nothing cancels.  K carries a margin of 0.4 % plus twice the bound on hit_test's rounding that the
+// hit pass derives (hit_form).  never = the ellipse does not exist (centre beside or behind the plane, origin inside,
+// anything not finite): such a primitive is never rejected.
+struct __align__(16) PlaneEllipse { float zx, zy, a11, a12, a22, r1, r2, rho; };     // r1 = a12 / a22, r2 = a12 / a11
+
+__device__ __forceinline__ PlaneEllipse plane_ellipse(const Geom& g, const FramePlane& f, float K0) {
+  PlaneEllipse e;
+  e.zx = e.zy = e.a11 = e.a12 = e.a22 = e.r1 = e.r2 = 0.f;
+  e.rho = __int_as_float(0x7f800000);                       // no value exceeds it: never rejected
+  const PrimWhiten pw = make_whiten(g);
+  const float vx = g.cx - f.ox, vy = g.cy - f.oy, vz = g.cz - f.oz;
+  const float va = vx * f.ax + vy * f.ay + vz * f.az;
+  const float dist = sqrtf(vx * vx + vy * vy + vz * vz);
+  if (!(va > 0.1f * dist) || !(dist > 0.f)) return e;
+  const float rva = 1.f / va;
+  const float ac = (vx * f.ux + vy * f.uy + vz * f.uz) * rva, bc = (vx * f.vx + vy * f.vy + vz * f.vz) * rva;
   const V3 x = whiten(pw, vx, vy, vz);
-  const V3 e0 = whiten(pw, f.ax, f.ay, f.az);
-  const V3 e1 = whiten(pw, f.ux, f.uy, f.uz);
-  const V3 e2 = whiten(pw, f.vx, f.vy, f.vz);
-  const V3 w0 = {x.y * e0.z - x.z * e0.y, x.z * e0.x - x.x * e0.z, x.x * e0.y - x.y * e0.x};
+  const V3 ec = {x.x * rva, x.y * rva, x.z * rva};          // direction of the centre: a + ac u + bc v
+  const V3 e1 = whiten(pw, f.ux, f.uy, f.uz), e2 = whiten(pw, f.vx, f.vy, f.vz);
   const V3 w1 = {x.y * e1.z - x.z * e1.y, x.z * e1.x - x.x * e1.z, x.x * e1.y - x.y * e1.x};
   const V3 w2 = {x.y * e2.z - x.z * e2.y, x.z * e2.x - x.x * e2.z, x.x * e2.y - x.y * e2.x};
-  const float K = K0 * 1.002f;
-  const float e00 = e0.x * e0.x + e0.y * e0.y + e0.z * e0.z;
-  const float e11 = e1.x * e1.x + e1.y * e1.y + e1.z * e1.z;
-  const float e22 = e2.x * e2.x + e2.y * e2.y + e2.z * e2.z;
-  const float a11 = (w1.x * w1.x + w1.y * w1.y + w1.z * w1.z) - K * e11;
-  const float a22 = (w2.x * w2.x + w2.y * w2.y + w2.z * w2.z) - K * e22;
+  const float S = fabsf(vx) + fabsf(vy) + fabsf(vz) + fabsf(f.ox) + fabsf(f.oy) + fabsf(f.oz);
+  const float K = K0 * 1.004f + 2e-5f * sqrtf(K0) * S * pw.ismax;
+  const float a11 = (w1.x * w1.x + w1.y * w1.y + w1.z * w1.z) - K * (e1.x * e1.x + e1.y * e1.y + e1.z * e1.z);
+  const float a22 = (w2.x * w2.x + w2.y * w2.y + w2.z * w2.z) - K * (e2.x * e2.x + e2.y * e2.y + e2.z * e2.z);
   const float a12 = (w1.x * w2.x + w1.y * w2.y + w1.z * w2.z) - K * (e1.x * e2.x + e1.y * e2.y + e1.z * e2.z);
-  const float b1 = (w0.x * w1.x + w0.y * w1.y + w0.z * w1.z) - K * (e0.x * e1.x + e0.y * e1.y + e0.z * e1.z);
-  const float b2 = (w0.x * w2.x + w0.y * w2.y + w0.z * w2.z) - K * (e0.x * e2.x + e0.y * e2.y + e0.z * e2.z);
-  const float c0 = (w0.x * w0.x + w0.y * w0.y + w0.z * w0.z) - K * e00;
-  if (!(fabsf(a11) + fabsf(a22) + fabsf(a12) + fabsf(b1) + fabsf(b2) + fabsf(c0) < 3.0e38f)) return false;
-  if (c0 <= 0.f) return false;   // the tile's central direction already reaches the ellipsoid
-  // edges alpha = a0 / a1 (quadratics in beta) and beta = b0 / b1 (quadratics in alpha)
-  float m = quad_min_1d(a22, fmaf(a12, f.a0, b2), fmaf(fmaf(a11, f.a0, 2.f * b1), f.a0, c0), f.b0, f.b1);
-  m = fminf(m, quad_min_1d(a22, fmaf(a12, f.a1, b2), fmaf(fmaf(a11, f.a1, 2.f * b1), f.a1, c0), f.b0, f.b1));
-  m = fminf(m, quad_min_1d(a11, fmaf(a12, f.b0, b1), fmaf(fmaf(a22, f.b0, 2.f * b2), f.b0, c0), f.a0, f.a1));
-  m = fminf(m, quad_min_1d(a11, fmaf(a12, f.b1, b1), fmaf(fmaf(a22, f.b1, 2.f * b2), f.b1, c0), f.a0, f.a1));
+  const float b1 = -K * (ec.x * e1.x + ec.y * e1.y + ec.z * e1.z), b2 = -K * (ec.x * e2.x + ec.y * e2.y + ec.z * e2.z);
+  const float c0 = -K * (ec.x * ec.x + ec.y * ec.y + ec.z * ec.z);
   const float det = a11 * a22 - a12 * a12;
-  if (a11 > 0.f && det > 0.f) {
-    const float rdet = __fdividef(1.f, det);
-    const float al = (a12 * b2 - a22 * b1) * rdet, be = (a12 * b1 - a11 * b2) * rdet;
-    if (al >= f.a0 && al <= f.a1 && be >= f.b0 && be <= f.b1) m = fminf(m, fmaf(b1, al, fmaf(b2, be, c0)));
-  }
-  const float dist = sqrtf(vx * vx + vy * vy + vz * vz);
-  // largest |e| over the rectangle
-  const float emax = sqrtf(e00) + fmaxf(fabsf(f.a0), fabsf(f.a1)) * sqrtf(e11) +
-                     fmaxf(fabsf(f.b0), fabsf(f.b1)) * sqrtf(e22);
-  const float tol = (2e-5f * sqrtf(K0) * dist * pw.ismax + 1e-4f * K0) * emax * emax;
-  return m > tol;
+  // (the forms lose their digits where the origin comes close to the ellipsoid)
+  if (!(a11 > 0.1f * K * (e1.x * e1.x + e1.y * e1.y + e1.z * e1.z)) || !(a22 > 0.1f * K * (e2.x * e2.x + e2.y * e2.y + e2.z * e2.z)) ||
+      !(det > 1e-3f * a11 * a22))
+    return e;
+  const float rdet = 1.f / det;
+  const float zx = (a12 * b2 - a22 * b1) * rdet, zy = (a12 * b1 - a11 * b2) * rdet;
+  const float rho = -(b1 * zx + b2 * zy) - c0;
+  if (!(rho > 0.f) || !(rho < 1e30f) || !(fabsf(zx) + fabsf(zy) < 1e3f)) return e;
+  e.zx = ac + zx; e.zy = bc + zy;
+  e.a11 = a11; e.a12 = a12; e.a22 = a22;
+  e.r1 = a12 / a22; e.r2 = a12 / a11;
+  e.rho = rho * 1.001f;
+  return e;
+}
+
+// The smallest value of the ellipse's form over the rectangle r = (a0, a1, b0, b1), relative to its centre: attained at the
+// centre, or on an edge that faces it.  Above rho no ray of the tile can hit (NaNs answer false).  The rectangle is widened
+// by the rounding of the centre's coordinates.
+__device__ __forceinline__ bool ellipse_misses(const float4 z /* zx zy a11 a12 */, const float4 w /* a22 r1 r2 rho */, const float4 r) {
+  const float pad = 1e-6f * (1.f + fabsf(z.x) + fabsf(z.y));
+  const float l1 = r.x - z.x - pad, h1 = r.y - z.x + pad, l2 = r.z - z.y - pad, h2 = r.w - z.y + pad;
+  const float xs = fminf(fmaxf(0.f, l1), h1), ys = fminf(fmaxf(0.f, l2), h2);
+  const float y1 = fminf(fmaxf(-w.y * xs, l2), h2), x2 = fminf(fmaxf(-w.z * ys, l1), h1);
+  const float f1 = z.z * xs * xs + (2.f * z.w * xs + w.x * y1) * y1;
+  const float f2 = z.z * x2 * x2 + (2.f * z.w * x2 + w.x * ys) * ys;
+  return fminf(f1, f2) > w.w && r.x == r.x;
 }
 
 __device__ __forceinline__ V3 load3(const float* __restrict__ p, int64_t i) {

@@ -57,7 +57,8 @@ struct Scratch {
   int32_t* px_off;       // [P+2] their exclusive prefix
   uint32_t* used32;      // [2*max_pairs] consumed-record mask halves per pair (when the caller gives none)
   int32_t* active[2];    // [T] each
-  TileFrame* tile_frame; // [T] ray frame of every tile (tile pre-test of the fused frame path)
+  FramePlane* plane;     // tangent plane of the frame, and
+  float4* tile_rect;     // [T] every tile's rectangle in it (tile pre-test of the fused frame path)
   int32_t* tile_len;     // [T] candidates per tile that the wave kernels traverse
   int32_t* counters;     // [kNumCounters]
   int64_t max_work;
@@ -108,7 +109,8 @@ inline Scratch carve_scratch(void* base, int n, int W, int H, int ts, int64_t ma
   s.active[0] = (int32_t*)take(4 * T);
   s.active[1] = (int32_t*)take(4 * T);
   s.counters = (int32_t*)take(4 * kNumCounters);
-  s.tile_frame = (TileFrame*)take(64 * T);
+  s.plane = (FramePlane*)take(sizeof(FramePlane));
+  s.tile_rect = (float4*)take(16 * T);
   s.tile_len = (int32_t*)take(4 * T);
   s.bytes = off;
   return s;

@@ -73,14 +73,14 @@ __global__ void __launch_bounds__(256) k_clear_used(const int32_t* __restrict__ 
 
 // ------------------------------------------------------------------------- frame begin ----
 // The fused frame path starts with one launch that prepares everything the chain behind it reads: unit ray directions
-// (from the caller's raw ones, when given), the ray frame of every tile for the binning pre-test, pixel state and output
+// (from the caller's raw ones, when given), the tiles' rectangles in the tangent plane for the binning pre-test, pixel state and output
 // image, the per-primitive counts, the binning's corner array and fill counters, the tile lists' cursors and the wave
 // counters, the status block.  (One warp per tile, two pixels per lane; the flat arrays by all threads.)  It replaces a
 // normalising launch, two preparing launches and four memsets.
 struct BeginArgs {
   const float* rays_o; const float* rays_raw; float* rays_d;   // rays_raw null: rays_d already holds unit directions
   int W, H, ntx, T;
-  TileFrame* frames; int32_t* fill; int32_t* zero; int64_t zero_words;     // corner array (or tile counts) of the binning
+  FramePlane* plane; float4* tile_rect; int32_t* fill; int32_t* zero; int64_t zero_words;     // corner array (or tile counts) of the binning
   float4* px_state; float2* px_depth; float* rgb; float* alpha; float* depth_t; float bgr, bgg, bgb;
   int32_t* active0; int32_t* counters; int64_t cnt_words; int32_t* prim_cnt;
   int32_t* status;                                             // null: the caller has reset it
@@ -96,89 +96,71 @@ __global__ void __launch_bounds__(256) k_frame_begin(const BeginArgs a) {
   if (blockIdx.x == 0 && threadIdx.x < kNumCounters)
     a.counters[threadIdx.x] = threadIdx.x == kCtrActive0 ? a.T : 0;
   if (a.status && blockIdx.x == 0 && threadIdx.x < MLPSP_STATUS_WORDS) a.status[threadIdx.x] = 0;
+  // the tangent plane (every thread computes the same one): around the central ray, u along the central image row
+  FramePlane f;
+  {
+    const int64_t row = (int64_t)(a.H / 2) * a.W;
+    const float* rays = a.rays_raw ? a.rays_raw : a.rays_d;
+    auto ray = [&](int x) {
+      const V3 d = {rays[(row + x) * 3], rays[(row + x) * 3 + 1], rays[(row + x) * 3 + 2]};
+      const float r = rsqrtf(d.x * d.x + d.y * d.y + d.z * d.z);
+      return V3{d.x * r, d.y * r, d.z * r};
+    };
+    const V3 o = load3(a.rays_o, row + a.W / 2), c = ray(a.W / 2), lft = ray(0), rgt = ray(a.W - 1);
+    float ux = rgt.x - lft.x, uy = rgt.y - lft.y, uz = rgt.z - lft.z;
+    if (!(ux * ux + uy * uy + uz * uz > 1e-10f)) {      // a column of pixels: any axis
+      ux = fabsf(c.x) < 0.57f ? 1.f : 0.f; uy = fabsf(c.x) < 0.57f ? 0.f : 1.f; uz = 0.f;
+    }
+    const float ua = ux * c.x + uy * c.y + uz * c.z;
+    ux -= ua * c.x; uy -= ua * c.y; uz -= ua * c.z;
+    const float r = rsqrtf(ux * ux + uy * uy + uz * uz);
+    f.ox = o.x; f.oy = o.y; f.oz = o.z; f.ax = c.x; f.ay = c.y; f.az = c.z;
+    f.ux = ux * r; f.uy = uy * r; f.uz = uz * r;
+    f.vx = f.ay * f.uz - f.az * f.uy; f.vy = f.az * f.ux - f.ax * f.uz; f.vz = f.ax * f.uy - f.ay * f.ux;
+    f.pad0 = f.pad1 = f.pad2 = f.pad3 = 0.f;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *a.plane = f;
+  }
   for (int tile = blockIdx.x * 8 + warp; tile < a.T; tile += gridDim.x * 8) {
     const int tx = tile % a.ntx, ty = tile / a.ntx;
-    V3 dd[2], o0;
     bool same = true;
-    float sx = 0.f, sy = 0.f, sz = 0.f;
+    float a0 = 3e38f, a1 = -3e38f, b0 = 3e38f, b1 = -3e38f;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int k = h * 32 + lane;
       const int x = tx * 8 + (k & 7), y = ty * 8 + (k >> 3);
-      const bool valid = x < a.W && y < a.H;
-      // pixels past the image edge repeat the edge pixel: they add no new ray
-      const int64_t pix = (int64_t)min(y, a.H - 1) * a.W + min(x, a.W - 1);
+      if (x >= a.W || y >= a.H) continue;
+      const int64_t pix = (int64_t)y * a.W + x;
       const V3 o = load3(a.rays_o, pix);
-      if (h == 0) { o0.x = __shfl_sync(0xffffffffu, o.x, 0); o0.y = __shfl_sync(0xffffffffu, o.y, 0); o0.z = __shfl_sync(0xffffffffu, o.z, 0); }
       V3 d;
       if (a.rays_raw) {
         d = load3(a.rays_raw, pix);
         const float nrm = fmaxf(__fsqrt_rn(ffma(d.z, d.z, ffma(d.y, d.y, fmul(d.x, d.x)))), 1e-12f);
         d = V3{fdiv(d.x, nrm), fdiv(d.y, nrm), fdiv(d.z, nrm)};
-        if (valid) { a.rays_d[pix * 3] = d.x; a.rays_d[pix * 3 + 1] = d.y; a.rays_d[pix * 3 + 2] = d.z; }
+        a.rays_d[pix * 3] = d.x; a.rays_d[pix * 3 + 1] = d.y; a.rays_d[pix * 3 + 2] = d.z;
       } else {
         d = V3{a.rays_d[pix * 3], a.rays_d[pix * 3 + 1], a.rays_d[pix * 3 + 2]};
       }
-      dd[h] = d;
-      same = same && o.x == o0.x && o.y == o0.y && o.z == o0.z;
-      sx += d.x; sy += d.y; sz += d.z;
-      if (valid) {
-        a.px_state[pix] = make_float4(0.f, 0.f, 0.f, 1.f);
-        a.rgb[pix * 3] = a.bgr; a.rgb[pix * 3 + 1] = a.bgg; a.rgb[pix * 3 + 2] = a.bgb;
-        a.alpha[pix] = 0.f;
-        if (a.depth_t) { a.depth_t[pix] = 0.f; a.px_depth[pix] = make_float2(0.f, 0.f); }
-      }
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      sx += __shfl_xor_sync(0xffffffffu, sx, off);
-      sy += __shfl_xor_sync(0xffffffffu, sy, off);
-      sz += __shfl_xor_sync(0xffffffffu, sz, off);
-    }
-    const float inv = rsqrtf(sx * sx + sy * sy + sz * sz);
-    const float ax = sx * inv, ay = sy * inv, az = sz * inv;
-    // u: the image's x direction made orthogonal to a (direction of pixel 7 minus pixel 0 of the first row);
-    // a fixed axis when the tile is one pixel wide
-    float ux = __shfl_sync(0xffffffffu, dd[0].x, 7) - __shfl_sync(0xffffffffu, dd[0].x, 0);
-    float uy = __shfl_sync(0xffffffffu, dd[0].y, 7) - __shfl_sync(0xffffffffu, dd[0].y, 0);
-    float uz = __shfl_sync(0xffffffffu, dd[0].z, 7) - __shfl_sync(0xffffffffu, dd[0].z, 0);
-    if (!(ux * ux + uy * uy + uz * uz > 1e-12f)) {
-      ux = fabsf(ax) < 0.57f ? 1.f : 0.f; uy = fabsf(ax) < 0.57f ? 0.f : 1.f; uz = 0.f;
-    }
-    const float ua = ux * ax + uy * ay + uz * az;
-    ux -= ua * ax; uy -= ua * ay; uz -= ua * az;
-    const float uinv = rsqrtf(ux * ux + uy * uy + uz * uz);
-    ux *= uinv; uy *= uinv; uz *= uinv;
-    const float vx = ay * uz - az * uy, vy = az * ux - ax * uz, vz = ax * uy - ay * ux;
-    float a0 = 3e38f, a1 = -3e38f, b0 = 3e38f, b1 = -3e38f, cmin = 3e38f;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const float da = dd[h].x * ax + dd[h].y * ay + dd[h].z * az;
-      const float al = (dd[h].x * ux + dd[h].y * uy + dd[h].z * uz) / da;
-      const float be = (dd[h].x * vx + dd[h].y * vy + dd[h].z * vz) / da;
-      const float len2 = dd[h].x * dd[h].x + dd[h].y * dd[h].y + dd[h].z * dd[h].z;
-      cmin = fminf(cmin, da * rsqrtf(len2));
-      same = same && (al == al) && (be == be) && fabsf(al) < 1e6f && fabsf(be) < 1e6f;
+      const float da = d.x * f.ax + d.y * f.ay + d.z * f.az, len2 = d.x * d.x + d.y * d.y + d.z * d.z;
+      const float al = (d.x * f.ux + d.y * f.uy + d.z * f.uz) / da, be = (d.x * f.vx + d.y * f.vy + d.z * f.vz) / da;
+      same = same && o.x == f.ox && o.y == f.oy && o.z == f.oz && da * rsqrtf(len2) > 0.26f && fabsf(al) < 1e3f && fabsf(be) < 1e3f;
       a0 = fminf(a0, al); a1 = fmaxf(a1, al); b0 = fminf(b0, be); b1 = fmaxf(b1, be);
+      a.px_state[pix] = make_float4(0.f, 0.f, 0.f, 1.f);
+      a.rgb[pix * 3] = a.bgr; a.rgb[pix * 3 + 1] = a.bgg; a.rgb[pix * 3 + 2] = a.bgb;
+      a.alpha[pix] = 0.f;
+      if (a.depth_t) { a.depth_t[pix] = 0.f; a.px_depth[pix] = make_float2(0.f, 0.f); }
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
       a0 = fminf(a0, __shfl_xor_sync(0xffffffffu, a0, off)); a1 = fmaxf(a1, __shfl_xor_sync(0xffffffffu, a1, off));
       b0 = fminf(b0, __shfl_xor_sync(0xffffffffu, b0, off)); b1 = fmaxf(b1, __shfl_xor_sync(0xffffffffu, b1, off));
-      cmin = fminf(cmin, __shfl_xor_sync(0xffffffffu, cmin, off));
     }
     same = __all_sync(0xffffffffu, same);
-    const bool ok = same && cmin > 0.5f && (ax == ax) && (ux == ux) && fabsf(o0.x) < 1e30f && fabsf(o0.y) < 1e30f &&
-                    fabsf(o0.z) < 1e30f;
     if (lane == 0) {
-      TileFrame f;
-      // inflate the rectangle: rounding of the coordinates themselves
-      const float pa = 1e-5f + 1e-3f * (a1 - a0), pb = 1e-5f + 1e-3f * (b1 - b0);
-      f.ox = o0.x; f.oy = o0.y; f.oz = o0.z; f.ax = ax; f.ay = ay; f.az = az;
-      f.ux = ux; f.uy = uy; f.uz = uz; f.vx = vx; f.vy = vy; f.vz = vz;
-      f.a0 = ok ? a0 - pa : 1.f; f.a1 = ok ? a1 + pa : -1.f;
-      f.b0 = b0 - pb; f.b1 = b1 + pb;
-      a.frames[tile] = f;
+      // inflate the rectangle: rounding of the coordinates and of the plane's frame
+      const float pa = 2e-6f * (1.f + fabsf(a0) + fabsf(a1)) * (1.f + fabsf(a0) + fabsf(a1) + fabsf(b0) + fabsf(b1)) + 1e-3f * (a1 - a0);
+      const float pb = 2e-6f * (1.f + fabsf(b0) + fabsf(b1)) * (1.f + fabsf(a0) + fabsf(a1) + fabsf(b0) + fabsf(b1)) + 1e-3f * (b1 - b0);
+      const float nan = __int_as_float(0x7fc00000);
+      a.tile_rect[tile] = same ? make_float4(a0 - pa, a1 + pa, b0 - pb, b1 + pb) : make_float4(nan, nan, nan, nan);
       a.fill[tile] = 0;
       a.active0[tile] = tile;
     }
@@ -190,7 +172,7 @@ int launch_frame_begin(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scrat
   BeginArgs a;
   a.rays_o = fr->rays_o; a.rays_raw = rays_raw; a.rays_d = const_cast<float*>(fr->rays_d);
   a.W = fr->width; a.H = fr->height; a.ntx = (fr->width + 7) / 8; a.T = num_tiles(fr->width, fr->height, 8);
-  a.frames = s.tile_frame; a.fill = s.tile_len;
+  a.plane = s.plane; a.tile_rect = s.tile_rect; a.fill = s.tile_len;
   const bool corners = bin_uses_corners(fr);
   a.zero = corners ? s.tile_diff : s.tile_cnt;
   a.zero_words = corners ? (int64_t)(a.ntx + 1) * ((fr->height + 7) / 8 + 1) : a.T + 1;
@@ -652,90 +634,6 @@ __device__ __forceinline__ float4 tetra_gates(const Hit& h, float lsx, float lsy
   return make_float4(e0 * inv, e1 * inv, e2 * inv, e3 * inv);
 }
 
-// One CTA per active tile.  Pairs with hits reserve their primitive-major range (one atomic per pair),
-// then threads walk the tile's RECORDS (not its pixels): record r of the tile-wave belongs to the pair
-// found by binary search in the slot prefix, and to the pixel of the (r - prefix)-th set mask bit.
-__global__ void __launch_bounds__(256) k_fill(
-    const float* __restrict__ rays_o, const float* __restrict__ rays_d, const float4* __restrict__ geom,
-    const int32_t* __restrict__ tile_offsets, const int32_t* __restrict__ tile_len, const int32_t* __restrict__ sorted_prims, int W, int H, int ntx,
-    float thr, const int32_t* __restrict__ active, const int32_t* __restrict__ active_count, int lo, int hi,
-    const uint32_t* __restrict__ masks32, const uint32_t* __restrict__ pair_base,
-    int32_t* __restrict__ prim_pos, RecIn* __restrict__ rec_in,
-    float* __restrict__ rec_t, float4* __restrict__ rec_gate, float beta, float tau, int exact_hits, int ref_arith,
-    const int32_t* __restrict__ status) {
-  chain_wait();
-  chain_release();
-  __shared__ uint32_t s_m[2][kWinMax];
-  __shared__ int32_t s_pref[kWinMax + 1];   // slot of the pair's first record, relative to the tile-wave
-  __shared__ int32_t s_q0[kWinMax];         // primitive-major position of the pair's first record
-  __shared__ float s_ray[64][6];
-  if (status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
-  const int n_active = *active_count;
-  const int tid = threadIdx.x;
-  for (int slot_i = blockIdx.x; slot_i < n_active; slot_i += gridDim.x) {
-  const int tile = active[slot_i];
-  const int s = tile_offsets[tile];
-  const int len = tile_len[tile];
-  const int wlo = min(lo, len), whi = min(hi, len);
-  const int nwin = whi - wlo;
-  if (nwin <= 0) continue;
-  if (tid < 64) {
-    const TilePix tp = tile_pixel(tile, tid, ntx, W, H);
-    V3 o = {0.f, 0.f, 0.f}, d = {0.f, 0.f, 0.f};
-    if (tp.valid) { o = load3(rays_o, tp.pix); d = load3(rays_d, tp.pix); }
-    s_ray[tid][0] = o.x; s_ray[tid][1] = o.y; s_ray[tid][2] = o.z;
-    s_ray[tid][3] = d.x; s_ray[tid][4] = d.y; s_ray[tid][5] = d.z;
-  }
-  const uint32_t slot_base = pair_base[s + wlo];
-  for (int j = tid; j < nwin; j += 256) {
-    const uint32_t m0 = masks32[2 * (size_t)(s + wlo + j)], m1 = masks32[2 * (size_t)(s + wlo + j) + 1];
-    s_m[0][j] = m0; s_m[1][j] = m1;
-    s_pref[j] = (int32_t)(pair_base[s + wlo + j] - slot_base);
-    const int c = __popc(m0) + __popc(m1);
-    int q0 = 0;
-    if (c > 0) {
-      const int p = sorted_prims[s + wlo + j];
-      q0 = atomicAdd(prim_pos + p, c);
-    }
-    s_q0[j] = q0;
-    if (j == nwin - 1) s_pref[nwin] = s_pref[j] + c;
-  }
-  __syncthreads();
-  const int total = s_pref[nwin];
-  for (int r = tid; r < total; r += 256) {
-    int a = 0, b = nwin - 1;                 // largest j with s_pref[j] <= r (empty pairs share a prefix
-    while (a < b) {                          //  with their successor, so the last such j is the owner)
-      const int mid = (a + b + 1) >> 1;
-      if (s_pref[mid] <= r) a = mid; else b = mid - 1;
-    }
-    const int j = a, k = r - s_pref[a];
-    const uint32_t m0 = s_m[0][j], m1 = s_m[1][j];
-    const int c0 = __popc(m0);
-    const int px = (k < c0) ? nth_set_bit(m0, k) : 32 + nth_set_bit(m1, k - c0);
-    const int p = sorted_prims[s + wlo + j];
-    const V3 o = {s_ray[px][0], s_ray[px][1], s_ray[px][2]}, d = {s_ray[px][3], s_ray[px][4], s_ray[px][5]};
-    Hit ht;
-    // the pair is known to hit: values only.  The feature gates divide the local offset by the scales, which
-    // magnifies its rounding, so frames with features keep the decision-grade arithmetic.
-    // Per-pixel ordering sorts by t: its order must be the decision-grade one too.
-    if (ref_arith) hit_test_ref(load_geom_ref(geom, p), o, d, thr, ht);    // the reference kernels' own values
-    else if (rec_gate || exact_hits) hit_test(load_geom(geom, p), o, d, thr, ht);
-    else hit_values_fast(load_geom(geom, p), o, d, ht);
-    const uint32_t slot = slot_base + (uint32_t)r;
-    RecIn rec;
-    rec.rdx = d.x; rec.rdy = d.y; rec.rdz = d.z; rec.dx = ht.dx; rec.dy = ht.dy; rec.dz = ht.dz;
-    rec.decay = ht.decay; rec.slot = slot;
-    rec_in[s_q0[j] + k] = rec;
-    if (rec_t) rec_t[slot] = ht.t;
-    if (rec_gate) {
-      const float4 ls = __ldg(geom + (size_t)p * 4 + 3);
-      rec_gate[slot] = tetra_gates(ht, ls.x, ls.y, ls.z, beta, tau);
-    }
-  }
-  __syncthreads();   // shared arrays are reused by the next tile of this CTA
-  }
-}
-
 // Transpose of the 32 x 32 bit matrix whose row l is lane l's word.
 __device__ __forceinline__ uint32_t transpose32(uint32_t w) {
   const int lane = threadIdx.x & 31;
@@ -747,6 +645,168 @@ __device__ __forceinline__ uint32_t transpose32(uint32_t w) {
     m ^= m << (s >> 1);
   }
   return w;
+}
+
+// One warp per chunk of 32 candidates of an active tile; nothing is shared between warps.  A candidate's lane reserves its
+// records' primitive-major range (one atomic per pair with a hit) and prepares its geometry once: rotation, M R^T v and v
+// for the tile's common origin.  The records of the chunk are then listed (pixel lanes walk their own hits, as in
+// compositing: the masks transposed) and dealt to the lanes, so every lane computes a record whatever the hits' pattern,
+// and neighbouring lanes write neighbouring records.  About 100 instructions per record where a search for the record's
+// pair and pixel, and the full geometry per record, took 350 (100k frame, 10.6 M records: 193 -> 135 us).
+// MODE 0: values only (no decision hangs on them: hardware reciprocal and exponential); 1: hit_test's own values, for the
+// feature gates, which divide the local offset by the scales, and for per-pixel ordering, which sorts by t; 2: the
+// reference kernels' arithmetic.
+constexpr int kFillWarps = 8;
+struct FillSmem { float4 geo[32][5]; float4 ray[32]; uint16_t list[1024]; };
+
+struct FillArgs {
+  const float* rays_o; const float* rays_d; const float4* geom;
+  const int32_t* tile_offsets; const int32_t* tile_len; const int32_t* sorted_prims; int W, H, ntx; float thr;
+  const int32_t* active; const int32_t* active_count; int lo, hi;
+  const uint2* masks; const uint32_t* pair_base; int32_t* prim_pos; float4* rec_in; float* rec_t; float4* rec_gate;
+  float beta, tau; int plain; const int32_t* status;      // plain: MODE 0 without the shared per-candidate geometry
+  int width, chunks, halves;                              // candidates per unit, units per window and half, 2: a unit is one half
+};
+
+template <int MODE>
+__global__ void __launch_bounds__(32 * kFillWarps, 4) k_fill(const FillArgs a) {
+  chain_wait();
+  chain_release();
+  __shared__ FillSmem s_all[kFillWarps];
+  if (a.status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
+  FillSmem& sm = s_all[warp];
+  const uint32_t lt = (1u << lane) - 1u;
+  const int per_tile = a.chunks * a.halves, units = *a.active_count * per_tile;
+  for (int unit = blockIdx.x * wpb + warp; unit < units; unit += gridDim.x * wpb) {
+    const int slot_i = per_tile == 1 ? unit : unit / per_tile;
+    const int part = unit - slot_i * per_tile, ch = a.halves == 2 ? part >> 1 : part;
+    const int h0 = a.halves == 2 ? part & 1 : 0, h1 = a.halves == 2 ? h0 + 1 : 2;
+    const int tile = a.active[slot_i];
+    const int s = a.tile_offsets[tile], len = a.tile_len[tile];
+    const int j0 = min(a.lo, len) + ch * a.width, whi = min(min(a.hi, len), j0 + a.width);
+    if (j0 >= whi) continue;
+    uint2 m = make_uint2(0u, 0u);
+    int p = 0, c = 0, q0 = 0;
+    uint32_t first = 0u;
+    if (j0 + lane < whi) {
+      m = a.masks[(size_t)s + j0 + lane];
+      first = a.pair_base[(size_t)s + j0 + lane];
+      c = (h0 == 0 ? __popc(m.x) : 0) + (h1 == 2 ? __popc(m.y) : 0);
+      if (c > 0) {
+        p = a.sorted_prims[s + j0 + lane];
+        q0 = atomicAdd(a.prim_pos + p, c);
+      }
+    }
+    if (!__any_sync(0xffffffffu, c > 0)) continue;
+    // rays of the tile's two halves; one origin is the usual case
+    V3 o[2], d[2];
+    bool same = true;
+    V3 o0 = {0.f, 0.f, 0.f};
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const TilePix tp = tile_pixel(tile, h * 32 + lane, a.ntx, a.W, a.H);
+      o[h] = d[h] = V3{0.f, 0.f, 0.f};
+      if (tp.valid) { o[h] = load3(a.rays_o, tp.pix); d[h] = load3(a.rays_d, tp.pix); }
+      if (h == 0) o0 = V3{__shfl_sync(0xffffffffu, o[0].x, 0), __shfl_sync(0xffffffffu, o[0].y, 0), __shfl_sync(0xffffffffu, o[0].z, 0)};
+      same = same && (!tp.valid || (o[h].x == o0.x && o[h].y == o0.y && o[h].z == o0.z));
+    }
+    const bool uni = MODE == 0 && !a.plain && __all_sync(0xffffffffu, same);
+    __syncwarp();
+    if (uni && c > 0) {
+      const Geom g = load_geom(a.geom, p);
+      // rows of R^T: R^T applied to the axes gives its columns
+      const V3 c0 = rot_conj_fast(g.qw, g.qx, g.qy, g.qz, V3{1.f, 0.f, 0.f}), c1 = rot_conj_fast(g.qw, g.qx, g.qy, g.qz, V3{0.f, 1.f, 0.f}),
+               c2 = rot_conj_fast(g.qw, g.qx, g.qy, g.qz, V3{0.f, 0.f, 1.f});
+      const V3 v = {g.cx - o0.x, g.cy - o0.y, g.cz - o0.z};
+      const V3 vl = rot_conj_fast(g.qw, g.qx, g.qy, g.qz, v);
+      sm.geo[lane][0] = make_float4(c0.x, c1.x, c2.x, vl.x * g.mx);
+      sm.geo[lane][1] = make_float4(c0.y, c1.y, c2.y, vl.y * g.my);
+      sm.geo[lane][2] = make_float4(c0.z, c1.z, c2.z, vl.z * g.mz);
+      sm.geo[lane][3] = make_float4(g.mx, g.my, g.mz, 0.f);
+      sm.geo[lane][4] = make_float4(v.x, v.y, v.z, 0.f);
+    }
+    int before = 0;                                       // this unit's records of the candidate in the first half
+    for (int h = h0; h < h1; ++h) {
+      const uint32_t mine = h ? m.y : m.x;
+      const int inc = warp_inclusive_scan(__popc(mine));
+      const int total = __shfl_sync(0xffffffffu, inc, 31), pref = inc - __popc(mine);
+      if (total == 0) continue;
+      // positions of this half's records behind the entries of the list
+      __syncwarp();
+      sm.geo[lane][3].w = __int_as_float(q0 + before - pref);
+      sm.geo[lane][4].w = __int_as_float((int)first + (h ? __popc(m.x) : 0) - pref);
+      before += __popc(mine);
+      const V3 dh = h ? d[1] : d[0], oh = h ? o[1] : o[0];
+      sm.ray[lane] = make_float4(dh.x, dh.y, dh.z, 0.f);
+      uint32_t todo = transpose32(mine);
+      while (__any_sync(0xffffffffu, todo != 0u)) {
+        const int j = todo ? __ffs(todo) - 1 : lane;
+        const uint32_t mj = __shfl_sync(0xffffffffu, mine, j);
+        const int pj = __shfl_sync(0xffffffffu, pref, j);
+        if (todo) sm.list[pj + __popc(mj & lt)] = (uint16_t)(j | (lane << 5));
+        todo &= todo - 1u;
+      }
+      __syncwarp();
+      for (int r = lane; r - lane < total; r += 32) {
+        const bool on = r < total;
+        const int e = on ? sm.list[r] : 0;
+        const int j = e & 31, px = e >> 5;
+        V3 oo = o0;
+        int pj = 0;
+        if (!uni) {        // a warp-wide exchange, so before the lanes part
+          oo = V3{__shfl_sync(0xffffffffu, oh.x, px), __shfl_sync(0xffffffffu, oh.y, px), __shfl_sync(0xffffffffu, oh.z, px)};
+          pj = __shfl_sync(0xffffffffu, p, j);
+        }
+        if (!on) continue;
+        const float4 ray = sm.ray[px];
+        const float4 g3 = sm.geo[j][3], g4 = sm.geo[j][4];
+        const int pos = __float_as_int(g3.w) + r;
+        const uint32_t slot = (uint32_t)(__float_as_int(g4.w) + r);
+        Hit ht;
+        if (MODE == 0 && uni) {
+          const float4 g0 = sm.geo[j][0], g1 = sm.geo[j][1], g2 = sm.geo[j][2];
+          const float lx = g0.x * ray.x + g0.y * ray.y + g0.z * ray.z, ly = g1.x * ray.x + g1.y * ray.y + g1.z * ray.z,
+                      lz = g2.x * ray.x + g2.y * ray.y + g2.z * ray.z;
+          const float denom = lx * lx * g3.x + ly * ly * g3.y + lz * lz * g3.z;
+          const float numer = lx * g0.w + ly * g1.w + lz * g2.w;
+          ht.t = __fdividef(numer, denom);
+          ht.dx = g4.x - ht.t * ray.x; ht.dy = g4.y - ht.t * ray.y; ht.dz = g4.z - ht.t * ray.z;
+          const float qx = g0.x * ht.dx + g0.y * ht.dy + g0.z * ht.dz, qy = g1.x * ht.dx + g1.y * ht.dy + g1.z * ht.dz,
+                      qz = g2.x * ht.dx + g2.y * ht.dy + g2.z * ht.dz;
+          ht.decay = __expf(-0.5f * (qx * qx * g3.x + qy * qy * g3.y + qz * qz * g3.z));
+        } else {
+          const V3 dd = {ray.x, ray.y, ray.z};
+          if (MODE == 2) hit_test_ref(load_geom_ref(a.geom, pj), oo, dd, a.thr, ht);
+          else if (MODE == 1) hit_test(load_geom(a.geom, pj), oo, dd, a.thr, ht);
+          else hit_values_fast(load_geom(a.geom, pj), oo, dd, ht);
+        }
+        // the record's 32 bytes in one store: a full sector
+        asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(a.rec_in + 2 * (size_t)pos), "f"(ray.x), "f"(ray.y),
+                     "f"(ray.z), "f"(ht.dx), "f"(ht.dy), "f"(ht.dz), "f"(ht.decay), "f"(__uint_as_float(slot)) : "memory");
+        if (a.rec_t) a.rec_t[slot] = ht.t;
+        if (MODE != 0 && a.rec_gate) {
+          const float4 ls = __ldg(a.geom + (size_t)pj * 4 + 3);
+          a.rec_gate[slot] = tetra_gates(ht, ls.x, ls.y, ls.z, a.beta, a.tau);
+        }
+      }
+      __syncwarp();
+    }
+  }
+}
+
+static int launch_fill(FillArgs a, bool exact, bool ref_arith, int tiles, int sms, bool idle_tail, cudaStream_t st) {
+  // 16 candidates per warp balance best on large frames (32: 957, 16: 939, 8: 1,000 us for the whole 100k frame); with few
+  // tiles the window is cut finer, so that the SMs get more and shorter warps
+  const bool small = (int64_t)tiles * ((a.hi - a.lo + 15) / 16) < (int64_t)sms * 8;
+  a.width = small ? 8 : 16;
+  a.halves = small ? 2 : 1;
+  a.chunks = (a.hi - a.lo + a.width - 1) / a.width;
+  const int64_t units = (int64_t)tiles * a.chunks * a.halves;
+  const int wpb = units >= sms * 2 * kFillWarps ? kFillWarps : 1;
+  const int grid = (int)std::min<int64_t>((units + wpb - 1) / wpb, idle_tail ? sms : sms * 32);
+  auto* kernel = ref_arith ? k_fill<2> : (exact ? k_fill<1> : k_fill<0>);
+  return cuda_check(launch_chained(kernel, dim3(grid), dim3(32 * wpb), 0, st, a), "fill");
 }
 
 // --------------------------------------------------------------------------- composite ----
@@ -1321,9 +1381,6 @@ int launch_render_sorted(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scr
   // lose 4 % of evaluator time with the second list, 500,000 gain 2 %, 2,000,000 with 64 hidden units gain 21 %).  (Record export keeps one list.)
   const bool split_small = tc_path && !keep && (int64_t)n * 3 > P;
   const int sms = sm_count();
-  // CTAs walk the active-tile list with a grid stride, so a wave with few (or no) live tiles costs a
-  // launch of a few thousand CTAs, not one per tile of the image
-  const int wave_grid = std::min(T, sms * 16);
   // per-pixel ordering: one wave over the whole lists, every pixel live
   const int nw = per_pixel ? 1 : (fr->num_waves > 0 ? fr->num_waves : (int)(sizeof(kDefaultWaves) / sizeof(int)));
   int lo = 0;
@@ -1335,7 +1392,6 @@ int launch_render_sorted(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scr
     const int cur = w & 1, nxt = cur ^ 1;
     // a last wave the caller expects to be idle: one CTA per SM walks whatever is left
     const bool idle_tail = fr->tail_hint == 1 && hi == fr->tile_capacity && w > 0;
-    const int grid_hits = idle_tail ? sms : wave_grid;
     const int grid_comp = idle_tail ? sms : std::min(T, sms * 32);
     const int cap_mlp = idle_tail ? sms : 0;
     const int32_t* act = s.active[cur];
@@ -1352,12 +1408,16 @@ int launch_render_sorted(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scr
     }
     rc = launch_prim_scan(s, n, nullptr, fr->status, st, split_small, w);
     if (rc) return rc;
-    { LaunchScope scope(kKFill, 1, st);
-    launch_chained(k_fill, dim3(grid_hits), dim3(256), 0, st, fr->rays_o, fr->rays_d, (const float4*)sc->geom, fr->tile_offsets, s.tile_len, fr->sorted_prims,
-                              W, H, ntx, fr->threshold, act, act_n, lo, hi, s.masks32, s.pair_base, s.prim_pos,
-                              s.rec_in, (want_t || per_pixel) ? s.rec_t : nullptr,
-                              (want_feat && sc->feat_slots > 1) ? s.rec_gate : nullptr, sc->gate_beta,
-                              sc->gate_tau, per_pixel ? 1 : 0, ref_arith ? 1 : 0, fr->status); }
+    {
+      LaunchScope scope(kKFill, 1, st);
+      float4* gate = (want_feat && sc->feat_slots > 1) ? s.rec_gate : nullptr;
+      const FillArgs fa = {fr->rays_o, fr->rays_d, (const float4*)sc->geom, fr->tile_offsets, s.tile_len, fr->sorted_prims, W, H, ntx,
+                           fr->threshold, act, act_n, lo, hi, reinterpret_cast<const uint2*>(s.masks32), s.pair_base,
+                           s.prim_pos, reinterpret_cast<float4*>(s.rec_in), (want_t || per_pixel) ? s.rec_t : nullptr, gate,
+                           sc->gate_beta, sc->gate_tau, keep ? 1 : 0, fr->status, 0, 0, 0};
+      rc = launch_fill(fa, gate || per_pixel, ref_arith, T, sms, idle_tail, st);
+      if (rc) return rc;
+    }
     if (tc_path)
       rc = launch_mlp_f16(sc, s.rec_in, s.work, s.counters, s.rec_out, keep ? s.rec_ext : nullptr, kOutAlpha,
                           fr->status, st, fr->precision == MLPSP_PRECISION_BF16, cap_mlp, split_small ? s.work_small : nullptr);
@@ -1457,7 +1517,6 @@ int launch_render_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scr
   // views 72.2 -> 65.8 ms of evaluator time)
   const bool split_small = tc_path && (int64_t)n * 20 > P * V;
   const int sms = sm_count();
-  const int wave_grid = std::min(T, sms * 16);
   const int nw = f0->num_waves > 0 ? f0->num_waves : (int)(sizeof(kDefaultWaves) / sizeof(int));
   int lo = 0;
   for (int w = 0; w < nw && lo < f0->tile_capacity; ++w) {
@@ -1467,7 +1526,6 @@ int launch_render_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scr
     MLPSP_REQUIRE(hi - lo <= kWinMax, MLPSP_E_LIMIT, "wave window beyond %d candidates", kWinMax);
     const int cur = w & 1, nxt = cur ^ 1;
     const bool idle_tail = f0->tail_hint == 1 && hi == f0->tile_capacity && w > 0;
-    const int grid_hits = idle_tail ? sms : wave_grid;
     const int grid_comp = idle_tail ? sms : std::min(T, sms * 32);
     const int cap_mlp = idle_tail ? sms : 0;
     int32_t* cnt = lead.prim_cnt + (size_t)(w & 1) * prim_cnt_stride(n);
@@ -1492,10 +1550,12 @@ int launch_render_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scr
       for (int v = 0; v < V; ++v) {
         const mlpsp_frame* fr = frs + v;
         const Scratch& s = ss[v];
-        launch_chained(k_fill, dim3(grid_hits), dim3(256), 0, st, fr->rays_o, fr->rays_d, (const float4*)sc->geom, fr->tile_offsets, s.tile_len, fr->sorted_prims,
-                                          W, H, ntx, f0->threshold, s.active[cur], s.counters + kCtrActive0 + cur, lo, hi, s.masks32,
-                                          s.pair_base, lead.prim_pos, lead.rec_in, nullptr, nullptr, sc->gate_beta,
-                                          sc->gate_tau, 0, ref_arith ? 1 : 0, f0->status);
+        const FillArgs fa = {fr->rays_o, fr->rays_d, (const float4*)sc->geom, fr->tile_offsets, s.tile_len, fr->sorted_prims, W, H, ntx,
+                             f0->threshold, s.active[cur], s.counters + kCtrActive0 + cur, lo, hi,
+                             reinterpret_cast<const uint2*>(s.masks32), s.pair_base, lead.prim_pos, reinterpret_cast<float4*>(lead.rec_in),
+                             nullptr, nullptr, sc->gate_beta, sc->gate_tau, 0, f0->status, 0, 0, 0};
+        rc = launch_fill(fa, false, ref_arith, T, sms, idle_tail, st);
+        if (rc) return rc;
       }
     }
     if (tc_path)
