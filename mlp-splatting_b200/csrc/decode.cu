@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(kDecThreads, 1) k_decode_tc(
       tc_fence_before();
       if (!__syncthreads_and(ok)) { ok = false; break; }
       // rows 0..127 -> columns [0, Ch), rows 52..179 -> [128, 128 + Ch)
-      if (tid == 0) {
+      if (warp == 0 && elect_one()) {
         const uint32_t wb = acquire(gbase);
         if (ok) {
           const uint64_t bd = smem_desc(wb, Ch * 16, 128);
@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(kDecThreads, 1) k_decode_tc(
         bad |= load_input_tile(feat, W, H, Cin, K1, (nt / tiles_x) * kDecTileH, (nt % tiles_x) * kDecTileW, smem + kSmA0,
                                tid - 32, kDecThreads - 32);
       }
-    } else if (tid == 0) {
+    } else if (elect_one()) {
       for (int tap = 0; tap < 9 && ok; ++tap) {
         const int g = gbase + 1 + tap;
         const uint32_t wb = acquire(g);
@@ -444,7 +444,7 @@ __global__ void __launch_bounds__(kDecThreads, 1) k_decode_tc(
     for (int sb = 0; sb < kDecSub; ++sb) { best[sb] = -3.0e38f; arg[sb] = 0; }
     for (int c = 0; c < out_chunks; ++c) {
       const int nc = min(128, n_pad - c * 128);
-      if (tid == 0) {
+      if (warp == 0 && elect_one()) {
         const int g = gbase + 10 + c;
         const uint32_t wb = acquire(g);
         if (ok) {
@@ -535,7 +535,7 @@ __global__ void __launch_bounds__(kDecThreads, 1) k_decode_tc(
     }
   }
 
-  if (!ok && tid == 0) {
+  if (!ok && warp == 0 && elect_one()) {
     atomicOr(status + MLPSP_ST_BITS, MLPSP_ST_TIMEOUT);
     // copies requested but never waited for may still be in flight: give each a bounded chance to land
     // before the shared memory is released

@@ -228,8 +228,8 @@ __global__ void __launch_bounds__(kFtThreads, 2) k_feature_tc(
       fence_async_smem();
       tc_fence_before();
       if (!__syncthreads_and(ok)) { ok = false; break; }
-      if (tid == 0) {
-        tc_fence_after();
+      if (warp == 0) tc_fence_after();
+      if (warp == 0 && elect_one()) {
         const uint32_t a_s = sb + (g & 1) * stage_bytes;
         const uint32_t hi_s = a_s + a_bytes, lo_s = hi_s + P::kCoefBytes;
         const uint64_t bh_desc = smem_desc(hi_s, 1024, 128), bl_desc = smem_desc(lo_s, 1024, 128);

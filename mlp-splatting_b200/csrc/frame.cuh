@@ -59,6 +59,7 @@ struct Scratch {
   int32_t* active[2];    // [T] each
   FramePlane* plane;     // tangent plane of the frame, and
   float4* tile_rect;     // [T] every tile's rectangle in it (tile pre-test of the fused frame path)
+  char* dir_table;       // encoded ray directions (images whose table is at most kDirTableMax)
   int32_t* tile_len;     // [T] candidates per tile that the wave kernels traverse
   int32_t* counters;     // [kNumCounters]
   int64_t max_work;
@@ -72,6 +73,10 @@ inline int num_tiles(int W, int H, int ts) { return ((W + ts - 1) / ts) * ((H + 
 
 constexpr int kScanItems = 4096;  // elements per block of the multi-block scans
 constexpr int kPrimScanItems = 1024;   // primitives per block of the per-primitive scan (256 threads, four each)
+
+// Used while the table fits beside the frame's other streams in the 126 MB L2: every record then reads 80 bytes of it
+constexpr int64_t kDirTableMax = 96ll << 20;
+inline int64_t dir_table_bytes(int W, int H) { return 5120ll * (((W + 7) / 8) * (int64_t)((H + 7) / 8)); }
 
 // Carve the scratch block.  base may be null (size query).
 inline Scratch carve_scratch(void* base, int n, int W, int H, int ts, int64_t max_pairs, int64_t max_records) {
@@ -112,6 +117,7 @@ inline Scratch carve_scratch(void* base, int n, int W, int H, int ts, int64_t ma
   s.plane = (FramePlane*)take(sizeof(FramePlane));
   s.tile_rect = (float4*)take(16 * T);
   s.tile_len = (int32_t*)take(4 * T);
+  s.dir_table = dir_table_bytes(W, H) <= kDirTableMax ? (char*)take(dir_table_bytes(W, H)) : nullptr;
   s.bytes = off;
   return s;
 }
@@ -241,7 +247,11 @@ int launch_mlp_f32(const mlpsp_scene* sc, const RecIn* rec_in, const int4* work,
 // work_small: the wave's small-group list (launch_prim_scan with split_small), or null when every item is on `work`
 int launch_mlp_f16(const mlpsp_scene* sc, const RecIn* rec_in, const int4* work,
                    const int32_t* counters, float4* rec_out, float4* rec_ext, int out_mode, int32_t* status,
-                   cudaStream_t st, bool bf16 = false, int grid_cap = 0, const int4* work_small = nullptr);
+                   cudaStream_t st, bool bf16 = false, int grid_cap = 0, const int4* work_small = nullptr,
+                   const char* dir_table = nullptr);
+// The encoded ray directions of a frame (5,120 bytes per tile), for records that name their pixel instead of carrying its
+// direction (launch_fill with the table flag; not together with a small-group list or record export).
+int launch_encode_directions(const mlpsp_scene* sc, const mlpsp_frame* fr, char* table, cudaStream_t st);
 int launch_scan_i32(const int32_t* in, int64_t n, int32_t* blk, int32_t* out, cudaStream_t st);
 int launch_export_records(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, int64_t* offsets, int32_t* ids,
                           float* x6, float* raw, int32_t* relu_masks, float* gates, int64_t max_out, int32_t max_hits,

@@ -32,11 +32,11 @@ namespace mlpsp {
 constexpr int kRows = kRowsPerItem;      // 128 = MMA M
 constexpr int kChunk = kRows * 16;       // bytes of one K chunk of an A tile: [128 rows][8 halves]
 constexpr int kN3 = 16;                  // 4 outputs padded to the smallest N
-constexpr int kA1Chunks = 9;             // 72 encoded inputs
+constexpr int kA1Chunks = 10;            // 72 encoded inputs and eight ones: two halves of 36 + 4
 
 // ---- packed weight image (per primitive) and shared-memory plan for F = 6, hidden width H = 32 or 64 ----
-// piece 1: W1 as [11 chunks][H rows][8 halves]: chunks 0..8 hold K = 0..71 in the order of enc_k(), chunk 9 is
-//          zero (it meets whatever follows the last A chunk), chunk 10 holds the eight terms of b1[h];
+// piece 1: W1 as [10 chunks][H rows][8 halves] in the order of enc_k(): the ray direction's 36 inputs and four terms of
+//          b1[h], the offset's 36 inputs and the other four terms (the A tile holds ones there);
 // piece 2: W2 as [H/8 + 1 chunks][H][8], the last one the terms of b2;
 // piece 3: W3 as [H/8 + 1 chunks][16][8] (rows 4..15 zero), the last one the terms of b3.
 template <int H>
@@ -45,37 +45,40 @@ struct Net {
   static constexpr int kWChunk = H * 16;
   static constexpr int kW3Chunk = kN3 * 16;
   static constexpr int kOffW1 = 0;
-  static constexpr int kBytesW1 = 11 * kWChunk;
+  static constexpr int kBytesW1 = kA1Chunks * kWChunk;
   static constexpr int kOffW2 = kOffW1 + kBytesW1;
   static constexpr int kBytesW2 = (H / 8 + 1) * kWChunk;
   static constexpr int kOffW3 = kOffW2 + kBytesW2;
   static constexpr int kBytesW3 = (H / 8 + 1) * kW3Chunk;
-  static constexpr int kWeightBytes = kOffW3 + kBytesW3;          // 9,472 (H = 32) / 22,784 (H = 64)
-  // shared memory: weight image | eight rows of ones, eight rows of zeros | layer-1 A tile | hidden A tile | barriers.
-  // The order matters: the second chunk of a bias K step on the weight side is "whatever follows" (the next
-  // piece, or the ones / zeros after the image), always finite, and meets the zero rows on the A side; the second
-  // chunk of the last layer-1 K step on the A side is the first hidden chunk and meets W1's zero chunk.
+  static constexpr int kWeightBytes = kOffW3 + kBytesW3;          // 8,960 (H = 32) / 21,760 (H = 64)
+  // shared memory: weight image | eight rows of ones, eight rows of zeros | layer-1 A tile | barriers.  The second chunk of a
+  // bias K step (layers 2 and 3) on the weight side is "whatever follows" (the next piece, or the ones / zeros after the
+  // image), always finite, and meets the zero rows on the A side.
   static constexpr int kOffConst = kWeightBytes;
   static constexpr int kOffA1 = kOffConst + 256;
-  static constexpr int kOffA2 = kOffA1 + kA1Chunks * kChunk;
-  static constexpr int kOffBar = kOffA2 + (H / 8) * kChunk;
-  static constexpr int kSmemBytes = kOffBar + 96;                  // 36,448 / 57,952
-  static constexpr int kTmemCols = 2 * H;   // D1 [0,H)  D2 [H,2H)  D3 [H,H+16)
-  // resident CTAs per SM: H = 32: shared memory would give 6, five leave each thread 80 registers (no spills; six
-  // measured no faster); H = 64: shared memory gives 3
-  static constexpr int kCtas = H == 32 ? 5 : 3;
+  static constexpr int kOffBar = kOffA1 + kA1Chunks * kChunk;
+  static constexpr int kSmemBytes = kOffBar + 96;                  // 29,792 / 42,592
+  // tensor memory: D1 and, once it has been read, D2 | D3 | the hidden layers' operand (H / 2 columns, two elements each)
+  static constexpr int kTmemCols = 2 * H;
+  static constexpr int kD1 = 0, kD2 = 0, kD3 = H, kA2 = H + kN3;
+  static_assert(kA2 + H / 2 <= kTmemCols, "tensor memory plan");
+  // resident CTAs per SM: H = 32: registers (64 a thread), H = 64: tensor memory
+  static constexpr int kCtas = H == 32 ? 6 : 4;
   static_assert(kWeightBytes % 16 == 0 && kBytesW1 % 16 == 0 && kBytesW2 % 16 == 0 && kBytesW3 % 16 == 0, "bulk-copy granularity");
 };
 
 // Position of an encoded input inside the K dimension of layer 1.  The reference orders K as
 // [sin(c,f) for c, f][cos(c,f) for c, f] (np_tile_kernels.cu:329-343); a dot product does not care, so
 // the A tile and the packed W1 rows both use an order in which the six (sin, cos) pairs of one input
-// coordinate are contiguous (six 32-bit words per coordinate):
-//   k' = 12 c + 4 (f / 2) + 2 is_cos + (f % 2).
-__host__ __device__ constexpr int enc_k(int c, int f, int is_cos) { return 12 * c + 4 * (f >> 1) + 2 * is_cos + (f & 1); }
-__host__ __device__ constexpr int enc_k_of_reference(int k) {
-  return k >= 72 ? k : enc_k((k % 36) / 6, (k % 36) % 6, k / 36);
+// coordinate are contiguous (six 32-bit words per coordinate) and the coordinates of the ray direction and of the
+// offset fill five chunks each, the last four halves of which carry the bias:
+//   k' = 40 (c / 3) + 12 (c % 3) + 4 (f / 2) + 2 is_cos + (f % 2).
+__host__ __device__ constexpr int enc_k(int c, int f, int is_cos) {
+  return 40 * (c / 3) + 12 * (c % 3) + 4 * (f >> 1) + 2 * is_cos + (f & 1);
 }
+__host__ __device__ constexpr int enc_k_of_reference(int k) { return enc_k((k % 36) / 6, (k % 36) % 6, k / 36); }
+// where term j of the layer-1 bias goes
+__host__ __device__ constexpr int enc_k_of_bias(int j) { return 40 * (j / 4) + 36 + j % 4; }
 
 // The six words of one input coordinate.  mult[f] is freq[f] * att[f].  LADDER: every band is exactly twice the
 // one before, so the phases are exact doublings of the first and sin / cos of the higher bands follow from the
@@ -105,34 +108,57 @@ __device__ __forceinline__ void encode_coord(float v, const float (&mult)[6], ui
 // a finite input gives finite phases (freq * att <= 101)
 __device__ __forceinline__ bool not_finite(float v) { return !(fabsf(v) < 1.0e30f); }
 
-// The first and the second part of a record's encoding, written to this thread's row of the layer-1 A tile
-// (row = generic pointer to the row's 16 bytes inside chunk 0; kChunk = bytes between the K chunks of the tile).
-// q0 = (rdx, rdy, rdz, dx), q1 = (dy, dz, decay, slot) are the record's two 16-byte halves; part 1 computes
-// coordinates 0..3 (chunks 0..5), part 2 coordinates 4 and 5.
+// Three coordinates and four ones: five chunks of this thread's row of the layer-1 A tile (row = generic pointer to the
+// row's 16 bytes inside the first of them; kChunk = bytes between the K chunks of the tile).
+template <bool BF16>
+constexpr uint32_t kOnes2 = BF16 ? 0x3f803f80u : 0x3c003c00u;
+
 template <bool LADDER, bool BF16, int kChunk = mlpsp::kChunk>
-__device__ __forceinline__ bool encode_part1(const float4 q0, const float (&mult)[6], char* row) {
+__device__ __forceinline__ bool encode_two(float x, float y, const float (&mult)[6], char* row) {
   uint32_t a[6], b[6];
-  encode_coord<LADDER, BF16>(q0.x, mult, a);
-  encode_coord<LADDER, BF16>(q0.y, mult, b);
+  encode_coord<LADDER, BF16>(x, mult, a);
+  encode_coord<LADDER, BF16>(y, mult, b);
   *reinterpret_cast<uint4*>(row) = make_uint4(a[0], a[1], a[2], a[3]);
   *reinterpret_cast<uint4*>(row + kChunk) = make_uint4(a[4], a[5], b[0], b[1]);
   *reinterpret_cast<uint4*>(row + 2 * kChunk) = make_uint4(b[2], b[3], b[4], b[5]);
-  encode_coord<LADDER, BF16>(q0.z, mult, a);
-  encode_coord<LADDER, BF16>(q0.w, mult, b);
-  *reinterpret_cast<uint4*>(row + 3 * kChunk) = make_uint4(a[0], a[1], a[2], a[3]);
-  *reinterpret_cast<uint4*>(row + 4 * kChunk) = make_uint4(a[4], a[5], b[0], b[1]);
-  *reinterpret_cast<uint4*>(row + 5 * kChunk) = make_uint4(b[2], b[3], b[4], b[5]);
-  return not_finite(q0.x) || not_finite(q0.y) || not_finite(q0.z) || not_finite(q0.w);
+  return not_finite(x) || not_finite(y);
 }
 template <bool LADDER, bool BF16, int kChunk = mlpsp::kChunk>
-__device__ __forceinline__ bool encode_part2(const float4 q1, const float (&mult)[6], char* row) {
-  uint32_t a[6], b[6];
-  encode_coord<LADDER, BF16>(q1.x, mult, a);
-  encode_coord<LADDER, BF16>(q1.y, mult, b);
-  *reinterpret_cast<uint4*>(row + 6 * kChunk) = make_uint4(a[0], a[1], a[2], a[3]);
-  *reinterpret_cast<uint4*>(row + 7 * kChunk) = make_uint4(a[4], a[5], b[0], b[1]);
-  *reinterpret_cast<uint4*>(row + 8 * kChunk) = make_uint4(b[2], b[3], b[4], b[5]);
-  return not_finite(q1.x) || not_finite(q1.y);
+__device__ __forceinline__ bool encode_one(float z, const float (&mult)[6], char* row) {
+  uint32_t a[6];
+  encode_coord<LADDER, BF16>(z, mult, a);
+  *reinterpret_cast<uint4*>(row + 3 * kChunk) = make_uint4(a[0], a[1], a[2], a[3]);
+  *reinterpret_cast<uint4*>(row + 4 * kChunk) = make_uint4(a[4], a[5], kOnes2<BF16>, kOnes2<BF16>);
+  return not_finite(z);
+}
+template <bool BF16, int kChunk = mlpsp::kChunk>
+__device__ __forceinline__ bool encode_three(bool ladder, float x, float y, float z, const float (&mult)[6], char* row) {
+  if (ladder) return encode_two<true, BF16, kChunk>(x, y, mult, row) | encode_one<true, BF16, kChunk>(z, mult, row);
+  return encode_two<false, BF16, kChunk>(x, y, mult, row) | encode_one<false, BF16, kChunk>(z, mult, row);
+}
+
+// The encodings of the ray directions of a frame, in the operand format: per tile [5 chunks][64 pixels][16 bytes], so that
+// the pixels of one tile -- neighbouring records of a primitive, mostly -- lie together in every chunk.
+constexpr int kDirTileBytes = 5 * 64 * 16, kDirChunk = 64 * 16;
+
+template <bool BF16>
+__global__ void __launch_bounds__(256) k_encode_directions(const float* __restrict__ rays_d, int W, int H, int ntx, int T,
+                                                           const float* __restrict__ freq, const float* __restrict__ att,
+                                                           char* __restrict__ table) {
+  chain_wait();
+  chain_release();
+  float mult[6];
+  bool ladder = true;
+#pragma unroll
+  for (int f = 0; f < 6; ++f) mult[f] = __ldg(freq + f) * __ldg(att + f);
+#pragma unroll
+  for (int f = 1; f < 6; ++f) ladder = ladder && mult[f] == 2.0f * mult[f - 1];
+  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < (int64_t)T * 64; i += (int64_t)gridDim.x * 256) {
+    const TilePix tp = tile_pixel((int)(i >> 6), (int)(i & 63), ntx, W, H);
+    if (!tp.valid) continue;
+    const V3 d = load3(rays_d, tp.pix);
+    encode_three<BF16, kDirChunk>(ladder, d.x, d.y, d.z, mult, table + (i >> 6) * kDirTileBytes + (i & 63) * 16);
+  }
 }
 
 // hidden layer epilogue: ReLU, operand format (RN), write this thread's row of the hidden A tile.  The biases are
@@ -165,6 +191,29 @@ __device__ __forceinline__ bool hidden_to_smem(const uint32_t (&acc)[32], char* 
   return (top & 0xffffu) >= inf16 || (top >> 16) >= inf16;
 }
 
+// the same for 16 columns, into the operand's columns of tensor memory (taddr: first column, this warp's lanes)
+template <bool KEEP, bool BF16>
+__device__ __forceinline__ uint32_t hidden_to_tmem(const uint32_t (&acc)[16], uint32_t taddr, int col, uint32_t& relu_mask) {
+  uint32_t top = 0u, w[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const float v0 = __uint_as_float(acc[2 * q]), v1 = __uint_as_float(acc[2 * q + 1]);
+    if (KEEP) {
+      relu_mask |= (v0 > 0.f ? 1u : 0u) << (col + 2 * q);
+      relu_mask |= (v1 > 0.f ? 1u : 0u) << (col + 2 * q + 1);
+    }
+    w[q] = pack_h2_relu<BF16>(v0, v1);
+    top = __vmaxu2(top, w[q]);
+  }
+  tmem_st8(taddr, w);
+  return top;
+}
+template <bool BF16>
+__device__ __forceinline__ bool overflowed(uint32_t top) {
+  const uint32_t inf16 = BF16 ? 0x7f80u : 0x7c00u;
+  return (top & 0xffffu) >= inf16 || (top >> 16) >= inf16;
+}
+
 // One work item = (primitive, first record, rows <= 128).  Items are dealt to CTAs round-robin
 // (item = blockIdx.x + k * gridDim.x): all items cost about the same, and a fixed deal lets a CTA
 // fetch the next items' descriptors, records and weight pieces while the current item is in flight.
@@ -179,10 +228,13 @@ __device__ __forceinline__ bool hidden_to_smem(const uint32_t (&acc)[32], char* 
 //   wait layer 2: hidden tile 2 of i written -> arrive | second part of the encoding of i+1
 constexpr int kMlpThreads = kRows + 32;
 
-template <bool KEEP, bool BF16, int H>
+// TAB: the records name their pixel, whose encoded direction is copied from the frame's table (k_encode_directions) into
+// the A tile by cp.async: half of the 72 sines and cosines of a record are those of its ray, and a pixel has about a dozen
+// records.  The record is then (offset, decay | slot, pixel); without it (direction, offset, decay, slot).
+template <bool KEEP, bool BF16, int H, bool TAB>
 __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
     const char* __restrict__ w16, const float* __restrict__ freq, const float* __restrict__ att,
-    const float4* __restrict__ rec_in, const int4* __restrict__ work,
+    const char* __restrict__ dir_table, const float4* __restrict__ rec_in, const int4* __restrict__ work,
     const int32_t* __restrict__ counters, float4* __restrict__ rec_out, float4* __restrict__ rec_ext, int out_mode,
     int32_t* __restrict__ status) {
   using N = Net<H>;
@@ -190,8 +242,6 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
   chain_wait();       // the work list and the records come from the previous kernels of the frame
   chain_release();
   extern __shared__ __align__(128) char smem[];
-  char* s_a1 = smem + N::kOffA1;
-  char* s_a2 = smem + N::kOffA2;
   // [0..2] weight pieces landed, [3..5] operand tile of layer 1 / 2 / 3 complete, [6] layer-1 MMAs done, [7] layer-2 / 3 MMAs done
   uint64_t* s_bar = reinterpret_cast<uint64_t*>(smem + N::kOffBar);
   uint32_t* s_misc = reinterpret_cast<uint32_t*>(s_bar + 8);          // [0] tmem base, [1] a wait gave up
@@ -201,7 +251,7 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
   int item = blockIdx.x;
   if (item >= G) return;                     // more CTAs than work: leave before touching tensor memory
   const int stride = (int)gridDim.x;
-  const uint32_t wb = smem_u32(smem), cst = wb + N::kOffConst, a1 = wb + N::kOffA1, a2 = wb + N::kOffA2;
+  const uint32_t wb = smem_u32(smem), cst = wb + N::kOffConst, a1 = wb + N::kOffA1;
   const uint32_t bar_w0 = smem_u32(&s_bar[0]), bar_r0 = smem_u32(&s_bar[3]), bar_a = smem_u32(&s_bar[6]), bar_b = smem_u32(&s_bar[7]);
   if (tid == 0) {
 #pragma unroll
@@ -212,16 +262,9 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kRows / 32) tmem_alloc(smem_u32(&s_misc[0]), N::kTmemCols);
-  // eight rows of ones, eight rows of zeros; the hidden tile starts finite (its first chunk is read, against zero
-  // weights, by the first layer-1 MMAs before any activation has been written)
   if (tid < 16) {
-    const uint32_t one2 = BF16 ? 0x3f803f80u : 0x3c003c00u;
-    const uint32_t v = tid < 8 ? one2 : 0u;
+    const uint32_t v = tid < 8 ? kOnes2<BF16> : 0u;
     *reinterpret_cast<uint4*>(smem + N::kOffConst + tid * 16) = make_uint4(v, v, v, v);
-  }
-  if (tid < kRows) {
-#pragma unroll
-    for (int c = 0; c < H / 8; ++c) *reinterpret_cast<uint4*>(s_a2 + c * kChunk + tid * 16) = make_uint4(0u, 0u, 0u, 0u);
   }
   fence_async_smem();
   tc_fence_before();
@@ -232,85 +275,101 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
 
   if (warp == kRows / 32) {
     // ------------------------------------------------------------------ issue warp ----
-    if (lane == 0) {
-      const uint64_t ones_desc = smem_desc(cst, 128, 0);   // rows of ones, then rows of zeros; every row group the same
-      const uint32_t idesc_h = instr_desc(kRows, H, BF16), idesc_o = instr_desc(kRows, kN3, BF16);
-      // Operand descriptors are built once; a K step only moves the start address, which sits in the low bits in
-      // units of 16 bytes (shared-memory addresses stay below 2^18, so the sum never carries out of the field).
-      const uint64_t a1_desc = smem_desc(a1, kChunk, 128), a2_desc = smem_desc(a2, kChunk, 128);
-      const uint64_t w1_desc = smem_desc(wb + N::kOffW1, N::kWChunk, 128), w2_desc = smem_desc(wb + N::kOffW2, N::kWChunk, 128);
-      const uint64_t w3_desc = smem_desc(wb + N::kOffW3, N::kW3Chunk, 128);
-      auto step = [](uint64_t desc, int bytes) { return desc + (uint64_t)(bytes >> 4); };
-      auto request = [&](int piece, int prim) {
-        const int off = piece == 0 ? N::kOffW1 : (piece == 1 ? N::kOffW2 : N::kOffW3);
-        const int bytes = piece == 0 ? N::kBytesW1 : (piece == 1 ? N::kBytesW2 : N::kBytesW3);
-        mbar_expect_tx(bar_w0 + 8 * piece, bytes);
-        bulk_g2s(wb + off, w16 + (size_t)prim * N::kWeightBytes + off, bytes, bar_w0 + 8 * piece);
-      };
-      int prim = __ldg(work + item).x;
-      uint32_t pend = 7u;                    // weight pieces requested and not yet waited for
-      request(0, prim); request(1, prim); request(2, prim);
-      uint32_t li = 0u;
-      for (;;) {
-        const uint32_t par = li & 1u;
-        const int next = item + stride;
-        const bool has_next = next < G;
-        int prim_n = 0;
-        if (has_next) prim_n = __ldg(work + next).x;
-        // ---- layer 1: D1[128xH] = A1[128x72] . W1^T + b1 ----
-        ok = mbar_wait(bar_r0, par) && mbar_wait(bar_w0, par);
-        pend &= ~1u;
-        // The second chunk of a bias K step reads the start of the next piece's region as don't-care data (it meets
-        // zeros), which must still be finite: before the first item all three pieces have to be in place, afterwards
-        // the regions always hold the previous or the incoming image.
-        if (ok && li == 0u) { ok = mbar_wait(bar_w0 + 8, 0u) && mbar_wait(bar_w0 + 16, 0u); }
-        if (!ok) break;
-        tc_fence_after();
+    const uint32_t idesc_h = instr_desc(kRows, H, BF16), idesc_o = instr_desc(kRows, kN3, BF16);
+    // Operand descriptors are built once; a K step only moves the start address, which sits in the low bits in
+    // units of 16 bytes (shared-memory addresses stay below 2^18, so the sum never carries out of the field).
+    const uint64_t a1_desc = smem_desc(a1, kChunk, 128);
+    const uint64_t ones_desc = smem_desc(cst, 128, 0);     // rows of ones, then rows of zeros; every row group the same
+    const uint64_t w1_desc = smem_desc(wb + N::kOffW1, N::kWChunk, 128), w2_desc = smem_desc(wb + N::kOffW2, N::kWChunk, 128);
+    const uint64_t w3_desc = smem_desc(wb + N::kOffW3, N::kW3Chunk, 128);
+    auto step = [](uint64_t desc, int bytes) { return desc + (uint64_t)(bytes >> 4); };
+    auto request = [&](int piece, int prim) {
+      const int off = piece == 0 ? N::kOffW1 : (piece == 1 ? N::kOffW2 : N::kOffW3);
+      const int bytes = piece == 0 ? N::kBytesW1 : (piece == 1 ? N::kBytesW2 : N::kBytesW3);
+      mbar_expect_tx(bar_w0 + 8 * piece, bytes);
+      bulk_g2s(wb + off, w16 + (size_t)prim * N::kWeightBytes + off, bytes, bar_w0 + 8 * piece);
+    };
+    // every lane waits, one issues
+    auto both = [&](uint32_t x, uint32_t y, uint32_t parity) {
+      return __all_sync(0xffffffffu, mbar_wait(x, parity) && mbar_wait(y, parity)) != 0;
+    };
+    auto done = [&](uint32_t x, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(x, parity)) != 0; };
+    int prim = __ldg(work + item).x;
+    uint32_t pend = 7u;                    // weight pieces requested and not yet waited for
+    if (elect_one()) { request(0, prim); request(1, prim); request(2, prim); }
+    uint32_t li = 0u;
+    for (;;) {
+      const uint32_t par = li & 1u;
+      const int next = item + stride;
+      const bool has_next = next < G;
+      int prim_n = 0;
+      if (has_next) prim_n = __ldg(work + next).x;
+      // ---- layer 1: D1[128xH] = A1[128x80] . W1^T, the biases included ----
+      ok = both(bar_r0, bar_w0, par);
+      pend &= ~1u;
+      // The second chunk of a bias K step (layers 2 and 3) reads the start of the next piece's region as don't-care data
+      // (it meets zeros), which must still be finite: before the first item all three pieces have to be in place,
+      // afterwards the regions always hold the previous or the incoming image.
+      if (ok && li == 0u) ok = both(bar_w0 + 8, bar_w0 + 16, 0u);
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          mma_f16(tmem, step(a1_desc, ks * 2 * kChunk), step(w1_desc, ks * 2 * N::kWChunk), idesc_h, ks > 0);
-        // K = 64..79: the last A chunk and whatever follows it (the first hidden chunk) meet W1's chunk 8 and zeros
-        mma_f16(tmem, step(a1_desc, 8 * kChunk), step(w1_desc, 8 * N::kWChunk), idesc_h, 1u);
-        mma_f16(tmem, ones_desc, step(w1_desc, 10 * N::kWChunk), idesc_h, 1u);
+        for (int ks = 0; ks < kA1Chunks / 2; ++ks)
+          mma_f16(tmem + N::kD1, step(a1_desc, ks * 2 * kChunk), step(w1_desc, ks * 2 * N::kWChunk), idesc_h, ks > 0);
         mma_commit(bar_a);
-        if (!mbar_wait(bar_a, par)) { ok = false; break; }
-        if (has_next) { request(0, prim_n); pend |= 1u; }          // W1 is no longer read
-        // ---- layer 2: D2[128xH] = H1[128xH] . W2^T + b2 ----
-        ok = mbar_wait(bar_r0 + 8, par) && mbar_wait(bar_w0 + 8, par);
-        pend &= ~2u;
-        if (!ok) break;
-        tc_fence_after();
+      }
+      __syncwarp();
+      if (!(ok = done(bar_a, par))) break;
+      if (has_next) {                                            // W1 is no longer read
+        if (elect_one()) request(0, prim_n);
+        pend |= 1u;
+      }
+      // ---- layer 2: D2[128xH] = H1[128xH] . W2^T + b2 ----
+      ok = both(bar_r0 + 8, bar_w0 + 8, par);
+      pend &= ~2u;
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one()) {
 #pragma unroll
         for (int ks = 0; ks < H / 16; ++ks)
-          mma_f16(tmem + H, step(a2_desc, ks * 2 * kChunk), step(w2_desc, ks * 2 * N::kWChunk), idesc_h, ks > 0);
-        mma_f16(tmem + H, ones_desc, step(w2_desc, (H / 8) * N::kWChunk), idesc_h, 1u);
+          mma_f16_ta(tmem + N::kD2, tmem + N::kA2 + ks * 8, step(w2_desc, ks * 2 * N::kWChunk), idesc_h, ks > 0);
+        mma_f16(tmem + N::kD2, ones_desc, step(w2_desc, (H / 8) * N::kWChunk), idesc_h, 1u);
         mma_commit(bar_b);
-        if (!mbar_wait(bar_b, 0u)) { ok = false; break; }
-        if (has_next) { request(1, prim_n); pend |= 2u; }
-        // ---- layer 3: D3[128x16] = H2[128xH] . W3^T + b3 (rows 4..15 of W3 are zero) ----
-        ok = mbar_wait(bar_r0 + 16, par) && mbar_wait(bar_w0 + 16, par);
-        pend &= ~4u;
-        if (!ok) break;
-        tc_fence_after();
+      }
+      __syncwarp();
+      if (!(ok = done(bar_b, 0u))) break;
+      if (has_next) {
+        if (elect_one()) request(1, prim_n);
+        pend |= 2u;
+      }
+      // ---- layer 3: D3[128x16] = H2[128xH] . W3^T + b3 (rows 4..15 of W3 are zero) ----
+      ok = both(bar_r0 + 16, bar_w0 + 16, par);
+      pend &= ~4u;
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one()) {
 #pragma unroll
         for (int ks = 0; ks < H / 16; ++ks)
-          mma_f16(tmem + H, step(a2_desc, ks * 2 * kChunk), step(w3_desc, ks * 2 * N::kW3Chunk), idesc_o, ks > 0);
-        mma_f16(tmem + H, ones_desc, step(w3_desc, (H / 8) * N::kW3Chunk), idesc_o, 1u);
+          mma_f16_ta(tmem + N::kD3, tmem + N::kA2 + ks * 8, step(w3_desc, ks * 2 * N::kW3Chunk), idesc_o, ks > 0);
+        mma_f16(tmem + N::kD3, ones_desc, step(w3_desc, (H / 8) * N::kW3Chunk), idesc_o, 1u);
         mma_commit(bar_b);
-        if (!mbar_wait(bar_b, 1u)) { ok = false; break; }
-        if (!has_next) break;
-        request(2, prim_n); pend |= 4u;
-        item = next;
-        prim = prim_n;
-        ++li;
       }
-      if (!ok) {
-        s_misc[1] = 1u;
-        // our own bulk copies may still be in flight: give them a bounded chance to land before the CTA's
-        // shared memory is released
-        for (int b = 0; b < 3; ++b)
-          if (pend & (1u << b)) mbar_wait(bar_w0 + 8 * b, li & 1u);
-      }
+      __syncwarp();
+      if (!(ok = done(bar_b, 1u))) break;
+      if (!has_next) break;
+      if (elect_one()) request(2, prim_n);
+      pend |= 4u;
+      item = next;
+      prim = prim_n;
+      ++li;
+    }
+    if (!ok) {
+      if (lane == 0) s_misc[1] = 1u;
+      // our own bulk copies may still be in flight: give them a bounded chance to land before the CTA's
+      // shared memory is released
+      for (int b = 0; b < 3; ++b)
+        if (pend & (1u << b)) mbar_wait(bar_w0 + 8 * b, li & 1u);
     }
     __syncwarp();
   } else {
@@ -331,18 +390,39 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
       r1 = make_float4(0.f, 0.f, 0.f, 0.f);     // the zero record, never stored
       if (tid < w.z) { r0 = __ldg(rec_in + 2 * (size_t)(w.y + tid)); r1 = __ldg(rec_in + 2 * (size_t)(w.y + tid) + 1); }
     };
-    auto rec_decay = [](const float4& r1) { return r1.z; };
-    auto rec_slot = [](const float4& r1) { return __float_as_uint(r1.w); };
+    auto rec_decay = [](const float4& r0, const float4& r1) { return TAB ? r0.w : r1.z; };
+    auto rec_slot = [](const float4& r1) { return TAB ? __float_as_uint(r1.x) : __float_as_uint(r1.w); };
+    // the pixel's encoded direction on its way to this thread's row of the A tile
+    auto copy_direction = [&](const float4& r1) {
+      const uint32_t pixel = __float_as_uint(r1.y);
+      const char* src = dir_table + (size_t)(pixel >> 6) * kDirTileBytes + (pixel & 63u) * 16;
+      const uint32_t dst = a1 + tid * 16;
+#pragma unroll
+      for (int c = 0; c < 5; ++c) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + c * kChunk), "l"(src + c * kDirChunk) : "memory");
+    };
+    auto direction_landed = [&]() { asm volatile("cp.async.wait_all;" ::: "memory"); };
+    char* my_row = smem + N::kOffA1 + tid * 16;
+    // a hidden layer of the warp's rows: accumulator columns from d on -> operand
+    auto hidden = [&](uint32_t d, uint32_t& relu_mask) {
+      uint32_t top = 0u;
+      relu_mask = 0u;
+#pragma unroll
+      for (int part = 0; part < H / 16; ++part) {
+        uint32_t acc[16];
+        tmem_ld16(trow + d + part * 16, acc);
+        top = __vmaxu2(top, hidden_to_tmem<KEEP, BF16>(acc, trow + N::kA2 + part * 8, part * 16, relu_mask));
+      }
+      return overflowed<BF16>(top);
+    };
     // the warp's rows of an operand tile are complete (and its reads of tensor memory have retired)
     auto tile_done = [&](uint32_t bar) {
+      tmem_st_wait();
       fence_async_smem();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
     };
-    char* my_row = s_a1 + tid * 16;
     bool bad = false;
-
     // ---- prologue: the first item's record, encoded in full ----
     float4 q0, q1;
     load_rec(wk, q0, q1);
@@ -351,11 +431,17 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
     // operand tiles keep whatever they held) and only reports its tiles complete
     if (warp * 32 < wk.z) {
       // rows past the end inside a live warp hold the zero record; their results are never stored
-      if (ladder) { bad |= encode_part1<true, BF16>(q0, mult, my_row); bad |= encode_part2<true, BF16>(q1, mult, my_row); }
-      else { bad |= encode_part1<false, BF16>(q0, mult, my_row); bad |= encode_part2<false, BF16>(q1, mult, my_row); }
+      if (TAB) {
+        copy_direction(q1);
+        bad |= encode_three<BF16>(ladder, q0.x, q0.y, q0.z, mult, my_row + 5 * kChunk);
+        direction_landed();
+      } else {
+        bad |= encode_three<BF16>(ladder, q0.x, q0.y, q0.z, mult, my_row);
+        bad |= encode_three<BF16>(ladder, q0.w, q1.x, q1.y, mult, my_row + 5 * kChunk);
+      }
     }
     tile_done(bar_r0);
-    float decay_c = rec_decay(q1);
+    float decay_c = rec_decay(q0, q1);
     uint32_t slot_c = rec_slot(q1);
     load_rec(wk_n, q0, q1);                    // the second item's record (zero record when there is none)
 
@@ -368,7 +454,7 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
       // output of the item whose layer-3 MMAs have just finished: (decay_p, slot_p), accumulator columns [H, H+4)
       if (!live_p) return;
       uint32_t o[4];
-      tmem_ld4(trow + H, o);
+      tmem_ld4(trow + N::kD3, o);
       if (valid_p) {
         const float o0 = __uint_as_float(o[0]), o1 = __uint_as_float(o[1]), o2 = __uint_as_float(o[2]), o3 = __uint_as_float(o[3]);
         const float sigma_raw = softplus_fast(o3);
@@ -402,41 +488,37 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
       ok = __all_sync(0xffffffffu, mbar_wait(bar_a, par) && ok);
       tc_fence_after();
       if (!ok) break;
+      // layer 1 no longer reads the A tile: the next item's directions are in flight over two round trips
+      if (TAB && next_live) copy_direction(q1);
       // the record this thread will load at the end of this item (for the item after the next) is asked into L2 now
       if (tid < wk_n2.z) asm volatile("prefetch.global.L2 [%0];" ::"l"(rec_in + 2 * (size_t)(wk_n2.y + tid)));
-      if (warp_live) {
-#pragma unroll
-        for (int part = 0; part < H / 32; ++part) {       // 32 accumulator columns = 4 K chunks of the hidden tile at a time
-          uint32_t acc[32];
-          tmem_ld32(trow + part * 32, acc);
-          bad |= hidden_to_smem<KEEP, BF16>(acc, s_a2 + part * 4 * kChunk, tid, relu1) && valid;
-        }
-      }
+      if (warp_live) bad |= hidden(N::kD1, relu1) && valid;
       tile_done(bar_r0 + 8);
       // ---- first part of the next item's encoding while layer 2 runs ----
-      if (next_live)
-        bad |= ladder ? encode_part1<true, BF16>(q0, mult, my_row) : encode_part1<false, BF16>(q0, mult, my_row);
+      if (next_live) {
+        if (!TAB) bad |= encode_three<BF16>(ladder, q0.x, q0.y, q0.z, mult, my_row);
+        else bad |= ladder ? encode_two<true, BF16>(q0.x, q0.y, mult, my_row + 5 * kChunk) : encode_two<false, BF16>(q0.x, q0.y, mult, my_row + 5 * kChunk);
+      }
       ok = __all_sync(0xffffffffu, mbar_wait(bar_b, 0u) && ok);
       tc_fence_after();
       if (!ok) break;
-      if (warp_live) {                                    // layer-2 MMAs have finished reading the hidden tile
-#pragma unroll
-        for (int part = 0; part < H / 32; ++part) {
-          uint32_t acc[32];
-          tmem_ld32(trow + H + part * 32, acc);
-          bad |= hidden_to_smem<KEEP, BF16>(acc, s_a2 + part * 4 * kChunk, tid, relu2) && valid;
-        }
-      }
+      if (warp_live) bad |= hidden(N::kD2, relu2) && valid;
       tile_done(bar_r0 + 16);
       // ---- second part of the next item's encoding while layer 3 runs ----
-      if (next_live)
-        bad |= ladder ? encode_part2<true, BF16>(q1, mult, my_row) : encode_part2<false, BF16>(q1, mult, my_row);
+      if (next_live) {
+        if (!TAB) {
+          bad |= encode_three<BF16>(ladder, q0.w, q1.x, q1.y, mult, my_row + 5 * kChunk);
+        } else {
+          bad |= ladder ? encode_one<true, BF16>(q0.z, mult, my_row + 5 * kChunk) : encode_one<false, BF16>(q0.z, mult, my_row + 5 * kChunk);
+          direction_landed();
+        }
+      }
       // this item becomes the one whose output is pending; the next one becomes current
       have_prev = true;
       live_p = warp_live; valid_p = valid; decay_p = decay_c; slot_p = slot_c; relu1_p = relu1; relu2_p = relu2;
       if (!has_next) break;
       tile_done(bar_r0);
-      decay_c = rec_decay(q1);
+      decay_c = rec_decay(q0, q1);
       slot_c = rec_slot(q1);
       item = next;
       wk = wk_n;
@@ -477,7 +559,7 @@ struct MiniNet {
   static constexpr int kOffA2 = kOffA1 + kA1Chunks * kMiniChunk;
   static constexpr int kOffPad = kOffA2 + (H / 8) * kMiniChunk;     // rows 32..127 of the last hidden chunk land here
   static constexpr int kOffBar = kOffPad + (kRows - kMiniRows) * 16;
-  static constexpr int kSmemBytes = kOffBar + 64;                   // 17,984 (H = 32) / 33,344 (H = 64)
+  static constexpr int kSmemBytes = kOffBar + 64;                   // 17,984 (H = 32) / 32,832 (H = 64)
   static constexpr int kTmemCols = H;
   static constexpr int kCtas = H == 32 ? 12 : 6;
 };
@@ -511,12 +593,9 @@ __global__ void __launch_bounds__(kMiniRows, MiniNet<H>::kCtas) k_mlp_tc_mini(
   }
   tmem_alloc(smem_u32(&s_misc[0]), M::kTmemCols);
   if (lane < 16) {
-    const uint32_t one2 = BF16 ? 0x3f803f80u : 0x3c003c00u;
-    const uint32_t v = lane < 8 ? one2 : 0u;
+    const uint32_t v = lane < 8 ? kOnes2<BF16> : 0u;
     *reinterpret_cast<uint4*>(smem + M::kOffConst + lane * 16) = make_uint4(v, v, v, v);
   }
-  // the hidden tile and the rows behind it start finite (they meet zero weights in the last layer-1 K step)
-  for (int i = lane; i < (M::kOffBar - M::kOffA2) / 16; i += kMiniRows) *reinterpret_cast<uint4*>(s_a2 + i * 16) = make_uint4(0u, 0u, 0u, 0u);
   fence_async_smem();
   tc_fence_before();
   __syncwarp();
@@ -554,13 +633,14 @@ __global__ void __launch_bounds__(kMiniRows, MiniNet<H>::kCtas) k_mlp_tc_mini(
   int4 wk = __ldg(work + item);
   int4 wk_n = (item + stride < G) ? __ldg(work + item + stride) : make_int4(0, 0, 0, 0);
   uint32_t pend = 0u;
-  if (lane == 0) { request(0, wk.x); request(1, wk.x); request(2, wk.x); pend = 7u; }
+  if (elect_one()) { request(0, wk.x); request(1, wk.x); request(2, wk.x); }
+  pend = 7u;
   char* my_row = s_a1 + lane * 16;
   bool bad = false, ok = true;
   float4 q0, q1;
   load_rec(wk, q0, q1);
-  if (ladder) { bad |= encode_part1<true, BF16, kMiniChunk>(q0, mult, my_row); bad |= encode_part2<true, BF16, kMiniChunk>(q1, mult, my_row); }
-  else { bad |= encode_part1<false, BF16, kMiniChunk>(q0, mult, my_row); bad |= encode_part2<false, BF16, kMiniChunk>(q1, mult, my_row); }
+  bad |= encode_three<BF16, kMiniChunk>(ladder, q0.x, q0.y, q0.z, mult, my_row);
+  bad |= encode_three<BF16, kMiniChunk>(ladder, q0.w, q1.x, q1.y, mult, my_row + 5 * kMiniChunk);
   float decay_c = q1.z;
   uint32_t slot_c = __float_as_uint(q1.w);
   load_rec(wk_n, q0, q1);
@@ -577,27 +657,27 @@ __global__ void __launch_bounds__(kMiniRows, MiniNet<H>::kCtas) k_mlp_tc_mini(
     if (next2 < G) wk_n2 = __ldg(work + next2);
     // ---- layer 1 ----
     tile_done();
-    if (lane == 0) {
-      bool landed = mbar_wait(bar_w0, par);
-      pend &= ~1u;
-      if (li == 0u) landed = landed && mbar_wait(bar_w0 + 8, 0u) && mbar_wait(bar_w0 + 16, 0u);   // see k_mlp_tc
-      if (landed) {
-        tc_fence_after();
+    bool landed = mbar_wait(bar_w0, par);
+    if (li == 0u) landed = landed && mbar_wait(bar_w0 + 8, 0u) && mbar_wait(bar_w0 + 16, 0u);   // see k_mlp_tc
+    pend &= ~1u;
+    ok = __all_sync(0xffffffffu, landed) != 0;
+    if (!ok) break;
+    tc_fence_after();
+    if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          mma_f16(tmem, step(a1_desc, ks * 2 * kMiniChunk), step(w1_desc, ks * 2 * N::kWChunk), idesc_h, ks > 0);
-        mma_f16(tmem, step(a1_desc, 8 * kMiniChunk), step(w1_desc, 8 * N::kWChunk), idesc_h, 1u);
-        mma_f16(tmem, ones_desc, step(w1_desc, 10 * N::kWChunk), idesc_h, 1u);
-      } else {
-        ok = false;
-      }
+      for (int ks = 0; ks < kA1Chunks / 2; ++ks)
+        mma_f16(tmem, step(a1_desc, ks * 2 * kMiniChunk), step(w1_desc, ks * 2 * N::kWChunk), idesc_h, ks > 0);
       mma_commit(bar_m);
     }
+    __syncwarp();
     if (next2 < G && lane < wk_n2.z) asm volatile("prefetch.global.L2 [%0];" ::"l"(rec_in + 2 * (size_t)(wk_n2.y + lane)));
     ok = __all_sync(0xffffffffu, mbar_wait(bar_m, ph++ & 1u) && ok);   // one completion per layer
     tc_fence_after();
     if (!ok) break;
-    if (lane == 0 && has_next) { request(0, wk_n.x); pend |= 1u; }
+    if (has_next) {
+      if (elect_one()) request(0, wk_n.x);
+      pend |= 1u;
+    }
 #pragma unroll
     for (int part = 0; part < H / 32; ++part) {
       uint32_t acc[32];
@@ -606,27 +686,27 @@ __global__ void __launch_bounds__(kMiniRows, MiniNet<H>::kCtas) k_mlp_tc_mini(
     }
     // ---- layer 2 (its accumulator takes the columns of layer 1) ----
     tile_done();
-    if (lane == 0) {
-      const bool landed = mbar_wait(bar_w0 + 8, par);
-      pend &= ~2u;
-      if (landed) {
-        tc_fence_after();
+    ok = __all_sync(0xffffffffu, mbar_wait(bar_w0 + 8, par)) != 0;
+    pend &= ~2u;
+    if (!ok) break;
+    tc_fence_after();
+    if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < H / 16; ++ks)
-          mma_f16(tmem, step(a2_desc, ks * 2 * kMiniChunk), step(w2_desc, ks * 2 * N::kWChunk), idesc_h, ks > 0);
-        mma_f16(tmem, ones_desc, step(w2_desc, (H / 8) * N::kWChunk), idesc_h, 1u);
-      } else {
-        ok = false;
-      }
+      for (int ks = 0; ks < H / 16; ++ks)
+        mma_f16(tmem, step(a2_desc, ks * 2 * kMiniChunk), step(w2_desc, ks * 2 * N::kWChunk), idesc_h, ks > 0);
+      mma_f16(tmem, ones_desc, step(w2_desc, (H / 8) * N::kWChunk), idesc_h, 1u);
       mma_commit(bar_m);
     }
+    __syncwarp();
     // first part of the next item's encoding while layer 2 runs (the layer-1 tile is free)
-    if (has_next)
-      bad |= ladder ? encode_part1<true, BF16, kMiniChunk>(q0, mult, my_row) : encode_part1<false, BF16, kMiniChunk>(q0, mult, my_row);
+    if (has_next) bad |= encode_three<BF16, kMiniChunk>(ladder, q0.x, q0.y, q0.z, mult, my_row);
     ok = __all_sync(0xffffffffu, mbar_wait(bar_m, ph++ & 1u) && ok);
     tc_fence_after();
     if (!ok) break;
-    if (lane == 0 && has_next) { request(1, wk_n.x); pend |= 2u; }
+    if (has_next) {
+      if (elect_one()) request(1, wk_n.x);
+      pend |= 2u;
+    }
 #pragma unroll
     for (int part = 0; part < H / 32; ++part) {
       uint32_t acc[32];
@@ -635,26 +715,26 @@ __global__ void __launch_bounds__(kMiniRows, MiniNet<H>::kCtas) k_mlp_tc_mini(
     }
     // ---- layer 3 ----
     tile_done();
-    if (lane == 0) {
-      const bool landed = mbar_wait(bar_w0 + 16, par);
-      pend &= ~4u;
-      if (landed) {
-        tc_fence_after();
+    ok = __all_sync(0xffffffffu, mbar_wait(bar_w0 + 16, par)) != 0;
+    pend &= ~4u;
+    if (!ok) break;
+    tc_fence_after();
+    if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < H / 16; ++ks)
-          mma_f16(tmem, step(a2_desc, ks * 2 * kMiniChunk), step(w3_desc, ks * 2 * N::kW3Chunk), idesc_o, ks > 0);
-        mma_f16(tmem, ones_desc, step(w3_desc, (H / 8) * N::kW3Chunk), idesc_o, 1u);
-      } else {
-        ok = false;
-      }
+      for (int ks = 0; ks < H / 16; ++ks)
+        mma_f16(tmem, step(a2_desc, ks * 2 * kMiniChunk), step(w3_desc, ks * 2 * N::kW3Chunk), idesc_o, ks > 0);
+      mma_f16(tmem, ones_desc, step(w3_desc, (H / 8) * N::kW3Chunk), idesc_o, 1u);
       mma_commit(bar_m);
     }
-    if (has_next)
-      bad |= ladder ? encode_part2<true, BF16, kMiniChunk>(q1, mult, my_row) : encode_part2<false, BF16, kMiniChunk>(q1, mult, my_row);
+    __syncwarp();
+    if (has_next) bad |= encode_three<BF16, kMiniChunk>(ladder, q0.w, q1.x, q1.y, mult, my_row + 5 * kMiniChunk);
     ok = __all_sync(0xffffffffu, mbar_wait(bar_m, ph++ & 1u) && ok);
     tc_fence_after();
     if (!ok) break;
-    if (lane == 0 && has_next) { request(2, wk_n.x); pend |= 4u; }
+    if (has_next) {
+      if (elect_one()) request(2, wk_n.x);
+      pend |= 4u;
+    }
     {
       uint32_t o[4];
       tmem_ld4(trow, o);
@@ -676,8 +756,8 @@ __global__ void __launch_bounds__(kMiniRows, MiniNet<H>::kCtas) k_mlp_tc_mini(
     load_rec(wk_n, q0, q1);
     ++li;
   }
-  if (!ok && lane == 0) {
-    atomicOr(status + MLPSP_ST_BITS, MLPSP_ST_TIMEOUT);
+  if (!ok) {
+    if (lane == 0) atomicOr(status + MLPSP_ST_BITS, MLPSP_ST_TIMEOUT);
     for (int b = 0; b < 3; ++b)
       if (pend & (1u << b)) mbar_wait(bar_w0 + 8 * b, li & 1u);
   }
@@ -734,9 +814,9 @@ __global__ void k_pack_weights(const float* __restrict__ W1, const float* __rest
   uint16_t* w2 = reinterpret_cast<uint16_t*>(dst + N::kOffW2);
   uint16_t* w3 = reinterpret_cast<uint16_t*>(dst + N::kOffW3);
   bool bad = false;
-  for (int i = threadIdx.x; i < H * 80; i += blockDim.x) {
-    const int h = i / 80, k = i % 80;                   // k >= 72: the zero chunk
-    const uint16_t v = to_lp<BF16>(k < 72 ? W1[(size_t)p * H * 72 + h * 72 + k] : 0.f, bad);
+  for (int i = threadIdx.x; i < H * 72; i += blockDim.x) {
+    const int h = i / 72, k = i % 72;
+    const uint16_t v = to_lp<BF16>(W1[(size_t)p * H * 72 + i], bad);
     const int kk = enc_k_of_reference(k);
     w1[(kk >> 3) * (H * 8) + h * 8 + (kk & 7)] = v;
   }
@@ -751,7 +831,10 @@ __global__ void k_pack_weights(const float* __restrict__ W1, const float* __rest
     w3[(k >> 3) * (kN3 * 8) + h * 8 + (k & 7)] = v;
   }
   for (int h = threadIdx.x; h < H; h += blockDim.x) {
-    bias_terms<BF16>(b1[(size_t)p * H + h], w1 + 10 * (H * 8) + h * 8, bad);
+    uint16_t t[8];
+    bias_terms<BF16>(b1[(size_t)p * H + h], t, bad);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) w1[(enc_k_of_bias(j) >> 3) * (H * 8) + h * 8 + (enc_k_of_bias(j) & 7)] = t[j];
     bias_terms<BF16>(b2[(size_t)p * H + h], w2 + (H / 8) * (H * 8) + h * 8, bad);
   }
   for (int h = threadIdx.x; h < kN3; h += blockDim.x) {
@@ -762,15 +845,15 @@ __global__ void k_pack_weights(const float* __restrict__ W1, const float* __rest
   if (bad && status) atomicOr(status + MLPSP_ST_BITS, MLPSP_ST_NUMERIC);
 }
 
-template <bool KEEP, bool BF16, int H>
-static int launch_one(const char* image, const mlpsp_scene* sc, const RecIn* rec_in, const int4* work, const int32_t* counters,
-                      float4* rec_out, float4* rec_ext, int out_mode, int32_t* status, cudaStream_t st, int grid) {
+template <bool KEEP, bool BF16, int H, bool TAB>
+static int launch_one(const char* image, const mlpsp_scene* sc, const char* dir_table, const RecIn* rec_in, const int4* work,
+                      const int32_t* counters, float4* rec_out, float4* rec_ext, int out_mode, int32_t* status, cudaStream_t st, int grid) {
   using N = Net<H>;
   static DeviceOnce attr_once;
   if (attr_once.first())
-    MLPSP_CUDA_OK(cudaFuncSetAttribute(k_mlp_tc<KEEP, BF16, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, N::kSmemBytes));
-  launch_chained(k_mlp_tc<KEEP, BF16, H>, dim3(grid), dim3(kMlpThreads), N::kSmemBytes, st, image, sc->freq, sc->att, reinterpret_cast<const float4*>(rec_in),
-                                                                   work, counters, rec_out, rec_ext, out_mode, status);
+    MLPSP_CUDA_OK(cudaFuncSetAttribute(k_mlp_tc<KEEP, BF16, H, TAB>, cudaFuncAttributeMaxDynamicSharedMemorySize, N::kSmemBytes));
+  launch_chained(k_mlp_tc<KEEP, BF16, H, TAB>, dim3(grid), dim3(kMlpThreads), N::kSmemBytes, st, image, sc->freq, sc->att, dir_table,
+                 reinterpret_cast<const float4*>(rec_in), work, counters, rec_out, rec_ext, out_mode, status);
   return MLPSP_OK;
 }
 
@@ -787,7 +870,7 @@ static int launch_mini(const char* image, const mlpsp_scene* sc, const RecIn* re
 }
 
 template <int H>
-static int launch_tc(const mlpsp_scene* sc, const char* image, const RecIn* rec_in, const int4* work, const int4* work_small,
+static int launch_tc(const mlpsp_scene* sc, const char* image, const char* dir_table, const RecIn* rec_in, const int4* work, const int4* work_small,
                      const int32_t* counters, float4* rec_out, float4* rec_ext, int out_mode, int32_t* status, cudaStream_t st,
                      bool bf16, int grid_cap) {
   using N = Net<H>;
@@ -801,11 +884,14 @@ static int launch_tc(const mlpsp_scene* sc, const char* image, const RecIn* rec_
       set_error("record export needs hidden width 32 (32-bit ReLU masks)");
       return MLPSP_E_LIMIT;
     }
-    rc = bf16 ? launch_one<true, true, 32>(image, sc, rec_in, work, counters, rec_out, rec_ext, out_mode, status, st, grid)
-              : launch_one<true, false, 32>(image, sc, rec_in, work, counters, rec_out, rec_ext, out_mode, status, st, grid);
+    rc = bf16 ? launch_one<true, true, 32, false>(image, sc, nullptr, rec_in, work, counters, rec_out, rec_ext, out_mode, status, st, grid)
+              : launch_one<true, false, 32, false>(image, sc, nullptr, rec_in, work, counters, rec_out, rec_ext, out_mode, status, st, grid);
+  } else if (dir_table) {
+    rc = bf16 ? launch_one<false, true, H, true>(image, sc, dir_table, rec_in, work, counters, rec_out, rec_ext, out_mode, status, st, grid)
+              : launch_one<false, false, H, true>(image, sc, dir_table, rec_in, work, counters, rec_out, rec_ext, out_mode, status, st, grid);
   } else {
-    rc = bf16 ? launch_one<false, true, H>(image, sc, rec_in, work, counters, rec_out, rec_ext, out_mode, status, st, grid)
-              : launch_one<false, false, H>(image, sc, rec_in, work, counters, rec_out, rec_ext, out_mode, status, st, grid);
+    rc = bf16 ? launch_one<false, true, H, false>(image, sc, nullptr, rec_in, work, counters, rec_out, rec_ext, out_mode, status, st, grid)
+              : launch_one<false, false, H, false>(image, sc, nullptr, rec_in, work, counters, rec_out, rec_ext, out_mode, status, st, grid);
   }
   if (rc) return rc;
   if (work_small && !rec_ext) {
@@ -819,9 +905,18 @@ static int launch_tc(const mlpsp_scene* sc, const char* image, const RecIn* rec_
   return cuda_check(cudaGetLastError(), "mlp_f16");
 }
 
+int launch_encode_directions(const mlpsp_scene* sc, const mlpsp_frame* fr, char* table, cudaStream_t st) {
+  const int T = num_tiles(fr->width, fr->height, 8), ntx = (fr->width + 7) / 8;
+  LaunchScope scope(kKMlp, 1, st);
+  auto* kernel = fr->precision == MLPSP_PRECISION_BF16 ? k_encode_directions<true> : k_encode_directions<false>;
+  return cuda_check(launch_chained(kernel, dim3((unsigned)std::min<int64_t>(((int64_t)T * 64 + 255) / 256, (int64_t)sm_count() * 64)), dim3(256), 0, st,
+                                   fr->rays_d, fr->width, fr->height, ntx, T, sc->freq, sc->att, table),
+                    "encode_directions");
+}
+
 int launch_mlp_f16(const mlpsp_scene* sc, const RecIn* rec_in, const int4* work,
                    const int32_t* counters, float4* rec_out, float4* rec_ext, int out_mode, int32_t* status,
-                   cudaStream_t st, bool bf16, int grid_cap, const int4* work_small) {
+                   cudaStream_t st, bool bf16, int grid_cap, const int4* work_small, const char* dir_table) {
   MLPSP_REQUIRE((sc->hidden == 32 || sc->hidden == 64) && sc->num_freq == 6, MLPSP_E_LIMIT,
                 "the tensor-core evaluator is built for 72->H->H->4 networks with H = 32 or 64 (6 frequencies)");
   const char* image = (const char*)(bf16 ? sc->wbf16 : sc->w16);
@@ -829,8 +924,8 @@ int launch_mlp_f16(const mlpsp_scene* sc, const RecIn* rec_in, const int4* work,
                 bf16 ? "bf16" : "fp16");
   MLPSP_REQUIRE((reinterpret_cast<uintptr_t>(image) & 15) == 0, MLPSP_E_ARG, "the packed weight image must be 16-byte aligned");
   if (sc->hidden == 64)
-    return launch_tc<64>(sc, image, rec_in, work, work_small, counters, rec_out, rec_ext, out_mode, status, st, bf16, grid_cap);
-  return launch_tc<32>(sc, image, rec_in, work, work_small, counters, rec_out, rec_ext, out_mode, status, st, bf16, grid_cap);
+    return launch_tc<64>(sc, image, dir_table, rec_in, work, work_small, counters, rec_out, rec_ext, out_mode, status, st, bf16, grid_cap);
+  return launch_tc<32>(sc, image, dir_table, rec_in, work, work_small, counters, rec_out, rec_ext, out_mode, status, st, bf16, grid_cap);
 }
 
 }  // namespace mlpsp

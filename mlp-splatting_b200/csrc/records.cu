@@ -664,7 +664,7 @@ struct FillArgs {
   const int32_t* tile_offsets; const int32_t* tile_len; const int32_t* sorted_prims; int W, H, ntx; float thr;
   const int32_t* active; const int32_t* active_count; int lo, hi;
   const uint2* masks; const uint32_t* pair_base; int32_t* prim_pos; float4* rec_in; float* rec_t; float4* rec_gate;
-  float beta, tau; int plain; const int32_t* status;      // plain: MODE 0 without the shared per-candidate geometry
+  float beta, tau; int plain, table; const int32_t* status;      // plain: MODE 0 without the shared per-candidate geometry; table: see below
   int width, chunks, halves;                              // candidates per unit, units per window and half, 2: a unit is one half
 };
 
@@ -781,9 +781,13 @@ __global__ void __launch_bounds__(32 * kFillWarps, 4) k_fill(const FillArgs a) {
           else if (MODE == 1) hit_test(load_geom(a.geom, pj), oo, dd, a.thr, ht);
           else hit_values_fast(load_geom(a.geom, pj), oo, dd, ht);
         }
-        // the record's 32 bytes in one store: a full sector
-        asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(a.rec_in + 2 * (size_t)pos), "f"(ray.x), "f"(ray.y),
-                     "f"(ray.z), "f"(ht.dx), "f"(ht.dy), "f"(ht.dz), "f"(ht.decay), "f"(__uint_as_float(slot)) : "memory");
+        // the record's 32 bytes in one store: a full sector.  (direction, offset, decay, slot), or, for an evaluator that
+        // looks the encoded direction up (table), (offset, decay, slot, pixel)
+        const float sl = __uint_as_float(slot), pixel = __uint_as_float((uint32_t)(tile * 64 + h * 32 + px));
+        float v[8] = {ray.x, ray.y, ray.z, ht.dx, ht.dy, ht.dz, ht.decay, sl};
+        if (a.table) { v[0] = ht.dx; v[1] = ht.dy; v[2] = ht.dz; v[3] = ht.decay; v[4] = sl; v[5] = pixel; }
+        asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(a.rec_in + 2 * (size_t)pos), "f"(v[0]), "f"(v[1]),
+                     "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
         if (a.rec_t) a.rec_t[slot] = ht.t;
         if (MODE != 0 && a.rec_gate) {
           const float4 ls = __ldg(a.geom + (size_t)pj * 4 + 3);
@@ -1380,6 +1384,11 @@ int launch_render_sorted(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scr
   // extra launch per wave costs more than the few remainders gain (measured: 250,000 primitives on 816,000 pixels
   // lose 4 % of evaluator time with the second list, 500,000 gain 2 %, 2,000,000 with 64 hidden units gain 21 %).  (Record export keeps one list.)
   const bool split_small = tc_path && !keep && (int64_t)n * 3 > P;
+  const bool table = tc_path && !keep && !split_small && s.dir_table && sc->num_freq == 6;
+  if (table) {
+    const int rc_dir = launch_encode_directions(sc, fr, s.dir_table, st);
+    if (rc_dir) return rc_dir;
+  }
   const int sms = sm_count();
   // per-pixel ordering: one wave over the whole lists, every pixel live
   const int nw = per_pixel ? 1 : (fr->num_waves > 0 ? fr->num_waves : (int)(sizeof(kDefaultWaves) / sizeof(int)));
@@ -1414,13 +1423,14 @@ int launch_render_sorted(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scr
       const FillArgs fa = {fr->rays_o, fr->rays_d, (const float4*)sc->geom, fr->tile_offsets, s.tile_len, fr->sorted_prims, W, H, ntx,
                            fr->threshold, act, act_n, lo, hi, reinterpret_cast<const uint2*>(s.masks32), s.pair_base,
                            s.prim_pos, reinterpret_cast<float4*>(s.rec_in), (want_t || per_pixel) ? s.rec_t : nullptr, gate,
-                           sc->gate_beta, sc->gate_tau, keep ? 1 : 0, fr->status, 0, 0, 0};
+                           sc->gate_beta, sc->gate_tau, keep ? 1 : 0, table ? 1 : 0, fr->status, 0, 0, 0};
       rc = launch_fill(fa, gate || per_pixel, ref_arith, T, sms, idle_tail, st);
       if (rc) return rc;
     }
     if (tc_path)
       rc = launch_mlp_f16(sc, s.rec_in, s.work, s.counters, s.rec_out, keep ? s.rec_ext : nullptr, kOutAlpha,
-                          fr->status, st, fr->precision == MLPSP_PRECISION_BF16, cap_mlp, split_small ? s.work_small : nullptr);
+                          fr->status, st, fr->precision == MLPSP_PRECISION_BF16, cap_mlp, split_small ? s.work_small : nullptr,
+                          table ? s.dir_table : nullptr);
     else
       rc = launch_mlp_f32(sc, s.rec_in, s.work, s.counters, s.rec_out, keep ? s.rec_ext : nullptr, kOutAlpha,
                           fr->status, st, cap_mlp);
@@ -1553,7 +1563,7 @@ int launch_render_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scr
         const FillArgs fa = {fr->rays_o, fr->rays_d, (const float4*)sc->geom, fr->tile_offsets, s.tile_len, fr->sorted_prims, W, H, ntx,
                              f0->threshold, s.active[cur], s.counters + kCtrActive0 + cur, lo, hi,
                              reinterpret_cast<const uint2*>(s.masks32), s.pair_base, lead.prim_pos, reinterpret_cast<float4*>(lead.rec_in),
-                             nullptr, nullptr, sc->gate_beta, sc->gate_tau, 0, f0->status, 0, 0, 0};
+                             nullptr, nullptr, sc->gate_beta, sc->gate_tau, 0, 0, f0->status, 0, 0, 0};
         rc = launch_fill(fa, false, ref_arith, T, sms, idle_tail, st);
         if (rc) return rc;
       }

@@ -179,10 +179,13 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
-    if (tid == 0) {
+    if (warp == 0) {
       tc_fence_after();
-      issue();
-      mma_commit(bar);
+      if (elect_one()) {
+        issue();
+        mma_commit(bar);
+      }
+      __syncwarp();
     }
   };
   auto wait_phase = [&]() -> bool {
