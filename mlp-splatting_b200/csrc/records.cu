@@ -620,17 +620,20 @@ int launch_prim_scan(const Scratch& s, int n, const int64_t* fixed, int32_t* sta
 }
 
 // -------------------------------------------------------------------------- fill pass ----
-// Feature gates (semantic_tetra_gates, np_tile_kernels.cu:97-124).
-__device__ __forceinline__ float4 tetra_gates(const Hit& h, float lsx, float lsy, float lsz, float beta, float tau) {
-  const float sx = det_exp(lsx), sy = det_exp(lsy), sz = det_exp(lsz);
-  const float ux = fminf(1.f, fmaxf(-1.f, h.qx / (beta * sx + 1e-6f)));
-  const float uy = fminf(1.f, fmaxf(-1.f, h.qy / (beta * sy + 1e-6f)));
-  const float uz = fminf(1.f, fmaxf(-1.f, h.qz / (beta * sz + 1e-6f)));
+// Feature gates (semantic_tetra_gates, np_tile_kernels.cu:97-124).  What depends on the primitive alone, the reciprocals
+// of beta * scale + 1e-6, is a function of its own: the fill pass prepares it once per candidate.
+__device__ __forceinline__ V3 gate_scales(const float4 ls, float beta) {
+  return {1.f / (beta * det_exp(ls.x) + 1e-6f), 1.f / (beta * det_exp(ls.y) + 1e-6f), 1.f / (beta * det_exp(ls.z) + 1e-6f)};
+}
+__device__ __forceinline__ float4 tetra_gates(const Hit& h, V3 inv_s, float tau) {
+  const float ux = fminf(1.f, fmaxf(-1.f, h.qx * inv_s.x));
+  const float uy = fminf(1.f, fmaxf(-1.f, h.qy * inv_s.y));
+  const float uz = fminf(1.f, fmaxf(-1.f, h.qz * inv_s.z));
   const float l0 = tau * (ux + uy + uz), l1 = tau * (ux - uy - uz);
   const float l2 = tau * (-ux + uy - uz), l3 = tau * (-ux - uy + uz);
   const float lm = fmaxf(fmaxf(l0, l1), fmaxf(l2, l3));
   const float e0 = __expf(l0 - lm), e1 = __expf(l1 - lm), e2 = __expf(l2 - lm), e3 = __expf(l3 - lm);
-  const float inv = 1.f / fmaxf(e0 + e1 + e2 + e3, 1e-8f);
+  const float inv = __fdividef(1.f, fmaxf(e0 + e1 + e2 + e3, 1e-8f));
   return make_float4(e0 * inv, e1 * inv, e2 * inv, e3 * inv);
 }
 
@@ -654,7 +657,8 @@ __device__ __forceinline__ uint32_t transpose32(uint32_t w) {
 // and neighbouring lanes write neighbouring records.  About 100 instructions per record where a search for the record's
 // pair and pixel, and the full geometry per record, took 350 (100k frame, 10.6 M records: 193 -> 135 us).
 // MODE 0: values only (no decision hangs on them: hardware reciprocal and exponential); 1: hit_test's own values, for the
-// feature gates, which divide the local offset by the scales, and for per-pixel ordering, which sorts by t; 2: the
+// feature gates, which divide the local offset by the scales, and for per-pixel ordering, which sorts by t (geometry and
+// gate scales staged per candidate as well: 270 -> 208 us of a 250k feature frame); 2: the
 // reference kernels' arithmetic.
 constexpr int kFillWarps = 8;
 struct FillSmem { float4 geo[32][5]; float4 ray[32]; uint16_t list[1024]; };
@@ -711,9 +715,21 @@ __global__ void __launch_bounds__(32 * kFillWarps, 4) k_fill(const FillArgs a) {
       if (h == 0) o0 = V3{__shfl_sync(0xffffffffu, o[0].x, 0), __shfl_sync(0xffffffffu, o[0].y, 0), __shfl_sync(0xffffffffu, o[0].z, 0)};
       same = same && (!tp.valid || (o[h].x == o0.x && o[h].y == o0.y && o[h].z == o0.z));
     }
-    const bool uni = MODE == 0 && !a.plain && __all_sync(0xffffffffu, same);
+    const bool uni = MODE != 2 && !(MODE == 0 && a.plain) && __all_sync(0xffffffffu, same);
     __syncwarp();
-    if (uni && c > 0) {
+    if (MODE == 1 && c > 0) {
+      // centre, quaternion, scales and, for a common origin, the local offset: hit_test's operands, so its bits
+      const Geom g = load_geom(a.geom, p);
+      const V3 vl = local_offset(g, o0);
+      V3 is = {0.f, 0.f, 0.f};
+      if (a.rec_gate) is = gate_scales(__ldg(a.geom + (size_t)p * 4 + 3), a.beta);
+      sm.geo[lane][0] = make_float4(g.cx, g.cy, g.cz, g.qw);
+      sm.geo[lane][1] = make_float4(g.qx, g.qy, g.qz, vl.x);
+      sm.geo[lane][2] = make_float4(vl.y, vl.z, is.x, is.y);
+      sm.geo[lane][3] = make_float4(g.mx, g.my, g.mz, 0.f);
+      sm.geo[lane][4] = make_float4(is.z, 0.f, 0.f, 0.f);
+    }
+    if (MODE == 0 && uni && c > 0) {
       const Geom g = load_geom(a.geom, p);
       // rows of R^T: R^T applied to the axes gives its columns
       const V3 c0 = rot_conj_fast(g.qw, g.qx, g.qy, g.qz, V3{1.f, 0.f, 0.f}), c1 = rot_conj_fast(g.qw, g.qx, g.qy, g.qz, V3{0.f, 1.f, 0.f}),
@@ -764,6 +780,7 @@ __global__ void __launch_bounds__(32 * kFillWarps, 4) k_fill(const FillArgs a) {
         const int pos = __float_as_int(g3.w) + r;
         const uint32_t slot = (uint32_t)(__float_as_int(g4.w) + r);
         Hit ht;
+        V3 is = {0.f, 0.f, 0.f};
         if (MODE == 0 && uni) {
           const float4 g0 = sm.geo[j][0], g1 = sm.geo[j][1], g2 = sm.geo[j][2];
           const float lx = g0.x * ray.x + g0.y * ray.y + g0.z * ray.z, ly = g1.x * ray.x + g1.y * ray.y + g1.z * ray.z,
@@ -778,8 +795,15 @@ __global__ void __launch_bounds__(32 * kFillWarps, 4) k_fill(const FillArgs a) {
         } else {
           const V3 dd = {ray.x, ray.y, ray.z};
           if (MODE == 2) hit_test_ref(load_geom_ref(a.geom, pj), oo, dd, a.thr, ht);
-          else if (MODE == 1) hit_test(load_geom(a.geom, pj), oo, dd, a.thr, ht);
-          else hit_values_fast(load_geom(a.geom, pj), oo, dd, ht);
+          else if (MODE == 1) {
+            const float4 g0 = sm.geo[j][0], g1 = sm.geo[j][1], g2 = sm.geo[j][2];
+            Geom g;
+            g.cx = g0.x; g.cy = g0.y; g.cz = g0.z; g.qw = g0.w; g.qx = g1.x; g.qy = g1.y; g.qz = g1.z;
+            g.mx = g3.x; g.my = g3.y; g.mz = g3.z; g.smax = 0.f;
+            is = V3{g2.z, g2.w, g4.x};
+            if (uni) hit_test_t<true>(g, oo, dd, V3{g1.w, g2.x, g2.y}, a.thr, ht);
+            else hit_test(g, oo, dd, a.thr, ht);
+          } else hit_values_fast(load_geom(a.geom, pj), oo, dd, ht);
         }
         // the record's 32 bytes in one store: a full sector.  (direction, offset, decay, slot), or, for an evaluator that
         // looks the encoded direction up (table), (offset, decay, slot, pixel)
@@ -790,8 +814,8 @@ __global__ void __launch_bounds__(32 * kFillWarps, 4) k_fill(const FillArgs a) {
                      "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
         if (a.rec_t) a.rec_t[slot] = ht.t;
         if (MODE != 0 && a.rec_gate) {
-          const float4 ls = __ldg(a.geom + (size_t)pj * 4 + 3);
-          a.rec_gate[slot] = tetra_gates(ht, ls.x, ls.y, ls.z, a.beta, a.tau);
+          if (MODE == 2) is = gate_scales(__ldg(a.geom + (size_t)pj * 4 + 3), a.beta);
+          a.rec_gate[slot] = tetra_gates(ht, is, a.tau);
         }
       }
       __syncwarp();
@@ -1660,7 +1684,7 @@ __global__ void __launch_bounds__(64) k_export(
       if (relu_masks) { relu_masks[r * 2] = (int32_t)__float_as_uint(re.z); relu_masks[r * 2 + 1] = (int32_t)__float_as_uint(re.w); }
       if (gates) {
         const float4 ls = __ldg(geom + (size_t)p * 4 + 3);
-        const float4 g = tetra_gates(h, ls.x, ls.y, ls.z, beta, tau);
+        const float4 g = tetra_gates(h, gate_scales(ls, beta), tau);
         float* q = gates + r * 4; q[0] = g.x; q[1] = g.y; q[2] = g.z; q[3] = g.w;
       }
     }
