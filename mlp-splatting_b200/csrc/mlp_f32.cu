@@ -5,6 +5,7 @@
 // One CTA per work item (primitive, up to 128 of its records); the primitive's FP32 weights are
 // staged once in shared memory and every thread evaluates one record.
 #include "frame.cuh"
+#include "tc.cuh"
 
 namespace mlpsp {
 
@@ -91,110 +92,374 @@ __global__ void __launch_bounds__(kRowsPerItem) k_mlp_f32(
   }
 }
 
-// The standard network (6 frequencies, hidden 32) with compile-time sizes: W1 sits transposed in shared memory
-// ([input][hidden], rows padded to 36 floats so that the staging stores spread over the banks and every row stays
-// 16-byte aligned), so the 32 hidden sums of one input take eight 128-bit broadcast loads instead of 32 scalar ones;
-// W2 rows are read the same way.  The order of every sum is the one described at the top of this file.
-constexpr int kSH = 32, kSF = 6, kSIN = 72, kSRow = 36;
-constexpr int kStdSmemFloats = kSIN * kSRow + kSH * kSH + kSH * 4 + kSH + kSH + 4;
+constexpr int kTIN = 72, kTF = 6;         // six frequencies
 
-__global__ void __launch_bounds__(kRowsPerItem) k_mlp_f32_std(
+__device__ __forceinline__ unsigned long long pack_f32x2(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack_f32x2(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ void fma_f32x2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+
+// The 72 -> 32 -> 32 -> 4 network: 64 threads per work item, one or two records per thread, the hidden sums in registers as
+// packed pairs of units (fma.rn.f32x2: two IEEE multiply-adds, so every sum keeps the order and the bits described at the top
+// of this file).  The weights lie transposed in shared memory ([input][unit]); a row of 32 weights takes eight broadcast
+// 16-byte reads, whose halves are the packed operands, and feeds 64 multiply-adds.  The next item's weights and records are
+// copied (asynchronously, transposed on the way) while the current one is computed.  Bound: FP32 multiply-adds, 3,456 per
+// record -- 36 G on the 100k frame, 1.0 ms at the chip's rate -- and the broadcast reads.  With one record per thread and
+// scalar multiply-adds the reads bounded it at 2.75 ms; this takes 2.26 ms (five CTAs per SM, 168 registers: 2.55).
+struct PairBuf {
+  static constexpr int kRow = 36;          // floats per row: 16-byte aligned, and the transposing copies spread over the banks
+  static constexpr int kW1 = 0, kW2 = kW1 + kTIN * kRow, kW3 = kW2 + 32 * kRow, kB1 = kW3 + 128, kB2 = kB1 + 32, kB3 = kB2 + 32,
+                       kRec = kB3 + 4, kFloats = kRec + kRowsPerItem * 8;
+};
+static_assert(PairBuf::kRec % 4 == 0 && PairBuf::kFloats % 4 == 0, "16-byte copies");
+constexpr int kPairThreads = 64, kPairCtas = 4;
+
+__device__ __forceinline__ void cp_async4(uint32_t dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// one row of 32 weights onto the sums of NR records
+template <int NR>
+__device__ __forceinline__ void row_fma(unsigned long long (&acc)[NR][16], const float* row, const float (&x)[NR]) {
+  unsigned long long xx[NR];
+#pragma unroll
+  for (int r = 0; r < NR; ++r) xx[r] = pack_f32x2(x[r], x[r]);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(row + 4 * k);
+#pragma unroll
+    for (int r = 0; r < NR; ++r) { fma_f32x2(acc[r][2 * k], w.x, xx[r]); fma_f32x2(acc[r][2 * k + 1], w.y, xx[r]); }
+  }
+}
+template <int NR>
+__device__ __forceinline__ void row_start(unsigned long long (&acc)[NR][16], const float* bias) {
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(bias + 4 * k);
+#pragma unroll
+    for (int r = 0; r < NR; ++r) { acc[r][2 * k] = b.x; acc[r][2 * k + 1] = b.y; }
+  }
+}
+// ReLU of the sums; bit u of mask: unit u is positive
+template <int NR>
+__device__ __forceinline__ void row_relu(const unsigned long long (&acc)[NR][16], float (&h)[NR][32], uint32_t (&mask)[NR], bool want) {
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    mask[r] = 0u;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const float2 v = unpack_f32x2(acc[r][k]);
+      h[r][2 * k] = v.x;
+      h[r][2 * k + 1] = v.y;
+    }
+    if (want) {
+#pragma unroll
+      for (int k = 0; k < 32; ++k) mask[r] |= (h[r][k] > 0.f ? 1u : 0u) << k;
+    }
+#pragma unroll
+    for (int k = 0; k < 32; ++k) h[r][k] = fmaxf(h[r][k], 0.f);
+  }
+}
+
+template <int NR>
+__device__ __forceinline__ void pair_eval(const float* sm, const float (&fr)[kTF], const float (&at)[kTF], int tid, int rows,
+                                          float4* __restrict__ rec_out, float4* __restrict__ rec_ext, int out_mode) {
+  using B = PairBuf;
+  unsigned long long acc[NR][16];
+  float h[NR][32];
+  uint32_t m1[NR], m2[NR];
+  row_start<NR>(acc, sm + B::kB1);
+#pragma unroll 1
+  for (int c = 0; c < 6; ++c) {
+    float v[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) v[r] = sm[B::kRec + (tid + r * kPairThreads) * 8 + c];
+    const float* row = sm + B::kW1 + c * kTF * B::kRow;
+#pragma unroll
+    for (int f = 0; f < kTF; ++f) {
+      float sn[NR], cs[NR];
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        const float ph = v[r] * fr[f] * at[f];
+        sn[r] = __sinf(ph);
+        cs[r] = __cosf(ph);
+      }
+      row_fma<NR>(acc, row + f * B::kRow, sn);
+      row_fma<NR>(acc, row + (f + kTIN / 2) * B::kRow, cs);
+    }
+  }
+  row_relu<NR>(acc, h, m1, rec_ext != nullptr);
+  row_start<NR>(acc, sm + B::kB2);
+#pragma unroll
+  for (int k = 0; k < 32; ++k) {
+    float x[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) x[r] = h[r][k];
+    row_fma<NR>(acc, sm + B::kW2 + k * B::kRow, x);
+  }
+  row_relu<NR>(acc, h, m2, rec_ext != nullptr);
+  float o[NR][4];
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[r][e] = sm[B::kB3 + e];
+  }
+#pragma unroll
+  for (int k = 0; k < 32; ++k) {
+    const float4 w = *reinterpret_cast<const float4*>(sm + B::kW3 + 4 * k);
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+      o[r][0] = fmaf(w.x, h[r][k], o[r][0]); o[r][1] = fmaf(w.y, h[r][k], o[r][1]);
+      o[r][2] = fmaf(w.z, h[r][k], o[r][2]); o[r][3] = fmaf(w.w, h[r][k], o[r][3]);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    const int rec = tid + r * kPairThreads;
+    if (rec >= rows) continue;
+    const float decay = sm[B::kRec + rec * 8 + 6];
+    const uint32_t slot = __float_as_uint(sm[B::kRec + rec * 8 + 7]);
+    const float sigma_raw = softplus_fast(o[r][3]);
+    float4 out;
+    out.x = sigmoid_fast(o[r][0]); out.y = sigmoid_fast(o[r][1]); out.z = sigmoid_fast(o[r][2]);
+    out.w = (out_mode == kOutAlpha) ? (1.f - __expf(-(sigma_raw * decay))) : sigma_raw;
+    rec_out[slot] = out;
+    if (rec_ext) rec_ext[slot] = make_float4(sigma_raw, o[r][3], __uint_as_float(m1[r]), __uint_as_float(m2[r]));
+  }
+}
+
+__global__ void __launch_bounds__(kPairThreads, kPairCtas) k_mlp_f32_pair(
     const float* __restrict__ W1, const float* __restrict__ b1, const float* __restrict__ W2,
     const float* __restrict__ b2, const float* __restrict__ W3, const float* __restrict__ b3,
     const float* __restrict__ freq, const float* __restrict__ att, const RecIn* __restrict__ rec_in,
-    const int4* __restrict__ work, int32_t* __restrict__ counters, float4* __restrict__ rec_out,
+    const int4* __restrict__ work, const int32_t* __restrict__ counters, float4* __restrict__ rec_out,
     float4* __restrict__ rec_ext, int out_mode, const int32_t* __restrict__ status) {
-  extern __shared__ __align__(16) float sW[];
-  __shared__ int s_item;
+  using B = PairBuf;
+  chain_wait();
+  chain_release();
+  extern __shared__ __align__(16) float sm[];
   if (status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
-  float* sW1T = sW;                          // [72][36]
-  float* sW2 = sW1T + kSIN * kSRow;          // [32][32]
-  float* sW3T = sW2 + kSH * kSH;             // [32][4]
-  float* sb1 = sW3T + kSH * 4;
-  float* sb2 = sb1 + kSH;
-  float* sb3 = sb2 + kSH;
+  const int tid = threadIdx.x, step = (int)gridDim.x;
+  const int G = counters[kCtrWork];
+  int item = blockIdx.x;
+  if (item >= G) return;
+  float fr[kTF], at[kTF];
+#pragma unroll
+  for (int f = 0; f < kTF; ++f) { fr[f] = __ldg(freq + f); at[f] = __ldg(att + f); }
+  const uint32_t s0 = smem_u32(sm);
+  auto copy = [&](const int4& w, int buf) {
+    const uint32_t d = s0 + 4u * (uint32_t)(buf * B::kFloats);
+    const size_t p = (size_t)w.x;
+    const float* w1 = W1 + p * (kTIN * 32);
+    int j = tid, h = 0;                                  // element i = u * 64 + tid of W1: unit h, input j
+#pragma unroll 4
+    for (int u = 0; u < kTIN * 32 / kPairThreads; ++u) {
+      cp_async4(d + 4u * (uint32_t)(B::kW1 + j * B::kRow + h), w1 + u * kPairThreads + tid);
+      j += kPairThreads;
+      if (j >= kTIN) { j -= kTIN; ++h; }
+    }
+    const float* w2 = W2 + p * (32 * 32);
+#pragma unroll 4
+    for (int u = 0; u < 32 * 32 / kPairThreads; ++u)
+      cp_async4(d + 4u * (uint32_t)(B::kW2 + (tid & 31) * B::kRow + 2 * u + (tid >> 5)), w2 + u * kPairThreads + tid);
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      cp_async4(d + 4u * (uint32_t)(B::kW3 + (tid & 31) * 4 + 2 * u + (tid >> 5)), W3 + p * 128 + u * kPairThreads + tid);
+    cp_async4(d + 4u * (uint32_t)(B::kB1 + tid), tid < 32 ? b1 + p * 32 + tid : b2 + p * 32 + tid - 32);
+    if (tid < 4) cp_async4(d + 4u * (uint32_t)(B::kB3 + tid), b3 + p * 4 + tid);
+    const char* rec = reinterpret_cast<const char*>(rec_in + w.y);
+    for (int c = tid; c < 2 * w.z; c += kPairThreads)    // the item's records, 32 bytes each
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 4u * (uint32_t)B::kRec + 16u * (uint32_t)c), "l"(rec + 16 * (size_t)c) : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // rows of a buffer that no record has filled are computed and dropped: let them hold numbers
+  for (int i = tid; i < kRowsPerItem * 8; i += kPairThreads) sm[B::kRec + i] = sm[B::kFloats + B::kRec + i] = 0.f;
+  __syncthreads();
+  int4 wk = __ldg(work + item), wn = wk;
+  copy(wk, 0);
+  if (item + step < G) wn = __ldg(work + item + step);
+  int buf = 0;
+  for (;;) {
+    const bool more = item + step < G;
+    int4 wn2 = wn;
+    if (more) {
+      copy(wn, buf ^ 1);
+      if (item + 2 * step < G) wn2 = __ldg(work + item + 2 * step);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    const float* cur = sm + buf * B::kFloats;
+    if (wk.z > kPairThreads) pair_eval<2>(cur, fr, at, tid, wk.z, rec_out, rec_ext, out_mode);
+    else if ((tid & ~31) < wk.z) pair_eval<1>(cur, fr, at, tid, wk.z, rec_out, rec_ext, out_mode);
+    if (!more) break;
+    __syncthreads();                       // the buffer has been read
+    item += step;
+    wk = wn;
+    wn = wn2;
+    buf ^= 1;
+  }
+}
+
+// The 72 -> 64 -> 64 -> 4 network, whose sums do not fit a thread's registers, as register-tiled products.  A work item's
+// records lie transposed in shared memory ([quantity][record], rows of 132 floats), the weights as [input][unit], and a
+// thread owns eight records of four units: per input three 16-byte reads feed 32 multiply-adds.  The next item's weights and
+// records are loaded into registers while the current one is computed.  Bound: FP32 multiply-adds, 9,216 per record; a
+// thread per record with scalar reads of its weights took 21.0 ms where this takes 5.1 (100k frame of 64-wide
+// layers).
+struct WideNet {
+  static constexpr int kH = 64, kThreads = 256, kWRow = kH + 4, kTRow = kRowsPerItem + 4;
+  static constexpr int kE = 0, kH1 = kE + kTIN * kTRow, kW1T = kH1 + kH * kTRow, kW2T = kW1T + kTIN * kWRow, kW3T = kW2T + kH * kWRow,
+                       kB1 = kW3T + 4 * kH, kB2 = kB1 + kH, kB3 = kB2 + kH, kFloats = kB3 + 4;
+  static constexpr int kCtas = 2;
+  static_assert(kH <= kTIN, "the second hidden layer takes the encoding's place");
+  static_assert(kCtas * (kFloats * 4 + 1024) <= 228 * 1024, "resident CTAs");
+};
+
+__global__ void __launch_bounds__(WideNet::kThreads, WideNet::kCtas) k_mlp_f32_wide(
+    const float* __restrict__ W1, const float* __restrict__ b1, const float* __restrict__ W2,
+    const float* __restrict__ b2, const float* __restrict__ W3, const float* __restrict__ b3,
+    const float* __restrict__ freq, const float* __restrict__ att, const RecIn* __restrict__ rec_in,
+    const int4* __restrict__ work, const int32_t* __restrict__ counters, float4* __restrict__ rec_out,
+    int out_mode, const int32_t* __restrict__ status) {
+  using N = WideNet;
+  constexpr int H = N::kH, kTRow = N::kTRow, kT = N::kThreads, kL1 = kTIN * H / kT, kL2 = H * H / kT;      // weights per thread
+  chain_wait();
+  chain_release();
+  extern __shared__ __align__(16) float sm[];
+  if (status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
   const int tid = threadIdx.x;
   const int G = counters[kCtrWork];
-  float fr[kSF], at[kSF];
+  int item = blockIdx.x;
+  if (item >= G) return;
+  float fr[kTF], at[kTF];
 #pragma unroll
-  for (int f = 0; f < kSF; ++f) { fr[f] = __ldg(freq + f); at[f] = __ldg(att + f); }
+  for (int f = 0; f < kTF; ++f) { fr[f] = __ldg(freq + f); at[f] = __ldg(att + f); }
+  const int rec = tid & (kRowsPerItem - 1), part = tid / kRowsPerItem;       // two threads encode a record
+  const int h4 = (tid % (H / 4)) * 4, r8 = (tid / (H / 4)) * 8;
+
+  float w1[kL1], w2[kL2], w3, bias = 0.f;
+  float4 q0, q1;
+  auto load = [&](const int4& w) {
+    const size_t p = (size_t)w.x;
+#pragma unroll
+    for (int u = 0; u < kL1; ++u) w1[u] = __ldg(W1 + p * (kTIN * H) + u * kT + tid);
+#pragma unroll
+    for (int u = 0; u < kL2; ++u) w2[u] = __ldg(W2 + p * (H * H) + u * kT + tid);
+    w3 = __ldg(W3 + p * (4 * H) + tid);
+    if (tid < H) bias = __ldg(b1 + p * H + tid);
+    else if (tid < 2 * H) bias = __ldg(b2 + p * H + tid - H);
+    else if (tid < 2 * H + 4) bias = __ldg(b3 + p * 4 + tid - 2 * H);
+    q0 = q1 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (rec < w.z) {
+      const float4* src = reinterpret_cast<const float4*>(rec_in) + 2 * (size_t)(w.y + rec);
+      q0 = __ldg(src);
+      q1 = __ldg(src + 1);
+    }
+  };
+  // acc[u][v] += w[k][h4 + u] * x[k][r8 + 2 v .. + 1]
+  unsigned long long acc[4][4];
+  auto step = [&](int x_off, int k, int w_off) {
+    const ulonglong2 xa = *reinterpret_cast<const ulonglong2*>(sm + x_off + k * kTRow + r8);
+    const ulonglong2 xb = *reinterpret_cast<const ulonglong2*>(sm + x_off + k * kTRow + r8 + 4);
+    const float4 w = *reinterpret_cast<const float4*>(sm + w_off + k * N::kWRow + h4);
+    const float wv[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const unsigned long long ww = pack_f32x2(wv[u], wv[u]);
+      fma_f32x2(acc[u][0], xa.x, ww); fma_f32x2(acc[u][1], xa.y, ww);
+      fma_f32x2(acc[u][2], xb.x, ww); fma_f32x2(acc[u][3], xb.y, ww);
+    }
+  };
+  auto start = [&](int b_off) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const float b = sm[b_off + h4 + u];
+#pragma unroll
+      for (int v = 0; v < 4; ++v) acc[u][v] = pack_f32x2(b, b);
+    }
+  };
+  auto relu_store = [&](int off) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const float2 a = unpack_f32x2(acc[u][0]), b = unpack_f32x2(acc[u][1]), c = unpack_f32x2(acc[u][2]), d = unpack_f32x2(acc[u][3]);
+      float* dst = sm + off + (h4 + u) * kTRow + r8;
+      *reinterpret_cast<float4*>(dst) = make_float4(fmaxf(a.x, 0.f), fmaxf(a.y, 0.f), fmaxf(b.x, 0.f), fmaxf(b.y, 0.f));
+      *reinterpret_cast<float4*>(dst + 4) = make_float4(fmaxf(c.x, 0.f), fmaxf(c.y, 0.f), fmaxf(d.x, 0.f), fmaxf(d.y, 0.f));
+    }
+  };
+
+  int4 wk = __ldg(work + item);
+  load(wk);
   for (;;) {
-    if (tid == 0) s_item = atomicAdd(counters + kCtrWorkNext, 1);
-    __syncthreads();
-    const int item = s_item;
-    if (item >= G) break;
-    const int4 wk = work[item];
-    const int p = wk.x;
-    for (int i = tid; i < kSH * kSIN; i += kRowsPerItem) {
-      const int h = i / kSIN, j = i - h * kSIN;
-      sW1T[j * kSRow + h] = W1[(size_t)p * kSH * kSIN + i];
-    }
-    for (int i = tid; i < kSH * kSH; i += kRowsPerItem) sW2[i] = W2[(size_t)p * kSH * kSH + i];
-    {
-      const int c = tid >> 5, q = tid & 31;   // 128 threads = 4 outputs x 32 hidden
-      sW3T[q * 4 + c] = W3[(size_t)p * 4 * kSH + c * kSH + q];
-    }
-    if (tid < kSH) { sb1[tid] = b1[(size_t)p * kSH + tid]; sb2[tid] = b2[(size_t)p * kSH + tid]; }
-    if (tid < 4) sb3[tid] = b3[(size_t)p * 4 + tid];
-    __syncthreads();
-    if (tid < wk.z) {
-      const RecIn r = rec_in[wk.y + tid];
-      const float v6[6] = {r.rdx, r.rdy, r.rdz, r.dx, r.dy, r.dz};
-      float h1[kSH];
+    const int rows = wk.z;
+    const float decay = q1.z;
+    const uint32_t slot = __float_as_uint(q1.w);
+    __syncthreads();                       // the previous item's layers have been read
 #pragma unroll
-      for (int k = 0; k < kSH / 4; ++k) {
-        const float4 b = reinterpret_cast<const float4*>(sb1)[k];
-        h1[4 * k] = b.x; h1[4 * k + 1] = b.y; h1[4 * k + 2] = b.z; h1[4 * k + 3] = b.w;
-      }
+    for (int u = 0; u < kL1; ++u) { const int i = u * kT + tid; sm[N::kW1T + (i % kTIN) * N::kWRow + i / kTIN] = w1[u]; }
+#pragma unroll
+    for (int u = 0; u < kL2; ++u) { const int i = u * kT + tid; sm[N::kW2T + (i % H) * N::kWRow + i / H] = w2[u]; }
+    sm[N::kW3T + (tid % H) * 4 + tid / H] = w3;
+    if (tid < 2 * H + 4) sm[N::kB1 + tid] = bias;
+    {
+      const float v6[6] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y};
 #pragma unroll
       for (int c = 0; c < 6; ++c) {
+        if ((c < 3) != (part == 0)) continue;
 #pragma unroll
-        for (int f = 0; f < kSF; ++f) {
+        for (int f = 0; f < kTF; ++f) {
           const float ph = v6[c] * fr[f] * at[f];
-          const float sn = __sinf(ph), cs = __cosf(ph);
-          const int j = c * kSF + f;
-          const float4* ws = reinterpret_cast<const float4*>(sW1T + j * kSRow);
-          const float4* wc = reinterpret_cast<const float4*>(sW1T + (j + kSIN / 2) * kSRow);
-#pragma unroll
-          for (int k = 0; k < kSH / 4; ++k) {
-            const float4 a = ws[k], b = wc[k];
-            h1[4 * k] = fmaf(b.x, cs, fmaf(a.x, sn, h1[4 * k]));
-            h1[4 * k + 1] = fmaf(b.y, cs, fmaf(a.y, sn, h1[4 * k + 1]));
-            h1[4 * k + 2] = fmaf(b.z, cs, fmaf(a.z, sn, h1[4 * k + 2]));
-            h1[4 * k + 3] = fmaf(b.w, cs, fmaf(a.w, sn, h1[4 * k + 3]));
-          }
+          sm[N::kE + (c * kTF + f) * kTRow + rec] = __sinf(ph);
+          sm[N::kE + (36 + c * kTF + f) * kTRow + rec] = __cosf(ph);
         }
       }
-      uint32_t m1 = 0u, m2 = 0u;
-#pragma unroll
-      for (int h = 0; h < kSH; ++h) {
-        if (h1[h] > 0.f) m1 |= 1u << h;
-        h1[h] = fmaxf(h1[h], 0.f);
-      }
-      float o0 = sb3[0], o1 = sb3[1], o2 = sb3[2], o3 = sb3[3];
+    }
+    const int next = item + (int)gridDim.x;
+    const bool more = next < G;
+    if (more) { wk = __ldg(work + next); load(wk); }
+    __syncthreads();
+    const bool live = r8 < rows;
+    if (live) {
+      start(N::kB1);
 #pragma unroll 4
-      for (int q = 0; q < kSH; ++q) {
-        float a = sb2[q];
-        const float4* row = reinterpret_cast<const float4*>(sW2 + q * kSH);
-#pragma unroll
-        for (int k = 0; k < kSH / 4; ++k) {
-          const float4 w = row[k];
-          a = fmaf(w.x, h1[4 * k], a); a = fmaf(w.y, h1[4 * k + 1], a);
-          a = fmaf(w.z, h1[4 * k + 2], a); a = fmaf(w.w, h1[4 * k + 3], a);
-        }
-        if (a > 0.f) m2 |= 1u << q;
-        a = fmaxf(a, 0.f);
-        const float4 w3 = reinterpret_cast<const float4*>(sW3T)[q];
-        o0 = fmaf(w3.x, a, o0); o1 = fmaf(w3.y, a, o1); o2 = fmaf(w3.z, a, o2); o3 = fmaf(w3.w, a, o3);
+      for (int j = 0; j < kTIN / 2; ++j) { step(N::kE, j, N::kW1T); step(N::kE, kTIN / 2 + j, N::kW1T); }
+      relu_store(N::kH1);
+    }
+    __syncthreads();
+    if (live) {
+      start(N::kB2);
+#pragma unroll 8
+      for (int k = 0; k < H; ++k) step(N::kH1, k, N::kW2T);
+      relu_store(N::kE);                   // the encoding has been read
+    }
+    __syncthreads();
+    if (tid < rows) {
+      float o0 = sm[N::kB3], o1 = sm[N::kB3 + 1], o2 = sm[N::kB3 + 2], o3 = sm[N::kB3 + 3];
+#pragma unroll 8
+      for (int q = 0; q < H; ++q) {
+        const float a = sm[N::kE + q * kTRow + tid];
+        const float4 w = *reinterpret_cast<const float4*>(sm + N::kW3T + q * 4);
+        o0 = fmaf(w.x, a, o0); o1 = fmaf(w.y, a, o1); o2 = fmaf(w.z, a, o2); o3 = fmaf(w.w, a, o3);
       }
       const float sigma_raw = softplus_fast(o3);
       float4 out;
       out.x = sigmoid_fast(o0); out.y = sigmoid_fast(o1); out.z = sigmoid_fast(o2);
-      out.w = (out_mode == kOutAlpha) ? (1.f - __expf(-(sigma_raw * r.decay))) : sigma_raw;
-      rec_out[r.slot] = out;
-      if (rec_ext) rec_ext[r.slot] = make_float4(sigma_raw, o3, __uint_as_float(m1), __uint_as_float(m2));
+      out.w = (out_mode == kOutAlpha) ? (1.f - __expf(-(sigma_raw * decay))) : sigma_raw;
+      rec_out[slot] = out;
     }
-    __syncthreads();
+    if (!more) break;
+    item = next;
   }
 }
 
@@ -211,11 +476,25 @@ int launch_mlp_f32(const mlpsp_scene* sc, const RecIn* rec_in, const int4* work,
   const int grid = grid_cap > 0 ? std::min(grid_cap, sms * 8) : sms * 8;
   int32_t* ctr = const_cast<int32_t*>(counters);
   LaunchScope scope(kKMlp, 1, st);
-  if (H == kSH && F == kSF) {
-    k_mlp_f32_std<<<grid, kRowsPerItem, sizeof(float) * kStdSmemFloats, st>>>(
-        sc->W1, sc->b1, sc->W2, sc->b2, sc->W3, sc->b3, sc->freq, sc->att, rec_in, work, ctr, rec_out, rec_ext, out_mode,
-        status);
-  } else if (H <= 32) {
+  if (F == kTF && H == 32) {
+    static_assert(2 * sizeof(float) * PairBuf::kFloats <= 48 * 1024, "no opt-in needed");
+    const int want = sms * kPairCtas;
+    return cuda_check(launch_chained(k_mlp_f32_pair, dim3(grid_cap > 0 ? std::min(grid_cap, want) : want), dim3(kPairThreads),
+                                     2 * sizeof(float) * PairBuf::kFloats, st, sc->W1, sc->b1, sc->W2, sc->b2, sc->W3, sc->b3, sc->freq, sc->att,
+                                     rec_in, work, ctr, rec_out, rec_ext, out_mode, status),
+                      "mlp_f32");
+  }
+  if (F == kTF && H == 64 && !rec_ext) {
+    using N = WideNet;
+    static DeviceOnce attr_once;
+    if (attr_once.first())
+      MLPSP_CUDA_OK(cudaFuncSetAttribute(k_mlp_f32_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, N::kFloats * 4));
+    const int want = sms * N::kCtas;
+    return cuda_check(launch_chained(k_mlp_f32_wide, dim3(grid_cap > 0 ? std::min(grid_cap, want) : want), dim3(N::kThreads), N::kFloats * 4, st,
+                                     sc->W1, sc->b1, sc->W2, sc->b2, sc->W3, sc->b3, sc->freq, sc->att, rec_in, work, ctr, rec_out, out_mode, status),
+                      "mlp_f32");
+  }
+  if (H <= 32) {
     k_mlp_f32<32><<<grid, kRowsPerItem, smem, st>>>(sc->W1, sc->b1, sc->W2, sc->b2, sc->W3, sc->b3, sc->freq, sc->att,
                                                    F, H, rec_in, work, ctr, rec_out, rec_ext, out_mode, status);
   } else {
