@@ -5,18 +5,24 @@
 // The reference adds C values to global memory per hit.  Per tile this is a product
 //   D^T [C x 64 pixels] = Attr^T [C x K] . Coef [K x 64 pixels],   K = (touched primitives of the tile) x S,
 // where Coef holds w * g_s of the consumed (pixel, primitive) records and zeros elsewhere.  One CTA owns one
-// (tile, block of 128 or 256 channels) and walks the tile's touched primitives 16 at a time:
+// (tile, block of up to 512 channels) and walks the tile's touched primitives 8 or 16 at a time:
 //   * the attribute rows (binary16, the reference's inference storage format, scannet/checkpoints.py:358-359) are
 //     gathered from this GPU's memory with cp.async into the MN-major core-matrix layout (eight K rows of eight
 //     channels = 128 bytes) that tcgen05.mma reads as its A operand: the channel dimension is M, so all 128 rows
 //     of the tensor core carry channels;
-//   * every thread turns four (pixel, primitive) cells into coefficients: weight and gates of the record when the
-//     pixel composited the primitive, zero otherwise, split into a binary16 head and a binary16 tail so that the
+//   * every thread turns two or four (pixel, primitive) cells into coefficients: weight and gates of the record when
+//     the pixel composited the primitive, zero otherwise, split into a binary16 head and a binary16 tail so that the
 //     two products together carry 22 mantissa bits (the attributes themselves are exact);
 //   * one thread issues the MMAs of the stage (128 x 64 x 16 each, FP32 accumulators in tensor memory) and commits
 //     them to the mbarrier that guards the stage's buffers; the other stage is filled meanwhile.
 // The copies and the record loads of the next stage are in flight while a stage is finished.
 // Afterwards each warp reads its 32 channels x 64 pixels from tensor memory and writes 128-byte lines of the map.
+//
+// The coefficients do not depend on the channel, so all channels share them where shared memory lets two CTAs of that
+// shape stay on an SM.  Bound: issue slots and the latency of the gather (each (tile, primitive) pair reads S * C * 2
+// bytes, from L2 for the most part); the map's own writes take 0.25 ms of a 1200 x 680 x 512 frame.  With blocks of 256
+// channels, every coefficient twice and addresses per copy, that frame (250k primitives) took 1.10 ms here, now 0.80;
+// a 957 x 541 x 128 one 0.26, now 0.24.
 //
 // Every wait on an mbarrier is bounded (MLPSP_ST_TIMEOUT), copies in flight are waited for, tensor memory is freed.
 #include "frame.cuh"
@@ -25,7 +31,6 @@
 namespace mlpsp {
 
 constexpr int kFtThreads = 256;
-constexpr int kFtPairs = 16;          // touched primitives per stage
 constexpr int kFtListMax = 2048;      // candidates of a tile the kernel looks at (kWinMax of the wave kernels)
 constexpr int kFtMeta = 256;          // touched primitives whose masks and bases are held in shared memory at a time
 
@@ -51,23 +56,25 @@ __host__ __device__ constexpr uint32_t ft_instr_desc(int M, int N) {
 
 // shared memory of one stage: A [K/8 groups of eight K rows][CB/8 groups of eight channels][8 rows][8 halves],
 // then the coefficient heads and tails [K/8 chunks][64 pixels][8 halves] each
-template <int S>
+// for PR primitives of S slots
+template <int S, int PR>
 struct FtPlan {
-  static constexpr int K = kFtPairs * S;                       // 16 / 64 / 80, a multiple of the MMA's K = 16
+  static constexpr int K = PR * S;
+  static_assert(K % 16 == 0, "whole MMA steps");
   __host__ __device__ static constexpr int a_bytes(int CB) { return K * CB * 2; }
   static constexpr int kCoefBytes = 64 * K * 2;
   __host__ __device__ static constexpr int stage_bytes(int CB) { return a_bytes(CB) + 2 * kCoefBytes; }
   __host__ __device__ static constexpr int smem_bytes(int CB) { return 2 * stage_bytes(CB) + 2 * kFtListMax + kFtMeta * 24 + 64; }
 };
 
-template <int S>
+template <int S, int PR>
 __global__ void __launch_bounds__(kFtThreads, 2) k_feature_tc(
     const int32_t* __restrict__ tile_offsets, const int32_t* __restrict__ tile_len, const int32_t* __restrict__ sorted_prims,
     int W, int H, int ntx, const uint32_t* __restrict__ used32, const uint32_t* __restrict__ masks32,
     const uint32_t* __restrict__ pair_base, const float* __restrict__ rec_w, const float4* __restrict__ rec_gate,
     const __half* __restrict__ feat16, int C, int CB, float* __restrict__ out_feat, int32_t* __restrict__ status) {
-  using P = FtPlan<S>;
-  constexpr int K = P::K;
+  using P = FtPlan<S, PR>;
+  constexpr int K = P::K, NC = PR / 4;              // NC cells per thread and stage
   extern __shared__ __align__(128) char smem[];
   __shared__ int warp_sums[32];
   if (status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
@@ -81,7 +88,7 @@ __global__ void __launch_bounds__(kFtThreads, 2) k_feature_tc(
   const uint32_t sb = smem_u32(smem);
   const uint32_t bar0 = smem_u32(&s_bar[0]);
   const int nb128 = CB / 128;
-  const uint32_t tmem_cols = nb128 == 2 ? 128u : 64u;
+  const uint32_t tmem_cols = nb128 > 2 ? 256u : (uint32_t)nb128 * 64u;
   if (tid == 0) {
     mbar_init(bar0, 1);
     mbar_init(bar0 + 8, 1);
@@ -114,81 +121,94 @@ __global__ void __launch_bounds__(kFtThreads, 2) k_feature_tc(
   const uint32_t idesc = ft_instr_desc(128, 64);
   bool ok = true;
   int gs = 0;                                     // stages issued so far: buffer = gs & 1, use of that buffer = gs >> 1
-  const int px = tid & 63;
+  const int half = warp & 1, px = half * 32 + lane, pl0 = (warp >> 1) * NC;     // this thread's cells of a stage: primitives pl0.. of pixel px
 
   // the MMAs that last read the buffer of stage g (two stages earlier) have finished
   auto buffer_free = [&](int g) {
     if (g >= 2) ok = mbar_wait(bar0 + 8 * (g & 1), (uint32_t)((g >> 1) - 1) & 1u) && ok;
   };
-  // Attribute rows of the 16 primitives from touched index t0 on (batch-local index l0): a warp copies eight K rows x
-  // four channel groups at a time, so that eight lanes fill one 128-byte core matrix (no bank conflicts) and four
-  // lanes read 64 contiguous bytes.  One cp.async group per stage.
+  // Attribute rows of the PR primitives from touched index l0 of the batch on: a warp copies eight K rows x four channel
+  // groups at a time, so that eight lanes fill one 128-byte core matrix (no bank conflicts) and four lanes read 64
+  // contiguous bytes; its rows stay, so the next copy is 64 bytes on.  One cp.async group per stage.
   auto issue_copies = [&](int g, int l0, int nb) {
-    const uint32_t a_s = sb + (g & 1) * stage_bytes;
-    const int gq_n = CB / 32;
-    for (int task = warp; task < (K / 8) * gq_n; task += kFtThreads / 32) {
-      const int kg = task / gq_n, gq = task - kg * gq_n;
-      const int k = kg * 8 + (lane & 7), grp = gq * 4 + (lane >> 3);
-      const int pl = k / S, sl = k - pl * S;
+    constexpr int KG = K / 8, parts = KG < kFtThreads / 32 ? kFtThreads / 32 / KG : 1;     // row groups; warps that share one
+    const int gq_n = CB / 32 / parts;
+    for (int task = warp; task < KG * parts; task += kFtThreads / 32) {
+      const int kg = task % KG, grp = (task / KG) * gq_n * 4 + (lane >> 3);
+      const int k = kg * 8 + (lane & 7), pl = k / S, sl = k - pl * S;
       const bool valid = l0 + pl < nb;
       const int prim = valid ? s_meta[l0 + pl].prim : 0;
       const __half* src = feat16 + ((size_t)prim * S + sl) * C + c0 + grp * 8;
-      ft_cp_async16(a_s + kg * lbo_a + grp * 128 + (lane & 7) * 16, src, valid);
+      uint32_t dst = sb + (g & 1) * stage_bytes + kg * lbo_a + grp * 128 + (lane & 7) * 16;
+#pragma unroll 4
+      for (int gq = 0; gq < gq_n; ++gq) {
+        ft_cp_async16(dst, src, valid);
+        src += 32;
+        dst += 512;
+      }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  // weight and gates of this thread's four (pixel, primitive) cells of a stage; zero where the pixel did not
-  // composite the primitive
-  auto load_cells = [&](int l0, int nb, float (&cw)[kFtPairs / 4], float4 (&cg)[kFtPairs / 4]) {
+  // weight and gates of this thread's cells of a stage; zero where the pixel did not composite the primitive
+  auto load_cells = [&](int l0, int nb, float (&cw)[NC], float4 (&cg)[NC]) {
 #pragma unroll
-    for (int i = 0; i < kFtPairs / 4; ++i) {
-      const int l = l0 + (tid >> 6) + 4 * i;
+    for (int i = 0; i < NC; ++i) {
+      const int l = l0 + pl0 + i;
       cw[i] = 0.f;
       cg[i] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (l < nb) {
-        const FtMeta m = s_meta[l];
-        const uint32_t u = px < 32 ? m.u0 : m.u1;
-        if ((u >> (px & 31)) & 1u) {
-          const uint32_t slot = m.base + (px < 32 ? __popc(m.m0 & ((1u << px) - 1u))
-                                                  : __popc(m.m0) + __popc(m.m1 & ((1u << (px - 32)) - 1u)));
+        const FtMeta& m = s_meta[l];
+        if (((half ? m.u1 : m.u0) >> lane) & 1u) {
+          const uint32_t slot = m.base + (half ? __popc(m.m0) : 0) + __popc((half ? m.m1 : m.m0) & ((1u << lane) - 1u));
           cw[i] = __ldg(rec_w + slot);
           if (S > 1) cg[i] = __ldg(rec_gate + slot);
         }
       }
     }
   };
+  // two coefficients -> packed heads and tails
+  auto split2 = [](float a, float b, uint32_t& hi, uint32_t& lo) {
+    const __half2 h = __floats2half2_rn(a, b);
+    const float2 f = __half22float2(h);
+    const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+  };
   // coefficients of the cells, head + tail in binary16; K index of slot sl of the stage's primitive pl is pl * S + sl,
   // element (pixel, k) sits at (k / 8) * 1024 + pixel * 16 + (k % 8) * 2
-  auto write_coefs = [&](int g, const float (&cw)[kFtPairs / 4], const float4 (&cg)[kFtPairs / 4]) {
+  auto write_coefs = [&](int g, const float (&cw)[NC], const float4 (&cg)[NC]) {
     char* coef_hi = smem + (g & 1) * stage_bytes + a_bytes;
     char* coef_lo = coef_hi + P::kCoefBytes;
+    if (S == 4) {                                       // two primitives fill the pixel's 16 bytes of one K group
 #pragma unroll
-    for (int i = 0; i < kFtPairs / 4; ++i) {
-      const int pl = (tid >> 6) + 4 * i;
-      const float w = cw[i];
-      float cf[5];
-      if (S == 1) { cf[0] = w; }
-      else if (S == 4) { cf[0] = w * cg[i].x; cf[1] = w * cg[i].y; cf[2] = w * cg[i].z; cf[3] = w * cg[i].w; }
-      else { cf[0] = w; cf[1] = w * cg[i].x; cf[2] = w * cg[i].y; cf[3] = w * cg[i].z; cf[4] = w * cg[i].w; }
-      __half hi[5], lo[5];
+      for (int i = 0; i < NC; i += 2) {
+        uint32_t h[4], l[4];
 #pragma unroll
-      for (int sl = 0; sl < S; ++sl) {
-        hi[sl] = __float2half_rn(cf[sl]);
-        lo[sl] = __float2half_rn(cf[sl] - __half2float(hi[sl]));
+        for (int j = 0; j < 2; ++j) {
+          split2(cw[i + j] * cg[i + j].x, cw[i + j] * cg[i + j].y, h[2 * j], l[2 * j]);
+          split2(cw[i + j] * cg[i + j].z, cw[i + j] * cg[i + j].w, h[2 * j + 1], l[2 * j + 1]);
+        }
+        const int off = ((pl0 + i) >> 1) * 1024 + px * 16;
+        *reinterpret_cast<uint4*>(coef_hi + off) = make_uint4(h[0], h[1], h[2], h[3]);
+        *reinterpret_cast<uint4*>(coef_lo + off) = make_uint4(l[0], l[1], l[2], l[3]);
       }
-      if (S == 4) {
-        const int off = (pl >> 1) * 1024 + px * 16 + (pl & 1) * 8;
-        *reinterpret_cast<uint2*>(coef_hi + off) = make_uint2((uint32_t)__half_as_ushort(hi[0]) | ((uint32_t)__half_as_ushort(hi[1]) << 16),
-                                                              (uint32_t)__half_as_ushort(hi[2]) | ((uint32_t)__half_as_ushort(hi[3]) << 16));
-        *reinterpret_cast<uint2*>(coef_lo + off) = make_uint2((uint32_t)__half_as_ushort(lo[0]) | ((uint32_t)__half_as_ushort(lo[1]) << 16),
-                                                              (uint32_t)__half_as_ushort(lo[2]) | ((uint32_t)__half_as_ushort(lo[3]) << 16));
-      } else {
+    } else if (S == 1) {                                // four primitives: eight of the sixteen bytes
+      uint32_t h[2], l[2];
+      split2(cw[0], cw[1], h[0], l[0]);
+      split2(cw[NC > 2 ? 2 : 0], cw[NC > 3 ? 3 : 0], h[1], l[1]);
+      const int off = (pl0 >> 3) * 1024 + px * 16 + (pl0 & 7) * 2;
+      *reinterpret_cast<uint2*>(coef_hi + off) = make_uint2(h[0], h[1]);
+      *reinterpret_cast<uint2*>(coef_lo + off) = make_uint2(l[0], l[1]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < NC; ++i) {
+        const float cf[5] = {cw[i], cw[i] * cg[i].x, cw[i] * cg[i].y, cw[i] * cg[i].z, cw[i] * cg[i].w};
 #pragma unroll
         for (int sl = 0; sl < S; ++sl) {
-          const int k = pl * S + sl;
-          const int off = (k >> 3) * 1024 + px * 16 + (k & 7) * 2;
-          *reinterpret_cast<__half*>(coef_hi + off) = hi[sl];
-          *reinterpret_cast<__half*>(coef_lo + off) = lo[sl];
+          const int k = (pl0 + i) * S + sl, off = (k >> 3) * 1024 + px * 16 + (k & 7) * 2;
+          const __half hi = __float2half_rn(cf[sl]);
+          *reinterpret_cast<__half*>(coef_hi + off) = hi;
+          *reinterpret_cast<__half*>(coef_lo + off) = __float2half_rn(cf[sl] - __half2float(hi));
         }
       }
     }
@@ -206,11 +226,11 @@ __global__ void __launch_bounds__(kFtThreads, 2) k_feature_tc(
       s_meta[l] = e;
     }
     __syncthreads();
-    // ---- stages of 16 primitives; the copies and the record loads of stage l+1 are in flight while stage l is
+    // ---- stages of PR primitives; the copies and the record loads of stage l+1 are in flight while stage l is
     // finished and handed to the tensor cores ----
-    const int nsb = (nb + kFtPairs - 1) / kFtPairs;
-    float cw[kFtPairs / 4];
-    float4 cg[kFtPairs / 4];
+    const int nsb = (nb + PR - 1) / PR;
+    float cw[NC];
+    float4 cg[NC];
     buffer_free(gs);
     issue_copies(gs, 0, nb);
     load_cells(0, nb, cw, cg);
@@ -219,10 +239,10 @@ __global__ void __launch_bounds__(kFtThreads, 2) k_feature_tc(
       const bool more = ls + 1 < nsb;
       if (more) {
         buffer_free(g + 1);
-        issue_copies(g + 1, (ls + 1) * kFtPairs, nb);
+        issue_copies(g + 1, (ls + 1) * PR, nb);
       }
       write_coefs(g, cw, cg);
-      if (more) load_cells((ls + 1) * kFtPairs, nb, cw, cg);
+      if (more) load_cells((ls + 1) * PR, nb, cw, cg);
       if (more) asm volatile("cp.async.wait_group 1;" ::: "memory");
       else asm volatile("cp.async.wait_group 0;" ::: "memory");
       fence_async_smem();
@@ -258,10 +278,10 @@ __global__ void __launch_bounds__(kFtThreads, 2) k_feature_tc(
   ok = __all_sync(0xffffffffu, ok);
   tc_fence_after();
   // ---- epilogue: warp = 32 channels of one 128-channel half, thread = channel, 64 pixels from tensor memory ----
-  const int q = warp & 3, h = warp >> 2;
-  if (h < nb128) {
-    const int c = c0 + h * 128 + q * 32 + lane;
-    const int x0 = (tile % ntx) * 8, y0 = (tile / ntx) * 8;
+  const int q = warp & 3;
+  const int x0 = (tile % ntx) * 8, y0 = (tile / ntx) * 8;
+  for (int h = warp >> 2; h < nb128; h += 2) {
+    float* dst = out_feat + ((size_t)y0 * W + x0) * C + c0 + h * 128 + q * 32 + lane;
 #pragma unroll 1
     for (int part = 0; part < 2; ++part) {
       uint32_t v[32];
@@ -271,10 +291,15 @@ __global__ void __launch_bounds__(kFtThreads, 2) k_feature_tc(
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] = 0u;
       }
+      // streaming stores: the map is not read again here, the attributes in L2 are
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const int x = x0 + (i & 7), y = y0 + part * 4 + (i >> 3);      // pixel part * 32 + i of the tile
-        if (x < W && y < H) out_feat[((size_t)y * W + x) * C + c] = __uint_as_float(v[i]);
+      for (int r = 0; r < 4; ++r) {
+        const int y = part * 4 + r;
+        if (y0 + y >= H) break;
+        float* row = dst + (size_t)y * W * C;
+#pragma unroll
+        for (int x = 0; x < 8; ++x)
+          if (x0 + x < W) __stcs(row + (size_t)x * C, __uint_as_float(v[r * 8 + x]));
       }
     }
   }
@@ -306,27 +331,29 @@ bool feature_tc_supported(const mlpsp_scene* sc) {
          (reinterpret_cast<uintptr_t>(sc->feat16) & 15) == 0;
 }
 
-template <int S>
-static int launch_ft(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, const uint32_t* used32, int T, int ntx,
+// Channels per CTA: all of them while two CTAs fit an SM.  Stages of 16 primitives take S * CB * 32 bytes of attributes
+// and S * 4,096 of coefficients, twice; eight primitives (whole K = 16 steps for four slots only) half of that.
+template <int S, int PR>
+static int launch_ft(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, const uint32_t* used32, int T, int ntx, int CB,
                      cudaStream_t st) {
-  const int C = sc->feat_dim;
-  const int CB = (C % 256 == 0) ? 256 : 128;
-  const int smem = FtPlan<S>::smem_bytes(CB);
+  const int smem = FtPlan<S, PR>::smem_bytes(CB);
   static DeviceOnce attr_once;
   if (attr_once.first())
-    MLPSP_CUDA_OK(cudaFuncSetAttribute(k_feature_tc<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, FtPlan<S>::smem_bytes(256)));
-  const dim3 grid(T, C / CB);
-  k_feature_tc<S><<<grid, kFtThreads, smem, st>>>(fr->tile_offsets, s.tile_len, fr->sorted_prims, fr->width, fr->height, ntx, used32,
-                                                  s.masks32, s.pair_base, s.rec_w, s.rec_gate, (const __half*)sc->feat16, C, CB,
-                                                  fr->feat, fr->status);
+    MLPSP_CUDA_OK(cudaFuncSetAttribute(k_feature_tc<S, PR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 113 * 1024));
+  const dim3 grid(T, sc->feat_dim / CB);
+  k_feature_tc<S, PR><<<grid, kFtThreads, smem, st>>>(fr->tile_offsets, s.tile_len, fr->sorted_prims, fr->width, fr->height, ntx, used32,
+                                                      s.masks32, s.pair_base, s.rec_w, s.rec_gate, (const __half*)sc->feat16, sc->feat_dim, CB,
+                                                      fr->feat, fr->status);
   return cuda_check(cudaGetLastError(), "feature_tc");
 }
 
 int launch_feature_tc(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, const uint32_t* used32, cudaStream_t st) {
   const int T = num_tiles(fr->width, fr->height, 8), ntx = (fr->width + 7) / 8;
-  if (sc->feat_slots == 1) return launch_ft<1>(sc, fr, s, used32, T, ntx, st);
-  if (sc->feat_slots == 4) return launch_ft<4>(sc, fr, s, used32, T, ntx, st);
-  return launch_ft<5>(sc, fr, s, used32, T, ntx, st);
+  const int C = sc->feat_dim, narrow = C % 256 == 0 ? 256 : 128;
+  if (sc->feat_slots == 1) return launch_ft<1, 16>(sc, fr, s, used32, T, ntx, C, st);
+  if (sc->feat_slots == 5) return launch_ft<5, 16>(sc, fr, s, used32, T, ntx, 128, st);
+  if (C <= 256) return launch_ft<4, 16>(sc, fr, s, used32, T, ntx, narrow, st);
+  return launch_ft<4, 8>(sc, fr, s, used32, T, ntx, C, st);
 }
 
 }  // namespace mlpsp
