@@ -108,132 +108,172 @@ __device__ __forceinline__ void fma_f32x2(unsigned long long& acc, unsigned long
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
 
-// The 72 -> 32 -> 32 -> 4 network: 64 threads per work item, one or two records per thread, the hidden sums in registers as
-// packed pairs of units (fma.rn.f32x2: two IEEE multiply-adds, so every sum keeps the order and the bits described at the top
-// of this file).  The weights lie transposed in shared memory ([input][unit]); a row of 32 weights takes eight broadcast
-// 16-byte reads, whose halves are the packed operands, and feeds 64 multiply-adds.  The next item's weights and records are
-// copied (asynchronously, transposed on the way) while the current one is computed.  Bound: FP32 multiply-adds, 3,456 per
-// record -- 36 G on the 100k frame, 1.0 ms at the chip's rate -- and the broadcast reads.  With one record per thread and
-// scalar multiply-adds the reads bounded it at 2.75 ms; this takes 2.26 ms (five CTAs per SM, 168 registers: 2.55).
+// The 72 -> 32 -> 32 -> 4 network: 64 threads per work item.  A thread owns up to four records of sixteen units (the other
+// half-warp the other sixteen), the sums in registers as packed pairs of units (fma.rn.f32x2: two IEEE multiply-adds, so
+// every sum keeps the order and the bits described at the top of this file).  The weights lie transposed in shared memory
+// ([input][unit]): four broadcast 16-byte reads per input, whose halves are the packed operands, feed 64 multiply-adds.  The
+// half-warps exchange the hidden units through shared memory, in the place of the first layer's weights and the records.
+// The weights are copied asynchronously and transposed on the way; six CTAs per SM (three warps on each scheduler) cover one
+// another's copies, and take their items from a counter.
+// Bound: FP32 multiply-adds, 3,456 per record -- 36 G on the 100k frame, 1.0 ms at the chip's rate, 1.2 with the rows that
+// fill up an item's last 32.  One record per thread with scalar multiply-adds, bounded by the broadcast reads (two cycles
+// each), took 2.75 ms; two records of all units per thread 2.26; this 1.86 (five CTAs of two buffers and a fixed order of
+// the items 2.31, seven or eight CTAs of 128 registers 2.08 and 1.97).
 struct PairBuf {
-  static constexpr int kRow = 36;          // floats per row: 16-byte aligned, and the transposing copies spread over the banks
-  static constexpr int kW1 = 0, kW2 = kW1 + kTIN * kRow, kW3 = kW2 + 32 * kRow, kB1 = kW3 + 128, kB2 = kB1 + 32, kB3 = kB2 + 32,
-                       kRec = kB3 + 4, kFloats = kRec + kRowsPerItem * 8;
+  static constexpr int kRow = 36;          // floats per row of weights: 16-byte aligned, conflict-free transposing copies
+  static constexpr int kRecRow = 12;       // floats per record: 16-byte aligned, neighbouring records on different banks
+  static constexpr int kW1 = 0, kRec = kW1 + kTIN * kRow, kW2 = kRec + kRowsPerItem * kRecRow, kW3 = kW2 + 32 * kRow, kB1 = kW3 + 128,
+                       kB2 = kB1 + 32, kB3 = kB2 + 32, kFloats = kB3 + 4;
+  static constexpr int kHid = 0, kHidWarp = 32 * 64;      // hidden units of a warp's records, after layer 1
+  static_assert(2 * kHidWarp <= kW2, "the hidden units take the place of W1 and the records");
+  static_assert(kRec % 4 == 0 && kW2 % 4 == 0 && kFloats % 4 == 0, "16-byte accesses");
 };
-static_assert(PairBuf::kRec % 4 == 0 && PairBuf::kFloats % 4 == 0, "16-byte copies");
-constexpr int kPairThreads = 64, kPairCtas = 4;
+constexpr int kPairThreads = 64, kPairCtas = 6;
 
 __device__ __forceinline__ void cp_async4(uint32_t dst, const float* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 
-// one row of 32 weights onto the sums of NR records
-template <int NR>
-__device__ __forceinline__ void row_fma(unsigned long long (&acc)[NR][16], const float* row, const float (&x)[NR]) {
-  unsigned long long xx[NR];
+// one row of sixteen weights onto the sums of R records
+template <int R>
+__device__ __forceinline__ void row_fma(unsigned long long (&acc)[R][8], const float* row, const float (&x)[R]) {
+  unsigned long long xx[R];
 #pragma unroll
-  for (int r = 0; r < NR; ++r) xx[r] = pack_f32x2(x[r], x[r]);
+  for (int r = 0; r < R; ++r) xx[r] = pack_f32x2(x[r], x[r]);
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
+  for (int k = 0; k < 4; ++k) {
     const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(row + 4 * k);
 #pragma unroll
-    for (int r = 0; r < NR; ++r) { fma_f32x2(acc[r][2 * k], w.x, xx[r]); fma_f32x2(acc[r][2 * k + 1], w.y, xx[r]); }
+    for (int r = 0; r < R; ++r) { fma_f32x2(acc[r][2 * k], w.x, xx[r]); fma_f32x2(acc[r][2 * k + 1], w.y, xx[r]); }
   }
 }
-template <int NR>
-__device__ __forceinline__ void row_start(unsigned long long (&acc)[NR][16], const float* bias) {
+template <int R>
+__device__ __forceinline__ void row_start(unsigned long long (&acc)[R][8], const float* bias) {
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
+  for (int k = 0; k < 4; ++k) {
     const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(bias + 4 * k);
 #pragma unroll
-    for (int r = 0; r < NR; ++r) { acc[r][2 * k] = b.x; acc[r][2 * k + 1] = b.y; }
+    for (int r = 0; r < R; ++r) { acc[r][2 * k] = b.x; acc[r][2 * k + 1] = b.y; }
   }
 }
-// ReLU of the sums; bit u of mask: unit u is positive
-template <int NR>
-__device__ __forceinline__ void row_relu(const unsigned long long (&acc)[NR][16], float (&h)[NR][32], uint32_t (&mask)[NR], bool want) {
+// R values of a lane as one vector of V >= R floats (V = 1, 2, 4)
+template <int R, int V>
+__device__ __forceinline__ void put_vec(float* p, const float (&x)[R]) {
+  if (V == 4) *reinterpret_cast<float4*>(p) = make_float4(x[0], x[R > 1 ? 1 : 0], x[R > 2 ? 2 : 0], x[R > 3 ? 3 : 0]);
+  else if (V == 2) *reinterpret_cast<float2*>(p) = make_float2(x[0], x[R > 1 ? 1 : 0]);
+  else *p = x[0];
+}
+template <int R, int V>
+__device__ __forceinline__ void get_vec(const float* p, float (&x)[R]) {
+  float v[4];
+  if (V == 4) { const float4 q = *reinterpret_cast<const float4*>(p); v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w; }
+  else if (V == 2) { const float2 q = *reinterpret_cast<const float2*>(p); v[0] = q.x; v[1] = q.y; }
+  else v[0] = *p;
 #pragma unroll
-  for (int r = 0; r < NR; ++r) {
-    mask[r] = 0u;
+  for (int r = 0; r < R; ++r) x[r] = v[r];
+}
+// ReLU of the sums to the warp's exchange area; bit u of mask: this half's unit u is positive
+template <int R, int V>
+__device__ __forceinline__ void relu_put(const unsigned long long (&acc)[R][8], float* hid, int lane, uint32_t (&mask)[R], bool want) {
+  const int half = lane >> 4, l16 = lane & 15;
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
+  for (int r = 0; r < R; ++r) mask[r] = 0u;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    float a[R], b[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
       const float2 v = unpack_f32x2(acc[r][k]);
-      h[r][2 * k] = v.x;
-      h[r][2 * k + 1] = v.y;
+      if (want) mask[r] |= ((v.x > 0.f ? 1u : 0u) | (v.y > 0.f ? 2u : 0u)) << (2 * k);
+      a[r] = fmaxf(v.x, 0.f);
+      b[r] = fmaxf(v.y, 0.f);
     }
-    if (want) {
-#pragma unroll
-      for (int k = 0; k < 32; ++k) mask[r] |= (h[r][k] > 0.f ? 1u : 0u) << k;
-    }
-#pragma unroll
-    for (int k = 0; k < 32; ++k) h[r][k] = fmaxf(h[r][k], 0.f);
+    put_vec<R, V>(hid + (half * 16 + 2 * k) * (16 * V) + l16 * V, a);
+    put_vec<R, V>(hid + (half * 16 + 2 * k + 1) * (16 * V) + l16 * V, b);
   }
 }
 
-template <int NR>
-__device__ __forceinline__ void pair_eval(const float* sm, const float (&fr)[kTF], const float (&at)[kTF], int tid, int rows,
-                                          float4* __restrict__ rec_out, float4* __restrict__ rec_ext, int out_mode) {
+// R * 32 records of an item; record r of a lane is warp * 16 R + 16 r + lane % 16
+template <int R>
+__device__ __forceinline__ void pair_eval(float* sm, const float* s_freq, int warp, int lane, int rows, float4* __restrict__ rec_out,
+                                          float4* __restrict__ rec_ext, int out_mode) {
   using B = PairBuf;
-  unsigned long long acc[NR][16];
-  float h[NR][32];
-  uint32_t m1[NR], m2[NR];
-  row_start<NR>(acc, sm + B::kB1);
+  constexpr int V = R == 3 ? 4 : R, NF = (R + 1) / 2;       // NF records finished per lane: those with r % 2 == half
+  const int half = lane >> 4, l16 = lane & 15, rec0 = warp * 16 * R + l16;
+  unsigned long long acc[R][8];
+  uint32_t m1[R], m2[R];
+  float decay[NF];
+  uint32_t slot[NF];
+#pragma unroll
+  for (int q = 0; q < NF; ++q) {
+    const int rec = rec0 + 16 * min(2 * q + half, R - 1);
+    decay[q] = sm[B::kRec + rec * B::kRecRow + 6];
+    slot[q] = __float_as_uint(sm[B::kRec + rec * B::kRecRow + 7]);
+  }
+  row_start<R>(acc, sm + B::kB1 + half * 16);
 #pragma unroll 1
   for (int c = 0; c < 6; ++c) {
-    float v[NR];
+    float v[R];
 #pragma unroll
-    for (int r = 0; r < NR; ++r) v[r] = sm[B::kRec + (tid + r * kPairThreads) * 8 + c];
-    const float* row = sm + B::kW1 + c * kTF * B::kRow;
+    for (int r = 0; r < R; ++r) v[r] = sm[B::kRec + (rec0 + 16 * r) * B::kRecRow + c];
+    const float* row = sm + B::kW1 + c * kTF * B::kRow + half * 16;
 #pragma unroll
     for (int f = 0; f < kTF; ++f) {
-      float sn[NR], cs[NR];
+      const float2 fa = *reinterpret_cast<const float2*>(s_freq + 2 * f);
+      float sn[R], cs[R];
 #pragma unroll
-      for (int r = 0; r < NR; ++r) {
-        const float ph = v[r] * fr[f] * at[f];
+      for (int r = 0; r < R; ++r) {
+        const float ph = v[r] * fa.x * fa.y;
         sn[r] = __sinf(ph);
         cs[r] = __cosf(ph);
       }
-      row_fma<NR>(acc, row + f * B::kRow, sn);
-      row_fma<NR>(acc, row + (f + kTIN / 2) * B::kRow, cs);
+      row_fma<R>(acc, row + f * B::kRow, sn);
+      row_fma<R>(acc, row + (f + kTIN / 2) * B::kRow, cs);
     }
   }
-  row_relu<NR>(acc, h, m1, rec_ext != nullptr);
-  row_start<NR>(acc, sm + B::kB2);
-#pragma unroll
+  __syncthreads();                         // W1 and the records have been read
+  float* hid = sm + B::kHid + warp * B::kHidWarp;
+  relu_put<R, V>(acc, hid, lane, m1, rec_ext != nullptr);
+  __syncwarp();
+  row_start<R>(acc, sm + B::kB2 + half * 16);
+#pragma unroll 4
   for (int k = 0; k < 32; ++k) {
-    float x[NR];
-#pragma unroll
-    for (int r = 0; r < NR; ++r) x[r] = h[r][k];
-    row_fma<NR>(acc, sm + B::kW2 + k * B::kRow, x);
+    float x[R];
+    get_vec<R, V>(hid + k * (16 * V) + l16 * V, x);
+    row_fma<R>(acc, sm + B::kW2 + k * B::kRow + half * 16, x);
   }
-  row_relu<NR>(acc, h, m2, rec_ext != nullptr);
-  float o[NR][4];
+  __syncwarp();
+  relu_put<R, V>(acc, hid, lane, m2, rec_ext != nullptr);
+  __syncwarp();
+  // outputs 2 * half and 2 * half + 1 of all R records
+  unsigned long long o[R];
 #pragma unroll
-  for (int r = 0; r < NR; ++r) {
-#pragma unroll
-    for (int e = 0; e < 4; ++e) o[r][e] = sm[B::kB3 + e];
-  }
-#pragma unroll
+  for (int r = 0; r < R; ++r) o[r] = *reinterpret_cast<const unsigned long long*>(sm + B::kB3 + 2 * half);
+#pragma unroll 8
   for (int k = 0; k < 32; ++k) {
-    const float4 w = *reinterpret_cast<const float4*>(sm + B::kW3 + 4 * k);
+    float x[R];
+    get_vec<R, V>(hid + k * (16 * V) + l16 * V, x);
+    const unsigned long long w = *reinterpret_cast<const unsigned long long*>(sm + B::kW3 + 4 * k + 2 * half);
 #pragma unroll
-    for (int r = 0; r < NR; ++r) {
-      o[r][0] = fmaf(w.x, h[r][k], o[r][0]); o[r][1] = fmaf(w.y, h[r][k], o[r][1]);
-      o[r][2] = fmaf(w.z, h[r][k], o[r][2]); o[r][3] = fmaf(w.w, h[r][k], o[r][3]);
+    for (int r = 0; r < R; ++r) fma_f32x2(o[r], w, pack_f32x2(x[r], x[r]));
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const unsigned long long other = __shfl_xor_sync(0xffffffffu, o[r], 16);
+    if (rec_ext) {
+      const uint32_t a = __shfl_xor_sync(0xffffffffu, m1[r], 16), b = __shfl_xor_sync(0xffffffffu, m2[r], 16);
+      m1[r] = half ? (m1[r] << 16) | a : m1[r] | (a << 16);
+      m2[r] = half ? (m2[r] << 16) | b : m2[r] | (b << 16);
     }
-  }
-#pragma unroll
-  for (int r = 0; r < NR; ++r) {
-    const int rec = tid + r * kPairThreads;
-    if (rec >= rows) continue;
-    const float decay = sm[B::kRec + rec * 8 + 6];
-    const uint32_t slot = __float_as_uint(sm[B::kRec + rec * 8 + 7]);
-    const float sigma_raw = softplus_fast(o[r][3]);
+    const int rec = rec0 + 16 * r;
+    if ((r & 1) != half || rec >= rows) continue;
+    const float2 lo = unpack_f32x2(half ? other : o[r]), hi = unpack_f32x2(half ? o[r] : other);
+    const float sigma_raw = softplus_fast(hi.y);
     float4 out;
-    out.x = sigmoid_fast(o[r][0]); out.y = sigmoid_fast(o[r][1]); out.z = sigmoid_fast(o[r][2]);
-    out.w = (out_mode == kOutAlpha) ? (1.f - __expf(-(sigma_raw * decay))) : sigma_raw;
-    rec_out[slot] = out;
-    if (rec_ext) rec_ext[slot] = make_float4(sigma_raw, o[r][3], __uint_as_float(m1[r]), __uint_as_float(m2[r]));
+    out.x = sigmoid_fast(lo.x); out.y = sigmoid_fast(lo.y); out.z = sigmoid_fast(hi.x);
+    out.w = (out_mode == kOutAlpha) ? (1.f - __expf(-(sigma_raw * decay[r / 2]))) : sigma_raw;
+    rec_out[slot[r / 2]] = out;
+    if (rec_ext) rec_ext[slot[r / 2]] = make_float4(sigma_raw, hi.y, __uint_as_float(m1[r]), __uint_as_float(m2[r]));
   }
 }
 
@@ -241,73 +281,84 @@ __global__ void __launch_bounds__(kPairThreads, kPairCtas) k_mlp_f32_pair(
     const float* __restrict__ W1, const float* __restrict__ b1, const float* __restrict__ W2,
     const float* __restrict__ b2, const float* __restrict__ W3, const float* __restrict__ b3,
     const float* __restrict__ freq, const float* __restrict__ att, const RecIn* __restrict__ rec_in,
-    const int4* __restrict__ work, const int32_t* __restrict__ counters, float4* __restrict__ rec_out,
+    const int4* __restrict__ work, const int32_t* __restrict__ counters, int32_t* __restrict__ cursor, float4* __restrict__ rec_out,
     float4* __restrict__ rec_ext, int out_mode, const int32_t* __restrict__ status) {
   using B = PairBuf;
   chain_wait();
   chain_release();
   extern __shared__ __align__(16) float sm[];
+  __shared__ __align__(8) float s_freq[2 * kTF];
+  __shared__ int s_next;
   if (status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
-  const int tid = threadIdx.x, step = (int)gridDim.x;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int G = counters[kCtrWork];
-  int item = blockIdx.x;
+  const int item = blockIdx.x;
   if (item >= G) return;
-  float fr[kTF], at[kTF];
-#pragma unroll
-  for (int f = 0; f < kTF; ++f) { fr[f] = __ldg(freq + f); at[f] = __ldg(att + f); }
+  if (tid < kTF) { s_freq[2 * tid] = __ldg(freq + tid); s_freq[2 * tid + 1] = __ldg(att + tid); }
   const uint32_t s0 = smem_u32(sm);
-  auto copy = [&](const int4& w, int buf) {
-    const uint32_t d = s0 + 4u * (uint32_t)(buf * B::kFloats);
+  // A warp copies eight inputs of four units at a time: whole 32-byte sectors, 32 different banks.
+  const int jl = lane & 7, hl = lane >> 3;
+  auto copy = [&](const int4& w) {
+    const uint32_t d = s0;
     const size_t p = (size_t)w.x;
-    const float* w1 = W1 + p * (kTIN * 32);
-    int j = tid, h = 0;                                  // element i = u * 64 + tid of W1: unit h, input j
-#pragma unroll 4
-    for (int u = 0; u < kTIN * 32 / kPairThreads; ++u) {
-      cp_async4(d + 4u * (uint32_t)(B::kW1 + j * B::kRow + h), w1 + u * kPairThreads + tid);
-      j += kPairThreads;
-      if (j >= kTIN) { j -= kTIN; ++h; }
-    }
-    const float* w2 = W2 + p * (32 * 32);
-#pragma unroll 4
-    for (int u = 0; u < 32 * 32 / kPairThreads; ++u)
-      cp_async4(d + 4u * (uint32_t)(B::kW2 + (tid & 31) * B::kRow + 2 * u + (tid >> 5)), w2 + u * kPairThreads + tid);
+    const float* w1 = W1 + p * (kTIN * 32) + (warp * 16 + hl) * kTIN + jl;
+    const float* w2 = W2 + p * (32 * 32) + (warp * 16 + hl) * 32 + jl;
+    const uint32_t d1 = d + 4u * (uint32_t)(B::kW1 + jl * B::kRow + warp * 16 + hl), d2 = d1 + 4u * (uint32_t)(B::kW2 - B::kW1);
 #pragma unroll
-    for (int u = 0; u < 2; ++u)
-      cp_async4(d + 4u * (uint32_t)(B::kW3 + (tid & 31) * 4 + 2 * u + (tid >> 5)), W3 + p * 128 + u * kPairThreads + tid);
+    for (int hb = 0; hb < 4; ++hb) {
+#pragma unroll
+      for (int jb = 0; jb < kTIN / 8; ++jb) cp_async4(d1 + 4u * (uint32_t)(jb * 8 * B::kRow + hb * 4), w1 + hb * 4 * kTIN + jb * 8);
+#pragma unroll
+      for (int jb = 0; jb < 4; ++jb) cp_async4(d2 + 4u * (uint32_t)(jb * 8 * B::kRow + hb * 4), w2 + hb * 4 * 32 + jb * 8);
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int j = (2 * warp + u) * 8 + jl;
+      cp_async4(d + 4u * (uint32_t)(B::kW3 + j * 4 + hl), W3 + p * 128 + hl * 32 + j);
+    }
     cp_async4(d + 4u * (uint32_t)(B::kB1 + tid), tid < 32 ? b1 + p * 32 + tid : b2 + p * 32 + tid - 32);
     if (tid < 4) cp_async4(d + 4u * (uint32_t)(B::kB3 + tid), b3 + p * 4 + tid);
     const char* rec = reinterpret_cast<const char*>(rec_in + w.y);
     for (int c = tid; c < 2 * w.z; c += kPairThreads)    // the item's records, 32 bytes each
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 4u * (uint32_t)B::kRec + 16u * (uint32_t)c), "l"(rec + 16 * (size_t)c) : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 4u * (uint32_t)(B::kRec + (c >> 1) * B::kRecRow + (c & 1) * 4)),
+                   "l"(rec + 16 * (size_t)c) : "memory");
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  // rows of a buffer that no record has filled are computed and dropped: let them hold numbers
-  for (int i = tid; i < kRowsPerItem * 8; i += kPairThreads) sm[B::kRec + i] = sm[B::kFloats + B::kRec + i] = 0.f;
-  __syncthreads();
-  int4 wk = __ldg(work + item), wn = wk;
-  copy(wk, 0);
-  if (item + step < G) wn = __ldg(work + item + step);
-  int buf = 0;
-  for (;;) {
-    const bool more = item + step < G;
-    int4 wn2 = wn;
-    if (more) {
-      copy(wn, buf ^ 1);
-      if (item + 2 * step < G) wn2 = __ldg(work + item + 2 * step);
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
+  auto ahead = [&](const int4& w) {
+    const char* w1 = reinterpret_cast<const char*>(W1 + (size_t)w.x * (kTIN * 32));
+    const char* w2 = reinterpret_cast<const char*>(W2 + (size_t)w.x * (32 * 32));
+    const char* rec = reinterpret_cast<const char*>(rec_in + w.y);
+    for (int l = tid; l < kTIN + 32 + 32; l += kPairThreads) {         // 128-byte lines of W1, W2 and the records
+      const char* q = l < kTIN ? w1 + l * 128 : (l < kTIN + 32 ? w2 + (l - kTIN) * 128 : rec + (l - kTIN - 32) * 128);
+      if (l < kTIN + 32 || (l - kTIN - 32) * 4 < w.z) asm volatile("prefetch.global.L2 [%0];" ::"l"(q));
     }
+  };
+  int4 wn = make_int4(0, 0, 0, 0);
+  // The items come from a counter: the warps of an SM's four schedulers do not all get on at the same pace.  The next item's
+  // number is fetched and its lines are brought into L2 while the current one is computed.
+  int4 wk = __ldg(work + item);
+  for (;;) {
+    copy(wk);
+    int next = G;
+    if (tid == 0) s_next = next = (int)gridDim.x + atomicAdd(cursor, 1);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    const float* cur = sm + buf * B::kFloats;
-    if (wk.z > kPairThreads) pair_eval<2>(cur, fr, at, tid, wk.z, rec_out, rec_ext, out_mode);
-    else if ((tid & ~31) < wk.z) pair_eval<1>(cur, fr, at, tid, wk.z, rec_out, rec_ext, out_mode);
+    next = s_next;
+    const bool more = next < G;
+    if (more) {
+      wn = __ldg(work + next);
+      ahead(wn);
+    }
+    // rows past the item's last record are computed from what the buffer holds and dropped
+    switch ((wk.z + 31) >> 5) {
+      case 1: pair_eval<1>(sm, s_freq, warp, lane, wk.z, rec_out, rec_ext, out_mode); break;
+      case 2: pair_eval<2>(sm, s_freq, warp, lane, wk.z, rec_out, rec_ext, out_mode); break;
+      case 3: pair_eval<3>(sm, s_freq, warp, lane, wk.z, rec_out, rec_ext, out_mode); break;
+      default: pair_eval<4>(sm, s_freq, warp, lane, wk.z, rec_out, rec_ext, out_mode);
+    }
     if (!more) break;
     __syncthreads();                       // the buffer has been read
-    item += step;
     wk = wn;
-    wn = wn2;
-    buf ^= 1;
   }
 }
 
@@ -477,11 +528,11 @@ int launch_mlp_f32(const mlpsp_scene* sc, const RecIn* rec_in, const int4* work,
   int32_t* ctr = const_cast<int32_t*>(counters);
   LaunchScope scope(kKMlp, 1, st);
   if (F == kTF && H == 32) {
-    static_assert(2 * sizeof(float) * PairBuf::kFloats <= 48 * 1024, "no opt-in needed");
+    static_assert(sizeof(float) * PairBuf::kFloats <= 48 * 1024, "no opt-in needed");
     const int want = sms * kPairCtas;
     return cuda_check(launch_chained(k_mlp_f32_pair, dim3(grid_cap > 0 ? std::min(grid_cap, want) : want), dim3(kPairThreads),
-                                     2 * sizeof(float) * PairBuf::kFloats, st, sc->W1, sc->b1, sc->W2, sc->b2, sc->W3, sc->b3, sc->freq, sc->att,
-                                     rec_in, work, ctr, rec_out, rec_ext, out_mode, status),
+                                     sizeof(float) * PairBuf::kFloats, st, sc->W1, sc->b1, sc->W2, sc->b2, sc->W3, sc->b3, sc->freq, sc->att,
+                                     rec_in, work, ctr, ctr + kCtrWorkNext, rec_out, rec_ext, out_mode, status),
                       "mlp_f32");
   }
   if (F == kTF && H == 64 && !rec_ext) {
