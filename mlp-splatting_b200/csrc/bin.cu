@@ -208,24 +208,38 @@ __global__ void __launch_bounds__(256) k_bin_count(const float4* __restrict__ ge
 // (+1, -1, -1, +1), and the 2-D prefix sum of that array is the number of rectangles over each tile.  Four atomics
 // per primitive instead of one per (tile, primitive) pair (100,000 against 2.9 million on the bench frame).
 // mats (optional): the view and projection matrices in device memory, in place of the camera's own.
-__global__ void __launch_bounds__(256) k_bin_corners(const float4* __restrict__ geom, int n, const BinCam host_cam,
-                                                     const BinMats mats, uint2* __restrict__ rect, int32_t* __restrict__ diff) {
+// OWN: a CTA per SM adds its primitives' corners up in shared memory and then to the array, whole lines at a time.
+// Bound by the scattered atomics otherwise; launch_bin has the rule (four views of 500k primitives: 265 -> 56 us).
+template <bool OWN>
+__global__ void __launch_bounds__(OWN ? 1024 : 256) k_bin_corners(const float4* __restrict__ geom, int n, const BinCam host_cam,
+                                                                  const BinMats mats, uint2* __restrict__ rect, int32_t* __restrict__ diff) {
   chain_wait();
   chain_release();
+  extern __shared__ int32_t s_diff[];
   __shared__ BinCam cam;
   device_camera(cam, host_cam, mats);
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  int r[4] = {1, 0, 1, 0};
-  const bool has = prim_rect(geom, p, cam, r);
-  rect[p] = has ? make_uint2((uint32_t)r[0] | ((uint32_t)r[1] << 16), (uint32_t)r[2] | ((uint32_t)r[3] << 16))
-                : make_uint2(1u, 1u);  // x0=1 > x1=0
-  if (has) {
-    const int sx = cam.ntx + 1;
-    atomicAdd(diff + r[2] * sx + r[0], 1);
-    atomicAdd(diff + r[2] * sx + r[1] + 1, -1);
-    atomicAdd(diff + (r[3] + 1) * sx + r[0], -1);
-    atomicAdd(diff + (r[3] + 1) * sx + r[1] + 1, 1);
+  const int sx = cam.ntx + 1, cells = sx * (cam.nty + 1);
+  int32_t* dst = OWN ? s_diff : diff;
+  if (OWN) {
+    for (int i = threadIdx.x; i < cells; i += blockDim.x) s_diff[i] = 0;
+    __syncthreads();
+  }
+  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
+    int r[4] = {1, 0, 1, 0};
+    const bool has = prim_rect(geom, p, cam, r);
+    rect[p] = has ? make_uint2((uint32_t)r[0] | ((uint32_t)r[1] << 16), (uint32_t)r[2] | ((uint32_t)r[3] << 16))
+                  : make_uint2(1u, 1u);  // x0=1 > x1=0
+    if (has) {
+      atomicAdd(dst + r[2] * sx + r[0], 1);
+      atomicAdd(dst + r[2] * sx + r[1] + 1, -1);
+      atomicAdd(dst + (r[3] + 1) * sx + r[0], -1);
+      atomicAdd(dst + (r[3] + 1) * sx + r[1] + 1, 1);
+    }
+  }
+  if (OWN) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < cells; i += blockDim.x)
+      if (s_diff[i]) atomicAdd(diff + i, s_diff[i]);
   }
 }
 
@@ -549,9 +563,17 @@ int launch_bin(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, c
   LaunchScope scope(kKBin, (n > 0 ? (order_lists ? 3 : 2) : 0) + (corners ? 1 : 1 + scan_launches(T)), st);
   if (corners) {
     static DeviceOnce attr_once;
-    if (attr_once.first())
+    if (attr_once.first()) {
       MLPSP_CUDA_OK(cudaFuncSetAttribute(k_bin_offsets, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    if (n > 0) launch_chained(k_bin_corners, dim3((n + 255) / 256), dim3(256), 0, st, (const float4*)sc->geom, n, cam, mats, s.rect, s.tile_diff);
+      MLPSP_CUDA_OK(cudaFuncSetAttribute(k_bin_corners<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    }
+    // an atomic of a warp on scattered cells is 32 sector operations, one on a line of cells four: the arrays of the SMs
+    // cost sms * cells / 8 of them, the direct way 4 n; below twice as many the direct way's fuller grid wins
+    const int sms = sm_count();
+    if (8 * (int64_t)n >= (int64_t)sms * (int64_t)(diff_bytes / 4) / 2)
+      launch_chained(k_bin_corners<true>, dim3(sms), dim3(1024), diff_bytes, st, (const float4*)sc->geom, n, cam, mats, s.rect, s.tile_diff);
+    else if (n > 0)
+      launch_chained(k_bin_corners<false>, dim3((n + 255) / 256), dim3(256), 0, st, (const float4*)sc->geom, n, cam, mats, s.rect, s.tile_diff);
     launch_chained(k_bin_offsets, dim3(1), dim3(1024), diff_bytes, st, s.tile_diff, cam.ntx, cam.nty, fr->tile_offsets, fr->tile_capacity,
                    fr->max_pairs, fr->status, s.counters);
   } else {
