@@ -6,8 +6,9 @@
 // eight bits (two passes up to 65,535 primitives, three beyond).  A block owns 4,096 consecutive items, a warp 512 of
 // them in order.  Per pass: the blocks' digit counts, one scan per digit over the blocks, and the scatter, which ranks
 // the items of a warp with match.any against per-warp digit counters, orders the block's items by digit in shared
-// memory and writes them out in runs, so equal ids keep their record order.  The last kernel writes the permutation,
-// the CSR offsets (by binary search in the sorted keys: no counting pass) and the caller's record rows in the new order.
+// memory and writes them out in runs, so equal ids keep their record order; the last pass writes the permutation and, when
+// rows are to be moved, its inverse.  The last kernel writes the CSR offsets (by binary search in the sorted keys: no
+// counting pass) and the caller's record rows in the new order.
 #include "frame.cuh"
 
 namespace mlpsp {
@@ -61,11 +62,12 @@ __global__ void __launch_bounds__(kGsThreads) k_gs_scan(int nblocks, int32_t* __
   if (threadIdx.x == 0) dtot[blockIdx.x] = run;
 }
 
-template <bool FIRST>
+// LAST: order and inverse (where given) instead of vals_out
+template <bool FIRST, bool LAST>
 __global__ void __launch_bounds__(kGsThreads) k_gs_scatter(
     const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals, int64_t n, int nprim, int shift, int dbits, int nblocks,
     const int32_t* __restrict__ ghist, const int32_t* __restrict__ dtot, uint32_t* __restrict__ keys_out,
-    uint32_t* __restrict__ vals_out) {
+    uint32_t* __restrict__ vals_out, int64_t* __restrict__ order, uint32_t* __restrict__ inverse) {
   chain_wait();
   chain_release();
   __shared__ int s_cnt[kGsWarps][kGsBins];   // running digit counts per warp, then each warp's first position of a digit
@@ -125,31 +127,31 @@ __global__ void __launch_bounds__(kGsThreads) k_gs_scatter(
       const uint2 it = s_item[j];
       const int dst = s_dst[(it.x >> shift) & dmask] + j;
       keys_out[dst] = it.x;
-      vals_out[dst] = it.y;
+      if (!LAST) vals_out[dst] = it.y;
+      else {
+        order[dst] = (int64_t)it.y;
+        if (inverse) inverse[it.y] = (uint32_t)dst;
+      }
     }
   }
 }
 
-// Permutation, CSR offsets and, where given, the records' rows in primitive-major order.  Bound by the random row
-// reads; every output is written in full lines (three consecutive threads move the three 8-byte words of an x6 row).
-// 4.3 M records of 48 bytes: see the figures at mlpsp_group_rows.
+// CSR offsets and, where given, the records' rows in primitive-major order.  Rows are read in the order they come in and
+// written to their places: a primitive's records come from neighbouring pixels, a few hundred kilobytes apart at most, so
+// the pieces of a line meet in L2 and memory sees whole lines both ways.  (The other way round, whole lines written and
+// rows fetched, memory delivers 64 bytes for each 8, 16 or 24.)  Bound: memory; 4.3 M records of 48 bytes 365 -> 182 us, the
+// scattered order of the last pass (31 us more) included.
+// Three consecutive threads move the three 8-byte words of an x6 row.
 __global__ void __launch_bounds__(256) k_gs_finish(
-    const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals, int64_t n, int nprim, int64_t* __restrict__ order,
+    const uint32_t* __restrict__ keys, const uint32_t* __restrict__ inverse, int64_t n, int nprim,
     int64_t* __restrict__ offsets, const float2* __restrict__ x6, const float4* __restrict__ d4, const int2* __restrict__ masks,
     float2* __restrict__ x6_out, float4* __restrict__ d4_out, int2* __restrict__ masks_out) {
   chain_wait();
   chain_release();
-  __shared__ uint32_t s_val[256];
+  __shared__ uint32_t s_dst[256];
   const int64_t base = (int64_t)blockIdx.x * 256;
   const int64_t i = base + threadIdx.x;
   const int rows = (int)max((int64_t)0, min((int64_t)256, n - base));
-  if (i < n) {
-    const uint32_t v = vals[i];
-    s_val[threadIdx.x] = v;
-    order[i] = (int64_t)v;
-    if (d4) d4_out[i] = __ldg(d4 + v);
-    if (masks) masks_out[i] = __ldg(masks + v);
-  }
   if (i <= nprim) {      // first position whose key is not below i
     int64_t lo = 0, hi = n;
     while (lo < hi) {
@@ -158,12 +160,19 @@ __global__ void __launch_bounds__(256) k_gs_finish(
     }
     offsets[i] = lo;
   }
+  if (!inverse) return;
+  if (i < n) {
+    const uint32_t v = inverse[i];
+    s_dst[threadIdx.x] = v;
+    if (d4) d4_out[v] = __ldg(d4 + i);
+    if (masks) masks_out[v] = __ldg(masks + i);
+  }
   if (!x6) return;
   __syncthreads();
 #pragma unroll
   for (int u = 0; u < 3; ++u) {
     const int w = u * 256 + threadIdx.x;
-    if (w < rows * 3) x6_out[base * 3 + w] = __ldg(x6 + (size_t)s_val[w / 3] * 3 + w % 3);
+    if (w < rows * 3) x6_out[(size_t)s_dst[w / 3] * 3 + w % 3] = __ldg(x6 + base * 3 + w);
   }
 }
 
@@ -237,20 +246,23 @@ static int group_rows(const int32_t* ids, int64_t R, int n, int64_t* offsets, in
   int32_t* hist = (int32_t*)(b + L.hist);
   const uint32_t* k_in = reinterpret_cast<const uint32_t*>(ids);
   const uint32_t* v_in = nullptr;
+  uint32_t* inverse = nullptr;
   for (int pass = 0; pass < g.passes; ++pass) {
     const int shift = pass * g.dbits;
+    const bool first = pass == 0, last = pass == g.passes - 1;
     uint32_t* k_out = (uint32_t*)(b + L.key[pass & 1]);
-    uint32_t* v_out = (uint32_t*)(b + L.val[pass & 1]);
-    if (pass == 0) launch_chained(k_gs_hist<true>, dim3(g.nblocks), dim3(kGsThreads), 0, st, k_in, R, n, shift, g.dbits, g.nblocks, hist);
-    else launch_chained(k_gs_hist<false>, dim3(g.nblocks), dim3(kGsThreads), 0, st, k_in, R, n, shift, g.dbits, g.nblocks, hist);
+    uint32_t* v_out = (uint32_t*)(b + L.val[pass & 1]);          // the last pass writes no values: their place takes the inverse
+    if (last && (x6 || d4 || masks)) inverse = v_out;
+    launch_chained(first ? k_gs_hist<true> : k_gs_hist<false>, dim3(g.nblocks), dim3(kGsThreads), 0, st, k_in, R, n, shift, g.dbits, g.nblocks, hist);
     launch_chained(k_gs_scan, dim3(1 << g.dbits), dim3(kGsThreads), 0, st, g.nblocks, hist, dtot);
-    if (pass == 0) launch_chained(k_gs_scatter<true>, dim3(g.nblocks), dim3(kGsThreads), 0, st, k_in, v_in, R, n, shift, g.dbits, g.nblocks, hist, dtot, k_out, v_out);
-    else launch_chained(k_gs_scatter<false>, dim3(g.nblocks), dim3(kGsThreads), 0, st, k_in, v_in, R, n, shift, g.dbits, g.nblocks, hist, dtot, k_out, v_out);
+    auto* scatter = first ? (last ? k_gs_scatter<true, true> : k_gs_scatter<true, false>) : (last ? k_gs_scatter<false, true> : k_gs_scatter<false, false>);
+    launch_chained(scatter, dim3(g.nblocks), dim3(kGsThreads), 0, st, k_in, v_in, R, n, shift, g.dbits, g.nblocks, hist, dtot, k_out, v_out,
+                   order, inverse);
     k_in = k_out;
     v_in = v_out;
   }
-  const int64_t span = std::max<int64_t>(R, (int64_t)n + 1);
-  launch_chained(k_gs_finish, dim3((unsigned)((span + 255) / 256)), dim3(256), 0, st, k_in, v_in, R, n, order, offsets,
+  const int64_t span = std::max<int64_t>(inverse ? R : 0, (int64_t)n + 1);
+  launch_chained(k_gs_finish, dim3((unsigned)((span + 255) / 256)), dim3(256), 0, st, k_in, inverse, R, n, offsets,
                  reinterpret_cast<const float2*>(x6), reinterpret_cast<const float4*>(d4), reinterpret_cast<const int2*>(masks),
                  reinterpret_cast<float2*>(x6_out), reinterpret_cast<float4*>(d4_out), reinterpret_cast<int2*>(masks_out));
   return cuda_check(cudaGetLastError(), who);
