@@ -224,27 +224,29 @@ __global__ void __launch_bounds__(128) k_reverse_finish(const float* __restrict_
 // --------------------------------------------------------- grouped weight gradients ----
 // Segments of the launch, planned on the device (no count travels to the host): the order of the items does not matter,
 // a primitive of several segments owns consecutive partial rows and an entry of the multi list, a primitive without
-// records an entry with no rows (its gradients are zero).
+// records (its gradients are zero) an entry at the other end of that list.
 __global__ void __launch_bounds__(256) k_vjp_plan(const int64_t* __restrict__ offsets, int n, int segment_size,
                                                   VjpItem* __restrict__ items, VjpItem* __restrict__ multi,
                                                   int32_t* __restrict__ counters) {
   chain_wait();
   chain_release();
   __shared__ int warp_sums[32];
-  __shared__ int base[3];
+  __shared__ int base[4];
   const int p = blockIdx.x * 256 + threadIdx.x;
   int64_t start = 0, count = 0;
   if (p < n) { start = offsets[p]; count = offsets[p + 1] - start; }
   const int segs = count > 0 ? (int)((count + segment_size - 1) / segment_size) : 0;
-  const int rows = segs > 1 ? segs : 0, listed = p < n && segs != 1;
-  int ts, tr, tm;
+  const int rows = segs > 1 ? segs : 0, listed = segs > 1, empty = p < n && segs == 0;
+  int ts, tr, tm, te;
   const int es = block_exclusive_scan(segs, warp_sums, ts);
   const int er = block_exclusive_scan(rows, warp_sums, tr);
   const int em = block_exclusive_scan(listed, warp_sums, tm);
+  const int ee = block_exclusive_scan(empty, warp_sums, te);
   if (threadIdx.x == 0) {
     base[0] = ts ? atomicAdd(counters + kVpItems, ts) : 0;
     base[1] = tr ? atomicAdd(counters + kVpRows, tr) : 0;
     base[2] = tm ? atomicAdd(counters + kVpMulti, tm) : 0;
+    base[3] = te ? atomicAdd(counters + kVpEmpty, te) : 0;
   }
   __syncthreads();
   for (int g = 0; g < segs; ++g) {
@@ -262,6 +264,7 @@ __global__ void __launch_bounds__(256) k_vjp_plan(const int64_t* __restrict__ of
     it.prim = p;
     multi[base[2] + em] = it;
   }
+  if (empty) multi[n - 1 - (base[3] + ee)].prim = p;
 }
 
 // IEEE FP32 on the CUDA cores, sums in record order.  A CTA of 128 threads takes 64 records at a time; everything per
@@ -463,13 +466,15 @@ __global__ void __launch_bounds__(kGfThreads, kGfCtas) k_grouped_vjp(
   if (bad) atomicOr(counters + kVpFlag, 1);
 }
 
-// The gradients of the primitives on the multi list: their partial rows in segment order (no rows: zero).
+// The gradients of the primitives on the multi list, their partial rows in segment order; and, unless the tensor-core
+// kernel has done it between its waits, the zeros of the primitives without records.
 __global__ void __launch_bounds__(256) k_vjp_reduce(const VjpItem* __restrict__ multi, const float* __restrict__ partial,
-                                                    VjpOut out, int32_t* __restrict__ counters) {
+                                                    VjpOut out, int n, int zeros, int aligned, int32_t* __restrict__ counters) {
   chain_wait();
   chain_release();
-  const int M = counters[kVpMulti];
+  const int M = counters[kVpMulti], E = zeros ? counters[kVpEmpty] : 0;
   bool bad = false;
+  for (int e = blockIdx.x; e < E; e += gridDim.x) vjp_zero(out, __ldg(&multi[n - 1 - e].prim), aligned, threadIdx.x, 256);
   for (int e = blockIdx.x; e < M; e += gridDim.x) {
     VjpItem it = load_item(multi + e);
     it.dest = -1;
@@ -487,8 +492,8 @@ __global__ void __launch_bounds__(256) k_vjp_reduce(const VjpItem* __restrict__ 
 }
 
 int launch_grouped_vjp_tc(bool bf16, const float* x6, const float* d4, const int32_t* masks, const VjpItem* items,
-                          int64_t max_items, int32_t* counters, const mlpsp_scene* sc, float scale, const VjpOut& out,
-                          float* partial, cudaStream_t st);
+                          int64_t max_items, const VjpItem* multi, int32_t* counters, const mlpsp_scene* sc, float scale,
+                          const VjpOut& out, float* partial, cudaStream_t st);
 
 // scratch of a launch: counters | items | multi list | partial rows
 struct VjpScratch { int64_t items, multi, partial, bytes, max_items, max_rows; };
@@ -518,8 +523,9 @@ static int weight_gradients(const mlpsp_scene* sc, const int64_t* offsets, const
   LaunchScope scope(kKMisc, R > 0 ? 3 : 2, st);
   MLPSP_CUDA_OK(cudaMemsetAsync(counters, 0, 4 * kVpCounters, st));
   launch_chained(k_vjp_plan, dim3((sc->n + 255) / 256), dim3(256), 0, st, offsets, sc->n, segment_size, items, multi, counters);
-  if (R > 0 && precision != MLPSP_PRECISION_F32) {
-    const int rc = launch_grouped_vjp_tc(precision == MLPSP_PRECISION_BF16, x6, d4, masks, items, L.max_items, counters, sc, loss_scale,
+  const bool tc = R > 0 && precision != MLPSP_PRECISION_F32;
+  if (tc) {
+    const int rc = launch_grouped_vjp_tc(precision == MLPSP_PRECISION_BF16, x6, d4, masks, items, L.max_items, multi, counters, sc, loss_scale,
                                          out, partial, st);
     if (rc) return rc;
   } else if (R > 0) {
@@ -529,7 +535,8 @@ static int weight_gradients(const mlpsp_scene* sc, const int64_t* offsets, const
     launch_chained(k_grouped_vjp, dim3((unsigned)std::min<int64_t>(L.max_items, (int64_t)sm_count() * kGfCtas)), dim3(kGfThreads), kGradSmem, st,
                    x6, d4, masks, items, counters, sc->freq, sc->att, sc->W1, sc->b1, sc->W2, sc->b2, sc->W3, loss_scale, out, partial);
   }
-  launch_chained(k_vjp_reduce, dim3((unsigned)std::min(sc->n, sm_count() * 8)), dim3(256), 0, st, multi, partial, out, counters);
+  launch_chained(k_vjp_reduce, dim3((unsigned)std::min(sc->n, sm_count() * 8)), dim3(256), 0, st, multi, partial, out, sc->n, tc ? 0 : 1,
+                 vjp_aligned(out), counters);
   if (flag_dev) MLPSP_CUDA_OK(cudaMemcpyAsync(flag_dev, counters + kVpFlag, 4, cudaMemcpyDeviceToDevice, st));
   if (flag_host) {
     HostWords& hw = host_words();

@@ -29,7 +29,26 @@ constexpr int kOW1 = 0, kOb1 = kOW1 + kGH * kGIN, kOW2 = kOb1 + kGH, kOb2 = kOW2
 static_assert(kGradLen == 3524, "gradient row layout");
 
 // plan counters (device int32)
-enum VjpCounter { kVpItems = 0, kVpRows = 1, kVpMulti = 2, kVpFlag = 3, kVpCounters = 4 };
+enum VjpCounter { kVpItems = 0, kVpRows = 1, kVpMulti = 2, kVpFlag = 3, kVpEmpty = 4, kVpCounters = 5 };
+
+// zero gradients of one primitive, by nthr threads (rows of 16-byte multiples; b = the tensors' bases aligned)
+__device__ __forceinline__ void vjp_zero(const VjpOut& o, int prim, int aligned, int t, int nthr) {
+  auto fill = [&](float* p, int64_t stride, int len) {
+    p += prim * stride;
+    if (aligned) {
+      for (int i = t; i < len / 4; i += nthr) reinterpret_cast<float4*>(p)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    } else {
+      for (int i = t; i < len; i += nthr) p[i] = 0.f;
+    }
+  };
+  fill(o.W1, o.sW1, kGH * kGIN); fill(o.b1, o.sb1, kGH); fill(o.W2, o.sW2, kGH * kGH); fill(o.b2, o.sb2, kGH);
+  fill(o.W3, o.sW3, 4 * kGH); fill(o.b3, o.sb3, 4);
+}
+inline int vjp_aligned(const VjpOut& o) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(o.W1) | reinterpret_cast<uintptr_t>(o.b1) | reinterpret_cast<uintptr_t>(o.W2) |
+                      reinterpret_cast<uintptr_t>(o.b2) | reinterpret_cast<uintptr_t>(o.W3) | reinterpret_cast<uintptr_t>(o.b3);
+  return (a & 15) == 0 && ((o.sW1 | o.sb1 | o.sW2 | o.sb2 | o.sW3 | o.sb3) & 3) == 0;
+}
 
 __device__ __forceinline__ VjpOut vjp_row(const VjpOut& o, float* partial, const VjpItem& it) {
   VjpOut r;

@@ -121,16 +121,24 @@ __device__ __forceinline__ void vjp_d2(uint32_t d01, uint32_t d23, uint32_t m2, 
 template <bool BF16, bool MASKS>
 __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
     const float* __restrict__ x6, const float* __restrict__ d4, const int32_t* __restrict__ masks,
-    const VjpItem* __restrict__ items, int32_t* __restrict__ counters, const float* __restrict__ freq,
-    const float* __restrict__ att, const float* __restrict__ W1, const float* __restrict__ b1, const float* __restrict__ W2,
+    const VjpItem* __restrict__ items, const VjpItem* __restrict__ multi, int n, int aligned, int32_t* __restrict__ counters,
+    const float* __restrict__ freq, const float* __restrict__ att, const float* __restrict__ W1, const float* __restrict__ b1, const float* __restrict__ W2,
     const float* __restrict__ b2, const float* __restrict__ W3, int vec, float scale, VjpOut out, float* __restrict__ partial) {
   chain_wait();
   chain_release();
   extern __shared__ __align__(128) char smem[];
-  const int G = counters[kVpItems];
-  int idx = blockIdx.x;
-  if (idx >= G) return;
+  const int G = counters[kVpItems], E = counters[kVpEmpty];
+  int idx = blockIdx.x, empty = blockIdx.x;      // segments; primitives without records, one between two waits
   const int tid = threadIdx.x, warp = tid >> 5;
+  auto zero_next = [&]() {
+    if (empty >= E) return;
+    vjp_zero(out, __ldg(&multi[n - 1 - empty].prim), aligned, tid, kVjpRows);
+    empty += (int)gridDim.x;
+  };
+  if (idx >= G) {
+    while (empty < E) zero_next();
+    return;
+  }
   uint64_t* s_bar = reinterpret_cast<uint64_t*>(smem + kVoBar);
   uint32_t* s_misc = reinterpret_cast<uint32_t*>(s_bar + 1);
   float* s_bias = reinterpret_cast<float*>(smem + kVoBias);
@@ -367,6 +375,7 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
     } else {
       more = false;
     }
+    zero_next();
     ok = wait_phase();
     if (!ok) break;
     {
@@ -431,6 +440,7 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
     if (!more) break;
   }
   if (ok) {
+    while (empty < E) zero_next();
     ok = wait_phase();
     if (ok) emit(it_p);
   }
@@ -442,8 +452,8 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
 }
 
 int launch_grouped_vjp_tc(bool bf16, const float* x6, const float* d4, const int32_t* masks, const VjpItem* items,
-                          int64_t max_items, int32_t* counters, const mlpsp_scene* sc, float scale, const VjpOut& out,
-                          float* partial, cudaStream_t st) {
+                          int64_t max_items, const VjpItem* multi, int32_t* counters, const mlpsp_scene* sc, float scale,
+                          const VjpOut& out, float* partial, cudaStream_t st) {
   static DeviceOnce attr_once;
   if (attr_once.first()) {
     MLPSP_CUDA_OK(cudaFuncSetAttribute(k_grouped_vjp_tc<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kVjpSmem));
@@ -455,8 +465,9 @@ int launch_grouped_vjp_tc(bool bf16, const float* x6, const float* d4, const int
                       : (masks ? k_grouped_vjp_tc<false, true> : k_grouped_vjp_tc<false, false>);
   const int vec = ((reinterpret_cast<uintptr_t>(sc->W1) | reinterpret_cast<uintptr_t>(sc->W2)) & 15) == 0 &&
                   (reinterpret_cast<uintptr_t>(x6) & 7) == 0;
-  const int grid = (int)std::min<int64_t>(max_items, (int64_t)sm_count() * kVjpCtas);
-  return cuda_check(launch_chained(kernel, dim3(grid), dim3(kVjpRows), kVjpSmem, st, x6, d4, masks, items, counters, sc->freq, sc->att,
+  const int grid = (int)std::min<int64_t>(std::max<int64_t>(max_items, sc->n), (int64_t)sm_count() * kVjpCtas);     // CTAs without segments write zeros
+  return cuda_check(launch_chained(kernel, dim3(grid), dim3(kVjpRows), kVjpSmem, st, x6, d4, masks, items, multi, sc->n, vjp_aligned(out),
+                                   counters, sc->freq, sc->att,
                                    sc->W1, sc->b1, sc->W2, sc->b2, sc->W3, vec, scale, out, partial),
                     "grouped_vjp_tc");
 }
