@@ -73,11 +73,10 @@ __device__ __forceinline__ void quat_adjoint(float w, float x, float y, float z,
 //   k_reverse_check     the argument checks of the caller (offsets, ids) as one status word;
 //   k_reverse_pixels    thread = pixel: the recurrence, the four adjoints of every record and
 //                       k = g_sigma * sigma_raw * decay, the weight of the record's geometry terms;
-//   k_reverse_geometry  thread = record.  decay = exp(-1/2 q^T M q) with q = R^T d, M = diag(exp(-2 ls)): the position,
-//                       log-scale and quaternion gradients of a primitive are linear in the nine sums of k q and
-//                       k q q^T over its records, so only those are accumulated -- in a shared-memory table first
-//                       (records that follow one another belong to neighbouring pixels, which mostly see the same
-//                       primitives), so that global memory sees one set of vector reductions per primitive and chunk;
+//   k_reverse_geometry  decay = exp(-1/2 q^T M q) with q = R^T d, M = diag(exp(-2 ls)): the position, log-scale and
+//                       quaternion gradients of a primitive are linear in the nine sums of k q and k q q^T over its
+//                       records, so only those are accumulated, a chunk of records at a time (records that follow one
+//                       another belong to neighbouring pixels, which mostly see the same primitives);
 //   k_reverse_finish    thread = primitive: the gradients from the nine sums.
 constexpr int kRevAcc = 12;          // floats per primitive: k q (3), k q q^T (6), padding to three 16-byte reductions
 
@@ -94,88 +93,146 @@ __global__ void __launch_bounds__(256) k_reverse_check(const int32_t* __restrict
   if (b) { atomicOr(bad, b); if (bad_host) atomicOr_system(const_cast<int32_t*>(bad_host), b); }
 }
 
-// Four records at a time: their loads do not depend on the recurrence, so they are in flight together.
-__global__ void __launch_bounds__(128) k_reverse_pixels(const int64_t* __restrict__ offsets, const float* __restrict__ raw,
+// A block's pixels own one run of records, which is brought into shared memory in whole lines; the outputs take their
+// records' places there and leave the same way.  A run beyond kRevStage records (about 12 per pixel is usual) is read and
+// written directly, four records at a time: their loads do not depend on the recurrence, so they are in flight together.
+// Bound: memory, 52 bytes per record; 4.3 M records in 480,000 pixels, all directly: 167 us, staged: 134.
+constexpr int kRevPixels = 128, kRevStage = 1536;
+__global__ void __launch_bounds__(kRevPixels) k_reverse_pixels(const int64_t* __restrict__ offsets, const float* __restrict__ raw,
                                  const float* __restrict__ grgb, const float* __restrict__ gt, int64_t pixels,
                                  float* __restrict__ d4, float* __restrict__ kw, const int32_t* __restrict__ bad) {
   chain_wait();
   chain_release();
-  const int64_t pix = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (pix >= pixels || *bad) return;
-  const float gr = grgb[pix * 3], gg = grgb[pix * 3 + 1], gb = grgb[pix * 3 + 2];
-  float behind = gt[pix];   // adjoint of the transmittance that reaches whatever lies behind the current record
-  const int64_t first = offsets[pix];
+  extern __shared__ __align__(16) float4 s_raw[];      // two per record
+  if (*bad) return;
+  const int tid = threadIdx.x;
+  const int64_t p0 = (int64_t)blockIdx.x * kRevPixels, p1 = min(p0 + kRevPixels, pixels), pix = p0 + tid;
+  const int64_t base = offsets[p0], run = offsets[p1] - base;
   const float4* raw4 = reinterpret_cast<const float4*>(raw);
-  for (int64_t r = offsets[pix + 1] - 1; r >= first; r -= 4) {
+  const bool staged = run <= kRevStage;
+  float gr = 0.f, gg = 0.f, gb = 0.f, behind = 0.f;
+  int64_t first = 0, last = -1;
+  if (pix < pixels) {
+    gr = grgb[pix * 3]; gg = grgb[pix * 3 + 1]; gb = grgb[pix * 3 + 2];
+    behind = gt[pix];   // adjoint of the transmittance that reaches whatever lies behind the current record
+    first = offsets[pix];
+    last = offsets[pix + 1] - 1;
+  }
+  // one record: its outputs, and the colour behind it
+  auto step = [&](const float4 a, const float4 c, float4& out, float& weight) {     // R, G, B, sigma_raw; trans before, alpha, decay, sigma logit
+    const float colour = gr * a.x + gg * a.y + gb * a.z;
+    const float g_alpha = c.x * (colour - behind);
+    behind = behind * (1.f - c.y) + colour * c.y;
+    const float g_sigma = g_alpha * __expf(-a.w * c.z);   // d alpha / d (sigma_raw * decay) = 1 - alpha
+    const float w = c.x * c.y, parked = g_sigma * c.z;
+    out = make_float4(gr * w * a.x * (1.f - a.x), gg * w * a.y * (1.f - a.y), gb * w * a.z * (1.f - a.z),
+                      parked * sigmoid_fast(c.w));        // softplus' = sigmoid
+    weight = parked * a.w;                                // g_decay * decay
+  };
+  if (staged) {
+    for (int i = tid; i < 2 * (int)run; i += kRevPixels) s_raw[i] = __ldg(raw4 + 2 * base + i);
+    __syncthreads();
+    for (int q = (int)(last - base); q >= (int)(first - base); --q) {
+      float4 out;
+      float weight;
+      step(s_raw[2 * q], s_raw[2 * q + 1], out, weight);
+      s_raw[2 * q] = out;
+      s_raw[2 * q + 1].x = weight;
+    }
+    __syncthreads();
+    for (int i = tid; i < (int)run; i += kRevPixels) {
+      *reinterpret_cast<float4*>(d4 + (base + i) * 4) = s_raw[2 * i];
+      kw[base + i] = s_raw[2 * i + 1].x;
+    }
+    return;
+  }
+  for (int64_t r = last; r >= first; r -= 4) {
     float4 a4[4], c4[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int64_t q = r - u >= first ? r - u : first;
-      a4[u] = __ldg(raw4 + 2 * q);         // R, G, B, sigma_raw
-      c4[u] = __ldg(raw4 + 2 * q + 1);     // trans before, alpha, decay, sigma logit
+      a4[u] = __ldg(raw4 + 2 * q);
+      c4[u] = __ldg(raw4 + 2 * q + 1);
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       if (r - u < first) break;
-      const float4 a = a4[u], c = c4[u];
-      const float colour = gr * a.x + gg * a.y + gb * a.z;
-      const float g_alpha = c.x * (colour - behind);
-      behind = behind * (1.f - c.y) + colour * c.y;
-      const float g_sigma = g_alpha * __expf(-a.w * c.z);   // d alpha / d (sigma_raw * decay) = 1 - alpha
-      const float w = c.x * c.y, parked = g_sigma * c.z;
-      *reinterpret_cast<float4*>(d4 + (r - u) * 4) =
-          make_float4(gr * w * a.x * (1.f - a.x), gg * w * a.y * (1.f - a.y), gb * w * a.z * (1.f - a.z),
-                      parked * sigmoid_fast(c.w));          // softplus' = sigmoid
-      kw[r - u] = parked * a.w;                             // g_decay * decay
+      float4 out;
+      step(a4[u], c4[u], out, kw[r - u]);
+      *reinterpret_cast<float4*>(d4 + (r - u) * 4) = out;
     }
   }
 }
 
-constexpr int kRevThreads = 256;
-constexpr int kRevChunk = 4096;      // records per CTA
-constexpr int kRevTable = 1024;      // shared-memory accumulator rows (a power of two)
+constexpr int kRevThreads = 256, kRevPer = 8;
+constexpr int kRevChunk = kRevThreads * kRevPer;      // records per CTA
+constexpr int kRevTable = 1024;      // rows of the chunk's table of primitives (a power of two)
 constexpr int kRevProbe = 16;        // probes before a record goes to global memory directly
+constexpr int kRevPiece = 16;        // records that one thread adds up
+constexpr int kRevUnits = kRevTable + kRevChunk / kRevPiece;
+constexpr int kRevSmem = (kRevChunk + 3 * kRevThreads) * 16;
+static_assert(kRevChunk <= 2048 && kRevPiece <= 32 && kRevTable <= 1024, "packing of a unit: start 11 bits, count - 1 5 bits, row 10 bits");
 
 __device__ __forceinline__ void red_add4(float* dst, float a, float b, float c, float d) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
-__global__ void __launch_bounds__(kRevThreads) k_reverse_geometry(
+// A chunk's records are ordered by primitive in shared memory -- a hash table of the primitives that counts its rows, a
+// prefix over the rows -- and a thread adds up to kRevPiece records of one primitive in registers; the sums leave three
+// 16-byte reductions at a time, a primitive's by neighbouring lanes.  Bound: the reductions in L2 and the record's 44 bytes.
+// With nine floating-point additions per record in shared memory (each a loop of compare-and-swap, on rows that
+// neighbouring pixels share) 4.3 M records took 246 us and 0.7 M 141; this takes 71 and about 40.
+__device__ __forceinline__ void reverse_terms(const float4 qt, float dx, float dy, float dz, float k, float (&v)[9]) {
+  const V3 q = rot_conj_fast(qt.x, qt.y, qt.z, qt.w, V3{dx, dy, dz});
+  const float kx = k * q.x, ky = k * q.y, kz = k * q.z;
+  v[0] += kx; v[1] += ky; v[2] += kz;
+  v[3] += kx * q.x; v[4] += ky * q.y; v[5] += kz * q.z;
+  v[6] += kx * q.y; v[7] += kx * q.z; v[8] += ky * q.z;
+}
+
+__global__ void __launch_bounds__(kRevThreads, 3) k_reverse_geometry(
     const int32_t* __restrict__ ids, const float* __restrict__ x6, const float* __restrict__ kw,
     const float* __restrict__ quats, int64_t total, float* __restrict__ acc, const int32_t* __restrict__ bad) {
   chain_wait();
   chain_release();
-  __shared__ int s_key[kRevTable];
-  __shared__ float s_acc[9][kRevTable];
+  extern __shared__ __align__(16) float4 s_rec[];      // [kRevChunk] offset and weight, by primitive; then the sums of a round
+  __shared__ int s_key[kRevTable], s_cnt[kRevTable];   // primitive, records (later: first record)
+  __shared__ uint32_t s_unit[kRevUnits];
+  __shared__ int warp_sums[32];
+  float4 (*s_sum)[3] = reinterpret_cast<float4(*)[3]>(s_rec + kRevChunk);
   if (*bad) return;
-  for (int i = threadIdx.x; i < kRevTable; i += kRevThreads) {
-    s_key[i] = -1;
+  const int tid = threadIdx.x;
+  for (int i = tid; i < kRevTable; i += kRevThreads) { s_key[i] = -1; s_cnt[i] = 0; }
+  const int64_t r0 = (int64_t)blockIdx.x * kRevChunk;
+  float4 rec[kRevPer];
+  int place[kRevPer];              // row << 16 | rank in it; -1: none
 #pragma unroll
-    for (int j = 0; j < 9; ++j) s_acc[j][i] = 0.f;
+  for (int u = 0; u < kRevPer; ++u) {
+    const int64_t r = r0 + u * kRevThreads + tid;
+    place[u] = r < total ? ids[r] : -1;
+    rec[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (r < total) rec[u] = make_float4(x6[r * 6 + 3], x6[r * 6 + 4], x6[r * 6 + 5], kw[r]);      // centre - foot point
   }
   __syncthreads();
-  const int64_t r0 = (int64_t)blockIdx.x * kRevChunk;
-  const int64_t r1 = r0 + kRevChunk < total ? r0 + kRevChunk : total;
-  for (int64_t r = r0 + threadIdx.x; r < r1; r += kRevThreads) {
-    const int p = ids[r];
-    const float k = kw[r];
-    const V3 d = {x6[r * 6 + 3], x6[r * 6 + 4], x6[r * 6 + 5]};            // centre - foot point
-    const float4 qt = __ldg(reinterpret_cast<const float4*>(quats) + p);
-    const V3 q = rot_conj_fast(qt.x, qt.y, qt.z, qt.w, d);
-    const float kx = k * q.x, ky = k * q.y, kz = k * q.z;
-    const float v[9] = {kx, ky, kz, kx * q.x, ky * q.y, kz * q.z, kx * q.y, kx * q.z, ky * q.z};
+#pragma unroll
+  for (int u = 0; u < kRevPer; ++u) {
+    const int p = place[u];
+    if (p < 0) continue;
     // the primitive's row of the table: linear probing from a multiplicative hash
-    int slot = (int)(((uint32_t)p * 2654435761u) >> 22) & (kRevTable - 1);
+    int row = (int)(((uint32_t)p * 2654435761u) >> 22) & (kRevTable - 1);
     bool placed = false;
     for (int probe = 0; probe < kRevProbe && !placed; ++probe) {
-      const int seen = atomicCAS(&s_key[slot], -1, p);
+      int seen = s_key[row];
+      if (seen == -1) seen = atomicCAS(&s_key[row], -1, p);
       if (seen == -1 || seen == p) placed = true;
-      else slot = (slot + 1) & (kRevTable - 1);
+      else row = (row + 1) & (kRevTable - 1);
     }
     if (placed) {
-#pragma unroll
-      for (int j = 0; j < 9; ++j) atomicAdd(&s_acc[j][slot], v[j]);
+      place[u] = (row << 16) | atomicAdd(&s_cnt[row], 1);
     } else {
+      place[u] = -1;
+      float v[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      reverse_terms(__ldg(reinterpret_cast<const float4*>(quats) + p), rec[u].x, rec[u].y, rec[u].z, rec[u].w, v);
       float* dst = acc + (size_t)p * kRevAcc;
       red_add4(dst, v[0], v[1], v[2], v[3]);
       red_add4(dst + 4, v[4], v[5], v[6], v[7]);
@@ -183,13 +240,51 @@ __global__ void __launch_bounds__(kRevThreads) k_reverse_geometry(
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < kRevTable; i += kRevThreads) {
-    const int p = s_key[i];
-    if (p < 0) continue;
-    float* dst = acc + (size_t)p * kRevAcc;
-    red_add4(dst, s_acc[0][i], s_acc[1][i], s_acc[2][i], s_acc[3][i]);
-    red_add4(dst + 4, s_acc[4][i], s_acc[5][i], s_acc[6][i], s_acc[7][i]);
-    red_add4(dst + 8, s_acc[8][i], 0.f, 0.f, 0.f);
+  // rows -> first records and pieces (a thread has kRevTable / kRevThreads rows in order)
+  constexpr int kRows = kRevTable / kRevThreads;
+  int cnt[kRows], mine = 0;
+#pragma unroll
+  for (int j = 0; j < kRows; ++j) {
+    cnt[j] = s_cnt[tid * kRows + j];
+    mine += (cnt[j] << 16) + (cnt[j] + kRevPiece - 1) / kRevPiece;
+  }
+  int all;
+  const int before = block_exclusive_scan(mine, warp_sums, all);
+  int start = before >> 16, unit = before & 0xffff;
+  const int units = all & 0xffff;
+#pragma unroll
+  for (int j = 0; j < kRows; ++j) {
+    s_cnt[tid * kRows + j] = start;
+    for (int c = 0; c < cnt[j]; c += kRevPiece)
+      s_unit[unit++] = (uint32_t)(start + c) | ((uint32_t)(min(kRevPiece, cnt[j] - c) - 1) << 11) | ((uint32_t)(tid * kRows + j) << 16);
+    start += cnt[j];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < kRevPer; ++u)
+    if (place[u] >= 0) s_rec[s_cnt[place[u] >> 16] + (place[u] & 0xffff)] = rec[u];
+  __syncthreads();
+  for (int b = 0; b < units; b += kRevThreads) {
+    if (b + tid < units) {
+      const uint32_t w = s_unit[b + tid];
+      const float4 qt = __ldg(reinterpret_cast<const float4*>(quats) + s_key[w >> 16]);
+      float v[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      const int from = w & 2047, to = from + 1 + ((w >> 11) & 31);
+      for (int i = from; i < to; ++i) {
+        const float4 e = s_rec[i];
+        reverse_terms(qt, e.x, e.y, e.z, e.w, v);
+      }
+      s_sum[tid][0] = make_float4(v[0], v[1], v[2], v[3]);
+      s_sum[tid][1] = make_float4(v[4], v[5], v[6], v[7]);
+      s_sum[tid][2] = make_float4(v[8], 0.f, 0.f, 0.f);
+    }
+    __syncthreads();
+    const int pieces = 3 * min(kRevThreads, units - b);
+    for (int i = tid; i < pieces; i += kRevThreads) {
+      const float4 e = s_sum[i / 3][i % 3];
+      red_add4(acc + (size_t)s_key[s_unit[b + i / 3] >> 16] * kRevAcc + (i % 3) * 4, e.x, e.y, e.z, e.w);
+    }
+    __syncthreads();
   }
 }
 
@@ -594,8 +689,12 @@ extern "C" int mlpsp_records_reverse_checked(const int32_t* ids, const int64_t* 
                  pixels, bad, findings_host ? hw.word : nullptr);
   if (findings_host) MLPSP_CUDA_OK(cudaEventRecord(ev, st));
   if (pixels > 0 && total_records > 0) {
-    launch_chained(k_reverse_pixels, dim3((unsigned)((pixels + 127) / 128)), dim3(128), 0, st, offsets, raw, grad_rgb, grad_t, pixels, d4, kw, bad);
-    launch_chained(k_reverse_geometry, dim3((unsigned)((total_records + kRevChunk - 1) / kRevChunk)), dim3(kRevThreads), 0, st, ids, x6, kw, quats,
+    static DeviceOnce attr_once;
+    if (attr_once.first())
+      MLPSP_CUDA_OK(cudaFuncSetAttribute(k_reverse_geometry, cudaFuncAttributeMaxDynamicSharedMemorySize, kRevSmem));
+    launch_chained(k_reverse_pixels, dim3((unsigned)((pixels + kRevPixels - 1) / kRevPixels)), dim3(kRevPixels), kRevStage * 32, st, offsets, raw, grad_rgb, grad_t, pixels, d4, kw, bad);
+    launch_chained(k_reverse_geometry, dim3((unsigned)((total_records + kRevChunk - 1) / kRevChunk)), dim3(kRevThreads),
+                   kRevSmem, st, ids, x6, kw, quats,
                    total_records, acc, bad);
   }
   if (n > 0) launch_chained(k_reverse_finish, dim3((n + 127) / 128), dim3(128), 0, st, acc, log_scales, quats, n, grad_pos, grad_log_scales, grad_quats);
