@@ -286,6 +286,11 @@ int mlpsp_export_records(const mlpsp_scene* scene, const mlpsp_frame* frame, int
                          float* x6, float* raw, int32_t* relu_masks, float* gates, int64_t max_out,
                          int32_t max_hits, int64_t* total_host, int32_t* worst_host, void* stream);
 
+/* The same rows behind a call of mlpsp_export_records on this frame that only counted (no outputs): total is the
+ * count it returned, every non-NULL array has room for it.  Does not count again and does not synchronise. */
+int mlpsp_export_counted_records(const mlpsp_scene* scene, const mlpsp_frame* frame, int32_t* ids, float* x6, float* raw,
+                                 int32_t* relu_masks, float* gates, int64_t total, void* stream);
+
 /* Grouped evaluator on explicit records (the forward counterpart of primitive_gemm.py's grouped
  * VJP): records are primitive-major, offsets[n+1] int64 as produced by group_records
  * (primitive_csr.py:23-29); x6[R,6]; out[R,4] = (R, G, B, sigma_raw). */

@@ -103,6 +103,7 @@ _SIGS = {
     "mlpsp_render_frame_rays": (C.c_int, [C.POINTER(Scene), C.POINTER(Frame), _fp, _fp, _fp, _fp, _fp]),
     "mlpsp_export_records": (C.c_int, [C.POINTER(Scene), C.POINTER(Frame), _fp, _fp, _fp, _fp, _fp, _fp, C.c_int64,
                                        C.c_int32, C.POINTER(C.c_int64), C.POINTER(C.c_int32), _fp]),
+    "mlpsp_export_counted_records": (C.c_int, [C.POINTER(Scene), C.POINTER(Frame), _fp, _fp, _fp, _fp, _fp, C.c_int64, _fp]),
     "mlpsp_mlp_grouped_scratch_bytes": (C.c_int64, [C.c_int64, C.c_int32]),
     "mlpsp_mlp_grouped": (C.c_int, [C.POINTER(Scene), C.c_int32, _fp, _fp, C.c_int64, _fp, _fp, C.c_int64, _fp, _fp]),
     "mlpsp_group_records_scratch_bytes": (C.c_int64, [C.c_int64, C.c_int32]),

@@ -350,7 +350,20 @@ extern "C" int mlpsp_export_records(const mlpsp_scene* sc, const mlpsp_frame* fr
   rc = get_scratch(sc, fr, s, "mlpsp_export_records");
   if (rc) return rc;
   return launch_export_records(sc, fr, s, offsets, ids, x6, raw, relu_masks, gates, max_out, max_hits, total_host,
-                               worst_host, (cudaStream_t)stream);
+                               worst_host, /*counted=*/false, (cudaStream_t)stream);
+}
+
+extern "C" int mlpsp_export_counted_records(const mlpsp_scene* sc, const mlpsp_frame* fr, int32_t* ids, float* x6, float* raw,
+                                            int32_t* relu_masks, float* gates, int64_t total, void* stream) {
+  int rc = check_frame_common(sc, fr, "mlpsp_export_counted_records");
+  if (rc) return rc;
+  MLPSP_REQUIRE(fr->keep_records == 1, MLPSP_E_ARG, "mlpsp_export_counted_records: the frame was not rendered with keep_records = 1");
+  MLPSP_REQUIRE(fr->rays_o && fr->rays_d && total >= 0, MLPSP_E_ARG, "mlpsp_export_counted_records: rays missing or negative total");
+  Scratch s;
+  rc = get_scratch(sc, fr, s, "mlpsp_export_counted_records");
+  if (rc) return rc;
+  return launch_export_records(sc, fr, s, nullptr, ids, x6, raw, relu_masks, gates, total, 0, nullptr, nullptr, /*counted=*/true,
+                               (cudaStream_t)stream);
 }
 
 // ------------------------------------------------------------ grouped evaluator on records ----

@@ -253,9 +253,10 @@ int launch_mlp_f16(const mlpsp_scene* sc, const RecIn* rec_in, const int4* work,
 // direction (launch_fill with the table flag; not together with a small-group list or record export).
 int launch_encode_directions(const mlpsp_scene* sc, const mlpsp_frame* fr, char* table, cudaStream_t st);
 int launch_scan_i32(const int32_t* in, int64_t n, int32_t* blk, int32_t* out, cudaStream_t st);
+// counted: the per-pixel counts and their prefix are those of the call before; writes the rows only
 int launch_export_records(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, int64_t* offsets, int32_t* ids,
                           float* x6, float* raw, int32_t* relu_masks, float* gates, int64_t max_out, int32_t max_hits,
-                          int64_t* total_host, int32_t* worst_host, cudaStream_t st);
+                          int64_t* total_host, int32_t* worst_host, bool counted, cudaStream_t st);
 
 // evaluator output modes
 constexpr int kOutAlpha = 0;     // (R,G,B, 1-exp(-softplus(o3)*decay)) scattered to rec.slot

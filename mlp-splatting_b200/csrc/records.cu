@@ -1621,9 +1621,13 @@ int launch_render_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scr
 // Pixel-major records in compositing order (np_tile_kernels.cu:3138-3154; training_wmma.cuh:223-256),
 // rebuilt after the frame from the consumed masks, the evaluator outputs kept per compositing slot
 // and a recomputed hit test.  Two passes like the reference: count per pixel, prefix, emit.  A pixel's lane walks the pairs
-// it consumed (the masks of 32 pairs transposed), so a warp takes as many rounds as its busiest pixel has records.  Bound:
-// the latency of a round's loads; a walk over the pairs that any pixel of the warp consumed took 218 us for 0.7 M records
-// (320 x 240), this 152.
+// it consumed (the masks of 32 pairs transposed) and lists its records in output order; the warp then writes the list, 32
+// records at a time, whose rows follow one another in memory (a row of the tile is one run).  More than kExportList records
+// of 32 pixels are written during the walk.  Bound: the stores' sectors.  A walk over the pairs that any pixel of the warp
+// consumed took 218 us for 0.7 M records (320 x 240), each pixel's own walk with its stores 152, this 123.
+constexpr int kExportList = 1024;
+struct ExportSmem { uint32_t slot[kExportList]; int32_t prim[kExportList]; uint8_t lane[kExportList]; int pix[32]; int64_t out[32]; };
+
 template <bool EMIT>
 __global__ void __launch_bounds__(64) k_export(
     const float* __restrict__ rays_o, const float* __restrict__ rays_d, const float4* __restrict__ geom,
@@ -1633,15 +1637,61 @@ __global__ void __launch_bounds__(64) k_export(
     const float* __restrict__ rec_tr, const float4* __restrict__ px_state, int32_t* __restrict__ px_cnt,
     const int32_t* __restrict__ px_off, int max_hits, int32_t* __restrict__ worst, int32_t* __restrict__ ids,
     float* __restrict__ x6, float* __restrict__ raw, int32_t* __restrict__ relu_masks, float* __restrict__ gates,
-    int64_t max_out, int ref_arith, const int32_t* __restrict__ status) {
+    int64_t max_out, int ref_arith, int vec, const int32_t* __restrict__ status) {
+  __shared__ ExportSmem s_all[EMIT ? 2 : 1];
   if (status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
   const int tile = blockIdx.x;
   const int s = tile_offsets[tile], e = s + tile_len[tile];
   const int lane = threadIdx.x & 31, half = threadIdx.x >> 5;
+  ExportSmem& sm = s_all[EMIT ? half : 0];
   const TilePix tp = tile_pixel(tile, half * 32 + lane, ntx, W, H);
-  V3 o = {0.f, 0.f, 0.f}, d = {0.f, 0.f, 0.f};
   int64_t out0 = 0;
-  if (EMIT && tp.valid) { o = load3(rays_o, tp.pix); d = load3(rays_d, tp.pix); out0 = px_off[tp.pix]; }
+  int own = 0, first_entry = 0, total = 0;            // records of this lane's pixel, their place among the warp's
+  if (EMIT) {
+    if (tp.valid) { out0 = px_off[tp.pix]; own = px_off[tp.pix + 1] - (int)out0; }
+    const int inc = warp_inclusive_scan(own);
+    first_entry = inc - own;
+    total = __shfl_sync(0xffffffffu, inc, 31);
+  }
+  // one record: slot of its evaluation, primitive, pixel, place in the output
+  auto emit = [&](uint32_t slot, int p, int pix, int64_t r) {
+    if (r >= max_out) return;
+    const float4 ro = rec_out[slot], re = rec_ext[slot];
+    const float tr = raw ? rec_tr[slot] : 0.f;
+    const V3 o = load3(rays_o, pix), d = load3(rays_d, pix);
+    Hit h;
+    if (ref_arith) hit_test_ref(load_geom_ref(geom, p), o, d, thr, h);
+    else hit_test(load_geom(geom, p), o, d, thr, h);
+    if (ids) ids[r] = p;
+    if (x6) {
+      if (vec) {
+        float2* q = reinterpret_cast<float2*>(x6) + r * 3;
+        q[0] = make_float2(d.x, d.y); q[1] = make_float2(d.z, h.dx); q[2] = make_float2(h.dy, h.dz);
+      } else {
+        float* q = x6 + r * 6; q[0] = d.x; q[1] = d.y; q[2] = d.z; q[3] = h.dx; q[4] = h.dy; q[5] = h.dz;
+      }
+    }
+    if (raw) {
+      if (vec) {
+        float4* q = reinterpret_cast<float4*>(raw) + r * 2;
+        q[0] = make_float4(ro.x, ro.y, ro.z, re.x); q[1] = make_float4(tr, ro.w, h.decay, re.y);
+      } else {
+        float* q = raw + r * 8;
+        q[0] = ro.x; q[1] = ro.y; q[2] = ro.z; q[3] = re.x; q[4] = tr; q[5] = ro.w; q[6] = h.decay; q[7] = re.y;
+      }
+    }
+    if (relu_masks) {
+      const int2 m = make_int2((int32_t)__float_as_uint(re.z), (int32_t)__float_as_uint(re.w));
+      if (vec) reinterpret_cast<int2*>(relu_masks)[r] = m;
+      else { relu_masks[r * 2] = m.x; relu_masks[r * 2 + 1] = m.y; }
+    }
+    if (gates) {
+      const float4 g = tetra_gates(h, gate_scales(__ldg(geom + (size_t)p * 4 + 3), beta), tau);
+      if (vec) reinterpret_cast<float4*>(gates)[r] = g;
+      else { float* q = gates + r * 4; q[0] = g.x; q[1] = g.y; q[2] = g.z; q[3] = g.w; }
+    }
+  };
+  const bool listed = EMIT && total <= kExportList;
   const uint32_t lt = (1u << lane) - 1u;
   int cnt = 0;
   for (int i0 = s; i0 < e; i0 += 32) {
@@ -1671,26 +1721,21 @@ __global__ void __launch_bounds__(64) k_export(
       if (!todo) continue;
       todo &= todo - 1u;
       const uint32_t slot = fj + __popc(hj & lt);
-      const int64_t r = out0 + cnt;
-      ++cnt;
-      if (r >= max_out) continue;
-      const float4 ro = rec_out[slot], re = rec_ext[slot];
-      const float tr = raw ? rec_tr[slot] : 0.f;
-      Hit h;
-      if (ref_arith) hit_test_ref(load_geom_ref(geom, p), o, d, thr, h);
-      else hit_test(load_geom(geom, p), o, d, thr, h);
-      if (ids) ids[r] = p;
-      if (x6) { float* q = x6 + r * 6; q[0] = d.x; q[1] = d.y; q[2] = d.z; q[3] = h.dx; q[4] = h.dy; q[5] = h.dz; }
-      if (raw) {
-        float* q = raw + r * 8;
-        q[0] = ro.x; q[1] = ro.y; q[2] = ro.z; q[3] = re.x; q[4] = tr; q[5] = ro.w; q[6] = h.decay; q[7] = re.y;
+      const int k = cnt++;
+      if (listed) {
+        if (k < own) { sm.slot[first_entry + k] = slot; sm.prim[first_entry + k] = p; sm.lane[first_entry + k] = (uint8_t)lane; }
+      } else {
+        emit(slot, p, tp.pix, out0 + k);
       }
-      if (relu_masks) { relu_masks[r * 2] = (int32_t)__float_as_uint(re.z); relu_masks[r * 2 + 1] = (int32_t)__float_as_uint(re.w); }
-      if (gates) {
-        const float4 ls = __ldg(geom + (size_t)p * 4 + 3);
-        const float4 g = tetra_gates(h, gate_scales(ls, beta), tau);
-        float* q = gates + r * 4; q[0] = g.x; q[1] = g.y; q[2] = g.z; q[3] = g.w;
-      }
+    }
+  }
+  if (listed) {
+    sm.pix[lane] = tp.valid ? tp.pix : 0;
+    sm.out[lane] = out0 - first_entry;
+    __syncwarp();
+    for (int k = lane; k < total; k += 32) {
+      const int l = sm.lane[k];
+      emit(sm.slot[k], sm.prim[k], sm.pix[l], sm.out[l] + k);
     }
   }
   if (!EMIT && tp.valid) {
@@ -1708,30 +1753,43 @@ __global__ void k_widen_i32(const int32_t* __restrict__ in, int64_t n, int64_t* 
 
 int launch_export_records(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, int64_t* offsets, int32_t* ids,
                           float* x6, float* raw, int32_t* relu_masks, float* gates, int64_t max_out, int32_t max_hits,
-                          int64_t* total_host, int32_t* worst_host, cudaStream_t st) {
+                          int64_t* total_host, int32_t* worst_host, bool counted, cudaStream_t st) {
   const int W = fr->width, H = fr->height, T = num_tiles(W, H, 8), ntx = (W + 7) / 8;
   const int64_t P = (int64_t)W * H;
   int32_t* worst = s.counters + kCtrScratch;     // [0] largest per-pixel count, [1] capacity flag
-  MLPSP_CUDA_OK(cudaMemsetAsync(worst, 0, 8, st));
-  LaunchScope scope(kKMisc, 3 + scan_launches(P), st);
-  k_export<false><<<T, 64, 0, st>>>(fr->rays_o, fr->rays_d, (const float4*)sc->geom, fr->tile_offsets, s.tile_len, fr->sorted_prims,
-                                    W, H, ntx, fr->threshold, sc->gate_beta, sc->gate_tau, s.used32, s.masks32,
-                                    s.pair_base, s.rec_out, s.rec_ext, s.rec_tr, s.px_state, s.px_cnt, nullptr, max_hits,
-                                    worst, nullptr, nullptr, nullptr, nullptr, nullptr, 0, fr->hit_arith == 1 ? 1 : 0, fr->status);
-  int rc = launch_scan_i32(s.px_cnt, P, s.scan_blk, s.px_off, st);
-  if (rc) return rc;
-  k_widen_i32<<<(unsigned)((P + 1 + 255) / 256), 256, 0, st>>>(s.px_off, P + 1, offsets);
-  int32_t h[3] = {0, 0, 0};
-  MLPSP_CUDA_OK(cudaMemcpyAsync(&h[0], s.px_off + P, 4, cudaMemcpyDeviceToHost, st));
-  MLPSP_CUDA_OK(cudaMemcpyAsync(&h[1], worst, 8, cudaMemcpyDeviceToHost, st));
-  MLPSP_CUDA_OK(cudaStreamSynchronize(st));
-  if (total_host) *total_host = h[0];
-  if (worst_host) *worst_host = h[2] ? -h[1] : h[1];
-  if ((ids || x6 || raw || relu_masks || gates) && max_out >= h[0] && h[0] > 0) {
+  const bool outputs = ids || x6 || raw || relu_masks || gates;
+  int64_t total = max_out;                       // counted: the caller holds this frame's total
+  if (!counted) {
+    LaunchScope scope(kKMisc, 2 + scan_launches(P), st);
+    HostWords& hw = host_words();
+    cudaEvent_t ev = nullptr;
+    int rc = hw.open(&ev);
+    if (rc) return rc;
+    MLPSP_CUDA_OK(cudaMemsetAsync(worst, 0, 8, st));
+    k_export<false><<<T, 64, 0, st>>>(fr->rays_o, fr->rays_d, (const float4*)sc->geom, fr->tile_offsets, s.tile_len, fr->sorted_prims,
+                                      W, H, ntx, fr->threshold, sc->gate_beta, sc->gate_tau, s.used32, s.masks32,
+                                      s.pair_base, s.rec_out, s.rec_ext, s.rec_tr, s.px_state, s.px_cnt, nullptr, max_hits,
+                                      worst, nullptr, nullptr, nullptr, nullptr, nullptr, 0, fr->hit_arith == 1 ? 1 : 0, 0, fr->status);
+    rc = launch_scan_i32(s.px_cnt, P, s.scan_blk, s.px_off, st);
+    if (rc) return rc;
+    k_widen_i32<<<(unsigned)((P + 1 + 255) / 256), 256, 0, st>>>(s.px_off, P + 1, offsets);
+    MLPSP_CUDA_OK(cudaMemcpyAsync(hw.word, s.px_off + P, 4, cudaMemcpyDeviceToHost, st));
+    MLPSP_CUDA_OK(cudaMemcpyAsync(hw.word + 1, worst, 8, cudaMemcpyDeviceToHost, st));
+    MLPSP_CUDA_OK(cudaEventRecord(ev, st));
+    MLPSP_CUDA_OK(cudaEventSynchronize(ev));
+    const volatile int32_t* h = hw.word;
+    total = h[0];
+    if (total_host) *total_host = h[0];
+    if (worst_host) *worst_host = h[2] ? -h[1] : h[1];
+  }
+  if (outputs && max_out >= total && total > 0) {
+    LaunchScope scope(kKMisc, 1, st);
+    const int vec = (reinterpret_cast<uintptr_t>(x6) & 7) == 0 && (reinterpret_cast<uintptr_t>(relu_masks) & 7) == 0 &&
+                    ((reinterpret_cast<uintptr_t>(raw) | reinterpret_cast<uintptr_t>(gates)) & 15) == 0;
     k_export<true><<<T, 64, 0, st>>>(fr->rays_o, fr->rays_d, (const float4*)sc->geom, fr->tile_offsets, s.tile_len, fr->sorted_prims,
                                      W, H, ntx, fr->threshold, sc->gate_beta, sc->gate_tau, s.used32, s.masks32,
                                      s.pair_base, s.rec_out, s.rec_ext, s.rec_tr, s.px_state, s.px_cnt, s.px_off, max_hits,
-                                     worst, ids, x6, raw, relu_masks, gates, max_out, fr->hit_arith == 1 ? 1 : 0, fr->status);
+                                     worst, ids, x6, raw, relu_masks, gates, max_out, fr->hit_arith == 1 ? 1 : 0, vec, fr->status);
   }
   return cuda_check(cudaGetLastError(), "export_records");
 }

@@ -425,9 +425,10 @@ def render_tiles_training_records(tensors, width, height, tile, threshold, beta,
     ro, rd, pos, ls, q, culled, offs, freq, att, W1, b1, W2, b2, W3, b3 = tensors[:15]
     dev = ro.device
     scene = PackedScene(pos, ls, q, W1, b1, W2, b2, W3, b3, freq, att, gate_beta=float(beta), gate_tau=float(temperature),
-                        device=dev, pack_f16=(precision == "float16"))
+                        device=dev, pack_f16=(precision == "float16"), _settle=False)
     r = FrameRenderer(int(width), int(height), device=dev, max_pairs=max(int(culled.numel()), 1),
                       tile_capacity=cfg["tile_candidate_capacity"])
+    scene._settle_pack()        # the weights have been packed while the buffers were made
     prec = L.PRECISION_F16 if (precision == "float16" and scene.has_f16) else L.PRECISION_F32
     return r.render_records(scene, ro.contiguous().float(), rd.contiguous().float(), float(threshold), max_hits=max_hits,
                             precision=prec, tile_lists=(culled, offs), rays_normalized=True,

@@ -64,7 +64,7 @@ class PackedScene:
     """
 
     def __init__(self, positions, log_scales, quats, W1, b1, W2, b2, W3, b3, freq, att, feat_attr=None,
-                 gate_beta=1.5, gate_tau=2.0, device="cuda", pack_f16=True, pack_bf16=False, feat_f16="exact"):
+                 gate_beta=1.5, gate_tau=2.0, device="cuda", pack_f16=True, pack_bf16=False, feat_f16="exact", _settle=True):
         """feat_f16: "exact" keeps a binary16 copy of feat_attr for the tensor-core feature compositing when every
         attribute is representable in binary16 (the reference's inference export stores them so,
         scannet/checkpoints.py:358-359), "round" keeps it even when the copy rounds, "off" never."""
@@ -101,6 +101,7 @@ class PackedScene:
             self.feat16 = None
             self.f16_rejected = False
             self.c = self._struct()
+            self._packing = None        # binary16 image whose status nobody has read yet
             self._pack_features(feat_f16)
             wbytes = int(lib.mlpsp_packed_weight_bytes(self.hidden, self.num_freq))
             if pack_f16 and wbytes > 0 and self.n > 0:
@@ -108,13 +109,9 @@ class PackedScene:
                 st = torch.zeros(L.STATUS_WORDS, device=d, dtype=torch.int32)
                 L.check(lib.mlpsp_pack_weights_f16(C.byref(self.c), L.ptr(w16), L.ptr(st), _stream_ptr(d)),
                         "mlpsp_pack_weights_f16")
-                # weights that are not finite in binary16 keep the scene on the FP32 evaluator, which is
-                # what the reference's per-frame overflow check amounts to (rgb_wmma.cuh:162-176, 260-272)
-                if int(st[L.ST_BITS].item()) & L.BIT_NUMERIC:
-                    self.f16_rejected = True
-                else:
-                    self.w16 = w16
-                self.c = self._struct()
+                self._packing = (w16, st)
+                if _settle:
+                    self._settle_pack()
             if pack_bf16 and wbytes > 0 and self.n > 0:
                 # the same image with bfloat16 operands (the bf16 flag of render_tiles_rgb_wmma, rgb_wmma.cuh:225)
                 wb = torch.empty(self.n * wbytes, device=d, dtype=torch.uint8)
@@ -124,6 +121,21 @@ class PackedScene:
                 if not (int(st[L.ST_BITS].item()) & L.BIT_NUMERIC):
                     self.wbf16 = wb
                 self.c = self._struct()
+
+    def _settle_pack(self):
+        """Reads the status of the binary16 packing (the constructor does, unless it was told to leave it to a caller that
+        has other work to do meanwhile)."""
+        if self._packing is None:
+            return
+        w16, st = self._packing
+        self._packing = None
+        # weights that are not finite in binary16 keep the scene on the FP32 evaluator, which is
+        # what the reference's per-frame overflow check amounts to (rgb_wmma.cuh:162-176, 260-272)
+        if int(st[L.ST_BITS].item()) & L.BIT_NUMERIC:
+            self.f16_rejected = True
+        else:
+            self.w16 = w16
+        self.c = self._struct()
 
     @classmethod
     def from_packed_image(cls, positions, log_scales, quats, freq, att, w16, hidden, feat_attr=None, gate_beta=1.5,
@@ -657,9 +669,8 @@ class FrameRenderer:
             masks = torch.empty((R, 2), device=d, dtype=torch.int32)
             gates = torch.empty((R, 4), device=d, dtype=torch.float32)
             if R > 0:
-                L.check(lib.mlpsp_export_records(C.byref(scene.c), C.byref(f), L.ptr(offsets), L.ptr(ids), L.ptr(x6),
-                                                 L.ptr(raw), L.ptr(masks), L.ptr(gates), R, int(max_hits),
-                                                 C.byref(total), C.byref(worst), st), "mlpsp_export_records")
+                L.check(lib.mlpsp_export_counted_records(C.byref(scene.c), C.byref(f), L.ptr(ids), L.ptr(x6), L.ptr(raw),
+                                                         L.ptr(masks), L.ptr(gates), R, st), "mlpsp_export_counted_records")
         return [rgb.clone(), alpha.clone(), ids, x6, raw, masks, gates, offsets]
 
     def bin(self, scene: PackedScene, view, proj, threshold, check=True):
