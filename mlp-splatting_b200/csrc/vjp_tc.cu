@@ -182,11 +182,13 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
 
   char* my = smem + tid * 16;
   uint32_t ph = 0u;
-  // tile writes visible to the tensor core, tensor-memory reads retired, then one thread issues and commits
-  auto issue_phase = [&](auto issue) {
+  bool ok = true;
+  // tile writes visible to the tensor core, tensor-memory reads retired, then one thread issues and commits; false in all
+  // threads when a wait has given up in one
+  auto issue_phase = [&](auto issue) -> bool {
     fence_async_smem();
     tc_fence_before();
-    __syncthreads();
+    if (!__syncthreads_and(ok)) return false;
     if (warp == 0) {
       tc_fence_after();
       if (elect_one()) {
@@ -195,12 +197,14 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
       }
       __syncwarp();
     }
+    return true;
   };
-  auto wait_phase = [&]() -> bool {
-    const bool done = mbar_wait(bar, ph & 1u);
+  // every thread waits for itself: what it touches next is its own (tile rows, tensor-memory lanes), and the barrier of the
+  // next issue_phase is the one that tells the CTA of a wait that gave up
+  auto wait_phase = [&]() {
+    ok = __all_sync(0xffffffffu, mbar_wait(bar, ph & 1u)) && ok;
     ++ph;
     tc_fence_after();
-    return __syncthreads_and(done) != 0;
   };
 
   // ---- a step's inputs in registers: one record per thread, and with a new primitive its weights ----
@@ -311,7 +315,7 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
   load_weights(it.prim);
   load_rec(it, 0);
   int sub = 0;
-  bool ok = true, pending = false, finished = false;      // gradient MMAs in flight; they complete segment it_p
+  bool pending = false, finished = false;      // gradient MMAs in flight; they complete segment it_p
 
   for (;;) {
     // ---- encoding (index c * 6 + f holds sin, 36 + c * 6 + f holds cos: scannet/cumodel.py:183-195) and D3,
@@ -332,9 +336,8 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
     const uint32_t d01 = pack_h2<BF16>(rg.x * scale, rg.y * scale), d23 = pack_h2<BF16>(rg.z * scale, rg.w * scale);
     uint32_t m1 = rm1, m2 = rm2;
     if (pending) {
-      ok = wait_phase();
-      if (!ok) break;
-      if (finished) emit(it_p);
+      wait_phase();
+      if (finished && ok) emit(it_p);
     }
     if (sub == 0) store_weights();
 #pragma unroll
@@ -346,7 +349,7 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
       vjp_d2<BF16>(d01, d23, m2, reinterpret_cast<const float4*>(s_w3), my + kVcD2 * kVjpChunk);
     }
     // ---- layer 1: K = 80 (the ones behind E meet the zero chunk of W1); with masks the first half of D1 ----
-    issue_phase([&]() {
+    ok = issue_phase([&]() {
       const uint64_t a = a_rows(kVcE);
 #pragma unroll
       for (int ks = 0; ks < 5; ++ks) mma_f16(tmem, adv(a, ks * 2 * kVjpChunk), adv(w1_desc, ks * 2 * 512), idesc_h, ks > 0);
@@ -355,6 +358,7 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
         for (int ks = 0; ks < 2; ++ks) mma_f16(tmem + kVtD1, adv(a_rows(kVcD2), ks * 2 * kVjpChunk), adv(w2t_desc, ks * 256), idesc_d1h, ks > 0);
       }
     });
+    if (!ok) break;
     // ---- the next step's loads, in flight from here on ----
     const int cnt = min(kVjpRows, it.rows - sub);
     const bool last = sub + kVjpRows >= it.rows;
@@ -376,8 +380,7 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
       more = false;
     }
     zero_next();
-    ok = wait_phase();
-    if (!ok) break;
+    wait_phase();
     {
       uint32_t acc[32];
       tmem_ld32(trow, acc);
@@ -390,7 +393,7 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
       vjp_adjoint<BF16, 16>(acc, m1, my + kVcD1 * kVjpChunk);
     }
     // ---- layer 2; with masks the second half of D1 ----
-    issue_phase([&]() {
+    ok = issue_phase([&]() {
       const uint64_t a = a_rows(kVcH1);
 #pragma unroll
       for (int ks = 0; ks < 2; ++ks) mma_f16(tmem, adv(a, ks * 2 * kVjpChunk), adv(w2_desc, ks * 2 * 512), idesc_h, ks > 0);
@@ -400,8 +403,8 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
           mma_f16(tmem + kVtD1, adv(a_rows(kVcD2), ks * 2 * kVjpChunk), adv(w2t_desc, 2 * 512 + ks * 256), idesc_d1h, ks > 0);
       }
     });
-    ok = wait_phase();
     if (!ok) break;
+    wait_phase();
     {
       uint32_t acc[32];
       tmem_ld32(trow, acc);
@@ -414,18 +417,18 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
       vjp_adjoint<BF16, 16>(acc, m1 >> 16, my + (kVcD1 + 2) * kVjpChunk);
     } else {
       vjp_d2<BF16>(d01, d23, m2, reinterpret_cast<const float4*>(s_w3), my + kVcD2 * kVjpChunk);
-      issue_phase([&]() {
+      ok = issue_phase([&]() {
 #pragma unroll
         for (int ks = 0; ks < 2; ++ks) mma_f16(tmem, adv(a_rows(kVcD2), ks * 2 * kVjpChunk), adv(w2t_desc, ks * 256), idesc_d1, ks > 0);
       });
-      ok = wait_phase();
       if (!ok) break;
+      wait_phase();
       uint32_t acc[32];
       tmem_ld32(trow, acc);
       vjp_adjoint<BF16, 32>(acc, m1, my + kVcD1 * kVjpChunk);
     }
     // ---- gradients: contraction over the block's records, 16 per MMA ----
-    issue_phase([&]() {
+    ok = issue_phase([&]() {
       const uint64_t e = mn(kVcE), h = mn(kVcH1), d1 = mn(kVcD1), d23t = mn(kVcD2);
       const int steps = (cnt + 15) >> 4;
       for (int ks = 0; ks < steps; ++ks) {
@@ -434,6 +437,7 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
         mma_f16(tmem + kVtG2, adv(h, ks * 256), adv(d23t, ks * 256), idesc_g2, acc);
       }
     });
+    if (!ok) break;
     pending = true;
     finished = last;
     it_p = it_c;
@@ -441,7 +445,7 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
   }
   if (ok) {
     while (empty < E) zero_next();
-    ok = wait_phase();
+    wait_phase();
     if (ok) emit(it_p);
   }
   if (bad) atomicOr(counters + kVpFlag, 1);
