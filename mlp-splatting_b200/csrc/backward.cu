@@ -93,23 +93,22 @@ __global__ void __launch_bounds__(256) k_reverse_check(const int32_t* __restrict
   if (b) { atomicOr(bad, b); if (bad_host) atomicOr_system(const_cast<int32_t*>(bad_host), b); }
 }
 
-// A block's pixels own one run of records, which is brought into shared memory in whole lines; the outputs take their
-// records' places there and leave the same way.  A run beyond kRevStage records (about 12 per pixel is usual) is read and
-// written directly, four records at a time: their loads do not depend on the recurrence, so they are in flight together.
-// Bound: memory, 52 bytes per record; 4.3 M records in 480,000 pixels, all directly: 167 us, staged: 134.
-constexpr int kRevPixels = 128, kRevStage = 1536;
+// A block's pixels own one run of records.  It is brought into shared memory in whole lines, from its end on, kRevStage
+// records at a time; a thread walks those of its pixel among them, the outputs take the records' places and leave the same
+// way.  Bound: memory, 52 bytes per record; 4.3 M records in 480,000 pixels read and written by the walk itself: 167 us,
+// staged: 74.
+constexpr int kRevPixels = 128, kRevStage = 1024;
 __global__ void __launch_bounds__(kRevPixels) k_reverse_pixels(const int64_t* __restrict__ offsets, const float* __restrict__ raw,
                                  const float* __restrict__ grgb, const float* __restrict__ gt, int64_t pixels,
                                  float* __restrict__ d4, float* __restrict__ kw, const int32_t* __restrict__ bad) {
   chain_wait();
   chain_release();
-  extern __shared__ __align__(16) float4 s_raw[];      // two per record
+  __shared__ __align__(16) float4 s_raw[2 * kRevStage];
   if (*bad) return;
   const int tid = threadIdx.x;
   const int64_t p0 = (int64_t)blockIdx.x * kRevPixels, p1 = min(p0 + kRevPixels, pixels), pix = p0 + tid;
-  const int64_t base = offsets[p0], run = offsets[p1] - base;
+  const int64_t base = offsets[p0], end = offsets[p1];
   const float4* raw4 = reinterpret_cast<const float4*>(raw);
-  const bool staged = run <= kRevStage;
   float gr = 0.f, gg = 0.f, gb = 0.f, behind = 0.f;
   int64_t first = 0, last = -1;
   if (pix < pixels) {
@@ -118,49 +117,32 @@ __global__ void __launch_bounds__(kRevPixels) k_reverse_pixels(const int64_t* __
     first = offsets[pix];
     last = offsets[pix + 1] - 1;
   }
-  // one record: its outputs, and the colour behind it
-  auto step = [&](const float4 a, const float4 c, float4& out, float& weight) {     // R, G, B, sigma_raw; trans before, alpha, decay, sigma logit
-    const float colour = gr * a.x + gg * a.y + gb * a.z;
-    const float g_alpha = c.x * (colour - behind);
-    behind = behind * (1.f - c.y) + colour * c.y;
-    const float g_sigma = g_alpha * __expf(-a.w * c.z);   // d alpha / d (sigma_raw * decay) = 1 - alpha
-    const float w = c.x * c.y, parked = g_sigma * c.z;
-    out = make_float4(gr * w * a.x * (1.f - a.x), gg * w * a.y * (1.f - a.y), gb * w * a.z * (1.f - a.z),
-                      parked * sigmoid_fast(c.w));        // softplus' = sigmoid
-    weight = parked * a.w;                                // g_decay * decay
-  };
-  if (staged) {
-    for (int i = tid; i < 2 * (int)run; i += kRevPixels) s_raw[i] = __ldg(raw4 + 2 * base + i);
+  const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_raw);
+  for (int64_t hi = end; hi > base;) {
+    const int64_t lo = max(base, hi - kRevStage);
+    const int run = (int)(hi - lo);
+    for (int i = tid; i < 2 * run; i += kRevPixels)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * (uint32_t)i), "l"(raw4 + 2 * lo + i) : "memory");
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    for (int q = (int)(last - base); q >= (int)(first - base); --q) {
-      float4 out;
-      float weight;
-      step(s_raw[2 * q], s_raw[2 * q + 1], out, weight);
-      s_raw[2 * q] = out;
-      s_raw[2 * q + 1].x = weight;
+    for (int q = (int)(min(last, hi - 1) - lo), q0 = (int)max(first - lo, (int64_t)0); q >= q0; --q) {
+      const float4 a = s_raw[2 * q], c = s_raw[2 * q + 1];  // R, G, B, sigma_raw; trans before, alpha, decay, sigma logit
+      const float colour = gr * a.x + gg * a.y + gb * a.z;
+      const float g_alpha = c.x * (colour - behind);
+      behind = behind * (1.f - c.y) + colour * c.y;
+      const float g_sigma = g_alpha * __expf(-a.w * c.z);   // d alpha / d (sigma_raw * decay) = 1 - alpha
+      const float w = c.x * c.y, parked = g_sigma * c.z;
+      s_raw[2 * q] = make_float4(gr * w * a.x * (1.f - a.x), gg * w * a.y * (1.f - a.y), gb * w * a.z * (1.f - a.z),
+                                 parked * sigmoid_fast(c.w));                               // softplus' = sigmoid
+      s_raw[2 * q + 1].x = parked * a.w;                    // g_decay * decay
     }
     __syncthreads();
-    for (int i = tid; i < (int)run; i += kRevPixels) {
-      *reinterpret_cast<float4*>(d4 + (base + i) * 4) = s_raw[2 * i];
-      kw[base + i] = s_raw[2 * i + 1].x;
+    for (int i = tid; i < run; i += kRevPixels) {
+      *reinterpret_cast<float4*>(d4 + (lo + i) * 4) = s_raw[2 * i];
+      kw[lo + i] = s_raw[2 * i + 1].x;
     }
-    return;
-  }
-  for (int64_t r = last; r >= first; r -= 4) {
-    float4 a4[4], c4[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int64_t q = r - u >= first ? r - u : first;
-      a4[u] = __ldg(raw4 + 2 * q);
-      c4[u] = __ldg(raw4 + 2 * q + 1);
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      if (r - u < first) break;
-      float4 out;
-      step(a4[u], c4[u], out, kw[r - u]);
-      *reinterpret_cast<float4*>(d4 + (r - u) * 4) = out;
-    }
+    hi = lo;
+    if (hi > base) __syncthreads();
   }
 }
 
@@ -692,7 +674,7 @@ extern "C" int mlpsp_records_reverse_checked(const int32_t* ids, const int64_t* 
     static DeviceOnce attr_once;
     if (attr_once.first())
       MLPSP_CUDA_OK(cudaFuncSetAttribute(k_reverse_geometry, cudaFuncAttributeMaxDynamicSharedMemorySize, kRevSmem));
-    launch_chained(k_reverse_pixels, dim3((unsigned)((pixels + kRevPixels - 1) / kRevPixels)), dim3(kRevPixels), kRevStage * 32, st, offsets, raw, grad_rgb, grad_t, pixels, d4, kw, bad);
+    launch_chained(k_reverse_pixels, dim3((unsigned)((pixels + kRevPixels - 1) / kRevPixels)), dim3(kRevPixels), 0, st, offsets, raw, grad_rgb, grad_t, pixels, d4, kw, bad);
     launch_chained(k_reverse_geometry, dim3((unsigned)((total_records + kRevChunk - 1) / kRevChunk)), dim3(kRevThreads),
                    kRevSmem, st, ids, x6, kw, quats,
                    total_records, acc, bad);
