@@ -47,7 +47,8 @@ def flop_per_record(hidden):
 
 def weight_image_bytes(hidden):
     """Bytes of one primitive's packed weight image (biases included), as the evaluator streams it per work item."""
-    return 9472 if hidden == 32 else 22784
+    from mlp_splatting_b200 import _lib
+    return int(_lib.load().mlpsp_packed_weight_bytes(hidden, 6))
 
 
 def peaks():
