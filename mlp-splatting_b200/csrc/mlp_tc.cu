@@ -32,11 +32,10 @@ namespace mlpsp {
 constexpr int kRows = kRowsPerItem;      // 128 = MMA M
 constexpr int kChunk = kRows * 16;       // bytes of one K chunk of an A tile: [128 rows][8 halves]
 constexpr int kN3 = 16;                  // 4 outputs padded to the smallest N
-constexpr int kA1Chunks = 10;            // 72 encoded inputs and eight ones: two halves of 36 + 4
+constexpr int kA1Chunks = 10;            // 72 encoded inputs and a constant chunk that meets the bias terms
 
 // ---- packed weight image (per primitive) and shared-memory plan for F = 6, hidden width H = 32 or 64 ----
-// piece 1: W1 as [10 chunks][H rows][8 halves] in the order of enc_k(): the ray direction's 36 inputs and four terms of
-//          b1[h], the offset's 36 inputs and the other four terms (the A tile holds ones there);
+// piece 1: W1 as [10 chunks][H rows][8 halves]: K = 0..71 in the order of enc_k(), then the eight terms of b1[h];
 // piece 2: W2 as [H/8 + 1 chunks][H][8], the last one the terms of b2;
 // piece 3: W3 as [H/8 + 1 chunks][16][8] (rows 4..15 zero), the last one the terms of b3.
 template <int H>
@@ -70,15 +69,12 @@ struct Net {
 // Position of an encoded input inside the K dimension of layer 1.  The reference orders K as
 // [sin(c,f) for c, f][cos(c,f) for c, f] (np_tile_kernels.cu:329-343); a dot product does not care, so
 // the A tile and the packed W1 rows both use an order in which the six (sin, cos) pairs of one input
-// coordinate are contiguous (six 32-bit words per coordinate) and the coordinates of the ray direction and of the
-// offset fill five chunks each, the last four halves of which carry the bias:
-//   k' = 40 (c / 3) + 12 (c % 3) + 4 (f / 2) + 2 is_cos + (f % 2).
-__host__ __device__ constexpr int enc_k(int c, int f, int is_cos) {
-  return 40 * (c / 3) + 12 * (c % 3) + 4 * (f >> 1) + 2 * is_cos + (f & 1);
-}
+// coordinate are contiguous (six 32-bit words per coordinate):
+//   k' = 12 c + 4 (f / 2) + 2 is_cos + (f % 2).
+// The ray direction's 36 inputs fill the chunks 0..3 and the first half of chunk 4, the offset's the rest.
+__host__ __device__ constexpr int enc_k(int c, int f, int is_cos) { return 12 * c + 4 * (f >> 1) + 2 * is_cos + (f & 1); }
 __host__ __device__ constexpr int enc_k_of_reference(int k) { return enc_k((k % 36) / 6, (k % 36) % 6, k / 36); }
-// where term j of the layer-1 bias goes
-__host__ __device__ constexpr int enc_k_of_bias(int j) { return 40 * (j / 4) + 36 + j % 4; }
+constexpr int kBiasChunk = 9;            // the terms of the layer-1 bias
 
 // The six words of one input coordinate.  mult[f] is freq[f] * att[f].  LADDER: every band is exactly twice the
 // one before, so the phases are exact doublings of the first and sin / cos of the higher bands follow from the
@@ -108,36 +104,49 @@ __device__ __forceinline__ void encode_coord(float v, const float (&mult)[6], ui
 // a finite input gives finite phases (freq * att <= 101)
 __device__ __forceinline__ bool not_finite(float v) { return !(fabsf(v) < 1.0e30f); }
 
-// Three coordinates and four ones: five chunks of this thread's row of the layer-1 A tile (row = generic pointer to the
-// row's 16 bytes inside the first of them; kChunk = bytes between the K chunks of the tile).
 template <bool BF16>
 constexpr uint32_t kOnes2 = BF16 ? 0x3f803f80u : 0x3c003c00u;
 
-template <bool LADDER, bool BF16, int kChunk = mlpsp::kChunk>
+// Three coordinates into this thread's row of the layer-1 A tile, the ray direction (OFF = false) or the offset (row =
+// generic pointer to the row's 16 bytes inside chunk 0; kChunk = bytes between the K chunks), the first two and the third.
+template <bool LADDER, bool BF16, bool OFF, int kChunk = mlpsp::kChunk>
 __device__ __forceinline__ bool encode_two(float x, float y, const float (&mult)[6], char* row) {
   uint32_t a[6], b[6];
   encode_coord<LADDER, BF16>(x, mult, a);
   encode_coord<LADDER, BF16>(y, mult, b);
-  *reinterpret_cast<uint4*>(row) = make_uint4(a[0], a[1], a[2], a[3]);
-  *reinterpret_cast<uint4*>(row + kChunk) = make_uint4(a[4], a[5], b[0], b[1]);
-  *reinterpret_cast<uint4*>(row + 2 * kChunk) = make_uint4(b[2], b[3], b[4], b[5]);
+  if (OFF) {
+    *reinterpret_cast<uint2*>(row + 4 * kChunk + 8) = make_uint2(a[0], a[1]);
+    *reinterpret_cast<uint4*>(row + 5 * kChunk) = make_uint4(a[2], a[3], a[4], a[5]);
+    *reinterpret_cast<uint4*>(row + 6 * kChunk) = make_uint4(b[0], b[1], b[2], b[3]);
+    *reinterpret_cast<uint2*>(row + 7 * kChunk) = make_uint2(b[4], b[5]);
+  } else {
+    *reinterpret_cast<uint4*>(row) = make_uint4(a[0], a[1], a[2], a[3]);
+    *reinterpret_cast<uint4*>(row + kChunk) = make_uint4(a[4], a[5], b[0], b[1]);
+    *reinterpret_cast<uint4*>(row + 2 * kChunk) = make_uint4(b[2], b[3], b[4], b[5]);
+  }
   return not_finite(x) || not_finite(y);
 }
-template <bool LADDER, bool BF16, int kChunk = mlpsp::kChunk>
+template <bool LADDER, bool BF16, bool OFF, int kChunk = mlpsp::kChunk>
 __device__ __forceinline__ bool encode_one(float z, const float (&mult)[6], char* row) {
   uint32_t a[6];
   encode_coord<LADDER, BF16>(z, mult, a);
-  *reinterpret_cast<uint4*>(row + 3 * kChunk) = make_uint4(a[0], a[1], a[2], a[3]);
-  *reinterpret_cast<uint4*>(row + 4 * kChunk) = make_uint4(a[4], a[5], kOnes2<BF16>, kOnes2<BF16>);
+  if (OFF) {
+    *reinterpret_cast<uint2*>(row + 7 * kChunk + 8) = make_uint2(a[0], a[1]);
+    *reinterpret_cast<uint4*>(row + 8 * kChunk) = make_uint4(a[2], a[3], a[4], a[5]);
+  } else {
+    *reinterpret_cast<uint4*>(row + 3 * kChunk) = make_uint4(a[0], a[1], a[2], a[3]);
+    *reinterpret_cast<uint2*>(row + 4 * kChunk) = make_uint2(a[4], a[5]);
+  }
   return not_finite(z);
 }
-template <bool BF16, int kChunk = mlpsp::kChunk>
+template <bool BF16, bool OFF, int kChunk = mlpsp::kChunk>
 __device__ __forceinline__ bool encode_three(bool ladder, float x, float y, float z, const float (&mult)[6], char* row) {
-  if (ladder) return encode_two<true, BF16, kChunk>(x, y, mult, row) | encode_one<true, BF16, kChunk>(z, mult, row);
-  return encode_two<false, BF16, kChunk>(x, y, mult, row) | encode_one<false, BF16, kChunk>(z, mult, row);
+  if (ladder) return encode_two<true, BF16, OFF, kChunk>(x, y, mult, row) | encode_one<true, BF16, OFF, kChunk>(z, mult, row);
+  return encode_two<false, BF16, OFF, kChunk>(x, y, mult, row) | encode_one<false, BF16, OFF, kChunk>(z, mult, row);
 }
 
-// The encodings of the ray directions of a frame, in the operand format: per tile [5 chunks][64 pixels][16 bytes], so that
+// The encodings of the ray directions of a frame, in the operand format: per tile [5 chunks][64 pixels][16 bytes] (of the last
+// one 8 bytes are used), so that
 // the pixels of one tile -- neighbouring records of a primitive, mostly -- lie together in every chunk.
 constexpr int kDirTileBytes = 5 * 64 * 16, kDirChunk = 64 * 16;
 
@@ -157,7 +166,7 @@ __global__ void __launch_bounds__(256) k_encode_directions(const float* __restri
     const TilePix tp = tile_pixel((int)(i >> 6), (int)(i & 63), ntx, W, H);
     if (!tp.valid) continue;
     const V3 d = load3(rays_d, tp.pix);
-    encode_three<BF16, kDirChunk>(ladder, d.x, d.y, d.z, mult, table + (i >> 6) * kDirTileBytes + (i & 63) * 16);
+    encode_three<BF16, false, kDirChunk>(ladder, d.x, d.y, d.z, mult, table + (i >> 6) * kDirTileBytes + (i & 63) * 16);
   }
 }
 
@@ -266,6 +275,12 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
     const uint32_t v = tid < 8 ? kOnes2<BF16> : 0u;
     *reinterpret_cast<uint4*>(smem + N::kOffConst + tid * 16) = make_uint4(v, v, v, v);
   }
+  // the constant chunk: ones, so that the bias rides in the last K step of layer 1; with KEEP zeros, and the bias a step of its
+  // own as in layers 2 and 3 (the order of the sums decides saved ReLU signs of values next to zero)
+  if (tid < kRows) {
+    const uint32_t v = KEEP ? 0u : kOnes2<BF16>;
+    *reinterpret_cast<uint4*>(smem + N::kOffA1 + kBiasChunk * kChunk + tid * 16) = make_uint4(v, v, v, v);
+  }
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
@@ -317,6 +332,7 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
 #pragma unroll
         for (int ks = 0; ks < kA1Chunks / 2; ++ks)
           mma_f16(tmem + N::kD1, step(a1_desc, ks * 2 * kChunk), step(w1_desc, ks * 2 * N::kWChunk), idesc_h, ks > 0);
+        if (KEEP) mma_f16(tmem + N::kD1, ones_desc, step(w1_desc, kBiasChunk * N::kWChunk), idesc_h, 1u);
         mma_commit(bar_a);
       }
       __syncwarp();
@@ -398,7 +414,8 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
       const char* src = dir_table + (size_t)(pixel >> 6) * kDirTileBytes + (pixel & 63u) * 16;
       const uint32_t dst = a1 + tid * 16;
 #pragma unroll
-      for (int c = 0; c < 5; ++c) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + c * kChunk), "l"(src + c * kDirChunk) : "memory");
+      for (int c = 0; c < 4; ++c) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + c * kChunk), "l"(src + c * kDirChunk) : "memory");
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 4 * kChunk), "l"(src + 4 * kDirChunk) : "memory");
     };
     auto direction_landed = [&]() { asm volatile("cp.async.wait_all;" ::: "memory"); };
     char* my_row = smem + N::kOffA1 + tid * 16;
@@ -433,11 +450,11 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
       // rows past the end inside a live warp hold the zero record; their results are never stored
       if (TAB) {
         copy_direction(q1);
-        bad |= encode_three<BF16>(ladder, q0.x, q0.y, q0.z, mult, my_row + 5 * kChunk);
+        bad |= encode_three<BF16, true>(ladder, q0.x, q0.y, q0.z, mult, my_row);
         direction_landed();
       } else {
-        bad |= encode_three<BF16>(ladder, q0.x, q0.y, q0.z, mult, my_row);
-        bad |= encode_three<BF16>(ladder, q0.w, q1.x, q1.y, mult, my_row + 5 * kChunk);
+        bad |= encode_three<BF16, false>(ladder, q0.x, q0.y, q0.z, mult, my_row);
+        bad |= encode_three<BF16, true>(ladder, q0.w, q1.x, q1.y, mult, my_row);
       }
     }
     tile_done(bar_r0);
@@ -496,8 +513,8 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
       tile_done(bar_r0 + 8);
       // ---- first part of the next item's encoding while layer 2 runs ----
       if (next_live) {
-        if (!TAB) bad |= encode_three<BF16>(ladder, q0.x, q0.y, q0.z, mult, my_row);
-        else bad |= ladder ? encode_two<true, BF16>(q0.x, q0.y, mult, my_row + 5 * kChunk) : encode_two<false, BF16>(q0.x, q0.y, mult, my_row + 5 * kChunk);
+        if (!TAB) bad |= encode_three<BF16, false>(ladder, q0.x, q0.y, q0.z, mult, my_row);
+        else bad |= ladder ? encode_two<true, BF16, true>(q0.x, q0.y, mult, my_row) : encode_two<false, BF16, true>(q0.x, q0.y, mult, my_row);
       }
       ok = __all_sync(0xffffffffu, mbar_wait(bar_b, 0u) && ok);
       tc_fence_after();
@@ -507,9 +524,9 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
       // ---- second part of the next item's encoding while layer 3 runs ----
       if (next_live) {
         if (!TAB) {
-          bad |= encode_three<BF16>(ladder, q0.w, q1.x, q1.y, mult, my_row + 5 * kChunk);
+          bad |= encode_three<BF16, true>(ladder, q0.w, q1.x, q1.y, mult, my_row);
         } else {
-          bad |= ladder ? encode_one<true, BF16>(q0.z, mult, my_row + 5 * kChunk) : encode_one<false, BF16>(q0.z, mult, my_row + 5 * kChunk);
+          bad |= ladder ? encode_one<true, BF16, true>(q0.z, mult, my_row) : encode_one<false, BF16, true>(q0.z, mult, my_row);
           direction_landed();
         }
       }
@@ -596,6 +613,7 @@ __global__ void __launch_bounds__(kMiniRows, MiniNet<H>::kCtas) k_mlp_tc_mini(
     const uint32_t v = lane < 8 ? kOnes2<BF16> : 0u;
     *reinterpret_cast<uint4*>(smem + M::kOffConst + lane * 16) = make_uint4(v, v, v, v);
   }
+  *reinterpret_cast<uint4*>(s_a1 + kBiasChunk * kMiniChunk + lane * 16) = make_uint4(kOnes2<BF16>, kOnes2<BF16>, kOnes2<BF16>, kOnes2<BF16>);
   fence_async_smem();
   tc_fence_before();
   __syncwarp();
@@ -639,8 +657,8 @@ __global__ void __launch_bounds__(kMiniRows, MiniNet<H>::kCtas) k_mlp_tc_mini(
   bool bad = false, ok = true;
   float4 q0, q1;
   load_rec(wk, q0, q1);
-  bad |= encode_three<BF16, kMiniChunk>(ladder, q0.x, q0.y, q0.z, mult, my_row);
-  bad |= encode_three<BF16, kMiniChunk>(ladder, q0.w, q1.x, q1.y, mult, my_row + 5 * kMiniChunk);
+  bad |= encode_three<BF16, false, kMiniChunk>(ladder, q0.x, q0.y, q0.z, mult, my_row);
+  bad |= encode_three<BF16, true, kMiniChunk>(ladder, q0.w, q1.x, q1.y, mult, my_row);
   float decay_c = q1.z;
   uint32_t slot_c = __float_as_uint(q1.w);
   load_rec(wk_n, q0, q1);
@@ -699,7 +717,7 @@ __global__ void __launch_bounds__(kMiniRows, MiniNet<H>::kCtas) k_mlp_tc_mini(
     }
     __syncwarp();
     // first part of the next item's encoding while layer 2 runs (the layer-1 tile is free)
-    if (has_next) bad |= encode_three<BF16, kMiniChunk>(ladder, q0.x, q0.y, q0.z, mult, my_row);
+    if (has_next) bad |= encode_three<BF16, false, kMiniChunk>(ladder, q0.x, q0.y, q0.z, mult, my_row);
     ok = __all_sync(0xffffffffu, mbar_wait(bar_m, ph++ & 1u) && ok);
     tc_fence_after();
     if (!ok) break;
@@ -727,7 +745,7 @@ __global__ void __launch_bounds__(kMiniRows, MiniNet<H>::kCtas) k_mlp_tc_mini(
       mma_commit(bar_m);
     }
     __syncwarp();
-    if (has_next) bad |= encode_three<BF16, kMiniChunk>(ladder, q0.w, q1.x, q1.y, mult, my_row + 5 * kMiniChunk);
+    if (has_next) bad |= encode_three<BF16, true, kMiniChunk>(ladder, q0.w, q1.x, q1.y, mult, my_row);
     ok = __all_sync(0xffffffffu, mbar_wait(bar_m, ph++ & 1u) && ok);
     tc_fence_after();
     if (!ok) break;
@@ -803,7 +821,7 @@ __device__ __forceinline__ void bias_terms(float b, uint16_t* dst /* [8] */, boo
 }
 
 // One CTA per primitive: its image is put together in shared memory and written in 16-byte pieces.  Bound: memory (13.8 KB
-// in, 8,960 bytes out at H = 32).  Two-byte stores straight to memory took 192 us for 20,000 primitives, this 133.
+// in, 8,960 bytes out at H = 32).  Two-byte stores straight to memory took 192 us for 20,000 primitives, this 103.
 constexpr int kPackThreads = 128;
 template <bool BF16, int H>
 __global__ void __launch_bounds__(kPackThreads) k_pack_weights(
@@ -836,10 +854,7 @@ __global__ void __launch_bounds__(kPackThreads) k_pack_weights(
   // the biases, a warp or two each
   for (int h = lane; h < H; h += 32) {
     if (warp == 0) {
-      uint16_t t[8];
-      bias_terms<BF16>(__ldg(b1 + p * H + h), t, bad);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) w1[(enc_k_of_bias(j) >> 3) * (H * 8) + h * 8 + (enc_k_of_bias(j) & 7)] = t[j];
+      bias_terms<BF16>(__ldg(b1 + p * H + h), w1 + kBiasChunk * (H * 8) + h * 8, bad);
     } else if (warp == 1) {
       bias_terms<BF16>(__ldg(b2 + p * H + h), w2 + (H / 8) * (H * 8) + h * 8, bad);
     }
