@@ -1408,7 +1408,11 @@ int launch_render_sorted(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scr
   // extra launch per wave costs more than the few remainders gain (measured: 250,000 primitives on 816,000 pixels
   // lose 4 % of evaluator time with the second list, 500,000 gain 2 %, 2,000,000 with 64 hidden units gain 21 %).  (Record export keeps one list.)
   const bool split_small = tc_path && !keep && (int64_t)n * 3 > P;
-  const bool table = tc_path && !keep && !split_small && s.dir_table && sc->num_freq == 6;
+  // Encoded ray directions from a table where a primitive owns many records: the table takes half of the special functions
+  // off the evaluator and adds 80 bytes per record to what it draws from L2.  With few records per weight image L2 is the
+  // scarcer of the two (evaluator without and with table: 100,000 primitives on 816,000 pixels 398 and 354 us, 60,000 on
+  // 305,000 220 and 214 us plus 6 for the table, 250,000 on 816,000 472 and 521 us).
+  const bool table = tc_path && !keep && (int64_t)n * 7 <= P && s.dir_table && sc->num_freq == 6;
   if (table) {
     const int rc_dir = launch_encode_directions(sc, fr, s.dir_table, st);
     if (rc_dir) return rc_dir;
