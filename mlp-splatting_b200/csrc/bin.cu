@@ -245,33 +245,42 @@ __global__ void __launch_bounds__(OWN ? 1024 : 256) k_bin_corners(const float4* 
 
 // One CTA turns the corner array into the tile offsets: prefix sums along the rows and then along the columns (in
 // shared memory) give the per-tile counts; their exclusive prefix in tile order is tile_offsets; the longest list,
-// the capacity check and the pair total of k_bin_finish ride along.
+// the capacity check and the pair total of k_bin_finish ride along.  Bound: latency of one CTA.  A warp takes a row at a
+// time, so that reads and writes of both memories follow one another (a run of tiles per thread had them 32 to a bank at
+// 1920 x 1080: 41 us, now OFFS_AFTER; 1200 x 680: 14 and OFFS2_AFTER).
+constexpr int kBinMaxRows = 1024;          // rows of tiles, one per thread
 __global__ void __launch_bounds__(1024) k_bin_offsets(const int32_t* __restrict__ diff, int ntx, int nty,
                                                       int32_t* __restrict__ tile_offsets, int capacity, int64_t max_pairs,
                                                       int32_t* __restrict__ status, int32_t* __restrict__ counters) {
   extern __shared__ int32_t s_cnt[];          // [(nty + 1)][(ntx + 1)]
+  __shared__ int s_row[kBinMaxRows];          // pairs of a row, then of the rows before it
   __shared__ int warp_sums[32];
   chain_wait();
   chain_release();
   const int sx = ntx + 1, T = ntx * nty, tid = threadIdx.x, lane = tid & 31;
-#pragma unroll 4
+#pragma unroll 8
   for (int i = tid; i < sx * (nty + 1); i += 1024) s_cnt[i] = diff[i];
   __syncthreads();
-  for (int y = tid >> 5; y < nty; y += 32) {          // a warp per row
+  // prefix of a row in place; returns its total
+  auto scan_row = [&](int32_t* row, bool exclusive, int& mx) {
     int acc = 0;
     for (int x0 = 0; x0 < ntx; x0 += 32) {
       const int x = x0 + lane;
-      int v = x < ntx ? s_cnt[y * sx + x] : 0;
+      const int own = x < ntx ? row[x] : 0;
+      int v = own;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const int u = __shfl_up_sync(0xffffffffu, v, o);
         if (lane >= o) v += u;
       }
-      v += acc;
-      acc = __shfl_sync(0xffffffffu, v, 31);
-      if (x < ntx) s_cnt[y * sx + x] = v;
+      if (x < ntx) row[x] = acc + v - (exclusive ? own : 0);
+      mx = max(mx, own);
+      acc += __shfl_sync(0xffffffffu, v, 31);
     }
-  }
+    return acc;
+  };
+  int mx = 0;
+  for (int y = tid >> 5; y < nty; y += 32) scan_row(s_cnt + y * sx, false, mx);
   __syncthreads();
   for (int x = tid; x < ntx; x += 1024) {             // a thread per column
     int acc = 0;
@@ -286,29 +295,22 @@ __global__ void __launch_bounds__(1024) k_bin_offsets(const int32_t* __restrict_
     for (; y < nty; ++y) { acc += s_cnt[y * sx + x]; s_cnt[y * sx + x] = acc; }
   }
   __syncthreads();
-  const int per = (T + 1023) / 1024;
-  const int b = min(T, tid * per), e = min(T, b + per);
-  int sum = 0, mx = 0;
-  int at = (b / ntx) * sx + b % ntx, col = b % ntx;   // a row of tiles is followed by one word of padding
-  for (int t = b; t < e; ++t) {
-    const int c = s_cnt[at];
-    sum += c;
-    mx = max(mx, c);
-    ++at;
-    if (++col == ntx) { col = 0; ++at; }
+  mx = 0;                                             // from here on: the longest list
+  for (int y = tid >> 5; y < nty; y += 32) {
+    const int sum = scan_row(s_cnt + y * sx, true, mx);
+    if (lane == 0) s_row[y] = sum;
   }
+  __syncthreads();
   int total;
-  int ex = block_exclusive_scan(sum, warp_sums, total);
-  at = (b / ntx) * sx + b % ntx;
-  col = b % ntx;
-  for (int t = b; t < e; ++t) {
-    tile_offsets[t] = ex;
-    ex += s_cnt[at];
-    ++at;
-    if (++col == ntx) { col = 0; ++at; }
+  const int before = block_exclusive_scan(tid < nty ? s_row[tid] : 0, warp_sums, total);
+  if (tid < nty) s_row[tid] = before;
+  __syncthreads();
+  for (int y = tid >> 5; y < nty; y += 32) {
+    const int base = s_row[y];
+    for (int x = lane; x < ntx; x += 32) tile_offsets[y * ntx + x] = base + s_cnt[y * sx + x];
   }
   mx = __reduce_max_sync(0xffffffffu, mx);
-  if ((tid & 31) == 0 && mx > 0) {
+  if (lane == 0 && mx > 0) {
     atomicMax(status + MLPSP_ST_MAX_TILE_LEN, mx);
     if (capacity > 0 && mx > capacity) atomicOr(status + MLPSP_ST_BITS, MLPSP_ST_TILE_CAPACITY);
   }
@@ -522,7 +524,8 @@ int launch_scan_i32(const int32_t* in, int64_t n, int32_t* blk, int32_t* out, cu
 constexpr int kSortCap = 2048;  // per-tile sort capacity (>= tile capacity 1536)
 
 bool bin_uses_corners(const mlpsp_frame* fr) {
-  return 4 * (size_t)((fr->width + fr->tile - 1) / fr->tile + 1) * ((fr->height + fr->tile - 1) / fr->tile + 1) <= 200 * 1024;
+  const int ntx = (fr->width + fr->tile - 1) / fr->tile, nty = (fr->height + fr->tile - 1) / fr->tile;
+  return nty <= kBinMaxRows && 4 * (size_t)(ntx + 1) * (nty + 1) <= 200 * 1024;
 }
 
 int launch_bin(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, cudaStream_t st, bool order_lists,
