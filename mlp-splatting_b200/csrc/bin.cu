@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(OWN ? 1024 : 256) k_bin_corners(const float4* 
 // shared memory) give the per-tile counts; their exclusive prefix in tile order is tile_offsets; the longest list,
 // the capacity check and the pair total of k_bin_finish ride along.  Bound: latency of one CTA.  A warp takes a row at a
 // time, so that reads and writes of both memories follow one another (a run of tiles per thread had them 32 to a bank at
-// 1920 x 1080: 41 us, now OFFS_AFTER; 1200 x 680: 14 and OFFS2_AFTER).
+// 1920 x 1080: 41 us, now 21; 1200 x 680: 14 and 11).
 constexpr int kBinMaxRows = 1024;          // rows of tiles, one per thread
 __global__ void __launch_bounds__(1024) k_bin_offsets(const int32_t* __restrict__ diff, int ntx, int nty,
                                                       int32_t* __restrict__ tile_offsets, int capacity, int64_t max_pairs,

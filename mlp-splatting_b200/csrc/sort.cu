@@ -1,48 +1,14 @@
 // Per-tile depth sort: key = t* of the tile-centre ray against each candidate
 // (scannet/cuda/np_tile_kernels.cu:483-518), stable ascending order (1914-1990).
 // Keys are positive floats (or the 1e30 sentinel), so their bit patterns order like the values and the
-// sort runs on the raw bits: a bitonic network over the 64-bit composite (key bits, tie-break); lists of up
-// to 256 candidates are sorted by one warp in registers (eight tiles per CTA), longer lists by a whole CTA in
-// shared memory.
+// sort runs on the raw bits of the 64-bit composite (key bits, tie-break): a bitonic network in registers over 32-bit
+// words that stand for the composites, whose order it then corrects (see cta_sort_composites).  Lists of up to 256
+// candidates are sorted by one warp (eight tiles per CTA), longer lists by a whole CTA.
 #include "frame.cuh"
 
 namespace mlpsp {
 
 constexpr int kSortCap = 2048;
-
-// ---- warp-level bitonic sort in shared memory: N (a power of two >= 32) elements per warp ----
-// Compare-exchange t of a stage works on elements i and i | j, where i is t with a zero bit inserted
-// at the position of j.  One __syncwarp per stage, no block barrier: eight tiles sort side by side
-// in one 256-thread CTA.
-template <typename T, int N, int THREADS = 32>
-__device__ __forceinline__ void warp_bitonic(T* buf) {
-  const int lane = threadIdx.x & (THREADS - 1);
-  constexpr int PER = (N / 2 + THREADS - 1) / THREADS;   // compare-exchanges per thread and stage
-#pragma unroll 1
-  for (int k = 2; k <= N; k <<= 1) {
-#pragma unroll 1
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      T a[PER], b[PER];
-      int ia[PER];
-      // all loads of the stage first, so their shared-memory latencies overlap
-#pragma unroll
-      for (int q = 0; q < PER; ++q) {
-        const int t = q * THREADS + lane;
-        ia[q] = ((t & ~(j - 1)) << 1) | (t & (j - 1));
-        if (N >= 2 * THREADS || t < N / 2) { a[q] = buf[ia[q]]; b[q] = buf[ia[q] | j]; }
-      }
-#pragma unroll
-      for (int q = 0; q < PER; ++q) {
-        const int t = q * THREADS + lane;
-        if (N >= 2 * THREADS || t < N / 2) {
-          const bool up = (ia[q] & k) == 0;
-          if (up ? (a[q] > b[q]) : (a[q] < b[q])) { buf[ia[q]] = b[q]; buf[ia[q] | j] = a[q]; }
-        }
-      }
-      if (THREADS == 32) __syncwarp(); else __syncthreads();
-    }
-  }
-}
 
 // Composite of one candidate: (depth key bits << 32) | tie-break.  FROM_SCATTER: the list comes straight
 // from the binning scatter in arbitrary order and holds distinct ids, so the id itself is the tie-break
@@ -87,6 +53,7 @@ __device__ __forceinline__ void write_sorted(const unsigned long long* buf, cons
 constexpr int kTilesPerCta = 8;
 constexpr int kWarpSortMax = 256;
 constexpr int kLongDraw = 4;
+constexpr int kFixPasses = 8;
 
 // ---- warp-level bitonic sort in registers: lane l holds the elements r * 32 + l, r < PER ----
 // A compare-exchange at distance j >= 32 pairs two registers of the same lane; at distance j < 32 it pairs the same
@@ -98,8 +65,11 @@ __device__ __forceinline__ unsigned long long shfl_xor_u64(unsigned long long v,
   return ((unsigned long long)hi << 32) | lo;
 }
 
-template <int PER>
-__device__ __forceinline__ void warp_bitonic_regs(unsigned long long (&v)[PER], int lane) {
+__device__ __forceinline__ unsigned long long shfl_xor_any(unsigned long long v, int j) { return shfl_xor_u64(v, j); }
+__device__ __forceinline__ uint32_t shfl_xor_any(uint32_t v, int j) { return __shfl_xor_sync(0xffffffffu, v, j); }
+
+template <int PER, typename T>
+__device__ __forceinline__ void warp_bitonic_regs(T (&v)[PER], int lane) {
   constexpr int N = PER * 32;
 #pragma unroll
   for (int k = 2; k <= N; k <<= 1) {
@@ -111,22 +81,18 @@ __device__ __forceinline__ void warp_bitonic_regs(unsigned long long (&v)[PER], 
         for (int r = 0; r < PER; ++r) {
           if ((r & jr) == 0) {
             const bool up = ((r * 32) & k) == 0;          // k >= 64 here: the lane bits do not reach it
-            const unsigned long long a = v[r], b = v[r | jr];
-            const bool swap = up ? (a > b) : (a < b);
-            v[r] = swap ? b : a;
-            v[r | jr] = swap ? a : b;
+            const T mn = min(v[r], v[r | jr]), mx = max(v[r], v[r | jr]);
+            v[r] = up ? mn : mx;
+            v[r | jr] = up ? mx : mn;
           }
         }
       } else {
 #pragma unroll
         for (int r = 0; r < PER; ++r) {
-          const unsigned long long a = v[r];
-          const unsigned long long b = shfl_xor_u64(a, j);
+          const T a = v[r], b = shfl_xor_any(a, j);
           const bool up = ((r * 32 + lane) & k) == 0;
           const bool lower = (lane & j) == 0;
-          const bool keep_min = lower == up;
-          const unsigned long long mn = a < b ? a : b, mx = a < b ? b : a;
-          v[r] = keep_min ? mn : mx;
+          v[r] = lower == up ? min(a, b) : max(a, b);
         }
       }
     }
@@ -136,15 +102,11 @@ __device__ __forceinline__ void warp_bitonic_regs(unsigned long long (&v)[PER], 
 // ---- CTA-level bitonic sort, PER elements per thread in registers: thread t holds the elements t * PER + r ----
 // Distances below PER stay inside a thread, distances below 32 * PER pair two lanes of a warp (shuffles); only the
 // remaining distances (6 of the 45 stages of a 512-element sort, 10 of 55 at 1,024) cross warps and go through
-// shared memory between two CTA barriers.  buf holds the elements on entry and, sorted, on return.
-template <int PER, int THREADS>
-__device__ __forceinline__ void cta_bitonic_hybrid(unsigned long long* buf) {
+// shared memory between two CTA barriers.  buf: N elements of shared memory that nobody else uses meanwhile.
+template <int PER, int THREADS, typename T>
+__device__ __forceinline__ void cta_bitonic_hybrid(T (&v)[PER], T* buf) {
   constexpr int N = PER * THREADS;
   const int tid = threadIdx.x;
-  unsigned long long v[PER];
-#pragma unroll
-  for (int r = 0; r < PER; ++r) v[r] = buf[tid * PER + r];
-  __syncthreads();
 #pragma unroll
   for (int k = 2; k <= N; k <<= 1) {
 #pragma unroll
@@ -154,22 +116,19 @@ __device__ __forceinline__ void cta_bitonic_hybrid(unsigned long long* buf) {
         for (int r = 0; r < PER; ++r) {
           if ((r & j) == 0) {
             const bool up = ((tid * PER + r) & k) == 0;
-            const unsigned long long a = v[r], b = v[r | j];
-            const bool swap = up ? (a > b) : (a < b);
-            v[r] = swap ? b : a;
-            v[r | j] = swap ? a : b;
+            const T mn = min(v[r], v[r | j]), mx = max(v[r], v[r | j]);
+            v[r] = up ? mn : mx;
+            v[r | j] = up ? mx : mn;
           }
         }
       } else if (j < 32 * PER) {
         const int jl = j / PER;
 #pragma unroll
         for (int r = 0; r < PER; ++r) {
-          const unsigned long long a = v[r];
-          const unsigned long long b = shfl_xor_u64(a, jl);
+          const T a = v[r], b = shfl_xor_any(a, jl);
           const bool up = ((tid * PER + r) & k) == 0;
           const bool keep_min = ((tid & jl) == 0) == up;
-          const unsigned long long mn = a < b ? a : b, mx = a < b ? b : a;
-          v[r] = keep_min ? mn : mx;
+          v[r] = keep_min ? min(a, b) : max(a, b);
         }
       } else {
 #pragma unroll
@@ -178,41 +137,130 @@ __device__ __forceinline__ void cta_bitonic_hybrid(unsigned long long* buf) {
 #pragma unroll
         for (int r = 0; r < PER; ++r) {
           const int e = tid * PER + r;
-          const unsigned long long a = v[r], b = buf[e ^ j];
+          const T a = v[r], b = buf[e ^ j];
           const bool keep_min = ((e & j) == 0) == ((e & k) == 0);
-          const unsigned long long mn = a < b ? a : b, mx = a < b ? b : a;
-          v[r] = keep_min ? mn : mx;
+          v[r] = keep_min ? min(a, b) : max(a, b);
         }
         __syncthreads();
       }
     }
   }
+}
+
+// The CTA sorts s_buf[0 .. len), len <= PER * THREADS, composites (key bits << 32 | tie-break).  The network runs on 32-bit
+// words -- the key's distance from the list's smallest, cut to 21 bits, and the element's place -- which costs a third of
+// the instructions of 64-bit ones; the composites then move once, and neighbours that the cut has left out of order are
+// exchanged.  Lists with long runs of equal keys (more than kFixPasses exchanges deep) fall back on the 64-bit network.
+// s_key: PER * THREADS words.  kmin, kmax: the list's smallest and largest key bits, sentinels apart.
+template <int PER, int THREADS>
+__device__ __forceinline__ void cta_sort_composites(unsigned long long* s_buf, uint32_t* s_key, int len, uint32_t kmin, uint32_t kmax) {
+  constexpr int N = PER * THREADS;
+  const int tid = threadIdx.x;
+  const uint32_t range = kmax >= kmin ? kmax - kmin : 0u;
+  const int cut = max(0, 11 - __clz((int)range));            // bits of the distance beyond 21
+  uint32_t v[PER];
 #pragma unroll
-  for (int r = 0; r < PER; ++r) buf[tid * PER + r] = v[r];
+  for (int r = 0; r < PER; ++r) {
+    const int e = tid * PER + r;
+    const uint32_t key = e < len ? (uint32_t)(s_buf[e] >> 32) : 0u;
+    v[r] = e < len ? (min((key - kmin) >> cut, 0x1fffffu) << 11) | (uint32_t)e : 0xffffffffu;
+  }
+  cta_bitonic_hybrid<PER, THREADS>(v, s_key);
+  unsigned long long c[PER];
+#pragma unroll
+  for (int r = 0; r < PER; ++r) c[r] = tid * PER + r < len ? s_buf[v[r] & 2047u] : ~0ull;
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < PER; ++r) s_buf[tid * PER + r] = c[r];
+  __syncthreads();
+  for (int pass = 0;; ++pass) {
+    bool wrong = false;
+    for (int e = tid; e < len - 1; e += THREADS) wrong = wrong || s_buf[e] > s_buf[e + 1];
+    if (!__syncthreads_or(wrong)) return;
+    if (pass == kFixPasses) break;
+    for (int parity = 0; parity < 2; ++parity) {
+      for (int e = 2 * tid + parity; e < len - 1; e += 2 * THREADS) {
+        const unsigned long long a = s_buf[e], b = s_buf[e + 1];
+        if (a > b) { s_buf[e] = b; s_buf[e + 1] = a; }
+      }
+      __syncthreads();
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < PER; ++r) c[r] = s_buf[tid * PER + r];
+  __syncthreads();
+  cta_bitonic_hybrid<PER, THREADS>(c, s_buf);
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < PER; ++r) s_buf[tid * PER + r] = c[r];
   __syncthreads();
 }
 
-// One tile's list (len <= PER * 32) sorted by one warp in registers and written out.
+// One tile's list (len <= PER * 32) sorted by one warp in registers and written out; buf: 256 composites of shared memory.
+// As cta_sort_composites, with 24 bits of the key's distance and a place of eight.
 template <int PER, bool FROM_SCATTER>
 __device__ __forceinline__ void sort_tile_in_registers(const float4* __restrict__ geom, int n, const int32_t* tile_prims,
                                                        int32_t* __restrict__ sorted_prims, float* __restrict__ keys_out,
-                                                       int s, int len, int span, V3 o, V3 d, int key_mode, int lane) {
-  unsigned long long v[PER];
+                                                       int s, int len, int span, V3 o, V3 d, int key_mode, int lane,
+                                                       unsigned long long* buf) {
+  unsigned long long c[PER];
+  uint32_t v[PER], kmin = 0xffffffffu, kmax = 0u;
 #pragma unroll
   for (int r = 0; r < PER; ++r) {
     const int e = r * 32 + lane;
-    v[r] = e < len ? make_composite<FROM_SCATTER>(geom, n, tile_prims[s + e], e, o, d, key_mode) : ~0ull;
+    c[r] = e < len ? make_composite<FROM_SCATTER>(geom, n, tile_prims[s + e], e, o, d, key_mode) : ~0ull;
+    if (e < len) {
+      buf[e] = c[r];
+      const uint32_t key = (uint32_t)(c[r] >> 32);
+      kmin = min(kmin, key);
+      if (key != __float_as_uint(MLPSP_SENTINEL_KEY)) kmax = max(kmax, key);
+    }
+  }
+  kmin = __reduce_min_sync(0xffffffffu, kmin);
+  kmax = __reduce_max_sync(0xffffffffu, kmax);
+  const int cut = max(0, 8 - __clz((int)(kmax >= kmin ? kmax - kmin : 0u)));
+#pragma unroll
+  for (int r = 0; r < PER; ++r) {
+    const int e = r * 32 + lane;
+    v[r] = e < len ? (min(((uint32_t)(c[r] >> 32) - kmin) >> cut, 0xffffffu) << 8) | (uint32_t)e : 0xffffffffu;
   }
   warp_bitonic_regs<PER>(v, lane);
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < PER; ++r) c[r] = r * 32 + lane < len ? buf[v[r] & 255u] : ~0ull;
+  for (int pass = 0;; ++pass) {
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < PER; ++r) if (r * 32 + lane < len) buf[r * 32 + lane] = c[r];
+    __syncwarp();
+    bool wrong = false;
+#pragma unroll
+    for (int r = 0; r < PER; ++r) if (r * 32 + lane + 1 < len) wrong = wrong || c[r] > buf[r * 32 + lane + 1];
+    if (!__any_sync(0xffffffffu, wrong)) break;
+    if (pass == kFixPasses) {
+      warp_bitonic_regs<PER>(c, lane);
+      break;
+    }
+    for (int parity = 0; parity < 2; ++parity) {
+      for (int e = 2 * lane + parity; e < len - 1; e += 64) {
+        const unsigned long long a = buf[e], b = buf[e + 1];
+        if (a > b) { buf[e] = b; buf[e + 1] = a; }
+      }
+      __syncwarp();
+    }
+#pragma unroll
+    for (int r = 0; r < PER; ++r) if (r * 32 + lane < len) c[r] = buf[r * 32 + lane];
+  }
 #pragma unroll
   for (int r = 0; r < PER; ++r) {
     const int e = r * 32 + lane;
     if (e < len) {
-      sorted_prims[s + e] = FROM_SCATTER ? (int32_t)(uint32_t)v[r] : tile_prims[s + (int)(uint32_t)v[r]];
-      if (keys_out) keys_out[s + e] = __uint_as_float((uint32_t)(v[r] >> 32));
+      sorted_prims[s + e] = FROM_SCATTER ? (int32_t)(uint32_t)c[r] : tile_prims[s + (int)(uint32_t)c[r]];
+      if (keys_out) keys_out[s + e] = __uint_as_float((uint32_t)(c[r] >> 32));
     }
   }
   for (int i = len + lane; i < span; i += 32) sorted_prims[s + i] = -1;
+  __syncwarp();
 }
 
 // end of k_sort_tiles: the grid may not complete before the grid it was launched behind has
@@ -228,6 +276,7 @@ __global__ void __launch_bounds__(256, 6) k_sort_tiles(
     const int32_t* __restrict__ tile_offsets, const int32_t* tile_prims, int W, int H, int ts, int ntx, int T, int cap,
     int32_t* __restrict__ sorted_prims, float* __restrict__ keys_out, int key_mode, int32_t* __restrict__ long_list,
     int32_t* __restrict__ long_count, const int32_t* __restrict__ list_len, int32_t* __restrict__ status) {
+  __shared__ unsigned long long s_buf[8][kWarpSortMax];
   // Launched behind k_sort_long as its programmatic dependent WITHOUT waiting for it here: the two kernels sort
   // disjoint tiles and run side by side.  What this kernel reads (the binned lists, the status word) was complete
   // before k_sort_long's CTAs got past their own wait, and none of this kernel's CTAs starts before all of them
@@ -254,15 +303,17 @@ __global__ void __launch_bounds__(256, 6) k_sort_tiles(
   const int cx = min(tx * ts + (ts >> 1), W - 1), cy = min(ty * ts + (ts >> 1), H - 1);
   const int64_t pc = (int64_t)cy * W + cx;
   const V3 o = load3(rays_o, pc), d = load3(rays_d, pc);
-  if (len <= 32) sort_tile_in_registers<1, IDSORT>(geom, n, tile_prims, sorted_prims, keys_out, s, len, span, o, d, key_mode, lane);
-  else if (len <= 64) sort_tile_in_registers<2, IDSORT>(geom, n, tile_prims, sorted_prims, keys_out, s, len, span, o, d, key_mode, lane);
-  else if (len <= 128) sort_tile_in_registers<4, IDSORT>(geom, n, tile_prims, sorted_prims, keys_out, s, len, span, o, d, key_mode, lane);
-  else sort_tile_in_registers<8, IDSORT>(geom, n, tile_prims, sorted_prims, keys_out, s, len, span, o, d, key_mode, lane);
+  if (len <= 32) sort_tile_in_registers<1, IDSORT>(geom, n, tile_prims, sorted_prims, keys_out, s, len, span, o, d, key_mode, lane, s_buf[threadIdx.x >> 5]);
+  else if (len <= 64) sort_tile_in_registers<2, IDSORT>(geom, n, tile_prims, sorted_prims, keys_out, s, len, span, o, d, key_mode, lane, s_buf[threadIdx.x >> 5]);
+  else if (len <= 128) sort_tile_in_registers<4, IDSORT>(geom, n, tile_prims, sorted_prims, keys_out, s, len, span, o, d, key_mode, lane, s_buf[threadIdx.x >> 5]);
+  else sort_tile_in_registers<8, IDSORT>(geom, n, tile_prims, sorted_prims, keys_out, s, len, span, o, d, key_mode, lane, s_buf[threadIdx.x >> 5]);
   }
 }
 
 // Long lists (more than kWarpSortMax candidates): one CTA per such tile, the same bitonic network with the elements in
-// the registers of the CTA's threads (cta_bitonic_hybrid).  Launched before k_sort_tiles, which runs beside it.
+// the registers of the CTA's threads.  Launched before k_sort_tiles, which runs beside it.  Bound: issue slots; with the
+// network on the 64-bit composites both kernels took 79 us on the 100k frame, 117 of a 500k view and 136 of a 1M one at
+// 1920 x 1080, now 55, 75 and 98.
 template <int THREADS, int CAP, bool IDSORT>
 __global__ void __launch_bounds__(THREADS) k_sort_long(
     const float* __restrict__ rays_o, const float* __restrict__ rays_d, const float4* __restrict__ geom, int n,
@@ -270,6 +321,9 @@ __global__ void __launch_bounds__(THREADS) k_sort_long(
     int32_t* __restrict__ sorted_prims, float* __restrict__ keys_out, int key_mode, int T,
     int32_t* __restrict__ cursor, const int32_t* __restrict__ list_len, const int32_t* __restrict__ status) {
   __shared__ __align__(16) unsigned long long s_buf[CAP];
+  __shared__ uint32_t s_key[CAP];
+  __shared__ uint2 s_range[THREADS / 32];
+  static_assert(CAP == 2048, "places of eleven bits");
   __shared__ int s_draw;
   __shared__ int4 s_list[kLongDraw];           // tile, start, span, length
   chain_wait();
@@ -305,13 +359,23 @@ __global__ void __launch_bounds__(THREADS) k_sort_long(
     const int cx = min(tx * ts + (ts >> 1), W - 1), cy = min(ty * ts + (ts >> 1), H - 1);
     const int64_t pc = (int64_t)cy * W + cx;
     const V3 o = load3(rays_o, pc), d = load3(rays_d, pc);
-    const int N = len <= CAP / 4 ? CAP / 4 : (len <= CAP / 2 ? CAP / 2 : CAP);
-    for (int i = threadIdx.x; i < N; i += THREADS)
-      s_buf[i] = (i < len) ? make_composite<IDSORT>(geom, n, tile_prims[s + i], i, o, d, key_mode) : ~0ull;
+    uint32_t kmin = 0xffffffffu, kmax = 0u;
+    for (int i = threadIdx.x; i < len; i += THREADS) {
+      const unsigned long long c = make_composite<IDSORT>(geom, n, tile_prims[s + i], i, o, d, key_mode);
+      s_buf[i] = c;
+      const uint32_t key = (uint32_t)(c >> 32);
+      kmin = min(kmin, key);
+      if (key != __float_as_uint(MLPSP_SENTINEL_KEY)) kmax = max(kmax, key);
+    }
+    kmin = __reduce_min_sync(0xffffffffu, kmin);
+    kmax = __reduce_max_sync(0xffffffffu, kmax);
+    if ((threadIdx.x & 31) == 0) s_range[threadIdx.x >> 5] = make_uint2(kmin, kmax);
     __syncthreads();
-    if (N == CAP / 4) cta_bitonic_hybrid<CAP / 4 / THREADS, THREADS>(s_buf);
-    else if (N == CAP / 2) cta_bitonic_hybrid<CAP / 2 / THREADS, THREADS>(s_buf);
-    else warp_bitonic<unsigned long long, CAP, THREADS>(s_buf);      // beyond 1,024 candidates: rare, in shared memory
+#pragma unroll
+    for (int w = 0; w < THREADS / 32; ++w) { kmin = min(kmin, s_range[w].x); kmax = max(kmax, s_range[w].y); }
+    if (len <= CAP / 4) cta_sort_composites<CAP / 4 / THREADS, THREADS>(s_buf, s_key, len, kmin, kmax);
+    else if (len <= CAP / 2) cta_sort_composites<CAP / 2 / THREADS, THREADS>(s_buf, s_key, len, kmin, kmax);
+    else cta_sort_composites<CAP / THREADS, THREADS>(s_buf, s_key, len, kmin, kmax);
     write_sorted<IDSORT>(s_buf, tile_prims, sorted_prims, keys_out, s, len, span, threadIdx.x, THREADS);
     __syncthreads();
     }
