@@ -570,10 +570,11 @@ int launch_bin(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, c
       MLPSP_CUDA_OK(cudaFuncSetAttribute(k_bin_offsets, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
       MLPSP_CUDA_OK(cudaFuncSetAttribute(k_bin_corners<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     }
-    // an atomic of a warp on scattered cells is 32 sector operations, one on a line of cells four: the arrays of the SMs
-    // cost sms * cells / 8 of them, the direct way 4 n; below twice as many the direct way's fuller grid wins
+    // an atomic of a warp on scattered cells is 32 sector operations, one on a line of cells four: the direct way costs 4 n
+    // of them, the arrays of the SMs sms * cells / 8; they win from about equal numbers on (100,000 primitives on 12,986
+    // cells: 20 us directly, 8 by arrays)
     const int sms = sm_count();
-    if (8 * (int64_t)n >= (int64_t)sms * (int64_t)(diff_bytes / 4) / 2)
+    if (n >= 8192 && 32 * (int64_t)n >= (int64_t)sms * (int64_t)(diff_bytes / 4))
       launch_chained(k_bin_corners<true>, dim3(sms), dim3(1024), diff_bytes, st, (const float4*)sc->geom, n, cam, mats, s.rect, s.tile_diff);
     else if (n > 0)
       launch_chained(k_bin_corners<false>, dim3((n + 255) / 256), dim3(256), 0, st, (const float4*)sc->geom, n, cam, mats, s.rect, s.tile_diff);
