@@ -31,32 +31,36 @@ namespace mlpsp {
 
 constexpr int kRows = kRowsPerItem;      // 128 = MMA M
 constexpr int kChunk = kRows * 16;       // bytes of one K chunk of an A tile: [128 rows][8 halves]
-constexpr int kN3 = 16;                  // 4 outputs padded to the smallest N
+constexpr int kN3 = 16, kOut = 4;        // the outputs, and the smallest N that holds them
 constexpr int kA1Chunks = 10;            // 72 encoded inputs and a constant chunk that meets the bias terms
 
 // ---- packed weight image (per primitive) and shared-memory plan for F = 6, hidden width H = 32 or 64 ----
 // piece 1: W1 as [10 chunks][H rows][8 halves]: K = 0..71 in the order of enc_k(), then the eight terms of b1[h];
 // piece 2: W2 as [H/8 + 1 chunks][H][8], the last one the terms of b2;
-// piece 3: W3 as [H/8 + 1 chunks][16][8] (rows 4..15 zero), the last one the terms of b3.
+// piece 3: W3 as [H/8 + 1 chunks][4][8], the last one the terms of b3.  The MMA has N = 16: its rows 4..7 are the next
+//          chunk's rows, its rows 8..15 rows 0..7 again (a row-group stride of zero); nobody looks at their columns.
+// With W3 padded to 16 rows an image took 8,960 / 21,760 bytes, and six small-group CTAs of 64-wide layers an SM's shared
+// memory; seven fit now (four views of a million primitives: that kernel 2.84 -> 2.64 ms).
 template <int H>
 struct Net {
   static_assert(H == 32 || H == 64, "hidden width of the tensor-core evaluator");
   static constexpr int kWChunk = H * 16;
-  static constexpr int kW3Chunk = kN3 * 16;
+  static constexpr int kW3Chunk = kOut * 16;
   static constexpr int kOffW1 = 0;
   static constexpr int kBytesW1 = kA1Chunks * kWChunk;
   static constexpr int kOffW2 = kOffW1 + kBytesW1;
   static constexpr int kBytesW2 = (H / 8 + 1) * kWChunk;
   static constexpr int kOffW3 = kOffW2 + kBytesW2;
   static constexpr int kBytesW3 = (H / 8 + 1) * kW3Chunk;
-  static constexpr int kWeightBytes = kOffW3 + kBytesW3;          // 8,960 (H = 32) / 21,760 (H = 64)
-  // shared memory: weight image | eight rows of ones, eight rows of zeros | layer-1 A tile | barriers.  The second chunk of a
-  // bias K step (layers 2 and 3) on the weight side is "whatever follows" (the next piece, or the ones / zeros after the
-  // image), always finite, and meets the zero rows on the A side.
-  static constexpr int kOffConst = kWeightBytes;
+  static constexpr int kWeightBytes = kOffW3 + kBytesW3;          // 8,000 (H = 32) / 20,032 (H = 64)
+  // shared memory: weight image | zeros | eight rows of ones, eight rows of zeros | layer-1 A tile | barriers.  The second chunk
+  // of a bias K step on the weight side is "whatever follows" (the next piece, or the zeros and constants after the image,
+  // kWChunk bytes from the start of W3 on), always finite, and meets the zero rows on the A side.
+  static constexpr int kOffConst = kOffW3 + (kBytesW3 + kW3Chunk > kWChunk ? (kBytesW3 + kW3Chunk + 127) / 128 * 128 : kWChunk);
+  static_assert(kOffConst % 128 == 0 && kOffConst >= kOffW3 + kWChunk && kOffConst >= kWeightBytes + kW3Chunk, "what the MMAs read behind the image");
   static constexpr int kOffA1 = kOffConst + 256;
   static constexpr int kOffBar = kOffA1 + kA1Chunks * kChunk;
-  static constexpr int kSmemBytes = kOffBar + 96;                  // 29,792 / 42,592
+  static constexpr int kSmemBytes = kOffBar + 96;                  // 29,024 / 41,312
   // tensor memory: D1 and, once it has been read, D2 | D3 | the hidden layers' operand (H / 2 columns, two elements each)
   static constexpr int kTmemCols = 2 * H;
   static constexpr int kD1 = 0, kD2 = 0, kD3 = H, kA2 = H + kN3;
@@ -275,6 +279,7 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
     const uint32_t v = tid < 8 ? kOnes2<BF16> : 0u;
     *reinterpret_cast<uint4*>(smem + N::kOffConst + tid * 16) = make_uint4(v, v, v, v);
   }
+  if (tid < (N::kOffConst - N::kWeightBytes) / 16) *reinterpret_cast<uint4*>(smem + N::kWeightBytes + tid * 16) = make_uint4(0u, 0u, 0u, 0u);
   // the constant chunk: ones, so that the bias rides in the last K step of layer 1; with KEEP zeros, and the bias a step of its
   // own as in layers 2 and 3 (the order of the sums decides saved ReLU signs of values next to zero)
   if (tid < kRows) {
@@ -296,7 +301,7 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
     const uint64_t a1_desc = smem_desc(a1, kChunk, 128);
     const uint64_t ones_desc = smem_desc(cst, 128, 0);     // rows of ones, then rows of zeros; every row group the same
     const uint64_t w1_desc = smem_desc(wb + N::kOffW1, N::kWChunk, 128), w2_desc = smem_desc(wb + N::kOffW2, N::kWChunk, 128);
-    const uint64_t w3_desc = smem_desc(wb + N::kOffW3, N::kW3Chunk, 128);
+    const uint64_t w3_desc = smem_desc(wb + N::kOffW3, N::kW3Chunk, 0);
     auto step = [](uint64_t desc, int bytes) { return desc + (uint64_t)(bytes >> 4); };
     auto request = [&](int piece, int prim) {
       const int off = piece == 0 ? N::kOffW1 : (piece == 1 ? N::kOffW2 : N::kOffW3);
@@ -563,7 +568,7 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
 // three idle ones through the same chain of MMA round trips, and only five of them fit an SM.  Here one warp IS
 // the CTA: the operand tiles hold 32 rows (chunk stride 512 bytes; the MMA still has M = 128 and reads, as rows
 // 32..127, whatever follows -- those accumulator rows are never looked at), the accumulators of the three layers
-// share 32 (H = 64: 64) columns of tensor memory, lane 0 issues the MMAs between __syncwarp()s, and 12 (6) such
+// share 32 (H = 64: 64) columns of tensor memory, lane 0 issues the MMAs between __syncwarp()s, and 12 (7) such
 // CTAs fit an SM.  Same weight pieces, same bias folding, same arithmetic as k_mlp_tc.
 constexpr int kMiniRows = kRowsPerSmallItem;
 constexpr int kMiniChunk = kMiniRows * 16;
@@ -571,14 +576,15 @@ constexpr int kMiniChunk = kMiniRows * 16;
 template <int H>
 struct MiniNet {
   using N = Net<H>;
-  static constexpr int kOffConst = N::kWeightBytes;
+  static constexpr int kOffConst = N::kOffConst;
   static constexpr int kOffA1 = kOffConst + 256;
   static constexpr int kOffA2 = kOffA1 + kA1Chunks * kMiniChunk;
-  static constexpr int kOffPad = kOffA2 + (H / 8) * kMiniChunk;     // rows 32..127 of the last hidden chunk land here
-  static constexpr int kOffBar = kOffPad + (kRows - kMiniRows) * 16;
-  static constexpr int kSmemBytes = kOffBar + 64;                   // 17,984 (H = 32) / 32,832 (H = 64)
+  static constexpr int kOffPad = kOffA2 + (H / 8) * kMiniChunk;     // rows 32..127 of the last hidden chunk land here (with the
+  static constexpr int kOffBar = kOffPad + (kRows - kMiniRows) * 16;  // weight image there instead an item takes 15 % longer)
+  static constexpr int kSmemBytes = kOffBar + 64;                   // 17,216 (H = 32) / 31,552 (H = 64)
   static constexpr int kTmemCols = H;
-  static constexpr int kCtas = H == 32 ? 12 : 6;
+  static constexpr int kCtas = H == 32 ? 12 : 7;
+  static_assert(kCtas * (kSmemBytes + 1024) <= 228 * 1024 && kCtas * kTmemCols <= 512, "resident CTAs");
 };
 
 template <bool BF16, int H>
@@ -613,6 +619,7 @@ __global__ void __launch_bounds__(kMiniRows, MiniNet<H>::kCtas) k_mlp_tc_mini(
     const uint32_t v = lane < 8 ? kOnes2<BF16> : 0u;
     *reinterpret_cast<uint4*>(smem + M::kOffConst + lane * 16) = make_uint4(v, v, v, v);
   }
+  if (lane < (N::kOffConst - N::kWeightBytes) / 16) *reinterpret_cast<uint4*>(smem + N::kWeightBytes + lane * 16) = make_uint4(0u, 0u, 0u, 0u);
   *reinterpret_cast<uint4*>(s_a1 + kBiasChunk * kMiniChunk + lane * 16) = make_uint4(kOnes2<BF16>, kOnes2<BF16>, kOnes2<BF16>, kOnes2<BF16>);
   fence_async_smem();
   tc_fence_before();
@@ -629,7 +636,7 @@ __global__ void __launch_bounds__(kMiniRows, MiniNet<H>::kCtas) k_mlp_tc_mini(
   const uint32_t idesc_h = instr_desc(kRows, H, BF16), idesc_o = instr_desc(kRows, kN3, BF16);
   const uint64_t a1_desc = smem_desc(a1, kMiniChunk, 128), a2_desc = smem_desc(a2, kMiniChunk, 128);
   const uint64_t w1_desc = smem_desc(wb + N::kOffW1, N::kWChunk, 128), w2_desc = smem_desc(wb + N::kOffW2, N::kWChunk, 128);
-  const uint64_t w3_desc = smem_desc(wb + N::kOffW3, N::kW3Chunk, 128);
+  const uint64_t w3_desc = smem_desc(wb + N::kOffW3, N::kW3Chunk, 0);
   auto step = [](uint64_t desc, int bytes) { return desc + (uint64_t)(bytes >> 4); };
   auto request = [&](int piece, int prim) {
     const int off = piece == 0 ? N::kOffW1 : (piece == 1 ? N::kOffW2 : N::kOffW3);
@@ -821,7 +828,7 @@ __device__ __forceinline__ void bias_terms(float b, uint16_t* dst /* [8] */, boo
 }
 
 // One CTA per primitive: its image is put together in shared memory and written in 16-byte pieces.  Bound: memory (13.8 KB
-// in, 8,960 bytes out at H = 32).  Two-byte stores straight to memory took 192 us for 20,000 primitives, this 103.
+// in, 8,000 bytes out at H = 32).  Two-byte stores straight to memory took 192 us for 20,000 primitives, this 103.
 constexpr int kPackThreads = 128;
 template <bool BF16, int H>
 __global__ void __launch_bounds__(kPackThreads) k_pack_weights(
@@ -847,9 +854,9 @@ __global__ void __launch_bounds__(kPackThreads) k_pack_weights(
     w2[(k >> 3) * (H * 8) + h * 8 + (k & 7)] = to_lp<BF16>(__ldg(W2 + p * (H * H) + i), bad);
   }
 #pragma unroll
-  for (int u = 0; u < kN3 * H / kPackThreads; ++u) {
+  for (int u = 0; u < kOut * H / kPackThreads; ++u) {
     const int i = u * kPackThreads + tid, h = i / H, k = i % H;
-    w3[(k >> 3) * (kN3 * 8) + h * 8 + (k & 7)] = h < 4 ? to_lp<BF16>(__ldg(W3 + p * (4 * H) + i), bad) : (uint16_t)0;
+    w3[(k >> 3) * (kOut * 8) + h * 8 + (k & 7)] = to_lp<BF16>(__ldg(W3 + p * (kOut * H) + i), bad);
   }
   // the biases, a warp or two each
   for (int h = lane; h < H; h += 32) {
@@ -859,11 +866,7 @@ __global__ void __launch_bounds__(kPackThreads) k_pack_weights(
       bias_terms<BF16>(__ldg(b2 + p * H + h), w2 + (H / 8) * (H * 8) + h * 8, bad);
     }
   }
-  if (warp == 2 && lane < kN3) {
-    uint16_t* row = w3 + (H / 8) * (kN3 * 8) + lane * 8;
-    if (lane < 4) bias_terms<BF16>(__ldg(b3 + p * 4 + lane), row, bad);
-    else for (int j = 0; j < 8; ++j) row[j] = 0;
-  }
+  if (warp == 2 && lane < kOut) bias_terms<BF16>(__ldg(b3 + p * kOut + lane), w3 + (H / 8) * (kOut * 8) + lane * 8, bad);
   __syncthreads();
   uint4* dst = reinterpret_cast<uint4*>(out + p * N::kWeightBytes);
   for (int i = tid; i < N::kWeightBytes / 16; i += kPackThreads) dst[i] = reinterpret_cast<const uint4*>(img)[i];
@@ -920,7 +923,7 @@ static int launch_tc(const mlpsp_scene* sc, const char* image, const char* dir_t
   }
   if (rc) return rc;
   if (work_small && !rec_ext) {
-    // the wave's small groups (at most 32 records) on their own kernel: one warp per item, twelve (six) items per SM
+    // the wave's small groups (at most 32 records) on their own kernel: one warp per item, twelve (seven) items per SM
     int grid_s = sms * MiniNet<H>::kCtas;
     if (grid_cap > 0) grid_s = std::min(grid_s, grid_cap);
     rc = bf16 ? launch_mini<true, H>(image, sc, rec_in, work_small, counters, rec_out, out_mode, status, st, grid_s)

@@ -762,7 +762,7 @@ class ViewBatchRenderer:
     """Several views of one scene per call (mlpsp_render_frames): one evaluator launch per wave serves all views.
 
     The reference renders view by view.  In a scene with many primitives a primitive owns only a few records per
-    view, and the evaluator then spends its time streaming weight images (9.0 or 21.8 KB per primitive, wave and
+    view, and the evaluator then spends its time streaming weight images (8.0 or 20.0 KB per primitive, wave and
     view); rendering a batch of views together lets a primitive's records of all views share one fetch.  Every
     view keeps its own tile lists, masks, pixel state and outputs (a FrameRenderer each); the per-primitive arrays
     and the record arrays are the first view's, sized for the whole batch.  rgb and alpha only; images are
