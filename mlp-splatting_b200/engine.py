@@ -651,14 +651,31 @@ class FrameRenderer:
         """Render and return the reference's record list [rgb, alpha, ids, x6, raw, masks, gates, offsets]
         (render_tiles_training_records, np_tile_kernels.cu:6897-6986): pixel-major, compositing order."""
         lib, d = self.lib, self.device
-        rgb, alpha = self.render(scene, rays_o, rays_d, threshold, keep_records=True, **kw)
-        f, _ = self._last_frame
+        checked = kw.pop("check", True)
+        total, worst = C.c_int64(0), C.c_int32(0)
+
+        def count(offsets, st):
+            f, _ = self._last_frame
+            L.check(lib.mlpsp_export_records(C.byref(scene.c), C.byref(f), L.ptr(offsets), None, None, None, None, None, 0,
+                                             int(max_hits), C.byref(total), C.byref(worst), st), "mlpsp_export_records")
+            return f
+
+        # The host waits once for the frame and the count of its records: the status word travels between the two.  A frame
+        # that reports anything is rendered again by the path that looks at the status first.
+        rgb, alpha = self.render(scene, rays_o, rays_d, threshold, keep_records=True, check=False, **kw)
         with torch.cuda.device(d):
             st = _stream_ptr(d)
             offsets = torch.empty(self.P + 1, device=d, dtype=torch.int64)
-            total, worst = C.c_int64(0), C.c_int32(0)
-            L.check(lib.mlpsp_export_records(C.byref(scene.c), C.byref(f), L.ptr(offsets), None, None, None, None, None, 0,
-                                             int(max_hits), C.byref(total), C.byref(worst), st), "mlpsp_export_records")
+            if checked:
+                self.status_host.copy_(self.status, non_blocking=True)
+            f = count(offsets, st)
+            if checked:
+                self._stats = self._status_np.copy()
+                if int(self._status_np[L.ST_BITS]):
+                    rgb, alpha = self.render(scene, rays_o, rays_d, threshold, keep_records=True, **kw)
+                    f = count(offsets, st)
+                elif kw.get("waves") is None and kw.get("sort_key", 0) != L.ORDER_PER_PIXEL:
+                    self._adapt_waves(int(self._status_np[L.ST_WAVES]))
             if worst.value < 0:
                 raise RenderError(f"render_tiles_training_records: tile-center backward hit capacity {max_hits} reached "
                                   "before transmittance termination; refusing to return truncated records")

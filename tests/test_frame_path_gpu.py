@@ -229,3 +229,16 @@ def test_export_lists_and_direct_rows_agree(per_tile):
     torch.testing.assert_close(before.float(), raw[:, 4], rtol=1e-4, atol=1e-6)
     if per_tile == 700:
         assert int((offsets[1:] - offsets[:-1]).max()) > 40
+
+
+def test_record_frame_that_outgrows_its_scratch():
+    """The count of a frame's records is launched before its status is known; an overflow renders and counts again."""
+    from mlp_splatting_b200.engine import FrameRenderer
+    scene, cam = small_case(W=61, H=43)
+    ps, got = _packed(scene, pack_f16=False), []
+    for most in (16_000_000, 1000):
+        r = FrameRenderer(61, 43, device=DEV, max_records=most)
+        got.append(r.render_records(ps, _t(cam["rays_o"]), _t(cam["rays_d"]), THR, view=cam["view"], proj=cam["proj"], precision=0))
+    assert r.max_records > 1000 and len(got[0][2]) > 1000
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
