@@ -1624,78 +1624,66 @@ int launch_render_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scr
 // ----------------------------------------------------------------------- record export ----
 // Pixel-major records in compositing order (np_tile_kernels.cu:3138-3154; training_wmma.cuh:223-256),
 // rebuilt after the frame from the consumed masks, the evaluator outputs kept per compositing slot
-// and a recomputed hit test.  Two passes like the reference: count per pixel, prefix, emit.  A pixel's lane walks the pairs
-// it consumed (the masks of 32 pairs transposed) and lists its records in output order; the warp then writes the list, 32
-// records at a time, whose rows follow one another in memory (a row of the tile is one run).  More than kExportList records
-// of 32 pixels are written during the walk.  Bound: the stores' sectors.  A walk over the pairs that any pixel of the warp
-// consumed took 218 us for 0.7 M records (320 x 240), each pixel's own walk with its stores 152, this 123.
-constexpr int kExportList = 1024;
-struct ExportSmem { uint32_t slot[kExportList]; int32_t prim[kExportList]; uint8_t lane[kExportList]; int pix[32]; int64_t out[32]; };
+// and a recomputed hit test.  Like the reference: count per pixel, prefix, emit.  A pixel's lane walks the pairs it consumed (the
+// masks of 32 pairs transposed); in the emitting walk it leaves each record's slot and pixel in the record's own row, and a
+// thread per record then makes the row of it, so that the walk's uneven tiles carry no arithmetic and rows are written whole.
+// (Without ids and rows of the records to leave them in, the walk emits.)  Bound: the latency of the walk's and the rows'
+// gathers; 0.7 M records (320 x 240): a walk over the pairs that any pixel of a warp consumed, emitting, took 218 us, each
+// pixel's own walk 152, with the records of a warp listed first 115, this 58.
+struct ExportArgs {
+  const float* rays_o; const float* rays_d; const float4* geom;
+  const int32_t* tile_offsets; const int32_t* tile_len; const int32_t* sorted_prims; int W, H, ntx; float thr, beta, tau;
+  const uint32_t* used32; const uint32_t* masks32; const uint32_t* pair_base; const float4* rec_out; const float4* rec_ext; const float* rec_tr;
+  const float4* px_state; int32_t* px_cnt; const int32_t* px_off; int max_hits; int32_t* worst;
+  int32_t* ids; float* x6; float* raw; int32_t* relu_masks; float* gates; int64_t max_out; int ref_arith, vec, place; const int32_t* status;
+};
+
+// one record: slot of its evaluation, primitive, pixel, place in the output
+__device__ __forceinline__ void export_row(const ExportArgs& a, uint32_t slot, int p, int pix, int64_t r) {
+  const float4 ro = __ldg(a.rec_out + slot), re = __ldg(a.rec_ext + slot);
+  const float tr = a.raw ? __ldg(a.rec_tr + slot) : 0.f;
+  const V3 o = load3(a.rays_o, pix), d = load3(a.rays_d, pix);
+  Hit h;
+  if (a.ref_arith) hit_test_ref(load_geom_ref(a.geom, p), o, d, a.thr, h);
+  else hit_test(load_geom(a.geom, p), o, d, a.thr, h);
+  if (a.ids && !a.place) a.ids[r] = p;
+  if (a.x6) {
+    if (a.vec) {
+      float2* q = reinterpret_cast<float2*>(a.x6) + r * 3;
+      q[0] = make_float2(d.x, d.y); q[1] = make_float2(d.z, h.dx); q[2] = make_float2(h.dy, h.dz);
+    } else {
+      float* q = a.x6 + r * 6; q[0] = d.x; q[1] = d.y; q[2] = d.z; q[3] = h.dx; q[4] = h.dy; q[5] = h.dz;
+    }
+  }
+  if (a.raw) {
+    if (a.vec) {
+      float4* q = reinterpret_cast<float4*>(a.raw) + r * 2;
+      q[0] = make_float4(ro.x, ro.y, ro.z, re.x); q[1] = make_float4(tr, ro.w, h.decay, re.y);
+    } else {
+      float* q = a.raw + r * 8;
+      q[0] = ro.x; q[1] = ro.y; q[2] = ro.z; q[3] = re.x; q[4] = tr; q[5] = ro.w; q[6] = h.decay; q[7] = re.y;
+    }
+  }
+  if (a.relu_masks) {
+    const int2 m = make_int2((int32_t)__float_as_uint(re.z), (int32_t)__float_as_uint(re.w));
+    if (a.vec) reinterpret_cast<int2*>(a.relu_masks)[r] = m;
+    else { a.relu_masks[r * 2] = m.x; a.relu_masks[r * 2 + 1] = m.y; }
+  }
+  if (a.gates) {
+    const float4 g = tetra_gates(h, gate_scales(__ldg(a.geom + (size_t)p * 4 + 3), a.beta), a.tau);
+    if (a.vec) reinterpret_cast<float4*>(a.gates)[r] = g;
+    else { float* q = a.gates + r * 4; q[0] = g.x; q[1] = g.y; q[2] = g.z; q[3] = g.w; }
+  }
+}
 
 template <bool EMIT>
-__global__ void __launch_bounds__(64) k_export(
-    const float* __restrict__ rays_o, const float* __restrict__ rays_d, const float4* __restrict__ geom,
-    const int32_t* __restrict__ tile_offsets, const int32_t* __restrict__ tile_len, const int32_t* __restrict__ sorted_prims, int W, int H, int ntx,
-    float thr, float beta, float tau, const uint32_t* __restrict__ used32, const uint32_t* __restrict__ masks32,
-    const uint32_t* __restrict__ pair_base, const float4* __restrict__ rec_out, const float4* __restrict__ rec_ext,
-    const float* __restrict__ rec_tr, const float4* __restrict__ px_state, int32_t* __restrict__ px_cnt,
-    const int32_t* __restrict__ px_off, int max_hits, int32_t* __restrict__ worst, int32_t* __restrict__ ids,
-    float* __restrict__ x6, float* __restrict__ raw, int32_t* __restrict__ relu_masks, float* __restrict__ gates,
-    int64_t max_out, int ref_arith, int vec, const int32_t* __restrict__ status) {
-  __shared__ ExportSmem s_all[EMIT ? 2 : 1];
-  if (status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
+__global__ void __launch_bounds__(64) k_export(const ExportArgs a) {
+  if (a.status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
   const int tile = blockIdx.x;
-  const int s = tile_offsets[tile], e = s + tile_len[tile];
+  const int s = a.tile_offsets[tile], e = s + a.tile_len[tile];
   const int lane = threadIdx.x & 31, half = threadIdx.x >> 5;
-  ExportSmem& sm = s_all[EMIT ? half : 0];
-  const TilePix tp = tile_pixel(tile, half * 32 + lane, ntx, W, H);
-  int64_t out0 = 0;
-  int own = 0, first_entry = 0, total = 0;            // records of this lane's pixel, their place among the warp's
-  if (EMIT) {
-    if (tp.valid) { out0 = px_off[tp.pix]; own = px_off[tp.pix + 1] - (int)out0; }
-    const int inc = warp_inclusive_scan(own);
-    first_entry = inc - own;
-    total = __shfl_sync(0xffffffffu, inc, 31);
-  }
-  // one record: slot of its evaluation, primitive, pixel, place in the output
-  auto emit = [&](uint32_t slot, int p, int pix, int64_t r) {
-    if (r >= max_out) return;
-    const float4 ro = rec_out[slot], re = rec_ext[slot];
-    const float tr = raw ? rec_tr[slot] : 0.f;
-    const V3 o = load3(rays_o, pix), d = load3(rays_d, pix);
-    Hit h;
-    if (ref_arith) hit_test_ref(load_geom_ref(geom, p), o, d, thr, h);
-    else hit_test(load_geom(geom, p), o, d, thr, h);
-    if (ids) ids[r] = p;
-    if (x6) {
-      if (vec) {
-        float2* q = reinterpret_cast<float2*>(x6) + r * 3;
-        q[0] = make_float2(d.x, d.y); q[1] = make_float2(d.z, h.dx); q[2] = make_float2(h.dy, h.dz);
-      } else {
-        float* q = x6 + r * 6; q[0] = d.x; q[1] = d.y; q[2] = d.z; q[3] = h.dx; q[4] = h.dy; q[5] = h.dz;
-      }
-    }
-    if (raw) {
-      if (vec) {
-        float4* q = reinterpret_cast<float4*>(raw) + r * 2;
-        q[0] = make_float4(ro.x, ro.y, ro.z, re.x); q[1] = make_float4(tr, ro.w, h.decay, re.y);
-      } else {
-        float* q = raw + r * 8;
-        q[0] = ro.x; q[1] = ro.y; q[2] = ro.z; q[3] = re.x; q[4] = tr; q[5] = ro.w; q[6] = h.decay; q[7] = re.y;
-      }
-    }
-    if (relu_masks) {
-      const int2 m = make_int2((int32_t)__float_as_uint(re.z), (int32_t)__float_as_uint(re.w));
-      if (vec) reinterpret_cast<int2*>(relu_masks)[r] = m;
-      else { relu_masks[r * 2] = m.x; relu_masks[r * 2 + 1] = m.y; }
-    }
-    if (gates) {
-      const float4 g = tetra_gates(h, gate_scales(__ldg(geom + (size_t)p * 4 + 3), beta), tau);
-      if (vec) reinterpret_cast<float4*>(gates)[r] = g;
-      else { float* q = gates + r * 4; q[0] = g.x; q[1] = g.y; q[2] = g.z; q[3] = g.w; }
-    }
-  };
-  const bool listed = EMIT && total <= kExportList;
+  const TilePix tp = tile_pixel(tile, half * 32 + lane, a.ntx, a.W, a.H);
+  const int64_t out0 = EMIT && tp.valid ? a.px_off[tp.pix] : 0;
   const uint32_t lt = (1u << lane) - 1u;
   int cnt = 0;
   for (int i0 = s; i0 < e; i0 += 32) {
@@ -1703,13 +1691,13 @@ __global__ void __launch_bounds__(64) k_export(
     uint32_t mine = 0u, hitm = 0u, first = 0u;       // pair idx: this half's consumed and hit pixels, the slot of its first record
     int prim = 0;
     if (idx < e) {
-      const uint2 uu = *reinterpret_cast<const uint2*>(used32 + 2 * (size_t)idx);
+      const uint2 uu = *reinterpret_cast<const uint2*>(a.used32 + 2 * (size_t)idx);
       mine = half ? uu.y : uu.x;
       if (EMIT && mine) {
-        const uint2 mm = *reinterpret_cast<const uint2*>(masks32 + 2 * (size_t)idx);
+        const uint2 mm = *reinterpret_cast<const uint2*>(a.masks32 + 2 * (size_t)idx);
         hitm = half ? mm.y : mm.x;
-        first = pair_base[idx] + (half ? __popc(mm.x) : 0);
-        prim = sorted_prims[idx];
+        first = a.pair_base[idx] + (half ? __popc(mm.x) : 0);
+        prim = a.sorted_prims[idx];
       }
     }
     if (!__any_sync(0xffffffffu, mine != 0u)) continue;
@@ -1725,29 +1713,31 @@ __global__ void __launch_bounds__(64) k_export(
       if (!todo) continue;
       todo &= todo - 1u;
       const uint32_t slot = fj + __popc(hj & lt);
-      const int k = cnt++;
-      if (listed) {
-        if (k < own) { sm.slot[first_entry + k] = slot; sm.prim[first_entry + k] = p; sm.lane[first_entry + k] = (uint8_t)lane; }
+      const int64_t r = out0 + cnt++;
+      if (r >= a.max_out) continue;
+      if (a.place) {
+        a.ids[r] = p;
+        *reinterpret_cast<int2*>(a.raw + r * 8) = make_int2((int)slot, tp.pix);
       } else {
-        emit(slot, p, tp.pix, out0 + k);
+        export_row(a, slot, p, tp.pix, r);
       }
     }
   }
-  if (listed) {
-    sm.pix[lane] = tp.valid ? tp.pix : 0;
-    sm.out[lane] = out0 - first_entry;
-    __syncwarp();
-    for (int k = lane; k < total; k += 32) {
-      const int l = sm.lane[k];
-      emit(sm.slot[k], sm.prim[k], sm.pix[l], sm.out[l] + k);
-    }
-  }
   if (!EMIT && tp.valid) {
-    px_cnt[tp.pix] = cnt;
-    atomicMax(worst, cnt);
-    const bool live = px_state[tp.pix].w >= MLPSP_TERM;
-    if (max_hits > 0 && cnt >= max_hits && (cnt > max_hits || live)) atomicOr(worst + 1, 1);
+    a.px_cnt[tp.pix] = cnt;
+    atomicMax(a.worst, cnt);
+    const bool live = a.px_state[tp.pix].w >= MLPSP_TERM;
+    if (a.max_hits > 0 && cnt >= a.max_hits && (cnt > a.max_hits || live)) atomicOr(a.worst + 1, 1);
   }
+}
+
+// the rows of the records that k_export has placed
+__global__ void __launch_bounds__(256) k_export_rows(const ExportArgs a, int64_t total) {
+  if (a.status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
+  const int64_t r = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (r >= total) return;
+  const int2 at = *reinterpret_cast<const int2*>(a.raw + r * 8);
+  export_row(a, (uint32_t)at.x, a.ids[r], at.y, r);
 }
 
 __global__ void k_widen_i32(const int32_t* __restrict__ in, int64_t n, int64_t* __restrict__ out) {
@@ -1763,6 +1753,11 @@ int launch_export_records(const mlpsp_scene* sc, const mlpsp_frame* fr, const Sc
   int32_t* worst = s.counters + kCtrScratch;     // [0] largest per-pixel count, [1] capacity flag
   const bool outputs = ids || x6 || raw || relu_masks || gates;
   int64_t total = max_out;                       // counted: the caller holds this frame's total
+  const int vec = (reinterpret_cast<uintptr_t>(x6) & 7) == 0 && (reinterpret_cast<uintptr_t>(relu_masks) & 7) == 0 &&
+                  ((reinterpret_cast<uintptr_t>(raw) | reinterpret_cast<uintptr_t>(gates)) & 15) == 0;
+  ExportArgs a = {fr->rays_o, fr->rays_d, (const float4*)sc->geom, fr->tile_offsets, s.tile_len, fr->sorted_prims, W, H, ntx, fr->threshold,
+                  sc->gate_beta, sc->gate_tau, s.used32, s.masks32, s.pair_base, s.rec_out, s.rec_ext, s.rec_tr, s.px_state, s.px_cnt, s.px_off,
+                  max_hits, worst, ids, x6, raw, relu_masks, gates, max_out, fr->hit_arith == 1 ? 1 : 0, vec, 0, fr->status};
   if (!counted) {
     LaunchScope scope(kKMisc, 2 + scan_launches(P), st);
     HostWords& hw = host_words();
@@ -1770,10 +1765,7 @@ int launch_export_records(const mlpsp_scene* sc, const mlpsp_frame* fr, const Sc
     int rc = hw.open(&ev);
     if (rc) return rc;
     MLPSP_CUDA_OK(cudaMemsetAsync(worst, 0, 8, st));
-    k_export<false><<<T, 64, 0, st>>>(fr->rays_o, fr->rays_d, (const float4*)sc->geom, fr->tile_offsets, s.tile_len, fr->sorted_prims,
-                                      W, H, ntx, fr->threshold, sc->gate_beta, sc->gate_tau, s.used32, s.masks32,
-                                      s.pair_base, s.rec_out, s.rec_ext, s.rec_tr, s.px_state, s.px_cnt, nullptr, max_hits,
-                                      worst, nullptr, nullptr, nullptr, nullptr, nullptr, 0, fr->hit_arith == 1 ? 1 : 0, 0, fr->status);
+    k_export<false><<<T, 64, 0, st>>>(a);
     rc = launch_scan_i32(s.px_cnt, P, s.scan_blk, s.px_off, st);
     if (rc) return rc;
     k_widen_i32<<<(unsigned)((P + 1 + 255) / 256), 256, 0, st>>>(s.px_off, P + 1, offsets);
@@ -1787,13 +1779,10 @@ int launch_export_records(const mlpsp_scene* sc, const mlpsp_frame* fr, const Sc
     if (worst_host) *worst_host = h[2] ? -h[1] : h[1];
   }
   if (outputs && max_out >= total && total > 0) {
-    LaunchScope scope(kKMisc, 1, st);
-    const int vec = (reinterpret_cast<uintptr_t>(x6) & 7) == 0 && (reinterpret_cast<uintptr_t>(relu_masks) & 7) == 0 &&
-                    ((reinterpret_cast<uintptr_t>(raw) | reinterpret_cast<uintptr_t>(gates)) & 15) == 0;
-    k_export<true><<<T, 64, 0, st>>>(fr->rays_o, fr->rays_d, (const float4*)sc->geom, fr->tile_offsets, s.tile_len, fr->sorted_prims,
-                                     W, H, ntx, fr->threshold, sc->gate_beta, sc->gate_tau, s.used32, s.masks32,
-                                     s.pair_base, s.rec_out, s.rec_ext, s.rec_tr, s.px_state, s.px_cnt, s.px_off, max_hits,
-                                     worst, ids, x6, raw, relu_masks, gates, max_out, fr->hit_arith == 1 ? 1 : 0, vec, fr->status);
+    a.place = ids && raw && vec ? 1 : 0;
+    LaunchScope scope(kKMisc, a.place ? 2 : 1, st);
+    k_export<true><<<T, 64, 0, st>>>(a);
+    if (a.place) k_export_rows<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(a, total);
   }
   return cuda_check(cudaGetLastError(), "export_records");
 }

@@ -207,8 +207,8 @@ def test_feature_channels_per_cta(case, slots, C):
 
 
 @pytest.mark.parametrize("per_tile", [1, 31, 33, 700])
-def test_export_lists_and_direct_rows_agree(per_tile):
-    """Record export below and above the list of a warp (1,024 records of 32 pixels), against the composited image."""
+def test_exported_rows_compose_the_image(per_tile):
+    """Record export from one candidate to long runs per pixel, against the composited image and itself."""
     from mlp_splatting_b200.engine import FrameRenderer
     scene, cam = small_case(n=per_tile, W=16, H=11, mu=-1.8 if per_tile < 100 else -2.3, seed=per_tile)
     scene["b3"] = scene["b3"].copy()
