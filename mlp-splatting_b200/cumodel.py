@@ -23,7 +23,7 @@ import torch
 from torch import nn
 
 from . import _lib as L
-from .engine import FrameRenderer, PackedScene
+from .engine import FrameRenderer, PackedScene, RenderError
 
 
 def _tile_ext_build_config(tile_size=None):
@@ -428,8 +428,18 @@ def render_tiles_training_records(tensors, width, height, tile, threshold, beta,
                         device=dev, pack_f16=(precision == "float16"), _settle=False)
     r = FrameRenderer(int(width), int(height), device=dev, max_pairs=max(int(culled.numel()), 1),
                       tile_capacity=cfg["tile_candidate_capacity"])
-    scene._settle_pack()        # the weights have been packed while the buffers were made
-    prec = L.PRECISION_F16 if (precision == "float16" and scene.has_f16) else L.PRECISION_F32
-    return r.render_records(scene, ro.contiguous().float(), rd.contiguous().float(), float(threshold), max_hits=max_hits,
-                            precision=prec, tile_lists=(culled, offs), rays_normalized=True,
-                            path_name="render_tiles_training_records")
+    # the frame follows the packing of the weights without a wait between; both are known when its records are counted
+    good = scene._trust_pack()
+
+    def records():
+        prec = L.PRECISION_F16 if (precision == "float16" and scene.has_f16) else L.PRECISION_F32
+        return r.render_records(scene, ro.contiguous().float(), rd.contiguous().float(), float(threshold), max_hits=max_hits,
+                                precision=prec, tile_lists=(culled, offs), rays_normalized=True,
+                                path_name="render_tiles_training_records")
+    try:
+        out = records()
+    except RenderError:
+        if good():
+            raise
+        out = None
+    return out if out is not None and good() else records()

@@ -125,17 +125,35 @@ class PackedScene:
     def _settle_pack(self):
         """Reads the status of the binary16 packing (the constructor does, unless it was told to leave it to a caller that
         has other work to do meanwhile)."""
-        if self._packing is None:
-            return
-        w16, st = self._packing
-        self._packing = None
+        if self._packing is not None:
+            w16, st = self._packing
+            self._packing = None
+            self._take_pack(w16, int(st[L.ST_BITS].item()))
+
+    def _take_pack(self, w16, bits):
         # weights that are not finite in binary16 keep the scene on the FP32 evaluator, which is
         # what the reference's per-frame overflow check amounts to (rgb_wmma.cuh:162-176, 260-272)
-        if int(st[L.ST_BITS].item()) & L.BIT_NUMERIC:
-            self.f16_rejected = True
-        else:
-            self.w16 = w16
+        self.f16_rejected = bool(bits & L.BIT_NUMERIC)
+        self.w16 = None if self.f16_rejected else w16
         self.c = self._struct()
+
+    def _trust_pack(self):
+        """Uses the binary16 image before its status is known and has the status copied to the host: for a caller that
+        waits for the stream later on and then asks the function returned whether the image was good."""
+        if self._packing is None:
+            return lambda: True
+        w16, st = self._packing
+        self._packing = None
+        host = torch.empty(L.STATUS_WORDS, dtype=torch.int32, pin_memory=True)
+        host.copy_(st, non_blocking=True)
+        self._take_pack(w16, 0)
+
+        def good():
+            bits = int(host[L.ST_BITS])
+            if bits & L.BIT_NUMERIC:
+                self._take_pack(w16, bits)
+            return not self.f16_rejected
+        return good
 
     @classmethod
     def from_packed_image(cls, positions, log_scales, quats, freq, att, w16, hidden, feat_attr=None, gate_beta=1.5,

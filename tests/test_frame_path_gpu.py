@@ -242,3 +242,20 @@ def test_record_frame_that_outgrows_its_scratch():
     assert r.max_records > 1000 and len(got[0][2]) > 1000
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+def test_training_records_with_weights_beyond_binary16():
+    """The frame is launched before the status of the weight packing is known; weights that do not fit give the FP32 records."""
+    from mlp_splatting_b200.cumodel import render_tiles_training_records
+    from mlp_splatting_b200.engine import FrameRenderer, normalize_rows
+    scene, cam = small_case(W=61, H=43)
+    scene["W2"] = scene["W2"].copy()
+    scene["W2"][3, 5, 7] = 1.0e6
+    ps = _packed(scene, pack_f16=False)
+    culled, offs = FrameRenderer(61, 43, device=DEV).bin(ps, cam["view"], cam["proj"], THR)
+    tensors = [_t(cam["rays_o"]), normalize_rows(_t(cam["rays_d"])), ps.positions, ps.log_scales, ps.quats_unit, culled, offs,
+               ps.freq, ps.att] + [_t(scene[k]) for k in WKEYS]
+    half, full = (render_tiles_training_records(tensors, 61, 43, 8, THR, 1.5, 2.0, precision=p) for p in ("float16", "float32"))
+    assert len(half[2]) > 1000
+    for a, b in zip(half, full):
+        assert torch.equal(a, b)
