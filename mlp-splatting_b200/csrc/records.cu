@@ -366,124 +366,62 @@ __device__ __forceinline__ int warp_inclusive_scan(int v) {
   return v;
 }
 
-// Windows of up to 32 CH candidates: one warp per tile, nothing shared between warps.
-constexpr int kHitWarps = 4;
-template <bool REF, int CH>
-__global__ void __launch_bounds__(32 * kHitWarps) k_hits_warp(const HitArgs a) {
+// One warp per (tile, part of its window): every parts-th chunk of 32 candidates, nothing shared between warps; a chunk's
+// record slots are one reservation.  The later a wave, the wider its window and the fewer its tiles, so windows of up to
+// kHitParts chunks are cut into chunks and longer ones into kHitParts parts (LOOP; registers for the loop would cost the
+// others occupancy): a part prepares its tile's rays again, a tenth of a chunk's work.  A warp per tile for windows up to 128
+// and a CTA per tile beyond took 72 us of a 60k-primitive 639 x 477 frame and 1,454 of four 1M views at 1920 x 1080, this
+// 58 and 1,374.
+constexpr int kHitWarps = 4, kHitParts = 8;
+template <bool REF, bool LOOP>
+__global__ void __launch_bounds__(32 * kHitWarps) k_hits(const HitArgs a, int parts) {
   chain_wait();
   chain_release();
   __shared__ float4 s_q[kHitWarps][64];
   if (a.status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) reset_wave(a);
-  const int n_active = *a.active_count;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-  for (int slot_i = blockIdx.x * wpb + warp; slot_i < n_active; slot_i += gridDim.x * wpb) {
+  const int units = *a.active_count * parts;
+  for (int unit = blockIdx.x * wpb + warp; unit < units; unit += gridDim.x * wpb) {
+    const int slot_i = parts == 1 ? unit : unit / parts, part = unit - slot_i * parts;
     const int tile = a.active[slot_i];
     const int s = a.tile_offsets[tile], len = a.tile_len[tile];
     const int wlo = min(a.lo, len), nwin = min(a.hi, len) - wlo;
-    if (nwin <= 0) continue;
+    if (part * 32 >= nwin) continue;
     const HitPixels h = hit_pixels(a.rays_o, a.rays_d, a.px_state, tile, a.ntx, a.W, a.H, a.K > 0.f);
-    int p[CH], c[CH], total = 0;
-#pragma unroll
-    for (int ch = 0; ch < CH; ++ch) {
-      const int j = ch * 32 + lane;
-      p[ch] = j < nwin ? a.sorted_prims[s + wlo + j] : -1;
-      c[ch] = 0;
-      if (ch * 32 < nwin) {
-        uint32_t m0, m1;
-        hit_chunk<REF>(h, a.rays_o, a.rays_d, a.geom, a.n, p[ch], min(32, nwin - ch * 32), a.K, a.thr, a.bound2, s_q[warp], m0, m1);
-        if (j < nwin) a.masks[(size_t)(s + wlo) + j] = make_uint2(m0, m1);
-        c[ch] = __popc(m0) + __popc(m1);
-        total += c[ch];
-        if (c[ch] > 0) atomicAdd(a.prim_cnt + p[ch], c[ch]);
-      }
-    }
-    total = __reduce_add_sync(0xffffffffu, total);
-    int base = 0;
-    if (lane == 0 && total > 0) {
-      base = atomicAdd(a.counters + kCtrRecords, total);
-      if ((int64_t)base + total > a.max_records) atomicOr(a.status + MLPSP_ST_BITS, MLPSP_ST_RECORD_OVERFLOW);
-    }
-    base = __shfl_sync(0xffffffffu, base, 0);
-#pragma unroll
-    for (int ch = 0; ch < CH; ++ch) {
-      if (ch * 32 < nwin) {
-        const int inc = warp_inclusive_scan(c[ch]);
-        if (ch * 32 + lane < nwin) a.pair_base[(size_t)(s + wlo) + ch * 32 + lane] = (uint32_t)(base + inc - c[ch]);
-        base += __shfl_sync(0xffffffffu, inc, 31);
-      }
-    }
-  }
-}
-
-// Wider windows: eight warps per tile, each takes every eighth chunk of 32 candidates.
-template <bool REF>
-__global__ void __launch_bounds__(256) k_hits(const HitArgs a) {
-  chain_wait();
-  chain_release();
-  __shared__ float4 s_q[8][64];
-  __shared__ uint2 s_m[kWinMax];
-  __shared__ int warp_sums[32];
-  __shared__ int s_tile_base, s_total;
-  if (a.status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
-  if (blockIdx.x == 0 && threadIdx.x == 0) reset_wave(a);
-  const int n_active = *a.active_count;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int slot_i = blockIdx.x; slot_i < n_active; slot_i += gridDim.x) {
-    const int tile = a.active[slot_i];
-    const int s = a.tile_offsets[tile], len = a.tile_len[tile];
-    const int wlo = min(a.lo, len), nwin = min(a.hi, len) - wlo;
-    if (nwin <= 0) continue;
-    __syncthreads();   // the previous tile's masks have been read
-    if (tid == 0) s_total = 0;
-    const HitPixels h = hit_pixels(a.rays_o, a.rays_d, a.px_state, tile, a.ntx, a.W, a.H, a.K > 0.f);
-    __syncthreads();
-    int mine = 0;
-    for (int j0 = warp * 32; j0 < nwin; j0 += 256) {
+    int j0 = part * 32;
+    do {
       const int j = j0 + lane;
-      const int p = j < nwin ? a.sorted_prims[s + wlo + j] : -1;
+      const size_t pair = (size_t)(s + wlo) + j;
+      const int p = j < nwin ? a.sorted_prims[pair] : -1;
       uint32_t m0, m1;
       hit_chunk<REF>(h, a.rays_o, a.rays_d, a.geom, a.n, p, min(32, nwin - j0), a.K, a.thr, a.bound2, s_q[warp], m0, m1);
       const int c = __popc(m0) + __popc(m1);
-      if (j < nwin) s_m[j] = a.masks[(size_t)(s + wlo) + j] = make_uint2(m0, m1);
       if (c > 0) atomicAdd(a.prim_cnt + p, c);
-      mine += c;
-    }
-    mine = __reduce_add_sync(0xffffffffu, mine);
-    if (lane == 0 && mine) atomicAdd(&s_total, mine);
-    __syncthreads();
-    if (tid == 0) {
-      const int total = s_total;
-      const int base = total > 0 ? atomicAdd(a.counters + kCtrRecords, total) : 0;
-      s_tile_base = base;
-      if ((int64_t)base + total > a.max_records) atomicOr(a.status + MLPSP_ST_BITS, MLPSP_ST_RECORD_OVERFLOW);
-    }
-    __syncthreads();
-    int running = s_tile_base;
-    for (int j0 = 0; j0 < nwin; j0 += 256) {
-      const int j = j0 + tid;
-      const int c = (j < nwin) ? __popc(s_m[j].x) + __popc(s_m[j].y) : 0;
-      int total;
-      const int ex = block_exclusive_scan(c, warp_sums, total);
-      if (j < nwin) a.pair_base[(size_t)(s + wlo) + j] = (uint32_t)(running + ex);
-      running += total;
-    }
+      const int inc = warp_inclusive_scan(c);
+      int base = 0;
+      if (lane == 31 && inc > 0) {
+        base = atomicAdd(a.counters + kCtrRecords, inc);
+        if ((int64_t)base + inc > a.max_records) atomicOr(a.status + MLPSP_ST_BITS, MLPSP_ST_RECORD_OVERFLOW);
+      }
+      base = __shfl_sync(0xffffffffu, base, 31);
+      if (j < nwin) {
+        a.masks[pair] = make_uint2(m0, m1);
+        a.pair_base[pair] = (uint32_t)(base + inc - c);
+      }
+    } while (LOOP && (j0 += parts * 32) < nwin);
   }
 }
 
 static int launch_hits(const HitArgs& a, bool ref_arith, int tiles, int sms, bool idle_tail, cudaStream_t st) {
-  const int win = a.hi - a.lo;
-  if (win > 128) {
-    const dim3 grid(idle_tail ? sms : std::min(tiles, sms * 8));
-    return cuda_check(ref_arith ? launch_chained(k_hits<true>, grid, dim3(256), 0, st, a) : launch_chained(k_hits<false>, grid, dim3(256), 0, st, a), "hits");
-  }
+  const int parts = std::min((a.hi - a.lo + 31) / 32, kHitParts);
   // small images spread their tiles over the SMs one warp at a time
-  const int wpb = tiles >= sms * 2 * kHitWarps ? kHitWarps : 1;
-  const dim3 grid(std::min((tiles + wpb - 1) / wpb, idle_tail ? sms : sms * 16)), block(32 * wpb);
-  auto* kernel = win <= 32 ? (ref_arith ? k_hits_warp<true, 1> : k_hits_warp<false, 1>)
-               : win <= 64 ? (ref_arith ? k_hits_warp<true, 2> : k_hits_warp<false, 2>)
-                           : (ref_arith ? k_hits_warp<true, 4> : k_hits_warp<false, 4>);
-  return cuda_check(launch_chained(kernel, grid, block, 0, st, a), "hits");
+  const int64_t units = (int64_t)tiles * parts;
+  const int wpb = units >= sms * 2 * kHitWarps ? kHitWarps : 1;
+  const dim3 grid((unsigned)std::min<int64_t>((units + wpb - 1) / wpb, idle_tail ? sms : sms * 16)), block(32 * wpb);
+  const bool loop = (a.hi - a.lo + 31) / 32 > parts;
+  auto* kernel = ref_arith ? (loop ? k_hits<true, true> : k_hits<true, false>) : (loop ? k_hits<false, true> : k_hits<false, false>);
+  return cuda_check(launch_chained(kernel, grid, block, 0, st, a, parts), "hits");
 }
 
 // Geometric hit masks of all pairs (no transmittance state): the superset the waves draw from.
