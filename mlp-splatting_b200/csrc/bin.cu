@@ -325,9 +325,10 @@ __global__ void __launch_bounds__(1024) k_bin_offsets(const int32_t* __restrict_
 // PRETEST: a (tile, primitive) pair that no ray of the tile can hit (ellipse_misses) is not
 // written; tile_fill then ends as the number of candidates kept per tile, packed at the front of the
 // tile's span of tile_prims (the span itself keeps the size the count pass gave it).
-// PPW primitives per warp: the pre-tested variant takes the pairs of eight primitives, whose ellipses one lane each
-// computes into shared memory; a pair is then one 16-byte load and about thirty operations (against a test of the
-// whitened quadratic form per pair: 102 -> 52 us on the 100k frame, 2.9 million pairs).
+// PPW primitives per warp, in the pre-tested variant 32 where a primitive covers fewer than eight tiles on average: one lane
+// each computes their ellipses into shared memory; a pair is then one 16-byte load and about thirty operations (against a
+// test of the whitened quadratic form per pair: 102 -> 52 us on the 100k frame, 2.9 million pairs).  With eight primitives of
+// two pairs each three quarters of the lanes idle through the ellipses (four 500k views: 272 us, with 32 205).
 template <bool PRETEST, int PPW>
 __global__ void __launch_bounds__(256) k_bin_scatter(int n, int ntx, const uint2* __restrict__ rect,
                                                      const int32_t* __restrict__ tile_offsets,
@@ -338,13 +339,15 @@ __global__ void __launch_bounds__(256) k_bin_scatter(int n, int ntx, const uint2
   chain_wait();
   chain_release();
   __shared__ WarpRects s_wr[8];
-  __shared__ float4 s_el[PRETEST ? 8 : 1][PPW][2];
+  __shared__ float4 s_el[PRETEST ? 8 : 1][PRETEST ? 32 : 1][2];
   if (status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gwarp = blockIdx.x * 8 + warp;
-  const int p = gwarp * PPW + lane;
+  const int ppw = PRETEST && (int64_t)status[MLPSP_ST_PAIRS] < 8 * (int64_t)n ? 32 : PPW;
+  if ((int64_t)gwarp * ppw >= n) return;
+  const int p = gwarp * ppw + lane;
   int x0 = 1, x1 = 0, y0 = 1, y1 = 0;
-  const bool mine = lane < PPW && p < n;
+  const bool mine = lane < ppw && p < n;
   if (mine) {
     const uint2 r = rect[p];
     x0 = r.x & 0xffff; x1 = r.x >> 16; y0 = r.y & 0xffff; y1 = r.y >> 16;
@@ -361,7 +364,7 @@ __global__ void __launch_bounds__(256) k_bin_scatter(int n, int ntx, const uint2
     if (PRETEST) {
       // q is the lane that brought the primitive: its ellipse sits in shared memory
       if (ellipse_misses(s_el[warp][q][0], s_el[warp][q][1], __ldg(tile_rect + t))) return;
-      id = gwarp * PPW + q;
+      id = gwarp * ppw + q;
     }
     const int slot = atomicAdd(tile_fill + t, 1);
     tile_prims[tile_offsets[t] + slot] = id;
