@@ -29,7 +29,7 @@ constexpr int kOW1 = 0, kOb1 = kOW1 + kGH * kGIN, kOW2 = kOb1 + kGH, kOb2 = kOW2
 static_assert(kGradLen == 3524, "gradient row layout");
 
 // plan counters (device int32)
-enum VjpCounter { kVpItems = 0, kVpRows = 1, kVpMulti = 2, kVpFlag = 3, kVpEmpty = 4, kVpCounters = 5 };
+enum VjpCounter { kVpItems = 0, kVpRows = 1, kVpMulti = 2, kVpFlag = 3, kVpEmpty = 4, kVpNext = 5, kVpCounters = 6 };
 
 // zero gradients of one primitive, by nthr threads (rows of 16-byte multiples; b = the tensors' bases aligned)
 __device__ __forceinline__ void vjp_zero(const VjpOut& o, int prim, int aligned, int t, int nthr) {

@@ -128,7 +128,8 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
   chain_release();
   extern __shared__ __align__(128) char smem[];
   const int G = counters[kVpItems], E = counters[kVpEmpty];
-  int idx = blockIdx.x, empty = blockIdx.x;      // segments; primitives without records, one between two waits
+  const int idx = blockIdx.x;
+  int empty = blockIdx.x;                        // primitives without records, one between two waits
   const int tid = threadIdx.x, warp = tid >> 5;
   auto zero_next = [&]() {
     if (empty >= E) return;
@@ -149,6 +150,10 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) tmem_alloc(smem_u32(&s_misc[0]), kVjpTmemCols);
+  // segments differ tenfold in length, so a CTA takes its first by its number and the others from a counter, two ahead
+  __shared__ int s_next;
+  auto draw = [&]() { if (tid == 0) s_next = (int)gridDim.x + atomicAdd(counters + kVpNext, 1); };
+  draw();
   // tiles: zeros, except the three chunks of ones; W1's last chunk stays zero
   {
     const uint32_t one2 = BF16 ? 0x3f803f80u : 0x3c003c00u;
@@ -309,9 +314,9 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
   };
 
   VjpItem it = load_item(items + idx), it_n = it, it_p = it;
-  const int stride = (int)gridDim.x;
-  bool has_n = idx + stride < G;
-  if (has_n) it_n = load_item(items + idx + stride);
+  bool has_n = s_next < G;
+  if (has_n) it_n = load_item(items + s_next);
+  __syncthreads();                 // before the next draw
   load_weights(it.prim);
   load_rec(it, 0);
   int sub = 0;
@@ -348,6 +353,7 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
       if (sub == 0) __syncthreads();                            // W3 of the new primitive
       vjp_d2<BF16>(d01, d23, m2, reinterpret_cast<const float4*>(s_w3), my + kVcD2 * kVjpChunk);
     }
+    if (sub == 0) draw();                                       // read after the barrier of this layer, at the segment's last block
     // ---- layer 1: K = 80 (the ones behind E meet the zero chunk of W1); with masks the first half of D1 ----
     ok = issue_phase([&]() {
       const uint64_t a = a_rows(kVcE);
@@ -371,11 +377,10 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
     } else if (has_n) {
       it = it_n;
       sub = 0;
-      idx += stride;
       load_rec(it, 0);
       load_weights(it.prim);
-      has_n = idx + stride < G;
-      if (has_n) it_n = load_item(items + idx + stride);
+      has_n = s_next < G;
+      if (has_n) it_n = load_item(items + s_next);
     } else {
       more = false;
     }
