@@ -384,10 +384,12 @@ __global__ void __launch_bounds__(kGfThreads, kGfCtas) k_grouped_vjp(
   float fr[6], at[6];
 #pragma unroll
   for (int f = 0; f < 6; ++f) { fr[f] = __ldg(freq + f); at[f] = __ldg(att + f); }
-  for (int idx = blockIdx.x; idx < G; idx += gridDim.x) {
+  __shared__ int s_next;
+  for (int idx = blockIdx.x; idx < G; idx = s_next) {            // (read behind the barriers of the item's blocks)
     const VjpItem it = load_item(items + idx);
     const size_t p = (size_t)it.prim;
     __syncthreads();                             // the previous item's last block has been consumed
+    if (tid == 0) s_next = (int)gridDim.x + atomicAdd(counters + kVpNext, 1);
 #pragma unroll
     for (int u = 0; u < 18; ++u) {               // W1 transposed: lane = row, so the stores are conflict-free
       const int k = u * 4 + (tid >> 5), h = tid & 31;
