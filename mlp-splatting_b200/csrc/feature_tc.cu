@@ -18,11 +18,9 @@
 // The copies and the record loads of the next stage are in flight while a stage is finished.
 // Afterwards each warp reads its 32 channels x 64 pixels from tensor memory and writes 128-byte lines of the map.
 //
-// The coefficients do not depend on the channel, so all channels share them where shared memory lets two CTAs of that
-// shape stay on an SM.  Bound: issue slots and the latency of the gather (each (tile, primitive) pair reads S * C * 2
-// bytes, from L2 for the most part); the map's own writes take 0.25 ms of a 1200 x 680 x 512 frame.  With blocks of 256
-// channels, every coefficient twice and addresses per copy, that frame (250k primitives) took 1.10 ms here, now 0.80;
-// a 957 x 541 x 128 one 0.26, now 0.24.
+// Bound: issue slots and the latency of the gather (each (tile, primitive) pair reads S * C * 2 bytes, from L2 for the most
+// part); the map's own writes take 0.25 ms of a 1200 x 680 x 512 frame.  With scalar coefficient code, addresses made for every
+// copy and two CTAs per SM, that frame (250k primitives) took 1.10 ms here, now 0.80; a 957 x 541 x 128 one 0.26, now 0.16.
 //
 // Every wait on an mbarrier is bounded (MLPSP_ST_TIMEOUT), copies in flight are waited for, tensor memory is freed.
 #include "frame.cuh"
