@@ -21,8 +21,14 @@
 //            wide feature vector is never formed.
 // Weight blocks (W1, the nine taps, the output chunks; <= 32 KB each) stream from the packed image (L2
 // resident) through a three-deep ring of bulk copies; a block's buffer is released by the commit of the MMAs
-// that read it.  While the issuing lane walks the nine taps the other warps fetch the next tile's input.  One
-// CTA per SM (225 KB of shared memory, all 512 tensor-memory columns).
+// that read it.  One CTA per SM (225 KB of shared memory, all 512 tensor-memory columns).
+//
+// Eight warps load inputs and run the epilogues, a ninth issues every MMA and a tenth every weight copy: a bulk
+// copy costs its lane about 70 cycles, and eight of them per tap in the lane that issues the MMAs held the nine
+// taps up to 13,800 cycles of 22,800 per tile (6,200 without them; the bound there is shared memory, which an MMA
+// of 128 x 128 x 16 reads for 64 cycles).  While the taps run the workers fetch the next tile's input, six units
+// in flight per thread, and its layer 1 is queued behind this tile's last output chunk, under the epilogue.
+// Measured (957 x 541, 128 -> 128 -> 20 classes): 340 -> 223 us.
 //
 // Every wait on an mbarrier is bounded; when one gives up the CTA raises MLPSP_ST_TIMEOUT, waits
 // (bounded) for its own copies in flight, frees its tensor memory and returns.
@@ -36,13 +42,15 @@ namespace mlpsp {
 constexpr int kDecTileW = 8, kDecTileH = 16;                       // 128 output pixels = MMA M
 constexpr int kHaloW = kDecTileW + 2, kHaloH = kDecTileH + 2;
 constexpr int kHaloPx = kHaloW * kHaloH;                           // 180
-constexpr int kDecThreads = 256;
-constexpr int kColGroups = kDecThreads / 128;                        // warps that share a tensor-memory lane quarter split the columns
+constexpr int kDecWorkers = 256;                                   // threads that load inputs and run the epilogues
+constexpr int kMmaWarp = kDecWorkers / 32, kCopyWarp = kMmaWarp + 1; // one warp issues the products, one the weight copies
+constexpr int kDecThreads = kDecWorkers + 64;
+constexpr int kDecAhead = 6;                                       // input units (32 bytes each) in flight per thread
+constexpr int kColGroups = kDecWorkers / 128;                        // warps that share a tensor-memory lane quarter split the columns
 constexpr int kDecBlock = 32768;                                   // one weight block: <= 128 x 128 halves
 constexpr int kDecRing = 3;
 constexpr int kStageFloats = 32 * 32;                               // one warp's output staging tile: 32 pixels x 32 columns, 16-byte units XOR-swizzled by pixel
-constexpr int kDecPieces = 8;                                      // bulk copies per weight block (block sizes are multiples of 1 KB)
-constexpr int kDecSub = 1;                                         // tiles that share one pass over the weights
+constexpr int kDecPieces = 2;                                      // bulk copies per weight block (block sizes are multiples of 1 KB)
 constexpr int kDecMaxBlocks = 16;                                  // per pass: W1, 9 taps, <= 6 output chunks
 constexpr int kDecMaxDim = 128;                                    // input and hidden width limit
 constexpr int kDecMaxOut = 768;
@@ -62,12 +70,12 @@ constexpr int kSmRing = 0;
 constexpr int kSmA0 = kSmRing + kDecRing * kDecBlock;                 //  98,304
 constexpr int kA0Pitch = kHaloPx + 1;                                 // 16-byte units between K chunks of the input tile (odd)
 constexpr int kSmH1 = kSmA0 + (kDecMaxDim / 8) * kA0Pitch * 16;       // +46,336
-constexpr int kSmBias = kSmH1 + kDecSub * kDecH1Bytes;                // +46,080
+constexpr int kSmBias = kSmH1 + kDecH1Bytes;                // +46,080
 constexpr int kSmHdr = kSmBias + 4 * (2 * kDecMaxDim + kDecMaxOut);   // + 4,096
 constexpr int kSmBar = kSmHdr + 256;
 constexpr int kSmMisc = kSmBar + 16 * 8;
 constexpr int kSmArg = kSmMisc + 64;                                  // [2][128] (value, index) pairs
-constexpr int kSmStage = kSmArg + kDecSub * kColGroups * 128 * 8;     // output staging tiles of the first eight warps
+constexpr int kSmStage = kSmArg + kColGroups * 128 * 8;     // output staging tiles of the first eight warps
 constexpr int kDecSmem = kSmStage + 8 * kStageFloats * 4;
 static_assert(kDecSmem <= 227 * 1024, "shared memory of the decoder");
 
@@ -100,8 +108,8 @@ static bool dec_layout(const mlpsp_decoder* d, int mode, DecHeader* h) {
   return nb <= kDecMaxBlocks;
 }
 
-// either half of a packed binary16 pair is inf or NaN
-__device__ __forceinline__ bool h2_nonfinite(uint32_t w) { return (w & 0x7c00u) == 0x7c00u || ((w >> 16) & 0x7c00u) == 0x7c00u; }
+// bit 15 or 31 set: that half of a packed binary16 pair is inf or NaN
+__device__ __forceinline__ uint32_t h2_range(uint32_t w) { return (w & 0x7fff7fffu) + 0x04000400u; }
 
 __device__ __forceinline__ uint16_t to_h16(float x, bool& bad) {
   const __half v = __float2half_rn(x);
@@ -183,17 +191,18 @@ __global__ void k_fold_text(const float* __restrict__ text, const float* __restr
 // consecutive 32-byte pieces of a pixel's feature row (coalesced); the odd pitch spreads the 16-byte stores
 // of one pixel's chunks over all banks.  Loads are issued four units ahead of their conversion.
 // Threads t = 0..nthr-1 of the CTA share the tile.
-__device__ __forceinline__ bool load_input_tile(const float* __restrict__ feat, int W, int H, int Cin, int K1,
+template <int B>
+__device__ __forceinline__ uint32_t load_input_tile(const float* __restrict__ feat, int W, int H, int Cin, int K1,
                                                 int ty0, int tx0, char* s_a0, int t, int nthr) {
   // unit u = (halo pixel r, 16-byte chunk kc), chunk fastest; the chunk count is padded to a power of two so that
   // the split is a shift and a mask
   const int nk = K1 >> 3, lg = nk > 8 ? 4 : (nk > 4 ? 3 : (nk > 2 ? 2 : 1)), units = kHaloPx << lg;
   const bool vec = (Cin & 7) == 0;
-  bool bad = false;
-  for (int u0 = t; u0 < units; u0 += 4 * nthr) {
-    float4 lo[4], hi[4];
+  uint32_t range = 0;
+  for (int u0 = t; u0 < units; u0 += B * nthr) {
+    float4 lo[B], hi[B];
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
+    for (int b = 0; b < B; ++b) {
       const int u = u0 + b * nthr;
       lo[b] = hi[b] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (u < units) {
@@ -216,33 +225,33 @@ __device__ __forceinline__ bool load_input_tile(const float* __restrict__ feat, 
       }
     }
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
+    for (int b = 0; b < B; ++b) {
       const int u = u0 + b * nthr;
       const int r = u >> lg, kc = u & ((1 << lg) - 1);
       if (u < units && kc < nk) {
         uint4 w;
         w.x = pack_h2<false>(lo[b].x, lo[b].y); w.y = pack_h2<false>(lo[b].z, lo[b].w);
         w.z = pack_h2<false>(hi[b].x, hi[b].y); w.w = pack_h2<false>(hi[b].z, hi[b].w);
-        bad |= h2_nonfinite(w.x) || h2_nonfinite(w.y) || h2_nonfinite(w.z) || h2_nonfinite(w.w);   // beyond binary16 range
+        range |= h2_range(w.x) | h2_range(w.y) | h2_range(w.z) | h2_range(w.w);   // beyond binary16 range
         *reinterpret_cast<uint4*>(s_a0 + (kc * kA0Pitch + r) * 16) = w;
       }
     }
   }
-  return bad;
+  return range;
 }
 
-// +bias, ReLU, binary16: 32 accumulator columns -> four 16-byte units of the next A operand
-__device__ __forceinline__ bool relu_pack(const uint32_t (&acc)[32], const float* bias, int j, uint4& out) {
+// +bias, ReLU, binary16: 32 accumulator columns -> four 16-byte units of the next A operand.  The halves are not
+// negative, so inf and NaN (0x7c00 and above) are those that reach bit 15 when 0x0400 is added; `range` collects it.
+__device__ __forceinline__ void relu_pack(const uint32_t (&acc)[32], const float* bias, int j, uint4& out, uint32_t& range) {
   uint32_t w[4];
-  bool bad = false;
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    w[e] = pack_h2_relu<false>(__uint_as_float(acc[j * 8 + e * 2]) + bias[j * 8 + e * 2],
-                               __uint_as_float(acc[j * 8 + e * 2 + 1]) + bias[j * 8 + e * 2 + 1]);
-    bad |= h2_nonfinite(w[e]);
+  for (int e = 0; e < 4; e += 2) {
+    const float4 b = *reinterpret_cast<const float4*>(bias + j * 8 + e * 2);
+    w[e] = pack_h2_relu<false>(__uint_as_float(acc[j * 8 + e * 2]) + b.x, __uint_as_float(acc[j * 8 + e * 2 + 1]) + b.y);
+    w[e + 1] = pack_h2_relu<false>(__uint_as_float(acc[j * 8 + e * 2 + 2]) + b.z, __uint_as_float(acc[j * 8 + e * 2 + 3]) + b.w);
+    range |= (w[e] + 0x04000400u) | (w[e + 1] + 0x04000400u);
   }
   out = make_uint4(w[0], w[1], w[2], w[3]);
-  return bad;
 }
 
 // n MMAs D (+)= A_k . B_k whose operand descriptors advance by fixed steps (in 16-byte units of the start-address
@@ -265,14 +274,14 @@ __global__ void __launch_bounds__(kDecThreads, 1) k_decode_tc(
   extern __shared__ __align__(128) char smem[];
   const DecHeader& hd = *reinterpret_cast<const DecHeader*>(smem + kSmHdr);
   float* s_bias = reinterpret_cast<float*>(smem + kSmBias);
-  uint64_t* s_bar = reinterpret_cast<uint64_t*>(smem + kSmBar);   // [0..1] full, [2..3] empty, [4] mma, [5] output chunk
+  uint64_t* s_bar = reinterpret_cast<uint64_t*>(smem + kSmBar);   // per ring buffer: full, empty; then layers 1 and 2, output chunk
   uint32_t* s_misc = reinterpret_cast<uint32_t*>(smem + kSmMisc);
   float2* s_arg = reinterpret_cast<float2*>(smem + kSmArg);
   if (status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
-  const int num_pairs = (num_tiles + kDecSub - 1) / kDecSub;
-  if ((int)blockIdx.x >= num_pairs) return;          // leave before touching tensor memory
+  if ((int)blockIdx.x >= num_tiles) return;          // leave before touching tensor memory
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int q = warp & 3, hsel = warp >> 2;           // tensor-memory lane quarter, column interleave
+  const bool worker = warp < kMmaWarp;
   if (tid < 64) reinterpret_cast<int32_t*>(smem + kSmHdr)[tid] = __ldg(reinterpret_cast<const int32_t*>(image) + tid);
   __syncthreads();
   const int Cin = hd.in_dim, K1 = hd.k1, Ch = hd.hidden, n_out = hd.n_out, n_pad = hd.n_pad, NB = hd.num_blocks;
@@ -295,23 +304,22 @@ __global__ void __launch_bounds__(kDecThreads, 1) k_decode_tc(
   tc_fence_after();
   const uint32_t tmem = s_misc[0];
   const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16);
-  const int n_my = (num_pairs - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int n_my = (num_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
   const int total_blocks = n_my * NB;
   const int out_chunks = (n_pad + 127) >> 7;
   const uint32_t idesc_h = instr_desc(128, Ch);
-  static_assert(kDecSub == 1, "the early fetch of the next input assumes one tile per pass");
-  const bool prefetch = true;
-  int issued = 0, landed = 0;            // issuing thread only: copies requested / copies waited for
+  int issued = 0;                        // copying lane only: blocks requested
   uint32_t ph_m = 0, ph_o = 0;
-  bool ok = true, bad = false;
+  bool ok = true;
+  uint32_t range = 0;                    // bits 15 and 31: an activation beyond the binary16 range
 
-  // issuing thread: request the copies of blocks issued..upto (ring order), each after the MMAs that read
+  // copying lane: request the copies of blocks issued..upto (ring order), each after the MMAs that read
   // the buffer's previous block have committed
   auto request = [&](int upto) {
     while (ok && issued <= upto && issued < total_blocks) {
       const int j = issued, b = j % kDecRing, use = j / kDecRing, blk = j % NB;
       if (use > 0 && !mbar_wait(bar_empty + 8 * b, (uint32_t)((use - 1) & 1))) { ok = false; break; }
-      // one bulk copy moves about 12 bytes per clock; eight pieces in flight share the barrier's byte count
+      // the pieces of a block share the barrier's byte count
       const uint32_t bytes = (uint32_t)hd.blk_bytes[blk], piece = bytes / kDecPieces;
       mbar_expect_tx(bar_full + 8 * b, bytes);
       for (int pc = 0; pc < kDecPieces; ++pc)
@@ -319,99 +327,88 @@ __global__ void __launch_bounds__(kDecThreads, 1) k_decode_tc(
       ++issued;
     }
   };
-  // issuing thread: wait for block g (requested here at the latest)
+  // issuing lane: wait for block g
   auto acquire = [&](int g) -> uint32_t {
-    request(g);
     const int b = g % kDecRing;
     if (ok && !mbar_wait(bar_full + 8 * b, (uint32_t)((g / kDecRing) & 1))) ok = false;
-    if (ok) landed = g + 1;
     tc_fence_after();
     return ring + b * kDecBlock;
   };
-  // issuing thread: the MMAs that read block g have been issued: their commit frees the buffer, and the copies
-  // that fit behind them are requested (the buffer of the block before g is free by then or very soon)
-  auto release = [&](int g) {
-    mma_commit(bar_empty + 8 * (g % kDecRing));
-    request(g + kDecRing - 1);
+  // issuing lane: the MMAs that read block g have been issued; their commit frees the buffer
+  auto release = [&](int g) { mma_commit(bar_empty + 8 * (g % kDecRing)); };
+
+  // issuing lane: layer 1 of the pass whose first weight block is g; rows 0..127 -> columns [0, Ch), rows 52..179 ->
+  // [128, 128 + Ch)
+  auto layer1 = [&](int g) {
+    const uint32_t wb = acquire(g);
+    if (!ok) return;
+    const uint64_t bd = smem_desc(wb, Ch * 16, 128);
+    for (int mt = 0; mt < 2; ++mt)
+      mma_chain(tmem + mt * 128, smem_desc(a0 + mt * 52 * 16, kA0Pitch * 16, 128), bd, 2 * kA0Pitch, 2 * Ch, K1 >> 4, idesc_h,
+                false);
+    mma_commit(bar_m);
+    release(g);
   };
 
+  if (warp == kCopyWarp && elect_one()) request(kDecRing - 1);
+  if (worker)
+    range |= load_input_tile<kDecAhead>(feat, W, H, Cin, K1, ((int)blockIdx.x / tiles_x) * kDecTileH,
+                                      ((int)blockIdx.x % tiles_x) * kDecTileW, smem + kSmA0, tid, kDecWorkers);
+  fence_async_smem();
+  tc_fence_before();
+  if (!__syncthreads_and(ok)) ok = false;
+  if (warp == kMmaWarp && elect_one()) layer1(0);
   for (int it = 0; it < n_my; ++it) {
-    const int pair = (int)blockIdx.x + it * (int)gridDim.x;
+    const int tile = (int)blockIdx.x + it * (int)gridDim.x;
     const int gbase = it * NB;
-    int ty0[kDecSub], tx0[kDecSub];
+    const int ty0 = (tile / tiles_x) * kDecTileH, tx0 = (tile % tiles_x) * kDecTileW;
+    // ---- hidden tile: layer 1 over the 180 halo pixels, issued one pass ahead ----
+    ok = __all_sync(0xffffffffu, mbar_wait(bar_m, ph_m) && ok);
+    ph_m ^= 1u;
+    tc_fence_after();
+    if (ok && worker) {
+      char* s_h1 = smem + kSmH1;
+      for (int mt = 0; mt < 2; ++mt) {
+        if (mt == 1 && q < 2) continue;               // rows 52..115 of the second product repeat the first
+        const int r = mt * 52 + q * 32 + lane;
+        const bool store = mt == 0 || r >= 128;
+        const int hy = r / kHaloW, hx = r - hy * kHaloW;
+        const int y = ty0 + hy - 1, x = tx0 + hx - 1;
+        const bool inside = y >= 0 && y < H && x >= 0 && x < W;   // outside: the 3x3 convolution's zero padding
+        for (int cc = hsel; cc < (Ch >> 5); cc += kColGroups) {
+          uint32_t acc[32];
+          tmem_ld32(trow + mt * 128 + cc * 32, acc);
 #pragma unroll
-    for (int sb = 0; sb < kDecSub; ++sb) {
-      const int tile = pair * kDecSub + sb;
-      // a tile past the end sits below the image: its loads give zeros and its stores are skipped
-      ty0[sb] = tile < num_tiles ? (tile / tiles_x) * kDecTileH : H;
-      tx0[sb] = tile < num_tiles ? (tile % tiles_x) * kDecTileW : 0;
-    }
-    // ---- per sub-tile: input, layer 1 over the 180 halo pixels, hidden tile ----
-    for (int sb = 0; sb < kDecSub; ++sb) {
-      if (!prefetch || it == 0) bad |= load_input_tile(feat, W, H, Cin, K1, ty0[sb], tx0[sb], smem + kSmA0, tid, kDecThreads);
-      fence_async_smem();
-      tc_fence_before();
-      if (!__syncthreads_and(ok)) { ok = false; break; }
-      // rows 0..127 -> columns [0, Ch), rows 52..179 -> [128, 128 + Ch)
-      if (warp == 0 && elect_one()) {
-        const uint32_t wb = acquire(gbase);
-        if (ok) {
-          const uint64_t bd = smem_desc(wb, Ch * 16, 128);
-          for (int mt = 0; mt < 2; ++mt)
-            mma_chain(tmem + mt * 128, smem_desc(a0 + mt * 52 * 16, kA0Pitch * 16, 128), bd, 2 * kA0Pitch, 2 * Ch, K1 >> 4,
-                      idesc_h, false);
-          mma_commit(bar_m);
-          if (sb == kDecSub - 1) release(gbase);
-        }
-      }
-      ok = __all_sync(0xffffffffu, mbar_wait(bar_m, ph_m) && ok);
-      ph_m ^= 1u;
-      tc_fence_after();
-      if (ok) {
-        char* s_h1 = smem + kSmH1 + sb * kDecH1Bytes;
-        for (int mt = 0; mt < 2; ++mt) {
-          if (mt == 1 && q < 2) continue;               // rows 52..115 of the second product repeat the first
-          const int r = mt * 52 + q * 32 + lane;
-          const bool store = mt == 0 || r >= 128;
-          const int hy = r / kHaloW, hx = r - hy * kHaloW;
-          const int y = ty0[sb] + hy - 1, x = tx0[sb] + hx - 1;
-          const bool inside = y >= 0 && y < H && x >= 0 && x < W;   // outside: the 3x3 convolution's zero padding
-          for (int cc = hsel; cc < (Ch >> 5); cc += kColGroups) {
-            uint32_t acc[32];
-            tmem_ld32(trow + mt * 128 + cc * 32, acc);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              uint4 w;
-              bad |= relu_pack(acc, s_bias + cc * 32, j, w);
-              if (store) *reinterpret_cast<uint4*>(s_h1 + ((cc * 4 + j) * kHaloPx + r) * 16) = inside ? w : make_uint4(0u, 0u, 0u, 0u);
-            }
+          for (int j = 0; j < 4; ++j) {
+            uint4 w;
+            relu_pack(acc, s_bias + cc * 32, j, w, range);
+            if (store) *reinterpret_cast<uint4*>(s_h1 + ((cc * 4 + j) * kHaloPx + r) * 16) = inside ? w : make_uint4(0u, 0u, 0u, 0u);
           }
         }
       }
-      fence_async_smem();
-      tc_fence_before();
-      if (!__syncthreads_and(ok)) { ok = false; break; }
     }
-    if (!ok) break;
-    // ---- layer 2: nine taps, each weight block serves every sub-tile; columns [256 + 128 sb, .. + Ch) ----
-    // While one lane issues them, the other warps fetch the next tile's input: layer 1 has finished
+    fence_async_smem();
+    tc_fence_before();
+    if (!__syncthreads_and(ok)) { ok = false; break; }
+    // ---- layer 2: nine taps into columns [256, 256 + Ch) ----
+    // While one lane issues them and another keeps the ring of weight blocks full (to the third block past the
+    // last tap: its buffer is the last tap's), the workers fetch the next tile's input: layer 1 has finished
     // reading the input tile.
-    if (warp != 0) {
-      if (prefetch && it + 1 < n_my) {
-        const int nt = ((int)blockIdx.x + (it + 1) * (int)gridDim.x) * kDecSub;
-        bad |= load_input_tile(feat, W, H, Cin, K1, (nt / tiles_x) * kDecTileH, (nt % tiles_x) * kDecTileW, smem + kSmA0,
-                               tid - 32, kDecThreads - 32);
-      }
+    if (worker) {
+      const int nt = tile + (int)gridDim.x;
+      if (it + 1 < n_my)
+        range |= load_input_tile<kDecAhead>(feat, W, H, Cin, K1, (nt / tiles_x) * kDecTileH, (nt % tiles_x) * kDecTileW,
+                                          smem + kSmA0, tid, kDecWorkers);
+    } else if (warp == kCopyWarp) {
+      if (elect_one()) request(gbase + 9 + kDecRing);
     } else if (elect_one()) {
       for (int tap = 0; tap < 9 && ok; ++tap) {
         const int g = gbase + 1 + tap;
         const uint32_t wb = acquire(g);
         if (!ok) break;
         const int shift = (tap / 3) * kHaloW + tap % 3;
-        const uint64_t bd = smem_desc(wb, Ch * 16, 128);
-        for (int sb = 0; sb < kDecSub; ++sb)
-          mma_chain(tmem + 256 + sb * 128, smem_desc(h1 + sb * kDecH1Bytes + shift * 16, kHaloPx * 16, kHaloW * 16), bd,
-                    2 * kHaloPx, 2 * Ch, Ch >> 4, idesc_h, tap != 0);
+        mma_chain(tmem + 256, smem_desc(h1 + shift * 16, kHaloPx * 16, kHaloW * 16), smem_desc(wb, Ch * 16, 128), 2 * kHaloPx,
+                  2 * Ch, Ch >> 4, idesc_h, tap != 0);
         release(g);
       }
       if (ok) mma_commit(bar_m);
@@ -419,89 +416,86 @@ __global__ void __launch_bounds__(kDecThreads, 1) k_decode_tc(
     ok = __all_sync(0xffffffffu, mbar_wait(bar_m, ph_m) && ok);
     ph_m ^= 1u;
     tc_fence_after();
-    const int m = q * 32 + lane;                       // this thread's output pixel of either sub-tile
-    if (ok) {
-      for (int sb = 0; sb < kDecSub; ++sb)
-        for (int cc = hsel; cc < (Ch >> 5); cc += kColGroups) {
-          uint32_t acc[32];
-          tmem_ld32(trow + 256 + sb * 128 + cc * 32, acc);
+    const int m = q * 32 + lane;                       // this thread's output pixel
+    if (ok && worker)
+      for (int cc = hsel; cc < (Ch >> 5); cc += kColGroups) {
+        uint32_t acc[32];
+        tmem_ld32(trow + 256 + cc * 32, acc);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            uint4 w;
-            bad |= relu_pack(acc, s_bias + Ch + cc * 32, j, w);
-            // the hidden tile of layer 3 reuses the halo tile: every MMA that read it has finished
-            *reinterpret_cast<uint4*>(smem + kSmH1 + sb * kDecH1Bytes + ((cc * 4 + j) * 128 + m) * 16) = w;
-          }
+        for (int j = 0; j < 4; ++j) {
+          uint4 w;
+          relu_pack(acc, s_bias + Ch + cc * 32, j, w, range);
+          // the hidden tile of layer 3 reuses the halo tile: every MMA that read it has finished
+          *reinterpret_cast<uint4*>(smem + kSmH1 + ((cc * 4 + j) * 128 + m) * 16) = w;
         }
-    }
+      }
     fence_async_smem();
     tc_fence_before();
     if (!__syncthreads_and(ok)) { ok = false; break; }
-    // ---- layer 3 in chunks of <= 128 output columns; sub-tile sb accumulates in columns [128 sb, ..) ----
-    float best[kDecSub];
-    int arg[kDecSub];
-#pragma unroll
-    for (int sb = 0; sb < kDecSub; ++sb) { best[sb] = -3.0e38f; arg[sb] = 0; }
+    // ---- layer 3 in chunks of <= 128 output columns, which accumulate in columns [384, ..) ----
+    // Behind the last chunk the issuing lane queues layer 1 of the next tile (its input is in place and its columns
+    // are free), so that it runs under this tile's last epilogue.
+    float best = -3.0e38f;
+    int arg = 0;
     for (int c = 0; c < out_chunks; ++c) {
       const int nc = min(128, n_pad - c * 128);
-      if (warp == 0 && elect_one()) {
-        const int g = gbase + 10 + c;
-        const uint32_t wb = acquire(g);
-        if (ok) {
-          const uint64_t bd = smem_desc(wb, nc * 16, 128);
-          for (int sb = 0; sb < kDecSub; ++sb)
-            mma_chain(tmem + sb * 128, smem_desc(h1 + sb * kDecH1Bytes, 128 * 16, 128), bd, 2 * 128, 2 * nc, Ch >> 4,
+      if (warp == kMmaWarp) {
+        if (elect_one()) {
+          const int g = gbase + 10 + c;
+          const uint32_t wb = acquire(g);
+          if (ok) {
+            mma_chain(tmem + 384, smem_desc(h1, 128 * 16, 128), smem_desc(wb, nc * 16, 128), 2 * 128, 2 * nc, Ch >> 4,
                       instr_desc(128, nc), false);
-          mma_commit(bar_o);
-          release(g);
+            mma_commit(bar_o);
+            release(g);
+            if (c == out_chunks - 1 && it + 1 < n_my) layer1(gbase + NB);
+          }
         }
+      } else if (warp == kCopyWarp && elect_one()) {
+        request(gbase + 10 + c + kDecRing);
       }
       ok = __all_sync(0xffffffffu, mbar_wait(bar_o, ph_o) && ok);
       ph_o ^= 1u;
       tc_fence_after();
-      if (ok) {
+      if (ok && worker) {
+        for (int cc = hsel; cc < (nc >> 5); cc += kColGroups) {
+          uint32_t acc[32];
+          tmem_ld32(trow + 384 + cc * 32, acc);
+          const int col0 = c * 128 + cc * 32;
+          const float* b3 = s_bias + 2 * Ch + col0;
+          if (classify) {
 #pragma unroll
-        for (int sb = 0; sb < kDecSub; ++sb) {
-          // decoded features: the first eight warps only (one staging tile each)
-          for (int cc = hsel; cc < (nc >> 5) && (classify || hsel < 2); cc += classify ? kColGroups : 2) {
-            uint32_t acc[32];
-            tmem_ld32(trow + sb * 128 + cc * 32, acc);
-            const int col0 = c * 128 + cc * 32;
-            const float* b3 = s_bias + 2 * Ch + col0;
-            if (classify) {
+            for (int e = 0; e < 32; ++e) {
+              const float v = __uint_as_float(acc[e]) + b3[e];
+              if (col0 + e < n_out && v > best) { best = v; arg = col0 + e; }
+            }
+          } else {
+            // 32 pixels x 32 columns of this warp go through a staging tile so that eight lanes write one pixel's
+            // 128 contiguous bytes; the 16-byte unit u of pixel row l sits at unit u ^ (l & 7): both the row
+            // writes and the transposed reads touch every bank once per eight lanes
+            float* stg = reinterpret_cast<float*>(smem + kSmStage) + warp * kStageFloats;
+            __syncwarp();
 #pragma unroll
-              for (int e = 0; e < 32; ++e) {
-                const float v = __uint_as_float(acc[e]) + b3[e];
-                if (col0 + e < n_out && v > best[sb]) { best[sb] = v; arg[sb] = col0 + e; }
-              }
-            } else {
-              // 32 pixels x 32 columns of this warp go through a staging tile so that eight lanes write one pixel's
-              // 128 contiguous bytes; the 16-byte unit u of pixel row l sits at unit u ^ (l & 7): both the row
-              // writes and the transposed reads touch every bank once per eight lanes
-              float* stg = reinterpret_cast<float*>(smem + kSmStage) + warp * kStageFloats;
-              __syncwarp();
+            for (int e = 0; e < 32; e += 4)
+              *reinterpret_cast<float4*>(stg + lane * 32 + (((e >> 2) ^ (lane & 7)) << 2)) =
+                  make_float4(__uint_as_float(acc[e]) + b3[e], __uint_as_float(acc[e + 1]) + b3[e + 1],
+                              __uint_as_float(acc[e + 2]) + b3[e + 2], __uint_as_float(acc[e + 3]) + b3[e + 3]);
+            __syncwarp();
+            const int cq = (lane & 7) * 4;
 #pragma unroll
-              for (int e = 0; e < 32; e += 4)
-                *reinterpret_cast<float4*>(stg + lane * 32 + (((e >> 2) ^ (lane & 7)) << 2)) =
-                    make_float4(__uint_as_float(acc[e]) + b3[e], __uint_as_float(acc[e + 1]) + b3[e + 1],
-                                __uint_as_float(acc[e + 2]) + b3[e + 2], __uint_as_float(acc[e + 3]) + b3[e + 3]);
-              __syncwarp();
-              const int cq = (lane & 7) * 4;
-#pragma unroll
-              for (int rr = 0; rr < 32; rr += 4) {
-                const int ml = rr + (lane >> 3), mm = q * 32 + ml;            // pixel of the tile this lane writes for
-                const int oy = ty0[sb] + (mm >> 3), ox = tx0[sb] + (mm & 7);
-                if (oy < H && ox < W) {
-                  const float4 v = *reinterpret_cast<const float4*>(stg + ml * 32 + ((((cq >> 2)) ^ (ml & 7)) << 2));
-                  float* dst = out + ((int64_t)oy * W + ox) * n_out + col0 + cq;
-                  if ((n_out & 3) == 0) {
-                    if (col0 + cq < n_out) *reinterpret_cast<float4*>(dst) = v;
-                  } else {
-                    if (col0 + cq < n_out) dst[0] = v.x;
-                    if (col0 + cq + 1 < n_out) dst[1] = v.y;
-                    if (col0 + cq + 2 < n_out) dst[2] = v.z;
-                    if (col0 + cq + 3 < n_out) dst[3] = v.w;
-                  }
+            for (int rr = 0; rr < 32; rr += 4) {
+              const int ml = rr + (lane >> 3), mm = q * 32 + ml;            // pixel of the tile this lane writes for
+              const int oy = ty0 + (mm >> 3), ox = tx0 + (mm & 7);
+              if (oy < H && ox < W) {
+                const float4 v = *reinterpret_cast<const float4*>(stg + ml * 32 + ((((cq >> 2)) ^ (ml & 7)) << 2));
+                float* dst = out + ((int64_t)oy * W + ox) * n_out + col0 + cq;
+                if ((n_out & 3) == 0) {
+                  if (col0 + cq < n_out) *reinterpret_cast<float4*>(dst) = v;
+                } else {
+                  if (col0 + cq < n_out) dst[0] = v.x;
+                  if (col0 + cq + 1 < n_out) dst[1] = v.y;
+                  if (col0 + cq + 2 < n_out) dst[2] = v.z;
+                  if (col0 + cq + 3 < n_out) dst[3] = v.w;
                 }
               }
             }
@@ -514,34 +508,28 @@ __global__ void __launch_bounds__(kDecThreads, 1) k_decode_tc(
     if (!ok) break;
     if (classify) {
       // the column interleaves of a pixel meet here; the lower class index wins a tie
-#pragma unroll
-      for (int sb = 0; sb < kDecSub; ++sb) s_arg[(sb * kColGroups + hsel) * 128 + m] = make_float2(best[sb], __int_as_float(arg[sb]));
+      if (worker) s_arg[hsel * 128 + m] = make_float2(best, __int_as_float(arg));
       __syncthreads();
       if (hsel == 0) {
-#pragma unroll
-        for (int sb = 0; sb < kDecSub; ++sb) {
-          const int py = ty0[sb] + (m >> 3), px = tx0[sb] + (m & 7);
-          float bv = best[sb];
-          int a = arg[sb];
-          for (int g = 1; g < kColGroups; ++g) {
-            const float2 o = s_arg[(sb * kColGroups + g) * 128 + m];
-            const int oa = __float_as_int(o.y);
-            if (o.x > bv || (o.x == bv && oa < a)) { bv = o.x; a = oa; }
-          }
-          if (py < H && px < W) labels[(int64_t)py * W + px] = a;
+        const int py = ty0 + (m >> 3), px = tx0 + (m & 7);
+        for (int g = 1; g < kColGroups; ++g) {
+          const float2 o = s_arg[g * 128 + m];
+          const int oa = __float_as_int(o.y);
+          if (o.x > best || (o.x == best && oa < arg)) { best = o.x; arg = oa; }
         }
+        if (py < H && px < W) labels[(int64_t)py * W + px] = arg;
       }
-      __syncthreads();
     }
   }
 
-  if (!ok && warp == 0 && elect_one()) {
+  if (!ok && warp == kCopyWarp && elect_one()) {
     atomicOr(status + MLPSP_ST_BITS, MLPSP_ST_TIMEOUT);
-    // copies requested but never waited for may still be in flight: give each a bounded chance to land
+    // the last copies requested, one per buffer, may still be in flight: give each a bounded chance to land
     // before the shared memory is released
-    for (int j = landed; j < issued; ++j) mbar_wait(bar_full + 8 * (j % kDecRing), (uint32_t)((j / kDecRing) & 1));
+    for (int j = issued > kDecRing ? issued - kDecRing : 0; j < issued; ++j)
+      mbar_wait(bar_full + 8 * (j % kDecRing), (uint32_t)((j / kDecRing) & 1));
   }
-  if (bad) atomicOr(status + MLPSP_ST_BITS, MLPSP_ST_NUMERIC);
+  if (range & 0x80008000u) atomicOr(status + MLPSP_ST_BITS, MLPSP_ST_NUMERIC);
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_free(tmem, 512);
@@ -731,7 +719,7 @@ extern "C" int mlpsp_decode_features(const mlpsp_decoder* dec, int32_t mode, con
   const int num_tiles = tiles_x * tiles_y;
   cudaStream_t st = (cudaStream_t)stream;
   LaunchScope scope(kKMisc, 1, st);
-  k_decode_tc<<<std::min((num_tiles + kDecSub - 1) / kDecSub, sms), kDecThreads, kDecSmem, st>>>((const char*)packed, feat, width, height, tiles_x, num_tiles,
+  k_decode_tc<<<std::min(num_tiles, sms), kDecThreads, kDecSmem, st>>>((const char*)packed, feat, width, height, tiles_x, num_tiles,
                                                                      out, reinterpret_cast<long long*>(labels), status);
   return cuda_check(cudaGetLastError(), "mlpsp_decode_features");
 }

@@ -259,3 +259,19 @@ def test_training_records_with_weights_beyond_binary16():
     assert len(half[2]) > 1000
     for a, b in zip(half, full):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("out_dim,classes,hidden,cin,W,H", [(300, 160, 64, 24, 170, 150), (768, 700, 128, 128, 161, 137), (128, 1, 96, 7, 8, 5000)])
+def test_decoder_queues_layer_one_behind_the_last_output_chunk(out_dim, classes, hidden, cin, W, H):
+    """Several tiles per CTA with one to six output chunks: the ring of weight blocks wraps at every offset."""
+    from mlp_splatting_b200 import synthetic as syn
+    from mlp_splatting_b200.feature_decoder import FeatureUpsampleDecoder
+    from oracle import oracle as orc
+    w, text = syn.make_decoder(cin, hidden, out_dim, classes, seed=W)
+    dec = FeatureUpsampleDecoder(cin, out_dim, hidden, device=torch.device(DEV))
+    dec.load_state_dict({k: torch.from_numpy(v) for k, v in w.items()})
+    x = syn.make_feature_map(W, H, cin, seed=H)
+    want = orc.decode_features(x, w, precision=1)
+    assert np.abs(dec.decode_hwc(_t(x)).cpu().numpy() - want).max() <= 2e-3
+    labels, margin = orc.classify_features(want, text)
+    assert not (dec.classify(_t(x), _t(text)).cpu().numpy() != labels)[margin > 2e-3].any()
