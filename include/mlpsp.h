@@ -375,7 +375,7 @@ int64_t mlpsp_grouped_gradient_floats(void);
  * loss_scale multiplies the adjoints before the cast and divides the sums after (the reference uses 4096 for
  * binary16, 1 otherwise).  *nonfinite: bit 0 = a sum is not finite -- the caller retries a mixed-precision call
  * with MLPSP_PRECISION_F32 and loss_scale 1 as primitive_gemm.py:64-98 does (the host mirror does);
- * bit 1 = a device-side wait gave up, results invalid. */
+ * bit 1 = a device-side wait gave up, results invalid; bit 2 = the offsets descend or leave the records, no gradients. */
 /* The segments follow from the offsets and segment_size, so the call plans them itself (seg_prim, seg_start, seg_offsets
  * and partial are checked and otherwise unused; its scratch comes from the stream's memory pool). */
 int mlpsp_grouped_weight_gradients(const mlpsp_scene* scene, const int64_t* offsets, const float* x6, const float* d4,
@@ -385,8 +385,8 @@ int mlpsp_grouped_weight_gradients(const mlpsp_scene* scene, const int64_t* offs
                                    int32_t* nonfinite, void* stream);
 
 /* The same gradients written to the six gradient tensors (dW1[n,32,72] db1[n,32] dW2[n,32,32] db2[n,32] dW3[n,4,32]
- * db3[n,4]), with the caller's scratch and without a prepared layout.  num_records = offsets[n].  *nonfinite_host (HOST)
- * receives the flag word described above; the call waits for it. */
+ * db3[n,4]), with the caller's scratch and without a prepared layout.  x6, d4 and relu_masks hold num_records rows, at
+ * least offsets[n].  *nonfinite_host (HOST) receives the flag word described above; the call waits for it. */
 int64_t mlpsp_weight_gradients_scratch_bytes(int64_t num_records, int32_t n, int32_t segment_size);
 int mlpsp_weight_gradients(const mlpsp_scene* scene, const int64_t* offsets, const float* x6, const float* d4,
                            const int32_t* relu_masks, int64_t num_records, int32_t segment_size, int32_t precision,

@@ -302,8 +302,11 @@ __global__ void __launch_bounds__(128) k_reverse_finish(const float* __restrict_
 // Segments of the launch, planned on the device (no count travels to the host): the order of the items does not matter,
 // a primitive of several segments owns consecutive partial rows and an entry of the multi list, a primitive without
 // records (its gradients are zero) an entry at the other end of that list.
-__global__ void __launch_bounds__(256) k_vjp_plan(const int64_t* __restrict__ offsets, int n, int segment_size,
-                                                  VjpItem* __restrict__ items, VjpItem* __restrict__ multi,
+// The lists are sized from the record count, the segments counted from the offsets: offsets that descend or leave
+// [0, records] set a flag bit, on which the kernels behind this one do nothing, and no item is written past the list.
+// (With every range ascending inside [0, records] the counts add up to no more than the records, and the lists hold them.)
+__global__ void __launch_bounds__(256) k_vjp_plan(const int64_t* __restrict__ offsets, int n, int64_t records, int segment_size,
+                                                  VjpItem* __restrict__ items, int64_t max_items, VjpItem* __restrict__ multi,
                                                   int32_t* __restrict__ counters) {
   chain_wait();
   chain_release();
@@ -311,7 +314,12 @@ __global__ void __launch_bounds__(256) k_vjp_plan(const int64_t* __restrict__ of
   __shared__ int base[4];
   const int p = blockIdx.x * 256 + threadIdx.x;
   int64_t start = 0, count = 0;
-  if (p < n) { start = offsets[p]; count = offsets[p + 1] - start; }
+  if (p < n) {
+    start = offsets[p];
+    const int64_t end = offsets[p + 1];
+    if (start < 0 || end < start || end > records) atomicOr(counters + kVpFlag, kVpBadPlan);
+    else count = end - start;
+  }
   const int segs = count > 0 ? (int)((count + segment_size - 1) / segment_size) : 0;
   const int rows = segs > 1 ? segs : 0, listed = segs > 1, empty = p < n && segs == 0;
   int ts, tr, tm, te;
@@ -332,7 +340,8 @@ __global__ void __launch_bounds__(256) k_vjp_plan(const int64_t* __restrict__ of
     it.rows = (int)min((int64_t)segment_size, count - (int64_t)g * segment_size);
     it.prim = p;
     it.dest = segs > 1 ? base[1] + er + g : -1;
-    items[base[0] + es + g] = it;
+    const uint32_t at = (uint32_t)(base[0] + es + g);
+    if (at < max_items) items[at] = it;
   }
   if (listed) {
     VjpItem it = {};
@@ -375,7 +384,7 @@ __global__ void __launch_bounds__(kGfThreads, kGfCtas) k_grouped_vjp(
   chain_wait();
   chain_release();
   extern __shared__ __align__(16) float sm[];
-  const int G = counters[kVpItems];
+  const int G = vjp_planned(counters, kVpItems);
   const int tid = threadIdx.x;
   const int hg = tid & 7, rg = tid >> 3;         // units 4 hg .. + 3 of records 4 rg .. + 3; gradient rows 2 rg, 2 rg + 1
   const float inv = 1.f / scale;
@@ -551,7 +560,7 @@ __global__ void __launch_bounds__(256) k_vjp_reduce(const VjpItem* __restrict__ 
                                                     VjpOut out, int n, int zeros, int aligned, int32_t* __restrict__ counters) {
   chain_wait();
   chain_release();
-  const int M = counters[kVpMulti], E = zeros ? counters[kVpEmpty] : 0;
+  const int M = vjp_planned(counters, kVpMulti), E = zeros ? vjp_planned(counters, kVpEmpty) : 0;
   bool bad = false;
   for (int e = blockIdx.x; e < E; e += gridDim.x) vjp_zero(out, __ldg(&multi[n - 1 - e].prim), aligned, threadIdx.x, 256);
   for (int e = blockIdx.x; e < M; e += gridDim.x) {
@@ -606,7 +615,8 @@ static int weight_gradients(const mlpsp_scene* sc, const int64_t* offsets, const
   float* partial = reinterpret_cast<float*>(base + L.partial);
   LaunchScope scope(kKMisc, R > 0 ? 3 : 2, st);
   MLPSP_CUDA_OK(cudaMemsetAsync(counters, 0, 4 * kVpCounters, st));
-  launch_chained(k_vjp_plan, dim3((sc->n + 255) / 256), dim3(256), 0, st, offsets, sc->n, segment_size, items, multi, counters);
+  launch_chained(k_vjp_plan, dim3((sc->n + 255) / 256), dim3(256), 0, st, offsets, sc->n, R, segment_size, items, L.max_items,
+                 multi, counters);
   const bool tc = R > 0 && precision != MLPSP_PRECISION_F32;
   if (tc) {
     const int rc = launch_grouped_vjp_tc(precision == MLPSP_PRECISION_BF16, x6, d4, masks, items, L.max_items, multi, counters, sc, loss_scale,

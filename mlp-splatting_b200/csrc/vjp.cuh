@@ -28,8 +28,13 @@ constexpr int kOW1 = 0, kOb1 = kOW1 + kGH * kGIN, kOW2 = kOb1 + kGH, kOb2 = kOW2
               kOb3 = kOW3 + 4 * kGH, kGradLen = kOb3 + 4;   // 3,524 = the reference's packed gradient row
 static_assert(kGradLen == 3524, "gradient row layout");
 
-// plan counters (device int32)
+// plan counters (device int32); the flag word holds the bits that mlpsp.h gives for *nonfinite
 enum VjpCounter { kVpItems = 0, kVpRows = 1, kVpMulti = 2, kVpFlag = 3, kVpEmpty = 4, kVpNext = 5, kVpCounters = 6 };
+constexpr int kVpBadPlan = 4;
+// a counter of the plan, 0 when the offsets were refused: a list that may be cut short or point past the records is not read
+__device__ __forceinline__ int vjp_planned(const int32_t* counters, int which) {
+  return (counters[kVpFlag] & kVpBadPlan) ? 0 : counters[which];
+}
 
 // zero gradients of one primitive, by nthr threads (rows of 16-byte multiples; b = the tensors' bases aligned)
 __device__ __forceinline__ void vjp_zero(const VjpOut& o, int prim, int aligned, int t, int nthr) {

@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
   chain_wait();
   chain_release();
   extern __shared__ __align__(128) char smem[];
-  const int G = counters[kVpItems], E = counters[kVpEmpty];
+  const int G = vjp_planned(counters, kVpItems), E = vjp_planned(counters, kVpEmpty);
   const int idx = blockIdx.x;
   int empty = blockIdx.x;                        // primitives without records, one between two waits
   const int tid = threadIdx.x, warp = tid >> 5;

@@ -231,6 +231,8 @@ def grouped_weight_gradients(csr, freq, attenuation, weights, *, dtype=torch.flo
                 C.byref(sc), L.ptr(csr.offsets), L.ptr(csr.x6), L.ptr(csr.grad4), L.ptr(csr.relu_masks), R, int(segment_size),
                 precisions[operand_dtype], float(operand_scale), *(L.ptr(g) for g in grads), L.ptr(scratch), nbytes,
                 C.byref(word), st), "mlpsp_weight_gradients")
+        if word.value & 4:
+            raise ValueError("CSR offsets must be non-negative, ascending and end within the records")
         if word.value & 2:
             raise RuntimeError("grouped_weight_gradients: a device-side wait gave up; results discarded")
         return grads, bool(word.value & 1)

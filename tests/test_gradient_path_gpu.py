@@ -98,3 +98,31 @@ def test_records_reverse_refuses_bad_offsets_and_ids():
         with pytest.raises(ValueError, match="pixel offsets"):
             primitive_records_reverse(ids, off, *args)
     primitive_records_reverse(ids, offsets, *args)          # the next call starts clean
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_weight_gradients_refuse_offsets_that_leave_the_records(dtype):
+    """Offsets past the rows, below zero or descending are found before an item or a record is touched; rows behind the last
+    offset are nobody's."""
+    from mlp_splatting_b200.primitive_csr import PrimitiveCSR
+    from mlp_splatting_b200.primitive_gemm import grouped_weight_gradients
+    counts = [40, 0, 1, 700, 129, 0, 330]
+    n, R, spare = len(counts), sum(counts), 77
+    g = torch.Generator(device=DEV)
+    g.manual_seed(17)
+    rnd = lambda *s: torch.randn(s, generator=g, device=DEV)
+    w = [rnd(n, 32, 72) * 0.2, rnd(n, 32), rnd(n, 32, 32) * 0.2, rnd(n, 32), rnd(n, 4, 32), rnd(n, 4)]
+    freq = torch.tensor(2.0 ** np.arange(6), device=DEV, dtype=torch.float32)
+    att = torch.exp(-0.5 * freq ** 2 * 1e-4)
+    x6, d3 = rnd(R + spare, 6), rnd(R + spare, 4) * 1e-3
+    offsets = torch.tensor(np.concatenate(([0], np.cumsum(counts))), device=DEV)
+    run = lambda off, rows: grouped_weight_gradients(PrimitiveCSR(off, None, x6[:rows], d3[:rows]), freq, att, w, dtype=dtype,
+                                                     segment_size=64)
+    want = run(offsets, R)
+    assert all(torch.equal(a, b) for a, b in zip(run(offsets, R + spare), want))
+    changed = lambda i, v: torch.cat([offsets[:i], offsets.new_tensor([v]), offsets[i + 1:]])
+    for off, rows in ((offsets, R - 1), (offsets, 1), (offsets, 0), (changed(n, R + 10**6), R), (changed(0, -5), R),
+                      (changed(4, 10), R), (changed(3, R), R), (changed(3, 2**40), R)):
+        with pytest.raises(ValueError, match="CSR offsets"):
+            run(off, rows)
+    assert all(torch.equal(a, b) for a, b in zip(run(offsets, R), want))          # the next call starts clean
