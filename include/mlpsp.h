@@ -342,7 +342,8 @@ int mlpsp_prepare_groups_static(const int64_t* offsets, int32_t n, int64_t segme
  * mlpsp_export_records; log_scales[n,3], quats[n,4] (unit); grad_rgb[pixels,3], grad_t[pixels] (adjoint of the
  * final transmittance); total_records = R = offsets[pixels].  Writes d4[R,4] (adjoints of the four pre-activation
  * MLP outputs) and the position / log-scale / quaternion gradients [n,3] [n,3] [n,4], which are zeroed first.
- * raw, d4 and quats must be 16-byte aligned. */
+ * raw, d4 and quats must be 16-byte aligned; the other arrays need their element's alignment only.
+ * Offsets or ids that break these rules leave d4 unwritten and the gradients zero. */
 int mlpsp_records_reverse(const int32_t* ids, const int64_t* offsets, const float* x6, const float* raw,
                           const float* log_scales, const float* quats, const float* grad_rgb, const float* grad_t,
                           int64_t pixels, int64_t total_records, int32_t n, float* d4, float* grad_pos,
@@ -350,8 +351,7 @@ int mlpsp_records_reverse(const int32_t* ids, const int64_t* offsets, const floa
 
 /* The same with the caller's scratch (mlpsp_records_reverse takes it from the stream's memory pool) and with the
  * argument checks on the device: *findings_host (HOST, or NULL) receives an OR of the bits below (0: none), for which
- * the call waits for the checks -- not for the gradients; with a bit set the outputs are undefined.  grad_quats must be
- * 16-byte aligned as well. */
+ * the call waits for the checks -- not for the gradients; with a bit set the outputs are undefined. */
 #define MLPSP_REVERSE_BAD_OFFSETS 1  /* offsets do not start at zero, end at total_records or ascend */
 #define MLPSP_REVERSE_BAD_IDS 2      /* an id outside [0, n) */
 int64_t mlpsp_records_reverse_scratch_bytes(int64_t total_records, int32_t n);

@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(kRevThreads, 3) k_reverse_geometry(
 
 __global__ void __launch_bounds__(128) k_reverse_finish(const float* __restrict__ acc, const float* __restrict__ logs,
                                                         const float* __restrict__ quats, int n, float* __restrict__ gp,
-                                                        float* __restrict__ gs, float* __restrict__ gq) {
+                                                        float* __restrict__ gs, float* __restrict__ gq, int gq_vec) {
   chain_wait();
   chain_release();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -295,7 +295,12 @@ __global__ void __launch_bounds__(128) k_reverse_finish(const float* __restrict_
   }
   float gquat[4];
   quat_adjoint(qt.x, qt.y, qt.z, qt.w, Gm, gquat);
-  *reinterpret_cast<float4*>(gq + (size_t)p * 4) = make_float4(gquat[0], gquat[1], gquat[2], gquat[3]);
+  if (gq_vec) {                      // the caller's rows are 16-byte aligned
+    *reinterpret_cast<float4*>(gq + (size_t)p * 4) = make_float4(gquat[0], gquat[1], gquat[2], gquat[3]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) gq[(size_t)p * 4 + i] = gquat[i];
+  }
 }
 
 // --------------------------------------------------------- grouped weight gradients ----
@@ -664,9 +669,8 @@ extern "C" int mlpsp_records_reverse_checked(const int32_t* ids, const int64_t* 
   MLPSP_REQUIRE(offsets && (n == 0 || (log_scales && quats && grad_pos && grad_log_scales && grad_quats)) &&
                     (pixels == 0 || (grad_rgb && grad_t)) && (total_records == 0 || (ids && x6 && raw && d4 && quats)),
                 MLPSP_E_ARG, "mlpsp_records_reverse: null pointer");
-  MLPSP_REQUIRE(((reinterpret_cast<uintptr_t>(raw) | reinterpret_cast<uintptr_t>(d4) | reinterpret_cast<uintptr_t>(quats) |
-                  reinterpret_cast<uintptr_t>(grad_quats)) & 15) == 0,
-                MLPSP_E_ARG, "mlpsp_records_reverse: raw, d4, quats and grad_quats must be 16-byte aligned");
+  MLPSP_REQUIRE(((reinterpret_cast<uintptr_t>(raw) | reinterpret_cast<uintptr_t>(d4) | reinterpret_cast<uintptr_t>(quats)) & 15) == 0,
+                MLPSP_E_ARG, "mlpsp_records_reverse: raw, d4 and quats must be 16-byte aligned");
   MLPSP_REQUIRE(scratch && scratch_bytes >= mlpsp_records_reverse_scratch_bytes(total_records, n), MLPSP_E_SCRATCH,
                 "mlpsp_records_reverse: scratch too small");
   cudaStream_t st = (cudaStream_t)stream;
@@ -696,7 +700,8 @@ extern "C" int mlpsp_records_reverse_checked(const int32_t* ids, const int64_t* 
                    kRevSmem, st, ids, x6, kw, quats,
                    total_records, acc, bad);
   }
-  if (n > 0) launch_chained(k_reverse_finish, dim3((n + 127) / 128), dim3(128), 0, st, acc, log_scales, quats, n, grad_pos, grad_log_scales, grad_quats);
+  if (n > 0) launch_chained(k_reverse_finish, dim3((n + 127) / 128), dim3(128), 0, st, acc, log_scales, quats, n, grad_pos, grad_log_scales, grad_quats,
+                            (reinterpret_cast<uintptr_t>(grad_quats) & 15) == 0 ? 1 : 0);
   MLPSP_CUDA_OK(cudaGetLastError());
   if (findings_host) {
     MLPSP_CUDA_OK(cudaEventSynchronize(ev));
@@ -709,11 +714,18 @@ extern "C" int mlpsp_records_reverse(const int32_t* ids, const int64_t* offsets,
                                      const float* log_scales, const float* quats, const float* grad_rgb,
                                      const float* grad_t, int64_t pixels, int64_t total_records, int32_t n, float* d4,
                                      float* grad_pos, float* grad_log_scales, float* grad_quats, void* stream) {
-  // the variant with the caller's scratch, which this signature has no room for: taken from the stream's pool
+  MLPSP_REQUIRE(pixels >= 0 && n >= 0, MLPSP_E_ARG, "mlpsp_records_reverse: negative size");
   MLPSP_REQUIRE(offsets && grad_pos && grad_log_scales && grad_quats, MLPSP_E_ARG, "mlpsp_records_reverse: null pointer");
-  const int64_t bytes = mlpsp_records_reverse_scratch_bytes(total_records, n);
-  MLPSP_REQUIRE(bytes >= 0, MLPSP_E_ARG, "mlpsp_records_reverse: negative size");
   cudaStream_t st = (cudaStream_t)stream;
+  if (pixels == 0) {             // nothing is read: zero gradients
+    MLPSP_CUDA_OK(cudaMemsetAsync(grad_pos, 0, sizeof(float) * 3 * (size_t)n, st));
+    MLPSP_CUDA_OK(cudaMemsetAsync(grad_log_scales, 0, sizeof(float) * 3 * (size_t)n, st));
+    return cuda_check(cudaMemsetAsync(grad_quats, 0, sizeof(float) * 4 * (size_t)n, st), "records_reverse");
+  }
+  MLPSP_REQUIRE(ids && x6 && raw && log_scales && quats && grad_rgb && grad_t && d4, MLPSP_E_ARG, "mlpsp_records_reverse: null pointer");
+  MLPSP_REQUIRE(total_records >= 0, MLPSP_E_ARG, "mlpsp_records_reverse: negative record count");
+  // the variant with the caller's scratch, which this signature has no room for: taken from the stream's pool
+  const int64_t bytes = mlpsp_records_reverse_scratch_bytes(total_records, n);
   char* work = nullptr;
   MLPSP_CUDA_OK(cudaMallocAsync(&work, bytes, st));
   const int rc = mlpsp_records_reverse_checked(ids, offsets, x6, raw, log_scales, quats, grad_rgb, grad_t, pixels, total_records, n,
