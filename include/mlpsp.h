@@ -375,9 +375,10 @@ int64_t mlpsp_grouped_gradient_floats(void);
  * loss_scale multiplies the adjoints before the cast and divides the sums after (the reference uses 4096 for
  * binary16, 1 otherwise).  *nonfinite: bit 0 = a sum is not finite -- the caller retries a mixed-precision call
  * with MLPSP_PRECISION_F32 and loss_scale 1 as primitive_gemm.py:64-98 does (the host mirror does);
- * bit 1 = a device-side wait gave up, results invalid; bit 2 = the offsets descend or leave the records, no gradients. */
-/* The segments follow from the offsets and segment_size, so the call plans them itself (seg_prim, seg_start, seg_offsets
- * and partial are checked and otherwise unused; its scratch comes from the stream's memory pool). */
+ * bit 1 = a device-side wait gave up, results invalid; bit 2 = the offsets descend or leave the records, or the layout
+ * does not belong to them: no gradients.
+ * Rows of partial that belong to a primitive's only segment are not written.  Work lists of 32 bytes per segment and per
+ * primitive come from the stream's memory pool. */
 int mlpsp_grouped_weight_gradients(const mlpsp_scene* scene, const int64_t* offsets, const float* x6, const float* d4,
                                    const int32_t* relu_masks, const int64_t* seg_prim, const int64_t* seg_start,
                                    const int64_t* seg_offsets, int64_t num_segments, int32_t segment_size,

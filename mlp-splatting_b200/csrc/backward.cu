@@ -12,7 +12,8 @@
 //   dW3 = D3^T H2, db3 = sum D3, dW2 = D2^T H1, db2 = sum D2, dW1 = D1^T E, db1 = sum D1.
 // A segment (at most segment_size records of one primitive) is summed by one CTA.  A primitive with one segment, the
 // usual case, gets its gradients straight from that CTA; the partial 3,524-vectors of the others are added in segment
-// order by a second kernel, so the result does not depend on scheduling.
+// order by a second kernel, so the result does not depend on scheduling.  mlpsp_weight_gradients plans the segments from
+// the offsets, mlpsp_grouped_weight_gradients takes the caller's.
 #include "frame.cuh"
 #include "vjp.cuh"
 
@@ -358,6 +359,59 @@ __global__ void __launch_bounds__(256) k_vjp_plan(const int64_t* __restrict__ of
   if (empty) multi[n - 1 - (base[3] + ee)].prim = p;
 }
 
+// The same lists from a layout that the caller has prepared: segment g is item g and, unless it is its primitive's only
+// one, partial row g.  A segment outside its primitive's records or list refuses the plan.
+__global__ void __launch_bounds__(256) k_vjp_plan_layout(const int64_t* __restrict__ offsets, int n, int segment_size,
+                                                         const int64_t* __restrict__ seg_prim, const int64_t* __restrict__ seg_start,
+                                                         const int64_t* __restrict__ seg_offsets, int G, VjpItem* __restrict__ items,
+                                                         VjpItem* __restrict__ multi, int32_t* __restrict__ counters) {
+  chain_wait();
+  chain_release();
+  __shared__ int warp_sums[32];
+  __shared__ int base[2];
+  const int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  bool ok = true;
+  if (t < G) {
+    const int64_t p = seg_prim[t], start = seg_start[t];
+    ok = p >= 0 && p < n;
+    if (ok) {
+      const int64_t begin = offsets[p], end = offsets[p + 1], g0 = seg_offsets[p], g1 = seg_offsets[p + 1];
+      ok = begin >= 0 && start >= begin && start < end && g0 <= t && t < g1;
+      VjpItem it = {};
+      it.start = start;
+      it.rows = (int)min((int64_t)segment_size, end - start);
+      it.prim = (int)p;
+      it.dest = g1 - g0 > 1 ? (int)t : -1;
+      items[t] = it;
+    }
+  }
+  VjpItem it = {};
+  it.prim = (int)t;
+  int listed = 0, empty = 0;
+  if (t < n) {
+    const int64_t g0 = seg_offsets[t], g1 = seg_offsets[t + 1];
+    if (g0 < 0 || g1 < g0 || g1 > G) {
+      ok = false;
+    } else {
+      it.start = g0;
+      it.rows = (int)(g1 - g0);
+      listed = it.rows > 1;
+      empty = it.rows == 0;
+    }
+  }
+  int tm, te;
+  const int em = block_exclusive_scan(listed, warp_sums, tm), ee = block_exclusive_scan(empty, warp_sums, te);
+  if (threadIdx.x == 0) {
+    base[0] = tm ? atomicAdd(counters + kVpMulti, tm) : 0;
+    base[1] = te ? atomicAdd(counters + kVpEmpty, te) : 0;
+    if (blockIdx.x == 0) counters[kVpItems] = G;
+  }
+  __syncthreads();
+  if (listed) multi[base[0] + em] = it;
+  if (empty) multi[n - 1 - (base[1] + ee)] = it;
+  if (!ok) atomicOr(counters + kVpFlag, kVpBadPlan);
+}
+
 // IEEE FP32 on the CUDA cores, sums in record order.  A CTA of 128 threads takes 64 records at a time; everything per
 // record lies transposed in shared memory ([quantity][record], rows of 68 floats: 16-byte reads of eight different rows
 // meet eight different bank groups), so that the record-major products (layers, adjoints) give a thread a tile of four
@@ -603,9 +657,30 @@ static VjpScratch vjp_scratch(int64_t R, int n, int segment_size) {
   return s;
 }
 
+// the kernels behind a plan: at most max_items segments, their partial rows added up
+static int run_vjp_plan(const mlpsp_scene* sc, const float* x6, const float* d4, const int32_t* masks, const VjpItem* items,
+                        int64_t max_items, const VjpItem* multi, int32_t* counters, int precision, float loss_scale,
+                        const VjpOut& out, float* partial, cudaStream_t st) {
+  const bool tc = max_items > 0 && precision != MLPSP_PRECISION_F32;
+  if (tc) {
+    const int rc = launch_grouped_vjp_tc(precision == MLPSP_PRECISION_BF16, x6, d4, masks, items, max_items, multi, counters, sc, loss_scale,
+                                         out, partial, st);
+    if (rc) return rc;
+  } else if (max_items > 0) {
+    static DeviceOnce attr_once;
+    if (attr_once.first())
+      MLPSP_CUDA_OK(cudaFuncSetAttribute(k_grouped_vjp, cudaFuncAttributeMaxDynamicSharedMemorySize, kGradSmem));
+    launch_chained(k_grouped_vjp, dim3((unsigned)std::min<int64_t>(max_items, (int64_t)sm_count() * kGfCtas)), dim3(kGfThreads), kGradSmem, st,
+                   x6, d4, masks, items, counters, sc->freq, sc->att, sc->W1, sc->b1, sc->W2, sc->b2, sc->W3, loss_scale, out, partial);
+  }
+  launch_chained(k_vjp_reduce, dim3((unsigned)std::min(sc->n, sm_count() * 8)), dim3(256), 0, st, multi, partial, out, sc->n, tc ? 0 : 1,
+                 vjp_aligned(out), counters);
+  return cuda_check(cudaGetLastError(), "weight_gradients");
+}
+
 static int weight_gradients(const mlpsp_scene* sc, const int64_t* offsets, const float* x6, const float* d4, const int32_t* masks,
                             int64_t R, int segment_size, int precision, float loss_scale, const VjpOut& out, void* scratch,
-                            int64_t scratch_bytes, int32_t* flag_host, int32_t* flag_dev, cudaStream_t st) {
+                            int64_t scratch_bytes, int32_t* flag_host, cudaStream_t st) {
   const VjpScratch L = vjp_scratch(R, sc->n, segment_size);
   MLPSP_REQUIRE(scratch && scratch_bytes >= L.bytes, MLPSP_E_SCRATCH, "mlpsp_weight_gradients: scratch needs %lld bytes", (long long)L.bytes);
   // Segments cut long primitives for the CTAs to share; where the records make many segments per CTA anyway, longer ones
@@ -622,31 +697,16 @@ static int weight_gradients(const mlpsp_scene* sc, const int64_t* offsets, const
   MLPSP_CUDA_OK(cudaMemsetAsync(counters, 0, 4 * kVpCounters, st));
   launch_chained(k_vjp_plan, dim3((sc->n + 255) / 256), dim3(256), 0, st, offsets, sc->n, R, segment_size, items, L.max_items,
                  multi, counters);
-  const bool tc = R > 0 && precision != MLPSP_PRECISION_F32;
-  if (tc) {
-    const int rc = launch_grouped_vjp_tc(precision == MLPSP_PRECISION_BF16, x6, d4, masks, items, L.max_items, multi, counters, sc, loss_scale,
-                                         out, partial, st);
-    if (rc) return rc;
-  } else if (R > 0) {
-    static DeviceOnce attr_once;
-    if (attr_once.first())
-      MLPSP_CUDA_OK(cudaFuncSetAttribute(k_grouped_vjp, cudaFuncAttributeMaxDynamicSharedMemorySize, kGradSmem));
-    launch_chained(k_grouped_vjp, dim3((unsigned)std::min<int64_t>(L.max_items, (int64_t)sm_count() * kGfCtas)), dim3(kGfThreads), kGradSmem, st,
-                   x6, d4, masks, items, counters, sc->freq, sc->att, sc->W1, sc->b1, sc->W2, sc->b2, sc->W3, loss_scale, out, partial);
-  }
-  launch_chained(k_vjp_reduce, dim3((unsigned)std::min(sc->n, sm_count() * 8)), dim3(256), 0, st, multi, partial, out, sc->n, tc ? 0 : 1,
-                 vjp_aligned(out), counters);
-  if (flag_dev) MLPSP_CUDA_OK(cudaMemcpyAsync(flag_dev, counters + kVpFlag, 4, cudaMemcpyDeviceToDevice, st));
-  if (flag_host) {
-    HostWords& hw = host_words();
-    cudaEvent_t ev = nullptr;
-    const int rc = hw.open(&ev);
-    if (rc) return rc;
-    MLPSP_CUDA_OK(cudaMemcpyAsync(hw.word, counters + kVpFlag, 4, cudaMemcpyDeviceToHost, st));
-    MLPSP_CUDA_OK(cudaEventRecord(ev, st));
-    MLPSP_CUDA_OK(cudaEventSynchronize(ev));
-    *flag_host = *static_cast<volatile int32_t*>(hw.word);
-  }
+  const int rc = run_vjp_plan(sc, x6, d4, masks, items, L.max_items, multi, counters, precision, loss_scale, out, partial, st);
+  if (rc) return rc;
+  HostWords& hw = host_words();
+  cudaEvent_t ev = nullptr;
+  const int opened = hw.open(&ev);
+  if (opened) return opened;
+  MLPSP_CUDA_OK(cudaMemcpyAsync(hw.word, counters + kVpFlag, 4, cudaMemcpyDeviceToHost, st));
+  MLPSP_CUDA_OK(cudaEventRecord(ev, st));
+  MLPSP_CUDA_OK(cudaEventSynchronize(ev));
+  *flag_host = *static_cast<volatile int32_t*>(hw.word);
   return cuda_check(cudaGetLastError(), "weight_gradients");
 }
 
@@ -736,15 +796,17 @@ extern "C" int mlpsp_records_reverse(const int32_t* ids, const int64_t* offsets,
 
 extern "C" int64_t mlpsp_grouped_gradient_floats(void) { return kGradLen; }
 
-static int check_gradient_args(const mlpsp_scene* sc, const float* d4, int64_t segment_size, int precision, float loss_scale,
-                               const char* who) {
+static int check_gradient_args(const mlpsp_scene* sc, int64_t segment_size, int precision, float loss_scale, const char* who) {
   MLPSP_REQUIRE(sc->hidden == kGH && sc->num_freq == 6, MLPSP_E_LIMIT,
-                "grouped backward requires the 72→32→32→4 architecture");
+                "grouped backward requires the 72->32->32->4 architecture");
   MLPSP_REQUIRE(sc->W1 && sc->b1 && sc->W2 && sc->b2 && sc->W3 && sc->freq && sc->att, MLPSP_E_ARG,
                 "%s: FP32 weights missing", who);
   MLPSP_REQUIRE(loss_scale > 0.f && segment_size > 0, MLPSP_E_ARG, "%s: bad loss scale, segment size or segment count", who);
   MLPSP_REQUIRE(precision == MLPSP_PRECISION_F32 || precision == MLPSP_PRECISION_F16 || precision == MLPSP_PRECISION_BF16,
                 MLPSP_E_ARG, "%s: unsupported operand precision %d", who, precision);
+  return MLPSP_OK;
+}
+static int check_gradient_rows(const float* d4, int precision, const char* who) {
   MLPSP_REQUIRE(precision == MLPSP_PRECISION_F32 || (reinterpret_cast<uintptr_t>(d4) & 15) == 0, MLPSP_E_ARG,
                 "%s: d4 must be 16-byte aligned", who);
   return MLPSP_OK;
@@ -760,7 +822,8 @@ extern "C" int mlpsp_weight_gradients(const mlpsp_scene* sc, const int64_t* offs
                                       float loss_scale, float* dW1, float* db1, float* dW2, float* db2, float* dW3, float* db3,
                                       void* scratch, int64_t scratch_bytes, int32_t* nonfinite_host, void* stream) {
   MLPSP_REQUIRE(sc && offsets && nonfinite_host && num_records >= 0, MLPSP_E_ARG, "mlpsp_weight_gradients: null pointer");
-  int rc = check_gradient_args(sc, d4, segment_size, precision, loss_scale, "mlpsp_weight_gradients");
+  int rc = check_gradient_args(sc, segment_size, precision, loss_scale, "mlpsp_weight_gradients");
+  if (!rc) rc = check_gradient_rows(d4, precision, "mlpsp_weight_gradients");
   if (rc) return rc;
   *nonfinite_host = 0;
   if (sc->n == 0) return MLPSP_OK;
@@ -769,7 +832,7 @@ extern "C" int mlpsp_weight_gradients(const mlpsp_scene* sc, const int64_t* offs
   MLPSP_REQUIRE(num_records / segment_size + sc->n < (1ll << 31), MLPSP_E_LIMIT, "mlpsp_weight_gradients: too many segments");
   const VjpOut out = {dW1, db1, dW2, db2, dW3, db3, kGH * kGIN, kGH, kGH * kGH, kGH, 4 * kGH, 4};
   return weight_gradients(sc, offsets, x6, d4, relu_masks, num_records, segment_size, precision, loss_scale, out, scratch,
-                          scratch_bytes, nonfinite_host, nullptr, (cudaStream_t)stream);
+                          scratch_bytes, nonfinite_host, (cudaStream_t)stream);
 }
 
 extern "C" int mlpsp_grouped_weight_gradients(const mlpsp_scene* sc, const int64_t* offsets, const float* x6,
@@ -778,26 +841,38 @@ extern "C" int mlpsp_grouped_weight_gradients(const mlpsp_scene* sc, const int64
                                               int32_t segment_size, int32_t precision, float loss_scale, float* partial,
                                               float* result, int32_t* nonfinite, void* stream) {
   MLPSP_REQUIRE(sc && offsets && result && nonfinite, MLPSP_E_ARG, "mlpsp_grouped_weight_gradients: null pointer");
+  int rc = check_gradient_args(sc, segment_size, precision, loss_scale, "mlpsp_grouped_weight_gradients");
+  if (rc) return rc;
   MLPSP_REQUIRE(num_segments >= 0 && num_segments < (1ll << 31), MLPSP_E_ARG,
                 "mlpsp_grouped_weight_gradients: bad loss scale, segment size or segment count");
   // every pointer a launch below reads is checked before the first CUDA call
   MLPSP_REQUIRE(sc->n == 0 || num_segments == 0 || (x6 && d4 && seg_prim && seg_start && seg_offsets && partial),
                 MLPSP_E_ARG, "mlpsp_grouped_weight_gradients: null pointer");
-  int rc = check_gradient_args(sc, d4, segment_size, precision, loss_scale, "mlpsp_grouped_weight_gradients");
-  if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   MLPSP_CUDA_OK(cudaMemsetAsync(nonfinite, 0, 4, st));
   if (sc->n == 0) return MLPSP_OK;
-  // The segments follow from the offsets and the segment size, so the launch plans them itself; its scratch, which this
-  // signature has no room for, comes from the stream's pool.  num_segments * segment_size bounds the record count.
-  const int64_t records = num_segments * segment_size;
-  const int64_t bytes = vjp_scratch(records, sc->n, segment_size).bytes;
+  if (num_segments == 0)       // no records at all: every primitive's gradient row is zero
+    return cuda_check(cudaMemsetAsync(result, 0, sizeof(float) * (size_t)sc->n * kGradLen, st), "grouped_weight_gradients");
+  rc = check_gradient_rows(d4, precision, "mlpsp_grouped_weight_gradients");
+  if (rc) return rc;
+  // the work lists, 32 bytes per segment and primitive, have no room in this signature: they come from the stream's pool
+  const int64_t item_bytes = align_up((int64_t)sizeof(VjpItem) * num_segments, 256);
   char* work = nullptr;
-  MLPSP_CUDA_OK(cudaMallocAsync(&work, bytes, st));
+  MLPSP_CUDA_OK(cudaMallocAsync(&work, 256 + item_bytes + (int64_t)sizeof(VjpItem) * sc->n, st));
+  int32_t* counters = reinterpret_cast<int32_t*>(work);
+  VjpItem* items = reinterpret_cast<VjpItem*>(work + 256);
+  VjpItem* multi = reinterpret_cast<VjpItem*>(work + 256 + item_bytes);
   float* r = result;
   const VjpOut out = {r + kOW1, r + kOb1, r + kOW2, r + kOb2, r + kOW3, r + kOb3, kGradLen, kGradLen, kGradLen, kGradLen, kGradLen, kGradLen};
-  rc = weight_gradients(sc, offsets, x6, d4, relu_masks, records, segment_size, precision, loss_scale, out, work, bytes, nullptr,
-                        nonfinite, st);
+  LaunchScope scope(kKMisc, 3, st);
+  rc = cuda_check(cudaMemsetAsync(counters, 0, 4 * kVpCounters, st), "grouped_weight_gradients");
+  if (!rc)
+    rc = cuda_check(launch_chained(k_vjp_plan_layout, dim3((unsigned)((std::max<int64_t>(num_segments, sc->n) + 255) / 256)), dim3(256), 0,
+                                   st, offsets, sc->n, segment_size, seg_prim, seg_start, seg_offsets, (int)num_segments, items, multi,
+                                   counters), "grouped_weight_gradients");
+  if (!rc)
+    rc = run_vjp_plan(sc, x6, d4, relu_masks, items, num_segments, multi, counters, precision, loss_scale, out, partial, st);
+  if (!rc) rc = cuda_check(cudaMemcpyAsync(nonfinite, counters + kVpFlag, 4, cudaMemcpyDeviceToDevice, st), "grouped_weight_gradients");
   cudaFreeAsync(work, st);
   return rc;
 }

@@ -50,3 +50,65 @@ def test_records_reverse_takes_gradients_of_any_alignment(shift):
     # pixels, but no arrays to read or write
     assert lib.mlpsp_records_reverse(None, L.ptr(offsets), *[None] * 6, P, 0, n, None, *(L.ptr(t) for t in (gp, gs, gq)),
                                      _stream()) == -1
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("with_masks", [True, False])
+def test_grouped_weight_gradients_over_a_prepared_layout(dtype, with_masks):
+    """The same bits as the call that plans its own segments; the caller's partial rows hold the sums of the primitives of
+    several segments and nothing else; a layout that does not belong to the offsets gives the flag and no access."""
+    from mlp_splatting_b200 import _lib as L
+    from mlp_splatting_b200.primitive_csr import PrimitiveCSR
+    from mlp_splatting_b200.primitive_gemm import grouped_weight_gradients, prepare_groups
+    counts = [0, 1, 64, 65, 0, 129, 700, 3, 0] + [2] * 600         # several blocks of the planning kernel
+    n, R, seg = len(counts), sum(counts), 64
+    g = torch.Generator(device=DEV)
+    g.manual_seed(23)
+    rnd = lambda *s: torch.randn(s, generator=g, device=DEV)
+    w = [rnd(n, 32, 72) * 0.2, rnd(n, 32) * 0.1, rnd(n, 32, 32) * 0.2, rnd(n, 32) * 0.1, rnd(n, 4, 32) * 0.2, rnd(n, 4) * 0.1]
+    x6, d3 = rnd(R, 6), rnd(R, 4) * 1e-3
+    masks = torch.randint(-2**31, 2**31 - 1, (R, 2), generator=g, device=DEV, dtype=torch.int32) if with_masks else None
+    freq = torch.tensor(2.0 ** np.arange(6), device=DEV, dtype=torch.float32)
+    att = torch.exp(-0.5 * freq ** 2 * 1e-4)
+    csr = PrimitiveCSR(torch.tensor(np.concatenate(([0], np.cumsum(counts))), device=DEV), None, x6, d3, masks)
+    layout = prepare_groups(csr, seg)
+    scale = 4096.0 if dtype == torch.float16 else 1.0
+    want = grouped_weight_gradients(csr, freq, att, w, dtype=dtype, segment_size=seg, loss_scale=scale, groups=layout)
+    want = torch.cat([t.flatten(1) for t in want], 1)
+    lib = L.load()
+    row = int(lib.mlpsp_grouped_gradient_floats())
+    sc = L.Scene()
+    sc.n, sc.hidden, sc.num_freq = n, 32, 6
+    sc.W1, sc.b1, sc.W2, sc.b2, sc.W3, sc.b3 = (L.ptr(t) for t in w)
+    sc.freq, sc.att = L.ptr(freq), L.ptr(att)
+    precision = {torch.float32: L.PRECISION_F32, torch.float16: L.PRECISION_F16, torch.bfloat16: L.PRECISION_BF16}[dtype]
+
+    def run(prims, starts, offs, G):
+        partial = torch.full((max(G, 1), row), float("nan"), device=DEV)
+        result = torch.full((n, row), float("nan"), device=DEV)
+        flag = torch.full((1,), -1, device=DEV, dtype=torch.int32)
+        L.check(lib.mlpsp_grouped_weight_gradients(
+            C.byref(sc), *(L.ptr(t) for t in (csr.offsets, x6, d3, masks, prims, starts, offs)), G, seg, precision, scale,
+            L.ptr(partial), L.ptr(result), L.ptr(flag), _stream()), "mlpsp_grouped_weight_gradients")
+        return partial, result, int(flag)
+
+    prims, starts, offs = layout.primitives, layout.starts, layout.offsets
+    G = prims.numel()
+    partial, result, flag = run(prims, starts, offs, G)
+    assert flag == 0 and torch.equal(result, want)
+    several = ((offs[1:] - offs[:-1]) > 1)[prims]
+    assert 0 < int(several.sum()) < G
+    assert torch.isfinite(partial[several]).all() and partial[~several].isnan().all()
+    _partial, result, flag = run(prims, starts, offs, 0)
+    assert flag == 0 and (result == 0).all()
+
+    def changed(t, i, v):
+        t = t.clone()
+        t[i] = v
+        return t
+
+    last = int(csr.offsets[-1])
+    for bad in ((changed(prims, 3, n), starts, offs), (changed(prims, 3, -1), starts, offs), (changed(prims, 0, 2), starts, offs),
+                (prims, changed(starts, 1, last), offs), (prims, changed(starts, 1, -1), offs),
+                (prims, starts, changed(offs, n, G + 1)), (prims, starts, changed(offs, 5, -1)), (prims, starts, changed(offs, 6, G))):
+        assert run(*bad, G)[2] & 4
