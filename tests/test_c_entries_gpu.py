@@ -112,3 +112,75 @@ def test_grouped_weight_gradients_over_a_prepared_layout(dtype, with_masks):
                 (prims, changed(starts, 1, last), offs), (prims, changed(starts, 1, -1), offs),
                 (prims, starts, changed(offs, n, G + 1)), (prims, starts, changed(offs, 5, -1)), (prims, starts, changed(offs, 6, G))):
         assert run(*bad, G)[2] & 4
+
+
+@pytest.mark.parametrize("n,R", [(1, 0), (1, 5), (7, 4097), (300, 10_000), (70_000, 50_001)])
+def test_group_records_against_a_stable_sort(n, R):
+    from mlp_splatting_b200 import _lib as L
+    g = torch.Generator(device=DEV)
+    g.manual_seed(n + R)
+    ids = torch.randint(0, n, (R,), generator=g, device=DEV, dtype=torch.int32)
+    offsets = torch.full((n + 1,), -1, device=DEV, dtype=torch.int64)
+    order = torch.full((R,), -1, device=DEV, dtype=torch.int64)
+    lib = L.load()
+    nbytes = int(lib.mlpsp_group_records_scratch_bytes(R, n))
+    scratch = torch.empty(nbytes, device=DEV, dtype=torch.uint8)
+    call = lambda size: lib.mlpsp_group_records(L.ptr(ids), R, n, L.ptr(offsets), L.ptr(order), L.ptr(scratch), size, _stream())
+    assert call(nbytes - 1) == -2            # the scratch is checked
+    L.check(call(nbytes), "mlpsp_group_records")
+    want = torch.zeros(n + 1, device=DEV, dtype=torch.int64)
+    want[1:] = torch.bincount(ids, minlength=n).cumsum(0)
+    assert torch.equal(offsets, want) and torch.equal(order, torch.argsort(ids, stable=True))
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("W,H", [(128, 96), (61, 43)])
+def test_render_frame_gives_the_image_of_the_fused_call(precision, W, H):
+    """Unit rays, host matrices and a status block that the caller resets, against the call that does these itself."""
+    from mlp_splatting_b200 import _lib as L
+    from mlp_splatting_b200.engine import FrameRenderer, PackedScene, normalize_rows
+    from tests.helpers import WKEYS, small_case
+    scene, cam = small_case(n=2000, W=W, H=H)
+    ps = PackedScene(scene["positions"], scene["log_scales"], scene["quats"], *[scene[k] for k in WKEYS], scene["freq"],
+                     scene["att"], device=DEV)
+    r = FrameRenderer(W, H, device=DEV)
+    ro, rd = torch.from_numpy(cam["rays_o"]).to(DEV), torch.from_numpy(cam["rays_d"]).to(DEV)
+    args = dict(view=cam["view"], proj=cam["proj"], precision=precision, waves=[32, 32, 64, 128, 256, 1536])
+    want = [t.clone() for t in r.render(ps, ro, rd, 5e-3, **args)]
+    words = r.status_host.clone()
+    assert float(want[1].max()) > 0.5
+    unit = normalize_rows(rd)
+    f = r._frame(ps, ro, unit, 5e-3, precision, cam["view"], cam["proj"], None, False, False, args["waves"])
+    r.rgb.fill_(float("nan"))
+    r.alpha.fill_(float("nan"))
+    lib = L.load()
+    L.check(lib.mlpsp_status_reset(L.ptr(r.status), _stream()), "mlpsp_status_reset")
+    L.check(lib.mlpsp_render_frame(C.byref(ps.c), C.byref(f), _stream()), "mlpsp_render_frame")
+    assert torch.equal(r.rgb, want[0]) and torch.equal(r.alpha, want[1])
+    assert torch.equal(r.status.cpu(), words)
+
+
+def test_export_records_in_one_call_gives_the_rows_of_the_counted_export():
+    from mlp_splatting_b200 import _lib as L
+    from mlp_splatting_b200.engine import FrameRenderer, PackedScene
+    from tests.helpers import WKEYS, small_case
+    scene, cam = small_case(n=1500, W=61, H=43)
+    ps = PackedScene(scene["positions"], scene["log_scales"], scene["quats"], *[scene[k] for k in WKEYS], scene["freq"],
+                     scene["att"], device=DEV)
+    r = FrameRenderer(61, 43, device=DEV)
+    ro, rd = torch.from_numpy(cam["rays_o"]).to(DEV), torch.from_numpy(cam["rays_d"]).to(DEV)
+    want = r.render_records(ps, ro, rd, 5e-3, view=cam["view"], proj=cam["proj"])[2:]
+    R = want[0].numel()
+    assert R > 1000
+    got = [torch.full_like(t, -7) for t in want]
+    f, _ = r._last_frame
+    total, worst = C.c_int64(-1), C.c_int32(-1)
+    lib = L.load()
+    call = lambda room: L.check(lib.mlpsp_export_records(
+        C.byref(ps.c), C.byref(f), L.ptr(got[5]), *(L.ptr(t) for t in got[:5]), room, 512, C.byref(total), C.byref(worst),
+        _stream()), "mlpsp_export_records")
+    call(R - 1)                                   # no room: the count and the offsets only
+    assert total.value == R and torch.equal(got[5], want[5]) and all((t == -7).all() for t in got[:5])
+    call(R)
+    assert total.value == R and worst.value == int((want[5][1:] - want[5][:-1]).max())
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
