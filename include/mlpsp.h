@@ -287,7 +287,8 @@ int mlpsp_export_records(const mlpsp_scene* scene, const mlpsp_frame* frame, int
                          int32_t max_hits, int64_t* total_host, int32_t* worst_host, void* stream);
 
 /* The same rows behind a call of mlpsp_export_records on this frame that only counted (no outputs): total is the
- * count it returned, every non-NULL array has room for it.  Does not count again and does not synchronise. */
+ * count it returned, every non-NULL array has room for it (no more rows are written than the frame has records).  Does not
+ * count again and does not synchronise. */
 int mlpsp_export_counted_records(const mlpsp_scene* scene, const mlpsp_frame* frame, int32_t* ids, float* x6, float* raw,
                                  int32_t* relu_masks, float* gates, int64_t total, void* stream);
 

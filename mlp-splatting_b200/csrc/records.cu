@@ -1669,11 +1669,11 @@ __global__ void __launch_bounds__(64) k_export(const ExportArgs a) {
   }
 }
 
-// the rows of the records that k_export has placed
+// the rows of the records that k_export has placed: no more than the frame has, whatever total the caller gives
 __global__ void __launch_bounds__(256) k_export_rows(const ExportArgs a, int64_t total) {
   if (a.status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
   const int64_t r = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  if (r >= total) return;
+  if (r >= total || r >= a.px_off[(size_t)a.W * a.H]) return;
   const int2 at = *reinterpret_cast<const int2*>(a.raw + r * 8);
   export_row(a, (uint32_t)at.x, a.ids[r], at.y, r);
 }

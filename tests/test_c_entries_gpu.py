@@ -184,3 +184,8 @@ def test_export_records_in_one_call_gives_the_rows_of_the_counted_export():
     call(R)
     assert total.value == R and worst.value == int((want[5][1:] - want[5][:-1]).max())
     assert all(torch.equal(a, b) for a, b in zip(got, want))
+    # a total beyond the frame's records: no row behind the last one is made
+    more = [torch.full((R + 1000, *t.shape[1:]), -7, device=DEV, dtype=t.dtype) for t in want[:5]]
+    L.check(lib.mlpsp_export_counted_records(C.byref(ps.c), C.byref(f), *(L.ptr(t) for t in more), R + 1000, _stream()),
+            "mlpsp_export_counted_records")
+    assert all(torch.equal(a[:R], b) and (a[R:] == -7).all() for a, b in zip(more, want))
