@@ -235,7 +235,7 @@ extern "C" int mlpsp_sort_tiles(const mlpsp_scene* sc, const mlpsp_frame* fr, fl
   rc = get_scratch(sc, fr, s, "mlpsp_sort_tiles");
   if (rc) return rc;
   // the active-tile list of the wave loop is free while the lists are being sorted
-  return launch_sort(sc, fr, keys_out, (cudaStream_t)stream, false, s.active[1], s.counters + kCtrScratch + 2);
+  return launch_sort(sc, fr, keys_out, (cudaStream_t)stream, false, s.counters + kCtrScratch + 2);
 }
 
 extern "C" int mlpsp_hit_masks(const mlpsp_scene* sc, const mlpsp_frame* fr, uint64_t* mask_geo, void* stream) {
@@ -278,7 +278,7 @@ static int render_frame(const mlpsp_scene* sc, const mlpsp_frame* fr, const floa
   }
   rc = launch_bin(sc, fr, s, st, /*order_lists=*/false, pretest, view_dev, proj_dev);
   if (rc) return rc;
-  rc = launch_sort(sc, fr, nullptr, st, /*unordered_input=*/true, s.active[1], s.counters + kCtrScratch + 2,
+  rc = launch_sort(sc, fr, nullptr, st, /*unordered_input=*/true, s.counters + kCtrScratch + 2,
                    pretest ? s.tile_len : nullptr);
   if (rc) return rc;
   return render_sorted_checked(sc, fr, s, st, pretest);
@@ -332,7 +332,7 @@ extern "C" int mlpsp_render_frames(const mlpsp_scene* sc, const mlpsp_frame* fra
     if (rc) return rc;
     rc = launch_bin(sc, fr, s, st, /*order_lists=*/false, pretest);
     if (rc) return rc;
-    rc = launch_sort(sc, fr, nullptr, st, /*unordered_input=*/true, s.active[1], s.counters + kCtrScratch + 2,
+    rc = launch_sort(sc, fr, nullptr, st, /*unordered_input=*/true, s.counters + kCtrScratch + 2,
                      pretest ? s.tile_len : nullptr);
     if (rc) return rc;
   }

@@ -229,11 +229,11 @@ int launch_frame_begin(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scrat
 int launch_bin_mosaic(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, const int32_t* tile_view,
                       const float* views_host, int num_views, cudaStream_t st);
 int launch_bin_raycone(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, cudaStream_t st);
-// long_list [T] / long_count [2]: device scratch (tiles that take the block-wide sort, their number, a tile cursor)
+// cursors [2]: device scratch, the tile cursors of the two sort kernels
 // list_len (optional): candidates actually present at the front of every tile's span (pre-tested binning);
 // the rest of the span is filled with -1 in sorted_prims
 int launch_sort(const mlpsp_scene* sc, const mlpsp_frame* fr, float* keys_out, cudaStream_t st, bool unordered_input,
-                int32_t* long_list, int32_t* long_count, const int32_t* list_len = nullptr);
+                int32_t* cursors, const int32_t* list_len = nullptr);
 int launch_hit_masks(const mlpsp_scene* sc, const mlpsp_frame* fr, uint64_t* mask_geo, cudaStream_t st);
 // lists_refined: launch_frame_begin has prepared the frame and s.tile_len holds the traversal length of every tile
 int launch_render_sorted(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, cudaStream_t st,

@@ -814,134 +814,131 @@ __global__ void __launch_bounds__(64) k_composite(
   float gtr = 0.f, gtg = 0.f, gtb = 0.f;
   if (STATS && tp.valid) { gtr = ps.gt_rgb[(size_t)tp.pix * 3]; gtg = ps.gt_rgb[(size_t)tp.pix * 3 + 1]; gtb = ps.gt_rgb[(size_t)tp.pix * 3 + 2]; }
   if (!STATS) {
-  for (int i0 = wlo; i0 < whi && __any_sync(0xffffffffu, act); i0 += 32) {
-    const int idx = i0 + lane;
-    uint32_t mine = 0u, first = 0u;       // pair i0 + lane: this half's hit mask and the slot of its first record
-    if (idx < whi) {
-      const uint2 mm = *reinterpret_cast<const uint2*>(masks32 + 2 * (size_t)(s + idx));
-      mine = half ? mm.y : mm.x;
-      first = pair_base[s + idx] + (half ? __popc(mm.x) : 0);
-    }
-    // A pixel meets about one candidate in eight, so every lane walks its own hits (bit j of todo: pair i0 + j) instead of
-    // the warp walking the pairs: four of a lane's records are requested at a time, whether its pixel will still be live or
-    // not, then blended in list order.
-    uint32_t todo = transpose32(mine), taken = 0u;
-    if (!act) todo = 0u;
-    while (__any_sync(0xffffffffu, todo != 0u)) {
-      float4 rr[4];
-      uint32_t slot4[4], bit4[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int j = todo ? __ffs(todo) - 1 : lane;
-        bit4[u] = todo & (0u - todo);
-        todo &= todo - 1u;
-        const uint32_t mj = __shfl_sync(0xffffffffu, mine, j), fj = __shfl_sync(0xffffffffu, first, j);
-        slot4[u] = fj + __popc(mj & lt);
-        rr[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (bit4[u]) rr[u] = rec_out[slot4[u]];
+    for (int i0 = wlo; i0 < whi && __any_sync(0xffffffffu, act); i0 += 32) {
+      const int idx = i0 + lane;
+      uint32_t mine = 0u, first = 0u;       // pair i0 + lane: this half's hit mask and the slot of its first record
+      if (idx < whi) {
+        const uint2 mm = *reinterpret_cast<const uint2*>(masks32 + 2 * (size_t)(s + idx));
+        mine = half ? mm.y : mm.x;
+        first = pair_base[s + idx] + (half ? __popc(mm.x) : 0);
       }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const bool take = act && bit4[u];
-        if (take) {
-          const float4 r = rr[u];
-          const float w = st.w * r.w;
-          st.x = fmaf(w, r.x, st.x); st.y = fmaf(w, r.y, st.y); st.z = fmaf(w, r.z, st.z);
-          if (depth_t) { dp.x = fmaf(w, rec_t[slot4[u]], dp.x); dp.y += w; }
-          if (rec_w) rec_w[slot4[u]] = w;
-          if (rec_tr) rec_tr[slot4[u]] = st.w;
-          st.w *= (1.f - r.w);
-          act = st.w >= MLPSP_TERM;
-          taken |= bit4[u];
-        }
-      }
+      // A pixel meets about one candidate in eight, so every lane walks its own hits (bit j of todo: pair i0 + j) instead of
+      // the warp walking the pairs: four of a lane's records are requested at a time, whether its pixel will still be live or
+      // not, then blended in list order.
+      uint32_t todo = transpose32(mine), taken = 0u;
       if (!act) todo = 0u;
+      while (__any_sync(0xffffffffu, todo != 0u)) {
+        float4 rr[4];
+        uint32_t slot4[4], bit4[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int j = todo ? __ffs(todo) - 1 : lane;
+          bit4[u] = todo & (0u - todo);
+          todo &= todo - 1u;
+          const uint32_t mj = __shfl_sync(0xffffffffu, mine, j), fj = __shfl_sync(0xffffffffu, first, j);
+          slot4[u] = fj + __popc(mj & lt);
+          rr[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (bit4[u]) rr[u] = rec_out[slot4[u]];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const bool take = act && bit4[u];
+          if (take) {
+            const float4 r = rr[u];
+            const float w = st.w * r.w;
+            st.x = fmaf(w, r.x, st.x); st.y = fmaf(w, r.y, st.y); st.z = fmaf(w, r.z, st.z);
+            if (depth_t) { dp.x = fmaf(w, rec_t[slot4[u]], dp.x); dp.y += w; }
+            if (rec_w) rec_w[slot4[u]] = w;
+            if (rec_tr) rec_tr[slot4[u]] = st.w;
+            st.w *= (1.f - r.w);
+            act = st.w >= MLPSP_TERM;
+            taken |= bit4[u];
+          }
+        }
+        if (!act) todo = 0u;
+      }
+      used += __popc(taken);
+      if (mask_used32) {
+        const uint32_t um = transpose32(taken);
+        if (um) mask_used32[2 * (size_t)(s + idx) + half] = um;
+      }
     }
-    used += __popc(taken);
-    if (mask_used32) {
-      const uint32_t um = transpose32(taken);
-      if (um) mask_used32[2 * (size_t)(s + idx) + half] = um;
-    }
-  }
     used = __reduce_add_sync(0xffffffffu, used);
   } else {
-  // statistics: the warp walks the pairs together, so that a pair's contributions are summed before they go to memory
-  for (int i0 = wlo; i0 < whi && __any_sync(0xffffffffu, act); i0 += 32) {
-    const int idx = i0 + lane;
-    uint2 mm = make_uint2(0u, 0u);
-    uint32_t bb = 0;
-    if (idx < whi) {
-      mm = *reinterpret_cast<const uint2*>(masks32 + 2 * (size_t)(s + idx));
-      bb = pair_base[s + idx];
-    }
-    const int cnt = min(32, whi - i0);
-    bool stop = false;
-    // four pairs at a time: the records a lane may need are requested first (whether its pixel is still live or
-    // not), then blended in list order, so the gathers of a batch overlap instead of forming a chain
-    for (int j0 = 0; j0 < cnt && !stop; j0 += 4) {
-      float4 rr[4];
-      uint32_t slot4[4], m04[4], mine4[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int j = min(j0 + u, 31);
-        const uint32_t m0 = __shfl_sync(0xffffffffu, mm.x, j), m1 = __shfl_sync(0xffffffffu, mm.y, j);
-        const uint32_t b = __shfl_sync(0xffffffffu, bb, j);
-        const uint32_t mine = (j0 + u < cnt) ? (half ? m1 : m0) : 0u;
-        m04[u] = m0; mine4[u] = mine;
-        slot4[u] = b + (half ? __popc(m0) : 0) + __popc(mine & lt);
-        rr[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if ((mine >> lane) & 1u) rr[u] = rec_out[slot4[u]];
+    // statistics: the warp walks the pairs together, so that a pair's contributions are summed before they go to memory
+    for (int i0 = wlo; i0 < whi && __any_sync(0xffffffffu, act); i0 += 32) {
+      const int idx = i0 + lane;
+      uint2 mm = make_uint2(0u, 0u);
+      uint32_t bb = 0;
+      if (idx < whi) {
+        mm = *reinterpret_cast<const uint2*>(masks32 + 2 * (size_t)(s + idx));
+        bb = pair_base[s + idx];
       }
+      const int cnt = min(32, whi - i0);
+      bool stop = false;
+      // four pairs at a time: the records a lane may need are requested first (whether its pixel is still live or
+      // not), then blended in list order, so the gathers of a batch overlap instead of forming a chain
+      for (int j0 = 0; j0 < cnt && !stop; j0 += 4) {
+        float4 rr[4];
+        uint32_t slot4[4], mine4[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int j = j0 + u;
-        const uint32_t mine = mine4[u];
-        if (stop || mine == 0u) continue;
-        const bool take = act && ((mine >> lane) & 1u);
-        float sw = 0.f, swerr = 0.f;
-        if (take) {
-          const uint32_t slot = slot4[u];
-          const float4 r = rr[u];
-          const float w = st.w * r.w;
-          st.x = fmaf(w, r.x, st.x); st.y = fmaf(w, r.y, st.y); st.z = fmaf(w, r.z, st.z);
-          if (STATS) {
+        for (int u = 0; u < 4; ++u) {
+          const int j = min(j0 + u, 31);
+          const uint32_t m0 = __shfl_sync(0xffffffffu, mm.x, j), m1 = __shfl_sync(0xffffffffu, mm.y, j);
+          const uint32_t b = __shfl_sync(0xffffffffu, bb, j);
+          const uint32_t mine = (j0 + u < cnt) ? (half ? m1 : m0) : 0u;
+          mine4[u] = mine;
+          slot4[u] = b + (half ? __popc(m0) : 0) + __popc(mine & lt);
+          rr[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if ((mine >> lane) & 1u) rr[u] = rec_out[slot4[u]];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int j = j0 + u;
+          const uint32_t mine = mine4[u];
+          if (stop || mine == 0u) continue;
+          const bool take = act && ((mine >> lane) & 1u);
+          float sw = 0.f, swerr = 0.f;
+          if (take) {
+            const uint32_t slot = slot4[u];
+            const float4 r = rr[u];
+            const float w = st.w * r.w;
+            st.x = fmaf(w, r.x, st.x); st.y = fmaf(w, r.y, st.y); st.z = fmaf(w, r.z, st.z);
             sw = w;
             if (w > 1e-1f) swerr = w * (fabsf(st.x - gtr) + fabsf(st.y - gtg) + fabsf(st.z - gtb));
+            if (depth_t) { dp.x = fmaf(w, rec_t[slot], dp.x); dp.y += w; }
+            if (rec_w) rec_w[slot] = w;
+            if (rec_tr) rec_tr[slot] = st.w;
+            st.w *= (1.f - r.w);
+            act = st.w >= MLPSP_TERM;
           }
-          if (depth_t) { dp.x = fmaf(w, rec_t[slot], dp.x); dp.y += w; }
-          if (rec_w) rec_w[slot] = w;
-          if (rec_tr) rec_tr[slot] = st.w;
-          st.w *= (1.f - r.w);
-          act = st.w >= MLPSP_TERM;
-        }
-        const uint32_t um = __ballot_sync(0xffffffffu, take);
-        if (STATS && um) {
-          // this half-tile's share of the pair's statistics: one atomic per array
-          const int n_hit = __popc(__ballot_sync(0xffffffffu, sw > 1e-8f));
-          const int n_con = __popc(__ballot_sync(0xffffffffu, sw > 1e-1f));
-          float tsum = sw, tmax = sw, terr = swerr;
+          const uint32_t um = __ballot_sync(0xffffffffu, take);
+          if (um) {
+            // this half-tile's share of the pair's statistics: one atomic per array
+            const int n_hit = __popc(__ballot_sync(0xffffffffu, sw > 1e-8f));
+            const int n_con = __popc(__ballot_sync(0xffffffffu, sw > 1e-1f));
+            float tsum = sw, tmax = sw, terr = swerr;
 #pragma unroll
-          for (int o = 16; o > 0; o >>= 1) {
-            tsum += __shfl_xor_sync(0xffffffffu, tsum, o);
-            tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
-            terr += __shfl_xor_sync(0xffffffffu, terr, o);
+            for (int o = 16; o > 0; o >>= 1) {
+              tsum += __shfl_xor_sync(0xffffffffu, tsum, o);
+              tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
+              terr += __shfl_xor_sync(0xffffffffu, terr, o);
+            }
+            if (lane == 0) {
+              const int p = ps.sorted_prims[s + i0 + j];
+              atomicAdd(ps.sum_w + p, tsum);
+              atomicMax(reinterpret_cast<int*>(ps.max_w + p), __float_as_int(tmax));   // w >= 0: bit order = value order
+              if (n_hit) atomicAdd(ps.hits + p, n_hit);
+              if (n_con) { atomicAdd(ps.contrib + p, n_con); atomicAdd(ps.sum_werr + p, terr); }
+            }
           }
-          if (lane == 0) {
-            const int p = ps.sorted_prims[s + i0 + j];
-            atomicAdd(ps.sum_w + p, tsum);
-            atomicMax(reinterpret_cast<int*>(ps.max_w + p), __float_as_int(tmax));   // w >= 0: bit order = value order
-            if (n_hit) atomicAdd(ps.hits + p, n_hit);
-            if (n_con) { atomicAdd(ps.contrib + p, n_con); atomicAdd(ps.sum_werr + p, terr); }
+          if (um) {
+            if (lane == 0) { used += __popc(um); if (mask_used32) mask_used32[2 * (size_t)(s + i0 + j) + half] = um; }
+            if (!__any_sync(0xffffffffu, act)) stop = true;
           }
         }
-        if (um) {
-          if (lane == 0) { used += __popc(um); if (mask_used32) mask_used32[2 * (size_t)(s + i0 + j) + half] = um; }
-          if (!__any_sync(0xffffffffu, act)) stop = true;
-        }
-        (void)m04;
       }
     }
-  }
   }
   if (tp.valid) {
     px_state[tp.pix] = st;

@@ -274,8 +274,8 @@ template <bool IDSORT>
 __global__ void __launch_bounds__(256, 6) k_sort_tiles(
     const float* __restrict__ rays_o, const float* __restrict__ rays_d, const float4* __restrict__ geom, int n,
     const int32_t* __restrict__ tile_offsets, const int32_t* tile_prims, int W, int H, int ts, int ntx, int T, int cap,
-    int32_t* __restrict__ sorted_prims, float* __restrict__ keys_out, int key_mode, int32_t* __restrict__ long_list,
-    int32_t* __restrict__ long_count, const int32_t* __restrict__ list_len, int32_t* __restrict__ status) {
+    int32_t* __restrict__ sorted_prims, float* __restrict__ keys_out, int key_mode, int32_t* __restrict__ cursor,
+    const int32_t* __restrict__ list_len, int32_t* __restrict__ status) {
   __shared__ unsigned long long s_buf[8][kWarpSortMax];
   // Launched behind k_sort_long as its programmatic dependent WITHOUT waiting for it here: the two kernels sort
   // disjoint tiles and run side by side.  What this kernel reads (the binned lists, the status word) was complete
@@ -283,11 +283,11 @@ __global__ void __launch_bounds__(256, 6) k_sort_tiles(
   // have.  The wait is at the end instead (sort_tiles_done), so that this grid's completion implies the other's.
   if (status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) { sort_tiles_done(); return; }
   const int lane = threadIdx.x & 31;
-  // warps draw tiles from a shared cursor (long_count[1]): list lengths differ by two orders of magnitude, and
+  // warps draw tiles from a shared cursor: list lengths differ by two orders of magnitude, and
   // a fixed deal would leave most warps of a CTA waiting for the one with the longest list
   for (;;) {
   int tile = 0;
-  if (lane == 0) tile = atomicAdd(long_count + 1, 1);
+  if (lane == 0) tile = atomicAdd(cursor, 1);
   tile = __shfl_sync(0xffffffffu, tile, 0);
   if (tile >= T) { sort_tiles_done(); return; }
   const int s = tile_offsets[tile];
@@ -383,15 +383,15 @@ __global__ void __launch_bounds__(THREADS) k_sort_long(
 }
 
 int launch_sort(const mlpsp_scene* sc, const mlpsp_frame* fr, float* keys_out, cudaStream_t st, bool unordered_input,
-                int32_t* long_list, int32_t* long_count, const int32_t* list_len) {
+                int32_t* cursors, const int32_t* list_len) {
   const int T = num_tiles(fr->width, fr->height, fr->tile);
   const int ntx = (fr->width + fr->tile - 1) / fr->tile;
   MLPSP_REQUIRE(fr->tile_capacity > 0 && fr->tile_capacity <= kSortCap, MLPSP_E_LIMIT,
                 "tile_capacity must be in [1, %d]", kSortCap);
-  MLPSP_REQUIRE(long_list && long_count, MLPSP_E_ARG, "sort: scratch for the long-tile list missing");
+  MLPSP_REQUIRE(cursors, MLPSP_E_ARG, "sort: scratch for the tile cursors missing");
   const int sms = sm_count();
   // tile cursors: [0] of k_sort_long, [1] of k_sort_tiles (a frame that k_frame_begin prepared starts with both at zero)
-  if (!list_len) MLPSP_CUDA_OK(cudaMemsetAsync(long_count, 0, 8, st));
+  if (!list_len) MLPSP_CUDA_OK(cudaMemsetAsync(cursors, 0, 8, st));
   LaunchScope scope(kKSort, 2, st);
   const int grid = std::min((T + kTilesPerCta - 1) / kTilesPerCta, sms * 6);
   const int grid_long = std::min(T, sms * 6);
@@ -400,16 +400,16 @@ int launch_sort(const mlpsp_scene* sc, const mlpsp_frame* fr, float* keys_out, c
   const int key_mode = fr->sort_key | ((fr->hit_arith == 1 && fr->sort_key == 0) ? 4 : 0);
   if (unordered_input) {
     launch_chained(k_sort_long<256, kSortCap, true>, dim3(grid_long), dim3(256), 0, st, fr->rays_o, fr->rays_d, geom, sc->n, fr->tile_offsets,
-                   fr->tile_prims, fr->width, fr->height, fr->tile, ntx, fr->sorted_prims, keys_out, key_mode, T, long_count, list_len, fr->status);
+                   fr->tile_prims, fr->width, fr->height, fr->tile, ntx, fr->sorted_prims, keys_out, key_mode, T, cursors, list_len, fr->status);
     launch_chained(k_sort_tiles<true>, dim3(grid), dim3(256), 0, st, fr->rays_o, fr->rays_d, geom, sc->n, fr->tile_offsets, fr->tile_prims,
-                   fr->width, fr->height, fr->tile, ntx, T, kSortCap, fr->sorted_prims, keys_out, key_mode, long_list, long_count,
-                   list_len, fr->status);
+                   fr->width, fr->height, fr->tile, ntx, T, kSortCap, fr->sorted_prims, keys_out, key_mode, cursors + 1, list_len,
+                   fr->status);
   } else {
     launch_chained(k_sort_long<256, kSortCap, false>, dim3(grid_long), dim3(256), 0, st, fr->rays_o, fr->rays_d, geom, sc->n, fr->tile_offsets,
-                   fr->tile_prims, fr->width, fr->height, fr->tile, ntx, fr->sorted_prims, keys_out, key_mode, T, long_count, list_len, fr->status);
+                   fr->tile_prims, fr->width, fr->height, fr->tile, ntx, fr->sorted_prims, keys_out, key_mode, T, cursors, list_len, fr->status);
     launch_chained(k_sort_tiles<false>, dim3(grid), dim3(256), 0, st, fr->rays_o, fr->rays_d, geom, sc->n, fr->tile_offsets, fr->tile_prims,
-                   fr->width, fr->height, fr->tile, ntx, T, kSortCap, fr->sorted_prims, keys_out, key_mode, long_list, long_count,
-                   list_len, fr->status);
+                   fr->width, fr->height, fr->tile, ntx, T, kSortCap, fr->sorted_prims, keys_out, key_mode, cursors + 1, list_len,
+                   fr->status);
   }
   return cuda_check(cudaGetLastError(), "sort_tiles");
 }
