@@ -189,7 +189,7 @@ __global__ void k_fold_text(const float* __restrict__ text, const float* __restr
 
 // Input tile with halo -> binary16 A operand [K1/8][kA0Pitch][8] in shared memory.  Consecutive lanes take
 // consecutive 32-byte pieces of a pixel's feature row (coalesced); the odd pitch spreads the 16-byte stores
-// of one pixel's chunks over all banks.  Loads are issued four units ahead of their conversion.
+// of one pixel's chunks over all banks.  Loads are issued B units ahead of their conversion.
 // Threads t = 0..nthr-1 of the CTA share the tile.
 template <int B>
 __device__ __forceinline__ uint32_t load_input_tile(const float* __restrict__ feat, int W, int H, int Cin, int K1,

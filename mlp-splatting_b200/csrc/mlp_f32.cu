@@ -3,7 +3,8 @@
 // layer 1 starts from the bias and accumulates (sin weight, cos weight) per (component, frequency);
 // layers 2 and 3 start from the bias and accumulate over ascending input index.
 // One CTA per work item (primitive, up to 128 of its records); the primitive's FP32 weights are
-// staged once in shared memory and every thread evaluates one record.
+// staged once in shared memory.  k_mlp_f32_pair (hidden 32) gives a thread up to four records of half the units,
+// k_mlp_f32_wide (hidden 64) register tiles, and k_mlp_f32, for every other shape, one record.
 #include "frame.cuh"
 #include "tc.cuh"
 

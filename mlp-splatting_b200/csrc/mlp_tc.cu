@@ -9,15 +9,17 @@
 //     rounds to the operand format and stores straight into the K-major A tile;
 //   * layer 1 (128x80 . 80xH), layer 2 (128xH . HxH) and layer 3 (128xH . Hx16, 4 columns used) are
 //     tcgen05.mma.kind::f16 instructions issued by one lane of a fifth warp, FP32 accumulators in tensor memory.
-//     The biases ride in the same instructions: one extra K step per layer multiplies a constant row
-//     of ones (eight rows of shared memory, broadcast to all 128 by a zero row stride) with the bias
-//     split into up to eight operand-format terms, so no thread ever adds a bias;
+//     The biases ride in the same instructions, split into up to eight operand-format terms, so no thread ever
+//     adds a bias: those of layer 1 meet a chunk of ones that fills its last K step, layers 2 and 3 (and layer 1
+//     where records are kept) take one extra K step against a constant row of ones (eight rows of shared memory,
+//     broadcast to all 128 by a zero row stride);
 //   * between layers every thread pulls its accumulator row back with tcgen05.ld, applies ReLU while
-//     rounding to the operand format and writes the next A tile; the epilogue applies sigmoid /
-//     softplus (and 1-exp(-sigma*decay)) and scatters one float4 per record to its compositing slot.
+//     rounding to the operand format and writes the next layer's A operand into tensor memory (tcgen05.st); the
+//     epilogue applies sigmoid / softplus (and 1-exp(-sigma*decay)) and scatters one float4 per record to its
+//     compositing slot.
 // The three layers of item i, the encoding of item i+1 and the output of item i-1 are software-pipelined:
-// every wait for a group of MMAs is preceded by independent work of a neighbouring item, so the
-// special-function pipe (the binding unit of this kernel) stays busy while the tensor pipe turns around.
+// every wait for a group of MMAs is preceded by independent work of a neighbouring item.  No single unit is full:
+// issue slots, shared memory and special functions are each about half used.
 //
 // Numerics follow the reference's tensor-core contract: operands and hidden activations rounded
 // to binary16 / bfloat16 (RN), FP32 accumulation from zero.
@@ -364,7 +366,7 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
         if (elect_one()) request(1, prim_n);
         pend |= 2u;
       }
-      // ---- layer 3: D3[128x16] = H2[128xH] . W3^T + b3 (rows 4..15 of W3 are zero) ----
+      // ---- layer 3: D3[128x16] = H2[128xH] . W3^T + b3 (of 16 columns the first four are looked at) ----
       ok = both(bar_r0 + 16, bar_w0 + 16, par);
       pend &= ~4u;
       if (!ok) break;
@@ -565,7 +567,7 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
 // ------------------------------------------------------------------ small groups ----
 // Work items of at most 32 records (the remainder of a primitive's records when it is small: most primitives of a
 // scene with millions of primitives own a few records per wave).  A 128-row item would carry one live warp and
-// three idle ones through the same chain of MMA round trips, and only five of them fit an SM.  Here one warp IS
+// three idle ones through the same chain of MMA round trips, and only six (H = 64: four) of them fit an SM.  Here one warp IS
 // the CTA: the operand tiles hold 32 rows (chunk stride 512 bytes; the MMA still has M = 128 and reads, as rows
 // 32..127, whatever follows -- those accumulator rows are never looked at), the accumulators of the three layers
 // share 32 (H = 64: 64) columns of tensor memory, lane 0 issues the MMAs between __syncwarp()s, and 12 (7) such

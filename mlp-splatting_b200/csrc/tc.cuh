@@ -61,10 +61,8 @@ __device__ __forceinline__ void tmem_free(uint32_t taddr, uint32_t cols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
 
-// One lane of a converged warp, the same one every time.  tcgen05.mma takes its descriptors from uniform registers; the
-// compiler emits it directly only where it knows that one thread executes it, which it does behind elect.sync.  Behind
-// `lane == 0` it emits a loop over the active lanes instead: about 100 cycles per MMA against 16 to 40 (five MMAs with a
-// commit and a wait: 895 -> 370 cycles, with the A operand in tensor memory 239).
+// One lane of a converged warp, the same one every time.  MMAs issued behind elect.sync instead of behind `lane == 0`, five
+// of them with a commit and a wait: 895 -> 370 cycles, with the A operand in tensor memory 239.
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
