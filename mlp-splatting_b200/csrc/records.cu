@@ -1344,10 +1344,18 @@ int launch_render_sorted(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scr
   // lose 4 % of evaluator time with the second list, 500,000 gain 2 %, 2,000,000 with 64 hidden units gain 21 %).  (Record export keeps one list.)
   const bool split_small = tc_path && !keep && (int64_t)n * 3 > P;
   // Encoded ray directions from a table where a primitive owns many records: the table takes half of the special functions
-  // off the evaluator and adds 80 bytes per record to what it draws from L2.  With few records per weight image L2 is the
-  // scarcer of the two (evaluator without and with table: 100,000 primitives on 816,000 pixels 398 and 354 us, 60,000 on
-  // 305,000 220 and 214 us plus 6 for the table, 250,000 on 816,000 472 and 521 us).
-  const bool table = tc_path && !keep && (int64_t)n * 7 <= P && s.dir_table && sc->num_freq == 6;
+  // off the evaluator and adds 80 bytes per record to what it draws from L2, and a launch.  With few records per weight image
+  // L2 is the scarcer of the two, and a small image has too few records to pay for the launch.  Whole frames with the table
+  // against without, 32-wide layers, by pixels per primitive:
+  //     320 x 240: 10 to 26 +4 %;  400 x 300: 7.1 +1 %, 40 +3 %;  480 x 360: 7.1 0, 11 -1.5 %, 40 -1 %;
+  //     639 x 477: 3.4 +6 %, 5.1 +1 %, 7.1 -1 %, 16 -4 %;  800 x 600: 7.1 -2.5 %, 16 -5.5 %;
+  //     1200 x 680: 3.3 +17 %, 5.8 +2.5 %, 7.0 +0.5 %, 8.2 -0.5 %, 16 -5 %, 40 -6 %
+  // and 64-wide ones, whose image is 2.5 times as large:
+  //     480 x 360: 11 to 150 +1 to +6 %;  639 x 477: 16 0, 25 to 150 +1 to +2 %;  800 x 600: 11 0, 16 -1 %, 60 -1.3 %;
+  //     1200 x 680: 8.2 +3.3 %, 11 +1.5 %, 16 0, 25 -1 %, 60 -1.3 %.
+  const bool wide = sc->hidden > 32;
+  const bool table = tc_path && !keep && (int64_t)n * (wide ? 20 : 7) <= P && P >= (wide ? 400000 : 150000) && s.dir_table &&
+                     sc->num_freq == 6;
   if (table) {
     const int rc_dir = launch_encode_directions(sc, fr, s.dir_table, st);
     if (rc_dir) return rc_dir;
@@ -1519,6 +1527,7 @@ int launch_render_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scr
     rc = launch_prim_scan(lead, n, nullptr, f0->status, st, split_small, w);
     if (rc) return rc;
     {
+      // (no table of ray directions: the records of a launch come from all views, and would have to name theirs)
       LaunchScope scope(kKFill, V, st);
       for (int v = 0; v < V; ++v) {
         const mlpsp_frame* fr = frs + v;

@@ -83,6 +83,23 @@ def test_frames_at_placement_and_fill_edges(n, W, H, precision, tol):
     np.testing.assert_allclose(rgb.cpu().numpy(), f["render"].rgb, atol=tol)
 
 
+@pytest.mark.parametrize("precision", [1, 2])
+@pytest.mark.parametrize("hidden,n,W,H", [(32, 2000, 483, 365), (32, 21_428, 500, 300), (64, 3000, 803, 501), (64, 20_000, 800, 500)])
+def test_frames_with_a_direction_table_equal_a_batch_without(precision, hidden, n, W, H):
+    """Frames on the table's side of its rule, on the line and with ragged tiles; a batch of views never takes the table."""
+    from mlp_splatting_b200 import synthetic
+    from mlp_splatting_b200.engine import FrameRenderer, PackedScene, ViewBatchRenderer
+    scene = synthetic.make_scene_device(n, 7, torch.device(DEV), mu=-3.5, hidden=hidden)
+    ps = PackedScene(scene["positions"], scene["log_scales"], scene["quats"], *[scene[k] for k in WKEYS], scene["freq"],
+                     scene["att"], device=DEV, pack_bf16=True)
+    cam = synthetic.make_camera(W, H)
+    ro, rd = _t(cam["rays_o"]), _t(cam["rays_d"])
+    got = FrameRenderer(W, H, device=DEV).render(ps, ro, rd, THR, view=cam["view"], proj=cam["proj"], precision=precision)
+    want = ViewBatchRenderer(W, H, 1, device=DEV).render(ps, [ro], [rd], THR, [cam["view"]], [cam["proj"]], precision=precision)[0]
+    assert float(want[1].max()) > 0.5
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
 @pytest.mark.parametrize("n", [257, 512, 513, 1024, 1025, 1500])
 @pytest.mark.parametrize("W,H", [(5, 3), (23, 17)])
 def test_long_lists_sort_exactly(n, W, H):
