@@ -388,7 +388,8 @@ int mlpsp_grouped_weight_gradients(const mlpsp_scene* scene, const int64_t* offs
 
 /* The same gradients written to the six gradient tensors (dW1[n,32,72] db1[n,32] dW2[n,32,32] db2[n,32] dW3[n,4,32]
  * db3[n,4]), with the caller's scratch and without a prepared layout.  x6, d4 and relu_masks hold num_records rows, at
- * least offsets[n].  *nonfinite_host (HOST) receives the flag word described above; the call waits for it. */
+ * least offsets[n].  segment_size is a hint: mixed-precision calls with many records double the segments as long as
+ * these are shorter than 4,096.  *nonfinite_host (HOST) receives the flag word described above; the call waits for it. */
 int64_t mlpsp_weight_gradients_scratch_bytes(int64_t num_records, int32_t n, int32_t segment_size);
 int mlpsp_weight_gradients(const mlpsp_scene* scene, const int64_t* offsets, const float* x6, const float* d4,
                            const int32_t* relu_masks, int64_t num_records, int32_t segment_size, int32_t precision,

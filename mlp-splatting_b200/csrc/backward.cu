@@ -683,9 +683,12 @@ static int weight_gradients(const mlpsp_scene* sc, const int64_t* offsets, const
                             int64_t scratch_bytes, int32_t* flag_host, cudaStream_t st) {
   const VjpScratch L = vjp_scratch(R, sc->n, segment_size);
   MLPSP_REQUIRE(scratch && scratch_bytes >= L.bytes, MLPSP_E_SCRATCH, "mlpsp_weight_gradients: scratch needs %lld bytes", (long long)L.bytes);
-  // Segments cut long primitives for the CTAs to share; where the records make many segments per CTA anyway, longer ones
-  // leave fewer partial rows to write and add (their sums stay in one accumulator all the same).  4.3 M records, 512 against
-  // 1,024 per segment: 727 and 693 us for the two kernels.
+  // segment_size is a hint.  Segments cut long primitives for the CTAs to share; where the records alone make more than
+  // sixteen full segments per CTA, longer ones leave fewer partial rows to write and add, and fewer ragged ends (their sums
+  // stay in one accumulator all the same).  512 against the rule's length: 5.9 M records of a 50,000-primitive scene (17,806
+  // segments, 12,593 of 1,024) 773 and 717 us, 9.5 M (24,337; 11,182 of 2,048) 1,093 and 973, 7.3 M of 100,000 primitives 1,036
+  // and 974, 4.3 M in primitives of 860 516 and 416, of 8,600 494 and 440; the same where no primitive has two segments; slower
+  // nowhere.  Below sixteen a doubling is no sure gain: 1.0 M records in primitives of 860 181 and 166 us, of 2,150 182 and 191.
   if (precision != MLPSP_PRECISION_F32)
     while (segment_size < 4096 && R / segment_size > (int64_t)sm_count() * 3 * 16) segment_size *= 2;
   char* base = reinterpret_cast<char*>(align_up((int64_t)reinterpret_cast<uintptr_t>(scratch), 256));

@@ -175,7 +175,8 @@ def grouped_weight_gradients(csr, freq, attenuation, weights, *, dtype=torch.flo
     weights) to that format and run every product on the tensor cores with FP32 accumulation over the segment;
     float16 adjoints are scaled by 4096 before the cast and unscaled in FP32 afterwards unless loss_scale says
     otherwise.  A non-finite mixed result is retried in unscaled FP32; a non-finite FP32 result raises
-    FloatingPointError and no gradients are returned.  block_size is the reference's Triton row block; it is
+    FloatingPointError and no gradients are returned.  segment_size is a hint: where there are many, the mixed-precision
+    modes double the segments as long as these are shorter than 4,096 records.  block_size is the reference's Triton row block; it is
     checked and otherwise unused (the kernels walk a segment 128 records at a time)."""
     import math
     w1, b1, w2, b2, w3, b3 = weights
