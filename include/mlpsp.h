@@ -45,6 +45,7 @@ extern "C" {
 #define MLPSP_ST_WORK_TOTAL 10     /* evaluator work items (blocks of at most 128 rows) of the whole frame */
 #define MLPSP_ST_PAIRS_KEPT 11     /* mlpsp_render_frame: candidate pairs left after the tile pre-test */
 #define MLPSP_ST_WORK_SMALL 12     /* of MLPSP_ST_WORK_TOTAL: items of the small-group list (at most 32 rows) */
+#define MLPSP_ST_LAST_TILES 13     /* tiles that were on the list of the last of these MLPSP_ST_WAVES */
 
 /* bits 1,2,4 match the reference validator (np_tile_kernels.cu:4499-4519) */
 #define MLPSP_ST_BAD_OFFSETS 1       /* tile_offsets not 0-based / monotone / in bounds */
@@ -163,6 +164,12 @@ typedef struct mlpsp_frame {
 
 const char* mlpsp_last_error(void);
 int mlpsp_abi_version(void);
+/* A wave schedule for frames of this size: writes the windows (at most MLPSP_MAX_WAVES, the last one reaches tile_capacity)
+ * and returns their number.  views > 1: a batch of mlpsp_render_frames; caller_lists: the lists have not been through the tile
+ * pre-test.  Any schedule gives the same image; this one may evaluate more records than num_waves = 0 (size max_records for
+ * it, or grow it when a frame reports MLPSP_ST_RECORD_OVERFLOW). */
+int mlpsp_wave_schedule(int32_t n, int32_t width, int32_t height, int32_t hidden, int32_t precision, int32_t views,
+                        int32_t caller_lists, int32_t tile_capacity, int32_t* wave_len);
 /* sizeof(mlpsp_scene), sizeof(mlpsp_frame) as compiled, for bindings that mirror the structs */
 int mlpsp_struct_sizes(int32_t* scene_bytes, int32_t* frame_bytes);
 

@@ -14,6 +14,7 @@ LIB_PATH = os.path.join(_HERE, "libmlpsp_b200.so")
 STATUS_WORDS = 16
 ST_BITS, ST_MAX_TILE_LEN, ST_PAIRS, ST_WAVES = 0, 1, 2, 3
 ST_RECORDS_LO, ST_USED_LO, ST_WAVE_RECORDS, ST_WORK_ITEMS, ST_WORK_TOTAL, ST_PAIRS_KEPT, ST_WORK_SMALL = 4, 6, 8, 9, 10, 11, 12
+ST_LAST_TILES = 13
 BIT_BAD_OFFSETS, BIT_TILE_CAPACITY, BIT_BAD_IDS = 1, 2, 4
 BIT_PAIR_OVERFLOW, BIT_RECORD_OVERFLOW, BIT_NUMERIC, BIT_TIMEOUT = 8, 16, 64, 128
 BIT_TILE_ORIGINS, BIT_CONE_TOO_WIDE, BIT_FEAT_INEXACT = 256, 512, 1024
@@ -65,6 +66,7 @@ class Decoder(C.Structure):
 _SIGS = {
     "mlpsp_last_error": (C.c_char_p, []),
     "mlpsp_abi_version": (C.c_int, []),
+    "mlpsp_wave_schedule": (C.c_int, [C.c_int32] * 8 + [C.POINTER(C.c_int32)]),
     "mlpsp_struct_sizes": (C.c_int, [C.POINTER(C.c_int32), C.POINTER(C.c_int32)]),
     "mlpsp_pack_geometry": (C.c_int, [_fp, _fp, _fp, C.c_int32, _fp, _fp]),
     "mlpsp_normalize_rows": (C.c_int, [_fp, _fp, C.c_int64, C.c_int32, _fp]),

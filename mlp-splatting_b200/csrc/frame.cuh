@@ -14,6 +14,7 @@ constexpr int kRowsPerSmallItem = 32;
 // counters[] slots (device int32)
 enum Counter {
   kCtrRecords = 0,   // records appended by the hit pass of the current wave
+  kCtrWaveTiles = 1, // tiles on the current wave's list (of all views of a batch)
   kCtrWorkNext = 2,  // dynamic work cursor of the evaluator
   kCtrActive0 = 3,   // active tile count, list 0
   kCtrActive1 = 4,   // active tile count, list 1

@@ -347,12 +347,13 @@ struct HitArgs {
   float thr, bound2, K;            // K <= 0: no quadratic form (thresholds the exponential underflows at)
   const int32_t* active; const int32_t* active_count; int lo, hi;
   const float4* px_state; uint2* masks; uint32_t* pair_base; int32_t* prim_cnt; int32_t* counters; int64_t max_records;
-  int32_t* status; int32_t* next_count;
+  int32_t* status; int32_t* next_count; int add_tiles;      // add_tiles: a view of a batch that is not its first
 };
 
 // the wave's counters start at zero, and the list its compositing pass will append to starts empty
 __device__ __forceinline__ void reset_wave(const HitArgs& a) {
   *a.next_count = 0;
+  a.counters[kCtrWaveTiles] = *a.active_count + (a.add_tiles ? a.counters[kCtrWaveTiles] : 0);
   a.counters[kCtrWork] = 0; a.counters[kCtrWorkSmall] = 0; a.counters[kCtrWorkNext] = 0; a.counters[kCtrWaveRecords] = 0;
 }
 
@@ -522,7 +523,10 @@ __global__ void __launch_bounds__(kPrimScanItems / 4) k_prim_alloc(
     atomicMax(status + MLPSP_ST_WORK_ITEMS, s_base[1] + tb + s_base[2] + tm);
     if (tb + tm) atomicAdd(status + MLPSP_ST_WORK_TOTAL, tb + tm);
     if (tm) atomicAdd(status + MLPSP_ST_WORK_SMALL, tm);
-    if (r0 == 0) atomicAdd(status + MLPSP_ST_WAVES, 1);
+    if (r0 == 0) {
+      atomicAdd(status + MLPSP_ST_WAVES, 1);
+      status[MLPSP_ST_LAST_TILES] = counters[kCtrWaveTiles];
+    }
   }
   __syncthreads();
   ea += s_base[0]; eb += s_base[1]; em += s_base[2];
@@ -1274,6 +1278,55 @@ __global__ void __launch_bounds__(kFeatThreads) k_feature_composite(
 // need more than the first hundred: the tail wave takes whatever is left
 static const int kDefaultWaves[] = {32, 32, 64, 128, 256, INT_MAX};
 
+// A schedule for the size of the work (for hosts that can give a frame more records when it asks for them; kDefaultWaves is
+// what num_waves = 0 means).  A wave costs some 25 us of dependent launches and, where primitives own few records, another
+// fetch of their weight images; a longer window costs records of pixels that end inside it.  So the first window is
+//     a = 70 (318,000 / P)^(1/3) (4 / r)^e,   P pixels, r pixels per primitive (at most 9), e = 0.4, or 0.55 for r < 4
+// (smaller primitives: fewer of a window's candidates hit a pixel), twice that where the lists come from the caller and have
+// not been through the tile pre-test, 65 for 70 in FP32; for a batch of views e = 0.8 for r < 4, and again times H / 32 (the
+// images' bytes).  Then a, 2a, 4a, or, on large images, two of a/2 (binary16: at least 32) for the a, and the rest; the smallest
+// frames take one window.
+// Whole frames, 32, 32, 64, 128, 256, rest against this, us:
+//     pixels  primitives  binary16     FP32             pixels  primitives   binary16        FP32
+//      5,696       3,560  284 -> 145   279 -> 163      318,159     198,849    806 -> 708   2,080 -> 1,981
+//     14,000       8,750  316 -> 182   358 -> 282      318,159      79,539    559 -> 502   1,475 -> 1,353
+//     35,840       8,960  247 -> 190   394 -> 354      318,159      10,605    440 -> 414   1,043 -> 1,041
+//     80,640      50,400  426 -> 313   750 -> 676      504,000     126,000    745 -> 712   2,187 -> 2,008
+//     80,640       2,688  214 -> 169   347 -> 303      808,640     202,160  1,071 -> 1,027 3,355 -> 3,125
+//    161,500      16,150  344 -> 322   731 -> 707      808,640      26,954    859 -> 825   2,565 -> 2,400
+// a record frame of 320 x 240 and 20,000 primitives 394 -> 296; four views at 1200 x 680 of 500,000 4,486 -> 4,251, at
+// 1920 x 1080 of 1,000,000 64-wide ones 10,867 -> 10,408.
+extern "C" int mlpsp_wave_schedule(int32_t n, int32_t width, int32_t height, int32_t hidden, int32_t precision, int32_t views,
+                                   int32_t caller_lists, int32_t tile_capacity, int32_t* wave_len) {
+  MLPSP_REQUIRE(n >= 0 && width > 0 && height > 0 && views > 0 && tile_capacity > 0 && wave_len, MLPSP_E_ARG,
+                "mlpsp_wave_schedule: bad argument");
+  const double P = (double)width * height, r = std::min(9.0, P / std::max(n, 1));
+  const bool f32 = precision == MLPSP_PRECISION_F32;
+  int count = 0;
+  if (P <= (f32 ? 16000.0 : 30000.0) && tile_capacity <= kWinMax) {
+    wave_len[count++] = tile_capacity;
+    return count;
+  }
+  double a = (f32 ? 65.0 : 70.0) * std::cbrt(318000.0 / P) * std::pow(4.0 / r, r >= 4.0 ? 0.4 : (views > 1 ? 0.8 : 0.55));
+  if (caller_lists) a *= 2.0;
+  if (views > 1) a *= std::max(1.0, hidden / 32.0);
+  const int first = (int)std::min(512.0, std::max(32.0, 8.0 * std::floor(a / 8.0 + 0.5)));
+  const bool halves = P >= (f32 ? 250000.0 : 450000.0);
+  int lo = 0;
+  auto add = [&](int len) {
+    len = std::min(std::min(len, kWinMax), tile_capacity - lo);
+    if (len > 0) { wave_len[count++] = len; lo += len; }
+  };
+  add(first);
+  const int second = halves ? std::max(first / 2, f32 ? 16 : 32) : first;
+  add(second);
+  if (halves) add(second);
+  add(2 * first);
+  add(4 * first);
+  while (lo < tile_capacity && count < MLPSP_MAX_WAVES) add(kWinMax);
+  return count;
+}
+
 int launch_hit_masks(const mlpsp_scene* sc, const mlpsp_frame* fr, uint64_t* mask_geo, cudaStream_t st) {
   const int T = num_tiles(fr->width, fr->height, fr->tile);
   const int ntx = (fr->width + 7) / 8;
@@ -1382,7 +1435,7 @@ int launch_render_sorted(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scr
       const HitArgs ha = {fr->rays_o, fr->rays_d, (const float4*)sc->geom, n, fr->tile_offsets, s.tile_len, fr->sorted_prims, W, H, ntx,
                           fr->threshold, miss_bound2(fr->threshold), form_threshold(fr->threshold), act, act_n, lo, hi, s.px_state,
                           reinterpret_cast<uint2*>(s.masks32), s.pair_base, s.prim_cnt + (size_t)(w & 1) * prim_cnt_stride(n), s.counters,
-                          fr->max_records, fr->status, s.counters + kCtrActive0 + nxt};
+                          fr->max_records, fr->status, s.counters + kCtrActive0 + nxt, 0};
       rc = launch_hits(ha, ref_arith, T, sms, idle_tail, st);
       if (rc) return rc;
     }
@@ -1519,7 +1572,7 @@ int launch_render_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scr
         const HitArgs ha = {fr->rays_o, fr->rays_d, (const float4*)sc->geom, n, fr->tile_offsets, s.tile_len, fr->sorted_prims, W, H, ntx,
                             f0->threshold, miss_bound2(f0->threshold), form_threshold(f0->threshold), s.active[cur],
                             s.counters + kCtrActive0 + cur, lo, hi, s.px_state, reinterpret_cast<uint2*>(s.masks32), s.pair_base, cnt,
-                            lead.counters, f0->max_records, f0->status, s.counters + kCtrActive0 + nxt};
+                            lead.counters, f0->max_records, f0->status, s.counters + kCtrActive0 + nxt, v > 0 ? 1 : 0};
         rc = launch_hits(ha, ref_arith, T, sms, idle_tail, st);
         if (rc) return rc;
       }

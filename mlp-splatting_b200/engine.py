@@ -264,6 +264,7 @@ class FrameStats:
     work_total: int = 0   # evaluator work items (blocks of at most 128 rows) of the whole frame
     pairs_kept: int = 0   # candidate pairs left after the tile pre-test (0 when it did not run)
     work_small: int = 0   # of work_total: small-group items (at most 32 rows)
+    last_tiles: int = 0   # tiles on the list of the last of these waves
 
 
 class RenderError(RuntimeError):
@@ -282,6 +283,53 @@ def raise_for_status(bits: int, max_len: int, capacity: int, path_name: str):
         raise RenderError(f"{path_name}: candidate primitive IDs must be in [0, num_primitives)")
     if bits & L.BIT_TIMEOUT:
         raise RenderError(f"{path_name}: a device-side wait gave up (status bit {L.BIT_TIMEOUT}); frame discarded")
+
+
+class WaveSchedule:
+    """The wave schedule a renderer gives its next frame (the image does not depend on it).
+
+    The library has one for the size of the work (mlpsp_wave_schedule); most frames never need its last waves, and each of
+    them still costs its launches.  After a frame whose status has been read, the next one is given the waves that one used
+    plus a catch-all, which is expected to be idle, or, when hardly any tile came as far as the last of them, that one as the
+    catch-all.  Hardly any: tiles times the longest list behind that wave at most 20,000 candidates, some 250,000 records that
+    might be evaluated too early, which cost what the launches of an idle wave do (10 us; 425 tiles of 12,750 with lists up to
+    1,193 took 160 us more on the 100k frame)."""
+
+    def __init__(self, width, height, capacity, views=1):
+        self.size, self.capacity, self.views = (int(width), int(height)), int(capacity), int(views)
+        self.key = None
+        self.default = self.given = None
+        self.idle_tail = False
+
+    def get(self, n, hidden, precision, caller_lists=False):
+        """(windows, whether the last one is expected to find no work) for a frame of this kind."""
+        key = (n, hidden, precision, caller_lists)
+        if key != self.key:
+            buf = (C.c_int32 * L.MAX_WAVES)()
+            count = L.load().mlpsp_wave_schedule(n, *self.size, hidden, precision, self.views, 1 if caller_lists else 0,
+                                                 self.capacity, buf)
+            if count <= 0:
+                L.check(count or -1, "mlpsp_wave_schedule")
+            self.key, self.default = key, list(buf[:count])
+            self.given, self.idle_tail = self.default, False
+        return self.given, self.idle_tail
+
+    def adapt(self, words):
+        """Takes the status words of the frame that was rendered with what get() returned last."""
+        g, used = self.given, int(words[L.ST_WAVES])
+        if g is None or used <= 0:
+            return
+        behind = max(0, int(words[L.ST_MAX_TILE_LEN]) - sum(g[:used - 1]))
+        few = int(words[L.ST_LAST_TILES]) * behind <= 20_000
+        if used >= len(g):
+            self.given, self.idle_tail = (g if few else self.default), False
+            return
+        merge = used >= 2 and few
+        head = g[:used - 1] if merge else g[:used]
+        if self.capacity - sum(head) > 2048:        # a window holds at most 2,048 candidates
+            self.given, self.idle_tail = self.default, False
+        else:
+            self.given, self.idle_tail = head + [self.capacity], not merge
 
 
 class FrameRenderer:
@@ -330,6 +378,7 @@ class FrameRenderer:
         self._buffers = 0           # counts reallocations of the buffers those structures point at
         self._status_np = self.status_host.numpy()
         self.f32_fallbacks = 0   # frames re-rendered in FP32 after an fp16 overflow
+        self._waves = WaveSchedule(self.W, self.H, self.capacity)
 
     @property
     def last_stats(self) -> "FrameStats | None":
@@ -448,7 +497,7 @@ class FrameRenderer:
         used = int(u[L.ST_USED_LO]) | (int(u[L.ST_USED_LO + 1]) << 32)
         return FrameStats(int(s[L.ST_PAIRS]), int(s[L.ST_MAX_TILE_LEN]), rec, used, int(s[L.ST_WAVES]),
                           int(s[L.ST_WAVE_RECORDS]), int(s[L.ST_WORK_ITEMS]), int(s[L.ST_WORK_TOTAL]), int(s[L.ST_PAIRS_KEPT]),
-                          int(s[L.ST_WORK_SMALL]))
+                          int(s[L.ST_WORK_SMALL]), int(s[L.ST_LAST_TILES]))
 
     def _read_status(self):
         self.status_host.copy_(self.status, non_blocking=True)
@@ -469,19 +518,6 @@ class FrameRenderer:
             self.max_records = int(max(stats.wave_records, self.max_records) * 2) + 4096
             return True
         return False
-
-    # Wave schedule carried from frame to frame.  The library's default schedule ends in waves that most frames
-    # never need; each of them still costs its launches.  After a frame whose status has been read, the next
-    # frame is given the waves that one used plus a single catch-all wave, which keeps any frame correct (the
-    # image does not depend on the schedule) and costs one idle wave instead of several.
-    DEFAULT_WAVES = (32, 32, 64, 128, 256)
-
-    def _adapt_waves(self, waves_used: int):
-        n = int(waves_used)
-        if n <= 0 or n > len(self.DEFAULT_WAVES):
-            self._auto_waves = None
-        else:
-            self._auto_waves = list(self.DEFAULT_WAVES[:n]) + [self.capacity]
 
     # -- stages -------------------------------------------------------------------------------
     def render(self, scene: PackedScene, rays_o, rays_d, threshold, view=None, proj=None, precision=None,
@@ -506,8 +542,7 @@ class FrameRenderer:
         if precision is None:
             precision = L.PRECISION_F16 if scene.has_f16 else L.PRECISION_F32
         auto = waves is None
-        if auto:
-            waves = getattr(self, "_auto_waves", None)
+        idle_tail = False
         view_dev = proj_dev = None
         if tile_lists is None and torch.is_tensor(view) and view.is_cuda:
             view_dev, proj_dev = view, torch.as_tensor(proj)
@@ -555,9 +590,11 @@ class FrameRenderer:
                     L.check(lib.mlpsp_validate_tile_lists(L.ptr(self.tile_offsets), L.ptr(self.tile_prims), self.T, m,
                                                           self.capacity, scene.n, L.ptr(self.status), st),
                             "mlpsp_validate_tile_lists")
+                if auto:
+                    waves, idle_tail = self._waves.get(scene.n, scene.hidden, precision, tile_lists is not None)
                 f = self._frame(scene, rays_o, rd, threshold, precision, view, proj, bg, want_depth, want_mask_used, waves,
                                 want_feat=want_feat, keep_records=keep_records, sort_key=sort_key, tile_rows=tile_rows,
-                                tile_pretest=tile_pretest, prim_stats=prim_stats, tail_hint=auto and waves is not None,
+                                tile_pretest=tile_pretest, prim_stats=prim_stats, tail_hint=idle_tail,
                                 hit_arith=hit_arith, outs=outs)
                 self._last_frame = (f, scene)
                 if tile_lists is None:
@@ -577,7 +614,7 @@ class FrameRenderer:
                 self._stats = words.copy()
                 if bits == 0:
                     if auto and sort_key != L.ORDER_PER_PIXEL:
-                        self._adapt_waves(int(words[L.ST_WAVES]))
+                        self._waves.adapt(words)
                     return result
                 stats = self.last_stats
                 if bits & (L.BIT_BAD_OFFSETS | L.BIT_TILE_CAPACITY | L.BIT_BAD_IDS | L.BIT_TIMEOUT):
@@ -693,7 +730,7 @@ class FrameRenderer:
                     rgb, alpha = self.render(scene, rays_o, rays_d, threshold, keep_records=True, **kw)
                     f = count(offsets, st)
                 elif kw.get("waves") is None and kw.get("sort_key", 0) != L.ORDER_PER_PIXEL:
-                    self._adapt_waves(int(self._status_np[L.ST_WAVES]))
+                    self._waves.adapt(self._status_np)
             if worst.value < 0:
                 raise RenderError(f"render_tiles_training_records: tile-center backward hit capacity {max_hits} reached "
                                   "before transmittance termination; refusing to return truncated records")
@@ -817,7 +854,7 @@ class ViewBatchRenderer:
         self.lib = self.lead.lib
         self.last_stats: FrameStats | None = None
         self.f32_fallbacks = 0
-        self._auto_waves = None
+        self._waves = WaveSchedule(self.lead.W, self.lead.H, self.lead.capacity, self.V)
 
     def render(self, scene: PackedScene, rays_o, rays_d, threshold, views, projs, precision=None, bg=None, waves=None,
                rays_normalized=False, path_name="render_tiles_forward_tilecenter", hit_arith=0):
@@ -828,9 +865,7 @@ class ViewBatchRenderer:
         lib, d, lead = self.lib, self.device, self.lead
         if precision is None:
             precision = L.PRECISION_F16 if scene.has_f16 else L.PRECISION_F32
-        auto = waves is None
-        if auto:
-            waves = self._auto_waves
+        auto, idle_tail = waves is None, False
         with torch.cuda.device(d):
             st = _stream_ptr(d)
             rds = []
@@ -842,19 +877,19 @@ class ViewBatchRenderer:
                     rds.append(r.rays_d_unit)
             for _attempt in range(10):
                 L.check(lib.mlpsp_status_reset(L.ptr(lead.status), st), "mlpsp_status_reset")
+                if auto:
+                    waves, idle_tail = self._waves.get(scene.n, scene.hidden, precision)
                 frames = (L.Frame * self.V)()
                 for v, r in enumerate(self.views):
                     f = r._frame(scene, rays_o[v], rds[v], threshold, precision, views[v], projs[v], bg, False, False, waves,
-                                 tail_hint=auto and waves is not None, hit_arith=hit_arith)
+                                 tail_hint=idle_tail, hit_arith=hit_arith)
                     f.status = L.ptr(lead.status)
                     frames[v] = f
                 L.check(lib.mlpsp_render_frames(C.byref(scene.c), frames, self.V, st), "mlpsp_render_frames")
                 bits, stats = lead._read_status()
                 self.last_stats = stats
                 if auto and bits == 0:
-                    n = int(stats.waves)
-                    self._auto_waves = (list(FrameRenderer.DEFAULT_WAVES[:n]) + [lead.capacity]
-                                        if 0 < n <= len(FrameRenderer.DEFAULT_WAVES) else None)
+                    self._waves.adapt(lead._status_np)
                 if bits & (L.BIT_BAD_OFFSETS | L.BIT_TILE_CAPACITY | L.BIT_BAD_IDS | L.BIT_TIMEOUT):
                     raise_for_status(bits, stats.max_tile_len, lead.capacity, path_name)
                 if bits & L.BIT_PAIR_OVERFLOW:
@@ -940,7 +975,7 @@ class FramePipeline:
         s["busy"] = False
         bits = int(r.status_host[L.ST_BITS])
         if bits == 0:
-            r._adapt_waves(int(r.status_host[L.ST_WAVES]))
+            r._waves.adapt(r._status_np)
             return
         # rare path: overflow / error / fp16 overflow -> redo this frame synchronously with full checks
         threshold, kw, out_rgb, out_alpha = s["kw"]
