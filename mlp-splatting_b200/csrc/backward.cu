@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(256) k_vjp_plan(const int64_t* __restrict__ of
   chain_wait();
   chain_release();
   __shared__ int warp_sums[32];
-  __shared__ int base[4];
+  __shared__ int base[5];
   const int p = blockIdx.x * 256 + threadIdx.x;
   int64_t start = 0, count = 0;
   if (p < n) {
@@ -328,8 +328,10 @@ __global__ void __launch_bounds__(256) k_vjp_plan(const int64_t* __restrict__ of
   }
   const int segs = count > 0 ? (int)((count + segment_size - 1) / segment_size) : 0;
   const int rows = segs > 1 ? segs : 0, listed = segs > 1, empty = p < n && segs == 0;
-  int ts, tr, tm, te;
-  const int es = block_exclusive_scan(segs, warp_sums, ts);
+  const int full = (int)(count / segment_size), part = segs - full;      // full segments, and a shorter last one
+  int ts, tp, tr, tm, te;
+  const int es = block_exclusive_scan(full, warp_sums, ts);
+  const int ep = block_exclusive_scan(part, warp_sums, tp);
   const int er = block_exclusive_scan(rows, warp_sums, tr);
   const int em = block_exclusive_scan(listed, warp_sums, tm);
   const int ee = block_exclusive_scan(empty, warp_sums, te);
@@ -338,6 +340,7 @@ __global__ void __launch_bounds__(256) k_vjp_plan(const int64_t* __restrict__ of
     base[1] = tr ? atomicAdd(counters + kVpRows, tr) : 0;
     base[2] = tm ? atomicAdd(counters + kVpMulti, tm) : 0;
     base[3] = te ? atomicAdd(counters + kVpEmpty, te) : 0;
+    base[4] = tp ? atomicAdd(counters + kVpParts, tp) : 0;
   }
   __syncthreads();
   for (int g = 0; g < segs; ++g) {
@@ -346,8 +349,8 @@ __global__ void __launch_bounds__(256) k_vjp_plan(const int64_t* __restrict__ of
     it.rows = (int)min((int64_t)segment_size, count - (int64_t)g * segment_size);
     it.prim = p;
     it.dest = segs > 1 ? base[1] + er + g : -1;
-    const uint32_t at = (uint32_t)(base[0] + es + g);
-    if (at < max_items) items[at] = it;
+    const uint32_t at = (uint32_t)(g < full ? base[0] + es + g : base[4] + ep);
+    if (at < max_items) items[g < full ? at : max_items - 1 - at] = it;
   }
   if (listed) {
     VjpItem it = {};
@@ -437,13 +440,13 @@ __device__ __forceinline__ float dot4(float acc, const float4 a, const float4 b)
 
 __global__ void __launch_bounds__(kGfThreads, kGfCtas) k_grouped_vjp(
     const float* __restrict__ x6, const float* __restrict__ d4, const int32_t* __restrict__ masks,
-    const VjpItem* __restrict__ items, int32_t* __restrict__ counters, const float* __restrict__ freq,
+    const VjpItem* __restrict__ items, int64_t max_items, int32_t* __restrict__ counters, const float* __restrict__ freq,
     const float* __restrict__ att, const float* __restrict__ W1, const float* __restrict__ b1, const float* __restrict__ W2,
     const float* __restrict__ b2, const float* __restrict__ W3, float scale, VjpOut out, float* __restrict__ partial) {
   chain_wait();
   chain_release();
   extern __shared__ __align__(16) float sm[];
-  const int G = vjp_planned(counters, kVpItems);
+  const VjpList list(items, max_items, counters);
   const int tid = threadIdx.x;
   const int hg = tid & 7, rg = tid >> 3;         // units 4 hg .. + 3 of records 4 rg .. + 3; gradient rows 2 rg, 2 rg + 1
   const float inv = 1.f / scale;
@@ -453,8 +456,8 @@ __global__ void __launch_bounds__(kGfThreads, kGfCtas) k_grouped_vjp(
 #pragma unroll
   for (int f = 0; f < 6; ++f) { fr[f] = __ldg(freq + f); at[f] = __ldg(att + f); }
   __shared__ int s_next;
-  for (int idx = blockIdx.x; idx < G; idx = s_next) {            // (read behind the barriers of the item's blocks)
-    const VjpItem it = load_item(items + idx);
+  for (int idx = blockIdx.x; idx < list.total; idx = s_next) {   // (read behind the barriers of the item's blocks)
+    const VjpItem it = list.at(idx);
     const size_t p = (size_t)it.prim;
     __syncthreads();                             // the previous item's last block has been consumed
     if (tid == 0) s_next = (int)gridDim.x + atomicAdd(counters + kVpNext, 1);
@@ -671,7 +674,7 @@ static int run_vjp_plan(const mlpsp_scene* sc, const float* x6, const float* d4,
     if (attr_once.first())
       MLPSP_CUDA_OK(cudaFuncSetAttribute(k_grouped_vjp, cudaFuncAttributeMaxDynamicSharedMemorySize, kGradSmem));
     launch_chained(k_grouped_vjp, dim3((unsigned)std::min<int64_t>(max_items, (int64_t)sm_count() * kGfCtas)), dim3(kGfThreads), kGradSmem, st,
-                   x6, d4, masks, items, counters, sc->freq, sc->att, sc->W1, sc->b1, sc->W2, sc->b2, sc->W3, loss_scale, out, partial);
+                   x6, d4, masks, items, max_items, counters, sc->freq, sc->att, sc->W1, sc->b1, sc->W2, sc->b2, sc->W3, loss_scale, out, partial);
   }
   launch_chained(k_vjp_reduce, dim3((unsigned)std::min(sc->n, sm_count() * 8)), dim3(256), 0, st, multi, partial, out, sc->n, tc ? 0 : 1,
                  vjp_aligned(out), counters);

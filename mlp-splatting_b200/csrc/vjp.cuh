@@ -29,12 +29,22 @@ constexpr int kOW1 = 0, kOb1 = kOW1 + kGH * kGIN, kOW2 = kOb1 + kGH, kOb2 = kOW2
 static_assert(kGradLen == 3524, "gradient row layout");
 
 // plan counters (device int32); the flag word holds the bits that mlpsp.h gives for *nonfinite
-enum VjpCounter { kVpItems = 0, kVpRows = 1, kVpMulti = 2, kVpFlag = 3, kVpEmpty = 4, kVpNext = 5, kVpCounters = 6 };
+enum VjpCounter { kVpItems = 0, kVpRows = 1, kVpMulti = 2, kVpFlag = 3, kVpEmpty = 4, kVpNext = 5, kVpParts = 6, kVpCounters = 7 };
 constexpr int kVpBadPlan = 4;
 // a counter of the plan, 0 when the offsets were refused: a list that may be cut short or point past the records is not read
 __device__ __forceinline__ int vjp_planned(const int32_t* counters, int which) {
   return (counters[kVpFlag] & kVpBadPlan) ? 0 : counters[which];
 }
+
+// The list of segments: kVpItems from the front of the array and kVpParts from its end backwards.  A plan puts the full segments
+// in front, so that CTAs end on the shorter remainders (with both in the primitives' order the last CTAs of 5.5 M records worked
+// 62 us after the first had run out).
+struct VjpList {
+  const VjpItem* items; const VjpItem* end; int front, total;
+  __device__ __forceinline__ VjpList(const VjpItem* items_, int64_t max_items, const int32_t* counters)
+      : items(items_), end(items_ + max_items), front(vjp_planned(counters, kVpItems)), total(front + vjp_planned(counters, kVpParts)) {}
+  __device__ __forceinline__ VjpItem at(int i) const { return load_item(i < front ? items + i : end - 1 - (i - front)); }
+};
 
 // zero gradients of one primitive, by nthr threads (rows of 16-byte multiples; b = the tensors' bases aligned)
 __device__ __forceinline__ void vjp_zero(const VjpOut& o, int prim, int aligned, int t, int nthr) {

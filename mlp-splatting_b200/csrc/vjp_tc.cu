@@ -19,12 +19,14 @@
 // The gradient accumulators stay in tensor memory for the whole segment and are written, divided by the scale, to the
 // primitive's gradient tensors, or -- for a primitive of several segments -- to the segment's partial row.
 //
-// What bounds it: the chain of MMA round trips of a block (operand tile complete -> fence -> CTA barrier -> one thread
-// issues and commits -> everyone waits on the mbarrier, bounded), about a microsecond each; bytes (weights in, gradients
-// out, 48 B per record) would take a quarter of the time.  So the chain is kept short -- with saved masks the adjoint
-// chain does not depend on the forward one, and the halves of D1 ride with layer 1 and layer 2: three round trips per
-// block instead of five -- the last one (the gradients) overlaps the next block's encoding, and the next block's
-// records and weights are loaded into registers while the current block's MMAs run.
+// What bounds it: the chain of a block (operand tile complete -> fence -> CTA barrier -> one thread issues and commits ->
+// everyone waits on the mbarrier, bounded): 7,300 cycles with three CTAs per SM, 6,700 with one, of which 1,700 are the issue of
+// the MMAs (47 cycles each, the time their operands take out of shared memory) and the rest instructions of the twelve warps;
+// bytes (weights in, gradients out, 48 B per record) would take a third of the time.  So the chain is kept short: with saved
+// masks the adjoint chain does not depend on the forward one, D1 rides with layer 1 and dW1 with layer 2, three round trips per
+// block; the last one (dW2, dW3) overlaps the next block's encoding, a finished segment's gradients leave and the next block's
+// records and weights arrive while layer 1 runs.  5.5 M records of 15,000 primitives, 35,000 more without records: 598 us with
+// dW1 in the last round trip, the gradients written between two blocks and weights loaded a row per lane, 546 so.  (Two threads per record, 256 per CTA: 840, by spills, and 855 with two CTAs per SM.)
 #include "frame.cuh"
 #include "tc.cuh"
 #include "vjp.cuh"
@@ -35,18 +37,20 @@ constexpr int kVjpRows = kVjpBlock, kVjpChunk = kVjpRows * 16;
 // chunk indices of the operand tiles
 constexpr int kVcE = 0, kVcOneE = 9, kVcH1 = 10, kVcOneH1 = 14, kVcH2 = 15, kVcOneH2 = 19, kVcD1 = 20, kVcD2 = 24,
               kVcD3 = 28, kVcEnd = 30;
-// weight operands ([K / 8 chunks][32 rows][8 elements], 512 bytes per chunk)
+// weight operands ([K / 8 chunks][32 rows][8 elements]); a chunk is 512 bytes and 16 more, so that the lanes of a warp, which
+// hold consecutive k of a row or two, store into different banks
+constexpr int kVjpWChunk = 528;
 constexpr int kVoW1 = kVcEnd * kVjpChunk;          // W1[h][j], 10 chunks (the last one zero: it meets the ones behind E)
-constexpr int kVoW2 = kVoW1 + 10 * 512;            // W2[q][h], 4 chunks
-constexpr int kVoW3 = kVoW2 + 4 * 512;             // W3[c][h], rounded to the operand format, as FP32: [32][4]
+constexpr int kVoW2 = kVoW1 + 10 * kVjpWChunk;     // W2[q][h], 4 chunks
+constexpr int kVoW3 = kVoW2 + 4 * kVjpWChunk;      // W3[c][h], rounded to the operand format, as FP32: [4][32]
 constexpr int kVoBias = kVoW3 + 512;               // b1[32], b2[32] as FP32
 constexpr int kVoBar = kVoBias + 256;
 constexpr int kVjpSmem = kVoBar + 16;
-// tensor memory: [0,32) layers, [32,64) dW1^T, [64,112) dW2^T | dW3^T, [112,128) one half of D1
-constexpr int kVjpTmemCols = 128, kVtG1 = 32, kVtG2 = 64, kVtD1 = 112;
+// tensor memory: 128 columns: [0,32) layers, [32,64) dW1^T, [64,112) dW2^T | dW3^T; and 32 of their own: D1
+constexpr int kVjpTmemCols = 128, kVjpTmemColsD1 = 32, kVtG1 = 32, kVtG2 = 64;
 constexpr int kVjpCtas = 3;
 static_assert((kVcH1 + 16) * kVjpChunk <= kVoW1, "an M = 128 window from any tile start stays inside the tiles");
-static_assert(kVjpCtas * (kVjpSmem + 1024) <= 227 * 1024, "resident CTAs");
+static_assert(kVjpCtas * (kVjpSmem + 1024) <= 227 * 1024 && kVjpCtas * (kVjpTmemCols + kVjpTmemColsD1) <= 512, "resident CTAs");
 
 // bits 15 / 16 of the instruction descriptor: A / B is MN-major
 constexpr uint32_t kMnA = 1u << 15, kMnB = 1u << 16;
@@ -64,18 +68,23 @@ __device__ __forceinline__ float2 unpack_h2(uint32_t w) {
 
 // ReLU + rounding of 32 accumulator columns (+ FP32 bias) into a hidden tile; returns the sign mask
 template <bool BF16>
-__device__ __forceinline__ uint32_t vjp_hidden(const uint32_t (&acc)[32], const float* __restrict__ bias, char* dst) {
+__device__ __forceinline__ uint32_t vjp_hidden(const uint32_t (&acc)[32], const float4* __restrict__ bias, char* dst) {
   uint32_t sign = 0u;
 #pragma unroll
   for (int kc = 0; kc < 4; ++kc) {
     uint32_t w[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < 4; q += 2) {
       const int j = kc * 8 + q * 2;
-      const float v0 = __uint_as_float(acc[j]) + bias[j], v1 = __uint_as_float(acc[j + 1]) + bias[j + 1];
+      const float4 b = bias[j / 4];
+      const float v0 = __uint_as_float(acc[j]) + b.x, v1 = __uint_as_float(acc[j + 1]) + b.y;
+      const float v2 = __uint_as_float(acc[j + 2]) + b.z, v3 = __uint_as_float(acc[j + 3]) + b.w;
       sign |= (v0 > 0.f ? 1u : 0u) << j;
       sign |= (v1 > 0.f ? 1u : 0u) << (j + 1);
+      sign |= (v2 > 0.f ? 1u : 0u) << (j + 2);
+      sign |= (v3 > 0.f ? 1u : 0u) << (j + 3);
       w[q] = pack_h2_relu<BF16>(v0, v1);
+      w[q + 1] = pack_h2_relu<BF16>(v2, v3);
     }
     *reinterpret_cast<uint4*>(dst + kc * kVjpChunk) = make_uint4(w[0], w[1], w[2], w[3]);
   }
@@ -99,18 +108,45 @@ __device__ __forceinline__ void vjp_adjoint(const uint32_t (&acc)[N], uint32_t m
   }
 }
 
+// pairs of FP32 values: two IEEE operations in one instruction
+__device__ __forceinline__ uint64_t pair_of(float x, float y) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ uint64_t pair_fma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t pair_mul(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
 // D2 = (D3 W3) * mask2 of one record, from the rounded operands
 template <bool BF16>
-__device__ __forceinline__ void vjp_d2(uint32_t d01, uint32_t d23, uint32_t m2, const float4* __restrict__ w3, char* dst) {
+__device__ __forceinline__ void vjp_d2(uint32_t d01, uint32_t d23, uint32_t m2, const float* __restrict__ w3, char* dst) {
   const float2 a = unpack_h2<BF16>(d01), b = unpack_h2<BF16>(d23);
+  const uint64_t d[4] = {pair_of(a.x, a.x), pair_of(a.y, a.y), pair_of(b.x, b.x), pair_of(b.y, b.y)};
 #pragma unroll
   for (int kc = 0; kc < 4; ++kc) {
     float v[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float4 w = w3[kc * 8 + i];
-      const float s = fmaf(a.x, w.x, fmaf(a.y, w.y, fmaf(b.x, w.z, b.y * w.w)));
-      v[i] = ((m2 >> (kc * 8 + i)) & 1u) ? s : 0.f;
+    for (int i = 0; i < 8; i += 4) {
+      ulonglong2 w = *reinterpret_cast<const ulonglong2*>(w3 + 3 * kGH + kc * 8 + i);
+      uint64_t s0 = pair_mul(d[3], w.x), s1 = pair_mul(d[3], w.y);
+#pragma unroll
+      for (int c = 2; c >= 0; --c) {
+        w = *reinterpret_cast<const ulonglong2*>(w3 + c * kGH + kc * 8 + i);
+        s0 = pair_fma(d[c], w.x, s0);
+        s1 = pair_fma(d[c], w.y, s1);
+      }
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(v[i]), "=f"(v[i + 1]) : "l"(s0));
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(v[i + 2]), "=f"(v[i + 3]) : "l"(s1));
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[i + u] = ((m2 >> (kc * 8 + i + u)) & 1u) ? v[i + u] : 0.f;
     }
     *reinterpret_cast<uint4*>(dst + kc * kVjpChunk) = pack8<BF16>(v);
   }
@@ -121,20 +157,44 @@ __device__ __forceinline__ void vjp_d2(uint32_t d01, uint32_t d23, uint32_t m2, 
 template <bool BF16, bool MASKS>
 __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
     const float* __restrict__ x6, const float* __restrict__ d4, const int32_t* __restrict__ masks,
-    const VjpItem* __restrict__ items, const VjpItem* __restrict__ multi, int n, int aligned, int32_t* __restrict__ counters,
+    const VjpItem* __restrict__ items, int64_t max_items, const VjpItem* __restrict__ multi, int n, int aligned, int32_t* __restrict__ counters,
     const float* __restrict__ freq, const float* __restrict__ att, const float* __restrict__ W1, const float* __restrict__ b1, const float* __restrict__ W2,
     const float* __restrict__ b2, const float* __restrict__ W3, int vec, float scale, VjpOut out, float* __restrict__ partial) {
   chain_wait();
   chain_release();
   extern __shared__ __align__(128) char smem[];
-  const int G = vjp_planned(counters, kVpItems), E = vjp_planned(counters, kVpEmpty);
+  const VjpList list(items, max_items, counters);
+  const int G = list.total, E = vjp_planned(counters, kVpEmpty);
   const int idx = blockIdx.x;
-  int empty = blockIdx.x;                        // primitives without records, one between two waits
   const int tid = threadIdx.x, warp = tid >> 5;
+  // primitives without records, one between two waits; the number of the next one is on its way
+  int empty = blockIdx.x, empty_prim = empty < E ? __ldg(&multi[n - 1 - empty].prim) : 0;
   auto zero_next = [&]() {
     if (empty >= E) return;
-    vjp_zero(out, __ldg(&multi[n - 1 - empty].prim), aligned, tid, kVjpRows);
+    const int prim = empty_prim;
     empty += (int)gridDim.x;
+    if (empty < E) empty_prim = __ldg(&multi[n - 1 - empty].prim);
+    if (!aligned) {
+      vjp_zero(out, prim, aligned, tid, kVjpRows);
+      return;
+    }
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4* w1 = reinterpret_cast<float4*>(out.W1 + prim * out.sW1) + tid;
+    float4* w2 = reinterpret_cast<float4*>(out.W2 + prim * out.sW2) + tid;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w1[i * kVjpRows] = zero;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) w2[i * kVjpRows] = zero;
+    if (tid < 64) {
+      w1[4 * kVjpRows] = zero;
+    } else if (tid < 96) {
+      reinterpret_cast<float4*>(out.W3 + prim * out.sW3)[tid - 64] = zero;
+    } else {
+      const int i = tid - 96;
+      if (i < 8) reinterpret_cast<float4*>(out.b1 + prim * out.sb1)[i] = zero;
+      else if (i < 16) reinterpret_cast<float4*>(out.b2 + prim * out.sb2)[i - 8] = zero;
+      else if (i == 16) *reinterpret_cast<float4*>(out.b3 + prim * out.sb3) = zero;
+    }
   };
   if (idx >= G) {
     while (empty < E) zero_next();
@@ -149,7 +209,10 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
     mbar_init(bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 0) tmem_alloc(smem_u32(&s_misc[0]), kVjpTmemCols);
+  if (warp == 0) {      // together three CTAs' allocations fit an SM, so neither waits for good while the first is held
+    tmem_alloc(smem_u32(&s_misc[0]), kVjpTmemCols, true);
+    tmem_alloc(smem_u32(&s_misc[1]), kVjpTmemColsD1);
+  }
   // segments differ tenfold in length, so a CTA takes its first by its number and the others from a counter, two ahead
   __shared__ int s_next;
   auto draw = [&]() { if (tid == 0) s_next = (int)gridDim.x + atomicAdd(counters + kVpNext, 1); };
@@ -162,7 +225,7 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
       const uint32_t v = (chunk == kVcOneE || chunk == kVcOneH1 || chunk == kVcOneH2) ? one2 : 0u;
       *reinterpret_cast<uint4*>(smem + (size_t)i * 16) = make_uint4(v, v, v, v);
     }
-    if (tid < 32) *reinterpret_cast<uint4*>(smem + kVoW1 + 9 * 512 + tid * 16) = make_uint4(0u, 0u, 0u, 0u);
+    if (tid < 32) *reinterpret_cast<uint4*>(smem + kVoW1 + 9 * kVjpWChunk + tid * 16) = make_uint4(0u, 0u, 0u, 0u);
   }
   float mult[6];
 #pragma unroll
@@ -170,11 +233,10 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = s_misc[0];
-  const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
+  const uint32_t tmem = s_misc[0], tmem_d1 = s_misc[1];
+  const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16), trow_d1 = tmem_d1 + ((uint32_t)(warp * 32) << 16);
 
   constexpr uint32_t idesc_h = instr_desc(kVjpRows, 32, BF16), idesc_d1 = instr_desc(kVjpRows, 32, BF16) | kMnB,
-                     idesc_d1h = instr_desc(kVjpRows, 16, BF16) | kMnB,
                      idesc_g1 = instr_desc(kVjpRows, 32, BF16) | kMnA | kMnB, idesc_g2 = instr_desc(kVjpRows, 48, BF16) | kMnA | kMnB;
   auto tile = [&](int chunk) { return sb + (uint32_t)chunk * kVjpChunk; };
   // record-major A operand (K-major): K chunks a chunk apart, groups of eight records 128 bytes apart
@@ -182,19 +244,20 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
   // MN-major operand: groups of eight elements a chunk apart, groups of eight records 128 bytes apart
   auto mn = [&](int chunk) { return smem_desc(tile(chunk), 128, kVjpChunk); };
   auto adv = [](uint64_t desc, int bytes) { return desc + (uint64_t)(bytes >> 4); };
-  const uint64_t w1_desc = smem_desc(sb + kVoW1, 512, 128), w2_desc = smem_desc(sb + kVoW2, 512, 128);
-  const uint64_t w2t_desc = smem_desc(sb + kVoW2, 128, 512);      // N = h (a chunk per eight), K = q (128 bytes per eight)
+  const uint64_t w1_desc = smem_desc(sb + kVoW1, kVjpWChunk, 128), w2_desc = smem_desc(sb + kVoW2, kVjpWChunk, 128);
+  const uint64_t w2t_desc = smem_desc(sb + kVoW2, 128, kVjpWChunk);      // N = h (a chunk per eight), K = q (128 bytes per eight)
 
   char* my = smem + tid * 16;
   uint32_t ph = 0u;
   bool ok = true;
-  // tile writes visible to the tensor core, tensor-memory reads retired, then one thread issues and commits; false in all
-  // threads when a wait has given up in one
+  // tile writes visible to the tensor core, tensor-memory reads retired, then one thread (of the warp that has no part in
+  // emit) issues and commits; false in all threads when a wait has given up in one
+  constexpr int kIssueWarp = 3;
   auto issue_phase = [&](auto issue) -> bool {
     fence_async_smem();
     tc_fence_before();
     if (!__syncthreads_and(ok)) return false;
-    if (warp == 0) {
+    if (warp == kIssueWarp) {
       tc_fence_after();
       if (elect_one()) {
         issue();
@@ -237,36 +300,40 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
       if (MASKS) { rm1 = (uint32_t)__ldg(masks + r * 2); rm2 = (uint32_t)__ldg(masks + r * 2 + 1); }
     }
   };
-  // W1 as 288 groups of eight consecutive k of one row, W2 as 128, W3 and the biases one value per thread
-  float wv[4][8], wr3 = 0.f, wrb = 0.f;
-  auto load8 = [&](const float* p, float (&v)[8]) {
-    if (vec) {
-      const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
-      v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = __ldg(p + i);
-    }
+  // W1 as 576 groups of four consecutive k of one row, W2 as 256, both in the order of memory, W3 and the biases one value per
+  // thread (eight k of a row per thread, a row per lane, took 32 cycles of the load unit per load instead of four)
+  float4 wv[7];
+  float wr3 = 0.f, wrb = 0.f;
+  auto load4 = [&](const float* p) {
+    return vec ? __ldg(reinterpret_cast<const float4*>(p)) : make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
   };
   auto load_weights = [&](int prim) {
     const float* w1 = W1 + (size_t)prim * (kGH * kGIN);
 #pragma unroll
-    for (int u = 0; u < 3; ++u) {
+    for (int u = 0; u < 5; ++u) {
       const int g = u * kVjpRows + tid;
-      if (u < 2 || g < 288) load8(w1 + (g & 31) * kGIN + (g >> 5) * 8, wv[u]);
+      if (u < 4 || g < 576) wv[u] = load4(w1 + 4 * g);
     }
-    load8(W2 + (size_t)prim * (kGH * kGH) + (tid & 31) * kGH + (tid >> 5) * 8, wv[3]);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) wv[5 + u] = load4(W2 + (size_t)prim * (kGH * kGH) + 4 * (u * kVjpRows + tid));
     wr3 = __ldg(W3 + (size_t)prim * (4 * kGH) + tid);
     if (tid < 64) wrb = __ldg((tid < 32 ? b1 : b2) + (size_t)prim * kGH + (tid & 31));
   };
   auto store_weights = [&]() {
+    auto put4 = [&](int off, int h, int k, const float4& v) {
+      *reinterpret_cast<uint2*>(smem + off + (k >> 3) * kVjpWChunk + h * 16 + (k & 4) * 2) = make_uint2(pack_h2<BF16>(v.x, v.y), pack_h2<BF16>(v.z, v.w));
+    };
 #pragma unroll
-    for (int u = 0; u < 3; ++u) {
-      const int g = u * kVjpRows + tid;
-      if (u < 2 || g < 288) *reinterpret_cast<uint4*>(smem + kVoW1 + (g >> 5) * 512 + (g & 31) * 16) = pack8<BF16>(wv[u]);
+    for (int u = 0; u < 5; ++u) {
+      const int g = u * kVjpRows + tid, h = g / (kGIN / 4);
+      if (u < 4 || g < 576) put4(kVoW1, h, 4 * (g - h * (kGIN / 4)), wv[u]);
     }
-    *reinterpret_cast<uint4*>(smem + kVoW2 + (tid >> 5) * 512 + (tid & 31) * 16) = pack8<BF16>(wv[3]);
-    s_w3[(tid & 31) * 4 + (tid >> 5)] = unpack_h2<BF16>(pack_h2<BF16>(wr3, 0.f)).x;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int g = u * kVjpRows + tid;
+      put4(kVoW2, g / (kGH / 4), 4 * (g % (kGH / 4)), wv[5 + u]);
+    }
+    s_w3[tid] = unpack_h2<BF16>(pack_h2<BF16>(wr3, 0.f)).x;
     if (tid < 64) s_bias[tid] = wrb;
   };
   // the gradients of a finished segment: accumulator lane = input of the layer (its ones lane: the bias), column = output
@@ -313,9 +380,9 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
     }
   };
 
-  VjpItem it = load_item(items + idx), it_n = it, it_p = it;
+  VjpItem it = list.at(idx), it_n = it, it_p = it;
   bool has_n = s_next < G;
-  if (has_n) it_n = load_item(items + s_next);
+  if (has_n) it_n = list.at(s_next);
   __syncthreads();                 // before the next draw
   load_weights(it.prim);
   load_rec(it, 0);
@@ -325,7 +392,7 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
   for (;;) {
     // ---- encoding (index c * 6 + f holds sin, 36 + c * 6 + f holds cos: scannet/cumodel.py:183-195) and D3,
     //      into registers while the previous block's gradient MMAs finish ----
-    const bool valid = sub + tid < it.rows;
+    //      (rows past the segment's end encode zeros; their adjoints are zero, so they add nothing to a gradient)
     uint32_t ew[36];                                            // 32-bit word = two consecutive encoding entries
 #pragma unroll
     for (int c = 0; c < 6; ++c) {
@@ -334,15 +401,14 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
         float s0, c0, s1, c1;
         __sincosf(rx[c] * mult[2 * g], &s0, &c0);
         __sincosf(rx[c] * mult[2 * g + 1], &s1, &c1);
-        ew[3 * c + g] = valid ? pack_h2<BF16>(s0, s1) : 0u;
-        ew[18 + 3 * c + g] = valid ? pack_h2<BF16>(c0, c1) : 0u;
+        ew[3 * c + g] = pack_h2<BF16>(s0, s1);
+        ew[18 + 3 * c + g] = pack_h2<BF16>(c0, c1);
       }
     }
     const uint32_t d01 = pack_h2<BF16>(rg.x * scale, rg.y * scale), d23 = pack_h2<BF16>(rg.z * scale, rg.w * scale);
     uint32_t m1 = rm1, m2 = rm2;
     if (pending) {
       wait_phase();
-      if (finished && ok) emit(it_p);
     }
     if (sub == 0) store_weights();
 #pragma unroll
@@ -351,20 +417,22 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
     *reinterpret_cast<uint4*>(my + kVcD3 * kVjpChunk) = make_uint4(d01, d23, 0u, 0u);
     if (MASKS) {
       if (sub == 0) __syncthreads();                            // W3 of the new primitive
-      vjp_d2<BF16>(d01, d23, m2, reinterpret_cast<const float4*>(s_w3), my + kVcD2 * kVjpChunk);
+      vjp_d2<BF16>(d01, d23, m2, s_w3, my + kVcD2 * kVjpChunk);
     }
     if (sub == 0) draw();                                       // read after the barrier of this layer, at the segment's last block
     // ---- layer 1: K = 80 (the ones behind E meet the zero chunk of W1); with masks the first half of D1 ----
     ok = issue_phase([&]() {
       const uint64_t a = a_rows(kVcE);
 #pragma unroll
-      for (int ks = 0; ks < 5; ++ks) mma_f16(tmem, adv(a, ks * 2 * kVjpChunk), adv(w1_desc, ks * 2 * 512), idesc_h, ks > 0);
+      for (int ks = 0; ks < 5; ++ks) mma_f16(tmem, adv(a, ks * 2 * kVjpChunk), adv(w1_desc, ks * 2 * kVjpWChunk), idesc_h, ks > 0);
       if (MASKS) {
 #pragma unroll
-        for (int ks = 0; ks < 2; ++ks) mma_f16(tmem + kVtD1, adv(a_rows(kVcD2), ks * 2 * kVjpChunk), adv(w2t_desc, ks * 256), idesc_d1h, ks > 0);
+        for (int ks = 0; ks < 2; ++ks) mma_f16(tmem_d1, adv(a_rows(kVcD2), ks * 2 * kVjpChunk), adv(w2t_desc, ks * 256), idesc_d1, ks > 0);
       }
     });
     if (!ok) break;
+    // ---- the finished segment's gradients, while layer 1 runs ----
+    if (pending && finished && ok) emit(it_p);
     // ---- the next step's loads, in flight from here on ----
     const int cnt = min(kVjpRows, it.rows - sub);
     const bool last = sub + kVjpRows >= it.rows;
@@ -380,7 +448,7 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
       load_rec(it, 0);
       load_weights(it.prim);
       has_n = s_next < G;
-      if (has_n) it_n = load_item(items + s_next);
+      if (has_n) it_n = list.at(s_next);
     } else {
       more = false;
     }
@@ -389,39 +457,39 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
     {
       uint32_t acc[32];
       tmem_ld32(trow, acc);
-      const uint32_t sign = vjp_hidden<BF16>(acc, s_bias, my + kVcH1 * kVjpChunk);
+      const uint32_t sign = vjp_hidden<BF16>(acc, reinterpret_cast<const float4*>(s_bias), my + kVcH1 * kVjpChunk);
       if (!MASKS) m1 = sign;
     }
     if (MASKS) {
-      uint32_t acc[16];
-      tmem_ld16(trow + kVtD1, acc);
-      vjp_adjoint<BF16, 16>(acc, m1, my + kVcD1 * kVjpChunk);
+      uint32_t acc[32];
+      tmem_ld32(trow_d1, acc);
+      vjp_adjoint<BF16, 32>(acc, m1, my + kVcD1 * kVjpChunk);
     }
-    // ---- layer 2; with masks the second half of D1 ----
+    // ---- layer 2; with masks dW1 behind it, contracting over the block's records, 16 per MMA ----
+    auto grad1 = [&]() {
+      const uint64_t e = mn(kVcE), d1 = mn(kVcD1);
+      const int steps = (cnt + 15) >> 4;
+      for (int ks = 0; ks < steps; ++ks) mma_f16(tmem + kVtG1, adv(e, ks * 256), adv(d1, ks * 256), idesc_g1, (sub_c > 0 || ks > 0) ? 1u : 0u);
+    };
     ok = issue_phase([&]() {
       const uint64_t a = a_rows(kVcH1);
 #pragma unroll
-      for (int ks = 0; ks < 2; ++ks) mma_f16(tmem, adv(a, ks * 2 * kVjpChunk), adv(w2_desc, ks * 2 * 512), idesc_h, ks > 0);
-      if (MASKS) {
-#pragma unroll
-        for (int ks = 0; ks < 2; ++ks)
-          mma_f16(tmem + kVtD1, adv(a_rows(kVcD2), ks * 2 * kVjpChunk), adv(w2t_desc, 2 * 512 + ks * 256), idesc_d1h, ks > 0);
-      }
+      for (int ks = 0; ks < 2; ++ks) mma_f16(tmem, adv(a, ks * 2 * kVjpChunk), adv(w2_desc, ks * 2 * kVjpWChunk), idesc_h, ks > 0);
     });
+    if (MASKS && ok && warp == kIssueWarp) {                             // not waited for before the last phase
+      if (elect_one()) grad1();
+      __syncwarp();
+    }
     if (!ok) break;
     wait_phase();
     {
       uint32_t acc[32];
       tmem_ld32(trow, acc);
-      const uint32_t sign = vjp_hidden<BF16>(acc, s_bias + 32, my + kVcH2 * kVjpChunk);
+      const uint32_t sign = vjp_hidden<BF16>(acc, reinterpret_cast<const float4*>(s_bias + 32), my + kVcH2 * kVjpChunk);
       if (!MASKS) m2 = sign;
     }
-    if (MASKS) {
-      uint32_t acc[16];
-      tmem_ld16(trow + kVtD1, acc);
-      vjp_adjoint<BF16, 16>(acc, m1 >> 16, my + (kVcD1 + 2) * kVjpChunk);
-    } else {
-      vjp_d2<BF16>(d01, d23, m2, reinterpret_cast<const float4*>(s_w3), my + kVcD2 * kVjpChunk);
+    if (!MASKS) {
+      vjp_d2<BF16>(d01, d23, m2, s_w3, my + kVcD2 * kVjpChunk);
       ok = issue_phase([&]() {
 #pragma unroll
         for (int ks = 0; ks < 2; ++ks) mma_f16(tmem, adv(a_rows(kVcD2), ks * 2 * kVjpChunk), adv(w2t_desc, ks * 256), idesc_d1, ks > 0);
@@ -432,15 +500,12 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
       tmem_ld32(trow, acc);
       vjp_adjoint<BF16, 32>(acc, m1, my + kVcD1 * kVjpChunk);
     }
-    // ---- gradients: contraction over the block's records, 16 per MMA ----
+    // ---- dW2 and dW3 (without masks dW1 too) ----
     ok = issue_phase([&]() {
-      const uint64_t e = mn(kVcE), h = mn(kVcH1), d1 = mn(kVcD1), d23t = mn(kVcD2);
+      if (!MASKS) grad1();
+      const uint64_t h = mn(kVcH1), d23t = mn(kVcD2);
       const int steps = (cnt + 15) >> 4;
-      for (int ks = 0; ks < steps; ++ks) {
-        const uint32_t acc = (sub_c > 0 || ks > 0) ? 1u : 0u;
-        mma_f16(tmem + kVtG1, adv(e, ks * 256), adv(d1, ks * 256), idesc_g1, acc);
-        mma_f16(tmem + kVtG2, adv(h, ks * 256), adv(d23t, ks * 256), idesc_g2, acc);
-      }
+      for (int ks = 0; ks < steps; ++ks) mma_f16(tmem + kVtG2, adv(h, ks * 256), adv(d23t, ks * 256), idesc_g2, (sub_c > 0 || ks > 0) ? 1u : 0u);
     });
     if (!ok) break;
     pending = true;
@@ -457,7 +522,10 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
   if (!ok && tid == 0) atomicOr(counters + kVpFlag, 2);
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_free(tmem, kVjpTmemCols);
+  if (warp == 0) {
+    tmem_free(tmem, kVjpTmemCols);
+    tmem_free(tmem_d1, kVjpTmemColsD1);
+  }
 }
 
 int launch_grouped_vjp_tc(bool bf16, const float* x6, const float* d4, const int32_t* masks, const VjpItem* items,
@@ -475,8 +543,8 @@ int launch_grouped_vjp_tc(bool bf16, const float* x6, const float* d4, const int
   const int vec = ((reinterpret_cast<uintptr_t>(sc->W1) | reinterpret_cast<uintptr_t>(sc->W2)) & 15) == 0 &&
                   (reinterpret_cast<uintptr_t>(x6) & 7) == 0;
   const int grid = (int)std::min<int64_t>(std::max<int64_t>(max_items, sc->n), (int64_t)sm_count() * kVjpCtas);     // CTAs without segments write zeros
-  return cuda_check(launch_chained(kernel, dim3(grid), dim3(kVjpRows), kVjpSmem, st, x6, d4, masks, items, multi, sc->n, vjp_aligned(out),
-                                   counters, sc->freq, sc->att,
+  return cuda_check(launch_chained(kernel, dim3(grid), dim3(kVjpRows), kVjpSmem, st, x6, d4, masks, items, max_items, multi, sc->n, vjp_aligned(out), counters,
+                                   sc->freq, sc->att,
                                    sc->W1, sc->b1, sc->W2, sc->b2, sc->W3, vec, scale, out, partial),
                     "grouped_vjp_tc");
 }
