@@ -415,13 +415,15 @@ __global__ void __launch_bounds__(256) k_vjp_plan_layout(const int64_t* __restri
   if (!ok) atomicOr(counters + kVpFlag, kVpBadPlan);
 }
 
-// IEEE FP32 on the CUDA cores, sums in record order.  A CTA of 128 threads takes 64 records at a time; everything per
-// record lies transposed in shared memory ([quantity][record], rows of 68 floats: 16-byte reads of eight different rows
-// meet eight different bank groups), so that the record-major products (layers, adjoints) give a thread a tile of four
-// records x four units and the contractions over the records (the gradients) 2 x 9 + 2 x 4 + 1 sums in registers, both
-// fed by 16-byte reads: 16 multiply-adds per two reads and 104 per nineteen.  Bound: FP32 issue (about 8,000 multiply-adds
-// per record).  A thread-per-record version with one 4-byte read per multiply-add took 616 us where this one takes
-// 150 us (117,000 records of 2,000 primitives).
+// IEEE FP32 on the CUDA cores, sums in record order over each half of the blocks.  A CTA of 128 threads takes 64 records at a
+// time; everything per record lies transposed in shared memory ([quantity][record], rows of 68 floats), so that the record-major
+// products (layers, adjoints) give a thread a tile of four records x four units and the contractions over the records (the
+// gradients) 4 x 9 + 4 x 4 + 2 sums in registers over 32 of the records, both fed by 16-byte reads.  Bound: what goes from shared
+// memory into registers, 128 bytes a cycle whether lanes read the same bytes or not (a tile of a x b costs a + b floats for a b
+// multiply-adds), then issue: load unit 74 %, issue slots 65, multiply-adds 49.  With 2 x 9 + 2 x 4 + 1 sums over all 64 records
+// per thread, hidden rows that share banks, weights loaded one by one and all of a thread's sincosf in a row (a third of the
+// instruction cache), 5.5 M records of 15,000 primitives took 3,930 us, so 3,090; 0.8 M of 9,800 887 and 718.  A warp per
+// segment with tiles of 4 x 8 (38 KB, six warps per SM) 3,880 and 957, of 8 x 8 (52 KB, four) 4,920 and 1,160: too few warps.
 constexpr int kGfRec = 64, kGfThreads = 128, kGfRow = kGfRec + 4, kGfCtas = 3;
 constexpr int kGfE = 0, kGfH1 = kGfE + kGIN * kGfRow, kGfH2 = kGfH1 + kGH * kGfRow, kGfD1 = kGfH2 + kGH * kGfRow,
               kGfD2 = kGfD1 + kGH * kGfRow, kGfD3 = kGfD2 + kGH * kGfRow, kGfMask = kGfD3 + 4 * kGfRow,
@@ -430,6 +432,9 @@ constexpr int kGfE = 0, kGfH1 = kGfE + kGIN * kGfRow, kGfH2 = kGfH1 + kGH * kGfR
 constexpr int kGradSmem = kGfFloats * 4;
 static_assert(kGfCtas * (kGradSmem + 1024) <= 228 * 1024, "resident CTAs");
 
+// Where the records r .. r + 3 lie in a row of a hidden tile: every eight rows the records begin four places further on, so that
+// neither the eight rows that a tile of units is written to nor the eight that a gradient is read from share banks.
+__device__ __forceinline__ int gf_turn(int r, int row) { return (r + 4 * (row >> 3)) & (kGfRec - 1); }
 __device__ __forceinline__ void fma4(float4& a, float s, const float4 v) {
   a.x = fmaf(s, v.x, a.x); a.y = fmaf(s, v.y, a.y); a.z = fmaf(s, v.z, a.z); a.w = fmaf(s, v.w, a.w);
 }
@@ -442,13 +447,15 @@ __global__ void __launch_bounds__(kGfThreads, kGfCtas) k_grouped_vjp(
     const float* __restrict__ x6, const float* __restrict__ d4, const int32_t* __restrict__ masks,
     const VjpItem* __restrict__ items, int64_t max_items, int32_t* __restrict__ counters, const float* __restrict__ freq,
     const float* __restrict__ att, const float* __restrict__ W1, const float* __restrict__ b1, const float* __restrict__ W2,
-    const float* __restrict__ b2, const float* __restrict__ W3, float scale, VjpOut out, float* __restrict__ partial) {
+    const float* __restrict__ b2, const float* __restrict__ W3, int vec, float scale, VjpOut out, float* __restrict__ partial) {
   chain_wait();
   chain_release();
   extern __shared__ __align__(16) float sm[];
   const VjpList list(items, max_items, counters);
   const int tid = threadIdx.x;
-  const int hg = tid & 7, rg = tid >> 3;         // units 4 hg .. + 3 of records 4 rg .. + 3; gradient rows 2 rg, 2 rg + 1
+  const int hg = tid & 7, rg = tid >> 3;         // units 4 hg .. + 3 of records 4 rg .. + 3
+  // gradients: rows 4 gq .. + 3, inputs hg + 8 i, over the records of one half of a block
+  const int half = tid >> 6, gq = (tid >> 3) & 7, th = tid & 63;
   const float inv = 1.f / scale;
   bool bad = false;
   uint32_t* sMask = reinterpret_cast<uint32_t*>(sm + kGfMask);
@@ -461,23 +468,39 @@ __global__ void __launch_bounds__(kGfThreads, kGfCtas) k_grouped_vjp(
     const size_t p = (size_t)it.prim;
     __syncthreads();                             // the previous item's last block has been consumed
     if (tid == 0) s_next = (int)gridDim.x + atomicAdd(counters + kVpNext, 1);
+    // lane = row of W1 and W2, four consecutive inputs a time; the transposed stores are conflict-free (inputs one by one cost the
+    // load unit 32 cycles each)
+    auto row4 = [&](const float* w) {
+      return vec ? __ldg(reinterpret_cast<const float4*>(w)) : make_float4(__ldg(w), __ldg(w + 1), __ldg(w + 2), __ldg(w + 3));
+    };
+    const int wr = tid & 31;
+    auto put_t = [&](int off, int k, const float4& v) {
+      sm[off + k * kGH + wr] = v.x; sm[off + (k + 1) * kGH + wr] = v.y; sm[off + (k + 2) * kGH + wr] = v.z; sm[off + (k + 3) * kGH + wr] = v.w;
+    };
+    float4 w1v[5], w2v[2];
 #pragma unroll
-    for (int u = 0; u < 18; ++u) {               // W1 transposed: lane = row, so the stores are conflict-free
-      const int k = u * 4 + (tid >> 5), h = tid & 31;
-      sm[kGfW1T + k * kGH + h] = __ldg(W1 + p * (kGH * kGIN) + h * kGIN + k);
+    for (int u = 0; u < 5; ++u) {
+      const int k = (u * 4 + (tid >> 5)) * 4;
+      if (u < 4 || k < kGIN) w1v[u] = row4(W1 + p * (kGH * kGIN) + wr * kGIN + k);
     }
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int e = u * kGfThreads + tid, q = e >> 5, h = e & 31;
-      sm[kGfW2 + q * kGfW2Row + h] = __ldg(W2 + p * (kGH * kGH) + e);
-      const int k = u * 4 + (tid >> 5), r = tid & 31;
-      sm[kGfW2T + k * kGH + r] = __ldg(W2 + p * (kGH * kGH) + r * kGH + k);
+    for (int u = 0; u < 2; ++u) w2v[u] = row4(W2 + p * (kGH * kGH) + wr * kGH + (u * 4 + (tid >> 5)) * 4);
+#pragma unroll
+    for (int u = 0; u < 5; ++u) {
+      const int k = (u * 4 + (tid >> 5)) * 4;
+      if (u < 4 || k < kGIN) put_t(kGfW1T, k, w1v[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int k = (u * 4 + (tid >> 5)) * 4;
+      put_t(kGfW2T, k, w2v[u]);
+      *reinterpret_cast<float4*>(sm + kGfW2 + wr * kGfW2Row + k) = w2v[u];
     }
     sm[kGfW3 + tid] = __ldg(W3 + p * (4 * kGH) + tid);
     if (tid < 2 * kGH) sm[kGfB + tid] = tid < kGH ? __ldg(b1 + p * kGH + tid) : __ldg(b2 + p * kGH + tid - kGH);
-    float g1[2][9], g2[2][4], g3 = 0.f, gb = 0.f;
+    float g1[4][9], g2[4][4], g3[2] = {0.f, 0.f}, gb = 0.f, gb3 = 0.f;
 #pragma unroll
-    for (int a = 0; a < 2; ++a) {
+    for (int a = 0; a < 4; ++a) {
 #pragma unroll
       for (int i = 0; i < 9; ++i) g1[a][i] = 0.f;
 #pragma unroll
@@ -491,10 +514,13 @@ __global__ void __launch_bounds__(kGfThreads, kGfCtas) k_grouped_vjp(
         const int rec = tid & (kGfRec - 1), part = tid >> 6;
         const bool valid = rec < cnt;
         const int64_t r = it.start + sub + rec;
+        float xs[3];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
+        for (int c = 0; c < 3; ++c) xs[c] = valid ? __ldg(x6 + r * 6 + part * 3 + c) : 0.f;
+#pragma unroll 1
+        for (int c = 0; c < 3; ++c) {             // (a loop: eighteen sincosf in a row take a third of the instruction cache)
           const int cc = part * 3 + c;
-          const float v = valid ? __ldg(x6 + r * 6 + cc) : 0.f;
+          const float v = c == 0 ? xs[0] : (c == 1 ? xs[1] : xs[2]);
 #pragma unroll
           for (int f = 0; f < 6; ++f) {
             float sn, cs;
@@ -517,13 +543,18 @@ __global__ void __launch_bounds__(kGfThreads, kGfCtas) k_grouped_vjp(
       }
       // a tile acc[u] = (four records) of unit h4 + u; gate: the records' mask bits of that unit
       float4 acc[4];
-      auto product = [&](int x_off, int K, int w_off, int w_row) {
-#pragma unroll 8
+      auto product8 = [&](int x_off, int K, int w_off, int w_row, int r) {
+#pragma unroll
         for (int k = 0; k < K; ++k) {
-          const float4 x = *reinterpret_cast<const float4*>(sm + x_off + k * kGfRow + r4);
+          const float4 x = *reinterpret_cast<const float4*>(sm + x_off + k * kGfRow + r);
           const float4 w = *reinterpret_cast<const float4*>(sm + w_off + k * w_row + h4);
           fma4(acc[0], w.x, x); fma4(acc[1], w.y, x); fma4(acc[2], w.z, x); fma4(acc[3], w.w, x);
         }
+      };
+      auto product = [&](int x_off, int K, int w_off, int w_row, bool turned) {
+#pragma unroll 1
+        for (int k = 0; k < K; k += 8)
+          product8(x_off + k * kGfRow, 8, w_off + k * w_row, w_row, turned ? gf_turn(r4, k) : r4);
       };
       auto hidden = [&](int dst, uint32_t (&m)[4]) {
         if (!masks) { m[0] = m[1] = m[2] = m[3] = 0u; }
@@ -535,7 +566,7 @@ __global__ void __launch_bounds__(kGfThreads, kGfCtas) k_grouped_vjp(
             m[2] |= (a.z > 0.f ? 1u : 0u) << u; m[3] |= (a.w > 0.f ? 1u : 0u) << u;
           }
           a.x = a.x > 0.f ? a.x : 0.f; a.y = a.y > 0.f ? a.y : 0.f; a.z = a.z > 0.f ? a.z : 0.f; a.w = a.w > 0.f ? a.w : 0.f;
-          *reinterpret_cast<float4*>(sm + dst + (h4 + u) * kGfRow + r4) = a;
+          *reinterpret_cast<float4*>(sm + dst + (h4 + u) * kGfRow + gf_turn(r4, h4)) = a;
         }
       };
       auto adjoint = [&](int dst, const uint32_t (&m)[4]) {
@@ -544,7 +575,7 @@ __global__ void __launch_bounds__(kGfThreads, kGfCtas) k_grouped_vjp(
           float4 a = acc[u];
           a.x = ((m[0] >> u) & 1u) ? a.x : 0.f; a.y = ((m[1] >> u) & 1u) ? a.y : 0.f;
           a.z = ((m[2] >> u) & 1u) ? a.z : 0.f; a.w = ((m[3] >> u) & 1u) ? a.w : 0.f;
-          *reinterpret_cast<float4*>(sm + dst + (h4 + u) * kGfRow + r4) = a;
+          *reinterpret_cast<float4*>(sm + dst + (h4 + u) * kGfRow + gf_turn(r4, h4)) = a;
         }
       };
       auto start = [&](const float* bias) {
@@ -552,48 +583,76 @@ __global__ void __launch_bounds__(kGfThreads, kGfCtas) k_grouped_vjp(
         for (int u = 0; u < 4; ++u) { const float b = bias ? bias[h4 + u] : 0.f; acc[u] = make_float4(b, b, b, b); }
       };
       start(sm + kGfB);
-      product(kGfE, kGIN, kGfW1T, kGH);
+      product(kGfE, kGIN, kGfW1T, kGH, false);
       hidden(kGfH1, m1);
       __syncthreads();
       start(sm + kGfB + kGH);
-      product(kGfH1, kGH, kGfW2T, kGH);
+      product(kGfH1, kGH, kGfW2T, kGH, true);
       hidden(kGfH2, m2);
       start(nullptr);
-      product(kGfD3, 4, kGfW3, kGH);
+      product8(kGfD3, 4, kGfW3, kGH, r4);
       adjoint(kGfD2, m2);
       __syncthreads();
       start(nullptr);
-      product(kGfD2, kGH, kGfW2, kGfW2Row);
+      product(kGfD2, kGH, kGfW2, kGfW2Row, true);
       adjoint(kGfD1, m1);
       __syncthreads();
-      // ---- sums over the block's records, four at a time (rows past the last record hold zero adjoints) ----
-      const int gr = rg * 2;
-      for (int r = 0; r < cnt; r += 4) {
+      // ---- sums over the records of the thread's half of the block, four at a time (rows past the last record hold zero adjoints) ----
+      const int gr = gq * 4, r_end = min(cnt, (half + 1) * (kGfRec / 2));
+      for (int r = half * (kGfRec / 2); r < r_end; r += 4) {
         auto at4 = [&](int off, int row) { return *reinterpret_cast<const float4*>(sm + off + row * kGfRow + r); };
+        auto turned4 = [&](int off, int row, int turn) { return *reinterpret_cast<const float4*>(sm + off + row * kGfRow + gf_turn(r, turn)); };
+        auto sum4 = [](float s, const float4 v) { return ((s + v.x) + v.y) + v.z + v.w; };
         {
-          const float4 a0 = at4(kGfD1, gr), a1 = at4(kGfD1, gr + 1);
+          float4 d[4];
+#pragma unroll
+          for (int a = 0; a < 4; ++a) d[a] = turned4(kGfD1, gr + a, gr);
 #pragma unroll
           for (int i = 0; i < 9; ++i) {
             const float4 e = at4(kGfE, hg + 8 * i);
-            g1[0][i] = dot4(g1[0][i], a0, e);
-            g1[1][i] = dot4(g1[1][i], a1, e);
+#pragma unroll
+            for (int a = 0; a < 4; ++a) g1[a][i] = dot4(g1[a][i], d[a], e);
           }
         }
         {
-          const float4 a0 = at4(kGfD2, gr), a1 = at4(kGfD2, gr + 1);
+          float4 d[4];
+#pragma unroll
+          for (int a = 0; a < 4; ++a) d[a] = turned4(kGfD2, gr + a, gr);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            const float4 e = at4(kGfH1, hg + 8 * i);
-            g2[0][i] = dot4(g2[0][i], a0, e);
-            g2[1][i] = dot4(g2[1][i], a1, e);
+            const float4 e = turned4(kGfH1, hg + 8 * i, 8 * i);
+#pragma unroll
+            for (int a = 0; a < 4; ++a) g2[a][i] = dot4(g2[a][i], d[a], e);
           }
         }
-        g3 = dot4(g3, at4(kGfD3, tid >> 5), at4(kGfH2, tid & 31));
-        if (tid < 68) {
-          const float4 v = tid < 32 ? at4(kGfD1, tid) : (tid < 64 ? at4(kGfD2, tid - 32) : at4(kGfD3, tid - 64));
-          gb = ((gb + v.x) + v.y) + v.z + v.w;
+        {
+          const float4 h = turned4(kGfH2, th & 31, th & 31);
+#pragma unroll
+          for (int c = 0; c < 2; ++c) g3[c] = dot4(g3[c], at4(kGfD3, (th >> 5) * 2 + c), h);
         }
+        gb = sum4(gb, turned4(th < 32 ? kGfD1 : kGfD2, th & 31, th & 31));
+        if (th < 4) gb3 = sum4(gb3, at4(kGfD3, th));
       }
+    }
+    // the halves' sums meet in shared memory: the first half adds and writes
+    {
+      auto each = [&](auto f) {
+        int j = 0;
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+#pragma unroll
+          for (int i = 0; i < 9; ++i) f(g1[a][i], j++);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) f(g2[a][i], j++);
+        }
+        f(g3[0], j++); f(g3[1], j++); f(gb, j++); f(gb3, j++);
+      };
+      static_assert(56 * 64 <= kGfH1 - kGfE, "room for one half's sums in the encoding's tile");
+      __syncthreads();                           // the last block's rows have been consumed
+      if (half == 1) each([&](float& v, int j) { sm[kGfE + j * 64 + th] = v; });
+      __syncthreads();
+      if (half == 1) continue;
+      each([&](float& v, int j) { v += sm[kGfE + j * 64 + th]; });
     }
     const VjpOut o = vjp_row(out, partial, it);
     auto put = [&](float* dst, float v) {
@@ -602,16 +661,16 @@ __global__ void __launch_bounds__(kGfThreads, kGfCtas) k_grouped_vjp(
       *dst = g;
     };
 #pragma unroll
-    for (int a = 0; a < 2; ++a) {
+    for (int a = 0; a < 4; ++a) {
 #pragma unroll
-      for (int i = 0; i < 9; ++i) put(o.W1 + (rg * 2 + a) * kGIN + hg + 8 * i, g1[a][i]);
+      for (int i = 0; i < 9; ++i) put(o.W1 + (gq * 4 + a) * kGIN + hg + 8 * i, g1[a][i]);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) put(o.W2 + (rg * 2 + a) * kGH + hg + 8 * i, g2[a][i]);
+      for (int i = 0; i < 4; ++i) put(o.W2 + (gq * 4 + a) * kGH + hg + 8 * i, g2[a][i]);
     }
-    put(o.W3 + tid, g3);
-    if (tid < 32) put(o.b1 + tid, gb);
-    else if (tid < 64) put(o.b2 + tid - 32, gb);
-    else if (tid < 68) put(o.b3 + tid - 64, gb);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) put(o.W3 + ((th >> 5) * 2 + c) * kGH + (th & 31), g3[c]);
+    put(th < 32 ? o.b1 + th : o.b2 + th - 32, gb);
+    if (th < 4) put(o.b3 + th, gb3);
   }
   if (bad) atomicOr(counters + kVpFlag, 1);
 }
@@ -673,8 +732,9 @@ static int run_vjp_plan(const mlpsp_scene* sc, const float* x6, const float* d4,
     static DeviceOnce attr_once;
     if (attr_once.first())
       MLPSP_CUDA_OK(cudaFuncSetAttribute(k_grouped_vjp, cudaFuncAttributeMaxDynamicSharedMemorySize, kGradSmem));
+    const int vec = ((reinterpret_cast<uintptr_t>(sc->W1) | reinterpret_cast<uintptr_t>(sc->W2)) & 15) == 0;
     launch_chained(k_grouped_vjp, dim3((unsigned)std::min<int64_t>(max_items, (int64_t)sm_count() * kGfCtas)), dim3(kGfThreads), kGradSmem, st,
-                   x6, d4, masks, items, max_items, counters, sc->freq, sc->att, sc->W1, sc->b1, sc->W2, sc->b2, sc->W3, loss_scale, out, partial);
+                   x6, d4, masks, items, max_items, counters, sc->freq, sc->att, sc->W1, sc->b1, sc->W2, sc->b2, sc->W3, vec, loss_scale, out, partial);
   }
   launch_chained(k_vjp_reduce, dim3((unsigned)std::min(sc->n, sm_count() * 8)), dim3(256), 0, st, multi, partial, out, sc->n, tc ? 0 : 1,
                  vjp_aligned(out), counters);
