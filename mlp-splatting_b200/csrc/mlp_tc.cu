@@ -5,10 +5,11 @@
 //   * the primitive's weight image (packed once per scene in the canonical K-major core-matrix
 //     layout, biases included) arrives in shared memory in three pieces, one per layer, each by a TMA
 //     bulk copy (cp.async.bulk) that signals its own mbarrier;
-//   * each of the 128 worker threads owns one record (row): it encodes the record (sin / cos of 36 phases),
-//     rounds to the operand format and stores straight into the K-major A tile;
+//   * each of the 128 worker threads of a group owns one record (row): it encodes the record (sin / cos of 36 phases),
+//     rounds to the operand format and stores the first 32 of the 80 K elements into a K-major tile in shared memory, the
+//     others into tensor memory;
 //   * layer 1 (128x80 . 80xH), layer 2 (128xH . HxH) and layer 3 (128xH . Hx16, 4 columns used) are
-//     tcgen05.mma.kind::f16 instructions issued by one lane of a fifth warp, FP32 accumulators in tensor memory.
+//     tcgen05.mma.kind::f16 instructions issued by one lane of the group's fifth warp, FP32 accumulators in tensor memory.
 //     The biases ride in the same instructions, split into up to eight operand-format terms, so no thread ever
 //     adds a bias: those of layer 1 meet a chunk of ones that fills its last K step, layers 2 and 3 (and layer 1
 //     where records are kept) take one extra K step against a constant row of ones (eight rows of shared memory,
@@ -18,14 +19,22 @@
 //     epilogue applies sigmoid / softplus (and 1-exp(-sigma*decay)) and scatters one float4 per record to its
 //     compositing slot.
 // The three layers of item i, the encoding of item i+1 and the output of item i-1 are software-pipelined:
-// every wait for a group of MMAs is preceded by independent work of a neighbouring item.  No single unit is full:
-// issue slots, shared memory and special functions are each about half used.
+// every wait for a group of MMAs is preceded by independent work of a neighbouring item.
+//
+// What bounds it: the chain of an item, 5,000 to 6,000 cycles, most of them instructions of its five warps at 60 % of the issue
+// slots; no other unit is half used.  So groups per SM and instructions count.  First wave of a 100,000-primitive frame at 1200 x
+// 680 (6.9 M records in windows of 40): 223 us with a CTA per group, six per SM, the whole layer-1 operand in shared memory; the
+// same with five per SM and most of it in tensor memory; 219 as six groups of one CTA; 188 with instructions taken out (warp
+// number known to be uniform, no zeroing of absent records, one check of the outputs for layer 2's overflow, selections in
+// softplus).  2, 3, 4, 5 groups: 432, 310, 255, 224.  As one CTA the groups' issue warps spread over the SM's four schedulers;
+// in CTAs of their own all are fifth warps and share one (a warp's number decides).
 //
 // Numerics follow the reference's tensor-core contract: operands and hidden activations rounded
 // to binary16 / bfloat16 (RN), FP32 accumulation from zero.
 //
 // Every wait on an mbarrier is bounded; when one gives up the CTA raises MLPSP_ST_TIMEOUT, waits
 // (bounded) for its own copies, frees its tensor memory and returns.
+#include <type_traits>
 #include "frame.cuh"
 #include "tc.cuh"
 
@@ -35,6 +44,8 @@ constexpr int kRows = kRowsPerItem;      // 128 = MMA M
 constexpr int kChunk = kRows * 16;       // bytes of one K chunk of an A tile: [128 rows][8 halves]
 constexpr int kN3 = 16, kOut = 4;        // the outputs, and the smallest N that holds them
 constexpr int kA1Chunks = 10;            // 72 encoded inputs and a constant chunk that meets the bias terms
+// of these in shared memory, and the columns of the others in tensor memory (two K elements each)
+constexpr int kA1SmemChunks = 4, kA1TmemCols = (kA1Chunks - kA1SmemChunks) * 4;
 
 // ---- packed weight image (per primitive) and shared-memory plan for F = 6, hidden width H = 32 or 64 ----
 // piece 1: W1 as [10 chunks][H rows][8 halves]: K = 0..71 in the order of enc_k(), then the eight terms of b1[h];
@@ -60,15 +71,18 @@ struct Net {
   // kWChunk bytes from the start of W3 on), always finite, and meets the zero rows on the A side.
   static constexpr int kOffConst = kOffW3 + (kBytesW3 + kW3Chunk > kWChunk ? (kBytesW3 + kW3Chunk + 127) / 128 * 128 : kWChunk);
   static_assert(kOffConst % 128 == 0 && kOffConst >= kOffW3 + kWChunk && kOffConst >= kWeightBytes + kW3Chunk, "what the MMAs read behind the image");
-  static constexpr int kOffA1 = kOffConst + 256;
-  static constexpr int kOffBar = kOffA1 + kA1Chunks * kChunk;
-  static constexpr int kSmemBytes = kOffBar + 96;                  // 29,024 / 41,312
-  // tensor memory: D1 and, once it has been read, D2 | D3 | the hidden layers' operand (H / 2 columns, two elements each)
-  static constexpr int kTmemCols = 2 * H;
-  static constexpr int kD1 = 0, kD2 = 0, kD3 = H, kA2 = H + kN3;
-  static_assert(kA2 + H / 2 <= kTmemCols, "tensor memory plan");
-  // resident CTAs per SM: H = 32: registers (64 a thread), H = 64: tensor memory
-  static constexpr int kCtas = H == 32 ? 6 : 4;
+  static constexpr int kOffA1 = kOffConst + 256;                   // chunks 0..3 of the layer-1 operand; the others lie in tensor memory
+  static constexpr int kOffBar = kOffA1 + kA1SmemChunks * kChunk;
+  static constexpr int kSmemBytes = kOffBar + 96;                  // 16,736 / 29,024
+  // tensor memory of a group: D1 and, once it has been read, D2 | the outputs | the hidden layers' operand (H / 2 columns, two
+  // elements each) | chunks 4..9 of the layer-1 operand.  D3 begins in the last eight columns of D2, which has been read by then:
+  // its columns 8..11 are the outputs again (see W3 above), past D2's end.
+  static constexpr int kTmemCols = H == 32 ? 80 : 128;
+  static constexpr int kD1 = 0, kD2 = 0, kD3 = H - 8, kOutputs = H, kA2 = H + 8, kA1 = kA2 + H / 2;
+  // groups of a CTA, which has an SM to itself: by tensor memory (and H = 32 by registers, 64 a thread)
+  static constexpr int kGroups = H == 32 ? 6 : 4, kGroupBytes = (kSmemBytes + 127) / 128 * 128;
+  static constexpr int kThreads = kGroups * (kRows + 32);
+  static_assert(kA1 + kA1TmemCols <= kTmemCols && kGroups * kTmemCols <= 512 && kGroups * kGroupBytes <= 227 * 1024, "plans");
   static_assert(kWeightBytes % 16 == 0 && kBytesW1 % 16 == 0 && kBytesW2 % 16 == 0 && kBytesW3 % 16 == 0, "bulk-copy granularity");
 };
 
@@ -107,8 +121,9 @@ __device__ __forceinline__ void encode_coord(float v, const float (&mult)[6], ui
   }
 }
 
-// a finite input gives finite phases (freq * att <= 101)
-__device__ __forceinline__ bool not_finite(float v) { return !(fabsf(v) < 1.0e30f); }
+// A finite input gives finite phases (freq * att <= 101).  A NaN passes here: its sines and cosines make every activation of the
+// first layer one, which that layer's check finds.
+__device__ __forceinline__ bool too_large(float x, float y, float z) { return fmaxf(fmaxf(fabsf(x), fabsf(y)), fabsf(z)) >= 1.0e30f; }
 
 template <bool BF16>
 constexpr uint32_t kOnes2 = BF16 ? 0x3f803f80u : 0x3c003c00u;
@@ -116,7 +131,7 @@ constexpr uint32_t kOnes2 = BF16 ? 0x3f803f80u : 0x3c003c00u;
 // Three coordinates into this thread's row of the layer-1 A tile, the ray direction (OFF = false) or the offset (row =
 // generic pointer to the row's 16 bytes inside chunk 0; kChunk = bytes between the K chunks), the first two and the third.
 template <bool LADDER, bool BF16, bool OFF, int kChunk = mlpsp::kChunk>
-__device__ __forceinline__ bool encode_two(float x, float y, const float (&mult)[6], char* row) {
+__device__ __forceinline__ void encode_two(float x, float y, const float (&mult)[6], char* row) {
   uint32_t a[6], b[6];
   encode_coord<LADDER, BF16>(x, mult, a);
   encode_coord<LADDER, BF16>(y, mult, b);
@@ -130,10 +145,9 @@ __device__ __forceinline__ bool encode_two(float x, float y, const float (&mult)
     *reinterpret_cast<uint4*>(row + kChunk) = make_uint4(a[4], a[5], b[0], b[1]);
     *reinterpret_cast<uint4*>(row + 2 * kChunk) = make_uint4(b[2], b[3], b[4], b[5]);
   }
-  return not_finite(x) || not_finite(y);
 }
 template <bool LADDER, bool BF16, bool OFF, int kChunk = mlpsp::kChunk>
-__device__ __forceinline__ bool encode_one(float z, const float (&mult)[6], char* row) {
+__device__ __forceinline__ void encode_one(float z, const float (&mult)[6], char* row) {
   uint32_t a[6];
   encode_coord<LADDER, BF16>(z, mult, a);
   if (OFF) {
@@ -143,12 +157,49 @@ __device__ __forceinline__ bool encode_one(float z, const float (&mult)[6], char
     *reinterpret_cast<uint4*>(row + 3 * kChunk) = make_uint4(a[0], a[1], a[2], a[3]);
     *reinterpret_cast<uint2*>(row + 4 * kChunk) = make_uint2(a[4], a[5]);
   }
-  return not_finite(z);
 }
 template <bool BF16, bool OFF, int kChunk = mlpsp::kChunk>
-__device__ __forceinline__ bool encode_three(bool ladder, float x, float y, float z, const float (&mult)[6], char* row) {
-  if (ladder) return encode_two<true, BF16, OFF, kChunk>(x, y, mult, row) | encode_one<true, BF16, OFF, kChunk>(z, mult, row);
-  return encode_two<false, BF16, OFF, kChunk>(x, y, mult, row) | encode_one<false, BF16, OFF, kChunk>(z, mult, row);
+__device__ __forceinline__ void encode_three(bool ladder, float x, float y, float z, const float (&mult)[6], char* row) {
+  if (ladder) {
+    encode_two<true, BF16, OFF, kChunk>(x, y, mult, row);
+    encode_one<true, BF16, OFF, kChunk>(z, mult, row);
+  } else {
+    encode_two<false, BF16, OFF, kChunk>(x, y, mult, row);
+    encode_one<false, BF16, OFF, kChunk>(z, mult, row);
+  }
+}
+
+// The same for the operand that lies half in shared, half in tensor memory: the first sixteen words of a direction go to the
+// row's chunks 0..3, the other two (w_rest) and the eighteen of an offset to the columns of chunks 4..8.
+template <bool LADDER, bool BF16>
+__device__ __forceinline__ bool split_direction(float x, float y, float z, const float (&mult)[6], char* row, uint32_t (&w_rest)[2]) {
+  uint32_t a[6], b[6], c[6];
+  encode_coord<LADDER, BF16>(x, mult, a);
+  encode_coord<LADDER, BF16>(y, mult, b);
+  encode_coord<LADDER, BF16>(z, mult, c);
+  *reinterpret_cast<uint4*>(row) = make_uint4(a[0], a[1], a[2], a[3]);
+  *reinterpret_cast<uint4*>(row + kChunk) = make_uint4(a[4], a[5], b[0], b[1]);
+  *reinterpret_cast<uint4*>(row + 2 * kChunk) = make_uint4(b[2], b[3], b[4], b[5]);
+  *reinterpret_cast<uint4*>(row + 3 * kChunk) = make_uint4(c[0], c[1], c[2], c[3]);
+  w_rest[0] = c[4]; w_rest[1] = c[5];
+  return too_large(x, y, z);
+}
+template <bool LADDER, bool BF16>
+__device__ __forceinline__ void split_offset_two(float x, float y, const float (&mult)[6], uint32_t col) {
+  uint32_t a[6], b[6];
+  encode_coord<LADDER, BF16>(x, mult, a);
+  tmem_st2(col + 2, a[0], a[1]);
+  tmem_st4(col + 4, a[2], a[3], a[4], a[5]);
+  encode_coord<LADDER, BF16>(y, mult, b);
+  tmem_st4(col + 8, b[0], b[1], b[2], b[3]);
+  tmem_st2(col + 12, b[4], b[5]);
+}
+template <bool LADDER, bool BF16>
+__device__ __forceinline__ void split_offset_one(float z, const float (&mult)[6], uint32_t col) {
+  uint32_t a[6];
+  encode_coord<LADDER, BF16>(z, mult, a);
+  tmem_st2(col + 14, a[0], a[1]);
+  tmem_st4(col + 16, a[2], a[3], a[4], a[5]);
 }
 
 // The encodings of the ray directions of a frame, in the operand format: per tile [5 chunks][64 pixels][16 bytes] (of the last
@@ -207,7 +258,7 @@ __device__ __forceinline__ bool hidden_to_smem(const uint32_t (&acc)[32], char* 
 }
 
 // the same for 16 columns, into the operand's columns of tensor memory (taddr: first column, this warp's lanes)
-template <bool KEEP, bool BF16>
+template <bool KEEP, bool BF16, bool CHECK>
 __device__ __forceinline__ uint32_t hidden_to_tmem(const uint32_t (&acc)[16], uint32_t taddr, int col, uint32_t& relu_mask) {
   uint32_t top = 0u, w[8];
 #pragma unroll
@@ -218,7 +269,7 @@ __device__ __forceinline__ uint32_t hidden_to_tmem(const uint32_t (&acc)[16], ui
       relu_mask |= (v1 > 0.f ? 1u : 0u) << (col + 2 * q + 1);
     }
     w[q] = pack_h2_relu<BF16>(v0, v1);
-    top = __vmaxu2(top, w[q]);
+    if (CHECK) top = __vmaxu2(top, w[q]);
   }
   tmem_st8(taddr, w);
   return top;
@@ -229,25 +280,24 @@ __device__ __forceinline__ bool overflowed(uint32_t top) {
   return (top & 0xffffu) >= inf16 || (top >> 16) >= inf16;
 }
 
-// One work item = (primitive, first record, rows <= 128).  Items are dealt to CTAs round-robin
-// (item = blockIdx.x + k * gridDim.x): all items cost about the same, and a fixed deal lets a CTA
+// One work item = (primitive, first record, rows <= 128).  Items are dealt to CTAs, then groups, round-robin
+// (item = blockIdx.x + (group + k * kGroups) * gridDim.x): all items cost about the same, and a fixed deal lets a group
 // fetch the next items' descriptors, records and weight pieces while the current item is in flight.
 //
-// A CTA is four worker warps (one record per thread) and one issue warp.  Nothing in the steady state is a
-// CTA-wide barrier: the workers tell the issue warp that an operand tile is complete through an mbarrier that
-// counts one arrival per worker warp, the issue warp (one lane) waits for that and for the layer's weight piece,
-// issues the layer's MMAs and commits them to the mbarrier the workers wait on.  It also refills each weight
-// piece as soon as the MMAs that read it have finished.  A worker warp, item i ("|" = while the MMAs run):
+// A CTA takes a whole SM and is kGroups groups of four worker warps (one record per thread) and an issue warp; the issue warps
+// are the last ones.  Groups share nothing but the allocation of tensor memory, and nothing in the steady state is a CTA-wide
+// barrier: the workers tell their issue warp that an operand tile is complete through an mbarrier that counts one arrival per
+// worker warp, the issue warp (one lane) waits for that and for the layer's weight piece, issues the layer's MMAs and commits
+// them to the mbarrier the workers wait on.  It also refills each weight piece as soon as the MMAs that read it have finished.  A
+// worker warp, item i ("|" = while the MMAs run):
 //   layer-1 tile of i complete -> arrive | output of i-1 (its layer-3 MMAs have finished by now)
 //   wait layer 1: hidden tile 1 of i written -> arrive | first part of the encoding of i+1
 //   wait layer 2: hidden tile 2 of i written -> arrive | second part of the encoding of i+1
-constexpr int kMlpThreads = kRows + 32;
-
 // TAB: the records name their pixel, whose encoded direction is copied from the frame's table (k_encode_directions) into
 // the A tile by cp.async: half of the 72 sines and cosines of a record are those of its ray, and a pixel has about a dozen
 // records.  The record is then (offset, decay | slot, pixel); without it (direction, offset, decay, slot).
 template <bool KEEP, bool BF16, int H, bool TAB>
-__global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
+__global__ void __launch_bounds__(Net<H>::kThreads, 1) k_mlp_tc(
     const char* __restrict__ w16, const float* __restrict__ freq, const float* __restrict__ att,
     const char* __restrict__ dir_table, const float4* __restrict__ rec_in, const int4* __restrict__ work,
     const int32_t* __restrict__ counters, float4* __restrict__ rec_out, float4* __restrict__ rec_ext, int out_mode,
@@ -256,46 +306,50 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
   static_assert(!KEEP || H == 32, "the record export keeps 32-bit ReLU masks");
   chain_wait();       // the work list and the records come from the previous kernels of the frame
   chain_release();
-  extern __shared__ __align__(128) char smem[];
+  extern __shared__ __align__(128) char smem_all[];
+  if (status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
+  const int G = counters[kCtrWork];
+  if ((int)blockIdx.x >= G) return;          // more CTAs than work: leave before touching tensor memory
+  const int warp = warp_of_cta(), lane = threadIdx.x & 31;
+  const bool issuer = warp >= 4 * N::kGroups;
+  const int group = issuer ? warp - 4 * N::kGroups : warp >> 2, wrow = warp & 3, tid = wrow * 32 + lane;      // tid: a worker's row
+  char* smem = smem_all + group * N::kGroupBytes;
   // [0..2] weight pieces landed, [3..5] operand tile of layer 1 / 2 / 3 complete, [6] layer-1 MMAs done, [7] layer-2 / 3 MMAs done
   uint64_t* s_bar = reinterpret_cast<uint64_t*>(smem + N::kOffBar);
-  uint32_t* s_misc = reinterpret_cast<uint32_t*>(s_bar + 8);          // [0] tmem base, [1] a wait gave up
-  if (status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int G = counters[kCtrWork];
-  int item = blockIdx.x;
-  if (item >= G) return;                     // more CTAs than work: leave before touching tensor memory
-  const int stride = (int)gridDim.x;
+  uint32_t* s_misc = reinterpret_cast<uint32_t*>(s_bar + 8);          // [0] tmem base (the first group's), [1] a wait gave up
+  int item = group * (int)gridDim.x + (int)blockIdx.x;
+  const int stride = N::kGroups * (int)gridDim.x;
   const uint32_t wb = smem_u32(smem), cst = wb + N::kOffConst, a1 = wb + N::kOffA1;
   const uint32_t bar_w0 = smem_u32(&s_bar[0]), bar_r0 = smem_u32(&s_bar[3]), bar_a = smem_u32(&s_bar[6]), bar_b = smem_u32(&s_bar[7]);
-  if (tid == 0) {
+  if (issuer) {
+    if (lane == 0) {
 #pragma unroll
-    for (int b = 0; b < 3; ++b) { mbar_init(bar_w0 + 8 * b, 1); mbar_init(bar_r0 + 8 * b, kRows / 32); }
-    mbar_init(bar_a, 1);
-    mbar_init(bar_b, 1);
-    s_misc[1] = 0u;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == kRows / 32) tmem_alloc(smem_u32(&s_misc[0]), N::kTmemCols);
-  if (tid < 16) {
-    const uint32_t v = tid < 8 ? kOnes2<BF16> : 0u;
-    *reinterpret_cast<uint4*>(smem + N::kOffConst + tid * 16) = make_uint4(v, v, v, v);
-  }
-  if (tid < (N::kOffConst - N::kWeightBytes) / 16) *reinterpret_cast<uint4*>(smem + N::kWeightBytes + tid * 16) = make_uint4(0u, 0u, 0u, 0u);
-  // the constant chunk: ones, so that the bias rides in the last K step of layer 1; with KEEP zeros, and the bias a step of its
-  // own as in layers 2 and 3 (the order of the sums decides saved ReLU signs of values next to zero)
-  if (tid < kRows) {
-    const uint32_t v = KEEP ? 0u : kOnes2<BF16>;
-    *reinterpret_cast<uint4*>(smem + N::kOffA1 + kBiasChunk * kChunk + tid * 16) = make_uint4(v, v, v, v);
+      for (int b = 0; b < 3; ++b) { mbar_init(bar_w0 + 8 * b, 1); mbar_init(bar_r0 + 8 * b, kRows / 32); }
+      mbar_init(bar_a, 1);
+      mbar_init(bar_b, 1);
+      s_misc[1] = 0u;
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    if (group == 0) tmem_alloc(smem_u32(&s_misc[0]), 512);
+  } else {
+    if (tid < 16) {
+      const uint32_t v = tid < 8 ? kOnes2<BF16> : 0u;
+      *reinterpret_cast<uint4*>(smem + N::kOffConst + tid * 16) = make_uint4(v, v, v, v);
+    }
+    if (tid < (N::kOffConst - N::kWeightBytes) / 16) *reinterpret_cast<uint4*>(smem + N::kWeightBytes + tid * 16) = make_uint4(0u, 0u, 0u, 0u);
   }
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = s_misc[0];
+  const uint32_t tmem_all = *reinterpret_cast<const uint32_t*>(smem_all + N::kOffBar + 64);
+  const uint32_t tmem = tmem_all + group * N::kTmemCols, a1t = tmem + N::kA1;
   bool ok = true;
 
-  if (warp == kRows / 32) {
+  if (item >= G) {
+    // fewer items than groups
+  } else if (issuer) {
     // ------------------------------------------------------------------ issue warp ----
     const uint32_t idesc_h = instr_desc(kRows, H, BF16), idesc_o = instr_desc(kRows, kN3, BF16);
     // Operand descriptors are built once; a K step only moves the start address, which sits in the low bits in
@@ -337,8 +391,11 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
       tc_fence_after();
       if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < kA1Chunks / 2; ++ks)
-          mma_f16(tmem + N::kD1, step(a1_desc, ks * 2 * kChunk), step(w1_desc, ks * 2 * N::kWChunk), idesc_h, ks > 0);
+        for (int ks = 0; ks < kA1Chunks / 2; ++ks) {
+          const uint64_t w = step(w1_desc, ks * 2 * N::kWChunk);
+          if (ks < kA1SmemChunks / 2) mma_f16(tmem + N::kD1, step(a1_desc, ks * 2 * kChunk), w, idesc_h, ks > 0);
+          else mma_f16_ta(tmem + N::kD1, a1t + (ks - kA1SmemChunks / 2) * 8, w, idesc_h, 1u);
+        }
         if (KEEP) mma_f16(tmem + N::kD1, ones_desc, step(w1_desc, kBiasChunk * N::kWChunk), idesc_h, 1u);
         mma_commit(bar_a);
       }
@@ -397,7 +454,13 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
     __syncwarp();
   } else {
     // ---------------------------------------------------------------- worker warps ----
-    const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);   // this warp's 32 lanes
+    const uint32_t trow = tmem + ((uint32_t)(wrow * 32) << 16), a1row = a1t + ((uint32_t)(wrow * 32) << 16);   // this warp's 32 lanes
+    // the constant chunk of layer 1: ones, so that the bias rides in its last K step; with KEEP zeros, and the bias a step of its
+    // own as in layers 2 and 3 (the order of the sums decides saved ReLU signs of values next to zero)
+    {
+      const uint32_t v = KEEP ? 0u : kOnes2<BF16>;
+      tmem_st4(a1row + (kBiasChunk - kA1SmemChunks) * 4, v, v, v, v);
+    }
     // phase multipliers freq[f] * att[f]; when every band is exactly twice the one before (equal
     // attenuation: FourierFeatureEncoding's bands, cumodel.py:163) the encoder takes the double-angle route
     float mult[6];
@@ -407,81 +470,99 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
 #pragma unroll
     for (int f = 1; f < 6; ++f) ladder = ladder && mult[f] == 2.0f * mult[f - 1];
     int4 wk = __ldg(work + item);
-    int4 wk_n = (item + stride < G) ? __ldg(work + item + stride) : make_int4(0, 0, 0, 0);
-    auto load_rec = [&](const int4& w, float4& r0, float4& r1) {
-      r0 = make_float4(0.f, 0.f, 0.f, 0.f);
-      r1 = make_float4(0.f, 0.f, 0.f, 0.f);     // the zero record, never stored
+    int4 wk_n = __ldg(work + min(item + stride, G - 1));       // (past the list's end: any item, and nobody encodes it)
+    auto load_rec = [&](const int4& w, float4& r0, float4& r1) {     // rows past the end keep their last record and store nothing
       if (tid < w.z) { r0 = __ldg(rec_in + 2 * (size_t)(w.y + tid)); r1 = __ldg(rec_in + 2 * (size_t)(w.y + tid) + 1); }
     };
     auto rec_decay = [](const float4& r0, const float4& r1) { return TAB ? r0.w : r1.z; };
     auto rec_slot = [](const float4& r1) { return TAB ? __float_as_uint(r1.x) : __float_as_uint(r1.w); };
-    // the pixel's encoded direction on its way to this thread's row of the A tile
+    // the pixel's encoded direction on its way to this thread's row of the A tile; its last two words
     auto copy_direction = [&](const float4& r1) {
       const uint32_t pixel = __float_as_uint(r1.y);
       const char* src = dir_table + (size_t)(pixel >> 6) * kDirTileBytes + (pixel & 63u) * 16;
       const uint32_t dst = a1 + tid * 16;
 #pragma unroll
       for (int c = 0; c < 4; ++c) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + c * kChunk), "l"(src + c * kDirChunk) : "memory");
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 4 * kChunk), "l"(src + 4 * kDirChunk) : "memory");
+      return __ldg(reinterpret_cast<const uint2*>(src + 4 * kDirChunk));
     };
     auto direction_landed = [&]() { asm volatile("cp.async.wait_all;" ::: "memory"); };
     char* my_row = smem + N::kOffA1 + tid * 16;
     // a hidden layer of the warp's rows: accumulator columns from d on -> operand
-    auto hidden = [&](uint32_t d, uint32_t& relu_mask) {
+    // (check: the first layer.  An infinite activation there may leave the second only sums of minus infinity, which its ReLU
+    // hides; one of the second makes every output infinite or not a number, which emit_output looks at.)
+    auto hidden = [&](uint32_t d, uint32_t& relu_mask, auto check) {
       uint32_t top = 0u;
       relu_mask = 0u;
 #pragma unroll
       for (int part = 0; part < H / 16; ++part) {
         uint32_t acc[16];
         tmem_ld16(trow + d + part * 16, acc);
-        top = __vmaxu2(top, hidden_to_tmem<KEEP, BF16>(acc, trow + N::kA2 + part * 8, part * 16, relu_mask));
+        const uint32_t t = hidden_to_tmem<KEEP, BF16, decltype(check)::value>(acc, trow + N::kA2 + part * 8, part * 16, relu_mask);
+        top = __vmaxu2(top, t);
       }
       return overflowed<BF16>(top);
     };
-    // the warp's rows of an operand tile are complete (and its reads of tensor memory have retired)
-    auto tile_done = [&](uint32_t bar) {
+    // the warp's rows of an operand tile are complete (and its reads of tensor memory have retired); in_smem: some of
+    // it was written to shared memory
+    auto tile_done = [&](uint32_t bar, bool in_smem = false) {
       tmem_st_wait();
-      fence_async_smem();
+      if (in_smem) fence_async_smem();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
     };
     bool bad = false;
+    uint2 rest = make_uint2(0u, 0u);           // the last two words of the next record's direction
+    auto direction = [&](float x, float y, float z) {
+      uint32_t w[2];
+      bad |= ladder ? split_direction<true, BF16>(x, y, z, mult, my_row, w) : split_direction<false, BF16>(x, y, z, mult, my_row, w);
+      rest = make_uint2(w[0], w[1]);
+    };
+    auto offset_two = [&](float x, float y) {
+      if (ladder) split_offset_two<true, BF16>(x, y, mult, a1row); else split_offset_two<false, BF16>(x, y, mult, a1row);
+    };
+    auto offset_one = [&](float x, float y, float z) {       // (x, y: for the check)
+      bad |= too_large(x, y, z);
+      if (ladder) split_offset_one<true, BF16>(z, mult, a1row); else split_offset_one<false, BF16>(z, mult, a1row);
+      tmem_st2(a1row, rest.x, rest.y);
+    };
     // ---- prologue: the first item's record, encoded in full ----
-    float4 q0, q1;
+    float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = q0;
     load_rec(wk, q0, q1);
     // MMA rows are independent and rows past the end of the primitive's records are never stored, so a
     // warp whose 32 rows are all past the end skips the encoding and the epilogues (its rows of the
     // operand tiles keep whatever they held) and only reports its tiles complete
-    if (warp * 32 < wk.z) {
-      // rows past the end inside a live warp hold the zero record; their results are never stored
+    if (wrow * 32 < wk.z) {
       if (TAB) {
-        copy_direction(q1);
-        bad |= encode_three<BF16, true>(ladder, q0.x, q0.y, q0.z, mult, my_row);
+        rest = copy_direction(q1);
+        offset_two(q0.x, q0.y);
+        offset_one(q0.x, q0.y, q0.z);
         direction_landed();
       } else {
-        bad |= encode_three<BF16, false>(ladder, q0.x, q0.y, q0.z, mult, my_row);
-        bad |= encode_three<BF16, true>(ladder, q0.w, q1.x, q1.y, mult, my_row);
+        direction(q0.x, q0.y, q0.z);
+        offset_two(q0.w, q1.x);
+        offset_one(q0.w, q1.x, q1.y);
       }
     }
-    tile_done(bar_r0);
+    tile_done(bar_r0, true);
     float decay_c = rec_decay(q0, q1);
     uint32_t slot_c = rec_slot(q1);
-    load_rec(wk_n, q0, q1);                    // the second item's record (zero record when there is none)
+    load_rec(wk_n, q0, q1);                    // the second item's record
 
     bool have_prev = false, live_p = false, valid_p = false;
     float decay_p = 0.f;
     uint32_t slot_p = 0u, relu1 = 0u, relu2 = 0u, relu1_p = 0u, relu2_p = 0u;
-    uint32_t li = 0u;                          // items this CTA has started: parity of the once-per-item barriers
+    uint32_t li = 0u;                          // items this group has started: parity of the once-per-item barriers
 
     auto emit_output = [&]() {
-      // output of the item whose layer-3 MMAs have just finished: (decay_p, slot_p), accumulator columns [H, H+4)
+      // output of the item whose layer-3 MMAs have just finished: (decay_p, slot_p), accumulator columns [H, H + 4)
       if (!live_p) return;
       uint32_t o[4];
-      tmem_ld4(trow + N::kD3, o);
+      tmem_ld4(trow + N::kOutputs, o);
       if (valid_p) {
         const float o0 = __uint_as_float(o[0]), o1 = __uint_as_float(o[1]), o2 = __uint_as_float(o[2]), o3 = __uint_as_float(o[3]);
         const float sigma_raw = softplus_fast(o3);
+        bad |= !(fabsf((o0 + o1) + (o2 + o3)) < 3.0e38f);
         float4 out;
         out.x = sigmoid_fast(o0); out.y = sigmoid_fast(o1); out.z = sigmoid_fast(o2);
         out.w = (out_mode == kOutAlpha) ? (1.f - __expf(-(sigma_raw * decay_p))) : sigma_raw;
@@ -493,15 +574,14 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
     for (;;) {
       const int nrows = wk.z;
       const bool valid = tid < nrows;
-      const bool warp_live = warp * 32 < nrows;
+      const bool warp_live = wrow * 32 < nrows;
       const int next = item + stride;
       const bool has_next = next < G;
-      const bool next_live = has_next && warp * 32 < wk_n.z;
+      const bool next_live = has_next && wrow * 32 < wk_n.z;
       const uint32_t par = li & 1u;
       // descriptor of the item after the next one
       const int next2 = next + stride;
-      int4 wk_n2 = make_int4(0, 0, 0, 0);
-      if (next2 < G) wk_n2 = __ldg(work + next2);
+      const int4 wk_n2 = __ldg(work + min(next2, G - 1));
       // ---- output of the previous item while layer 1 of this one runs ----
       if (have_prev) {
         ok = __all_sync(0xffffffffu, mbar_wait(bar_b, 1u) && ok);   // warp-uniform: tcgen05.ld is .sync.aligned
@@ -513,27 +593,29 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
       tc_fence_after();
       if (!ok) break;
       // layer 1 no longer reads the A tile: the next item's directions are in flight over two round trips
-      if (TAB && next_live) copy_direction(q1);
-      // the record this thread will load at the end of this item (for the item after the next) is asked into L2 now
-      if (tid < wk_n2.z) asm volatile("prefetch.global.L2 [%0];" ::"l"(rec_in + 2 * (size_t)(wk_n2.y + tid)));
-      if (warp_live) bad |= hidden(N::kD1, relu1) && valid;
+      if (TAB && next_live) rest = copy_direction(q1);
+      // the record this thread will load at the end of this item (for the item after the next) is asked into L2 now (with the
+      // table of directions L2 is busy enough: 100k frame 816 us, without 811)
+      if (!TAB && tid < wk_n2.z) asm volatile("prefetch.global.L2 [%0];" ::"l"(rec_in + 2 * (size_t)(wk_n2.y + tid)));
+      if (warp_live) bad |= hidden(N::kD1, relu1, std::true_type{}) && valid;
       tile_done(bar_r0 + 8);
       // ---- first part of the next item's encoding while layer 2 runs ----
       if (next_live) {
-        if (!TAB) bad |= encode_three<BF16, false>(ladder, q0.x, q0.y, q0.z, mult, my_row);
-        else bad |= ladder ? encode_two<true, BF16, true>(q0.x, q0.y, mult, my_row) : encode_two<false, BF16, true>(q0.x, q0.y, mult, my_row);
+        if (!TAB) direction(q0.x, q0.y, q0.z);
+        else offset_two(q0.x, q0.y);
       }
       ok = __all_sync(0xffffffffu, mbar_wait(bar_b, 0u) && ok);
       tc_fence_after();
       if (!ok) break;
-      if (warp_live) bad |= hidden(N::kD2, relu2) && valid;
+      if (warp_live) hidden(N::kD2, relu2, std::false_type{});
       tile_done(bar_r0 + 16);
       // ---- second part of the next item's encoding while layer 3 runs ----
       if (next_live) {
         if (!TAB) {
-          bad |= encode_three<BF16, true>(ladder, q0.w, q1.x, q1.y, mult, my_row);
+          offset_two(q0.w, q1.x);
+          offset_one(q0.w, q1.x, q1.y);
         } else {
-          bad |= ladder ? encode_one<true, BF16, true>(q0.z, mult, my_row) : encode_one<false, BF16, true>(q0.z, mult, my_row);
+          offset_one(q0.x, q0.y, q0.z);
           direction_landed();
         }
       }
@@ -541,7 +623,7 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
       have_prev = true;
       live_p = warp_live; valid_p = valid; decay_p = decay_c; slot_p = slot_c; relu1_p = relu1; relu2_p = relu2;
       if (!has_next) break;
-      tile_done(bar_r0);
+      tile_done(bar_r0, true);
       decay_c = rec_decay(q0, q1);
       slot_c = rec_slot(q1);
       item = next;
@@ -560,8 +642,8 @@ __global__ void __launch_bounds__(kMlpThreads, Net<H>::kCtas) k_mlp_tc(
   }
   tc_fence_before();
   __syncthreads();
-  if (tid == 0 && s_misc[1]) atomicOr(status + MLPSP_ST_BITS, MLPSP_ST_TIMEOUT);
-  if (warp == kRows / 32) tmem_free(tmem, N::kTmemCols);
+  if (issuer && lane == 0 && s_misc[1]) atomicOr(status + MLPSP_ST_BITS, MLPSP_ST_TIMEOUT);
+  if (issuer && group == 0) tmem_free(tmem_all, 512);
 }
 
 // ------------------------------------------------------------------ small groups ----
@@ -646,9 +728,7 @@ __global__ void __launch_bounds__(kMiniRows, MiniNet<H>::kCtas) k_mlp_tc_mini(
     mbar_expect_tx(bar_w0 + 8 * piece, bytes);
     bulk_g2s(wb + off, w16 + (size_t)prim * N::kWeightBytes + off, bytes, bar_w0 + 8 * piece);
   };
-  auto load_rec = [&](const int4& w, float4& r0, float4& r1) {
-    r0 = make_float4(0.f, 0.f, 0.f, 0.f);
-    r1 = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto load_rec = [&](const int4& w, float4& r0, float4& r1) {       // rows past the end keep their last record and store nothing
     if (lane < w.z) { r0 = __ldg(rec_in + 2 * (size_t)(w.y + lane)); r1 = __ldg(rec_in + 2 * (size_t)(w.y + lane) + 1); }
   };
   // the warp's writes to an operand tile are visible to the tensor core, its reads of tensor memory have retired
@@ -658,16 +738,24 @@ __global__ void __launch_bounds__(kMiniRows, MiniNet<H>::kCtas) k_mlp_tc_mini(
     __syncwarp();
   };
   int4 wk = __ldg(work + item);
-  int4 wk_n = (item + stride < G) ? __ldg(work + item + stride) : make_int4(0, 0, 0, 0);
+  int4 wk_n = __ldg(work + min(item + stride, G - 1));
   uint32_t pend = 0u;
   if (elect_one()) { request(0, wk.x); request(1, wk.x); request(2, wk.x); }
   pend = 7u;
   char* my_row = s_a1 + lane * 16;
   bool bad = false, ok = true;
-  float4 q0, q1;
+  float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = q0;
   load_rec(wk, q0, q1);
-  bad |= encode_three<BF16, false, kMiniChunk>(ladder, q0.x, q0.y, q0.z, mult, my_row);
-  bad |= encode_three<BF16, true, kMiniChunk>(ladder, q0.w, q1.x, q1.y, mult, my_row);
+  auto direction = [&]() {
+    encode_three<BF16, false, kMiniChunk>(ladder, q0.x, q0.y, q0.z, mult, my_row);
+    bad |= too_large(q0.x, q0.y, q0.z);
+  };
+  auto offset = [&]() {
+    encode_three<BF16, true, kMiniChunk>(ladder, q0.w, q1.x, q1.y, mult, my_row);
+    bad |= too_large(q0.w, q1.x, q1.y);
+  };
+  direction();
+  offset();
   float decay_c = q1.z;
   uint32_t slot_c = __float_as_uint(q1.w);
   load_rec(wk_n, q0, q1);
@@ -680,8 +768,7 @@ __global__ void __launch_bounds__(kMiniRows, MiniNet<H>::kCtas) k_mlp_tc_mini(
     const bool has_next = next < G;
     const uint32_t par = li & 1u;
     const int next2 = next + stride;
-    int4 wk_n2 = make_int4(0, 0, 0, 0);
-    if (next2 < G) wk_n2 = __ldg(work + next2);
+    const int4 wk_n2 = __ldg(work + min(next2, G - 1));
     // ---- layer 1 ----
     tile_done();
     bool landed = mbar_wait(bar_w0, par);
@@ -697,7 +784,7 @@ __global__ void __launch_bounds__(kMiniRows, MiniNet<H>::kCtas) k_mlp_tc_mini(
       mma_commit(bar_m);
     }
     __syncwarp();
-    if (next2 < G && lane < wk_n2.z) asm volatile("prefetch.global.L2 [%0];" ::"l"(rec_in + 2 * (size_t)(wk_n2.y + lane)));
+    if (lane < wk_n2.z) asm volatile("prefetch.global.L2 [%0];" ::"l"(rec_in + 2 * (size_t)(wk_n2.y + lane)));
     ok = __all_sync(0xffffffffu, mbar_wait(bar_m, ph++ & 1u) && ok);   // one completion per layer
     tc_fence_after();
     if (!ok) break;
@@ -726,7 +813,7 @@ __global__ void __launch_bounds__(kMiniRows, MiniNet<H>::kCtas) k_mlp_tc_mini(
     }
     __syncwarp();
     // first part of the next item's encoding while layer 2 runs (the layer-1 tile is free)
-    if (has_next) bad |= encode_three<BF16, false, kMiniChunk>(ladder, q0.x, q0.y, q0.z, mult, my_row);
+    if (has_next) direction();
     ok = __all_sync(0xffffffffu, mbar_wait(bar_m, ph++ & 1u) && ok);
     tc_fence_after();
     if (!ok) break;
@@ -738,7 +825,7 @@ __global__ void __launch_bounds__(kMiniRows, MiniNet<H>::kCtas) k_mlp_tc_mini(
     for (int part = 0; part < H / 32; ++part) {
       uint32_t acc[32];
       tmem_ld32(trow + part * 32, acc);
-      bad |= hidden_to_smem<false, BF16, kMiniChunk>(acc, s_a2 + part * 4 * kMiniChunk, lane, relu_unused) && valid;
+      hidden_to_smem<false, BF16, kMiniChunk>(acc, s_a2 + part * 4 * kMiniChunk, lane, relu_unused);      // (checked at the outputs, see k_mlp_tc)
     }
     // ---- layer 3 ----
     tile_done();
@@ -754,7 +841,7 @@ __global__ void __launch_bounds__(kMiniRows, MiniNet<H>::kCtas) k_mlp_tc_mini(
       mma_commit(bar_m);
     }
     __syncwarp();
-    if (has_next) bad |= encode_three<BF16, true, kMiniChunk>(ladder, q0.w, q1.x, q1.y, mult, my_row);
+    if (has_next) offset();
     ok = __all_sync(0xffffffffu, mbar_wait(bar_m, ph++ & 1u) && ok);
     tc_fence_after();
     if (!ok) break;
@@ -768,6 +855,7 @@ __global__ void __launch_bounds__(kMiniRows, MiniNet<H>::kCtas) k_mlp_tc_mini(
       if (valid) {
         const float o0 = __uint_as_float(o[0]), o1 = __uint_as_float(o[1]), o2 = __uint_as_float(o[2]), o3 = __uint_as_float(o[3]);
         const float sigma_raw = softplus_fast(o3);
+        bad |= !(fabsf((o0 + o1) + (o2 + o3)) < 3.0e38f);
         float4 out;
         out.x = sigmoid_fast(o0); out.y = sigmoid_fast(o1); out.z = sigmoid_fast(o2);
         out.w = (out_mode == kOutAlpha) ? (1.f - __expf(-(sigma_raw * decay_c))) : sigma_raw;
@@ -881,8 +969,8 @@ static int launch_one(const char* image, const mlpsp_scene* sc, const char* dir_
   using N = Net<H>;
   static DeviceOnce attr_once;
   if (attr_once.first())
-    MLPSP_CUDA_OK(cudaFuncSetAttribute(k_mlp_tc<KEEP, BF16, H, TAB>, cudaFuncAttributeMaxDynamicSharedMemorySize, N::kSmemBytes));
-  launch_chained(k_mlp_tc<KEEP, BF16, H, TAB>, dim3(grid), dim3(kMlpThreads), N::kSmemBytes, st, image, sc->freq, sc->att, dir_table,
+    MLPSP_CUDA_OK(cudaFuncSetAttribute(k_mlp_tc<KEEP, BF16, H, TAB>, cudaFuncAttributeMaxDynamicSharedMemorySize, N::kGroups * N::kGroupBytes));
+  launch_chained(k_mlp_tc<KEEP, BF16, H, TAB>, dim3(grid), dim3(N::kThreads), N::kGroups * N::kGroupBytes, st, image, sc->freq, sc->att, dir_table,
                  reinterpret_cast<const float4*>(rec_in), work, counters, rec_out, rec_ext, out_mode, status);
   return MLPSP_OK;
 }
@@ -903,10 +991,8 @@ template <int H>
 static int launch_tc(const mlpsp_scene* sc, const char* image, const char* dir_table, const RecIn* rec_in, const int4* work, const int4* work_small,
                      const int32_t* counters, float4* rec_out, float4* rec_ext, int out_mode, int32_t* status, cudaStream_t st,
                      bool bf16, int grid_cap) {
-  using N = Net<H>;
   const int sms = sm_count();
-  int grid = sms * N::kCtas;
-  if (grid_cap > 0) grid = std::min(grid, grid_cap);
+  const int grid = grid_cap > 0 ? std::min(sms, grid_cap) : sms;
   LaunchScope scope(kKMlp, (work_small && !rec_ext) ? 2 : 1, st);
   int rc;
   if (rec_ext) {

@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(kVjpRows, kVjpCtas) k_grouped_vjp_tc(
   const VjpList list(items, max_items, counters);
   const int G = list.total, E = vjp_planned(counters, kVpEmpty);
   const int idx = blockIdx.x;
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = warp_of_cta();
   // primitives without records, one between two waits; the number of the next one is on its way
   int empty = blockIdx.x, empty_prim = empty < E ? __ldg(&multi[n - 1 - empty].prim) : 0;
   auto zero_next = [&]() {
