@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(32 * kHitWarps) k_hits(const HitArgs a, int pa
   __shared__ float4 s_q[kHitWarps][64];
   if (a.status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) reset_wave(a);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, warp = warp_of_cta(), wpb = blockDim.x >> 5;
   const int units = *a.active_count * parts;
   for (int unit = blockIdx.x * wpb + warp; unit < units; unit += gridDim.x * wpb) {
     const int slot_i = parts == 1 ? unit : unit / parts, part = unit - slot_i * parts;
@@ -620,7 +620,7 @@ __global__ void __launch_bounds__(32 * kFillWarps, 4) k_fill(const FillArgs a) {
   chain_release();
   __shared__ FillSmem s_all[kFillWarps];
   if (a.status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, warp = warp_of_cta(), wpb = blockDim.x >> 5;
   FillSmem& sm = s_all[warp];
   const uint32_t lt = (1u << lane) - 1u;
   const int per_tile = a.chunks * a.halves, units = *a.active_count * per_tile;
@@ -807,7 +807,7 @@ __global__ void __launch_bounds__(64) k_composite(
   const int s = tile_offsets[tile];
   const int len = tile_len[tile];
   const int wlo = min(lo, len), whi = min(hi, len);
-  const int lane = threadIdx.x & 31, half = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, half = warp_of_cta();
   const TilePix tp = tile_pixel(tile, half * 32 + lane, ntx, W, H);
   float4 st = make_float4(0.f, 0.f, 0.f, 0.f);
   float2 dp = make_float2(0.f, 0.f);
