@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(kDecThreads, 1) k_decode_tc(
   float2* s_arg = reinterpret_cast<float2*>(smem + kSmArg);
   if (status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
   if ((int)blockIdx.x >= num_tiles) return;          // leave before touching tensor memory
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_of_cta(), lane = tid & 31;
   const int q = warp & 3, hsel = warp >> 2;           // tensor-memory lane quarter, column interleave
   const bool worker = warp < kMmaWarp;
   if (tid < 64) reinterpret_cast<int32_t*>(smem + kSmHdr)[tid] = __ldg(reinterpret_cast<const int32_t*>(image) + tid);

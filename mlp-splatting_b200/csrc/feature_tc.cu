@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(kFtThreads, PR == 8 ? 4 : 2) k_feature_tc(
   __shared__ int warp_sums[32];
   if (status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
   const int tile = blockIdx.x, c0 = blockIdx.y * CB;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = warp_of_cta();
   const int stage_bytes = P::stage_bytes(CB);
   uint16_t* s_idx = reinterpret_cast<uint16_t*>(smem + 2 * stage_bytes);            // touched candidates of the tile
   FtMeta* s_meta = reinterpret_cast<FtMeta*>(smem + 2 * stage_bytes + 2 * kFtListMax);

@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(kPairThreads, kPairCtas) k_mlp_f32_pair(
   __shared__ __align__(8) float s_freq[2 * kTF];
   __shared__ int s_next;
   if (status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_of_cta(), lane = tid & 31;
   const int G = counters[kCtrWork];
   const int item = blockIdx.x;
   if (item >= G) return;
