@@ -19,7 +19,8 @@ TILE_CAPACITY = 1536  # MLPSP_TILE_CANDIDATE_CAPACITY default of the reference l
 
 
 def _stream_ptr(device):
-    return C.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    """cudaStream_t of the current stream, without the torch.cuda.Stream object around it (two microseconds of every call)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
 
 
 class _on:
@@ -31,7 +32,7 @@ class _on:
 
     def __enter__(self):
         self.ctx = None
-        if torch.cuda.current_device() != (self.d.index if self.d.index is not None else torch.cuda.current_device()):
+        if self.d.index is not None and torch.cuda.current_device() != self.d.index:
             self.ctx = torch.cuda.device(self.d)
             self.ctx.__enter__()
 
@@ -41,6 +42,8 @@ class _on:
 
 
 def _dev_f32(x, device):
+    if isinstance(x, torch.Tensor) and x.dtype == torch.float32 and x.device == device and x.is_contiguous():
+        return x
     t = torch.as_tensor(x)
     return t.to(device=device, dtype=torch.float32).contiguous()
 
@@ -73,7 +76,7 @@ class PackedScene:
         if self.device.type != "cuda":
             raise RuntimeError("PackedScene must live on a CUDA device; there is no CPU path")
         d = self.device
-        with torch.cuda.device(d):
+        with _on(d):
             self.positions = _dev_f32(positions, d)
             self.log_scales = _dev_f32(log_scales, d)
             self.quats_unit = normalize_rows(_dev_f32(quats, d))
@@ -166,7 +169,7 @@ class PackedScene:
         self.device = d = torch.device(device)
         if d.type != "cuda":
             raise RuntimeError("PackedScene must live on a CUDA device; there is no CPU path")
-        with torch.cuda.device(d):
+        with _on(d):
             self.positions, self.log_scales = _dev_f32(positions, d), _dev_f32(log_scales, d)
             self.quats_unit = normalize_rows(_dev_f32(quats, d))
             self.W1 = self.b1 = self.W2 = self.b2 = self.W3 = self.b3 = None
@@ -232,7 +235,7 @@ class PackedScene:
                              f"({int(t.shape[1]) if t.ndim == 2 else tuple(t.shape)}).")
         tn = t / t.norm(dim=1, keepdim=True).clamp_min(1e-12)
         view = copy.copy(self)
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             view.feat_attr = torch.matmul(self.feat_attr, tn.t()).contiguous()
         view.feat_dim = int(t.shape[0])
         view.feat16 = None          # the projected scores are not binary16 values
@@ -669,7 +672,7 @@ class FrameRenderer:
                 c._buffers += 1
             c.tile_prims[:m].copy_(prims16)
             c.tile_offsets.copy_(offs16)
-            with torch.cuda.device(d):
+            with _on(d):
                 st = _stream_ptr(d)
                 L.check(self.lib.mlpsp_status_reset(L.ptr(c.status), st), "mlpsp_status_reset")
                 L.check(self.lib.mlpsp_validate_tile_lists(L.ptr(c.tile_offsets), L.ptr(c.tile_prims), c.T, m, c.capacity,
@@ -695,7 +698,7 @@ class FrameRenderer:
                       sort_key=0, path_name="render_tiles_forward_tilecenter", tile_lists=None, **kw):
         """One frame with the reference's tile_size = 16 semantics (see tile16_lists); other arguments as render(),
         tile_lists on the 16x16 grid."""
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             rd = rays_d if rays_normalized else normalize_rows(rays_d)
             prims8, offs8 = self.tile16_lists(scene, rays_o, rd, threshold, view, proj, sort_key=sort_key, path_name=path_name,
                                               lists16=tile_lists)
@@ -718,7 +721,7 @@ class FrameRenderer:
         # The host waits once for the frame and the count of its records: the status word travels between the two.  A frame
         # that reports anything is rendered again by the path that looks at the status first.
         rgb, alpha = self.render(scene, rays_o, rays_d, threshold, keep_records=True, check=False, **kw)
-        with torch.cuda.device(d):
+        with _on(d):
             st = _stream_ptr(d)
             offsets = torch.empty(self.P + 1, device=d, dtype=torch.int64)
             if checked:
@@ -748,7 +751,7 @@ class FrameRenderer:
     def bin(self, scene: PackedScene, view, proj, threshold, check=True):
         """Binning only: returns (culled_prim_indices[M] int32, tile_offsets[T+1] int32) views."""
         lib, d = self.lib, self.device
-        with torch.cuda.device(d):
+        with _on(d):
             st = _stream_ptr(d)
             for _attempt in range(3):
                 L.check(lib.mlpsp_status_reset(L.ptr(self.status), st), "mlpsp_status_reset")
@@ -774,7 +777,7 @@ class FrameRenderer:
             raise ValueError("view_matrices must contain at least one view")
         if int(tv.min()) < 0 or int(tv.max()) >= views.shape[0]:
             raise ValueError("tile_view_ids contains out-of-range view indices")
-        with torch.cuda.device(d):
+        with _on(d):
             st = _stream_ptr(d)
             for _attempt in range(3):
                 L.check(lib.mlpsp_status_reset(L.ptr(self.status), st), "mlpsp_status_reset")
@@ -793,7 +796,7 @@ class FrameRenderer:
     def bin_raycone(self, scene: PackedScene, rays_o, rays_d, threshold):
         """Ray-cone culling from the actual rays (scannet/camera.py:102-146): (ids, offsets, status bits)."""
         lib, d = self.lib, self.device
-        with torch.cuda.device(d):
+        with _on(d):
             st = _stream_ptr(d)
             for _attempt in range(3):
                 L.check(lib.mlpsp_status_reset(L.ptr(self.status), st), "mlpsp_status_reset")
@@ -812,7 +815,7 @@ class FrameRenderer:
 
     def sort(self, scene: PackedScene, rays_o, rays_d_unit, pairs, want_keys=False, sort_key=0, hit_arith=0):
         lib, d = self.lib, self.device
-        with torch.cuda.device(d):
+        with _on(d):
             st = _stream_ptr(d)
             f = self._frame(scene, rays_o, rays_d_unit, 0.5, 0, None, None, None, False, False, None, sort_key=sort_key,
                             hit_arith=hit_arith)
@@ -822,7 +825,7 @@ class FrameRenderer:
 
     def hit_masks(self, scene: PackedScene, rays_o, rays_d_unit, threshold, pairs, hit_arith=0):
         lib, d = self.lib, self.device
-        with torch.cuda.device(d):
+        with _on(d):
             st = _stream_ptr(d)
             f = self._frame(scene, rays_o, rays_d_unit, threshold, 0, None, None, None, False, False, None, hit_arith=hit_arith)
             out = torch.zeros(max(pairs, 1), device=d, dtype=torch.int64)
@@ -866,7 +869,7 @@ class ViewBatchRenderer:
         if precision is None:
             precision = L.PRECISION_F16 if scene.has_f16 else L.PRECISION_F32
         auto, idle_tail = waves is None, False
-        with torch.cuda.device(d):
+        with _on(d):
             st = _stream_ptr(d)
             rds = []
             for v, r in enumerate(self.views):

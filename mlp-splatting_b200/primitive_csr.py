@@ -11,6 +11,7 @@ from dataclasses import dataclass
 import torch
 
 from . import _lib as L
+from .engine import _on, _stream_ptr
 
 
 @dataclass
@@ -34,8 +35,8 @@ def _group(primitive_ids, num_primitives, x6=None, grad4=None, relu_masks=None):
     outs = [None if t is None else torch.empty_like(t) for t in (x6, grad4, relu_masks)]
     nbytes = int(lib.mlpsp_group_records_scratch_bytes(R, n))
     scratch = torch.empty(nbytes, device=dev, dtype=torch.uint8)
-    with torch.cuda.device(dev):
-        st = C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
+    with _on(dev):
+        st = _stream_ptr(dev)
         L.check(lib.mlpsp_group_rows(L.ptr(ids), R, n, L.ptr(x6), L.ptr(grad4), L.ptr(relu_masks), L.ptr(offsets), L.ptr(order),
                                      *(L.ptr(t) for t in outs), L.ptr(scratch), nbytes, st), "mlpsp_group_rows")
     return offsets, order, outs
@@ -90,8 +91,8 @@ def primitive_records_reverse(ids, offsets, x6, raw, log_scales, quats, grad_rgb
     nbytes = int(lib.mlpsp_records_reverse_scratch_bytes(total, n))
     scratch = torch.empty(nbytes, device=dev, dtype=torch.uint8)
     found = C.c_int32(0)
-    with torch.cuda.device(dev):
-        st = C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
+    with _on(dev):
+        st = _stream_ptr(dev)
         L.check(lib.mlpsp_records_reverse_checked(
             L.ptr(ids), L.ptr(offsets), L.ptr(x6), L.ptr(raw), L.ptr(log_scales), L.ptr(quats), L.ptr(grad_rgb), L.ptr(grad_t),
             pixels, total, n, L.ptr(d4), L.ptr(gp), L.ptr(gs), L.ptr(gq), L.ptr(scratch), nbytes, C.byref(found), st),

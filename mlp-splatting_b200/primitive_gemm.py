@@ -17,6 +17,7 @@ from dataclasses import dataclass
 import torch
 
 from . import _lib as L
+from .engine import _on, _stream_ptr
 
 
 @dataclass(frozen=True)
@@ -64,8 +65,8 @@ def prepare_groups(csr, segment_size=512):
     n = int(csr.offsets.numel()) - 1
     group_offsets = torch.empty(n + 1, device=dev, dtype=torch.int64)
     total = C.c_int64(0)
-    with torch.cuda.device(dev):
-        st = C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
+    with _on(dev):
+        st = _stream_ptr(dev)
         L.check(lib.mlpsp_prepare_groups(L.ptr(csr.offsets), n, segment_size, L.ptr(group_offsets), None, None, 0,
                                          C.byref(total), st), "mlpsp_prepare_groups")
         G = int(total.value)
@@ -113,8 +114,8 @@ def grouped_forward(csr_offsets, x6, scene, *, dtype=torch.float16):
     nbytes = int(lib.mlpsp_mlp_grouped_scratch_bytes(R, scene.n))
     scratch = torch.empty(nbytes, device=dev, dtype=torch.uint8)
     status = torch.zeros(L.STATUS_WORDS, device=dev, dtype=torch.int32)
-    with torch.cuda.device(dev):
-        st = C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
+    with _on(dev):
+        st = _stream_ptr(dev)
         prec = L.PRECISION_F16 if dtype == torch.float16 else L.PRECISION_F32
         L.check(lib.mlpsp_mlp_grouped(C.byref(scene.c), prec, L.ptr(csr_offsets), L.ptr(x6), R, L.ptr(out),
                                       L.ptr(scratch), nbytes, L.ptr(status), st), "mlpsp_mlp_grouped")
@@ -226,8 +227,8 @@ def grouped_weight_gradients(csr, freq, attenuation, weights, *, dtype=torch.flo
         grads = [torch.empty_like(w) for w in weights]
         scratch = torch.empty(nbytes, device=dev, dtype=torch.uint8)
         word = C.c_int32(0)
-        with torch.cuda.device(dev):
-            st = C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
+        with _on(dev):
+            st = _stream_ptr(dev)
             L.check(lib.mlpsp_weight_gradients(
                 C.byref(sc), L.ptr(csr.offsets), L.ptr(csr.x6), L.ptr(csr.grad4), L.ptr(csr.relu_masks), R, int(segment_size),
                 precisions[operand_dtype], float(operand_scale), *(L.ptr(g) for g in grads), L.ptr(scratch), nbytes,
