@@ -341,19 +341,33 @@ __device__ __forceinline__ void hit_chunk(const HitPixels& h, const float* __res
   }
 }
 
+// A launch serves up to kViewsPerLaunch views of a batch, a row of CTAs each (blockIdx.y): launched view by view, the later waves of
+// a batch, a few microseconds of work per view, were mostly launches, and each view ended in a tail of its own (four 500k views of
+// 1200 x 680: 4,006 -> 3,720 us, three 200k views of 640 x 480: 1,830 -> 1,687).  Arguments travel by value, 300 bytes a view.
+constexpr int kViewsPerLaunch = 8;
+template <typename A, int V>
+struct Views { A v[V]; int count; };
+template <int V> __device__ __forceinline__ int view_of_cta() { return V == 1 ? 0 : (int)blockIdx.y; }
+
 struct HitArgs {
   const float* rays_o; const float* rays_d; const float4* geom; int n;
   const int32_t* tile_offsets; const int32_t* tile_len; const int32_t* sorted_prims; int W, H, ntx;
   float thr, bound2, K;            // K <= 0: no quadratic form (thresholds the exponential underflows at)
   const int32_t* active; const int32_t* active_count; int lo, hi;
   const float4* px_state; uint2* masks; uint32_t* pair_base; int32_t* prim_cnt; int32_t* counters; int64_t max_records;
-  int32_t* status; int32_t* next_count; int add_tiles;      // add_tiles: a view of a batch that is not its first
+  int32_t* status; int32_t* next_count; int add_tiles;      // add_tiles: a launch for a batch that is not its first
 };
 
-// the wave's counters start at zero, and the list its compositing pass will append to starts empty
-__device__ __forceinline__ void reset_wave(const HitArgs& a) {
-  *a.next_count = 0;
-  a.counters[kCtrWaveTiles] = *a.active_count + (a.add_tiles ? a.counters[kCtrWaveTiles] : 0);
+// the wave's counters start at zero, and the lists its compositing pass will append to start empty
+template <int V>
+__device__ __forceinline__ void reset_wave(const Views<HitArgs, V>& b) {
+  const HitArgs& a = b.v[0];
+  int tiles = a.add_tiles ? a.counters[kCtrWaveTiles] : 0;
+  for (int v = 0; v < (V == 1 ? 1 : b.count); ++v) {
+    *b.v[v].next_count = 0;
+    tiles += *b.v[v].active_count;
+  }
+  a.counters[kCtrWaveTiles] = tiles;
   a.counters[kCtrWork] = 0; a.counters[kCtrWorkSmall] = 0; a.counters[kCtrWorkNext] = 0; a.counters[kCtrWaveRecords] = 0;
 }
 
@@ -374,13 +388,14 @@ __device__ __forceinline__ int warp_inclusive_scan(int v) {
 // and a CTA per tile beyond took 72 us of a 60k-primitive 639 x 477 frame and 1,454 of four 1M views at 1920 x 1080, this
 // 58 and 1,374.
 constexpr int kHitWarps = 4, kHitParts = 8;
-template <bool REF, bool LOOP>
-__global__ void __launch_bounds__(32 * kHitWarps) k_hits(const HitArgs a, int parts) {
+template <bool REF, bool LOOP, int V>
+__global__ void __launch_bounds__(32 * kHitWarps) k_hits(const __grid_constant__ Views<HitArgs, V> b, int parts) {
   chain_wait();
   chain_release();
   __shared__ float4 s_q[kHitWarps][64];
+  const HitArgs& a = b.v[view_of_cta<V>()];
   if (a.status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
-  if (blockIdx.x == 0 && threadIdx.x == 0) reset_wave(a);
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) reset_wave<V>(b);
   const int lane = threadIdx.x & 31, warp = warp_of_cta(), wpb = blockDim.x >> 5;
   const int units = *a.active_count * parts;
   for (int unit = blockIdx.x * wpb + warp; unit < units; unit += gridDim.x * wpb) {
@@ -414,15 +429,34 @@ __global__ void __launch_bounds__(32 * kHitWarps) k_hits(const HitArgs a, int pa
   }
 }
 
-static int launch_hits(const HitArgs& a, bool ref_arith, int tiles, int sms, bool idle_tail, cudaStream_t st) {
+// one launch for the views args[0 .. count)
+template <int V, typename A, typename... KArgs>
+static cudaError_t launch_views(void (*kernel)(Views<A, V>, KArgs...), dim3 grid, dim3 block, cudaStream_t st, const A* args, int count, KArgs... rest) {
+  Views<A, V> b = {};
+  b.count = count;
+  for (int v = 0; v < count; ++v) b.v[v] = args[v];
+  grid.y = (unsigned)count;
+  return launch_chained(kernel, grid, block, 0, st, b, rest...);
+}
+
+static int launch_hits(const HitArgs* args, int views, bool ref_arith, int tiles, int sms, bool idle_tail, cudaStream_t st) {
+  const HitArgs& a = args[0];
   const int parts = std::min((a.hi - a.lo + 31) / 32, kHitParts);
   // small images spread their tiles over the SMs one warp at a time
   const int64_t units = (int64_t)tiles * parts;
-  const int wpb = units >= sms * 2 * kHitWarps ? kHitWarps : 1;
+  const int wpb = units * views >= sms * 2 * kHitWarps ? kHitWarps : 1;
   const dim3 grid((unsigned)std::min<int64_t>((units + wpb - 1) / wpb, idle_tail ? sms : sms * 16)), block(32 * wpb);
   const bool loop = (a.hi - a.lo + 31) / 32 > parts;
-  auto* kernel = ref_arith ? (loop ? k_hits<true, true> : k_hits<true, false>) : (loop ? k_hits<false, true> : k_hits<false, false>);
-  return cuda_check(launch_chained(kernel, grid, block, 0, st, a, parts), "hits");
+  cudaError_t e = cudaSuccess;
+  if (views == 1) {
+    auto* kernel = ref_arith ? (loop ? k_hits<true, true, 1> : k_hits<true, false, 1>) : (loop ? k_hits<false, true, 1> : k_hits<false, false, 1>);
+    e = launch_views<1>(kernel, grid, block, st, args, 1, parts);
+  } else {
+    constexpr int N = kViewsPerLaunch;
+    auto* kernel = ref_arith ? (loop ? k_hits<true, true, N> : k_hits<true, false, N>) : (loop ? k_hits<false, true, N> : k_hits<false, false, N>);
+    e = launch_views<N>(kernel, grid, block, st, args, views, parts);
+  }
+  return cuda_check(e, "hits");
 }
 
 // Geometric hit masks of all pairs (no transmittance state): the superset the waves draw from.
@@ -614,11 +648,12 @@ struct FillArgs {
   int width, chunks, halves;                              // candidates per unit, units per window and half, 2: a unit is one half
 };
 
-template <int MODE>
-__global__ void __launch_bounds__(32 * kFillWarps, 4) k_fill(const FillArgs a) {
+template <int MODE, int V>
+__global__ void __launch_bounds__(32 * kFillWarps, 4) k_fill(const __grid_constant__ Views<FillArgs, V> b) {
   chain_wait();
   chain_release();
   __shared__ FillSmem s_all[kFillWarps];
+  const FillArgs& a = b.v[view_of_cta<V>()];
   if (a.status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
   const int lane = threadIdx.x & 31, warp = warp_of_cta(), wpb = blockDim.x >> 5;
   FillSmem& sm = s_all[warp];
@@ -765,18 +800,24 @@ __global__ void __launch_bounds__(32 * kFillWarps, 4) k_fill(const FillArgs a) {
   }
 }
 
-static int launch_fill(FillArgs a, bool exact, bool ref_arith, int tiles, int sms, bool idle_tail, cudaStream_t st) {
+static int launch_fill(FillArgs* args, int views, bool exact, bool ref_arith, int tiles, int sms, bool idle_tail, cudaStream_t st) {
   // 16 candidates per warp balance best on large frames (32: 957, 16: 939, 8: 1,000 us for the whole 100k frame); with few
   // tiles the window is cut finer, so that the SMs get more and shorter warps
-  const bool small = (int64_t)tiles * ((a.hi - a.lo + 15) / 16) < (int64_t)sms * 8;
-  a.width = small ? 8 : 16;
-  a.halves = small ? 2 : 1;
-  a.chunks = (a.hi - a.lo + a.width - 1) / a.width;
-  const int64_t units = (int64_t)tiles * a.chunks * a.halves;
-  const int wpb = units >= sms * 2 * kFillWarps ? kFillWarps : 1;
-  const int grid = (int)std::min<int64_t>((units + wpb - 1) / wpb, idle_tail ? sms : sms * 32);
-  auto* kernel = ref_arith ? k_fill<2> : (exact ? k_fill<1> : k_fill<0>);
-  return cuda_check(launch_chained(kernel, dim3(grid), dim3(32 * wpb), 0, st, a), "fill");
+  const int window = args[0].hi - args[0].lo;
+  const bool small = (int64_t)tiles * views * ((window + 15) / 16) < (int64_t)sms * 8;
+  const int width = small ? 8 : 16, halves = small ? 2 : 1, chunks = (window + width - 1) / width;
+  for (int v = 0; v < views; ++v) { args[v].width = width; args[v].halves = halves; args[v].chunks = chunks; }
+  const int64_t units = (int64_t)tiles * chunks * halves;
+  const int wpb = units * views >= sms * 2 * kFillWarps ? kFillWarps : 1;
+  const dim3 grid((unsigned)std::min<int64_t>((units + wpb - 1) / wpb, idle_tail ? sms : sms * 32)), block(32 * wpb);
+  cudaError_t e = cudaSuccess;
+  if (views == 1) {
+    e = launch_views<1>(ref_arith ? k_fill<2, 1> : (exact ? k_fill<1, 1> : k_fill<0, 1>), grid, block, st, args, 1);
+  } else {
+    constexpr int N = kViewsPerLaunch;
+    e = launch_views<N>(ref_arith ? k_fill<2, N> : (exact ? k_fill<1, N> : k_fill<0, N>), grid, block, st, args, views);
+  }
+  return cuda_check(e, "fill");
 }
 
 // --------------------------------------------------------------------------- composite ----
@@ -786,19 +827,30 @@ struct PrimStats {
   float* sum_w; float* max_w; int32_t* hits; float* sum_werr; int32_t* contrib;
 };
 
-template <bool STATS>
-__global__ void __launch_bounds__(64) k_composite(
-    PrimStats ps,
-    const int32_t* __restrict__ tile_offsets, const int32_t* __restrict__ tile_len, int W, int H, int ntx, const int32_t* __restrict__ active,
-    const int32_t* __restrict__ active_count, int lo, int hi, const uint32_t* __restrict__ masks32,
-    const uint32_t* __restrict__ pair_base, const float4* __restrict__ rec_out, const float* __restrict__ rec_t,
-    float4* __restrict__ px_state, float2* __restrict__ px_depth, float* __restrict__ rgb,
-    float* __restrict__ alpha, float* __restrict__ depth_t, uint32_t* __restrict__ mask_used32,
-    float* __restrict__ rec_w, float* __restrict__ rec_tr, float bgr, float bgg, float bgb, int has_bg,
-    int32_t* __restrict__ next_active,
-    int32_t* __restrict__ next_count, int32_t* __restrict__ status) {
+struct CompositeArgs {
+  PrimStats ps;
+  const int32_t* tile_offsets; const int32_t* tile_len; int W, H, ntx; const int32_t* active; const int32_t* active_count; int lo, hi;
+  const uint32_t* masks32; const uint32_t* pair_base; const float4* rec_out; const float* rec_t; float4* px_state; float2* px_depth;
+  float* rgb; float* alpha; float* depth_t; uint32_t* mask_used32; float* rec_w; float* rec_tr; float bgr, bgg, bgb; int has_bg;
+  int32_t* next_active; int32_t* next_count; int32_t* status;
+};
+
+template <bool STATS, int V>
+__global__ void __launch_bounds__(64) k_composite(const __grid_constant__ Views<CompositeArgs, V> views) {
   chain_wait();
   chain_release();
+  const CompositeArgs& a = views.v[view_of_cta<V>()];
+  const PrimStats& ps = a.ps;
+  const int32_t* __restrict__ tile_offsets = a.tile_offsets; const int32_t* __restrict__ tile_len = a.tile_len;
+  const int W = a.W, H = a.H, ntx = a.ntx, lo = a.lo, hi = a.hi, has_bg = a.has_bg;
+  const int32_t* __restrict__ active = a.active; const int32_t* __restrict__ active_count = a.active_count;
+  const uint32_t* __restrict__ masks32 = a.masks32; const uint32_t* __restrict__ pair_base = a.pair_base;
+  const float4* __restrict__ rec_out = a.rec_out; const float* __restrict__ rec_t = a.rec_t;
+  float4* __restrict__ px_state = a.px_state; float2* __restrict__ px_depth = a.px_depth;
+  float* __restrict__ rgb = a.rgb; float* __restrict__ alpha = a.alpha; float* __restrict__ depth_t = a.depth_t;
+  uint32_t* __restrict__ mask_used32 = a.mask_used32; float* __restrict__ rec_w = a.rec_w; float* __restrict__ rec_tr = a.rec_tr;
+  const float bgr = a.bgr, bgg = a.bgg, bgb = a.bgb;
+  int32_t* __restrict__ next_active = a.next_active; int32_t* __restrict__ next_count = a.next_count; int32_t* __restrict__ status = a.status;
   __shared__ int s_live[2];
   if (status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
   const int n_active = *active_count;
@@ -1436,7 +1488,7 @@ int launch_render_sorted(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scr
                           fr->threshold, miss_bound2(fr->threshold), form_threshold(fr->threshold), act, act_n, lo, hi, s.px_state,
                           reinterpret_cast<uint2*>(s.masks32), s.pair_base, s.prim_cnt + (size_t)(w & 1) * prim_cnt_stride(n), s.counters,
                           fr->max_records, fr->status, s.counters + kCtrActive0 + nxt, 0};
-      rc = launch_hits(ha, ref_arith, T, sms, idle_tail, st);
+      rc = launch_hits(&ha, 1, ref_arith, T, sms, idle_tail, st);
       if (rc) return rc;
     }
     rc = launch_prim_scan(s, n, nullptr, fr->status, st, split_small, w);
@@ -1444,11 +1496,11 @@ int launch_render_sorted(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scr
     {
       LaunchScope scope(kKFill, 1, st);
       float4* gate = (want_feat && sc->feat_slots > 1) ? s.rec_gate : nullptr;
-      const FillArgs fa = {fr->rays_o, fr->rays_d, (const float4*)sc->geom, fr->tile_offsets, s.tile_len, fr->sorted_prims, W, H, ntx,
+      FillArgs fa = {fr->rays_o, fr->rays_d, (const float4*)sc->geom, fr->tile_offsets, s.tile_len, fr->sorted_prims, W, H, ntx,
                            fr->threshold, act, act_n, lo, hi, reinterpret_cast<const uint2*>(s.masks32), s.pair_base,
                            s.prim_pos, reinterpret_cast<float4*>(s.rec_in), (want_t || per_pixel) ? s.rec_t : nullptr, gate,
                            sc->gate_beta, sc->gate_tau, keep ? 1 : 0, table ? 1 : 0, fr->status, 0, 0, 0};
-      rc = launch_fill(fa, gate || per_pixel, ref_arith, T, sms, idle_tail, st);
+      rc = launch_fill(&fa, 1, gate || per_pixel, ref_arith, T, sms, idle_tail, st);
       if (rc) return rc;
     }
     if (tc_path)
@@ -1467,19 +1519,14 @@ int launch_render_sorted(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scr
                                                                  want_feat ? s.rec_w : nullptr, fr->status);
       break;
     }
-    { LaunchScope scope(kKComposite, 1, st);
-    if (want_stats)
-      launch_chained(k_composite<true>, dim3(grid_comp), dim3(64), 0, st, pstats, fr->tile_offsets, s.tile_len, W, H, ntx, act, act_n, lo, hi, s.masks32, s.pair_base,
-                                  s.rec_out, want_t ? s.rec_t : nullptr, s.px_state, s.px_depth, fr->rgb,
-                                  fr->alpha, fr->depth_t, used32, want_feat ? s.rec_w : nullptr,
-                                  keep ? s.rec_tr : nullptr, bg[0], bg[1], bg[2], has_bg,
-                                  s.active[nxt], s.counters + kCtrActive0 + nxt, fr->status);
-    else
-    launch_chained(k_composite<false>, dim3(grid_comp), dim3(64), 0, st, pstats, fr->tile_offsets, s.tile_len, W, H, ntx, act, act_n, lo, hi, s.masks32, s.pair_base,
-                                  s.rec_out, want_t ? s.rec_t : nullptr, s.px_state, s.px_depth, fr->rgb,
-                                  fr->alpha, fr->depth_t, used32, want_feat ? s.rec_w : nullptr,
-                                  keep ? s.rec_tr : nullptr, bg[0], bg[1], bg[2], has_bg,
-                                  s.active[nxt], s.counters + kCtrActive0 + nxt, fr->status); }
+    {
+      LaunchScope scope(kKComposite, 1, st);
+      const CompositeArgs ca = {pstats, fr->tile_offsets, s.tile_len, W, H, ntx, act, act_n, lo, hi, s.masks32, s.pair_base,
+                                s.rec_out, want_t ? s.rec_t : nullptr, s.px_state, s.px_depth, fr->rgb, fr->alpha, fr->depth_t, used32,
+                                want_feat ? s.rec_w : nullptr, keep ? s.rec_tr : nullptr, bg[0], bg[1], bg[2], has_bg,
+                                s.active[nxt], s.counters + kCtrActive0 + nxt, fr->status};
+      launch_views<1>(want_stats ? k_composite<true, 1> : k_composite<false, 1>, dim3(grid_comp), dim3(64), st, &ca, 1);
+    }
     lo = hi;
   }
   if (fr->mask_used && used32 != (uint32_t*)fr->mask_used)
@@ -1550,7 +1597,7 @@ int launch_render_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scr
   // (measured with and without: fourview_500k in one batch of 4 views 2.51 -> 2.31 ms, stress_2m in batches of 16
   // views 72.2 -> 65.8 ms of evaluator time)
   const bool split_small = tc_path && (int64_t)n * 20 > P * V;
-  const int sms = sm_count();
+  const int sms = sm_count(), groups = (V + kViewsPerLaunch - 1) / kViewsPerLaunch;
   const int nw = f0->num_waves > 0 ? f0->num_waves : (int)(sizeof(kDefaultWaves) / sizeof(int));
   int lo = 0;
   for (int w = 0; w < nw && lo < f0->tile_capacity; ++w) {
@@ -1565,15 +1612,18 @@ int launch_render_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scr
     int32_t* cnt = lead.prim_cnt + (size_t)(w & 1) * prim_cnt_stride(n);
     int rc = MLPSP_OK;
     {
-      LaunchScope scope(kKHits, V, st);
+      LaunchScope scope(kKHits, groups, st);
+      HitArgs ha[kViewsPerLaunch];
       for (int v = 0; v < V; ++v) {
         const mlpsp_frame* fr = frs + v;
         const Scratch& s = ss[v];
-        const HitArgs ha = {fr->rays_o, fr->rays_d, (const float4*)sc->geom, n, fr->tile_offsets, s.tile_len, fr->sorted_prims, W, H, ntx,
+        const int q = v % kViewsPerLaunch;
+        ha[q] = {fr->rays_o, fr->rays_d, (const float4*)sc->geom, n, fr->tile_offsets, s.tile_len, fr->sorted_prims, W, H, ntx,
                             f0->threshold, miss_bound2(f0->threshold), form_threshold(f0->threshold), s.active[cur],
                             s.counters + kCtrActive0 + cur, lo, hi, s.px_state, reinterpret_cast<uint2*>(s.masks32), s.pair_base, cnt,
                             lead.counters, f0->max_records, f0->status, s.counters + kCtrActive0 + nxt, v > 0 ? 1 : 0};
-        rc = launch_hits(ha, ref_arith, T, sms, idle_tail, st);
+        if (q + 1 < kViewsPerLaunch && v + 1 < V) continue;
+        rc = launch_hits(ha, q + 1, ref_arith, T, sms, idle_tail, st);
         if (rc) return rc;
       }
     }
@@ -1581,15 +1631,18 @@ int launch_render_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scr
     if (rc) return rc;
     {
       // (no table of ray directions: the records of a launch come from all views, and would have to name theirs)
-      LaunchScope scope(kKFill, V, st);
+      LaunchScope scope(kKFill, groups, st);
+      FillArgs fa[kViewsPerLaunch];
       for (int v = 0; v < V; ++v) {
         const mlpsp_frame* fr = frs + v;
         const Scratch& s = ss[v];
-        const FillArgs fa = {fr->rays_o, fr->rays_d, (const float4*)sc->geom, fr->tile_offsets, s.tile_len, fr->sorted_prims, W, H, ntx,
+        const int q = v % kViewsPerLaunch;
+        fa[q] = {fr->rays_o, fr->rays_d, (const float4*)sc->geom, fr->tile_offsets, s.tile_len, fr->sorted_prims, W, H, ntx,
                              f0->threshold, s.active[cur], s.counters + kCtrActive0 + cur, lo, hi,
                              reinterpret_cast<const uint2*>(s.masks32), s.pair_base, lead.prim_pos, reinterpret_cast<float4*>(lead.rec_in),
                              nullptr, nullptr, sc->gate_beta, sc->gate_tau, 0, 0, f0->status, 0, 0, 0};
-        rc = launch_fill(fa, false, ref_arith, T, sms, idle_tail, st);
+        if (q + 1 < kViewsPerLaunch && v + 1 < V) continue;
+        rc = launch_fill(fa, q + 1, false, ref_arith, T, sms, idle_tail, st);
         if (rc) return rc;
       }
     }
@@ -1600,17 +1653,21 @@ int launch_render_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scr
       rc = launch_mlp_f32(sc, lead.rec_in, lead.work, lead.counters, lead.rec_out, nullptr, kOutAlpha, f0->status, st, cap_mlp);
     if (rc) return rc;
     {
-      LaunchScope scope(kKComposite, V, st);
+      LaunchScope scope(kKComposite, groups, st);
+      CompositeArgs ca[kViewsPerLaunch];
       for (int v = 0; v < V; ++v) {
         const mlpsp_frame* fr = frs + v;
         const Scratch& s = ss[v];
         float bg[3] = {0.f, 0.f, 0.f};
         const int has_bg = fr->bg_color != nullptr;
         if (has_bg) { bg[0] = fr->bg_color[0]; bg[1] = fr->bg_color[1]; bg[2] = fr->bg_color[2]; }
-        launch_chained(k_composite<false>, dim3(grid_comp), dim3(64), 0, st, no_stats, fr->tile_offsets, s.tile_len, W, H, ntx, s.active[cur],
-                                                     s.counters + kCtrActive0 + cur, lo, hi, s.masks32, s.pair_base, lead.rec_out, nullptr,
-                                                     s.px_state, s.px_depth, fr->rgb, fr->alpha, nullptr, nullptr, nullptr, nullptr, bg[0],
-                                                     bg[1], bg[2], has_bg, s.active[nxt], s.counters + kCtrActive0 + nxt, f0->status);
+        const int q = v % kViewsPerLaunch;
+        ca[q] = {no_stats, fr->tile_offsets, s.tile_len, W, H, ntx, s.active[cur], s.counters + kCtrActive0 + cur, lo, hi, s.masks32,
+                 s.pair_base, lead.rec_out, nullptr, s.px_state, s.px_depth, fr->rgb, fr->alpha, nullptr, nullptr, nullptr, nullptr,
+                 bg[0], bg[1], bg[2], has_bg, s.active[nxt], s.counters + kCtrActive0 + nxt, f0->status};
+        if (q + 1 < kViewsPerLaunch && v + 1 < V) continue;
+        if (q == 0) launch_views<1>(k_composite<false, 1>, dim3(grid_comp), dim3(64), st, ca, 1);
+        else launch_views<kViewsPerLaunch>(k_composite<false, kViewsPerLaunch>, dim3(grid_comp), dim3(64), st, ca, q + 1);
       }
     }
     lo = hi;

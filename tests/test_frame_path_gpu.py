@@ -292,3 +292,31 @@ def test_decoder_queues_layer_one_behind_the_last_output_chunk(out_dim, classes,
     assert np.abs(dec.decode_hwc(_t(x)).cpu().numpy() - want).max() <= 2e-3
     labels, margin = orc.classify_features(want, text)
     assert not (dec.classify(_t(x), _t(text)).cpu().numpy() != labels)[margin > 2e-3].any()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("views,n,mu,W,H", [(1, 300, -3.0, 17, 9), (2, 8192, -5.0, 129, 95), (8, 40, -2.5, 40, 24), (9, 9000, -5.0, 113, 90),
+                                            (17, 500, -3.2, 33, 17)])
+def test_batches_at_the_edges_of_a_launch(precision, views, n, mu, W, H):
+    """One view, a full launch of eight and one beyond it, raw and normalised rays, against the frames rendered alone (the same
+    arithmetic per record, hence equal bits); windows of which the last ones find no live tiles."""
+    from mlp_splatting_b200 import synthetic
+    from mlp_splatting_b200.engine import FrameRenderer, ViewBatchRenderer, normalize_rows
+    scene = synthetic.make_scene(n, 5, mu=mu)
+    ps, single = _packed(scene), FrameRenderer(W, H, device=DEV, tile_capacity=2048)
+    cams = [synthetic.make_camera(W, H, azimuth_deg=31.0 * v) for v in range(views)]
+    ros, rds = [_t(c["rays_o"]) for c in cams], [_t(c["rays_d"]) for c in cams]
+    vs, prs = [c["view"] for c in cams], [c["proj"] for c in cams]
+    want, pairs, records = [], 0, 0
+    for v in range(views):
+        rgb, alpha = single.render(ps, ros[v], rds[v], THR, view=vs[v], proj=prs[v], precision=precision, waves=[16, 64, 512, 1024])
+        want.append((rgb.clone(), alpha.clone()))
+        pairs, records = single.last_stats.pairs, records + single.last_stats.records
+    batch = ViewBatchRenderer(W, H, views, device=DEV, tile_capacity=2048)
+    for normalized in (False, True):
+        got = batch.render(ps, ros, [normalize_rows(d) for d in rds] if normalized else rds, THR, vs, prs, precision=precision,
+                           waves=[16, 64, 512, 1024], rays_normalized=normalized)
+        for (rgb, alpha), (rgb_w, alpha_w) in zip(got, want):
+            assert torch.equal(rgb, rgb_w) and torch.equal(alpha, alpha_w)
+        assert batch.last_stats.records == records and batch.last_stats.pairs == pairs      # the pairs are the last view's
+    assert records > 0
