@@ -267,7 +267,7 @@ static int render_frame(const mlpsp_scene* sc, const mlpsp_frame* fr, const floa
   // consumed-record masks are indexed by position in the full sorted list, so the pre-test stays off for them
   const bool pretest = fr->tile_pretest == 0 && fr->mask_used == nullptr && fr->tile == 8;
   if (pretest) {
-    rc = launch_frame_begin(sc, fr, s, rays_raw, reset_status, s.prim_cnt, st);
+    rc = launch_frame_begin(sc, fr, &s, 1, &rays_raw, reset_status, st);
     if (rc) return rc;
   } else {
     if (reset_status) MLPSP_CUDA_OK(cudaMemsetAsync(fr->status, 0, 4 * MLPSP_STATUS_WORDS, st));
@@ -324,13 +324,20 @@ extern "C" int mlpsp_render_frames(const mlpsp_scene* sc, const mlpsp_frame* fra
   MLPSP_REQUIRE(f0->num_waves >= 0 && f0->num_waves <= MLPSP_MAX_WAVES, MLPSP_E_ARG, "render: bad num_waves");
   cudaStream_t st = (cudaStream_t)stream;
   const bool pretest = f0->tile_pretest == 0;
+  if (pretest) {
+    const int rc = launch_frame_begin(sc, frames, ss.data(), num_frames, nullptr, false, st);
+    if (rc) return rc;
+  }
+  if (pretest && sc->n > 0 && num_frames > 1 && bin_uses_corners(f0)) {
+    int rc = launch_bin_batch(sc, frames, ss.data(), num_frames, st);
+    if (!rc) rc = launch_sort_batch(sc, frames, ss.data(), num_frames, st);
+    if (rc) return rc;
+    return launch_render_batch(sc, frames, ss.data(), num_frames, st, true);
+  }
   for (int v = 0; v < num_frames; ++v) {
     const mlpsp_frame* fr = frames + v;
     const Scratch& s = ss[(size_t)v];
-    int rc = MLPSP_OK;
-    if (pretest) rc = launch_frame_begin(sc, fr, s, nullptr, false, v == 0 ? s.prim_cnt : nullptr, st);
-    if (rc) return rc;
-    rc = launch_bin(sc, fr, s, st, /*order_lists=*/false, pretest);
+    int rc = launch_bin(sc, fr, s, st, /*order_lists=*/false, pretest);
     if (rc) return rc;
     rc = launch_sort(sc, fr, nullptr, st, /*unordered_input=*/true, s.counters + kCtrScratch + 2,
                      pretest ? s.tile_len : nullptr);

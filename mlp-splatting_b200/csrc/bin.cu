@@ -210,14 +210,18 @@ __global__ void __launch_bounds__(256) k_bin_count(const float4* __restrict__ ge
 // mats (optional): the view and projection matrices in device memory, in place of the camera's own.
 // OWN: a CTA per SM adds its primitives' corners up in shared memory and then to the array, whole lines at a time.
 // Bound by the scattered atomics otherwise; launch_bin has the rule (four views of 500k primitives: 265 -> 56 us).
-template <bool OWN>
-__global__ void __launch_bounds__(OWN ? 1024 : 256) k_bin_corners(const float4* __restrict__ geom, int n, const BinCam host_cam,
-                                                                  const BinMats mats, uint2* __restrict__ rect, int32_t* __restrict__ diff) {
+struct CornerArgs { BinCam cam; BinMats mats; uint2* rect; int32_t* diff; };
+template <bool OWN, int V>
+__global__ void __launch_bounds__(OWN ? 1024 : 256) k_bin_corners(const __grid_constant__ Views<CornerArgs, V> views,
+                                                                  const float4* __restrict__ geom, int n) {
   chain_wait();
   chain_release();
   extern __shared__ int32_t s_diff[];
   __shared__ BinCam cam;
-  device_camera(cam, host_cam, mats);
+  const CornerArgs& a = views.v[view_of_cta<V>()];
+  uint2* __restrict__ rect = a.rect;
+  int32_t* __restrict__ diff = a.diff;
+  device_camera(cam, a.cam, a.mats);
   const int sx = cam.ntx + 1, cells = sx * (cam.nty + 1);
   int32_t* dst = OWN ? s_diff : diff;
   if (OWN) {
@@ -249,9 +253,14 @@ __global__ void __launch_bounds__(OWN ? 1024 : 256) k_bin_corners(const float4* 
 // time, so that reads and writes of both memories follow one another (a run of tiles per thread had them 32 to a bank at
 // 1920 x 1080: 41 us, now 21; 1200 x 680: 14 and 11).
 constexpr int kBinMaxRows = 1024;          // rows of tiles, one per thread
-__global__ void __launch_bounds__(1024) k_bin_offsets(const int32_t* __restrict__ diff, int ntx, int nty,
-                                                      int32_t* __restrict__ tile_offsets, int capacity, int64_t max_pairs,
-                                                      int32_t* __restrict__ status, int32_t* __restrict__ counters) {
+// report: the status block's pair total is this view's
+struct OffsetArgs { const int32_t* diff; int32_t* tile_offsets; int64_t max_pairs; int32_t* status; int32_t* counters; int report; };
+template <int V>
+__global__ void __launch_bounds__(1024) k_bin_offsets(const __grid_constant__ Views<OffsetArgs, V> views, int ntx, int nty, int capacity) {
+  const OffsetArgs& a = views.v[view_of_cta<V>()];
+  const int32_t* __restrict__ diff = a.diff;
+  int32_t* __restrict__ tile_offsets = a.tile_offsets;
+  int32_t* __restrict__ status = a.status;
   extern __shared__ int32_t s_cnt[];          // [(nty + 1)][(ntx + 1)]
   __shared__ int s_row[kBinMaxRows];          // pairs of a row, then of the rows before it
   __shared__ int warp_sums[32];
@@ -316,9 +325,9 @@ __global__ void __launch_bounds__(1024) k_bin_offsets(const int32_t* __restrict_
   }
   if (tid == 0) {
     tile_offsets[T] = total;
-    status[MLPSP_ST_PAIRS] = total;
-    counters[kCtrPairs] = total;
-    if (total < 0 || (int64_t)total > max_pairs) atomicOr(status + MLPSP_ST_BITS, MLPSP_ST_PAIR_OVERFLOW);
+    if (a.report) status[MLPSP_ST_PAIRS] = total;
+    a.counters[kCtrPairs] = total;
+    if (total < 0 || (int64_t)total > a.max_pairs) atomicOr(status + MLPSP_ST_BITS, MLPSP_ST_PAIR_OVERFLOW);
   }
 }
 
@@ -329,21 +338,29 @@ __global__ void __launch_bounds__(1024) k_bin_offsets(const int32_t* __restrict_
 // each computes their ellipses into shared memory; a pair is then one 16-byte load and about thirty operations (against a
 // test of the whitened quadratic form per pair: 102 -> 52 us on the 100k frame, 2.9 million pairs).  With eight primitives of
 // two pairs each three quarters of the lanes idle through the ellipses (four 500k views: 272 us, with 32 205).
-template <bool PRETEST, int PPW>
-__global__ void __launch_bounds__(256) k_bin_scatter(int n, int ntx, const uint2* __restrict__ rect,
-                                                     const int32_t* __restrict__ tile_offsets,
-                                                     int32_t* __restrict__ tile_fill, int32_t* __restrict__ tile_prims,
-                                                     const float4* __restrict__ geom,
-                                                     const FramePlane* __restrict__ plane, const float4* __restrict__ tile_rect,
-                                                     float K0, const int32_t* __restrict__ status) {
+struct ScatterArgs {
+  const uint2* rect; const int32_t* tile_offsets; int32_t* tile_fill; int32_t* tile_prims; const FramePlane* plane;
+  const float4* tile_rect; const int32_t* counters; const int32_t* status;
+};
+template <bool PRETEST, int PPW, int V>
+__global__ void __launch_bounds__(256) k_bin_scatter(const __grid_constant__ Views<ScatterArgs, V> views, int n, int ntx,
+                                                     const float4* __restrict__ geom, float K0) {
   chain_wait();
   chain_release();
+  const ScatterArgs& a = views.v[view_of_cta<V>()];
+  const uint2* __restrict__ rect = a.rect;
+  const int32_t* __restrict__ tile_offsets = a.tile_offsets;
+  int32_t* __restrict__ tile_fill = a.tile_fill;
+  int32_t* __restrict__ tile_prims = a.tile_prims;
+  const FramePlane* __restrict__ plane = a.plane;
+  const float4* __restrict__ tile_rect = a.tile_rect;
+  const int32_t* __restrict__ status = a.status;
   __shared__ WarpRects s_wr[8];
   __shared__ float4 s_el[PRETEST ? 8 : 1][PRETEST ? 32 : 1][2];
   if (status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gwarp = blockIdx.x * 8 + warp;
-  const int ppw = PRETEST && (int64_t)status[MLPSP_ST_PAIRS] < 8 * (int64_t)n ? 32 : PPW;
+  const int ppw = PRETEST && (int64_t)a.counters[kCtrPairs] < 8 * (int64_t)n ? 32 : PPW;
   if ((int64_t)gwarp * ppw >= n) return;
   const int p = gwarp * ppw + lane;
   int x0 = 1, x1 = 0, y0 = 1, y1 = 0;
@@ -531,12 +548,8 @@ bool bin_uses_corners(const mlpsp_frame* fr) {
   return nty <= kBinMaxRows && 4 * (size_t)(ntx + 1) * (nty + 1) <= 200 * 1024;
 }
 
-int launch_bin(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, cudaStream_t st, bool order_lists,
-               bool pretest, const float* view_dev, const float* proj_dev) {
-  const int T = num_tiles(fr->width, fr->height, fr->tile);
-  BinCam cam;
-  const BinMats mats = {view_dev, proj_dev};
-  for (int i = 0; i < 16; ++i) { cam.view[i] = view_dev ? 0.f : fr->view[i]; cam.proj[i] = view_dev ? 0.f : fr->proj[i]; }
+static int bin_camera(const mlpsp_frame* fr, bool matrices, BinCam& cam) {
+  for (int i = 0; i < 16; ++i) { cam.view[i] = matrices ? fr->view[i] : 0.f; cam.proj[i] = matrices ? fr->proj[i] : 0.f; }
   cam.radius_mult = (float)sqrt(-2.0 * log((double)fr->threshold));
   cam.focal = bin_focal(cam.proj[0], cam.proj[5], fr->width, fr->height);
   cam.W = fr->width; cam.H = fr->height; cam.ts = fr->tile;
@@ -551,6 +564,43 @@ int launch_bin(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, c
   MLPSP_REQUIRE(cam.ntx < 65536 && cam.nty < 65536, MLPSP_E_LIMIT, "tile grid beyond 65535 per axis");
   MLPSP_REQUIRE(fr->tile_capacity > 0 && fr->tile_capacity <= kSortCap, MLPSP_E_LIMIT,
                 "tile_capacity must be in [1, %d]", kSortCap);
+  return MLPSP_OK;
+}
+
+static int corner_shared_memory() {
+  static DeviceOnce attr_once;
+  if (!attr_once.first()) return MLPSP_OK;
+  auto allow = [](const void* kernel) {
+    return cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024), "bin");
+  };
+  constexpr int N = kViewsPerLaunch;
+  const void* kernels[4] = {(const void*)k_bin_offsets<1>, (const void*)k_bin_offsets<N>, (const void*)k_bin_corners<true, 1>,
+                            (const void*)k_bin_corners<true, N>};
+  for (const void* k : kernels)
+    if (const int rc = allow(k)) return rc;
+  return MLPSP_OK;
+}
+
+// the count pass of n > 0 primitives for the given views: corners, then offsets
+template <int V>
+static void launch_corners(const float4* geom, int n, const CornerArgs* ca, const OffsetArgs* oa, int views, int capacity, cudaStream_t st) {
+  const int ntx = ca[0].cam.ntx, nty = ca[0].cam.nty, cells = (ntx + 1) * (nty + 1), sms = sm_count();
+  // an atomic of a warp on scattered cells is 32 sector operations, one on a line of cells four: the direct way costs 4 n
+  // of them, the arrays of the SMs sms * cells / 8; they win from about equal numbers on (100,000 primitives on 12,986
+  // cells: 20 us directly, 8 by arrays)
+  if (n >= 8192 && 32 * (int64_t)n >= (int64_t)sms * cells)
+    launch_views<V>(k_bin_corners<true, V>, dim3(sms), dim3(1024), 4 * (size_t)cells, st, ca, views, geom, n);
+  else if (n > 0)
+    launch_views<V>(k_bin_corners<false, V>, dim3((n + 255) / 256), dim3(256), 0, st, ca, views, geom, n);
+  launch_views<V>(k_bin_offsets<V>, dim3(1), dim3(1024), 4 * (size_t)cells, st, oa, views, ntx, nty, capacity);
+}
+
+int launch_bin(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, cudaStream_t st, bool order_lists,
+               bool pretest, const float* view_dev, const float* proj_dev) {
+  const int T = num_tiles(fr->width, fr->height, fr->tile);
+  BinCam cam;
+  const BinMats mats = {view_dev, proj_dev};
+  if (const int rc = bin_camera(fr, !view_dev, cam)) return rc;
   MLPSP_REQUIRE(!(pretest && order_lists), MLPSP_E_ARG, "bin: the tile pre-test leaves the lists in scatter order");
   MLPSP_REQUIRE(!pretest || (fr->tile == 8 && fr->rays_o && fr->rays_d), MLPSP_E_ARG,
                 "bin: the tile pre-test needs 8x8 tiles and the frame's rays");
@@ -567,38 +617,56 @@ int launch_bin(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, c
     MLPSP_CUDA_OK(cudaMemsetAsync(fill, 0, 4 * (size_t)T, st));
   }
   LaunchScope scope(kKBin, (n > 0 ? (order_lists ? 3 : 2) : 0) + (corners ? 1 : 1 + scan_launches(T)), st);
+  const float4* geom = (const float4*)sc->geom;
   if (corners) {
-    static DeviceOnce attr_once;
-    if (attr_once.first()) {
-      MLPSP_CUDA_OK(cudaFuncSetAttribute(k_bin_offsets, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-      MLPSP_CUDA_OK(cudaFuncSetAttribute(k_bin_corners<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    }
-    // an atomic of a warp on scattered cells is 32 sector operations, one on a line of cells four: the direct way costs 4 n
-    // of them, the arrays of the SMs sms * cells / 8; they win from about equal numbers on (100,000 primitives on 12,986
-    // cells: 20 us directly, 8 by arrays)
-    const int sms = sm_count();
-    if (n >= 8192 && 32 * (int64_t)n >= (int64_t)sms * (int64_t)(diff_bytes / 4))
-      launch_chained(k_bin_corners<true>, dim3(sms), dim3(1024), diff_bytes, st, (const float4*)sc->geom, n, cam, mats, s.rect, s.tile_diff);
-    else if (n > 0)
-      launch_chained(k_bin_corners<false>, dim3((n + 255) / 256), dim3(256), 0, st, (const float4*)sc->geom, n, cam, mats, s.rect, s.tile_diff);
-    launch_chained(k_bin_offsets, dim3(1), dim3(1024), diff_bytes, st, s.tile_diff, cam.ntx, cam.nty, fr->tile_offsets, fr->tile_capacity,
-                   fr->max_pairs, fr->status, s.counters);
+    if (const int rc = corner_shared_memory()) return rc;
+    const CornerArgs ca = {cam, mats, s.rect, s.tile_diff};
+    const OffsetArgs oa = {s.tile_diff, fr->tile_offsets, fr->max_pairs, fr->status, s.counters, 1};
+    launch_corners<1>(geom, n, &ca, &oa, 1, fr->tile_capacity, st);
   } else {
-    if (n > 0) launch_chained(k_bin_count, dim3((n + 255) / 256), dim3(256), 0, st, (const float4*)sc->geom, n, cam, mats, s.rect, s.tile_cnt);
+    if (n > 0) launch_chained(k_bin_count, dim3((n + 255) / 256), dim3(256), 0, st, geom, n, cam, mats, s.rect, s.tile_cnt);
     int rc = launch_scan_i32(s.tile_cnt, T, s.scan_blk, fr->tile_offsets, st);
     if (rc) return rc;
     launch_chained(k_bin_finish, dim3(std::min(64, (T + 255) / 256)), dim3(256), 0, st, s.tile_cnt, T, fr->tile_offsets, fr->tile_capacity,
                    fr->max_pairs, fr->status, s.counters);
   }
   if (n > 0) {
+    const ScatterArgs sa = {s.rect, fr->tile_offsets, fill, fr->tile_prims, s.plane, s.tile_rect, s.counters, fr->status};
     if (pretest)
-      launch_chained(k_bin_scatter<true, 8>, dim3((n + 63) / 64), dim3(256), 0, st, n, cam.ntx, s.rect, fr->tile_offsets, fill, fr->tile_prims,
-                                                           (const float4*)sc->geom, s.plane, s.tile_rect,
-                                                           (float)(-2.0 * log((double)fr->threshold)), fr->status);
+      launch_views<1>(k_bin_scatter<true, 8, 1>, dim3((n + 63) / 64), dim3(256), 0, st, &sa, 1, n, cam.ntx, geom,
+                      (float)(-2.0 * log((double)fr->threshold)));
     else
-      launch_chained(k_bin_scatter<false, 32>, dim3((n + 255) / 256), dim3(256), 0, st, n, cam.ntx, s.rect, fr->tile_offsets, fill, fr->tile_prims,
-                                                            nullptr, nullptr, nullptr, 0.f, fr->status);
+      launch_views<1>(k_bin_scatter<false, 32, 1>, dim3((n + 255) / 256), dim3(256), 0, st, &sa, 1, n, cam.ntx, geom, 0.f);
     if (order_lists) k_sort_ids<256, kSortCap><<<T, 256, 0, st>>>(fr->tile_offsets, fr->tile_prims, fr->status);
+  }
+  return cuda_check(cudaGetLastError(), "bin");
+}
+
+// The views of a batch side by side, not one behind the other: k_bin_offsets is one CTA per view, and each view's sort ends in a
+// tail of its long lists (with launch_sort_batch: four 500k views of 1200 x 680 3,720 -> 3,657 us for all of it, two 1M views of
+// 1920 x 1080 9,820 -> 9,550).
+int launch_bin_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scratch* ss, int views, cudaStream_t st) {
+  constexpr int N = kViewsPerLaunch;
+  const int n = sc->n;
+  const float4* geom = (const float4*)sc->geom;
+  if (const int rc = corner_shared_memory()) return rc;
+  LaunchScope scope(kKBin, 3 * ((views + N - 1) / N), st);
+  for (int v0 = 0; v0 < views; v0 += N) {
+    const int count = std::min(N, views - v0);
+    CornerArgs ca[N];
+    OffsetArgs oa[N];
+    ScatterArgs sa[N];
+    for (int q = 0; q < count; ++q) {
+      const mlpsp_frame* fr = frs + v0 + q;
+      const Scratch& s = ss[v0 + q];
+      if (const int rc = bin_camera(fr, true, ca[q].cam)) return rc;
+      ca[q].mats = {nullptr, nullptr}; ca[q].rect = s.rect; ca[q].diff = s.tile_diff;
+      oa[q] = {s.tile_diff, fr->tile_offsets, fr->max_pairs, fr->status, s.counters, v0 + q == views - 1};
+      sa[q] = {s.rect, fr->tile_offsets, s.tile_len, fr->tile_prims, s.plane, s.tile_rect, s.counters, fr->status};
+    }
+    launch_corners<N>(geom, n, ca, oa, count, frs->tile_capacity, st);
+    launch_views<N>(k_bin_scatter<true, 8, N>, dim3((n + 63) / 64), dim3(256), 0, st, sa, count, n, ca[0].cam.ntx, geom,
+                    (float)(-2.0 * log((double)frs->threshold)));
   }
   return cuda_check(cudaGetLastError(), "bin");
 }

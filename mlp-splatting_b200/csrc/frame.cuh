@@ -147,6 +147,25 @@ inline cudaError_t launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 bloc
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(std::forward<Args>(args))...);
 }
 
+// A launch serves up to kViewsPerLaunch views of a batch, a row of CTAs each (blockIdx.y): launched view by view, the later waves of
+// a batch, a few microseconds of work per view, were mostly launches, and each view ended in a tail of its own (four 500k views of
+// 1200 x 680: 4,006 -> 3,720 us, three 200k views of 640 x 480: 1,830 -> 1,687).  Arguments travel by value, 300 bytes a view.
+constexpr int kViewsPerLaunch = 8;
+template <typename A, int V>
+struct Views { A v[V]; int count; };
+template <int V> __device__ __forceinline__ int view_of_cta() { return V == 1 ? 0 : (int)blockIdx.y; }
+
+// one launch for the views args[0 .. count)
+template <int V, typename A, typename... KArgs, typename... Args>
+inline cudaError_t launch_views(void (*kernel)(Views<A, V>, KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A* args,
+                                int count, const Args&... rest) {
+  Views<A, V> b = {};
+  b.count = count;
+  for (int v = 0; v < count; ++v) b.v[v] = args[v];
+  grid.y = (unsigned)count;
+  return launch_chained(kernel, grid, block, smem, st, b, rest...);
+}
+
 // Kernel classes for the launch counter and the optional per-class device timing.
 enum KernelClass { kKBin = 0, kKSort, kKHits, kKScan, kKFill, kKMlp, kKComposite, kKMisc, kNumKernelClasses };
 
@@ -224,9 +243,13 @@ int launch_bin(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, c
                bool pretest = false, const float* view_dev = nullptr, const float* proj_dev = nullptr);
 // the count pass adds rectangle corners (the corner array fits one CTA's shared memory: frames to about 3,500 x 3,500)
 bool bin_uses_corners(const mlpsp_frame* fr);
-// everything the fused path reads, in one launch (see k_frame_begin); prim_cnt null: the counts are another frame's
-int launch_frame_begin(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, const float* rays_raw, bool reset_status,
-                       int32_t* prim_cnt, cudaStream_t st);
+// everything the fused path reads of a frame or of a batch's views, in one launch for eight of them (see k_frame_begin)
+int launch_frame_begin(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scratch* ss, int views, const float* const* rays_raw,
+                       bool reset_status, cudaStream_t st);
+// launch_bin and launch_sort for the views of a batch that launch_frame_begin has prepared (bin_uses_corners, at least one
+// primitive, lists in scatter order), one launch for eight of them
+int launch_bin_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scratch* ss, int views, cudaStream_t st);
+int launch_sort_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scratch* ss, int views, cudaStream_t st);
 int launch_bin_mosaic(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, const int32_t* tile_view,
                       const float* views_host, int num_views, cudaStream_t st);
 int launch_bin_raycone(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, cudaStream_t st);

@@ -86,9 +86,11 @@ struct BeginArgs {
   int32_t* status;                                             // null: the caller has reset it
 };
 
-__global__ void __launch_bounds__(256) k_frame_begin(const BeginArgs a) {
+template <int V>
+__global__ void __launch_bounds__(256) k_frame_begin(const __grid_constant__ Views<BeginArgs, V> b) {
   chain_wait();
   chain_release();
+  const BeginArgs& a = b.v[view_of_cta<V>()];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t gid = (int64_t)blockIdx.x * 256 + threadIdx.x, gn = (int64_t)gridDim.x * 256;
   for (int64_t i = gid; i * 4 < a.cnt_words; i += gn) *reinterpret_cast<int4*>(a.prim_cnt + i * 4) = make_int4(0, 0, 0, 0);
@@ -167,8 +169,8 @@ __global__ void __launch_bounds__(256) k_frame_begin(const BeginArgs a) {
   }
 }
 
-int launch_frame_begin(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, const float* rays_raw, bool reset_status,
-                       int32_t* prim_cnt, cudaStream_t st) {
+static BeginArgs begin_args(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, const float* rays_raw, bool reset_status,
+                            int32_t* prim_cnt) {
   BeginArgs a;
   a.rays_o = fr->rays_o; a.rays_raw = rays_raw; a.rays_d = const_cast<float*>(fr->rays_d);
   a.W = fr->width; a.H = fr->height; a.ntx = (fr->width + 7) / 8; a.T = num_tiles(fr->width, fr->height, 8);
@@ -182,9 +184,25 @@ int launch_frame_begin(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scrat
   a.active0 = s.active[0]; a.counters = s.counters;
   a.prim_cnt = prim_cnt; a.cnt_words = prim_cnt ? 2 * (int64_t)prim_cnt_stride(sc->n) : 0;
   a.status = reset_status ? fr->status : nullptr;
-  LaunchScope scope(kKMisc, 1, st);
-  const int grid = std::max((a.T + 7) / 8, (int)std::min<int64_t>(sm_count() * 8, (a.cnt_words / 4 + 255) / 256));
-  return cuda_check(launch_chained(k_frame_begin, dim3(grid), dim3(256), 0, st, a), "frame_begin");
+  return a;
+}
+
+int launch_frame_begin(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scratch* ss, int views, const float* const* rays_raw,
+                       bool reset_status, cudaStream_t st) {
+  LaunchScope scope(kKMisc, (views + kViewsPerLaunch - 1) / kViewsPerLaunch, st);
+  cudaError_t e = cudaSuccess;
+  for (int v0 = 0; v0 < views && e == cudaSuccess; v0 += kViewsPerLaunch) {
+    BeginArgs a[kViewsPerLaunch];
+    const int count = std::min(kViewsPerLaunch, views - v0);
+    // the per-primitive counts are the first view's
+    for (int q = 0; q < count; ++q)
+      a[q] = begin_args(sc, frs + v0 + q, ss[v0 + q], rays_raw ? rays_raw[v0 + q] : nullptr, reset_status && v0 + q == 0,
+                        v0 + q == 0 ? ss[0].prim_cnt : nullptr);
+    const dim3 grid(std::max((a[0].T + 7) / 8, (int)std::min<int64_t>(sm_count() * 8, (a[0].cnt_words / 4 + 255) / 256)));
+    if (count == 1) e = launch_views<1>(k_frame_begin<1>, grid, dim3(256), 0, st, a, 1);
+    else e = launch_views<kViewsPerLaunch>(k_frame_begin<kViewsPerLaunch>, grid, dim3(256), 0, st, a, count);
+  }
+  return cuda_check(e, "frame_begin");
 }
 
 // --------------------------------------------------------------------------- hit pass ----
@@ -341,14 +359,6 @@ __device__ __forceinline__ void hit_chunk(const HitPixels& h, const float* __res
   }
 }
 
-// A launch serves up to kViewsPerLaunch views of a batch, a row of CTAs each (blockIdx.y): launched view by view, the later waves of
-// a batch, a few microseconds of work per view, were mostly launches, and each view ended in a tail of its own (four 500k views of
-// 1200 x 680: 4,006 -> 3,720 us, three 200k views of 640 x 480: 1,830 -> 1,687).  Arguments travel by value, 300 bytes a view.
-constexpr int kViewsPerLaunch = 8;
-template <typename A, int V>
-struct Views { A v[V]; int count; };
-template <int V> __device__ __forceinline__ int view_of_cta() { return V == 1 ? 0 : (int)blockIdx.y; }
-
 struct HitArgs {
   const float* rays_o; const float* rays_d; const float4* geom; int n;
   const int32_t* tile_offsets; const int32_t* tile_len; const int32_t* sorted_prims; int W, H, ntx;
@@ -429,16 +439,6 @@ __global__ void __launch_bounds__(32 * kHitWarps) k_hits(const __grid_constant__
   }
 }
 
-// one launch for the views args[0 .. count)
-template <int V, typename A, typename... KArgs>
-static cudaError_t launch_views(void (*kernel)(Views<A, V>, KArgs...), dim3 grid, dim3 block, cudaStream_t st, const A* args, int count, KArgs... rest) {
-  Views<A, V> b = {};
-  b.count = count;
-  for (int v = 0; v < count; ++v) b.v[v] = args[v];
-  grid.y = (unsigned)count;
-  return launch_chained(kernel, grid, block, 0, st, b, rest...);
-}
-
 static int launch_hits(const HitArgs* args, int views, bool ref_arith, int tiles, int sms, bool idle_tail, cudaStream_t st) {
   const HitArgs& a = args[0];
   const int parts = std::min((a.hi - a.lo + 31) / 32, kHitParts);
@@ -450,11 +450,11 @@ static int launch_hits(const HitArgs* args, int views, bool ref_arith, int tiles
   cudaError_t e = cudaSuccess;
   if (views == 1) {
     auto* kernel = ref_arith ? (loop ? k_hits<true, true, 1> : k_hits<true, false, 1>) : (loop ? k_hits<false, true, 1> : k_hits<false, false, 1>);
-    e = launch_views<1>(kernel, grid, block, st, args, 1, parts);
+    e = launch_views<1>(kernel, grid, block, 0, st, args, 1, parts);
   } else {
     constexpr int N = kViewsPerLaunch;
     auto* kernel = ref_arith ? (loop ? k_hits<true, true, N> : k_hits<true, false, N>) : (loop ? k_hits<false, true, N> : k_hits<false, false, N>);
-    e = launch_views<N>(kernel, grid, block, st, args, views, parts);
+    e = launch_views<N>(kernel, grid, block, 0, st, args, views, parts);
   }
   return cuda_check(e, "hits");
 }
@@ -812,10 +812,10 @@ static int launch_fill(FillArgs* args, int views, bool exact, bool ref_arith, in
   const dim3 grid((unsigned)std::min<int64_t>((units + wpb - 1) / wpb, idle_tail ? sms : sms * 32)), block(32 * wpb);
   cudaError_t e = cudaSuccess;
   if (views == 1) {
-    e = launch_views<1>(ref_arith ? k_fill<2, 1> : (exact ? k_fill<1, 1> : k_fill<0, 1>), grid, block, st, args, 1);
+    e = launch_views<1>(ref_arith ? k_fill<2, 1> : (exact ? k_fill<1, 1> : k_fill<0, 1>), grid, block, 0, st, args, 1);
   } else {
     constexpr int N = kViewsPerLaunch;
-    e = launch_views<N>(ref_arith ? k_fill<2, N> : (exact ? k_fill<1, N> : k_fill<0, N>), grid, block, st, args, views);
+    e = launch_views<N>(ref_arith ? k_fill<2, N> : (exact ? k_fill<1, N> : k_fill<0, N>), grid, block, 0, st, args, views);
   }
   return cuda_check(e, "fill");
 }
@@ -1525,7 +1525,7 @@ int launch_render_sorted(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scr
                                 s.rec_out, want_t ? s.rec_t : nullptr, s.px_state, s.px_depth, fr->rgb, fr->alpha, fr->depth_t, used32,
                                 want_feat ? s.rec_w : nullptr, keep ? s.rec_tr : nullptr, bg[0], bg[1], bg[2], has_bg,
                                 s.active[nxt], s.counters + kCtrActive0 + nxt, fr->status};
-      launch_views<1>(want_stats ? k_composite<true, 1> : k_composite<false, 1>, dim3(grid_comp), dim3(64), st, &ca, 1);
+      launch_views<1>(want_stats ? k_composite<true, 1> : k_composite<false, 1>, dim3(grid_comp), dim3(64), 0, st, &ca, 1);
     }
     lo = hi;
   }
@@ -1666,8 +1666,8 @@ int launch_render_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scr
                  s.pair_base, lead.rec_out, nullptr, s.px_state, s.px_depth, fr->rgb, fr->alpha, nullptr, nullptr, nullptr, nullptr,
                  bg[0], bg[1], bg[2], has_bg, s.active[nxt], s.counters + kCtrActive0 + nxt, f0->status};
         if (q + 1 < kViewsPerLaunch && v + 1 < V) continue;
-        if (q == 0) launch_views<1>(k_composite<false, 1>, dim3(grid_comp), dim3(64), st, ca, 1);
-        else launch_views<kViewsPerLaunch>(k_composite<false, kViewsPerLaunch>, dim3(grid_comp), dim3(64), st, ca, q + 1);
+        if (q == 0) launch_views<1>(k_composite<false, 1>, dim3(grid_comp), dim3(64), 0, st, ca, 1);
+        else launch_views<kViewsPerLaunch>(k_composite<false, kViewsPerLaunch>, dim3(grid_comp), dim3(64), 0, st, ca, q + 1);
       }
     }
     lo = hi;

@@ -270,12 +270,24 @@ __device__ __forceinline__ void sort_tiles_done() {
 
 // Short lists: one warp per tile, eight tiles per CTA.  Tiles with more than kWarpSortMax candidates are left to
 // k_sort_long, which gives each of them a CTA of its own.
-template <bool IDSORT>
-__global__ void __launch_bounds__(256, 6) k_sort_tiles(
-    const float* __restrict__ rays_o, const float* __restrict__ rays_d, const float4* __restrict__ geom, int n,
-    const int32_t* __restrict__ tile_offsets, const int32_t* tile_prims, int W, int H, int ts, int ntx, int T, int cap,
-    int32_t* __restrict__ sorted_prims, float* __restrict__ keys_out, int key_mode, int32_t* __restrict__ cursor,
-    const int32_t* __restrict__ list_len, int32_t* __restrict__ status) {
+// cursors: [0] of k_sort_long, [1] of k_sort_tiles
+struct SortArgs {
+  const float* rays_o; const float* rays_d; const int32_t* tile_offsets; const int32_t* tile_prims; int32_t* sorted_prims; float* keys_out;
+  int32_t* cursors; const int32_t* list_len; int32_t* status;
+};
+struct SortShape { int W, H, ts, ntx, T, key_mode; };
+
+template <bool IDSORT, int V>
+__global__ void __launch_bounds__(256, 6) k_sort_tiles(const __grid_constant__ Views<SortArgs, V> views, const float4* __restrict__ geom, int n,
+                                                       const SortShape shape, int cap) {
+  const SortArgs& a = views.v[view_of_cta<V>()];
+  const float* __restrict__ rays_o = a.rays_o; const float* __restrict__ rays_d = a.rays_d;
+  const int32_t* __restrict__ tile_offsets = a.tile_offsets; const int32_t* tile_prims = a.tile_prims;
+  int32_t* __restrict__ sorted_prims = a.sorted_prims; float* __restrict__ keys_out = a.keys_out;
+  int32_t* __restrict__ cursor = a.cursors + 1;
+  const int32_t* __restrict__ list_len = a.list_len;
+  int32_t* __restrict__ status = a.status;
+  const int W = shape.W, H = shape.H, ts = shape.ts, ntx = shape.ntx, T = shape.T, key_mode = shape.key_mode;
   __shared__ unsigned long long s_buf[8][kWarpSortMax];
   // Launched behind k_sort_long as its programmatic dependent WITHOUT waiting for it here: the two kernels sort
   // disjoint tiles and run side by side.  What this kernel reads (the binned lists, the status word) was complete
@@ -314,12 +326,17 @@ __global__ void __launch_bounds__(256, 6) k_sort_tiles(
 // the registers of the CTA's threads.  Launched before k_sort_tiles, which runs beside it.  Bound: issue slots; with the
 // network on the 64-bit composites both kernels took 79 us on the 100k frame, 117 of a 500k view and 136 of a 1M one at
 // 1920 x 1080, now 55, 75 and 98.
-template <int THREADS, int CAP, bool IDSORT>
-__global__ void __launch_bounds__(THREADS) k_sort_long(
-    const float* __restrict__ rays_o, const float* __restrict__ rays_d, const float4* __restrict__ geom, int n,
-    const int32_t* __restrict__ tile_offsets, const int32_t* tile_prims, int W, int H, int ts, int ntx,
-    int32_t* __restrict__ sorted_prims, float* __restrict__ keys_out, int key_mode, int T,
-    int32_t* __restrict__ cursor, const int32_t* __restrict__ list_len, const int32_t* __restrict__ status) {
+template <int THREADS, int CAP, bool IDSORT, int V>
+__global__ void __launch_bounds__(THREADS) k_sort_long(const __grid_constant__ Views<SortArgs, V> views, const float4* __restrict__ geom, int n,
+                                                       const SortShape shape) {
+  const SortArgs& a = views.v[view_of_cta<V>()];
+  const float* __restrict__ rays_o = a.rays_o; const float* __restrict__ rays_d = a.rays_d;
+  const int32_t* __restrict__ tile_offsets = a.tile_offsets; const int32_t* tile_prims = a.tile_prims;
+  int32_t* __restrict__ sorted_prims = a.sorted_prims; float* __restrict__ keys_out = a.keys_out;
+  int32_t* __restrict__ cursor = a.cursors;
+  const int32_t* __restrict__ list_len = a.list_len;
+  const int32_t* __restrict__ status = a.status;
+  const int W = shape.W, H = shape.H, ts = shape.ts, ntx = shape.ntx, T = shape.T, key_mode = shape.key_mode;
   __shared__ __align__(16) unsigned long long s_buf[CAP];
   __shared__ uint32_t s_key[CAP];
   __shared__ uint2 s_range[THREADS / 32];
@@ -382,35 +399,48 @@ __global__ void __launch_bounds__(THREADS) k_sort_long(
   }
 }
 
+template <bool IDSORT, int V>
+static void launch_sort_kernels(const mlpsp_scene* sc, const mlpsp_frame* fr, const SortArgs* args, int views, cudaStream_t st) {
+  const int T = num_tiles(fr->width, fr->height, fr->tile), ntx = (fr->width + fr->tile - 1) / fr->tile, sms = sm_count();
+  // k_sort_tiles runs beside k_sort_long, whose CTAs must all have started for that: they share the SMs between the views
+  const int grid = std::min((T + kTilesPerCta - 1) / kTilesPerCta, sms * 6);
+  const int grid_long = std::min(T, (sms * 6 + views - 1) / views);
+  // the reference kernels' arithmetic exists for the tile-centre key only (sort_key 0)
+  const int key_mode = fr->sort_key | ((fr->hit_arith == 1 && fr->sort_key == 0) ? 4 : 0);
+  const SortShape shape = {fr->width, fr->height, fr->tile, ntx, T, key_mode};
+  const float4* geom = (const float4*)sc->geom;
+  launch_views<V>(k_sort_long<256, kSortCap, IDSORT, V>, dim3(grid_long), dim3(256), 0, st, args, views, geom, sc->n, shape);
+  launch_views<V>(k_sort_tiles<IDSORT, V>, dim3(grid), dim3(256), 0, st, args, views, geom, sc->n, shape, kSortCap);
+}
+
+int launch_sort_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scratch* ss, int views, cudaStream_t st) {
+  constexpr int N = kViewsPerLaunch;
+  LaunchScope scope(kKSort, 2 * ((views + N - 1) / N), st);
+  for (int v0 = 0; v0 < views; v0 += N) {
+    SortArgs a[N];
+    const int count = std::min(N, views - v0);
+    for (int q = 0; q < count; ++q) {
+      const mlpsp_frame* fr = frs + v0 + q;
+      const Scratch& s = ss[v0 + q];
+      a[q] = {fr->rays_o, fr->rays_d, fr->tile_offsets, fr->tile_prims, fr->sorted_prims, nullptr, s.counters + kCtrScratch + 2, s.tile_len,
+              fr->status};
+    }
+    launch_sort_kernels<true, N>(sc, frs, a, count, st);
+  }
+  return cuda_check(cudaGetLastError(), "sort_tiles");
+}
+
 int launch_sort(const mlpsp_scene* sc, const mlpsp_frame* fr, float* keys_out, cudaStream_t st, bool unordered_input,
                 int32_t* cursors, const int32_t* list_len) {
-  const int T = num_tiles(fr->width, fr->height, fr->tile);
-  const int ntx = (fr->width + fr->tile - 1) / fr->tile;
   MLPSP_REQUIRE(fr->tile_capacity > 0 && fr->tile_capacity <= kSortCap, MLPSP_E_LIMIT,
                 "tile_capacity must be in [1, %d]", kSortCap);
   MLPSP_REQUIRE(cursors, MLPSP_E_ARG, "sort: scratch for the tile cursors missing");
-  const int sms = sm_count();
-  // tile cursors: [0] of k_sort_long, [1] of k_sort_tiles (a frame that k_frame_begin prepared starts with both at zero)
+  // a frame that k_frame_begin prepared starts with both cursors at zero
   if (!list_len) MLPSP_CUDA_OK(cudaMemsetAsync(cursors, 0, 8, st));
   LaunchScope scope(kKSort, 2, st);
-  const int grid = std::min((T + kTilesPerCta - 1) / kTilesPerCta, sms * 6);
-  const int grid_long = std::min(T, sms * 6);
-  const float4* geom = (const float4*)sc->geom;
-  // the reference kernels' arithmetic exists for the tile-centre key only (sort_key 0)
-  const int key_mode = fr->sort_key | ((fr->hit_arith == 1 && fr->sort_key == 0) ? 4 : 0);
-  if (unordered_input) {
-    launch_chained(k_sort_long<256, kSortCap, true>, dim3(grid_long), dim3(256), 0, st, fr->rays_o, fr->rays_d, geom, sc->n, fr->tile_offsets,
-                   fr->tile_prims, fr->width, fr->height, fr->tile, ntx, fr->sorted_prims, keys_out, key_mode, T, cursors, list_len, fr->status);
-    launch_chained(k_sort_tiles<true>, dim3(grid), dim3(256), 0, st, fr->rays_o, fr->rays_d, geom, sc->n, fr->tile_offsets, fr->tile_prims,
-                   fr->width, fr->height, fr->tile, ntx, T, kSortCap, fr->sorted_prims, keys_out, key_mode, cursors + 1, list_len,
-                   fr->status);
-  } else {
-    launch_chained(k_sort_long<256, kSortCap, false>, dim3(grid_long), dim3(256), 0, st, fr->rays_o, fr->rays_d, geom, sc->n, fr->tile_offsets,
-                   fr->tile_prims, fr->width, fr->height, fr->tile, ntx, fr->sorted_prims, keys_out, key_mode, T, cursors, list_len, fr->status);
-    launch_chained(k_sort_tiles<false>, dim3(grid), dim3(256), 0, st, fr->rays_o, fr->rays_d, geom, sc->n, fr->tile_offsets, fr->tile_prims,
-                   fr->width, fr->height, fr->tile, ntx, T, kSortCap, fr->sorted_prims, keys_out, key_mode, cursors + 1, list_len,
-                   fr->status);
-  }
+  const SortArgs a = {fr->rays_o, fr->rays_d, fr->tile_offsets, fr->tile_prims, fr->sorted_prims, keys_out, cursors, list_len, fr->status};
+  if (unordered_input) launch_sort_kernels<true, 1>(sc, fr, &a, 1, st);
+  else launch_sort_kernels<false, 1>(sc, fr, &a, 1, st);
   return cuda_check(cudaGetLastError(), "sort_tiles");
 }
 
