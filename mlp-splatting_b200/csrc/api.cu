@@ -279,7 +279,7 @@ static int render_frame(const mlpsp_scene* sc, const mlpsp_frame* fr, const floa
   rc = launch_bin(sc, fr, s, st, /*order_lists=*/false, pretest, view_dev, proj_dev);
   if (rc) return rc;
   rc = launch_sort(sc, fr, nullptr, st, /*unordered_input=*/true, s.counters + kCtrScratch + 2,
-                   pretest ? s.tile_len : nullptr);
+                   pretest ? &s : nullptr);
   if (rc) return rc;
   return render_sorted_checked(sc, fr, s, st, pretest);
 }
@@ -340,7 +340,7 @@ extern "C" int mlpsp_render_frames(const mlpsp_scene* sc, const mlpsp_frame* fra
     int rc = launch_bin(sc, fr, s, st, /*order_lists=*/false, pretest);
     if (rc) return rc;
     rc = launch_sort(sc, fr, nullptr, st, /*unordered_input=*/true, s.counters + kCtrScratch + 2,
-                     pretest ? s.tile_len : nullptr);
+                     pretest ? &s : nullptr);
     if (rc) return rc;
   }
   return launch_render_batch(sc, frames, ss.data(), num_frames, st, pretest);

@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(1024) k_bin_offsets(const __grid_constant__ Vi
 // two pairs each three quarters of the lanes idle through the ellipses (four 500k views: 272 us, with 32 205).
 struct ScatterArgs {
   const uint2* rect; const int32_t* tile_offsets; int32_t* tile_fill; int32_t* tile_prims; const FramePlane* plane;
-  const float4* tile_rect; const int32_t* counters; const int32_t* status;
+  const float4* tile_rect; int32_t* counters; int32_t* long_tiles; const int32_t* status;
 };
 template <bool PRETEST, int PPW, int V>
 __global__ void __launch_bounds__(256) k_bin_scatter(const __grid_constant__ Views<ScatterArgs, V> views, int n, int ntx,
@@ -385,6 +385,7 @@ __global__ void __launch_bounds__(256) k_bin_scatter(const __grid_constant__ Vie
     }
     const int slot = atomicAdd(tile_fill + t, 1);
     tile_prims[tile_offsets[t] + slot] = id;
+    if (PRETEST && slot == kWarpSortMax) a.long_tiles[atomicAdd(a.counters + kCtrLongTiles, 1)] = t;      // once per long tile
   });
 }
 
@@ -631,7 +632,7 @@ int launch_bin(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, c
                    fr->max_pairs, fr->status, s.counters);
   }
   if (n > 0) {
-    const ScatterArgs sa = {s.rect, fr->tile_offsets, fill, fr->tile_prims, s.plane, s.tile_rect, s.counters, fr->status};
+    const ScatterArgs sa = {s.rect, fr->tile_offsets, fill, fr->tile_prims, s.plane, s.tile_rect, s.counters, s.tile_fill, fr->status};
     if (pretest)
       launch_views<1>(k_bin_scatter<true, 8, 1>, dim3((n + 63) / 64), dim3(256), 0, st, &sa, 1, n, cam.ntx, geom,
                       (float)(-2.0 * log((double)fr->threshold)));
@@ -662,7 +663,7 @@ int launch_bin_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scratc
       if (const int rc = bin_camera(fr, true, ca[q].cam)) return rc;
       ca[q].mats = {nullptr, nullptr}; ca[q].rect = s.rect; ca[q].diff = s.tile_diff;
       oa[q] = {s.tile_diff, fr->tile_offsets, fr->max_pairs, fr->status, s.counters, v0 + q == views - 1};
-      sa[q] = {s.rect, fr->tile_offsets, s.tile_len, fr->tile_prims, s.plane, s.tile_rect, s.counters, fr->status};
+      sa[q] = {s.rect, fr->tile_offsets, s.tile_len, fr->tile_prims, s.plane, s.tile_rect, s.counters, s.tile_fill, fr->status};
     }
     launch_corners<N>(geom, n, ca, oa, count, frs->tile_capacity, st);
     launch_views<N>(k_bin_scatter<true, 8, N>, dim3((n + 63) / 64), dim3(256), 0, st, sa, count, n, ca[0].cam.ntx, geom,

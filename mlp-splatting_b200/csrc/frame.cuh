@@ -19,8 +19,9 @@ enum Counter {
   kCtrActive0 = 3,   // active tile count, list 0
   kCtrActive1 = 4,   // active tile count, list 1
   kCtrPairs = 5,     // total candidate pairs (binning)
-  kCtrScratch = 6,   // three words (record export, long-tile list of the sort)
+  kCtrScratch = 6,   // four words (record export, cursors of the sort)
   kCtrWaveRecords = 10, // records of the current wave
+  kCtrLongTiles = 11, // tiles on the sort's list of long ones
   kCtrWork = 12,     // evaluator work items of the current wave, and, as the upper half of the same 64-bit word,
   kCtrWorkSmall = 13, // small-group work items
   kNumCounters = 16
@@ -36,7 +37,7 @@ struct __align__(16) RecIn {
 struct Scratch {
   int32_t* tile_cnt;     // [T+1]
   int32_t* tile_diff;    // [(nty+1)*(ntx+1)] rectangle corners of the count pass (2-D difference array)
-  int32_t* tile_fill;    // [T]
+  int32_t* tile_fill;    // [T] pairs written per tile; in the fused path, which counts in tile_len, the list of long tiles
   uint2* rect;           // [n]  (x0 | x1<<16, y0 | y1<<16); x0 > x1 marks "culled"
   int32_t* scan_blk;     // block sums of the multi-block scans
   float4* px_state;      // [P] (C.r, C.g, C.b, transmittance)
@@ -254,10 +255,12 @@ int launch_bin_mosaic(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratc
                       const float* views_host, int num_views, cudaStream_t st);
 int launch_bin_raycone(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, cudaStream_t st);
 // cursors [2]: device scratch, the tile cursors of the two sort kernels
-// list_len (optional): candidates actually present at the front of every tile's span (pre-tested binning);
-// the rest of the span is filled with -1 in sorted_prims
+// prepared (optional): the scratch of a pre-tested binning, which knows the candidates actually present at the front of every
+// tile's span (the rest of the span is filled with -1 in sorted_prims) and lists the long tiles
 int launch_sort(const mlpsp_scene* sc, const mlpsp_frame* fr, float* keys_out, cudaStream_t st, bool unordered_input,
-                int32_t* cursors, const int32_t* list_len = nullptr);
+                int32_t* cursors, const Scratch* prepared = nullptr);
+// lists longer than this are sorted by a CTA
+constexpr int kWarpSortMax = 256;
 int launch_hit_masks(const mlpsp_scene* sc, const mlpsp_frame* fr, uint64_t* mask_geo, cudaStream_t st);
 // lists_refined: launch_frame_begin has prepared the frame and s.tile_len holds the traversal length of every tile
 int launch_render_sorted(const mlpsp_scene* sc, const mlpsp_frame* fr, const Scratch& s, cudaStream_t st,

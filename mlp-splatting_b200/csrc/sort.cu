@@ -51,9 +51,10 @@ __device__ __forceinline__ void write_sorted(const unsigned long long* buf, cons
 }
 
 constexpr int kTilesPerCta = 8;
-constexpr int kWarpSortMax = 256;
 constexpr int kLongDraw = 4;
+constexpr int kLongCtas = 6;            // CTAs of k_sort_long per SM
 constexpr int kFixPasses = 8;
+constexpr int kBucketMax = 32;          // candidates in one bucket of a list that is sorted by buckets
 
 // ---- warp-level bitonic sort in registers: lane l holds the elements r * 32 + l, r < PER ----
 // A compare-exchange at distance j >= 32 pairs two registers of the same lane; at distance j < 32 it pairs the same
@@ -270,10 +271,10 @@ __device__ __forceinline__ void sort_tiles_done() {
 
 // Short lists: one warp per tile, eight tiles per CTA.  Tiles with more than kWarpSortMax candidates are left to
 // k_sort_long, which gives each of them a CTA of its own.
-// cursors: [0] of k_sort_long, [1] of k_sort_tiles
+// cursors: [0] of k_sort_long, [1] of k_sort_tiles.  long_tiles, long_count: the tiles of k_sort_long, or null
 struct SortArgs {
   const float* rays_o; const float* rays_d; const int32_t* tile_offsets; const int32_t* tile_prims; int32_t* sorted_prims; float* keys_out;
-  int32_t* cursors; const int32_t* list_len; int32_t* status;
+  int32_t* cursors; const int32_t* list_len; const int32_t* long_tiles; const int32_t* long_count; int32_t* status;
 };
 struct SortShape { int W, H, ts, ntx, T, key_mode; };
 
@@ -322,12 +323,106 @@ __global__ void __launch_bounds__(256, 6) k_sort_tiles(const __grid_constant__ V
   }
 }
 
-// Long lists (more than kWarpSortMax candidates): one CTA per such tile, the same bitonic network with the elements in
-// the registers of the CTA's threads.  Launched before k_sort_tiles, which runs beside it.  Bound: issue slots; with the
-// network on the 64-bit composites both kernels took 79 us on the 100k frame, 117 of a 500k view and 136 of a 1M one at
-// 1920 x 1080, now 55, 75 and 98.
+// One tile's list (len <= PER * THREADS) sorted by the CTA and written out.  The keys' range is cut into CAP buckets: a
+// candidate draws its place in its bucket with one atomic in shared memory, a prefix over the buckets gives their starts, the
+// composites move there, and each one's place inside the bucket, of a handful, is the number of smaller ones.  A list
+// with more than kBucketMax candidates in one bucket (equal keys, an outlier that stretches the range) takes the network.
+// s_buf: CAP composites, s_bucket: CAP words, s_range: a word pair per warp.
+template <int PER, int THREADS, int CAP, bool IDSORT>
+__device__ __forceinline__ void sort_tile_by_cta(const float4* __restrict__ geom, int n, const int32_t* tile_prims,
+                                                 int32_t* __restrict__ sorted_prims, float* __restrict__ keys_out, int s, int len, int span,
+                                                 V3 o, V3 d, int key_mode, unsigned long long* s_buf, uint32_t* s_bucket, uint2* s_range) {
+  constexpr int OWN = CAP / THREADS;                  // buckets per thread in the prefix
+  static_assert(OWN % 4 == 0, "buckets are read four at a time");
+  const int tid = threadIdx.x, lane = tid & 31;
+  unsigned long long c[PER];
+  uint32_t kmin = 0xffffffffu, kmax = 0u;
+  for (int i = tid; i < CAP / 4; i += THREADS) reinterpret_cast<uint4*>(s_bucket)[i] = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+  for (int r = 0; r < PER; ++r) {
+    const int i = r * THREADS + tid;
+    c[r] = ~0ull;
+    if (i < len) {
+      c[r] = make_composite<IDSORT>(geom, n, tile_prims[s + i], i, o, d, key_mode);
+      const uint32_t key = (uint32_t)(c[r] >> 32);
+      kmin = min(kmin, key);
+      if (key != __float_as_uint(MLPSP_SENTINEL_KEY)) kmax = max(kmax, key);
+    }
+  }
+  kmin = __reduce_min_sync(0xffffffffu, kmin);
+  kmax = __reduce_max_sync(0xffffffffu, kmax);
+  if (lane == 0) s_range[tid >> 5] = make_uint2(kmin, kmax);
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < THREADS / 32; ++w) { kmin = min(kmin, s_range[w].x); kmax = max(kmax, s_range[w].y); }
+  // the map from keys to buckets is monotone: each of its operations is
+  const float scale = kmax > kmin ? (float)(CAP - 1) / (float)(kmax - kmin) : 0.f;
+  auto bucket_of = [&](unsigned long long v) { return (uint32_t)fminf((float)((uint32_t)(v >> 32) - kmin) * scale, (float)(CAP - 1)); };
+  uint32_t place[PER];                                // bucket, place in it
+#pragma unroll
+  for (int r = 0; r < PER; ++r) {
+    if (r * THREADS + tid >= len) continue;
+    const uint32_t b = bucket_of(c[r]);
+    place[r] = b << 16 | atomicAdd(s_bucket + b, 1u);
+  }
+  __syncthreads();
+  uint32_t own[OWN], sum = 0u, deepest = 0u;
+#pragma unroll
+  for (int j = 0; j < OWN; j += 4) {
+    const uint4 q = reinterpret_cast<const uint4*>(s_bucket)[(tid * OWN + j) >> 2];
+    own[j] = q.x; own[j + 1] = q.y; own[j + 2] = q.z; own[j + 3] = q.w;
+  }
+#pragma unroll
+  for (int j = 0; j < OWN; ++j) { deepest = max(deepest, own[j]); sum += own[j]; }
+  uint32_t upto = sum;
+#pragma unroll
+  for (int k = 1; k < 32; k <<= 1) {
+    const uint32_t u = __shfl_up_sync(0xffffffffu, upto, k);
+    if (lane >= k) upto += u;
+  }
+  if (lane == 31) s_range[tid >> 5].x = upto;         // (all have read the ranges before the barrier above)
+  if (__syncthreads_or(deepest > kBucketMax)) {
+#pragma unroll
+    for (int r = 0; r < PER; ++r) if (r * THREADS + tid < len) s_buf[r * THREADS + tid] = c[r];
+    __syncthreads();
+    cta_sort_composites<PER, THREADS>(s_buf, s_bucket, len, kmin, kmax);
+    write_sorted<IDSORT>(s_buf, tile_prims, sorted_prims, keys_out, s, len, span, tid, THREADS);
+    __syncthreads();
+    return;
+  }
+  uint32_t start = upto - sum;
+  for (int w = 0; w < (tid >> 5); ++w) start += s_range[w].x;
+#pragma unroll
+  for (int j = 0; j < OWN; j += 4) {
+    uint4 q;
+    q.x = start; start += own[j]; q.y = start; start += own[j + 1]; q.z = start; start += own[j + 2]; q.w = start; start += own[j + 3];
+    reinterpret_cast<uint4*>(s_bucket)[(tid * OWN + j) >> 2] = q;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < PER; ++r)
+    if (r * THREADS + tid < len) s_buf[s_bucket[place[r] >> 16] + (place[r] & 0xffffu)] = c[r];
+  __syncthreads();
+  for (int e = tid; e < span; e += THREADS) {
+    if (e >= len) { sorted_prims[s + e] = -1; continue; }
+    const unsigned long long v = s_buf[e];
+    const uint32_t b = bucket_of(v);
+    const int lo = (int)s_bucket[b], hi = b + 1 < CAP ? (int)s_bucket[b + 1] : len;
+    int at = s + lo;
+    for (int j = lo; j < hi; ++j) at += s_buf[j] < v ? 1 : 0;
+    sorted_prims[at] = IDSORT ? (int32_t)(uint32_t)v : tile_prims[s + (int)(uint32_t)v];
+    if (keys_out) keys_out[at] = __uint_as_float((uint32_t)(v >> 32));
+  }
+  __syncthreads();
+}
+
+// Long lists (more than kWarpSortMax candidates): one CTA per such tile.  Launched before k_sort_tiles, which runs beside it.
+// Bound: the gathers of the candidates' geometry and shared memory.  Both kernels on the 100k frame, a 500k view and four of
+// them in one batch: the bitonic network on every list, one CTA's registers filling an SM, 61, 77 and 311 us; five CTAs per SM
+// drawing from the list of long tiles 60, 72 and 279; buckets 55, 58 and 208; six CTAs per SM, with a few spilled registers
+// in the variant for the longest lists, 52, 58 and 198 (four: 55, 61, 217).
 template <int THREADS, int CAP, bool IDSORT, int V>
-__global__ void __launch_bounds__(THREADS) k_sort_long(const __grid_constant__ Views<SortArgs, V> views, const float4* __restrict__ geom, int n,
+__global__ void __launch_bounds__(THREADS, kLongCtas) k_sort_long(const __grid_constant__ Views<SortArgs, V> views, const float4* __restrict__ geom, int n,
                                                        const SortShape shape) {
   const SortArgs& a = views.v[view_of_cta<V>()];
   const float* __restrict__ rays_o = a.rays_o; const float* __restrict__ rays_d = a.rays_d;
@@ -338,7 +433,7 @@ __global__ void __launch_bounds__(THREADS) k_sort_long(const __grid_constant__ V
   const int32_t* __restrict__ status = a.status;
   const int W = shape.W, H = shape.H, ts = shape.ts, ntx = shape.ntx, T = shape.T, key_mode = shape.key_mode;
   __shared__ __align__(16) unsigned long long s_buf[CAP];
-  __shared__ uint32_t s_key[CAP];
+  __shared__ __align__(16) uint32_t s_bucket[CAP];
   __shared__ uint2 s_range[THREADS / 32];
   static_assert(CAP == 2048, "places of eleven bits");
   __shared__ int s_draw;
@@ -346,20 +441,20 @@ __global__ void __launch_bounds__(THREADS) k_sort_long(const __grid_constant__ V
   chain_wait();
   chain_release();
   if (status[MLPSP_ST_BITS] & MLPSP_ST_FATAL) return;
-  // CTAs draw tiles from a shared cursor: long lists cluster in the dense part of the image (on the
-  // 100,000-primitive bench frame 2,301 of 12,750 tiles hold more than 256 candidates), so a fixed deal leaves
-  // most CTAs idle behind the ones that met several.  A draw is kLongDraw tiles a band of the image apart, which do not
-  // cluster, and the next one is on its way meanwhile: most tiles are short, and a draw of each cost two round trips to
-  // memory (both sort kernels, 100k frame: 89 -> 79 us).
+  // CTAs draw tiles from a shared cursor.  The pre-tested binning lists the long ones as their fill passes the limit, the
+  // densest first, so that every draw is one sort and the last ones are short.  Without that list a draw is
+  // kLongDraw tiles a band of the image apart, since long lists cluster in its dense part.
   const int bands = (T + kLongDraw - 1) / kLongDraw;
+  const int32_t* __restrict__ long_tiles = a.long_tiles;
+  const int draws = long_tiles ? *a.long_count : bands, per_draw = long_tiles ? 1 : kLongDraw;
   int draw = 0;
   if (threadIdx.x == 0) draw = atomicAdd(cursor, 1);
   for (;;) {
     if (threadIdx.x == 0) { s_draw = draw; draw = atomicAdd(cursor, 1); }
     __syncthreads();
-    if (s_draw >= bands) return;
-    if (threadIdx.x < kLongDraw) {
-      const int tile = s_draw + threadIdx.x * bands;
+    if (s_draw >= draws) return;
+    if (threadIdx.x < per_draw) {
+      const int tile = long_tiles ? long_tiles[s_draw] : s_draw + threadIdx.x * bands;
       int4 e = make_int4(tile, 0, 0, 0);
       if (tile < T) {
         e.y = tile_offsets[tile];
@@ -369,32 +464,16 @@ __global__ void __launch_bounds__(THREADS) k_sort_long(const __grid_constant__ V
       s_list[threadIdx.x] = e;
     }
     __syncthreads();
-    for (int u = 0; u < kLongDraw; ++u) {
+    for (int u = 0; u < per_draw; ++u) {
     const int tile = s_list[u].x, s = s_list[u].y, span = s_list[u].z, len = s_list[u].w;
     if (len <= kWarpSortMax) continue;        // k_sort_tiles' (uniform over the CTA)
     const int tx = tile % ntx, ty = tile / ntx;
     const int cx = min(tx * ts + (ts >> 1), W - 1), cy = min(ty * ts + (ts >> 1), H - 1);
     const int64_t pc = (int64_t)cy * W + cx;
     const V3 o = load3(rays_o, pc), d = load3(rays_d, pc);
-    uint32_t kmin = 0xffffffffu, kmax = 0u;
-    for (int i = threadIdx.x; i < len; i += THREADS) {
-      const unsigned long long c = make_composite<IDSORT>(geom, n, tile_prims[s + i], i, o, d, key_mode);
-      s_buf[i] = c;
-      const uint32_t key = (uint32_t)(c >> 32);
-      kmin = min(kmin, key);
-      if (key != __float_as_uint(MLPSP_SENTINEL_KEY)) kmax = max(kmax, key);
-    }
-    kmin = __reduce_min_sync(0xffffffffu, kmin);
-    kmax = __reduce_max_sync(0xffffffffu, kmax);
-    if ((threadIdx.x & 31) == 0) s_range[threadIdx.x >> 5] = make_uint2(kmin, kmax);
-    __syncthreads();
-#pragma unroll
-    for (int w = 0; w < THREADS / 32; ++w) { kmin = min(kmin, s_range[w].x); kmax = max(kmax, s_range[w].y); }
-    if (len <= CAP / 4) cta_sort_composites<CAP / 4 / THREADS, THREADS>(s_buf, s_key, len, kmin, kmax);
-    else if (len <= CAP / 2) cta_sort_composites<CAP / 2 / THREADS, THREADS>(s_buf, s_key, len, kmin, kmax);
-    else cta_sort_composites<CAP / THREADS, THREADS>(s_buf, s_key, len, kmin, kmax);
-    write_sorted<IDSORT>(s_buf, tile_prims, sorted_prims, keys_out, s, len, span, threadIdx.x, THREADS);
-    __syncthreads();
+    if (len <= CAP / 4) sort_tile_by_cta<CAP / 4 / THREADS, THREADS, CAP, IDSORT>(geom, n, tile_prims, sorted_prims, keys_out, s, len, span, o, d, key_mode, s_buf, s_bucket, s_range);
+    else if (len <= CAP / 2) sort_tile_by_cta<CAP / 2 / THREADS, THREADS, CAP, IDSORT>(geom, n, tile_prims, sorted_prims, keys_out, s, len, span, o, d, key_mode, s_buf, s_bucket, s_range);
+    else sort_tile_by_cta<CAP / THREADS, THREADS, CAP, IDSORT>(geom, n, tile_prims, sorted_prims, keys_out, s, len, span, o, d, key_mode, s_buf, s_bucket, s_range);
     }
   }
 }
@@ -404,7 +483,7 @@ static void launch_sort_kernels(const mlpsp_scene* sc, const mlpsp_frame* fr, co
   const int T = num_tiles(fr->width, fr->height, fr->tile), ntx = (fr->width + fr->tile - 1) / fr->tile, sms = sm_count();
   // k_sort_tiles runs beside k_sort_long, whose CTAs must all have started for that: they share the SMs between the views
   const int grid = std::min((T + kTilesPerCta - 1) / kTilesPerCta, sms * 6);
-  const int grid_long = std::min(T, (sms * 6 + views - 1) / views);
+  const int grid_long = std::min(T, (sms * kLongCtas + views - 1) / views);
   // the reference kernels' arithmetic exists for the tile-centre key only (sort_key 0)
   const int key_mode = fr->sort_key | ((fr->hit_arith == 1 && fr->sort_key == 0) ? 4 : 0);
   const SortShape shape = {fr->width, fr->height, fr->tile, ntx, T, key_mode};
@@ -423,7 +502,7 @@ int launch_sort_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scrat
       const mlpsp_frame* fr = frs + v0 + q;
       const Scratch& s = ss[v0 + q];
       a[q] = {fr->rays_o, fr->rays_d, fr->tile_offsets, fr->tile_prims, fr->sorted_prims, nullptr, s.counters + kCtrScratch + 2, s.tile_len,
-              fr->status};
+              s.tile_fill, s.counters + kCtrLongTiles, fr->status};
     }
     launch_sort_kernels<true, N>(sc, frs, a, count, st);
   }
@@ -431,14 +510,16 @@ int launch_sort_batch(const mlpsp_scene* sc, const mlpsp_frame* frs, const Scrat
 }
 
 int launch_sort(const mlpsp_scene* sc, const mlpsp_frame* fr, float* keys_out, cudaStream_t st, bool unordered_input,
-                int32_t* cursors, const int32_t* list_len) {
+                int32_t* cursors, const Scratch* prepared) {
   MLPSP_REQUIRE(fr->tile_capacity > 0 && fr->tile_capacity <= kSortCap, MLPSP_E_LIMIT,
                 "tile_capacity must be in [1, %d]", kSortCap);
   MLPSP_REQUIRE(cursors, MLPSP_E_ARG, "sort: scratch for the tile cursors missing");
   // a frame that k_frame_begin prepared starts with both cursors at zero
-  if (!list_len) MLPSP_CUDA_OK(cudaMemsetAsync(cursors, 0, 8, st));
+  if (!prepared) MLPSP_CUDA_OK(cudaMemsetAsync(cursors, 0, 8, st));
   LaunchScope scope(kKSort, 2, st);
-  const SortArgs a = {fr->rays_o, fr->rays_d, fr->tile_offsets, fr->tile_prims, fr->sorted_prims, keys_out, cursors, list_len, fr->status};
+  const SortArgs a = {fr->rays_o, fr->rays_d, fr->tile_offsets, fr->tile_prims, fr->sorted_prims, keys_out, cursors,
+                      prepared ? prepared->tile_len : nullptr, prepared ? prepared->tile_fill : nullptr,
+                      prepared ? prepared->counters + kCtrLongTiles : nullptr, fr->status};
   if (unordered_input) launch_sort_kernels<true, 1>(sc, fr, &a, 1, st);
   else launch_sort_kernels<false, 1>(sc, fr, &a, 1, st);
   return cuda_check(cudaGetLastError(), "sort_tiles");

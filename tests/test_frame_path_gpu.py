@@ -320,3 +320,31 @@ def test_batches_at_the_edges_of_a_launch(precision, views, n, mu, W, H):
             assert torch.equal(rgb, rgb_w) and torch.equal(alpha, alpha_w)
         assert batch.last_stats.records == records and batch.last_stats.pairs == pairs      # the pairs are the last view's
     assert records > 0
+
+
+@pytest.mark.parametrize("n", [257, 512, 513, 1025, 2000])
+@pytest.mark.parametrize("depths", ["equal", "outlier", "pairs", "spread"])
+def test_long_lists_of_any_depths_sort_exactly(n, depths):
+    """Lists whose keys fall into one bucket (all equal, or one far candidate that stretches the range), into few, into all:
+    the order is the stable one, and the frame that lists its own long tiles draws what one with given lists draws."""
+    from mlp_splatting_b200.engine import FrameRenderer
+    from oracle import oracle as orc
+    W, H = 23, 17
+    scene, cam = small_case(n=n, W=W, H=H, mu=-1.0, seed=n)
+    p = scene["positions"]
+    if depths != "spread":
+        p[:] = p[:1] if depths != "pairs" else p[np.arange(n) // 2]
+        scene["quats"][:], scene["log_scales"][:] = scene["quats"][:1], scene["log_scales"][:1]
+    if depths == "outlier":
+        p[0] += 40.0 * cam["rays_d"].reshape(H, W, 3)[H // 2, W // 2]
+    ps, r = _packed(scene), FrameRenderer(W, H, device=DEV, tile_capacity=2048)
+    prims, offs = (t.clone() for t in r.bin(ps, cam["view"], cam["proj"], THR))
+    rd = orc.normalize_rows(cam["rays_d"])
+    got = r.sort(ps, _t(cam["rays_o"]), _t(rd), int(prims.numel()))
+    want = orc.sort_tiles(cam["rays_o"], rd, ps.geom.cpu().numpy()[:n], offs.cpu().numpy(), prims.cpu().numpy(), W, H, 8)
+    np.testing.assert_array_equal(got.cpu().numpy(), want)
+    assert int((offs[1:] - offs[:-1]).max()) > 256
+    kw = dict(view=cam["view"], proj=cam["proj"], precision=1)
+    given = [t.clone() for t in r.render(ps, _t(cam["rays_o"]), _t(cam["rays_d"]), THR, tile_lists=(prims, offs), **kw)]
+    own = r.render(ps, _t(cam["rays_o"]), _t(cam["rays_d"]), THR, **kw)
+    assert torch.equal(own[0], given[0]) and torch.equal(own[1], given[1]) and float(own[1].max()) > 0.0
