@@ -358,7 +358,8 @@ class Workload:
     def make_batches(self, per_view):
         """Multi-view workloads whose units are whole views render them in batches (mlpsp_render_frames): one
         evaluator launch per wave serves every view of a batch, so a primitive's weights are fetched once per wave
-        instead of once per wave and view.  per_view = [(pairs, records)] of the views rendered alone (sizing)."""
+        instead of once per wave and view.  per_view = [(pairs, records)] of the views rendered alone: a first size, since a
+        batch has windows of its own and evaluates other records in vain than its views alone (size_and_count)."""
         from mlp_splatting_b200.engine import ViewBatchRenderer
         self.batches = []
         cap = self.view_batch
@@ -405,11 +406,16 @@ class Workload:
                 per_view.append((self.r.last_stats.pairs, self.r.last_stats.records))
             self.make_batches(per_view)
             if self.batches:
-                # the batches evaluate the same records in fewer, fuller work items
+                # the batches composite the same records out of fewer, fuller work items; each is sized from its own frame
+                # (growing has doubled the arrays of one that needed more)
                 self.frame()
-                tot["work_total"] = sum(br.last_stats.work_total for br, _ in self.batches)
-                tot["work_small"] = sum(br.last_stats.work_small for br, _ in self.batches)
-                assert sum(br.last_stats.records for br, _ in self.batches) == tot["records"]
+                for br, _ in self.batches:
+                    br.lead.max_records = int(1.1 * br.last_stats.records) + 65536
+                self.frame()
+                used = tot["used"]
+                tot = {k: sum(getattr(br.last_stats, k) for br, _ in self.batches) for k in tot}
+                if tot["used"] != used:
+                    raise RuntimeError(f"{self.name}: the batches composite {tot['used']} records, their views alone {used}")
             stats.records, stats.used, stats.work_total, stats.work_small = tot["records"], tot["used"], tot["work_total"], tot["work_small"]
         self.stats = stats
         return stats
