@@ -288,6 +288,14 @@ def raise_for_status(bits: int, max_len: int, capacity: int, path_name: str):
         raise RenderError(f"{path_name}: a device-side wait gave up (status bit {L.BIT_TIMEOUT}); frame discarded")
 
 
+class _Windows:
+    """What one kind of frame has been found to need."""
+    __slots__ = ("default", "given", "idle_tail")
+
+    def __init__(self, default):
+        self.default, self.given, self.idle_tail = default, default, False
+
+
 class WaveSchedule:
     """The wave schedule a renderer gives its next frame (the image does not depend on it).
 
@@ -296,43 +304,73 @@ class WaveSchedule:
     plus a catch-all, which is expected to be idle, or, when hardly any tile came as far as the last of them, that one as the
     catch-all.  Hardly any: tiles times the longest list behind that wave at most 20,000 candidates, some 250,000 records that
     might be evaluated too early, which cost what the launches of an idle wave do (10 us; 425 tiles of 12,750 with lists up to
-    1,193 took 160 us more on the 100k frame)."""
+    1,193 took 160 us more on the 100k frame).
+
+    What was learned is kept by the kind of frame (layers, precision, whose lists, the library's windows), so that calls of two
+    kinds may alternate."""
+
+    KINDS = 16          # kinds of frames remembered; beyond that the one that was asked for longest ago is forgotten
 
     def __init__(self, width, height, capacity, views=1):
         self.size, self.capacity, self.views = (int(width), int(height)), int(capacity), int(views)
-        self.key = None
-        self.default = self.given = None
-        self.idle_tail = False
+        self._kinds = {}
+        self._calls = {}            # library's windows of earlier arguments
+        self._now = None
+        self._args = None
+
+    def _library(self, n, hidden, precision, caller_lists):
+        buf = (C.c_int32 * L.MAX_WAVES)()
+        count = L.load().mlpsp_wave_schedule(n, *self.size, hidden, precision, self.views, 1 if caller_lists else 0, self.capacity,
+                                             buf)
+        if count <= 0:
+            L.check(count or -1, "mlpsp_wave_schedule")
+        return list(buf[:count])
+
+    @property
+    def default(self):
+        """The library's schedule for the kind of frame that get() was asked for last."""
+        return self._now and self._now.default
+
+    @property
+    def given(self):
+        return self._now and self._now.given
 
     def get(self, n, hidden, precision, caller_lists=False):
         """(windows, whether the last one is expected to find no work) for a frame of this kind."""
-        key = (n, hidden, precision, caller_lists)
-        if key != self.key:
-            buf = (C.c_int32 * L.MAX_WAVES)()
-            count = L.load().mlpsp_wave_schedule(n, *self.size, hidden, precision, self.views, 1 if caller_lists else 0,
-                                                 self.capacity, buf)
-            if count <= 0:
-                L.check(count or -1, "mlpsp_wave_schedule")
-            self.key, self.default = key, list(buf[:count])
-            self.given, self.idle_tail = self.default, False
-        return self.given, self.idle_tail
+        args = (n, hidden, precision, caller_lists)
+        if args != self._args:
+            first = self._calls.get(args)
+            if first is None:
+                if len(self._calls) >= 4 * self.KINDS:
+                    self._calls.clear()
+                first = self._calls[args] = self._library(*args)
+            kind = (hidden, precision, caller_lists, *first)
+            e = self._kinds.pop(kind, None)
+            if e is None:
+                if len(self._kinds) >= self.KINDS:
+                    del self._kinds[next(iter(self._kinds))]
+                e = _Windows(first)
+            self._kinds[kind] = self._now = e       # (dictionaries keep their order: the last one is the youngest)
+            self._args = args
+        return self._now.given, self._now.idle_tail
 
     def adapt(self, words):
         """Takes the status words of the frame that was rendered with what get() returned last."""
-        g, used = self.given, int(words[L.ST_WAVES])
-        if g is None or used <= 0:
+        e, used = self._now, int(words[L.ST_WAVES])
+        if e is None or used <= 0:
             return
+        g, full = e.given, e.default
         behind = max(0, int(words[L.ST_MAX_TILE_LEN]) - sum(g[:used - 1]))
         few = int(words[L.ST_LAST_TILES]) * behind <= 20_000
         if used >= len(g):
-            self.given, self.idle_tail = (g if few else self.default), False
+            e.given, e.idle_tail = (g if few else full), False
             return
         merge = used >= 2 and few
         head = g[:used - 1] if merge else g[:used]
         if self.capacity - sum(head) > 2048:        # a window holds at most 2,048 candidates
-            self.given, self.idle_tail = self.default, False
+            e.given, e.idle_tail = full, False
         else:
-            self.given, self.idle_tail = head + [self.capacity], not merge
+            e.given, e.idle_tail = head + [self.capacity], not merge
 
 
 class FrameRenderer:

@@ -54,3 +54,36 @@ def test_a_frame_that_goes_further_brings_the_full_schedule_back():
     assert frame(2, 9_000) == (full, False)
     assert frame(len(full), 9_000) == (full, False)
     assert s.get(100_001, 32, 1) == (full, False)             # another scene starts over
+
+
+def _words(waves=1, evaluated=0, composited=0, kept=0, tiles=0, longest=1536):
+    w = np.zeros(L.STATUS_WORDS, np.int32)
+    w[L.ST_WAVES], w[L.ST_LAST_TILES], w[L.ST_MAX_TILE_LEN], w[L.ST_PAIRS_KEPT] = waves, tiles, longest, kept
+    for word, v in ((L.ST_RECORDS_LO, evaluated), (L.ST_USED_LO, composited)):
+        w[word:word + 2] = np.array([v], np.uint64).view(np.int32)
+    return w
+
+
+@pytest.mark.parametrize("kinds", [[(2_000, 32, 1, False), (2_000, 32, 1, True)],          # own and given lists
+                                   [(100_000, 32, 1, False), (100_000, 32, 0, False)],     # binary16 and its FP32 fallback
+                                   [(100_000, 32, 1, False), (3_000, 64, 1, False)]])      # two scenes
+def test_calls_of_two_kinds_keep_what_each_has_learned(kinds):
+    s = WaveSchedule(640, 480, 1536)
+    learned = []
+    for kind in kinds:
+        full = list(s.get(*kind)[0])
+        s.adapt(_words(waves=2, tiles=5_000))
+        assert s.get(*kind) == (full[:2] + [1536], True)
+        learned.append(s.get(*kind))
+    for _ in range(3):
+        for kind, want in zip(kinds, learned):
+            assert s.get(*kind) == want
+    # a few more primitives, the same windows: the same kind
+    assert s.get(kinds[-1][0] + 3, *kinds[-1][1:]) == learned[-1]
+
+
+def test_the_number_of_kinds_is_bounded():
+    s = WaveSchedule(640, 480, 1536)
+    for n in range(1_000, 400_000, 700):
+        s.get(n, 32, n % 2)
+    assert len(s._kinds) <= s.KINDS and len(s._calls) <= 4 * s.KINDS
