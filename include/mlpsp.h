@@ -170,6 +170,12 @@ int mlpsp_abi_version(void);
  * it, or grow it when a frame reports MLPSP_ST_RECORD_OVERFLOW). */
 int mlpsp_wave_schedule(int32_t n, int32_t width, int32_t height, int32_t hidden, int32_t precision, int32_t views,
                         int32_t caller_lists, int32_t tile_capacity, int32_t* wave_len);
+/* The same with what a caller may know beyond the sizes: list_pairs, the candidates of all tiles in lists it gives (-1: the
+ * library's own lists), and finer, how often the windows are to be halved (a schedule of one window: first the several
+ * windows of its size) because frames of this kind evaluated far more records than they composited
+ * (MLPSP_ST_RECORDS_LO, MLPSP_ST_USED_LO).  The windows stop at 32 candidates. */
+int mlpsp_wave_schedule_finer(int32_t n, int32_t width, int32_t height, int32_t hidden, int32_t precision, int32_t views,
+                              int64_t list_pairs, int32_t tile_capacity, int32_t finer, int32_t* wave_len);
 /* sizeof(mlpsp_scene), sizeof(mlpsp_frame) as compiled, for bindings that mirror the structs */
 int mlpsp_struct_sizes(int32_t* scene_bytes, int32_t* frame_bytes);
 

@@ -67,6 +67,7 @@ _SIGS = {
     "mlpsp_last_error": (C.c_char_p, []),
     "mlpsp_abi_version": (C.c_int, []),
     "mlpsp_wave_schedule": (C.c_int, [C.c_int32] * 8 + [C.POINTER(C.c_int32)]),
+    "mlpsp_wave_schedule_finer": (C.c_int, [C.c_int32] * 6 + [C.c_int64, C.c_int32, C.c_int32, C.POINTER(C.c_int32)]),
     "mlpsp_struct_sizes": (C.c_int, [C.POINTER(C.c_int32), C.POINTER(C.c_int32)]),
     "mlpsp_pack_geometry": (C.c_int, [_fp, _fp, _fp, C.c_int32, _fp, _fp]),
     "mlpsp_normalize_rows": (C.c_int, [_fp, _fp, C.c_int64, C.c_int32, _fp]),

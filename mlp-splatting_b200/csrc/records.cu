@@ -1348,20 +1348,33 @@ static const int kDefaultWaves[] = {32, 32, 64, 128, 256, INT_MAX};
 //    161,500      16,150  344 -> 322   731 -> 707      808,640      26,954    859 -> 825   2,565 -> 2,400
 // a record frame of 320 x 240 and 20,000 primitives 394 -> 296; four views at 1200 x 680 of 500,000 4,486 -> 4,251, at
 // 1920 x 1080 of 1,000,000 64-wide ones 10,867 -> 10,408.
-extern "C" int mlpsp_wave_schedule(int32_t n, int32_t width, int32_t height, int32_t hidden, int32_t precision, int32_t views,
-                                   int32_t caller_lists, int32_t tile_capacity, int32_t* wave_len) {
-  MLPSP_REQUIRE(n >= 0 && width > 0 && height > 0 && views > 0 && tile_capacity > 0 && wave_len, MLPSP_E_ARG,
-                "mlpsp_wave_schedule: bad argument");
+//
+// How many of a window's candidates hit a pixel is not known here, since it follows from the splats' sizes.  The rows above
+// are scenes with 6 to 12 composited records per pixel; where splats are large or stand in deep stacks, windows of this length
+// evaluate several times what is composited.  So a caller that reads the counts of a frame can ask for windows halved `finer`
+// times (one window: first the several of its size), and lists that the caller gave tell their mean length beforehand: one
+// window is for up to 100,000 candidates (FP32 30,000) in all.  Evaluated and composited records per pixel, us, of one
+// window and of 104, 104, 208, 416, rest, binary16:
+//     200 x 150: own lists  24 / 11  178 | 185,  49 / 13  209 | 183,  67 / 16  216 | 167,  95 / 23  262 | 205
+//     200 x 150: given, of 68,000 24 / 11  188 | 219,  105,000 49 / 13  215 | 215,  117,000 67 / 16  234 | 205,  135,000 269 | 220
+//     128 x 96:  own lists   6 / 6  107 | 128,  23 / 12  125 | 144,  33 / 15  128 | 137
+// and of 72, 72, 144, 288, rest against 32, 32, 64, 128, 256, rest at 320 x 240 in FP32: 33 / 18  584 | 517,  43 / 23  733 | 608.
+static int wave_schedule(int32_t n, int32_t width, int32_t height, int32_t hidden, int32_t precision, int32_t views,
+                         int64_t list_pairs, int32_t tile_capacity, int32_t finer, int32_t* wave_len) {
   const double P = (double)width * height, r = std::min(9.0, P / std::max(n, 1));
   const bool f32 = precision == MLPSP_PRECISION_F32;
   int count = 0;
-  if (P <= (f32 ? 16000.0 : 30000.0) && tile_capacity <= kWinMax) {
-    wave_len[count++] = tile_capacity;
-    return count;
+  if (P <= (f32 ? 16000.0 : 30000.0) && list_pairs <= (f32 ? 30000 : 100000) && tile_capacity <= kWinMax) {
+    if (finer == 0) {
+      wave_len[count++] = tile_capacity;
+      return count;
+    }
+    --finer;
   }
   double a = (f32 ? 65.0 : 70.0) * std::cbrt(318000.0 / P) * std::pow(4.0 / r, r >= 4.0 ? 0.4 : (views > 1 ? 0.8 : 0.55));
-  if (caller_lists) a *= 2.0;
+  if (list_pairs >= 0) a *= 2.0;
   if (views > 1) a *= std::max(1.0, hidden / 32.0);
+  a = std::ldexp(a, -std::min(finer, 16));
   const int first = (int)std::min(512.0, std::max(32.0, 8.0 * std::floor(a / 8.0 + 0.5)));
   const bool halves = P >= (f32 ? 250000.0 : 450000.0);
   int lo = 0;
@@ -1377,6 +1390,20 @@ extern "C" int mlpsp_wave_schedule(int32_t n, int32_t width, int32_t height, int
   add(4 * first);
   while (lo < tile_capacity && count < MLPSP_MAX_WAVES) add(kWinMax);
   return count;
+}
+
+extern "C" int mlpsp_wave_schedule(int32_t n, int32_t width, int32_t height, int32_t hidden, int32_t precision, int32_t views,
+                                   int32_t caller_lists, int32_t tile_capacity, int32_t* wave_len) {
+  MLPSP_REQUIRE(n >= 0 && width > 0 && height > 0 && views > 0 && tile_capacity > 0 && wave_len, MLPSP_E_ARG,
+                "mlpsp_wave_schedule: bad argument");
+  return wave_schedule(n, width, height, hidden, precision, views, caller_lists ? 0 : -1, tile_capacity, 0, wave_len);
+}
+
+extern "C" int mlpsp_wave_schedule_finer(int32_t n, int32_t width, int32_t height, int32_t hidden, int32_t precision, int32_t views,
+                                         int64_t list_pairs, int32_t tile_capacity, int32_t finer, int32_t* wave_len) {
+  MLPSP_REQUIRE(n >= 0 && width > 0 && height > 0 && views > 0 && list_pairs >= -1 && tile_capacity > 0 && finer >= 0 && wave_len,
+                MLPSP_E_ARG, "mlpsp_wave_schedule_finer: bad argument");
+  return wave_schedule(n, width, height, hidden, precision, views, list_pairs, tile_capacity, finer, wave_len);
 }
 
 int launch_hit_masks(const mlpsp_scene* sc, const mlpsp_frame* fr, uint64_t* mask_geo, cudaStream_t st) {

@@ -289,11 +289,12 @@ def raise_for_status(bits: int, max_len: int, capacity: int, path_name: str):
 
 
 class _Windows:
-    """What one kind of frame has been found to need."""
-    __slots__ = ("default", "given", "idle_tail")
+    """What one kind of frame has been found to need: how often its windows are halved, and what the next frame is given."""
+    __slots__ = ("levels", "seen", "level", "given", "idle_tail", "waste")
 
-    def __init__(self, default):
-        self.default, self.given, self.idle_tail = default, default, False
+    def __init__(self, first, waste):
+        self.levels, self.level, self.given, self.idle_tail, self.waste = [first], 0, first, False, waste
+        self.seen = [None]          # records evaluated in vain by the first frame at each level
 
 
 class WaveSchedule:
@@ -305,6 +306,12 @@ class WaveSchedule:
     catch-all.  Hardly any: tiles times the longest list behind that wave at most 20,000 candidates, some 250,000 records that
     might be evaluated too early, which cost what the launches of an idle wave do (10 us; 425 tiles of 12,750 with lists up to
     1,193 took 160 us more on the 100k frame).
+
+    The size of the work does not tell how deep the splats overlap.  Where a frame evaluated more than 1.6 times the records
+    that it composited, and so many in vain that they cost more than the launches of another wave (800,000, in FP32 300,000, of
+    32-wide layers), the next one has windows of half the length.  Longer ones come back once twice as many in vain would be
+    far below that, and no more than half of what the first frame with these windows had.  (At the library's own windows 100k and 500k frames stand at 1.2 to 1.45, frames of few large
+    splats at 1.8 to 4: 1,500 of 0.14 on 200 x 150 pixels 262 us in one window and 205 in several.)
 
     What was learned is kept by the kind of frame (layers, precision, whose lists, the library's windows), so that calls of two
     kinds may alternate."""
@@ -318,50 +325,77 @@ class WaveSchedule:
         self._now = None
         self._args = None
 
-    def _library(self, n, hidden, precision, caller_lists):
+    def _library(self, n, hidden, precision, list_pairs, finer):
         buf = (C.c_int32 * L.MAX_WAVES)()
-        count = L.load().mlpsp_wave_schedule(n, *self.size, hidden, precision, self.views, 1 if caller_lists else 0, self.capacity,
-                                             buf)
+        count = L.load().mlpsp_wave_schedule_finer(n, *self.size, hidden, precision, self.views, list_pairs, self.capacity, finer,
+                                                   buf)
         if count <= 0:
-            L.check(count or -1, "mlpsp_wave_schedule")
+            L.check(count or -1, "mlpsp_wave_schedule_finer")
         return list(buf[:count])
 
     @property
     def default(self):
-        """The library's schedule for the kind of frame that get() was asked for last."""
-        return self._now and self._now.default
+        """The library's schedule, at the present length of its windows, for the kind of frame that get() was asked for last."""
+        return self._now and self._now.levels[self._now.level]
 
     @property
     def given(self):
         return self._now and self._now.given
 
-    def get(self, n, hidden, precision, caller_lists=False):
-        """(windows, whether the last one is expected to find no work) for a frame of this kind."""
-        args = (n, hidden, precision, caller_lists)
+    def get(self, n, hidden, precision, caller_lists=False, list_pairs=0):
+        """(windows, whether the last one is expected to find no work) for a frame of this kind; list_pairs: candidates in
+        the caller's lists."""
+        args = (n, hidden, precision, int(list_pairs) if caller_lists else -1)
         if args != self._args:
             first = self._calls.get(args)
             if first is None:
                 if len(self._calls) >= 4 * self.KINDS:
                     self._calls.clear()
-                first = self._calls[args] = self._library(*args)
+                first = self._calls[args] = self._library(*args, 0)
             kind = (hidden, precision, caller_lists, *first)
             e = self._kinds.pop(kind, None)
             if e is None:
                 if len(self._kinds) >= self.KINDS:
                     del self._kinds[next(iter(self._kinds))]
-                e = _Windows(first)
+                e = _Windows(first, (300_000 if precision == L.PRECISION_F32 else 800_000) * 32 // max(hidden, 32))
             self._kinds[kind] = self._now = e       # (dictionaries keep their order: the last one is the youngest)
             self._args = args
         return self._now.given, self._now.idle_tail
 
+    def _resize(self, e, w):
+        """Shorter or longer windows from the records that the last frame evaluated and composited; True if they changed."""
+        used = w[L.ST_USED_LO] & 0xffffffff | w[L.ST_USED_LO + 1] << 32
+        vain = (w[L.ST_RECORDS_LO] & 0xffffffff | w[L.ST_RECORDS_LO + 1] << 32) - used
+        if e.seen[e.level] is None:
+            e.seen[e.level] = vain
+        if vain > e.waste and vain > 0.6 * used:
+            if e.level + 1 == len(e.levels):
+                e.levels.append(self._library(*self._args, e.level + 1))
+                e.seen.append(None)
+            if e.levels[e.level + 1] == e.levels[e.level]:
+                return False
+            e.level += 1
+            e.seen[e.level] = None
+        elif e.level and vain <= max(0.4 * e.waste, 0.2 * used) and 2 * vain <= e.seen[e.level]:
+            if len(e.levels[e.level - 1]) == 1:
+                # one window evaluates every hit: no more than the lists' candidates times their tiles' pixels
+                if 64 * (w[L.ST_PAIRS_KEPT] or w[L.ST_PAIRS]) - used > e.waste:
+                    return False
+            e.level -= 1
+        else:
+            return False
+        e.given, e.idle_tail = e.levels[e.level], False
+        return True
+
     def adapt(self, words):
         """Takes the status words of the frame that was rendered with what get() returned last."""
-        e, used = self._now, int(words[L.ST_WAVES])
-        if e is None or used <= 0:
+        e, w = self._now, words.tolist()
+        used = w[L.ST_WAVES]
+        if e is None or used <= 0 or self._resize(e, w):
             return
-        g, full = e.given, e.default
-        behind = max(0, int(words[L.ST_MAX_TILE_LEN]) - sum(g[:used - 1]))
-        few = int(words[L.ST_LAST_TILES]) * behind <= 20_000
+        g, full = e.given, e.levels[e.level]
+        behind = max(0, w[L.ST_MAX_TILE_LEN] - sum(g[:used - 1]))
+        few = w[L.ST_LAST_TILES] * behind <= 20_000
         if used >= len(g):
             e.given, e.idle_tail = (g if few else full), False
             return
@@ -632,7 +666,8 @@ class FrameRenderer:
                                                           self.capacity, scene.n, L.ptr(self.status), st),
                             "mlpsp_validate_tile_lists")
                 if auto:
-                    waves, idle_tail = self._waves.get(scene.n, scene.hidden, precision, tile_lists is not None)
+                    waves, idle_tail = self._waves.get(scene.n, scene.hidden, precision, tile_lists is not None,
+                                                       tile_lists[0].numel() if tile_lists is not None else 0)
                 f = self._frame(scene, rays_o, rd, threshold, precision, view, proj, bg, want_depth, want_mask_used, waves,
                                 want_feat=want_feat, keep_records=keep_records, sort_key=sort_key, tile_rows=tile_rows,
                                 tile_pretest=tile_pretest, prim_stats=prim_stats, tail_hint=idle_tail,

@@ -348,3 +348,20 @@ def test_long_lists_of_any_depths_sort_exactly(n, depths):
     given = [t.clone() for t in r.render(ps, _t(cam["rays_o"]), _t(cam["rays_d"]), THR, tile_lists=(prims, offs), **kw)]
     own = r.render(ps, _t(cam["rays_o"]), _t(cam["rays_d"]), THR, **kw)
     assert torch.equal(own[0], given[0]) and torch.equal(own[1], given[1]) and float(own[1].max()) > 0.0
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_deep_stacks_of_large_splats_get_shorter_windows_and_the_same_image(precision):
+    """1,500 splats of 0.14 on 200 x 150 pixels: several times as many hits as a pixel composites before it is opaque."""
+    from mlp_splatting_b200.engine import FrameRenderer
+    scene, cam = small_case(n=1_500, W=200, H=150, mu=-2.0, seed=7)
+    ps, ro, rd = _packed(scene), _t(cam["rays_o"]), _t(cam["rays_d"])
+    kw = dict(view=cam["view"], proj=cam["proj"], precision=precision)
+    want = [t.clone() for t in FrameRenderer(200, 150, device=DEV).render(ps, ro, rd, THR, waves=[16] * 7 + [1536], **kw)]
+    r = FrameRenderer(200, 150, device=DEV)
+    evaluated = []
+    for _ in range(6):
+        rgb, alpha = r.render(ps, ro, rd, THR, **kw)
+        assert torch.equal(rgb, want[0]) and torch.equal(alpha, want[1])
+        evaluated.append(r.last_stats.records)
+    assert evaluated[-1] < 0.8 * evaluated[0] and r.last_stats.used <= evaluated[-1]

@@ -87,3 +87,56 @@ def test_the_number_of_kinds_is_bounded():
     for n in range(1_000, 400_000, 700):
         s.get(n, 32, n % 2)
     assert len(s._kinds) <= s.KINDS and len(s._calls) <= 4 * s.KINDS
+
+
+@pytest.mark.parametrize("precision, vain", [(1, 1_500_000), (0, 400_000)])
+def test_deep_overlap_gets_shorter_windows_and_gives_them_back(precision, vain):
+    s = WaveSchedule(140, 100, 1536)
+    one = list(s.get(3_000, 32, precision)[0])
+    assert one == [1536]
+    s.adapt(_words(evaluated=200_000 + vain, composited=200_000, kept=30_000))
+    several = list(s.get(3_000, 32, precision)[0])
+    assert len(several) > 1 and several[0] < 512 and sum(several) >= 1536
+    sizes = [several[0]]
+    for _ in range(8):              # and shorter yet while that is not enough, down to 32
+        s.adapt(_words(waves=2, evaluated=200_000 + vain, composited=200_000, kept=30_000))
+        given, _ = s.get(3_000, 32, precision)
+        assert sum(given) >= 1536 and 1536 - sum(given[:-1]) <= 2048
+        sizes.append(s.default[0])
+    assert sizes[-1] == 32 and all(b <= a for a, b in zip(sizes, sizes[1:]))
+    for _ in range(8):              # little in vain: longer again, but not one window while the lists could fill it
+        s.adapt(_words(waves=2, evaluated=210_000, composited=200_000, kept=30_000))
+    assert s.default == several
+    s.adapt(_words(waves=2, evaluated=210_000, composited=200_000, kept=7_000))
+    assert s.get(3_000, 32, precision) == (one, False)
+
+
+def test_windows_that_help_are_kept():
+    s = WaveSchedule(200, 150, 1536)
+    assert s.get(1_500, 32, 1)[0] == [1536]
+    vain = {0: 2_100_000, 1: 900_000, 2: 290_000}       # by how often the windows were halved: each is a third of the last
+    seen = []
+    for _ in range(12):
+        level = s._now.level
+        seen.append(level)
+        s.adapt(_words(waves=3, evaluated=700_000 + vain[level], composited=700_000, kept=60_000))
+    assert seen == [0, 1] + [2] * 10
+
+
+def test_ordinary_ratios_leave_the_windows_alone():
+    s = WaveSchedule(1200, 680, 1536)
+    full = list(s.get(100_000, 32, 1)[0])
+    s.adapt(_words(waves=len(full), evaluated=11_300_000, composited=7_800_000, tiles=9_000))       # 3.5 M in vain, 1.45 times
+    assert s.get(100_000, 32, 1) == (full, False)
+    small = WaveSchedule(128, 96, 1536)
+    assert small.get(500, 32, 1) == ([1536], False)
+    small.adapt(_words(evaluated=400_000, composited=187_000))      # 2.1 times, but few: another wave costs more
+    assert small.get(500, 32, 1) == ([1536], False)
+
+
+@pytest.mark.parametrize("precision, few, many", [(1, 100_000, 100_001), (0, 30_000, 30_001)])
+def test_one_window_is_not_for_long_given_lists(precision, few, many):
+    s = WaveSchedule(140, 100, 2048)
+    assert s.get(3_000, 32, precision, True, few)[0] == [2048]
+    assert len(s.get(3_000, 32, precision, True, many)[0]) > 1
+    assert s.get(3_000, 32, precision)[0] == [2048]
