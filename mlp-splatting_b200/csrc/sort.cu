@@ -1,9 +1,9 @@
 // Per-tile depth sort: key = t* of the tile-centre ray against each candidate
 // (scannet/cuda/np_tile_kernels.cu:483-518), stable ascending order (1914-1990).
 // Keys are positive floats (or the 1e30 sentinel), so their bit patterns order like the values and the
-// sort runs on the raw bits of the 64-bit composite (key bits, tie-break): a bitonic network in registers over 32-bit
-// words that stand for the composites, whose order it then corrects (see cta_sort_composites).  Lists of up to 256
-// candidates are sorted by one warp (eight tiles per CTA), longer lists by a whole CTA.
+// sort runs on the raw bits of the 64-bit composite (key bits, tie-break).  Lists of up to 256 candidates are sorted by one
+// warp (eight tiles per CTA), a bitonic network in registers over 32-bit words that stand for the composites, whose order
+// it then corrects; longer lists by a whole CTA, through buckets of their keys.
 #include "frame.cuh"
 
 namespace mlpsp {
@@ -54,7 +54,7 @@ constexpr int kTilesPerCta = 8;
 constexpr int kLongDraw = 4;
 constexpr int kLongCtas = 6;            // CTAs of k_sort_long per SM
 constexpr int kFixPasses = 8;
-constexpr int kBucketMax = 32;          // candidates in one bucket of a list that is sorted by buckets
+constexpr int kBucketMax = 128;         // candidates in one bucket of a list that is sorted by buckets
 
 // ---- warp-level bitonic sort in registers: lane l holds the elements r * 32 + l, r < PER ----
 // A compare-exchange at distance j >= 32 pairs two registers of the same lane; at distance j < 32 it pairs the same
@@ -100,105 +100,48 @@ __device__ __forceinline__ void warp_bitonic_regs(T (&v)[PER], int lane) {
   }
 }
 
-// ---- CTA-level bitonic sort, PER elements per thread in registers: thread t holds the elements t * PER + r ----
-// Distances below PER stay inside a thread, distances below 32 * PER pair two lanes of a warp (shuffles); only the
-// remaining distances (6 of the 45 stages of a 512-element sort, 10 of 55 at 1,024) cross warps and go through
-// shared memory between two CTA barriers.  buf: N elements of shared memory that nobody else uses meanwhile.
-template <int PER, int THREADS, typename T>
-__device__ __forceinline__ void cta_bitonic_hybrid(T (&v)[PER], T* buf) {
-  constexpr int N = PER * THREADS;
-  const int tid = threadIdx.x;
-#pragma unroll
-  for (int k = 2; k <= N; k <<= 1) {
-#pragma unroll
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      if (j < PER) {
-#pragma unroll
-        for (int r = 0; r < PER; ++r) {
-          if ((r & j) == 0) {
-            const bool up = ((tid * PER + r) & k) == 0;
-            const T mn = min(v[r], v[r | j]), mx = max(v[r], v[r | j]);
-            v[r] = up ? mn : mx;
-            v[r | j] = up ? mx : mn;
-          }
-        }
-      } else if (j < 32 * PER) {
-        const int jl = j / PER;
-#pragma unroll
-        for (int r = 0; r < PER; ++r) {
-          const T a = v[r], b = shfl_xor_any(a, jl);
-          const bool up = ((tid * PER + r) & k) == 0;
-          const bool keep_min = ((tid & jl) == 0) == up;
-          v[r] = keep_min ? min(a, b) : max(a, b);
-        }
-      } else {
-#pragma unroll
-        for (int r = 0; r < PER; ++r) buf[tid * PER + r] = v[r];
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < PER; ++r) {
-          const int e = tid * PER + r;
-          const T a = v[r], b = buf[e ^ j];
-          const bool keep_min = ((e & j) == 0) == ((e & k) == 0);
-          v[r] = keep_min ? min(a, b) : max(a, b);
-        }
-        __syncthreads();
+// The CTA sorts s_buf[0 .. len) by a bitonic network in shared memory, two of its stages (distances j and j / 2) per pass: the
+// way of lists whose keys crowd into few buckets.  Loops and not an unrolled network in registers, so that it adds neither
+// registers nor code to the kernel around it.  In passes at distances up to 64 a warp's exchanges stay among the same
+// 128 elements, and only the warp has to keep step.
+template <int THREADS>
+__device__ __forceinline__ void cta_bitonic_shared(unsigned long long* s_buf, int len) {
+  int n = 128;
+  while (n < len) n <<= 1;
+  for (int e = len + (int)threadIdx.x; e < n; e += THREADS) s_buf[e] = ~0ull;
+  __syncthreads();
+  auto exchange = [](unsigned long long& x, unsigned long long& y, bool up) {
+    const unsigned long long lo = min(x, y), hi = max(x, y);
+    x = up ? lo : hi;
+    y = up ? hi : lo;
+  };
+#pragma unroll 1
+  for (int k = 2; k <= n; k <<= 1) {
+#pragma unroll 1
+    for (int j = k >> 1; j > 0; j >>= 2) {
+      const int q = max(j >> 1, 1);
+#pragma unroll 1
+      for (int i = threadIdx.x; i < n / 4; i += THREADS) {
+        unsigned long long* p = s_buf + ((i & ~(q - 1)) << 2 | (i & (q - 1)));
+        const int e = (int)(p - s_buf);
+        unsigned long long v0 = p[0], v1 = p[q], v2 = p[2 * q], v3 = p[3 * q];
+        const bool up = (e & k) == 0;
+        if (j > 1) { exchange(v0, v2, up); exchange(v1, v3, up); }
+        exchange(v0, v1, up);
+        exchange(v2, v3, ((e + 2 * q) & k) == 0);
+        p[0] = v0; p[q] = v1; p[2 * q] = v2; p[3 * q] = v3;
       }
+      if (max(j, j >> 2 ? j >> 2 : k) > 64) __syncthreads();
+      else __syncwarp();
     }
   }
-}
-
-// The CTA sorts s_buf[0 .. len), len <= PER * THREADS, composites (key bits << 32 | tie-break).  The network runs on 32-bit
-// words -- the key's distance from the list's smallest, cut to 21 bits, and the element's place -- which costs a third of
-// the instructions of 64-bit ones; the composites then move once, and neighbours that the cut has left out of order are
-// exchanged.  Lists with long runs of equal keys (more than kFixPasses exchanges deep) fall back on the 64-bit network.
-// s_key: PER * THREADS words.  kmin, kmax: the list's smallest and largest key bits, sentinels apart.
-template <int PER, int THREADS>
-__device__ __forceinline__ void cta_sort_composites(unsigned long long* s_buf, uint32_t* s_key, int len, uint32_t kmin, uint32_t kmax) {
-  constexpr int N = PER * THREADS;
-  const int tid = threadIdx.x;
-  const uint32_t range = kmax >= kmin ? kmax - kmin : 0u;
-  const int cut = max(0, 11 - __clz((int)range));            // bits of the distance beyond 21
-  uint32_t v[PER];
-#pragma unroll
-  for (int r = 0; r < PER; ++r) {
-    const int e = tid * PER + r;
-    const uint32_t key = e < len ? (uint32_t)(s_buf[e] >> 32) : 0u;
-    v[r] = e < len ? (min((key - kmin) >> cut, 0x1fffffu) << 11) | (uint32_t)e : 0xffffffffu;
-  }
-  cta_bitonic_hybrid<PER, THREADS>(v, s_key);
-  unsigned long long c[PER];
-#pragma unroll
-  for (int r = 0; r < PER; ++r) c[r] = tid * PER + r < len ? s_buf[v[r] & 2047u] : ~0ull;
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < PER; ++r) s_buf[tid * PER + r] = c[r];
-  __syncthreads();
-  for (int pass = 0;; ++pass) {
-    bool wrong = false;
-    for (int e = tid; e < len - 1; e += THREADS) wrong = wrong || s_buf[e] > s_buf[e + 1];
-    if (!__syncthreads_or(wrong)) return;
-    if (pass == kFixPasses) break;
-    for (int parity = 0; parity < 2; ++parity) {
-      for (int e = 2 * tid + parity; e < len - 1; e += 2 * THREADS) {
-        const unsigned long long a = s_buf[e], b = s_buf[e + 1];
-        if (a > b) { s_buf[e] = b; s_buf[e + 1] = a; }
-      }
-      __syncthreads();
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < PER; ++r) c[r] = s_buf[tid * PER + r];
-  __syncthreads();
-  cta_bitonic_hybrid<PER, THREADS>(c, s_buf);
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < PER; ++r) s_buf[tid * PER + r] = c[r];
-  __syncthreads();
 }
 
 // One tile's list (len <= PER * 32) sorted by one warp in registers and written out; buf: 256 composites of shared memory.
-// As cta_sort_composites, with 24 bits of the key's distance and a place of eight.
+// The network runs on 32-bit words -- the key's distance from the list's smallest, cut to 24 bits, and the element's place --
+// which costs a third of the instructions of 64-bit ones; the composites then move once, and neighbours that the cut has left
+// out of order are exchanged.  Lists with long runs of equal keys (more than kFixPasses exchanges deep) fall back on the
+// 64-bit network.
 template <int PER, bool FROM_SCATTER>
 __device__ __forceinline__ void sort_tile_in_registers(const float4* __restrict__ geom, int n, const int32_t* tile_prims,
                                                        int32_t* __restrict__ sorted_prims, float* __restrict__ keys_out,
@@ -326,7 +269,9 @@ __global__ void __launch_bounds__(256, 6) k_sort_tiles(const __grid_constant__ V
 // One tile's list (len <= PER * THREADS) sorted by the CTA and written out.  The keys' range is cut into CAP buckets: a
 // candidate draws its place in its bucket with one atomic in shared memory, a prefix over the buckets gives their starts, the
 // composites move there, and each one's place inside the bucket, of a handful, is the number of smaller ones.  A list
-// with more than kBucketMax candidates in one bucket (equal keys, an outlier that stretches the range) takes the network.
+// with more than kBucketMax candidates in one bucket (an outlier that stretches the range of many equal keys) takes the
+// network.  (A place costs a read per candidate of the bucket, the network some 36 passes over all: lists of a thin wall with
+// another behind it, sort of a 400,000-primitive view, network beyond 32 in a bucket 141 us, beyond 64, 128, 200: 102, 101, 100.)
 // s_buf: CAP composites, s_bucket: CAP words, s_range: a word pair per warp.
 template <int PER, int THREADS, int CAP, bool IDSORT>
 __device__ __forceinline__ void sort_tile_by_cta(const float4* __restrict__ geom, int n, const int32_t* tile_prims,
@@ -355,25 +300,31 @@ __device__ __forceinline__ void sort_tile_by_cta(const float4* __restrict__ geom
   __syncthreads();
 #pragma unroll
   for (int w = 0; w < THREADS / 32; ++w) { kmin = min(kmin, s_range[w].x); kmax = max(kmax, s_range[w].y); }
-  // the map from keys to buckets is monotone: each of its operations is
-  const float scale = kmax > kmin ? (float)(CAP - 1) / (float)(kmax - kmin) : 0.f;
-  auto bucket_of = [&](unsigned long long v) { return (uint32_t)fminf((float)((uint32_t)(v >> 32) - kmin) * scale, (float)(CAP - 1)); };
-  uint32_t place[PER];                                // bucket, place in it
+  // the map from composites to buckets is monotone: each of its operations is.  Where all keys but sentinels are equal (lists
+  // for per-pixel ordering), the tie-breaks take the keys' place, and sentinels the last bucket
+  const bool equal = kmax <= kmin;
+  const float scale = (float)(CAP - 1) / (float)(equal ? (IDSORT ? n : len) : (int)(kmax - kmin));
+  auto bucket_of = [&](unsigned long long v) {
+    const uint32_t key = (uint32_t)(v >> 32);
+    const float x = equal ? (key == kmin ? (float)(uint32_t)v : (float)CAP * 4294967296.f) : (float)(key - kmin);
+    return (uint32_t)fminf(x * scale, (float)(CAP - 1));
+  };
+  uint32_t place[(PER + 3) / 4] = {};                 // in its bucket, a byte each (deeper buckets take the network)
+  static_assert(kBucketMax < 255, "places of a byte");
 #pragma unroll
-  for (int r = 0; r < PER; ++r) {
-    if (r * THREADS + tid >= len) continue;
-    const uint32_t b = bucket_of(c[r]);
-    place[r] = b << 16 | atomicAdd(s_bucket + b, 1u);
-  }
+  for (int r = 0; r < PER; ++r)
+    if (r * THREADS + tid < len)
+      place[r >> 2] |= min(atomicAdd(s_bucket + bucket_of(c[r]), 1u), 255u) << (r & 3) * 8;
   __syncthreads();
-  uint32_t own[OWN], sum = 0u, deepest = 0u;
+  uint32_t sum = 0u, deepest = 0u;
+  uint4* own_s = reinterpret_cast<uint4*>(s_bucket) + tid * (OWN / 4);
+  uint4 own[OWN / 4];
 #pragma unroll
-  for (int j = 0; j < OWN; j += 4) {
-    const uint4 q = reinterpret_cast<const uint4*>(s_bucket)[(tid * OWN + j) >> 2];
-    own[j] = q.x; own[j + 1] = q.y; own[j + 2] = q.z; own[j + 3] = q.w;
+  for (int j = 0; j < OWN / 4; ++j) {
+    const uint4 q = own[j] = own_s[j];
+    deepest = max(max(max(deepest, q.x), q.y), max(q.z, q.w));
+    sum += q.x + q.y + q.z + q.w;
   }
-#pragma unroll
-  for (int j = 0; j < OWN; ++j) { deepest = max(deepest, own[j]); sum += own[j]; }
   uint32_t upto = sum;
 #pragma unroll
   for (int k = 1; k < 32; k <<= 1) {
@@ -384,8 +335,7 @@ __device__ __forceinline__ void sort_tile_by_cta(const float4* __restrict__ geom
   if (__syncthreads_or(deepest > kBucketMax)) {
 #pragma unroll
     for (int r = 0; r < PER; ++r) if (r * THREADS + tid < len) s_buf[r * THREADS + tid] = c[r];
-    __syncthreads();
-    cta_sort_composites<PER, THREADS>(s_buf, s_bucket, len, kmin, kmax);
+    cta_bitonic_shared<THREADS>(s_buf, len);
     write_sorted<IDSORT>(s_buf, tile_prims, sorted_prims, keys_out, s, len, span, tid, THREADS);
     __syncthreads();
     return;
@@ -393,15 +343,15 @@ __device__ __forceinline__ void sort_tile_by_cta(const float4* __restrict__ geom
   uint32_t start = upto - sum;
   for (int w = 0; w < (tid >> 5); ++w) start += s_range[w].x;
 #pragma unroll
-  for (int j = 0; j < OWN; j += 4) {
-    uint4 q;
-    q.x = start; start += own[j]; q.y = start; start += own[j + 1]; q.z = start; start += own[j + 2]; q.w = start; start += own[j + 3];
-    reinterpret_cast<uint4*>(s_bucket)[(tid * OWN + j) >> 2] = q;
+  for (int j = 0; j < OWN / 4; ++j) {
+    const uint4 q = own[j];
+    own_s[j] = make_uint4(start, start + q.x, start + q.x + q.y, start + q.x + q.y + q.z);
+    start += q.x + q.y + q.z + q.w;
   }
   __syncthreads();
 #pragma unroll
   for (int r = 0; r < PER; ++r)
-    if (r * THREADS + tid < len) s_buf[s_bucket[place[r] >> 16] + (place[r] & 0xffffu)] = c[r];
+    if (r * THREADS + tid < len) s_buf[s_bucket[bucket_of(c[r])] + (place[r >> 2] >> (r & 3) * 8 & 0xffu)] = c[r];
   __syncthreads();
   for (int e = tid; e < span; e += THREADS) {
     if (e >= len) { sorted_prims[s + e] = -1; continue; }
@@ -418,9 +368,10 @@ __device__ __forceinline__ void sort_tile_by_cta(const float4* __restrict__ geom
 
 // Long lists (more than kWarpSortMax candidates): one CTA per such tile.  Launched before k_sort_tiles, which runs beside it.
 // Bound: the gathers of the candidates' geometry and shared memory.  Both kernels on the 100k frame, a 500k view and four of
-// them in one batch: the bitonic network on every list, one CTA's registers filling an SM, 61, 77 and 311 us; five CTAs per SM
-// drawing from the list of long tiles 60, 72 and 279; buckets 55, 58 and 208; six CTAs per SM, with a few spilled registers
-// in the variant for the longest lists, 52, 58 and 198 (four: 55, 61, 217).
+// them in one batch: the bitonic network in registers on every list, 64 registers a thread, 61, 77 and 311 us; five CTAs per SM
+// drawing from the list of long tiles 60, 72 and 279; buckets 55, 58 and 208; six CTAs per SM (40 registers, of which the
+// network in registers, as the way of crowded lists, spilled 380 bytes) 52, 58 and 198; that network in shared memory, by
+// loops (spills 40 bytes), 52, 56 and 196.  Given lists, 3,456 of 12,750 longer than 256: 112 -> 88, all keys equal 175 -> 63.
 template <int THREADS, int CAP, bool IDSORT, int V>
 __global__ void __launch_bounds__(THREADS, kLongCtas) k_sort_long(const __grid_constant__ Views<SortArgs, V> views, const float4* __restrict__ geom, int n,
                                                        const SortShape shape) {

@@ -365,3 +365,42 @@ def test_deep_stacks_of_large_splats_get_shorter_windows_and_the_same_image(prec
         assert torch.equal(rgb, want[0]) and torch.equal(alpha, want[1])
         evaluated.append(r.last_stats.records)
     assert evaluated[-1] < 0.8 * evaluated[0] and r.last_stats.used <= evaluated[-1]
+
+
+@pytest.mark.parametrize("n", [257, 520, 1500])
+@pytest.mark.parametrize("kind", ["few behind", "many behind", "all behind", "wall", "thick wall"])
+def test_long_lists_of_crowded_keys_sort_exactly(n, kind):
+    """Keys that crowd into few buckets.  Behind the camera: equal keys sorted by their tie-breaks, and the largest key there is,
+    which fits one bucket, does not, or is all that there is.  Walls: up to 128 in a bucket, and beyond."""
+    from mlp_splatting_b200.engine import FrameRenderer
+    from oracle import oracle as orc
+    W, H = 23, 17
+    scene, cam = small_case(n=n, W=W, H=H, mu=-1.0, seed=n)
+    rng = np.random.default_rng(n)
+    rd = orc.normalize_rows(cam["rays_d"])
+    d = rd.reshape(H, W, 3)[H // 2, W // 2]
+    p, eye = scene["positions"], cam["rays_o"][0]
+    order = rng.permutation(n)
+    if "behind" in kind:
+        p[:] = p[:1]
+        scene["quats"][:], scene["log_scales"][:] = scene["quats"][:1], scene["log_scales"][:1]
+        m = {"few": 60, "many": n // 2, "all": n}[kind.split()[0]]
+        p[order[:m]] = eye - 2.0 * d
+    else:
+        step = 2e-3 if kind == "wall" else 2e-5
+        depth = 2.0 + step * rng.permutation(n).astype(np.float32) / n
+        depth[order[: n // 8]] += 6.0
+        p[:] = eye + depth[:, None] * d
+        scene["quats"][:] = scene["quats"][:1]
+        scene["log_scales"][:] = -1.0
+    ps, r = _packed(scene), FrameRenderer(W, H, device=DEV, tile_capacity=2048)
+    prims = np.tile(rng.permutation(n).astype(np.int32), r.T)           # every tile lists every primitive
+    offs = (np.arange(r.T + 1) * n).astype(np.int32)
+    r.tile_prims[: prims.size].copy_(_t(prims))
+    r.tile_offsets.copy_(_t(offs))
+    got, keys = r.sort(ps, _t(cam["rays_o"]), _t(rd), prims.size, want_keys=True)
+    want, want_keys = orc.sort_tiles(cam["rays_o"], rd, ps.geom.cpu().numpy()[:n], offs, prims, W, H, 8, want_keys=True)
+    np.testing.assert_array_equal(got.cpu().numpy(), want)
+    np.testing.assert_array_equal(keys.cpu().numpy(), want_keys)
+    behind = int((want_keys[:n] == np.float32(1e30)).sum())
+    assert behind == (m if "behind" in kind else 0)
