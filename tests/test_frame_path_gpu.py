@@ -404,3 +404,51 @@ def test_long_lists_of_crowded_keys_sort_exactly(n, kind):
     np.testing.assert_array_equal(keys.cpu().numpy(), want_keys)
     behind = int((want_keys[:n] == np.float32(1e30)).sum())
     assert behind == (m if "behind" in kind else 0)
+
+
+@pytest.mark.parametrize("hidden", [32, 64])
+@pytest.mark.parametrize("small_groups", [False, True])
+def test_overflow_of_layer_two_alone_falls_back_to_fp32(hidden, small_groups):
+    """Weights and first activations within binary16, second ones beyond it: only the evaluator's outputs show it.  Once in
+    the evaluator of full blocks, once where every work item is a small group."""
+    from mlp_splatting_b200.engine import FrameRenderer
+    n, W, H, mu = (6_000, 64, 48, -4.6) if small_groups else (300, 64, 48, -3.0)
+    scene, cam = small_case(n=n, W=W, H=H, mu=mu, hidden=hidden)
+    ro, rd, kw = _t(cam["rays_o"]), _t(cam["rays_d"]), dict(view=cam["view"], proj=cam["proj"])
+    r = FrameRenderer(W, H, device=DEV)
+    r.render(_packed(scene), ro, rd, THR, precision=1, **kw)
+    work = r.last_stats
+    assert r.f32_fallbacks == 0 and work.work_total > 0 and (work.work_small == work.work_total) == small_groups
+    scene["b1"][:] = 1.0
+    scene["W1"][:] *= 0.1
+    scene["W2"][:, 0, :] = 3.0e4
+    ps = _packed(scene)
+    assert ps.has_f16
+    rgb = r.render(ps, ro, rd, THR, precision=1, **kw)[0].clone()
+    assert r.f32_fallbacks == 1
+    assert torch.isfinite(rgb).all() and torch.equal(rgb, r.render(ps, ro, rd, THR, precision=0, **kw)[0])
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_batch_on_an_image_beyond_the_corner_array(precision):
+    """More rows of tiles than one CTA's corner array: the views of a batch are binned and sorted one by one, and the binning
+    lists the tiles with long lists."""
+    from mlp_splatting_b200 import synthetic
+    from mlp_splatting_b200.engine import FrameRenderer, ViewBatchRenderer
+    W, H, views = 24, 8 * 1025, 3
+    scene = synthetic.make_scene(900, 5, mu=-1.6)
+    ps = _packed(scene)
+    cams = [synthetic.make_camera(W, H, azimuth_deg=31.0 * v) for v in range(views)]
+    ros, rds = [_t(c["rays_o"]) for c in cams], [_t(c["rays_d"]) for c in cams]
+    vs, prs = [c["view"] for c in cams], [c["proj"] for c in cams]
+    single, want = FrameRenderer(W, H, device=DEV, tile_capacity=2048), []
+    for v in range(views):
+        rgb, alpha = single.render(ps, ros[v], rds[v], THR, view=vs[v], proj=prs[v], precision=precision, tile_pretest=False)
+        want.append((rgb.clone(), alpha.clone()))
+        assert 256 < single.last_stats.max_tile_len
+    batch = ViewBatchRenderer(W, H, views, device=DEV, tile_capacity=2048)
+    for _ in range(2):
+        got = batch.render(ps, ros, rds, THR, vs, prs, precision=precision)
+        assert batch.last_stats.pairs_kept > 0
+        for (rgb, alpha), (rgb_w, alpha_w) in zip(got, want):
+            assert torch.equal(rgb, rgb_w) and torch.equal(alpha, alpha_w) and float(alpha.max()) > 0.1

@@ -126,3 +126,32 @@ def test_weight_gradients_refuse_offsets_that_leave_the_records(dtype):
         with pytest.raises(ValueError, match="CSR offsets"):
             run(off, rows)
     assert all(torch.equal(a, b) for a, b in zip(run(offsets, R), want))          # the next call starts clean
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("shifted", [("W1",), ("W2",), ("W1", "b1", "W2", "b2", "W3", "b3")])
+def test_weight_gradients_of_weights_at_any_alignment(dtype, shifted):
+    """Masters whose first element lies four bytes beyond a 16-byte boundary (a slice of one flat parameter, say): the same
+    values through four-byte loads, hence the same bits."""
+    from mlp_splatting_b200.primitive_csr import PrimitiveCSR
+    from mlp_splatting_b200.primitive_gemm import grouped_weight_gradients
+    counts = [0, 1, 63, 200, 128, 700]
+    n, R = len(counts), sum(counts)
+    g = torch.Generator(device=DEV)
+    g.manual_seed(8)
+    rnd = lambda *s: torch.randn(s, generator=g, device=DEV)
+    w = dict(W1=rnd(n, 32, 72) * 0.2, b1=rnd(n, 32) * 0.1, W2=rnd(n, 32, 32) * 0.2, b2=rnd(n, 32) * 0.1, W3=rnd(n, 4, 32) * 0.2,
+             b3=rnd(n, 4) * 0.1)
+    moved = {}
+    for k, t in w.items():
+        flat = torch.empty(t.numel() + 1, device=DEV)
+        moved[k] = flat[1:].view(t.shape).copy_(t) if k in shifted else t
+        assert moved[k].data_ptr() % 16 == (4 if k in shifted else 0) and moved[k].is_contiguous()
+    freq = torch.tensor(2.0 ** np.arange(6) * np.pi, device=DEV, dtype=torch.float32)
+    att = torch.exp(-0.5 * freq ** 2 * 1e-4)
+    offsets = torch.tensor(np.concatenate(([0], np.cumsum(counts))), device=DEV)
+    csr = PrimitiveCSR(offsets, torch.arange(R, device=DEV), rnd(R, 6), rnd(R, 4) * 1e-3, None)
+    want = grouped_weight_gradients(csr, freq, att, list(w.values()), dtype=dtype)
+    got = grouped_weight_gradients(csr, freq, att, list(moved.values()), dtype=dtype)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b) and float(b.abs().max()) > 0
