@@ -360,11 +360,11 @@ __device__ __forceinline__ TilePix tile_pixel(int tile, int k, int ntx, int W, i
   return r;
 }
 
-// Output activations (np_tile_kernels.cu:75-83); values, not decisions, so hardware exp is fine.
 // The warp's number in its CTA, as a value the compiler knows to be the same in all lanes: what is computed from it (work units,
 // descriptors, addresses) then takes one scalar instruction instead of a vector one.  All lanes must call it.
 __device__ __forceinline__ int warp_of_cta() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
 
+// Output activations (np_tile_kernels.cu:75-83); values, not decisions, so hardware exp is fine.
 __device__ __forceinline__ float sigmoid_fast(float x) { return __fdividef(1.0f, 1.0f + __expf(-x)); }
 __device__ __forceinline__ float softplus_fast(float x) {
   // log(1 + e) on the hardware logarithm: within 1e-7 absolute of log1p over [-20, 20], far below what the

@@ -26,7 +26,8 @@
 // masks the adjoint chain does not depend on the forward one, D1 rides with layer 1 and dW1 with layer 2, three round trips per
 // block; the last one (dW2, dW3) overlaps the next block's encoding, a finished segment's gradients leave and the next block's
 // records and weights arrive while layer 1 runs.  5.5 M records of 15,000 primitives, 35,000 more without records: 598 us with
-// dW1 in the last round trip, the gradients written between two blocks and weights loaded a row per lane, 546 so.  (Two threads per record, 256 per CTA: 840, by spills, and 855 with two CTAs per SM.)
+// dW1 in the last round trip, the gradients written between two blocks and weights loaded a row per lane, 546 so.  (Two threads
+// per record, 256 per CTA: 840, by spills, and 855 with two CTAs per SM.)
 #include "frame.cuh"
 #include "tc.cuh"
 #include "vjp.cuh"
