@@ -677,8 +677,8 @@ def main():
     ap.add_argument("--other-workloads-multi", action="store_true",
                     help="also run the other workloads' short measurements when several ranks are used")
     ap.add_argument("--e2e-depth", type=int, default=8,
-                    help="frames in flight in the end-to-end arm (measured on one B200: 2 -> 731, 3 -> 867, 4 -> 899, "
-                         "6 -> 971, 8 -> 984, 12 -> 990 frames/s)")
+                    help="frames in flight in the end-to-end arm (measured on one B200: 2 -> 1,203, 3 -> 1,503, 4 -> 1,563, "
+                         "6 -> 1,571, 8 -> 1,530, 12 -> 1,529 frames/s)")
     ap.add_argument("--view-batch", type=int, default=16,
                     help="views of a multi-view workload rendered per call (0 or 1: view by view, as the reference does)")
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])

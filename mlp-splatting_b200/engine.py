@@ -310,8 +310,9 @@ class WaveSchedule:
     The size of the work does not tell how deep the splats overlap.  Where a frame evaluated more than 1.6 times the records
     that it composited, and so many in vain that they cost more than the launches of another wave (800,000, in FP32 300,000, of
     32-wide layers), the next one has windows of half the length.  Longer ones come back once twice as many in vain would be
-    far below that, and no more than half of what the first frame with these windows had.  (At the library's own windows 100k and 500k frames stand at 1.2 to 1.45, frames of few large
-    splats at 1.8 to 4: 1,500 of 0.14 on 200 x 150 pixels 262 us in one window and 205 in several.)
+    far below that, and no more than half of what the first frame with these windows had.  (At the library's own windows
+    100k and 500k frames stand at 1.2 to 1.45, frames of few large splats at 1.8 to 4: 1,500 of 0.14 on 200 x 150 pixels 262 us
+    in one window and 205 in several.)
 
     What was learned is kept by the kind of frame (layers, precision, whose lists, the library's windows), so that calls of two
     kinds may alternate."""
